@@ -1,4 +1,4 @@
-// Exact temperature / top-k / top-p / categorical selection over the WHOLE vocabulary, one CTA per row, plus the
+// Exact temperature / top-k / top-p / categorical selection over the WHOLE vocabulary, a cluster of CTAs per row, plus the
 // sequence bookkeeping of the step — the second (and last) launch of a sampling decode step at any tp.
 //
 // Reference behaviour: the HF Flax warpers as configured by /root/reference/jax_llama/generation.py:28-41 —
@@ -9,22 +9,37 @@
 //
 //   * every token gets the 64-bit sort key (order-preserving bits of its scaled logit, ~index): larger key = better,
 //     equal logits order by LOWER index — selection is deterministic whatever the thread arrival order;
-//   * "the element whose interval of the descending cumulative sum contains `target`" is found by a radix select
-//     (11 + 11 + 10 bits of the value, then the index among exact ties) over integer histograms.  With unit weights
-//     this is the k-th largest element (top-k); with probability weights it is the nucleus boundary (top-p) and the
-//     sampled token (inverse CDF at u·Z).  Probabilities are exp(z − max) in 2^-40 fixed point, so every histogram
-//     is an integer sum: associative, hence bit-identical on every rank and every run (float atomics are not);
+//   * the question asked of a row is always "the element whose interval of the descending cumulative sum contains `target`":
+//     with unit weights it is the k-th largest element (top-k), with probability weights the nucleus boundary (top-p) and the
+//     sampled token (inverse CDF at u·Z).  Probabilities are exp(z − max) in 2^-40 fixed point, so every sum is an integer sum:
+//     associative, hence bit-identical on every rank and every run (float atomics are not);
+//   * a cluster of up to 8 CTAs shares a row.  ONE pass over the logits fills a histogram (counts and masses) over equal steps of
+//     z below the row's maximum; its prefix sums answer all three questions down to a bin, because top-k and top-p only cut the
+//     same cumulative sum off at an earlier point.  The few elements of the bin are then gathered and ranked exactly; a bin with
+//     more than SF_CAND elements (plateaus, coarse logits) is first narrowed by histograms over its own (key, ~index) range.
+//     What bounds it is the chain of cluster barriers and short passes, not the 0.5 MB of a row: 4 rows of 128256, top-p 0.95, on
+//     one B200: 632 us with one CTA per row and three radix passes per question (the top bits of normal logits fall into a few
+//     dozen bins, so its 64-bit shared-memory atomics serialised), 30 us now;
+//   * rows that hold a NaN or whose maximum is not finite take the radix select that the first form of this kernel ran for every
+//     row (sf_select): their masses are not sums of probabilities, and what they return stays what it was.
 //   * tensor parallelism: the decode kernel stores every rank's logits shard into every rank's [B, V] buffer with
 //     multimem.st, so all ranks run this kernel on identical inputs with the same Philox stream (seed, step, row) and
 //     pick the same token without a broadcast.  The kernel first waits for the arg-max candidate packets of all ranks
 //     (they are published after a system fence that follows the logits stores).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "jllama_b200.h"
+
+namespace cg = cooperative_groups;
 
 namespace jl {
 
 constexpr int SF_THREADS = 1024;
 constexpr int SF_BINS = 2048;
+constexpr int SF_CAND = 256;                       // elements ranked directly (four threads each)
+constexpr int SF_MAX_CLUSTER = 8;
+constexpr float SF_STEP = 2047.0f / 28.0f;         // bins per unit of z: beyond 28 below the maximum a mass is zero (28 > 40 ln 2)
 constexpr float SF_FIX = 1099511627776.f;          // 2^40
 
 __device__ __forceinline__ uint32_t sf_key(float z) {
@@ -60,8 +75,11 @@ struct SfRow {
 __device__ __forceinline__ bool sf_in_set(const SfRow& r, uint32_t key, int i) {
   return key > r.kmin || (key == r.kmin && i <= r.imax);
 }
+// z = x · inv_temp rounded to fp32, and its distance to the maximum likewise: never contracted into one operation, so that every pass
+// over a row sees the same keys, bins and masses
+__device__ __forceinline__ float sf_scaled(float x, float inv_temp) { return __fmul_rn(x, inv_temp); }
 __device__ __forceinline__ unsigned long long sf_mass(const SfRow& r, float z) {
-  return (unsigned long long)(exp2f((z - r.zmax) * 1.4426950408889634f) * SF_FIX);
+  return (unsigned long long)(exp2f(__fmul_rn(__fsub_rn(z, r.zmax), 1.4426950408889634f)) * SF_FIX);
 }
 
 // Descending scan of the histogram (warp 0): the bin in which the running sum (starting at `base`) first exceeds
@@ -120,7 +138,7 @@ __device__ void sf_select(const SfRow& r, unsigned long long target, bool target
     for (int b = threadIdx.x; b < SF_BINS; b += SF_THREADS) hist[b] = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < r.V; i += SF_THREADS) {
-      const float z = r.x[i] * r.inv_temp;
+      const float z = sf_scaled(r.x[i], r.inv_temp);
       const uint32_t key = sf_key(z);
       if (!sf_in_set(r, key, i)) continue;
       if (done > 0 && (key >> (32 - done)) != (prefix >> (32 - done))) continue;
@@ -166,7 +184,7 @@ __device__ void sf_select(const SfRow& r, unsigned long long target, bool target
   if (threadIdx.x == 0) { *s_idx = 0x7fffffff; *s_bin = 0; }
   __syncthreads();
   for (int i = threadIdx.x; i < r.V; i += SF_THREADS) {
-    const uint32_t key = sf_key(r.x[i] * r.inv_temp);
+    const uint32_t key = sf_key(sf_scaled(r.x[i], r.inv_temp));
     if (key == prefix && sf_in_set(r, key, i)) { atomicMin(s_idx, i); atomicAdd(s_bin, 1); }
   }
   __syncthreads();
@@ -185,7 +203,7 @@ __device__ void sf_select(const SfRow& r, unsigned long long target, bool target
       for (int b = threadIdx.x; b < SF_BINS; b += SF_THREADS) hist[b] = 0;
       __syncthreads();
       for (int i = threadIdx.x; i < r.V; i += SF_THREADS) {
-        const uint32_t key = sf_key(r.x[i] * r.inv_temp);
+        const uint32_t key = sf_key(sf_scaled(r.x[i], r.inv_temp));
         if (key != prefix || !sf_in_set(r, key, i)) continue;
         if (idone > 0 && (i >> (17 - idone)) != (ipre >> (17 - idone))) continue;
         // ascending index order = descending (nb − 1 − digit)
@@ -210,7 +228,7 @@ struct SampleFullParams {
   const float* logits;      // [B, ld] fp32 (full vocabulary)
   int V, ld, B;
   float inv_temp, top_p;
-  int top_k, greedy;
+  int top_k;
   unsigned long long seed;
   const int* step;
   int* tok;
@@ -221,13 +239,306 @@ struct SampleFullParams {
   int* cur_len; int* cache_len; int* step_rw; int* n_unfinished;
 };
 
-__global__ void __launch_bounds__(SF_THREADS) sample_full_kernel(const SampleFullParams p) {
+// Rows whose masses are not probabilities (a NaN, an infinite maximum): one CTA, radix selects over the whole row.
+__device__ int sf_radix_row(SfRow r, int top_k, float top_p, float u01, unsigned long long* hist) {
+  __shared__ unsigned long long s_before, s_total;
+  __shared__ int s_bin, s_idx;
+  uint32_t key; int idx; unsigned long long before, total;
+  if (top_k > 0 && top_k < r.V) {
+    sf_select<true>(r, (unsigned long long)(top_k - 1), false, 0.0, hist, &s_bin, &s_before, &s_total, &s_idx, &key, &idx, &before, &total);
+    r.kmin = key; r.imax = idx;
+  }
+  if (top_p < 1.0f) {
+    sf_select<false>(r, 0, true, (double)top_p, hist, &s_bin, &s_before, &s_total, &s_idx, &key, &idx, &before, &total);
+    r.kmin = key; r.imax = idx;
+  }
+  // inverse CDF over the kept set, descending order
+  sf_select<false>(r, 0, true, (double)u01, hist, &s_bin, &s_before, &s_total, &s_idx, &key, &idx, &before, &total);
+  return idx;
+}
+
+struct SfShared {
+  // this CTA's histogram of the level in work: counts, and masses (< 2^41) in three 14-bit digits, so that 32-bit atomics cannot
+  // overflow for a slice of up to 2^17 elements
+  unsigned int cnt[SF_BINS], m0[SF_BINS], m1[SF_BINS], m2[SF_BINS];
+  // rank 0 of the cluster: prefix sums before each bin (one more entry: the total) of the first level, and of the narrowing level
+  unsigned long long pm[SF_BINS + 1], rm[SF_BINS + 1];
+  unsigned int pc[SF_BINS + 1], rc[SF_BINS + 1];
+  unsigned long long cand[SF_CAND], cmass[SF_CAND];
+  unsigned long long warp_m[32];
+  unsigned int warp_c[32];
+  // rank 0's decisions, written into every CTA
+  int bin, n;
+  unsigned long long klo, khi;
+  // rank 0: where the gathered elements and the range of a bin meet; the answer of a question
+  unsigned int n_cand;
+  unsigned long long rlo[SF_MAX_CLUSTER], rhi[SF_MAX_CLUSTER];
+  unsigned long long base_m; unsigned int base_c;
+  unsigned long long res_comp, res_before, res_mass;
+};
+
+struct SfBest {
+  unsigned long long best[SF_MAX_CLUSTER];         // per CTA: best (key, ~index) of its slice
+  unsigned int odd[SF_MAX_CLUSTER];                // per CTA: it saw a NaN
+  unsigned long long best_local;
+  unsigned int odd_local;
+};
+
+// (a barrier of one CTA costs less than a cluster's)
+__device__ __forceinline__ void sf_sync(cg::cluster_group& cl, int size) {
+  if (size > 1) cl.sync(); else __syncthreads();
+}
+
+// One row as its cluster sees it.
+struct SfCluster {
+  SfShared* s;
+  const float* x;
+  int V, lo, hi, vec;           // this CTA's slice [lo, hi)
+  float inv_temp, zmax;
+  uint32_t kmax;                // key of the row's maximum
+  int rank, size;
+  bool count_all;               // elements without mass count too (a top-k question will be asked)
+  SfRow row;
+
+  template <typename F> __device__ __forceinline__ void for_slice(F f) const {
+    if (vec) {                                              // lo is a multiple of four
+      for (int i = lo + 4 * (int)threadIdx.x; i < hi; i += 4 * SF_THREADS) {
+        if (i + 4 <= hi) {
+          const float4 v = *reinterpret_cast<const float4*>(x + i);
+          f(v.x, i); f(v.y, i + 1); f(v.z, i + 2); f(v.w, i + 3);
+        } else {
+          for (int j = i; j < hi; ++j) f(x[j], j);
+        }
+      }
+    } else {
+      for (int i = lo + (int)threadIdx.x; i < hi; i += SF_THREADS) f(x[i], i);
+    }
+  }
+  // monotone in z: larger z, smaller or equal bin
+  __device__ __forceinline__ int bin_of(float z) const {
+    const float d = __fmul_rn(__fsub_rn(zmax, z), SF_STEP);
+    return d < (float)(SF_BINS - 1) ? (int)d : SF_BINS - 1;
+  }
+  static __device__ __forceinline__ unsigned long long comp(uint32_t key, int i) {
+    return ((unsigned long long)key << 32) | (unsigned)(0x7fffffff - i);
+  }
+  static __device__ __forceinline__ float z_of(unsigned long long c) {
+    const uint32_t k = (uint32_t)(c >> 32);
+    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+  }
+  __device__ __forceinline__ void add(int bin, unsigned long long m) const {
+    atomicAdd(&s->cnt[bin], 1u);
+    if (m) {
+      const unsigned d0 = (unsigned)m & 0x3fffu, d1 = (unsigned)(m >> 14) & 0x3fffu, d2 = (unsigned)(m >> 28);
+      if (d0) atomicAdd(&s->m0[bin], d0);
+      if (d1) atomicAdd(&s->m1[bin], d1);
+      if (d2) atomicAdd(&s->m2[bin], d2);
+    }
+  }
+  __device__ __forceinline__ void clear() const {
+    for (int b = threadIdx.x; b < SF_BINS; b += SF_THREADS) { s->cnt[b] = 0; s->m0[b] = 0; s->m1[b] = 0; s->m2[b] = 0; }
+    __syncthreads();
+  }
+  // all CTAs' histograms -> exclusive prefix sums in rank 0 (pm / pc, or rm / rc); every CTA adds up its share of the bins
+  __device__ void merge(bool narrow) const {
+    cg::cluster_group cl = cg::this_cluster();
+    sf_sync(cl, size);                                              // every CTA's histogram is complete
+    SfShared* lead = cl.map_shared_rank(s, 0);
+    unsigned long long* tm = narrow ? lead->rm : lead->pm;
+    unsigned int* tc = narrow ? lead->rc : lead->pc;
+    const int share = SF_BINS / size;
+    for (int b = rank * share + threadIdx.x; b < (rank + 1) * share; b += SF_THREADS) {
+      unsigned long long m = 0;
+      unsigned int c = 0;
+      for (int r = 0; r < size; ++r) {
+        const SfShared* o = cl.map_shared_rank(s, r);
+        c += o->cnt[b];
+        m += (unsigned long long)o->m0[b] + ((unsigned long long)o->m1[b] << 14) + ((unsigned long long)o->m2[b] << 28);
+      }
+      tm[b] = m; tc[b] = c;
+    }
+    sf_sync(cl, size);                                              // rank 0 holds all totals
+    if (rank != 0) return;
+    unsigned long long* lm = narrow ? s->rm : s->pm;
+    unsigned int* lc = narrow ? s->rc : s->pc;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const unsigned long long m0 = lm[2 * t], m1 = lm[2 * t + 1];
+    const unsigned int c0 = lc[2 * t], c1 = lc[2 * t + 1];
+    unsigned long long im = m0 + m1;
+    unsigned int ic = c0 + c1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long a = __shfl_up_sync(0xffffffffu, im, o);
+      const unsigned int c = __shfl_up_sync(0xffffffffu, ic, o);
+      if (lane >= o) { im += a; ic += c; }
+    }
+    if (lane == 31) { s->warp_m[w] = im; s->warp_c[w] = ic; }
+    __syncthreads();
+    if (w == 0) {
+      unsigned long long a = s->warp_m[lane];
+      unsigned int c = s->warp_c[lane];
+      const unsigned long long a0 = a;
+      const unsigned int cc0 = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long u = __shfl_up_sync(0xffffffffu, a, o);
+        const unsigned int v = __shfl_up_sync(0xffffffffu, c, o);
+        if (lane >= o) { a += u; c += v; }
+      }
+      s->warp_m[lane] = a - a0; s->warp_c[lane] = c - cc0;
+    }
+    __syncthreads();
+    const unsigned long long em = s->warp_m[w] + im - (m0 + m1);
+    const unsigned int ec = s->warp_c[w] + ic - (c0 + c1);
+    lm[2 * t] = em; lm[2 * t + 1] = em + m0;
+    lc[2 * t] = ec; lc[2 * t + 1] = ec + c0;
+    if (t == SF_THREADS - 1) { lm[SF_BINS] = em + m0 + m1; lc[SF_BINS] = ec + c0 + c1; }
+    __syncthreads();
+  }
+  // rank 0: the bin whose interval holds `target` (relative to the prefix arrays) -> s->bin, s->n, base_m / base_c advanced
+  __device__ __forceinline__ void find(const unsigned long long* lm, const unsigned int* lc, bool by_count, unsigned long long target) const {
+    if (threadIdx.x == 0) { s->bin = SF_BINS - 1; s->n = 0; }      // (a target beyond the total: nothing)
+    __syncthreads();
+    for (int b = threadIdx.x; b < SF_BINS; b += SF_THREADS) {
+      const unsigned long long a = by_count ? lc[b] : lm[b], e = by_count ? lc[b + 1] : lm[b + 1];
+      if (a <= target && target < e) { s->bin = b; s->n = (int)(lc[b + 1] - lc[b]); }
+    }
+    __syncthreads();
+  }
+  // rank 0's bin, n and range into every CTA
+  __device__ __forceinline__ void publish() const {
+    cg::cluster_group cl = cg::this_cluster();
+    if (rank == 0) {
+      __syncthreads();
+      if (threadIdx.x > 0 && (int)threadIdx.x < size) {
+        SfShared* o = cl.map_shared_rank(s, (int)threadIdx.x);
+        o->bin = s->bin; o->n = s->n; o->klo = s->klo; o->khi = s->khi;
+      }
+    }
+    sf_sync(cl, size);
+  }
+  // The element whose interval of the descending cumulative sum (counts or masses) holds `target` (rank 0's value counts; it lies
+  // below the total).  Executed by all CTAs of the cluster in step; the answer is in rank 0's res_*.
+  __device__ void select(bool by_count, unsigned long long target) const {
+    cg::cluster_group cl = cg::this_cluster();
+    SfShared* lead = cl.map_shared_rank(s, 0);
+    if (rank == 0) {
+      find(s->pm, s->pc, by_count, target);
+      if (threadIdx.x == 0) {
+        s->base_m = s->pm[s->bin]; s->base_c = s->pc[s->bin];
+        s->n_cand = 0;
+        s->res_comp = 0x7fffffffull; s->res_before = 0; s->res_mass = 0;
+      }
+    }
+    publish();
+    int bin = s->bin, n = s->n;
+    unsigned long long klo = 0, khi = ~0ull;
+    if (n > SF_CAND) {                                      // too many to rank: the range of the bin's elements ...
+      unsigned long long mn = ~0ull, mx = 0ull;
+      for_slice([&](float v, int i) {
+        const float z = sf_scaled(v, inv_temp);
+        if (bin_of(z) != bin || !(count_all || sf_mass(row, z) > 0)) return;
+        const unsigned long long c = comp(sf_key(z), i);
+        mn = c < mn ? c : mn;
+        mx = c > mx ? c : mx;
+      });
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long a = __shfl_xor_sync(0xffffffffu, mn, o), b = __shfl_xor_sync(0xffffffffu, mx, o);
+        mn = a < mn ? a : mn;
+        mx = b > mx ? b : mx;
+      }
+      if ((threadIdx.x & 31) == 0) { s->warp_m[threadIdx.x >> 5] = mn; s->cmass[threadIdx.x >> 5] = mx; }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int w = 1; w < SF_THREADS / 32; ++w) {
+          mn = s->warp_m[w] < mn ? s->warp_m[w] : mn;
+          mx = s->cmass[w] > mx ? s->cmass[w] : mx;
+        }
+        lead->rlo[rank] = mn; lead->rhi[rank] = mx;
+      }
+      sf_sync(cl, size);
+      if (rank == 0 && threadIdx.x == 0) {
+        for (int r = 0; r < size; ++r) {
+          mn = s->rlo[r] < mn ? s->rlo[r] : mn;
+          mx = s->rhi[r] > mx ? s->rhi[r] : mx;
+        }
+        s->klo = mn; s->khi = mx;
+      }
+      publish();
+      klo = s->klo; khi = s->khi;
+      for (int level = 0; level < 6 && n > SF_CAND; ++level) {       // ... cut into 2048 parts, until few enough are left (64 bits: six times)
+        const unsigned long long range = khi - klo;
+        const int bits = 64 - __clzll((long long)range), shift = bits > 11 ? bits - 11 : 0;
+        clear();
+        for_slice([&](float v, int i) {
+          const float z = sf_scaled(v, inv_temp);
+          const unsigned long long c = comp(sf_key(z), i);
+          if (c < klo || c > khi) return;
+          const unsigned long long m = sf_mass(row, z);
+          if (!count_all && m == 0) return;
+          add((int)((khi - c) >> shift), m);
+        });
+        merge(true);
+        if (rank == 0) {
+          find(s->rm, s->rc, by_count, target - (by_count ? (unsigned long long)s->base_c : s->base_m));
+          if (threadIdx.x == 0) {
+            s->base_m += s->rm[s->bin]; s->base_c += s->rc[s->bin];
+            const unsigned long long top = khi - ((unsigned long long)s->bin << shift);
+            const unsigned long long span = (1ull << shift) - 1ull;
+            s->khi = top;
+            s->klo = top - klo > span ? top - span : klo;
+          }
+        }
+        publish();
+        n = s->n; klo = s->klo; khi = s->khi;
+      }
+      bin = -1;
+    }
+    for_slice([&](float v, int i) {                          // gather
+      const float z = sf_scaled(v, inv_temp);
+      if (bin >= 0 && bin_of(z) != bin) return;
+      const unsigned long long c = comp(sf_key(z), i);
+      if (bin < 0 && (c < klo || c > khi)) return;
+      if (!count_all && sf_mass(row, z) == 0) return;
+      const unsigned slot = atomicAdd(&lead->n_cand, 1u);
+      if (slot < SF_CAND) lead->cand[slot] = c;
+    });
+    sf_sync(cl, size);
+    if (rank != 0) return;
+    const int nc = min((int)s->n_cand, SF_CAND);
+    if ((int)threadIdx.x < nc) s->cmass[threadIdx.x] = sf_mass(row, z_of(s->cand[threadIdx.x]));
+    __syncthreads();
+    const int c = threadIdx.x >> 2;
+    const unsigned long long mine = c < nc ? s->cand[c] : 0ull;
+    unsigned long long bm = 0;
+    unsigned int bc = 0;
+    for (int j = threadIdx.x & 3; j < nc; j += 4)
+      if (s->cand[j] > mine) { bm += s->cmass[j]; ++bc; }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) { bm += __shfl_xor_sync(0xffffffffu, bm, o); bc += __shfl_xor_sync(0xffffffffu, bc, o); }
+    if (c < nc && (threadIdx.x & 3) == 0) {
+      bm += s->base_m;
+      const unsigned long long m = s->cmass[c];
+      const bool hit = by_count ? (unsigned long long)bc + s->base_c == target : bm <= target && target - bm < m;
+      if (hit) { s->res_comp = mine; s->res_before = bm; s->res_mass = m; }
+    }
+    __syncthreads();
+  }
+};
+
+// GREEDY (temperature 0): the arg-max alone, without the histograms' shared memory and registers (two CTAs fit an SM).
+template <bool GREEDY>
+__global__ void __launch_bounds__(SF_THREADS, GREEDY ? 2 : 1) sample_full_kernel(const SampleFullParams p) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ unsigned long long hist[SF_BINS];
-  __shared__ unsigned long long s_before, s_total, s_kk;
-  __shared__ int s_bin, s_idx, s_last;
-  const int row = blockIdx.x;
+  extern __shared__ __align__(16) unsigned char sf_smem[];
+  SfShared& sh = *reinterpret_cast<SfShared*>(sf_smem);
+  __shared__ int s_last;
+  __shared__ SfBest sb;
+  cg::cluster_group cl = cg::this_cluster();
+  const int csize = (int)cl.num_blocks(), crank = (int)cl.block_rank();
+  const int row = blockIdx.x / csize;
   if (p.cand != nullptr) {
     // every (rank, CTA) of the decode kernel has published its candidate for this row ⇒ its logits stores landed
     const unsigned int gen_now = *reinterpret_cast<const volatile unsigned int*>(p.gen);
@@ -250,46 +561,81 @@ __global__ void __launch_bounds__(SF_THREADS) sample_full_kernel(const SampleFul
     __threadfence_system();
     __syncthreads();
   }
-  SfRow r;
-  r.x = p.logits + (size_t)row * p.ld; r.V = p.V; r.inv_temp = p.inv_temp; r.kmin = 0; r.imax = 0x7fffffff;
-  // ---- max of the scaled logits and the best (key, ~index) in one pass
-  unsigned long long best = 0;
-  for (int i = threadIdx.x; i < p.V; i += SF_THREADS) {
-    const unsigned long long kk = ((unsigned long long)sf_key(r.x[i] * p.inv_temp) << 32) | (unsigned)(0x7fffffff - i);
-    best = kk > best ? kk : best;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long t = __shfl_xor_sync(0xffffffffu, best, o);
-    best = t > best ? t : best;
-  }
-  if (threadIdx.x == 0) s_kk = 0;
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) atomicMax(&s_kk, best);
-  __syncthreads();
-  best = s_kk;
-  int token = 0x7fffffff - (int)(best & 0xffffffffu);
+  SfCluster q;
+  q.s = &sh; q.x = p.logits + (size_t)row * p.ld; q.V = p.V; q.inv_temp = p.inv_temp; q.rank = crank; q.size = csize;
   {
-    const uint32_t k = (uint32_t)(best >> 32);
-    const uint32_t u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-    r.zmax = __uint_as_float(u);
+    const int per = (p.V / csize + 4) & ~3;                 // a multiple of four, csize of them cover V
+    q.lo = min(p.V, crank * per);
+    q.hi = min(p.V, q.lo + per);
   }
-  if (!p.greedy) {
-    uint32_t key; int idx; unsigned long long before, total;
-    if (p.top_k > 0 && p.top_k < p.V) {
-      sf_select<true>(r, (unsigned long long)(p.top_k - 1), false, 0.0, hist, &s_bin, &s_before, &s_total, &s_idx, &key, &idx,
-                      &before, &total);
-      r.kmin = key; r.imax = idx;
+  q.vec = ((uintptr_t)q.x & 15) == 0;
+  q.count_all = !GREEDY && p.top_k > 0 && p.top_k < p.V;
+  // ---- best (key, ~index) of the row: the arg-max, and the maximum of the scaled logits
+  if (threadIdx.x == 0) { sb.best_local = 0; sb.odd_local = 0; }
+  __syncthreads();
+  {
+    unsigned long long best = 0;
+    bool nan = false;
+    q.for_slice([&](float v, int i) {
+      const float z = sf_scaled(v, p.inv_temp);
+      const unsigned long long kk = SfCluster::comp(sf_key(z), i);
+      best = kk > best ? kk : best;
+      nan |= !(z == z);
+    });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long t = __shfl_xor_sync(0xffffffffu, best, o);
+      best = t > best ? t : best;
     }
-    if (p.top_p < 1.0f) {
-      sf_select<false>(r, 0, true, (double)p.top_p, hist, &s_bin, &s_before, &s_total, &s_idx, &key, &idx, &before, &total);
-      r.kmin = key; r.imax = idx;
-    }
-    // inverse CDF over the kept set, descending order
+    const bool any_nan = __any_sync(0xffffffffu, nan);
+    if ((threadIdx.x & 31) == 0) { atomicMax(&sb.best_local, best); if (any_nan) sb.odd_local = 1; }
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < csize) {
+    SfBest* o = cl.map_shared_rank(&sb, (int)threadIdx.x);
+    o->best[crank] = sb.best_local; o->odd[crank] = sb.odd_local;
+  }
+  sf_sync(cl, csize);
+  unsigned long long best = 0;
+  bool odd = false;
+  for (int r = 0; r < csize; ++r) { best = sb.best[r] > best ? sb.best[r] : best; odd |= sb.odd[r] != 0; }
+  int token = 0x7fffffff - (int)(best & 0xffffffffu);
+  q.zmax = SfCluster::z_of(best);
+  q.row = SfRow{q.x, p.V, p.inv_temp, q.zmax, 0u, 0x7fffffff};
+  if constexpr (!GREEDY) {
+    // Philox of (step, row) against the total of the kept set: the same target whatever the route
     const float u01 = sf_uniform(p.seed, (unsigned)(p.step ? *p.step : 0), (unsigned)row);
-    sf_select<false>(r, 0, true, (double)u01, hist, &s_bin, &s_before, &s_total, &s_idx, &key, &idx, &before, &total);
-    token = idx;
+    if (odd || !(fabsf(q.zmax) < INFINITY)) {
+      if (crank == 0) token = sf_radix_row(q.row, p.top_k, p.top_p, u01, reinterpret_cast<unsigned long long*>(sh.cnt));
+    } else {
+      q.clear();
+      q.for_slice([&](float v, int) {
+        const float z = sf_scaled(v, p.inv_temp);
+        const unsigned long long m = sf_mass(q.row, z);
+        if (q.count_all || m > 0) q.add(q.bin_of(z), m);
+      });
+      q.merge(false);
+      unsigned long long total = crank == 0 ? sh.pm[SF_BINS] : 0;
+      // target of a fraction of the kept set's mass Z: max(fraction·Z, 1) − 1 (a token is kept while the mass before it is < fraction·Z)
+      auto target_of = [&](double fraction) {
+        unsigned long long t = (unsigned long long)((double)total * fraction);
+        if (t > total) t = total;
+        return t > 0 ? t - 1 : 0;
+      };
+      if (q.count_all) {
+        q.select(true, (unsigned long long)(p.top_k - 1));
+        if (crank == 0) total = sh.res_before + sh.res_mass;
+      }
+      if (p.top_p < 1.0f) {
+        q.select(false, target_of((double)p.top_p));
+        if (crank == 0) total = sh.res_before + sh.res_mass;
+      }
+      q.select(false, target_of((double)u01));
+      if (crank == 0) token = 0x7fffffff - (int)(sh.res_comp & 0xffffffffu);
+    }
   }
+  sf_sync(cl, csize);                                                // no CTA leaves while another may still write into its shared memory
+  if (crank != 0) return;
   if (threadIdx.x == 0) {
     if (token < 0 || token >= p.V) token = 0;
     p.tok[row] = token;
@@ -299,7 +645,7 @@ __global__ void __launch_bounds__(SF_THREADS) sample_full_kernel(const SampleFul
   __syncthreads();
   if (threadIdx.x == 0) {
     const int prev = atomicAdd(p.ticket, 1);
-    s_last = prev == (int)gridDim.x - 1;
+    s_last = prev == p.B - 1;
     if (s_last) *p.ticket = 0;
   }
   __syncthreads();
@@ -346,13 +692,43 @@ extern "C" JL_API int jl_sample_full(const float* logits, int B, int V, int ld, 
   if (num_sms <= 0) num_sms = 148;
   SampleFullParams p{};
   p.logits = logits; p.V = V; p.ld = ld; p.B = B;
-  p.greedy = temperature == 0.0f;
-  p.inv_temp = p.greedy ? 1.0f : 1.0f / temperature;
+  const bool greedy = temperature == 0.0f;
+  p.inv_temp = greedy ? 1.0f : 1.0f / temperature;
   p.top_k = top_k; p.top_p = top_p; p.seed = seed; p.step = step; p.tok = tok;
   p.cand = (const uint2*)cand; p.gen = gen; p.tp = tp; p.grid = num_sms; p.two_l = 2 * L; p.rank = rank;
   p.ticket = ticket; p.next_ids = next_ids; p.finished = finished; p.sequences = sequences;
   p.max_len = max_len; p.eos = eos; p.pad = pad;
   p.cur_len = cur_len; p.cache_len = cache_len; p.step_rw = step_rw; p.n_unfinished = n_unfinished;
-  JL_CUDA(launch_pdl(sample_full_kernel, dim3(B), dim3(SF_THREADS), 0, (cudaStream_t)stream, p));
+  // CTAs per row: as many as leave every CTA a slice of at least 4096 logits (below that the barriers cost more than the slice) and
+  // all rows' CTAs resident at once, one per SM.  Clusters of eight only where two thirds of the SMs hold them: a cluster stays within
+  // one GPC, and 16 of eight did not all fit (16 rows of 128256: 51 us in clusters of eight, 38 us of four).
+  // Measured, nucleus 0.95, one CTA with radix passes -> now: 1 x 8000 78 -> 19 us, 1 x 32000 177 -> 25, 4 x 128256 632 -> 29,
+  // 24 x 128256 650 -> 39, 64 x 128256 645 -> 59, 200 x 128256 1062 -> 180, 2000 x 8000 685 -> 191; equal logits 27.4 ms -> 70 us.
+  int C = 1;
+  while (C < SF_MAX_CLUSTER && V / (2 * C) >= 4096 && (long)B * 2 * C <= (2 * C < SF_MAX_CLUSTER ? num_sms : num_sms * 2 / 3)) C *= 2;
+  auto* kernel = greedy ? sample_full_kernel<true> : sample_full_kernel<false>;
+  const size_t smem = greedy ? 0 : sizeof(SfShared);
+  if (!greedy) JL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)B * C);
+  cfg.blockDim = dim3(SF_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (pdl_enabled()) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (C > 1) {                                               // (a grid without the attribute is one of clusters of one)
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = C;
+    attr[na].val.clusterDim.y = 1;
+    attr[na++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  count_launch();
+  JL_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
   return JL_OK;
 }

@@ -72,3 +72,73 @@ def test_same_seed_same_tokens_different_seed_different_tokens():
     b = K.sample_full(x, temperature=0.9, top_k=50, top_p=0.9, seed=1, step=step)
     c = K.sample_full(x, temperature=0.9, top_k=50, top_p=0.9, seed=2, step=step)
     assert torch.equal(a, b) and not torch.equal(a, c)
+
+
+def uniform_of(seed, step, row):
+    """Philox-4x32-10 keyed by the seed at counter (step, row), as a number in (0, 1)."""
+    m = 0xFFFFFFFF
+    c = [step & m, row & m, 0x9E3779B9, 0xBB67AE85]
+    k = [seed & m, (seed >> 32) & m]
+    for _ in range(10):
+        p0, p1 = 0xD2511F53 * c[0], 0xCD9E8D57 * c[2]
+        c = [(p1 >> 32) ^ c[1] ^ k[0], p1 & m, (p0 >> 32) ^ c[3] ^ k[1], p0 & m]
+        k = [(k[0] + 0x9E3779B9) & m, (k[1] + 0xBB67AE85) & m]
+    return ((c[0] >> 8) + 0.5) / 16777216.0
+
+
+@pytest.mark.parametrize("rows,vocab,pitch,kind", [
+    (1, 128256, 0, "normal"), (4, 128256, 0, "normal"), (30, 131072, 0, "normal"), (200, 8195, 1, "normal"), (3, 8191, 2, "normal"),
+    (2, 8192, 0, "normal"), (5, 77, 3, "normal"), (2, 1, 0, "normal"), (3, 50001, 0, "coarse"), (2, 16384, 0, "plateau"), (4, 32003, 5, "masked"),
+    (2, 40000, 0, "far")])
+@pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (0, 0.9), (300, 0.95), (7, 1.0)])
+def test_tokens_are_the_inverse_cdf_of_the_kept_set(rows, vocab, pitch, kind, top_k, top_p):
+    """Slices of one to eight CTAs, rows without 16-byte alignment, bins with many equal or neighbouring values, masked tokens."""
+    g = torch.Generator().manual_seed(rows * vocab)
+    x = torch.randn(rows, vocab + pitch, generator=g) * 3.0
+    if kind == "coarse":
+        x = (x * 2).round() / 2                            # a few dozen values, thousands of tokens on each
+    elif kind == "plateau":
+        x = x * 1e-4 + 50.0                                # everything within one bin, neighbouring floats
+    elif kind == "masked":
+        x[:, ::3] = float("-inf")
+    elif kind == "far":
+        x[:, 100:] -= 1000.0                               # most tokens have no mass: a large top-k reaches into them
+    x = x.cuda()[:, :vocab]
+    tok = K.sample_full(x, temperature=0.75, top_k=top_k, top_p=top_p, seed=12345678901, step=torch.tensor([9], dtype=torch.int32, device="cuda"))
+    inv_temp = torch.tensor(1.0) / torch.tensor(0.75)       # the kernel's float32 scale
+    for r in range(rows):
+        z = (x[r].cpu() * inv_temp).double()
+        order = torch.sort(z, descending=True, stable=True).indices
+        if top_k and top_k < vocab:
+            order = order[:top_k]
+        p = torch.exp(z[order] - z.max())
+        if top_p < 1.0:
+            before = torch.cumsum(p, 0) - p
+            # exponentials and fixed point differ from float64 by about 2^-21 of a mass: tokens that close to the cut may go either way
+            sure = order[before < top_p * p.sum() * (1 - 2e-6)]
+            order = order[before < top_p * p.sum() * (1 + 2e-6)]
+            p = p[:order.numel()]
+            lo_total, hi_total = p[:sure.numel()].sum().item(), p.sum().item()
+        else:
+            lo_total = hi_total = p.sum().item()
+        u = uniform_of(12345678901, 9, r)
+        edge = torch.cumsum(p, 0)
+        i = int((order == int(tok[r])).nonzero().item())   # outside the kept set: no such element
+        before, after = (edge[i] - p[i]).item(), edge[i].item()
+        slack = 4e-6 * hi_total
+        assert before <= u * hi_total + slack and after >= u * lo_total - slack, (r, u, before, after, hi_total)
+
+
+@pytest.mark.parametrize("bad", ["nan", "inf", "all_masked"])
+def test_rows_without_probabilities_still_give_a_token(bad):
+    x = torch.randn(3, 20000, generator=torch.Generator().manual_seed(1)).cuda()
+    if bad == "nan":
+        x[1, 77] = float("nan")
+    elif bad == "inf":
+        x[1, 77] = float("inf")
+    else:
+        x[1] = float("-inf")
+    y = K.sample_full(x, temperature=0.9, top_p=0.9, seed=3)
+    assert bool(((y >= 0) & (y < 20000)).all())
+    clean = K.sample_full(x[[0, 0, 2]].contiguous(), temperature=0.9, top_p=0.9, seed=3)
+    assert y[0] == clean[0] and y[2] == clean[2]

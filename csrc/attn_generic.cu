@@ -11,7 +11,7 @@
 //  * attn_rows_kernel   — 16 queries of one head per CTA against key / value tiles of 32 rows staged in shared memory
 //    (one key per lane for the scores, one value column per lane for the output), online softmax in fp32, causal over
 //    slots [pad_left[b], slot], optional output gate sigmoid(g) per head or per channel.  Prompts of any length; exact path for
-//    float32 and for head sizes the tensor-core kernels are not built for.
+//    float32 and for head sizes the tensor-core kernels (flash_wide.cu: 64 to 256 channels, values of 64 or 128) are not built for.
 //  * attn_decode_kernel — one CTA per (row, head) for a single new token: its warps take interleaved blocks of 32 keys
 //    and merge their (max, sum, output) triples in shared memory (what runs when the caller brings no scratch).
 //  * attn_split_kernel + attn_merge_kernel — a single new token with the keys split over CTAs: a CTA stages 32-key tiles
@@ -25,6 +25,7 @@
 // window limits a query to the last `window` slots up to its own.
 //
 // Input q / k / v / gate are columns of one fp32 projection buffer (row pitch ldy), as the fused projection writes them.
+#include "flash_wide.cuh"
 #include "jllama_b200.h"
 #include "seq_types.cuh"
 
@@ -944,6 +945,14 @@ static int attn_launch(const void* q, const void* k_cache, const void* v_cache, 
   AttnParams p{B, S, H, G, D, Dv, T_cap, ldk, ldv, k_bs, k_hs, v_bs, v_hs, window, scale, cache_len, pad_left, gate, ldg, sink, out32,
                chunk, sink_logit, vcos, vsin, v_max_pos, v_layout, softcap, gate_cols};
   cudaStream_t st = (cudaStream_t)stream;
+  // Prompts of the head shapes the tensor-core kernel is built for.  It is the faster one at every length (a row of it costs a 64-key
+  // step what a row of attn_rows_kernel costs per key or two); fp32 outputs stay here, where probabilities have all 24 bits.
+  if (dtype == DT_BF16 && out32 == nullptr && softcap == 0.0f && vcos == nullptr && !gate_cols && scale > 0.0f &&
+      flash_wide_takes(S, D, Dv, T_cap, ldk, ldv, k_bs, k_hs, v_bs, v_hs, q, k_cache, v_cache, out)) {
+    const FlashWide w{(__nv_bfloat16*)out, cache_len, pad_left, B, S, H, G, scale * 1.4426950408889634f, window, chunk, sink, sink_logit,
+                      gate, ldg};
+    return flash_wide_launch(w, D, Dv, T_cap, ldk, ldv, k_bs, k_hs, v_bs, v_hs, q, k_cache, v_cache, st);
+  }
   if (S == 1 && scratch != nullptr && splits >= 1 && splits <= 64) {
     const int dp = ((D + 3) & ~3) + 4;
     const int rb = H / G < AS_WARPS * AS_RW ? H / G : AS_WARPS * AS_RW, nblk = (H / G + rb - 1) / rb;

@@ -250,5 +250,8 @@ int make_tmap_slab_bf16_plain(CUtensorMap* out, const void* base, uint64_t rows,
 // 3-D variant: [d2, rows, cols] with element strides (ld2, ld1, 1); box {64, box_rows, 1}.
 int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d2, uint64_t rows, uint64_t cols,
                       uint64_t ld2, uint64_t ld1, uint32_t box_rows);
+// 4-D variant: [d3, d2, rows, cols] with element strides (ld3, ld2, ld1, 1) in any order of size; box {64, box_rows, 1, 1}.
+int make_tmap_4d_bf16(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t d2, uint64_t d3, uint64_t ld1,
+                      uint64_t ld2, uint64_t ld3, uint32_t box_rows);
 
 }  // namespace jl

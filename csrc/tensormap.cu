@@ -41,7 +41,7 @@ static int encode(CUtensorMap* out, const void* base, int rank, const cuuint64_t
       set_error("TMA stride %llu bytes is not a multiple of 16", (unsigned long long)strides_bytes[i]);
       return JL_ERR_ARG;
     }
-  cuuint32_t estr[3] = {1, 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims,
                   strides_bytes, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -102,6 +102,14 @@ int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d2, uint64_t 
   cuuint64_t strides[2] = {ld1 * 2, ld2 * 2};
   cuuint32_t box[3] = {64, box_rows, 1};
   return encode(out, base, 3, dims, strides, box);
+}
+
+int make_tmap_4d_bf16(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t d2, uint64_t d3, uint64_t ld1,
+                      uint64_t ld2, uint64_t ld3, uint32_t box_rows) {
+  cuuint64_t dims[4] = {cols, rows, d2, d3};
+  cuuint64_t strides[3] = {ld1 * 2, ld2 * 2, ld3 * 2};
+  cuuint32_t box[4] = {64, box_rows, 1, 1};
+  return encode(out, base, 4, dims, strides, box);
 }
 
 }  // namespace jl

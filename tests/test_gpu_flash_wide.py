@@ -1,0 +1,85 @@
+"""Prompt attention of the generic head shapes on tensor cores (csrc/flash_wide.cu) against a float64 statement.
+
+The inputs are bfloat16 and exact in float64; what the kernel rounds is a probability as hi + lo bfloat16 (2^-17 of it), fp32 sums, and the
+output once to bfloat16 (2^-9 of a value): |error| <= 2^-8 |value| + 2^-14 of the largest value is twice what these give."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from jax_llama_b200.ops import seq_kernels as SK  # noqa: E402
+
+F64 = torch.float64
+
+
+def expected(q, k, v, scale, start, pads, window, chunk, sink, gate):
+    """q [B, S, H, D]; k [B, T, G, D]; v [B, T, G, Dv] -> [B, S, H, Dv]."""
+    B, S, H, D = q.shape
+    T, G = k.shape[1], k.shape[2]
+    i = torch.arange(start, start + S)[:, None]
+    j = torch.arange(T)[None, :]
+    out = torch.zeros(B, S, H, v.shape[-1], dtype=F64)
+    for b in range(B):
+        seen = (j <= i) & (j >= pads[b])
+        if window:
+            seen &= j > i - window
+        if chunk:
+            seen &= (j - pads[b]) // chunk == (i - pads[b]) // chunk
+        for h in range(H):
+            s = (q[b, :, h] @ k[b, :, h * G // H].T * scale).masked_fill(~seen, -math.inf)
+            m = s.max(-1, keepdim=True).values.clamp_min(-1e30)
+            e = torch.exp(s - m)
+            den = e.sum(-1, keepdim=True)
+            if sink is not None:
+                den = torch.where(den > 0, den + torch.exp(sink[h] - m), den)
+            out[b, :, h] = torch.where(den > 0, (e @ v[b, :, h * G // H]) / den.clamp_min(1e-300), 0.0)
+            if gate is not None:
+                out[b, :, h] *= torch.sigmoid(gate[b * S:(b + 1) * S, h:h + 1])
+    return out
+
+
+@pytest.mark.parametrize("D,Dv,B,S,start,T,H,G,window,chunk,extras,token_major", [
+    (192, 128, 1, 129, 0, 129, 4, 4, 0, 0, False, True), (192, 128, 2, 300, 0, 300, 2, 2, 100, 0, True, True),
+    (192, 64, 1, 2, 126, 140, 4, 2, 0, 0, False, False), (128, 128, 2, 64, 0, 64, 4, 1, 0, 0, True, False),
+    (128, 64, 1, 65, 63, 200, 2, 1, 7, 0, False, False), (64, 128, 3, 63, 0, 63, 3, 3, 0, 50, True, True),
+    (64, 64, 1, 257, 0, 257, 2, 2, 64, 0, False, False), (256, 128, 1, 200, 57, 257, 2, 1, 0, 64, False, False),
+    (256, 64, 2, 31, 0, 31, 2, 2, 0, 0, True, True)])
+def test_against_float64(D, Dv, B, S, start, T, H, G, window, chunk, extras, token_major):
+    g = torch.Generator().manual_seed(D + S)
+    bf = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16)              # noqa: E731
+    q, k, v = bf(B, S, H, D) * 2, bf(B, T, G, D), bf(B, T, G, Dv)
+    pads = [(5 + 20 * b) % max(S, 2) for b in range(B)] if start == 0 else [11] * B
+    sink = torch.randn(H, generator=g) if extras else None
+    gate = torch.randn(B * S, H, generator=g) if extras else None
+    scale = D ** -0.5
+    want = expected(q.to(F64), k.to(F64), v.to(F64), scale, start, pads, window, chunk, None if sink is None else sink.to(F64),
+                    None if gate is None else gate.to(F64))
+    layout = {}
+    if token_major:                                        # [B·T, G, d] rows, as a projection writes them
+        kc, vc = k.cuda(), v.cuda()
+        layout = dict(T_cap=T, ldk=G * D, ldv=G * Dv, strides=(T * G * D, D, T * G * Dv, Dv))
+    else:                                                  # [B, G, T, d] caches
+        kc, vc = k.transpose(1, 2).contiguous().cuda(), v.transpose(1, 2).contiguous().cuda()
+    lens = torch.tensor([start], dtype=torch.int32, device="cuda")
+    got = SK.attn_masked(q.reshape(B * S, H * D).contiguous().cuda(), kc, vc, lens, torch.tensor(pads, dtype=torch.int32, device="cuda"), B, S, H, G,
+                         D, Dv, scale, gate=None if gate is None else gate.cuda(), window=window, chunk=chunk, sink=extras,
+                         sink_logit=None if sink is None else sink.cuda(), **layout).double().cpu().view(B, S, H, Dv)
+    assert bool(torch.isfinite(got).all())
+    assert bool(((got - want).abs() <= 2 ** -8 * want.abs() + 2 ** -14 * want.abs().max()).all()), (got - want).abs().max()
+
+
+def test_probabilities_keep_more_than_one_bfloat16():
+    """Two keys whose values cancel: (p0 - p1) / (p0 + p1) of nearly equal probabilities is lost when they are rounded to 8 bits."""
+    D, S = 128, 2
+    q = torch.zeros(1, S, 1, D, dtype=torch.bfloat16)
+    q[0, :, 0, 0] = 1.0
+    k = torch.zeros(1, S, 1, D, dtype=torch.bfloat16)
+    k[0, 1, 0, 0] = 2 ** -9                                 # scores 0 and 2^-9: p1 / p0 = 1.00195
+    v = torch.ones(1, S, 1, 128, dtype=torch.bfloat16)
+    v[0, 0] = -1.0
+    want = math.tanh(2 ** -10)
+    got = SK.attn_windowed(q.view(S, D).cuda(), k.transpose(1, 2).contiguous().cuda(), v.transpose(1, 2).contiguous().cuda(),
+                           torch.zeros(1, dtype=torch.int32, device="cuda"), None, 1, S, 1, 1, D, 128, S, D, 128, 0, 1.0)
+    assert abs(float(got[1, 0]) - want) <= 2 ** -6 * want   # one bfloat16 would give 0 or 2^-9, off by all of it

@@ -574,14 +574,16 @@ __global__ void __launch_bounds__(SF_THREADS, GREEDY ? 2 : 1) sample_full_kernel
   if (threadIdx.x == 0) { sb.best_local = 0; sb.odd_local = 0; }
   __syncthreads();
   {
-    unsigned long long best = 0;
+    uint32_t bk = 0;                                        // a thread's indices ascend: the first of equal keys stays
+    int bi = 0x7fffffff;
     bool nan = false;
     q.for_slice([&](float v, int i) {
       const float z = sf_scaled(v, p.inv_temp);
-      const unsigned long long kk = SfCluster::comp(sf_key(z), i);
-      best = kk > best ? kk : best;
-      nan |= !(z == z);
+      const uint32_t key = sf_key(z);
+      if (key > bk || bi == 0x7fffffff) { bk = key; bi = i; }
+      if (!GREEDY) nan |= !(z == z);
     });
+    unsigned long long best = bi == 0x7fffffff ? 0 : SfCluster::comp(bk, bi);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const unsigned long long t = __shfl_xor_sync(0xffffffffu, best, o);

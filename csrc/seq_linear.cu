@@ -1,6 +1,7 @@
 // Linear layers for any shape and for bfloat16 or true float32 operands: y = act(x W^T) with W [N, K] (out, in).
 //
-//  * linear_rows_kernel  (M <= 8: decode)  — weight-streaming: a CTA owns ROWS output features, its 8 warps split K, each
+//  * linear_mma_rows_kernel (bfloat16, M = 5 .. 8: decode) — weight-streaming through mma.sync: see there.
+//  * linear_rows_kernel  (M <= 8: fewer tokens, float32, pitches without 16-byte rows) — weight-streaming: a CTA owns ROWS output features, its 8 warps split K, each
 //    lane reads 16 bytes of every row per step (all loads issued before the first use) and keeps ROWS x M fp32
 //    accumulators; activations come from L1; the warps' sums meet in shared memory in a fixed order.
 //  * linear_tiled_kernel (any M)           — 64 x 64 x 16 shared-memory tiles, 4 x 4 outputs per thread, fp32 FMA.  This is
@@ -116,6 +117,110 @@ __global__ void __launch_bounds__(LR_WARPS * 32) linear_rows_kernel(const T* __r
   }
 }
 
+// bfloat16 weights of a decode step of 5 to 8 tokens, streamed once, tokens as the 8 columns of mma.sync.m16n8k16 (products exact,
+// fp32 sums).  A warp takes 16 output features and one of KS parts of K in batches of 256 k: lane (g = lane / 4, t = lane % 4) loads the
+// 16-byte chunks t, t + 4, ... of rows g and g + 8 straight into A fragments, and the same chunks of token g into B fragments (the order of
+// k inside a product is free as long as both agree: MMA v of chunk u uses words 2v, 2v + 1), so a batch is 16 weight loads in flight
+// per lane, 8 token loads (L1) and 16 MMAs.  The FMA kernel is bound by issue there: it unpacks every weight and multiplies it once per token.
+// The tensor core truncates when it adds, so a chain of sums is two MMAs long (32 k) and meets the rest in rounded fp32 additions:
+// fp32 results are 0.8 to 1.0e-7 off float64, those of the FMA kernel 0.8 to 0.9e-7, and a layer's or a model's output is not further
+// off than before.  The KS warps of a CTA meet in shared memory, neighbours first.
+// 8 tokens on one B200, FMA kernel -> this one (features x K): 32000 x 2048 83.5 -> 26.2 us, 8192 x 2048 23.8 -> 10.5, 2048 x 8192
+// 16.2 -> 10.6, 2048 x 2048 7.9 -> 4.4.  Up to 4 tokens the FMA kernel, whose loads run along a row (512 contiguous bytes against 64), is
+// as fast or faster (2 tokens: 2048 x 8192 7.9 against 10.5), and with fewer than 96 groups of 16 features too (8 tokens, 1024 x 5464:
+// 7.4 against 8.9: a warp's batches run one after the other).
+constexpr int LM_U = 8, LM_BATCH = 32 * LM_U;        // chunk groups of 32 k in flight; k of a batch
+
+__device__ __forceinline__ uint4 lm_load(const void* p) {      // touched once: no line in L1 (the tokens live there)
+  uint4 r;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  return r;
+}
+__device__ __forceinline__ void lm_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <typename OutT, int KS>
+__global__ void __launch_bounds__((KS > 4 ? KS : 4) * 32) linear_mma_rows_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
+                                                                                 const __nv_bfloat16* __restrict__ w, OutT* __restrict__ out,
+                                                                                 int ldo, int M, int N, int K, int act, float p0, float p1,
+                                                                                 LinearGroup gr) {
+  constexpr int WARPS = KS > 4 ? KS : 4, GROUPS = WARPS / KS;
+  __shared__ float red[WARPS][16][9];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int part = warp % KS, n0 = (blockIdx.x * GROUPS + warp / KS) * 16;
+  const int seg = ((K + KS - 1) / KS + 31) / 32 * 32;
+  const int k0 = part * seg, k1 = min(K, k0 + seg);
+  const long long z = blockIdx.y;
+  pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
+  pdl_launch_dependents();
+  if (gr.w_index && gr.w_index[z] < 0) return;             // a batch without a matrix (uniform for the CTA): nothing is written
+  w += (gr.w_index ? (long long)gr.w_index[z] : z) * gr.w_bs;
+  x += (z / gr.x_div) * gr.x_bs;
+  out += z * gr.o_bs;
+  float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  const __nv_bfloat16* w0 = w + (size_t)min(n0 + g, N - 1) * K;
+  const __nv_bfloat16* w1 = w + (size_t)min(n0 + g + 8, N - 1) * K;
+  const __nv_bfloat16* xr = x + (size_t)min(g, M - 1) * ldx;
+  const bool tok = g < M;
+  if (n0 < N) {
+    for (int kb = k0; kb < k1; kb += LM_BATCH) {
+      uint4 a[LM_U], b[LM_U], c[LM_U];
+#pragma unroll
+      for (int u = 0; u < LM_U; ++u) {                     // all loads of the batch before the first use
+        const int k = kb + 32 * u + 8 * t;
+        const bool on = k < k1;                            // K is a multiple of 8
+        a[u] = on ? lm_load(w0 + k) : make_uint4(0u, 0u, 0u, 0u);
+        b[u] = on ? lm_load(w1 + k) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int u = 0; u < LM_U; ++u) {
+        const int k = kb + 32 * u + 8 * t;
+        c[u] = tok && k < k1 ? *reinterpret_cast<const uint4*>(xr + k) : make_uint4(0u, 0u, 0u, 0u);
+      }
+      float d[LM_U][4] = {};
+#pragma unroll
+      for (int u = 0; u < LM_U; ++u) {
+        lm_mma(d[u], a[u].x, b[u].x, a[u].y, b[u].y, c[u].x, c[u].y);
+        lm_mma(d[u], a[u].z, b[u].z, a[u].w, b[u].w, c[u].z, c[u].w);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        sum[i] += ((d[0][i] + d[1][i]) + (d[2][i] + d[3][i])) + ((d[4][i] + d[5][i]) + (d[6][i] + d[7][i]));
+    }
+  }
+  red[warp][g][2 * t] = sum[0]; red[warp][g][2 * t + 1] = sum[1];
+  red[warp][g + 8][2 * t] = sum[2]; red[warp][g + 8][2 * t + 1] = sum[3];
+  __syncthreads();
+  for (int i = threadIdx.x; i < GROUPS * 16 * M; i += WARPS * 32) {
+    const int gi = i / (16 * M), m = i / 16 % M, r = i % 16;
+    float s[KS];
+#pragma unroll
+    for (int q = 0; q < KS; ++q) s[q] = red[gi * KS + q][r][m];
+#pragma unroll
+    for (int o = 1; o < KS; o <<= 1)
+#pragma unroll
+      for (int q = 0; q < KS; q += 2 * o) s[q] += s[q + o];          // neighbouring parts first
+    const int n = (blockIdx.x * GROUPS + gi) * 16 + r;
+    if (n < N) out[(size_t)m * ldo + n] = from_f<OutT>(apply_act(s[0], act, p0, p1));
+  }
+}
+
+template <typename OutT>
+static void lm_launch(const __nv_bfloat16* x, int ldx, const __nv_bfloat16* w, OutT* out, int ldo, int M, int N, int K, int act, float p0,
+                      float p1, cudaStream_t st, const LinearGroup& g, int nbatch) {
+  // parts of K: some 14 warps on every SM (8 KB in flight each), each part at least half a batch long
+  const long groups = (long)((N + 15) / 16) * nbatch;
+  int ks = 1;
+  while (ks < 16 && groups * ks < 148 * 14 && K >= 2 * ks * (LM_BATCH / 2)) ks *= 2;
+  const int per = (ks > 4 ? 1 : 4 / ks) * 16;
+  const dim3 grid((N + per - 1) / per, nbatch), block((ks > 4 ? ks : 4) * 32);
+#define JL_LM(KS_) case KS_: JL_LAUNCH_PDL((linear_mma_rows_kernel<OutT, KS_>), grid, block, 0, st, x, ldx, w, out, ldo, M, N, K, act, p0, p1, g); break;
+  switch (ks) { JL_LM(1) JL_LM(2) JL_LM(4) JL_LM(8) JL_LM(16) }
+#undef JL_LM
+}
+
 constexpr int LT_BM = 64, LT_BN = 64, LT_BK = 16;
 
 template <typename T, typename OutT>
@@ -185,6 +290,12 @@ static int launch_linear(const void* x, int ldx, const void* w, void* out, int l
     constexpr int VN = Vec<T>::N;
     const int vec_ok = (K % VN == 0) && (ldx % VN == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) &&
                        (g.x_bs % VN == 0) && (g.w_bs % VN == 0);
+    if constexpr (sizeof(T) == 2) {
+      if (vec_ok && M > 4 && (long)((N + 15) / 16) * nbatch >= 96) {
+        lm_launch<OutT>((const T*)x, ldx, (const T*)w, (OutT*)out, ldo, M, N, K, act, p0, p1, st, g, nbatch);
+        return cudaGetLastError() == cudaSuccess ? JL_OK : JL_ERR_CUDA;
+      }
+    }
     const dim3 blocks((N + LR_ROWS - 1) / LR_ROWS, nbatch);
 #define JL_LR(MM)                                                                                                       \
   case MM:                                                                                                              \

@@ -15,6 +15,7 @@
 
 #include "jllama_b200.h"
 #include "seq_types.cuh"
+#include "tcgen05.cuh"
 
 namespace jl {
 
@@ -36,7 +37,7 @@ struct GlaParams {
   float* state;                        // [B][H][D][Dv] fp32, read and written
   float* o;                            // [B*S][H][Dv] fp32
   // time chunks of the prompt scan (gla_stream_kernel): NC chunks of L tokens per row
-  int NC, L, mode;                     // mode 0: one chunk, state in / out; 1: local scan from zero, no read-out; 3: read-out pass
+  int NC, L;
   float* cstate;                       // [B][NC][H][D][Dv]: local end states (after mode 1), incoming states (after the combine)
   float* cdecay;                       // [B][NC][H][D]: product of the chunk's decays per key channel
   // retention (jl_retention_scan): one fixed decay per head instead of the projected one, rotary embedding of q and k at the
@@ -63,11 +64,8 @@ __device__ __forceinline__ float scan_value(const GlaParams& p, size_t m, int h,
   return p.aux ? v * p.aux[m * p.ld_aux + p.H + h] : v;
 }
 
-// q, k and alpha of channel d of head h for the token whose projection row is yr (position pos).
-template <typename T>
-__device__ __forceinline__ void scan_channel(const GlaParams& p, size_t m, int h, int d, int pos,
-                                             const float* __restrict__ zs, const T* __restrict__ a2, const T* __restrict__ a2b,
-                                             float& qv, float& kv, float& av) {
+// q and k of channel d of head h for the token whose projection row is y[m] (position pos).
+__device__ __forceinline__ void scan_qk(const GlaParams& p, size_t m, int h, int d, int pos, float& qv, float& kv) {
   const float* yr = p.y + m * p.ldy;
   const int hq = p.qk_div > 1 ? h / p.qk_div : h;
   const float* qh = yr + p.q_off + hq * p.D;
@@ -84,6 +82,14 @@ __device__ __forceinline__ void scan_channel(const GlaParams& p, size_t m, int h
     qv = qh[d] * p.q_scale;
     kv = kh[d] * p.k_scale;
   }
+}
+
+// q, k and alpha; zs: the token's low-rank decay input
+template <typename T>
+__device__ __forceinline__ void scan_channel(const GlaParams& p, size_t m, int h, int d, int pos,
+                                             const float* __restrict__ zs, const T* __restrict__ a2, const T* __restrict__ a2b,
+                                             float& qv, float& kv, float& av) {
+  scan_qk(p, m, h, d, pos, qv, kv);
   if (p.aux) { av = p.aux[m * p.ld_aux + h]; return; }
   if (p.head_decay) { av = p.head_decay[h]; return; }
   const int n = h * p.D + d;
@@ -178,175 +184,301 @@ __global__ void __launch_bounds__(GS_THREADS, 3) gla_scan_kernel(GlaParams p, co
 // Prompts: the same recurrence in two launches.  gla_prep_kernel is token-parallel: it forms alpha (low-rank product,
 // bias, log-sigmoid, exponential — fp32), scales q, and writes q | k | alpha | v of every (token, head) as one
 // contiguous fp32 record laid out exactly like the scan's shared-memory stage ([3][P][DP + 4] then the value row,
-// padded to 16 bytes).  gla_stream_kernel then only copies records with cp.async, two stages deep (the copy of the next
-// GS_TS tokens runs under the arithmetic of the current ones), and advances the state.  The fused kernel above pays two
+// padded to 16 bytes).  In gla_stream_kernel one thread copies records with bulk copies, two stages deep (the copy of the next
+// GS_TS tokens runs under the arithmetic of the current ones), and all advance the state.  The fused kernel above pays two
 // dependent DRAM round trips and the transcendental math per 8 tokens on the critical path of a sequential loop; here
 // the loop sees shared memory only.
 //
-// A thread of the streaming kernel owns a DP x C tile of the state: DP key channels of C adjacent value columns.  The
-// loop is bound by shared-memory reads of q, k and alpha (every thread needs them for its channels), so the tile is
-// wide in columns (C = 4: the reads are shared by four columns) and short in channels (DP = 8), and the P = D / DP
-// lanes of a column group add their partial read-outs with shuffles.  Key sizes above 256 take DP = 32, C = 1.
+// A thread of the streaming kernel owns a DP x C = 16 x 4 tile of the state: 16 key channels of 4 adjacent value columns, the P = D / 16
+// lanes of a column group adjacent.  What bounds the loop is the path from shared memory to registers (128 bytes a cycle and SM,
+// broadcast or not): q, k and alpha of a thread's channels are read once for its four columns, 12 reads of 16 bytes per token for 64
+// state elements (the former 32 x 1 tile: 24 reads for 32), and channels go in pairs through packed fp32 instructions
+// (fma.rn.f32x2: two rounded FMAs), three for two state elements of one token.  A group's partial read-outs meet by
+// exchanging halves: P = 4 lanes need three shuffles for four columns and end with one column each.
+// 2048 tokens, 16 heads of 64 x 128, one row on one B200, both passes: 189 us with the 32 x 1 tile, 93 us with this one.
 constexpr int GS_TS = 16;        // tokens per pipeline stage
+constexpr int GT_DP = 16, GT_C = 4, GT_PITCH = GT_DP + 4;      // 16 channels in rows of 20 floats: the lanes of a group read different banks
+constexpr int GT_MAX_D = 256;    // wider keys: the fused kernel above
 
-struct GlaTile { int DP, C, P; };
-static GlaTile gla_tile(int D) {
-  // measured (2048 tokens, D 64, Dv 128): 0.80 ms with the 32 x 1 tile, 1.22 ms with 8 x 4 (its three shuffle levels per
-  // token lengthen the dependent chain, and the loop is bound by latency, not by shared-memory bandwidth);
-  // JLLAMA_GLA_TILE=8 selects the wide tile for A/B
-  static const bool wide = [] { const char* e = getenv("JLLAMA_GLA_TILE"); return e && e[0] == '8'; }();
-  GlaTile t{32, 1, 1};
-  if (wide && D <= 256) t = GlaTile{8, 4, 1};
-  while (t.P * t.DP < D) t.P *= 2;
-  return t;
+__host__ __device__ inline int gla_lanes(int D) {
+  int P = 1;
+  while (P * GT_DP < D) P *= 2;
+  return P;
 }
-__host__ __device__ inline int gla_record_floats(int P, int DP, int Dv) { return 3 * P * (DP + 4) + ((Dv + 3) & ~3); }
+// threads of a CTA: whole warps that cover the value columns, at most 128
+inline int gla_threads(int P, int Dv) {
+  const int t = ((Dv + GT_C - 1) / GT_C * P + 31) / 32 * 32;
+  return t < GS_THREADS ? t : GS_THREADS;
+}
+__host__ __device__ inline int gla_record_floats(int P, int Dv) { return 3 * P * GT_PITCH + ((Dv + 3) & ~3); }
+
+// A thread forms one slot of the records (a channel of a head, or a value column) for GP_TOK tokens: the channel's row of A2 is read once
+// for all of them.  (One CTA per token, its threads walking all channels, read A2 once per token: 60 us for 2048 tokens of 16 x 64 channels
+// against 42 us.)
+constexpr int GP_TOK = 8, GP_THREADS = 256;
 
 template <typename T>
-__global__ void __launch_bounds__(128) gla_prep_kernel(GlaParams p, const T* __restrict__ a2, const T* __restrict__ a2b,
-                                                       float* __restrict__ rec, int DP) {
+__global__ void __launch_bounds__(GP_THREADS) gla_prep_kernel(GlaParams p, const T* __restrict__ a2, const T* __restrict__ a2b,
+                                                              float* __restrict__ rec) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
   pdl_launch_dependents();
-  extern __shared__ float zs[];                                 // [R]
-  const int m = blockIdx.x;
-  const float* yr = p.y + (size_t)m * p.ldy;
-  const int pos = scan_position(p, m / p.S, m % p.S);
-  for (int r = threadIdx.x; r < p.R; r += blockDim.x) zs[r] = yr[p.a_off + r];
+  extern __shared__ float zs[];                                 // [GP_TOK][R]
+  const int M = p.B * p.S, m0 = blockIdx.x * GP_TOK, nt = min(GP_TOK, M - m0);
+  for (int i = threadIdx.x; i < nt * p.R; i += GP_THREADS) zs[i] = p.y[(size_t)(m0 + i / p.R) * p.ldy + p.a_off + i % p.R];
   __syncthreads();
-  const int P = p.P, pitch = DP + 4, RF = gla_record_floats(P, DP, p.Dv);
-  float* out = rec + (size_t)m * p.H * RF;
-  const int per_head = P * DP;
-  for (int i = threadIdx.x; i < p.H * per_head; i += blockDim.x) {
-    const int h = i / per_head, d = i % per_head;
-    float qv = 0.0f, kv = 0.0f, av = 1.0f;
-    if (d < p.D) scan_channel<T>(p, (size_t)m, h, d, pos, zs, a2, a2b, qv, kv, av);
-    float* o = out + (size_t)h * RF + (d / DP) * pitch + d % DP;
-    o[0] = qv; o[P * pitch] = kv; o[2 * P * pitch] = av;
+  const int P = p.P, RF = gla_record_floats(P, p.Dv), per_head = P * GT_DP, dvp = (p.Dv + 3) & ~3;
+  const int i = blockIdx.y * GP_THREADS + threadIdx.x;
+  if (i >= p.H * per_head) {                                    // a value column
+    const int j = i - p.H * per_head;
+    if (j >= p.H * dvp) return;
+    const int h = j / dvp, c = j % dvp;
+    float* out = rec + ((size_t)m0 * p.H + h) * RF + 3 * P * GT_PITCH + c;
+    float v[GP_TOK];
+#pragma unroll
+    for (int t = 0; t < GP_TOK; ++t) v[t] = t < nt ? scan_value(p, (size_t)(m0 + t), h, c) : 0.0f;
+#pragma unroll
+    for (int t = 0; t < GP_TOK; ++t) if (t < nt) out[(size_t)t * p.H * RF] = v[t];
+    return;
   }
-  const int dvp = (p.Dv + 3) & ~3;
-  for (int i = threadIdx.x; i < p.H * dvp; i += blockDim.x) {
-    const int h = i / dvp, c = i % dvp;
-    out[(size_t)h * RF + 3 * P * pitch + c] = scan_value(p, (size_t)m, h, c);
+  const int h = i / per_head, d = i % per_head;
+  float* out = rec + ((size_t)m0 * p.H + h) * RF + (d / GT_DP) * GT_PITCH + d % GT_DP;
+  float qv[GP_TOK], kv[GP_TOK], av[GP_TOK];
+#pragma unroll
+  for (int t = 0; t < GP_TOK; ++t) { qv[t] = kv[t] = 0.0f; av[t] = 1.0f; }
+  if (d < p.D) {
+#pragma unroll
+    for (int t = 0; t < GP_TOK; ++t)
+      if (t < nt) scan_qk(p, (size_t)(m0 + t), h, d, scan_position(p, (m0 + t) / p.S, (m0 + t) % p.S), qv[t], kv[t]);
+    if (p.aux || p.head_decay) {
+#pragma unroll
+      for (int t = 0; t < GP_TOK; ++t) if (t < nt) av[t] = p.aux ? p.aux[(size_t)(m0 + t) * p.ld_aux + h] : p.head_decay[h];
+    } else {
+      const int n = h * p.D + d;
+      const float bias = to_f(a2b[n]);
+#pragma unroll
+      for (int t = 0; t < GP_TOK; ++t) av[t] = bias;
+      for (int r = 0; r < p.R; ++r) {
+        const float a = to_f(a2[(size_t)n * p.R + r]);
+#pragma unroll
+        for (int t = 0; t < GP_TOK; ++t) av[t] = fmaf(a, t < nt ? zs[t * p.R + r] : 0.0f, av[t]);
+      }
+#pragma unroll
+      for (int t = 0; t < GP_TOK; ++t) av[t] = expf(log_sigmoid(av[t]) * p.inv_tau);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < GP_TOK; ++t) {
+    if (t >= nt) break;
+    float* o = out + (size_t)t * p.H * RF;
+    o[0] = qv[t]; o[P * GT_PITCH] = kv[t]; o[2 * P * GT_PITCH] = av[t];
   }
 }
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gsrc) : "memory");
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, int bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void fence_generic_to_bulk() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-template <int DP, int C>
-__global__ void __launch_bounds__(GS_THREADS, 2) gla_stream_kernel(GlaParams p, const float* __restrict__ rec) {
+__device__ __forceinline__ unsigned long long f2_dup(float v) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float2 f2_split(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_join(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+// P lanes of a column group; MODE 0: one chunk, state in / out; 1: local scan of a chunk from zero, no read-out; 3: read-out pass
+template <int P, int MODE>
+__global__ void __launch_bounds__(GS_THREADS, 3) gla_stream_kernel(GlaParams p, const float* __restrict__ rec) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
   pdl_launch_dependents();
   extern __shared__ float4 smem4[];
+  __shared__ __align__(8) unsigned long long bars[2];
   float* smem = reinterpret_cast<float*>(smem4);
-  constexpr int PITCH = DP + 4;
-  const int P = p.P, groups = GS_THREADS / P, cols = groups * C;        // value columns per CTA
+  const int nthreads = blockDim.x, cols = nthreads / P * GT_C;          // value columns per CTA
   const int tid = threadIdx.x, part = tid % P, grp = tid / P;
-  const int col0 = blockIdx.x * cols + grp * C;                         // first of this thread's C columns
+  const int col0 = blockIdx.x * cols + grp * GT_C;                      // first of this thread's columns
   const int h = blockIdx.y, b = blockIdx.z / p.NC, chunk = blockIdx.z % p.NC;
-  const bool idle = (int)blockIdx.x * cols + (tid & ~31) / P * C >= p.Dv;  // warp-uniform: no column of this warp exists
-  const int QKA = 3 * P * PITCH;                                        // floats of q | k | alpha per token
+  const bool idle = (int)blockIdx.x * cols + (tid & ~31) / P * GT_C >= p.Dv;      // warp-uniform: no column of this warp exists
+  constexpr int QKA = 3 * P * GT_PITCH;                                 // floats of q | k | alpha per token
   const int SF = QKA + cols;                                            // floats per token in a stage
-  const int RF = gla_record_floats(P, DP, p.Dv);
-  float st[DP][C];
-  const int d0 = part * DP;
-  float* sbase = p.mode == 0 ? p.state + (((size_t)b * p.H + h) * p.D) * p.Dv
-                             : p.cstate + ((((size_t)b * p.NC + chunk) * p.H + h) * p.D) * p.Dv;
-  float ap[DP];                                                         // mode 1: product of this chunk's decays
+  const int RF = gla_record_floats(P, p.Dv);
+  const bool vec = p.Dv % 4 == 0;
+  unsigned long long st[GT_DP / 2][GT_C];                               // pairs of channels
+  const int d0 = part * GT_DP;
+  float* sbase = MODE == 0 ? p.state + (((size_t)b * p.H + h) * p.D) * p.Dv
+                           : p.cstate + ((((size_t)b * p.NC + chunk) * p.H + h) * p.D) * p.Dv;
+  auto load_row = [&](int r, float (&v)[GT_C]) {
+    const float* src = sbase + (size_t)(d0 + r) * p.Dv + col0;
+    if (MODE == 1 || d0 + r >= p.D || col0 >= p.Dv) {
 #pragma unroll
-  for (int r = 0; r < DP; ++r) {
-    ap[r] = 1.0f;
+      for (int c = 0; c < GT_C; ++c) v[c] = 0.0f;
+    } else if (vec) {
+      load4(src, v);
+    } else {
 #pragma unroll
-    for (int c = 0; c < C; ++c)
-      st[r][c] = (p.mode != 1 && col0 + c < p.Dv && d0 + r < p.D) ? sbase[(size_t)(d0 + r) * p.Dv + col0 + c] : 0.0f;
+      for (int c = 0; c < GT_C; ++c) v[c] = col0 + c < p.Dv ? src[c] : 0.0f;
+    }
+  };
+#pragma unroll
+  for (int r = 0; r < GT_DP; r += 2) {
+    float v0[GT_C], v1[GT_C];
+    load_row(r, v0);
+    load_row(r + 1, v1);
+#pragma unroll
+    for (int c = 0; c < GT_C; ++c) st[r / 2][c] = f2_join(v0[c], v1[c]);
   }
+  const bool decays = MODE == 1 && blockIdx.x == 0 && (tid & ~31) == 0;  // warp-uniform: this warp multiplies up the chunk's decays
+  unsigned long long ap[GT_DP / 2];
+#pragma unroll
+  for (int r = 0; r < GT_DP / 2; ++r) ap[r] = f2_dup(1.0f);
+  // columns of a finished read-out that this lane holds after the exchange, and whether it writes them
+  constexpr int NOUT = P == 1 ? 4 : (P == 2 ? 2 : 1), REST = P >= 4 ? P / 4 - 1 : 0;
+  const int ocol = col0 + (P >= 2 && (part & (P / 2)) ? 2 : 0) + (P >= 4 && (part & (P / 4)) ? 1 : 0);
+  const bool writes = (part & REST) == 0;
   const int t_begin = chunk * p.L, t_end = min(p.S, t_begin + p.L);     // this CTA's tokens of row b
   const int first = max(t_begin, (p.pad_left ? p.pad_left[b] : 0) - (p.cache_len ? *p.cache_len : 0));
-  if (part == 0 && p.mode != 1)
+  if (part == 0 && MODE != 1)
     for (int s = t_begin; s < min(first, t_end); ++s)
-      for (int c = 0; c < C; ++c)
+      for (int c = 0; c < GT_C; ++c)
         if (col0 + c < p.Dv) p.o[((size_t)(b * p.S + s) * p.H + h) * p.Dv + col0 + c] = 0.0f;
-  const int vcols4 = cols / 4, q4 = QKA / 4, dvp = (p.Dv + 3) & ~3;
+  // one thread copies: the records of a stage's tokens as they lie (a local scan leaves the queries out), two stages ahead of their use
+  const int dvp = (p.Dv + 3) & ~3, vcol0 = blockIdx.x * cols;
+  constexpr int Q0 = MODE == 1 ? P * GT_PITCH : 0;
+  const uint32_t full = tc::smem_u32(bars);
+  const float* row0 = rec + ((size_t)b * p.S * p.H + h) * RF;
   auto issue = [&](int s0, int stage) {
-    const int nt = min(GS_TS, t_end - s0);
-    float* dst = smem + (size_t)stage * GS_TS * SF;
-    for (int i = tid; i < nt * (q4 + vcols4); i += GS_THREADS) {
-      const int t = i / (q4 + vcols4), c = i % (q4 + vcols4);
-      const float* src = rec + ((size_t)(b * p.S + s0 + t) * p.H + h) * RF;
-      if (c < q4) cp_async16(dst + t * SF + 4 * c, src + 4 * c);
-      else if ((int)(blockIdx.x * cols) + 4 * (c - q4) < dvp)
-        cp_async16(dst + t * SF + QKA + 4 * (c - q4), src + QKA + blockIdx.x * cols + 4 * (c - q4));
+    const int nt = min(GS_TS, t_end - s0), nv = min(cols, dvp - vcol0);
+    const uint32_t bar = full + 8u * stage;
+    const float* src = row0 + (size_t)s0 * p.H * RF;
+    uint32_t dst = tc::smem_u32(smem + (size_t)stage * GS_TS * SF);
+    tc::mbar_expect_tx(bar, (uint32_t)(nt * (QKA - Q0 + nv) * 4));
+    for (int t = 0; t < nt; ++t, src += (size_t)p.H * RF, dst += 4 * SF) {
+      if (vcol0 == 0) {
+        bulk_copy(dst + 4 * Q0, src + Q0, (QKA - Q0 + nv) * 4, bar);
+      } else {
+        bulk_copy(dst + 4 * Q0, src + Q0, (QKA - Q0) * 4, bar);
+        bulk_copy(dst + 4 * QKA, src + QKA + vcol0, nv * 4, bar);
+      }
     }
-    cp_async_commit();
   };
-  int stage = 0;
-  if (first < t_end) issue(first, 0);
-  for (int s0 = first; s0 < t_end; s0 += GS_TS, stage ^= 1) {
-    if (s0 + GS_TS < t_end) { issue(s0 + GS_TS, stage ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
-    __syncthreads();
+  if (tid == 0) {
+    tc::mbar_init(full, 1); tc::mbar_init(full + 8, 1);
+    tc::fence_barrier_init();
+    if (first < t_end) issue(first, 0);
+    if (first + GS_TS < t_end) issue(first + GS_TS, 1);
+  }
+  __syncthreads();
+  int stage = 0, phase = 0;
+  for (int s0 = first; s0 < t_end; s0 += GS_TS) {
+    tc::mbar_wait(full + 8u * stage, phase);
     const int nt = idle ? 0 : min(GS_TS, t_end - s0);
     const float* base = smem + (size_t)stage * GS_TS * SF;
     for (int t = 0; t < nt; ++t) {
       const float* tk = base + t * SF;
-      float v[C];
-      if constexpr (C == 4) {
-        const float4 vv = *reinterpret_cast<const float4*>(tk + QKA + grp * C);
-        v[0] = vv.x; v[1] = vv.y; v[2] = vv.z; v[3] = vv.w;
-      } else {
-#pragma unroll
-        for (int c = 0; c < C; ++c) v[c] = tk[QKA + grp * C + c];
+      unsigned long long v[GT_C];
+      {
+        const float4 vv = *reinterpret_cast<const float4*>(tk + QKA + grp * GT_C);
+        v[0] = f2_dup(vv.x); v[1] = f2_dup(vv.y); v[2] = f2_dup(vv.z); v[3] = f2_dup(vv.w);
       }
-      const float4* qt = reinterpret_cast<const float4*>(tk + part * PITCH);
-      const float4* kt = reinterpret_cast<const float4*>(tk + (P + part) * PITCH);
-      const float4* at = reinterpret_cast<const float4*>(tk + (2 * P + part) * PITCH);
-      float acc[C][2];
+      const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(tk + part * GT_PITCH);
+      const ulonglong2* kt = reinterpret_cast<const ulonglong2*>(tk + (P + part) * GT_PITCH);
+      const ulonglong2* at = reinterpret_cast<const ulonglong2*>(tk + (2 * P + part) * GT_PITCH);
+      unsigned long long acc[GT_C][2];
 #pragma unroll
-      for (int c = 0; c < C; ++c) acc[c][0] = acc[c][1] = 0.0f;
+      for (int c = 0; c < GT_C; ++c) acc[c][0] = acc[c][1] = 0ull;       // (two zeros)
 #pragma unroll
-      for (int r = 0; r < DP / 4; ++r) {
-        const float4 al = at[r], kk = kt[r], qq = qt[r];
-        const float a4[4] = {al.x, al.y, al.z, al.w}, k4[4] = {kk.x, kk.y, kk.z, kk.w}, q4v[4] = {qq.x, qq.y, qq.z, qq.w};
+      for (int r = 0; r < GT_DP / 4; ++r) {
+        const ulonglong2 al = at[r], kk = kt[r];
+        ulonglong2 qq = make_ulonglong2(0ull, 0ull);
+        if (MODE != 1) qq = qt[r];
+        if (MODE == 1 && decays) { ap[2 * r] = f2_mul(ap[2 * r], al.x); ap[2 * r + 1] = f2_mul(ap[2 * r + 1], al.y); }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          ap[4 * r + j] *= a4[j];
-#pragma unroll
-          for (int c = 0; c < C; ++c) {
-            st[4 * r + j][c] = fmaf(a4[j], st[4 * r + j][c], k4[j] * v[c]);
-            acc[c][j & 1] = fmaf(q4v[j], st[4 * r + j][c], acc[c][j & 1]);
+        for (int c = 0; c < GT_C; ++c) {
+          st[2 * r][c] = f2_fma(al.x, st[2 * r][c], f2_mul(kk.x, v[c]));
+          st[2 * r + 1][c] = f2_fma(al.y, st[2 * r + 1][c], f2_mul(kk.y, v[c]));
+          if (MODE != 1) {
+            acc[c][0] = f2_fma(qq.x, st[2 * r][c], acc[c][0]);
+            acc[c][1] = f2_fma(qq.y, st[2 * r + 1][c], acc[c][1]);
           }
         }
       }
-      if (p.mode == 1) continue;                              // local scan: the read-outs come in the second pass
-      float o[C];
+      if constexpr (MODE != 1) {                              // (a local scan leaves the read-outs to the second pass)
+      float o[GT_C];
 #pragma unroll
-      for (int c = 0; c < C; ++c) {
-        o[c] = acc[c][0] + acc[c][1];
-        for (int off = P >> 1; off > 0; off >>= 1) o[c] += __shfl_xor_sync(0xffffffffu, o[c], off);
+      for (int c = 0; c < GT_C; ++c) {
+        const float2 x = f2_split(acc[c][0]), y = f2_split(acc[c][1]);
+        o[c] = (x.x + x.y) + (y.x + y.y);
       }
-      if (part == 0) {
-        float* dst = p.o + ((size_t)(b * p.S + s0 + t) * p.H + h) * p.Dv + col0;
-        if (C == 4 && col0 + 3 < p.Dv && (p.Dv & 3) == 0) {
-          *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
-        } else {
+      if constexpr (P >= 2) {                                 // keep two columns, give two
+        const bool up = (part & (P / 2)) != 0;
+        const float g0 = __shfl_xor_sync(0xffffffffu, up ? o[0] : o[2], P / 2), g1 = __shfl_xor_sync(0xffffffffu, up ? o[1] : o[3], P / 2);
+        o[0] = (up ? o[2] : o[0]) + g0;
+        o[1] = (up ? o[3] : o[1]) + g1;
+      }
+      if constexpr (P >= 4) {                                 // keep one, give one
+        const bool up = (part & (P / 4)) != 0;
+        const float g0 = __shfl_xor_sync(0xffffffffu, up ? o[0] : o[1], P / 4);
+        o[0] = (up ? o[1] : o[0]) + g0;
 #pragma unroll
-          for (int c = 0; c < C; ++c) if (col0 + c < p.Dv) dst[c] = o[c];
-        }
+        for (int off = P / 8; off > 0; off >>= 1) o[0] += __shfl_xor_sync(0xffffffffu, o[0], off);
+      }
+      if (writes) {
+        float* dst = p.o + ((size_t)(b * p.S + s0 + t) * p.H + h) * p.Dv + ocol;
+#pragma unroll
+        for (int c = 0; c < NOUT; ++c) if (ocol + c < p.Dv) dst[c] = o[c];
+      }
       }
     }
-    __syncthreads();                                          // the stage is free for the copy after next
+    __syncthreads();                                          // the stage is free
+    if (tid == 0 && s0 + 2 * GS_TS < t_end) {
+      fence_generic_to_bulk();                                // (its reads come before the copy that overwrites it)
+      issue(s0 + 2 * GS_TS, stage);
+    }
+    stage ^= 1;
+    phase ^= stage == 0;
   }
-  if (p.mode == 3) return;
+  if (MODE == 3) return;
 #pragma unroll
-  for (int r = 0; r < DP; ++r) {
+  for (int r = 0; r < GT_DP / 2; ++r) {
+    float2 x[GT_C];
 #pragma unroll
-    for (int c = 0; c < C; ++c)
-      if (col0 + c < p.Dv && d0 + r < p.D) sbase[(size_t)(d0 + r) * p.Dv + col0 + c] = st[r][c];
-    if (p.mode == 1 && blockIdx.x == 0 && grp == 0 && d0 + r < p.D)
-      p.cdecay[(((size_t)b * p.NC + chunk) * p.H + h) * p.D + d0 + r] = ap[r];
+    for (int c = 0; c < GT_C; ++c) x[c] = f2_split(st[r][c]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int d = d0 + 2 * r + e;
+      if (d >= p.D || col0 >= p.Dv) continue;
+      float* dst = sbase + (size_t)d * p.Dv + col0;
+      const float v[GT_C] = {e ? x[0].y : x[0].x, e ? x[1].y : x[1].x, e ? x[2].y : x[2].x, e ? x[3].y : x[3].x};
+      if (vec) store4(dst, v);
+      else
+        for (int c = 0; c < GT_C; ++c) if (col0 + c < p.Dv) dst[c] = v[c];
+    }
+    if (decays && grp == 0) {
+      const float2 a = f2_split(ap[r]);
+      float* dst = p.cdecay + (((size_t)b * p.NC + chunk) * p.H + h) * p.D + d0 + 2 * r;
+      if (d0 + 2 * r < p.D) dst[0] = a.x;
+      if (d0 + 2 * r + 1 < p.D) dst[1] = a.y;
+    }
   }
 }
 
@@ -359,11 +491,22 @@ __global__ void gla_combine_kernel(GlaParams p) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t b = i / per_row, e = i % per_row, hd = e / p.Dv;           // hd = h * D + d
     float s = p.state[i];
-    for (int c = 0; c < p.NC; ++c) {
-      float* slot = p.cstate + ((size_t)b * p.NC + c) * per_row + e;
-      const float local = *slot;
-      *slot = s;
-      s = fmaf(p.cdecay[((size_t)b * p.NC + c) * p.H * p.D + hd], s, local);
+    for (int c0 = 0; c0 < p.NC; c0 += 8) {                    // eight chunks' loads in flight
+      float local[8], dec[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int c = c0 + u;
+        if (c >= p.NC) break;
+        local[u] = p.cstate[((size_t)b * p.NC + c) * per_row + e];
+        dec[u] = p.cdecay[((size_t)b * p.NC + c) * p.H * p.D + hd];
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int c = c0 + u;
+        if (c >= p.NC) break;
+        p.cstate[((size_t)b * p.NC + c) * per_row + e] = s;
+        s = fmaf(dec[u], s, local[u]);
+      }
     }
     p.state[i] = s;
   }
@@ -373,16 +516,15 @@ __global__ void gla_combine_kernel(GlaParams p) {
 
 using namespace jl;
 
-// Time chunks of a prompt scan.  One token costs a few hundred nanoseconds of dependent latency however many heads and
-// rows run beside it (measured: 2048 tokens take 0.76 ms for 1 head and 0.94 ms for 64), so while the grid is short
-// of one resident wave (two CTAs per SM) the prompt is cut into chunks that run side by side, in two passes.  Beyond
-// a wave the second pass is pure cost (8 rows x 16 heads: 1.21 ms unchunked, 1.84 ms in 4 chunks).
+// Time chunks of a prompt scan.  A token costs some 250 cycles of dependent latency however few warps run, so while the grid is short
+// of three CTAs per SM the prompt is cut into chunks that run side by side, in two passes (a local scan without read-outs, two thirds
+// of the work, then the read-out pass) with a small kernel between them.  16 heads of 64 x 128, 2048 tokens of one row, both passes: 170 us in 10
+// chunks, 143 in 20, 105 in 27 (one wave), 115 in 32.
 static int gla_chunks(int B, int S, int H, int D, int Dv) {
   static const int forced = [] { const char* e = getenv("JLLAMA_GLA_CHUNKS"); return e ? atoi(e) : 0; }();
-  const GlaTile t = gla_tile(D);
-  const int tcols = GS_THREADS / t.P * t.C;
-  const long ctas = (long)B * H * ((Dv + tcols - 1) / tcols);
-  int nc = (int)(296 / (ctas > 0 ? ctas : 1));
+  const int P = gla_lanes(D), threads = gla_threads(P, Dv), cols = threads / P * GT_C;
+  const long warps = (long)B * H * ((Dv + cols - 1) / cols) * (threads / 32);
+  int nc = (int)(148L * 12 / (warps > 0 ? warps : 1));
   if (forced > 0) nc = forced;
   if (nc > S / 64) nc = S / 64;
   if (nc > 64) nc = 64;
@@ -390,11 +532,41 @@ static int gla_chunks(int B, int S, int H, int D, int Dv) {
 }
 
 extern "C" JL_API size_t jl_gla_scan_ws_floats(int B, int S, int H, int D, int Dv) {
-  const GlaTile t = gla_tile(D);
   const int nc = gla_chunks(B, S, H, D, Dv);
-  size_t n = (size_t)B * S * H * gla_record_floats(t.P, t.DP, Dv);
+  size_t n = (size_t)B * S * H * gla_record_floats(gla_lanes(D), Dv);
   if (nc > 1) n += (size_t)B * nc * H * D * Dv + (size_t)B * nc * H * D;
   return n;
+}
+
+template <int P>
+static int launch_stream(GlaParams p, float* ws, cudaStream_t st) {
+  const int B = p.B, S = p.S, H = p.H, D = p.D, Dv = p.Dv;
+  const int threads = gla_threads(P, Dv), cols = threads / P * GT_C;
+  const size_t smem = (size_t)2 * GS_TS * (3 * P * GT_PITCH + cols) * sizeof(float);
+  const int nc = gla_chunks(B, S, H, D, Dv);
+  p.NC = nc;
+  p.L = nc > 1 ? ((S + nc - 1) / nc + GS_TS - 1) / GS_TS * GS_TS : S;
+  p.cstate = ws + (size_t)B * S * H * gla_record_floats(P, Dv);
+  p.cdecay = p.cstate + (size_t)B * nc * H * D * Dv;
+  const dim3 grid((Dv + cols - 1) / cols, H, B * nc), block(threads);
+  if (smem > 48 * 1024) {
+    JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  }
+  if (nc == 1) {
+    JL_LAUNCH_PDL((gla_stream_kernel<P, 0>), grid, block, smem, st, p, ws);
+    JL_CUDA(cudaGetLastError());
+    return JL_OK;
+  }
+  const size_t total = (size_t)B * H * D * Dv;
+  JL_LAUNCH_PDL((gla_stream_kernel<P, 1>), grid, block, smem, st, p, ws);
+  JL_CUDA(cudaGetLastError());
+  JL_LAUNCH_PDL(gla_combine_kernel, dim3((unsigned)((total + 255) / 256 < 1184 ? (total + 255) / 256 : 1184)), dim3(256), 0, st, p);
+  JL_CUDA(cudaGetLastError());
+  JL_LAUNCH_PDL((gla_stream_kernel<P, 3>), grid, block, smem, st, p, ws);
+  JL_CUDA(cudaGetLastError());
+  return JL_OK;
 }
 
 // Both scans (projected decays; fixed decays with rotary q / k) share the kernels: what differs is in p.
@@ -408,38 +580,21 @@ static int launch_scan(GlaParams p, const void* a2, const void* a2_bias, float* 
   const size_t smem = (size_t)(3 * GS_TC * P * GS_PITCH + GS_TC * cols + GS_TC * R) * sizeof(float);
   JL_CHECK_ARG(smem <= 200 * 1024, "jl_gla_scan: key size %d with rank %d does not fit the staging buffer", D, R);
   dim3 grid((Dv + cols - 1) / cols, H, B), block(GS_THREADS);
-  if (ws != nullptr && D <= 256) {                           // (wider keys: the fused kernel below)                           // prompts: token-parallel preparation, then the pipelined scan
+  if (ws != nullptr && D <= GT_MAX_D) {                      // prompts: token-parallel preparation, then the pipe
     cudaStream_t st = (cudaStream_t)stream;
-    const GlaTile t = gla_tile(D);
-    JL_CHECK_ARG(t.P <= 32, "jl_gla_scan: key size %d above %d", D, 32 * t.DP);
-    p.P = t.P;
-    const int tcols = GS_THREADS / t.P * t.C;
-      JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(gla_prep_kernel<T>, dim3(B * S), dim3(128), R * sizeof(float), st, p, (const T*)a2, (const T*)a2_bias, ws, t.DP));
+    p.P = gla_lanes(D);
+    const int slots = H * (p.P * GT_DP + ((Dv + 3) & ~3));
+    const dim3 pgrid((B * S + GP_TOK - 1) / GP_TOK, (slots + GP_THREADS - 1) / GP_THREADS);
+    JL_CHECK_ARG(GP_TOK * R * sizeof(float) <= 48 * 1024, "jl_gla_scan: rank %d does not fit the staging buffer", R);
+    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(gla_prep_kernel<T>, pgrid, dim3(GP_THREADS), GP_TOK * R * sizeof(float), st, p, (const T*)a2, (const T*)a2_bias, ws));
     JL_CUDA(cudaGetLastError());
-    const size_t smem2 = (size_t)2 * GS_TS * (3 * t.P * (t.DP + 4) + tcols) * sizeof(float);
-    JL_CHECK_ARG(smem2 <= 200 * 1024, "jl_gla_scan: key size %d does not fit the pipeline stages", D);
-    const int nc = gla_chunks(B, S, H, D, Dv);
-    p.NC = nc;
-    p.L = nc > 1 ? ((S + nc - 1) / nc + GS_TS - 1) / GS_TS * GS_TS : S;
-    p.cstate = ws + (size_t)B * S * H * gla_record_floats(t.P, t.DP, Dv);
-    p.cdecay = p.cstate + (size_t)B * nc * H * D * Dv;
-    dim3 grid2((Dv + tcols - 1) / tcols, H, B * nc);
-    if (t.DP == 8 && smem2 > 48 * 1024)
-      JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
-    if (t.DP == 32 && smem2 > 48 * 1024)
-      JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<32, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
-    for (int pass = 0; pass < (nc > 1 ? 2 : 1); ++pass) {
-      p.mode = nc > 1 ? (pass == 0 ? 1 : 3) : 0;
-          if (t.DP == 8) JL_LAUNCH_PDL((gla_stream_kernel<8, 4>), dim3(grid2), dim3(block), smem2, st, p, ws);
-      else JL_LAUNCH_PDL((gla_stream_kernel<32, 1>), dim3(grid2), dim3(block), smem2, st, p, ws);
-      JL_CUDA(cudaGetLastError());
-      if (pass == 0 && nc > 1) {
-        const size_t total = (size_t)B * H * D * Dv;
-              JL_LAUNCH_PDL(gla_combine_kernel, dim3((unsigned)((total + 255) / 256 < 1184 ? (total + 255) / 256 : 1184)), dim3(256), 0, st, p);
-        JL_CUDA(cudaGetLastError());
-      }
+    switch (p.P) {
+      case 1: return launch_stream<1>(p, ws, st);
+      case 2: return launch_stream<2>(p, ws, st);
+      case 4: return launch_stream<4>(p, ws, st);
+      case 8: return launch_stream<8>(p, ws, st);
+      default: return launch_stream<16>(p, ws, st);
     }
-    return JL_OK;
   }
   if (smem > 48 * 1024) {
     if (dtype == DT_BF16) JL_CUDA(cudaFuncSetAttribute(gla_scan_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

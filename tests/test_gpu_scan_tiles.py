@@ -1,0 +1,41 @@
+"""The prompt scans of the linear recurrences (csrc/gla_scan.cu) at the edges of their tiles, stages and time chunks, against float64.
+
+S tokens of fp32 sums and products: every read-out is a sum over at most S tokens and D channels of products of decays, keys, values and
+queries, each rounded a bounded number of times per token it passes; 2^-23 · (S + D) of the largest read-out bounds that by a wide margin, and
+what a wrong tile, lane or chunk would leave is of the order of the read-out itself."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from jax_llama_b200.ops import seq_kernels as SK  # noqa: E402
+
+
+@pytest.mark.parametrize("B,S,H,D,Dv", [(1, 9, 1, 10, 7), (2, 16, 3, 16, 64), (1, 17, 2, 33, 129), (3, 130, 1, 64, 128), (1, 700, 2, 64, 128),
+                                        (2, 257, 2, 100, 36), (1, 200, 1, 128, 640), (1, 1000, 1, 256, 65), (2, 64, 40, 32, 64), (1, 333, 3, 17, 260)])
+def test_projected_decays_over_a_prompt(B, S, H, D, Dv):
+    g = torch.Generator().manual_seed(S * D + Dv)
+    R = 5
+    cols = 2 * H * D + H * Dv + R
+    y = torch.randn(B * S, cols, generator=g)
+    a2, bias = torch.randn(H * D, R, generator=g) * 0.5, 2.0 + torch.randn(H * D, generator=g)
+    state = torch.randn(B, H, D, Dv, generator=g)
+    pads = [0] + [min(S - 1, 5 + 21 * b) for b in range(1, B)]
+    tau = 4.0
+    want = torch.zeros(B, S, H, Dv, dtype=torch.float64)
+    end = state.double().clone()
+    yd = y.double().view(B, S, cols)
+    q, k = yd[..., :H * D].reshape(B, S, H, D) * 0.25, yd[..., H * D:2 * H * D].reshape(B, S, H, D)
+    v = yd[..., 2 * H * D:2 * H * D + H * Dv].reshape(B, S, H, Dv)
+    alpha = torch.sigmoid(yd[..., -R:] @ a2.double().T + bias.double()).pow(1.0 / tau).view(B, S, H, D)
+    for b in range(B):
+        for t in range(pads[b], S):
+            end[b] = alpha[b, t, :, :, None] * end[b] + k[b, t, :, :, None] * v[b, t, :, None]
+            want[b, t] = torch.einsum("hdv,hd->hv", end[b], q[b, t])
+    got_state = state.clone().cuda()
+    got = SK.gla_scan(y.cuda(), 0, H * D, 2 * H * D, 2 * H * D + H * Dv, a2.cuda(), bias.cuda(), got_state,
+                      torch.zeros(1, dtype=torch.int32, device="cuda"), torch.tensor(pads, dtype=torch.int32, device="cuda"), B, S, H, D, Dv, 0.25,
+                      tau).double().cpu().view(B, S, H, Dv)
+    tol = 2.0 ** -23 * (S + D)
+    assert float((got - want).abs().max()) <= tol * float(want.abs().max())
+    assert float((got_state.double().cpu() - end).abs().max()) <= tol * float(end.abs().max())

@@ -1,0 +1,28 @@
+// Host interface of the float32 linears on tensor cores (linear_f32.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+namespace jl {
+
+// Many small products in one launch.  Plain batches: batch z reads x + (z / x_div) * x_bs, weights
+// w + (w_index ? w_index[z] : z) * w_bs (w_index[z] < 0: the batch is skipped) and writes out + z * o_bs (per-head matrices; one expert per (token, choice) pair when
+// decoding a mixture of experts: x_div = choices per token, so that the pairs of a token read the same input row).
+// Sorted rows (tiled kernels only): the rows come in tiles of LT_BM that each belong to one weight matrix, tile_group[tile]
+// (< 0: empty tile); row position p reads input row row_src[p] (< 0: padding, read as zero; nullptr: p itself) and writes
+// output row p — the prompt path of a mixture of experts after its tokens were sorted by expert.
+struct LinearGroup {
+  long long x_bs, w_bs, o_bs;
+  int x_div;
+  const int* w_index;
+  const int* tile_group;
+  const int* row_src;
+};
+
+constexpr int LT_BM = 64;           // rows of a sorted tile
+
+// whether the tensor-core kernel takes these sizes, pitches and addresses
+bool linear_f32_takes(int M, int K, int ldx, const LinearGroup& g, const void* x, const void* w);
+cudaError_t linear_f32_launch(const float* x, int ldx, const float* w, float* out, int ldo, int M, int N, int K, int act, float p0, float p1,
+                              cudaStream_t st, const LinearGroup& g, int nbatch);
+
+}  // namespace jl

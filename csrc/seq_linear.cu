@@ -4,29 +4,17 @@
 //  * linear_rows_kernel  (M <= 8: fewer tokens, float32, pitches without 16-byte rows) — weight-streaming: a CTA owns ROWS output features, its 8 warps split K, each
 //    lane reads 16 bytes of every row per step (all loads issued before the first use) and keeps ROWS x M fp32
 //    accumulators; activations come from L1; the warps' sums meet in shared memory in a fixed order.
-//  * linear_tiled_kernel (any M)           — 64 x 64 x 16 shared-memory tiles, 4 x 4 outputs per thread, fp32 FMA.  This is
-//    the exact float32 path and the fall-back for pitches the tensor-core GEMM does not take.
+//  * linear_f32_kernel   (float32, M > 8, linear_f32.cu) — tensor cores with the accuracy of fp32 FMAs.
+//  * linear_tiled_kernel (any M)           — 64 x 64 x 16 shared-memory tiles, 4 x 4 outputs per thread, fp32 FMA: the fall-back
+//    for sizes, pitches and addresses that the tensor-core kernels do not take.
 //
-// Products and sums are fp32 (fmaf), never TF32.  The output is fp32 or the operand type, written at a column offset
+// Products and sums are fp32 (or as good: linear_f32.cu), never TF32.  The output is fp32 or the operand type, written at a column offset
 // of a wider row (ldo) so that projections that share an input can share an output buffer.
 #include "jllama_b200.h"
+#include "linear_f32.cuh"
 #include "seq_types.cuh"
 
 namespace jl {
-
-// Many small products in one launch.  Plain batches: batch z reads x + (z / x_div) * x_bs, weights
-// w + (w_index ? w_index[z] : z) * w_bs (w_index[z] < 0: the batch is skipped) and writes out + z * o_bs (per-head matrices; one expert per (token, choice) pair when
-// decoding a mixture of experts: x_div = choices per token, so that the pairs of a token read the same input row).
-// Sorted rows (tiled kernel only): the rows come in tiles of LT_BM that each belong to one weight matrix, tile_group[tile]
-// (< 0: empty tile); row position p reads input row row_src[p] (< 0: padding, read as zero; nullptr: p itself) and writes
-// output row p — the prompt path of a mixture of experts after its tokens were sorted by expert.
-struct LinearGroup {
-  long long x_bs, w_bs, o_bs;
-  int x_div;
-  const int* w_index;
-  const int* tile_group;
-  const int* row_src;
-};
 
 constexpr int LR_ROWS = 4;      // output features per warp
 constexpr int LR_MAXM = 8;
@@ -221,7 +209,7 @@ static void lm_launch(const __nv_bfloat16* x, int ldx, const __nv_bfloat16* w, O
 #undef JL_LM
 }
 
-constexpr int LT_BM = 64, LT_BN = 64, LT_BK = 16;
+constexpr int LT_BN = 64, LT_BK = 16;              // (LT_BM rows: linear_f32.cuh)
 
 template <typename T, typename OutT>
 __global__ void __launch_bounds__(256) linear_tiled_kernel(const T* __restrict__ x, int ldx, const T* __restrict__ w,
@@ -305,6 +293,11 @@ static int launch_linear(const void* x, int ldx, const void* w, void* out, int l
     switch (M) { JL_LR(1) JL_LR(2) JL_LR(3) JL_LR(4) JL_LR(5) JL_LR(6) JL_LR(7) JL_LR(8) }
 #undef JL_LR
   } else {
+    if constexpr (sizeof(T) == 4 && sizeof(OutT) == 4) {
+      if (linear_f32_takes(M, K, ldx, g, x, w))
+        return linear_f32_launch((const float*)x, ldx, (const float*)w, (float*)out, ldo, M, N, K, act, p0, p1, st, g, nbatch) == cudaSuccess
+                   ? JL_OK : JL_ERR_CUDA;
+    }
     dim3 grid((N + LT_BN - 1) / LT_BN, (M + LT_BM - 1) / LT_BM, g.tile_group ? 1 : nbatch);
     JL_LAUNCH_PDL((linear_tiled_kernel<T, OutT>), dim3(grid), dim3(256), 0, st, (const T*)x, ldx, (const T*)w, (OutT*)out, ldo, M, N, K, act, p0, p1, g);
   }

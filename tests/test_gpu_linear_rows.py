@@ -40,3 +40,56 @@ def test_decode_rows_of_chosen_matrices():
             assert bool((out[part] == 7.0).all())
         else:
             check(out[part], x[part], w[e])
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 1, 256), (9, 300, 260), (31, 129, 1024), (33, 127, 320), (64, 1000, 2052), (65, 128, 5464), (128, 257, 512), (129, 4100, 256),
+                                   (300, 3000, 516), (1000, 640, 2048)])
+def test_float32_rows(M, N, K):
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    check(SK.linear(x, w), x, w)
+    check(SK.linear(x, w, act=SK.ACT_RELU), x, w, torch.relu)
+    wide = torch.randn(M, K + 12, generator=g).cuda()       # rows of a wider matrix
+    check(SK.linear(wide[:, 4:4 + K], w), wide[:, 4:4 + K], w)
+
+
+def test_float32_is_as_good_as_fused_multiply_add():
+    """Six products of three bfloat16 parts: 2^-22 of a sum of 2048 terms, where one part alone is off by 2^-9."""
+    g = torch.Generator().manual_seed(5)
+    x, w = torch.randn(100, 2048, generator=g).cuda(), torch.randn(500, 2048, generator=g).cuda()
+    ref = x.double() @ w.double().T
+    assert float((SK.linear(x, w).double() - ref).norm() / ref.norm()) < 2.0 ** -22
+
+
+def test_float32_batches_and_sorted_rows():
+    g = torch.Generator().manual_seed(6)
+    n, rows, N, K = 5, 20, 140, 384
+    x, w = torch.randn(n * rows, K, generator=g).cuda(), torch.randn(4, N, K, generator=g).cuda()
+    index = torch.tensor([2, -1, 0, 3, 2], dtype=torch.int32, device="cuda")
+    out = torch.full((n * rows, N), 7.0, device="cuda")
+    SK.linear_batched(x, w, out, nbatch=n, rows=rows, x_bs=rows * K, o_bs=rows * N, w_index=index)
+    for z, e in enumerate(index.tolist()):
+        part = slice(z * rows, (z + 1) * rows)
+        assert bool((out[part] == 7.0).all()) if e < 0 else check(out[part], x[part], w[e]) is None
+    group = torch.tensor([1, -1, 3], dtype=torch.int32, device="cuda")              # tiles of 64 sorted rows
+    src = torch.randint(0, n * rows, (192,), generator=g).to(torch.int32)
+    src[50:64] = -1                                                                 # padding rows read as zero
+    out = torch.full((192, N), 7.0, device="cuda")
+    SK.linear_sorted(x, w, out, group, src.cuda())
+    gathered = torch.where(src[:, None].cuda() >= 0, x[src.clamp_min(0).long().cuda()], torch.zeros((), device="cuda"))
+    check(out[:64], gathered[:64], w[1])
+    check(out[128:], gathered[128:], w[3])
+    assert bool((out[64:128] == 7.0).all()) and bool((out[50:64] == 0.0).all())
+
+
+def test_float32_infinities_and_nan_stay_what_they_are():
+    x, w = torch.ones(20, 512, device="cuda"), torch.randn(300, 512, generator=torch.Generator().manual_seed(7)).cuda()
+    x[3, 100], x[5, 7], x[6, 8] = float("inf"), float("nan"), 3.0e38
+    w[9, 200] = float("-inf")
+    w[10, 8] = 3.0e38
+    got, want = SK.linear(x, w), (x.double() @ w.double().T).float()
+    same = torch.isfinite(want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    assert torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+    keep = same & (torch.arange(20, device="cuda")[:, None] != 6)
+    assert float((got - want)[keep].abs().max()) < 1e-3

@@ -36,14 +36,11 @@ struct GemmParams {
   int a_blocks, b_blocks;   // tile counts
   int stages;
   uint64_t hint_a, hint_b;
-  // ---- split-K for swap-AB launches with fewer weight-row tiles than SMs (decode at batch 9..128: N = 4096
-  // gives 32 tiles, i.e. 22 % of the SMs streaming): each tile's K range is cut into `ksplit` work items, the
-  // fp32 partials meet in `ws` ([ksplit][features][tokens]); once all splits of a tile have arrived (ticket) each of
-  // them sums its share of the tokens in split order — deterministic — and runs the epilogue.  ksplit == 1: off.
+  // ---- split-K for swap-AB launches with fewer weight-row tiles than SMs (decode and short prompts: N = 4096 gives 32 tiles, i.e. 22 %
+  // of the SMs streaming): the CTAs of a cluster of `ksplit` share a tile, each takes a part of its K, the fp32 partials meet in
+  // distributed shared memory and each CTA sums its share of the tokens in rank order — deterministic, no scratch in global memory and
+  // nothing that launches on other streams could share — and runs the epilogue.  ksplit == 1: off.
   int ksplit;
-  float* ws;
-  int* tickets;                      // [2][ticket_half]: arrivals, completions per tile; zero between launches
-  int ticket_half;
   unsigned long long* trace;         // optional [grid][16] %globaltimer stamps (jl_gemm_set_trace), NULL = off
   // ---- grouped B operand (normal orientation only): the B tensor holds `groups` matrices of group_rows rows one after
   // the other and A-tile a uses matrix tile_group[a] (< 0: a padding tile, any matrix will do — nobody reads its rows).
@@ -64,6 +61,19 @@ __device__ __forceinline__ void gemm_stamp(const GemmParams& p, int ev) {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     p.trace[(size_t)blockIdx.x * 16 + ev] = t;
   }
+}
+
+__device__ __forceinline__ void gemm_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void gemm_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t gemm_mapa(uint32_t local_addr, int rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float gemm_ld_cluster(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
 }
 
 template <int BN, int EPI, bool SWAP, bool OUT_F32>
@@ -121,7 +131,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     }
   }
   const int num_tiles = a_blocks * p.b_blocks;
-  const int num_work = num_tiles * ksplit;              // (tile, K split) items; split-major so neighbours differ in tile
+  const int num_work = num_tiles * ksplit;              // (tile, K split) items; the splits of a tile are the CTAs of a cluster
 
   if (warp == 0) {
     // ===================================================== TMA producer
@@ -132,7 +142,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         // the weights do not depend on the previous kernel: fill the ring with A tiles NOW — they stream from HBM
         // while that kernel runs its tail — and only then wait for it; the activation tiles follow after the wait
         if ((int)blockIdx.x < num_work) {
-          const int t = blockIdx.x % num_tiles, split = blockIdx.x / num_tiles;
+          const int t = blockIdx.x / ksplit, split = blockIdx.x % ksplit;
           const int kb0 = split * num_kb / ksplit, kb1 = (split + 1) * num_kb / ksplit;
           const int a_blk = t % a_blocks;
           pre = kb1 - kb0 < stages ? kb1 - kb0 : stages;
@@ -145,7 +155,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       }
       gemm_stamp(p, 2);
       for (int wi = blockIdx.x; wi < num_work; wi += gridDim.x) {
-        const int t = wi % num_tiles, split = wi / num_tiles;
+        const int t = wi / ksplit, split = wi % ksplit;
         const int kb0 = split * num_kb / ksplit, kb1 = (split + 1) * num_kb / ksplit;
         const int b_blk = t / a_blocks;
         const int a_blk = t % a_blocks;
@@ -175,7 +185,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0; int it = 0;
       for (int wi = blockIdx.x; wi < num_work; wi += gridDim.x, ++it) {
-        const int split = wi / num_tiles;
+        const int split = wi % ksplit;
         const int kb0 = split * num_kb / ksplit, kb1 = (split + 1) * num_kb / ksplit;
         const int as = it & 1; const uint32_t aphase = (it >> 1) & 1;
         tc::mbar_wait(tempty_bar(as), aphase ^ 1);          // epilogue has drained this accumulator
@@ -203,7 +213,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     int it = 0;
     if constexpr (SWAP) pdl_wait();                         // residual, output, split-K scratch: after the previous kernel
     for (int wi = blockIdx.x; wi < num_work; wi += gridDim.x, ++it) {
-      const int t = wi % num_tiles, split = wi / num_tiles;
+      const int t = wi / ksplit, split = wi % ksplit;
       const int b_blk = t / a_blocks;
       const int a_blk = t % a_blocks;
       const int as = it & 1; const uint32_t aphase = (it >> 1) & 1;
@@ -312,14 +322,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         } else {
           // swap-AB: lanes are weight rows (output features), columns are tokens
           if (ksplit > 1) {
-            // fp32 partial of this K split: ws[split][feature][token] — a thread's tokens are contiguous, so both this
-            // store and the finish below move 4 tokens per instruction
-            if (ra < p.Ra) {
-              float* wrow = p.ws + ((size_t)split * p.Ra + ra) * (size_t)(p.b_blocks * BN) + cb0;
+            // fp32 partial of this K split, [token][feature] in shared memory: the ring is free (one work item per CTA, all its MMAs done)
+            const uint32_t part = smem_base + (uint32_t)(c0 * GEMM_BM + quarter * 32 + lane) * 4;
 #pragma unroll
-              for (int j = 0; j < CH; j += 4)
-                *reinterpret_cast<uint4*>(wrow + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-            }
+            for (int j = 0; j < CH; ++j) asm volatile("st.shared.b32 [%0], %1;" ::"r"(part + j * (GEMM_BM * 4)), "r"(v[j]) : "memory");
           } else {
             // transposed store: for a fixed token the 32 lanes write 32 consecutive features (coalesced)
 #pragma unroll
@@ -332,69 +338,53 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       if (lane == 0) tc::mbar_arrive(tempty_bar(as));
       if constexpr (SWAP) {
         if (ksplit > 1) {
-          // ---- split-K finish, shared by the K splits of the tile: all of them run at the same time (one work item
-          // per CTA, see launch_gemm), so each publishes its partial, waits until the tile's ticket shows all ksplit
-          // arrivals and then sums + emits ITS share of the tile's tokens (ksplit 16-byte loads per 4 tokens; when the
-          // last split to arrive did the whole tile alone, with scalar loads, the finish was 10 us of a 25 us GEMM).
-          // Sums run in split order: deterministic.
-          // publish: the four warps' partial stores, one barrier, then ONE fence + arrival (cumulative: it orders the
-          // stores of all 128 threads; 128 separate fences cost ~1 us more)
-          asm volatile("bar.sync 1, 128;" ::: "memory");                // the four epilogue warps
-          if (threadIdx.x == 128) {
-            gemm_stamp(p, 6);
-            __threadfence();
-            atomicAdd(p.tickets + t, 1);
-            unsigned spins = 0;
-            while (ld_acquire_gpu_u32(reinterpret_cast<const unsigned int*>(p.tickets + t)) < (unsigned)ksplit) {
-              if (++spins > (1u << 26)) {
-                printf("jllama_b200: gemm split-K timed out waiting for tile %d (block %d)\n", t, (int)blockIdx.x);
-                __trap();
-              }
-            }
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
+          // ---- split-K finish: once all partials of the cluster are there, every CTA sums and emits ITS share of the tile's tokens
+          if (threadIdx.x == 128) gemm_stamp(p, 6);
+          gemm_cluster_arrive();
+          gemm_cluster_wait();
           if (threadIdx.x == 128) gemm_stamp(p, 7);
-          {
-            // this split's share of the tile's tokens, 4 (one 16-byte load per split) at a time; the residual values
-            // are requested first, the partials (L2, written by other SMs: ld.cg) of all splits right behind them
-            const int per = ((BN + ksplit - 1) / ksplit + 3) & ~3;
-            const int j_lo = split * per, j_hi = j_lo + per < BN ? j_lo + per : BN;
-            const size_t tok_pitch = (size_t)(p.b_blocks * BN), split_stride = (size_t)p.Ra * tok_pitch;
-            const bool row_ok = ra < p.Ra;                  // (all lanes stay in the loop: the SwiGLU emit shuffles)
-            const float* wrow = p.ws + (size_t)(row_ok ? ra : 0) * tok_pitch + b_blk * BN;
-#pragma unroll 2
-            for (int j0 = j_lo; j0 < j_hi; j0 += 4) {
-              float rr[4] = {0.f, 0.f, 0.f, 0.f};
-              if constexpr (EPI == EPI_RESIDUAL) {
+          const uint32_t part = smem_base + (uint32_t)(quarter * 32 + lane) * 4;
+          const int per = ((BN + ksplit - 1) / ksplit + 3) & ~3, j_hi = split * per + per < BN ? split * per + per : BN;
+          for (int j0 = split * per; j0 < j_hi; j0 += 4) {
+            float rr[4] = {0.f, 0.f, 0.f, 0.f};
+            if constexpr (EPI == EPI_RESIDUAL) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                  const int tok = b_blk * BN + j0 + u;
-                  if (tok < p.Rb && row_ok) rr[u] = __bfloat162float(p.residual[(size_t)tok * p.ldo + ra]);
-                }
+              for (int u = 0; u < 4; ++u) {
+                const int tok = b_blk * BN + j0 + u;
+                if (tok < p.Rb && ra < p.Ra) rr[u] = __bfloat162float(p.residual[(size_t)tok * p.ldo + ra]);
               }
-              float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-              for (int sp = 0; sp < ksplit; ++sp) {
-                const float4 pv = __ldcg(reinterpret_cast<const float4*>(wrow + sp * split_stride + j0));
-                acc.x += pv.x; acc.y += pv.y; acc.z += pv.z; acc.w += pv.w;
-              }
-              const float x[4] = {acc.x, acc.y, acc.z, acc.w};
-#pragma unroll
-              for (int u = 0; u < 4; ++u) swap_emit(b_blk * BN + j0 + u, x[u], true, rr[u]);
             }
+            float q[8][4];                                // all ranks' four tokens in flight; a warp reads 128 bytes of a rank
+#pragma unroll
+            for (int sp = 0; sp < 8; ++sp)
+              if (sp < ksplit) {
+                const uint32_t at = gemm_mapa(part + j0 * (GEMM_BM * 4), sp);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) q[sp][u] = gemm_ld_cluster(at + u * (GEMM_BM * 4));
+              }
+            float x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              x[u] = q[0][u];
+#pragma unroll
+              for (int sp = 1; sp < 8; ++sp) if (sp < ksplit) x[u] += q[sp][u];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) swap_emit(b_blk * BN + j0 + u, x[u], true, rr[u]);
           }
-          // the last split to finish re-arms the tile's two counters for the next launch
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (threadIdx.x == 128) {
-            gemm_stamp(p, 8);
-            int* done = p.tickets + p.ticket_half + t;
-            if (atomicAdd(done, 1) == ksplit - 1) { *done = 0; p.tickets[t] = 0; }
-          }
+          if (threadIdx.x == 128) gemm_stamp(p, 8);
         }
       }
     }
   }
 
+  if constexpr (SWAP) {
+    if (ksplit > 1) {
+      if (warp < 4) { gemm_cluster_arrive(); gemm_cluster_wait(); }     // (the epilogue warps passed this barrier above)
+      gemm_cluster_arrive();                              // no CTA leaves while its partial may still be read
+      gemm_cluster_wait();
+    }
+  }
   tc::fence_before_sync();
   __syncthreads();
   if (threadIdx.x == 0) gemm_stamp(p, 9);
@@ -403,13 +393,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
 static unsigned long long* g_gemm_trace = nullptr;
 
-// Caller-provided scratch for split-K (jl_gemm_set_workspace), one per device; none registered → no split-K
-struct SplitKWorkspace { float* ws; size_t ws_bytes; int* tickets; int n_tickets; };
-static SplitKWorkspace g_splitk[16] = {};
-static SplitKWorkspace splitk_workspace() {
+// whether the caller allows split-K on a device (jl_gemm_set_workspace)
+static bool g_splitk[16] = {};
+static bool splitk_allowed() {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return SplitKWorkspace{};
-  return g_splitk[dev];
+  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 16 && g_splitk[dev];
 }
 
 template <int BN, int EPI, bool SWAP, bool OUT_F32>
@@ -431,16 +419,13 @@ static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int R
   int grid = p.a_blocks * p.b_blocks;
   p.ksplit = 1;
   if constexpr (SWAP) {
-    // few weight-row tiles (N <= ~9k at decode batch sizes): cut K so that (nearly) every SM streams weights.  Every
-    // (tile, split) item gets its own CTA — the shared finish in the kernel relies on all splits running at once.
-    const SplitKWorkspace wsp = splitk_workspace();
-    if (wsp.ws != nullptr && Rb <= 64 && grid * 2 <= num_sms && grid <= wsp.n_tickets / 2) {
+    // few weight-row tiles (N <= ~9k): cut K so that (nearly) every SM streams weights, at least 4 k-blocks (256 columns) per CTA
+    if (grid * 2 <= num_sms && splitk_allowed()) {
       int ks = num_sms / grid;
-      if (ks > num_kb / 4) ks = num_kb / 4;               // at least 4 k-blocks (256 columns) per item
-      if (ks > 16) ks = 16;
-      while (ks > 1 && (size_t)ks * Ra * (size_t)(p.b_blocks * BN) * sizeof(float) > wsp.ws_bytes) --ks;
+      if (ks > num_kb / 4) ks = num_kb / 4;
+      if (ks > 8) ks = 8;                                  // portable cluster size
       if (ks > 1) {
-        p.ksplit = ks; p.ws = wsp.ws; p.tickets = wsp.tickets; p.ticket_half = wsp.n_tickets / 2;
+        p.ksplit = ks;
         grid *= ks;
       }
     }
@@ -450,9 +435,7 @@ static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int R
   // memory (10 stages).  Short decode GEMMs (wqkv, wo, w2 at batch 9..128) stay under half of it, so that the CTAs of
   // the NEXT kernel of the chain fit on the same SM and their weight prefetch — issued before they wait for this
   // grid — runs under our epilogue and split-K finish; those prologue / tail latencies were most of a 25 us GEMM.
-  // A split-K launch always takes the small ring: its CTAs wait for each other, so all of them must become resident
-  // even while CTAs of a neighbouring kernel (the previous one draining, the next one prefetching) share the SMs:
-  // two ring-sized CTAs per SM always fit.
+  // A split-K launch always takes the small ring too (its partial tile, at most 64 KB, fits).
   int budget = 200 * 1024;
   if (SWAP && (p.ksplit > 1 || (size_t)Ra * K * 2 / grid <= (size_t)1280 * 1024)) budget = 100 * 1024;
   int stages = (int)(budget / STAGE_BYTES);
@@ -462,7 +445,26 @@ static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int R
   const size_t smem = (size_t)stages * STAGE_BYTES + 8 * (2 * stages + 4) + 16 + 1024;
   auto kern = gemm_kernel<BN, EPI, SWAP, OUT_F32>;
   JL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  JL_CUDA(launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS), smem, stream, ta, tb, p));
+  if (p.ksplit == 1) {
+    JL_CUDA(launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS), smem, stream, ta, tb, p));
+    return JL_OK;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.ksplit;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  count_launch();
+  JL_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
   return JL_OK;
 }
 
@@ -491,8 +493,8 @@ static int dispatch_gemm(const void* x, const void* w, const GemmParams& p, int 
 
 using namespace jl;
 
-// Registers (or, with ws == NULL, removes) the split-K scratch of the CURRENT device: `ws` fp32 workspace of
-// ws_bytes, `tickets` n_tickets ints that must be zero.  The library keeps the pointers; the caller owns the memory.
+// Allows (or, with ws == NULL, forbids) split-K on the CURRENT device.  The partials meet in distributed shared memory: the scratch and
+// the tickets are not touched.
 // Optional timeline of the single-CTA kernel: [grid][16] u64 device buffer (0 entry, 1 set-up done, 2 producer past
 // the dependency wait, 3 first stage landed, 4 last MMA issued, 5 accumulator complete, 6 partial published,
 // 7 all splits arrived, 8 share emitted, 9 exit); NULL switches it off.
@@ -502,7 +504,8 @@ extern "C" JL_API int jl_gemm_set_workspace(void* ws, size_t ws_bytes, int* tick
   int dev = 0;
   JL_CUDA(cudaGetDevice(&dev));
   JL_CHECK_ARG(dev >= 0 && dev < 16, "jl_gemm_set_workspace: device %d out of range", dev);
-  g_splitk[dev] = SplitKWorkspace{(float*)ws, ws ? ws_bytes : 0, tickets, ws ? n_tickets : 0};
+  (void)ws_bytes; (void)tickets; (void)n_tickets;
+  g_splitk[dev] = ws != nullptr;
   return JL_OK;
 }
 

@@ -61,13 +61,10 @@ int jl_gemv_tma(const void* x, const void* w, const void* norm_w, const void* re
  * SwiGLU needs N % 16 == 0. */
 int jl_gemm(const void* x, const void* w, const void* residual, void* out, int M, int N, int K, int mode,
             int out_f32, int num_sms, void* stream);
-/* Optional scratch for jl_gemm on the CURRENT device: with it, small-batch (M <= 128) launches that have fewer
- * 128-row weight tiles than half the SMs (N = 4096: 32 tiles) split K over the idle SMs; partial sums meet in `ws`
- * (fp32, ws_bytes); once all splits of a tile have arrived (`tickets`: n_tickets ints, zero on entry and between
- * calls, half of them arrival and half completion counters) each split adds the partials of its share of the tokens
- * in split order and runs the epilogue — results do not depend on arrival order.  The splits of a tile wait for each
- * other, so such a launch needs its CTAs resident together (at most one per SM is launched).  The caller owns both
- * buffers and keeps them alive; ws == NULL unregisters.  Calls that share the scratch must be ordered on one stream. */
+/* Allows split-K in jl_gemm on the CURRENT device (ws != NULL; NULL forbids it): small-batch (M <= 128) launches that have fewer
+ * 128-row weight tiles than half the SMs (N = 4096: 32 tiles) then split K over the CTAs of a cluster; partial sums meet in
+ * distributed shared memory, each CTA adds the partials of its share of the tokens in rank order and runs the epilogue —
+ * results do not depend on timing.  The buffers themselves are not used. */
 int jl_gemm_set_workspace(void* ws, size_t ws_bytes, int* tickets, int n_tickets);
 /* Timeline hook of the single-CTA GEMM kernel for scripts/gemm_trace.py: [grid][16] u64 device buffer of
  * %globaltimer stamps, NULL = off (default). */

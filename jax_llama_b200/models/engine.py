@@ -129,7 +129,7 @@ class B200Engine:
         self._mega_peer: Optional[Tuple] = None
         self.mega_write_logits = False      # True: the decode kernel also stores the fp32 [B, V] logits (tests, forward-style use)
         if self.device.type == "cuda":
-            K.ensure_gemm_workspace(self.device)          # split-K scratch of the small-batch GEMMs (before any capture)
+            K.ensure_gemm_workspace(self.device)          # the small-batch GEMMs may split K
         # Prefill at tp > 1 runs over NVLS (parallel/comm.py `NvlsPrefill`): sequence-parallel when the token count is a
         # multiple of 128·tp, otherwise tcgen05 GEMM + in-switch all-reduce kernel.  JLLAMA_SP=0 forces the latter.
         self.sequence_parallel_prefill = os.environ.get("JLLAMA_SP", "1") != "0"

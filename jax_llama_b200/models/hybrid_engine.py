@@ -430,7 +430,7 @@ class HybridEngine(B200Engine):
         With at most `BRANCH_OVERLAP_ROWS` rows (decoding) the two branches of a layer run on two streams: neither
         fills the GPU alone and a step is a chain of short dependent kernels, so the feed-forward's chain hides behind
         the mixer's.  Inside a graph capture the fork and join become edges of the captured graph.  Wider steps stay on
-        one stream (their tensor-core GEMMs share one split-K workspace)."""
+        one stream (their tensor-core GEMMs fill the GPU)."""
         eps, mult = self.eps, float(self.config.residual_mult)
         stack = [self.layers[i] for i in self.runs]
         n = len(stack)

@@ -737,7 +737,7 @@ class ParallelMixer(Mixer):
     def _both(self, h: torch.Tensor, B: int, S: int, cache: "object", layer: int, rope: Optional[Tuple]) -> Tuple[MixerParts, MixerParts]:
         """With a few rows (decoding) neither side fills the GPU and each is a chain of short dependent kernels, so the right
         side runs on a second stream beside the left one (inside a graph capture the fork and join become edges of the
-        captured graph).  Prompts stay on one stream: their tensor-core GEMMs share one split-K workspace."""
+        captured graph).  Prompts stay on one stream: their tensor-core GEMMs fill the GPU."""
         views = [_CacheView(cache, layer, i) for i in range(2)]
         if B * S <= self.OVERLAP_ROWS:
             main = torch.cuda.current_stream()

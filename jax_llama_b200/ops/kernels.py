@@ -35,16 +35,16 @@ def num_sms(device: Optional[torch.device] = None) -> int:
 _GEMM_WS: dict = {}
 
 
-def ensure_gemm_workspace(device: Optional[torch.device] = None, nbytes: int = 32 << 20) -> None:
-    """Give the library its split-K scratch for this device (fp32 partials + per-tile tickets).  Small-batch
-    GEMMs with few weight-row tiles (N = 4096 at batch 9..128) then spread their K range over all SMs.  Done once,
-    outside any stream capture (the engine calls it at construction); without it such GEMMs simply do not split."""
+def ensure_gemm_workspace(device: Optional[torch.device] = None, nbytes: int = 4) -> None:
+    """Allow split-K on this device: small-batch GEMMs with few weight-row tiles (N = 4096 at batch 9..128) then spread their K
+    range over all SMs, a cluster per tile (the partial sums meet in distributed shared memory: the registered buffer is only the
+    permission).  Done once, outside any stream capture (the engine calls it at construction); without it such GEMMs do not split."""
     idx = torch.cuda.current_device() if device is None or device.index is None else device.index
     if idx in _GEMM_WS or torch.cuda.is_current_stream_capturing() or os.environ.get("JLLAMA_NO_SPLITK") == "1":
         return
     with torch.cuda.device(idx):
         ws = torch.empty(nbytes // 4, dtype=torch.float32, device=f"cuda:{idx}")
-        tickets = torch.zeros(2048, dtype=torch.int32, device=f"cuda:{idx}")
+        tickets = torch.zeros(2, dtype=torch.int32, device=f"cuda:{idx}")
         _lib.check(_lib.lib().jl_gemm_set_workspace(ws.data_ptr(), ws.numel() * 4, tickets.data_ptr(), tickets.numel()),
                    "jl_gemm_set_workspace")
     _GEMM_WS[idx] = (ws, tickets)

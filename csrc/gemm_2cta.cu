@@ -14,8 +14,13 @@
 //     rows beyond M are clipped by the tensor map.
 // All TMA loads here read this GPU's own memory through tensor maps over local buffers.
 //
-// Used for token-major GEMMs with M >= 256 and N a multiple of 256 (every prefill GEMM of the LLaMA shapes); other
-// shapes take the single-CTA kernel (gemm_tcgen05.cu).  Replaces the cuBLAS GEMMs XLA emitted for
+// fp32 results (the projections of the hybrid family) leave the same way in 32 x 32 boxes of 128-byte rows, swizzled, through two
+// staging buffers per warp.  2048 tokens on one B200, single-CTA kernel -> this one: 10928 x 2048 91 -> 73 us, 6160 x 2048
+// 57 -> 46, 2048 x 5464 60 -> 43.
+//
+// Used for token-major GEMMs with M >= 256 and N and K multiples of 256 and 64 (every prefill GEMM of the LLaMA shapes); plain bf16 and
+// fp32 results with any N and K that are multiples of 8 (the tensor maps read zeros and clip beyond the matrix).  Other shapes take the
+// single-CTA kernel (gemm_tcgen05.cu).  Replaces the cuBLAS GEMMs XLA emitted for
 // /root/reference/jax_llama/model.py:119-150 (wq/wk/wv/wo) and :311-338 (w1/w2/w3).
 #include <stdlib.h>
 
@@ -31,10 +36,11 @@ constexpr int G2_THREADS = 256;       // warp0 TMA, warp1 MMA (leader), warp2 TM
 constexpr uint32_t G2_A_BYTES = G2_BM * G2_BK * 2;                 // 16 KB
 constexpr uint32_t G2_B_BYTES = (G2_BN / 2) * G2_BK * 2;           // 16 KB
 constexpr uint32_t G2_STAGE_BYTES = G2_A_BYTES + G2_B_BYTES;
-constexpr uint32_t G2_EPI_BYTES = 4 * 32 * 64 * 2;                 // per CTA: 4 warps x [32 rows][64 cols] bf16
+constexpr uint32_t G2_EPI_BYTES = 4 * 32 * 64 * 2;                 // per CTA: 4 warps x [32 rows][64 cols] bf16 (fp32: [32][32], twice)
 constexpr uint32_t G2_PEER_MASK = 0xFEFFFFFFu;                     // shared::cluster address of the same offset in CTA 0
 
-enum { G2_PLAIN = 0, G2_RESIDUAL = 1, G2_SWIGLU = 2 };
+enum { G2_PLAIN = 0, G2_RESIDUAL = 1, G2_SWIGLU = 2, G2_F32 = 3 };
+__host__ __device__ constexpr uint32_t g2_epi_bytes(int epi) { return epi == G2_F32 ? 2 * G2_EPI_BYTES : G2_EPI_BYTES; }
 
 struct Gemm2Params {
   const __nv_bfloat16* residual;
@@ -101,7 +107,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   const uint32_t smem_base = (tc::smem_u32(smem_raw) + 1023u) & ~1023u;
   const int stages = p.stages;
   const uint32_t epi_smem = smem_base + stages * G2_STAGE_BYTES;
-  const uint32_t bars = epi_smem + G2_EPI_BYTES;            // full[stages] | empty[stages] | tfull[2] | tempty[2]
+  const uint32_t bars = epi_smem + g2_epi_bytes(EPI);       // full[stages] | empty[stages] | tfull[2] | tempty[2]
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (stages + s); };
   auto tfull_bar = [&](int s) { return bars + 8u * (2 * stages + s); };
@@ -188,8 +194,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   } else if (warp >= 4) {
     // ===================================================== epilogue: TMEM → registers → shared → TMA store
     const int quarter = warp & 3;                           // TMEM lanes [32·quarter, 32·quarter+32)
-    const uint32_t my_smem = epi_smem + quarter * (32 * 64 * 2);
-    uint8_t* my_ptr = epi_ptr + quarter * (32 * 64 * 2);
+    const uint32_t my_smem = epi_smem + quarter * (g2_epi_bytes(EPI) / 4);
+    uint8_t* my_ptr = epi_ptr + quarter * (g2_epi_bytes(EPI) / 4);
     const uint32_t tempty_leader = g2_mapa(tempty_bar(0), 0);
     int it = 0;
     for (int t = pair; t < num_tiles; t += n_pairs, ++it) {
@@ -200,6 +206,29 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       const int row0 = a_blk * 2 * G2_BM + (int)rank * G2_BM + quarter * 32;      // first token row of this warp
       const int ra = row0 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + as * G2_BN;
+      if constexpr (EPI == G2_F32) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < G2_BN; c0 += 32) {
+          uint32_t v[32];
+          tc::tmem_ld32(t_row + c0, v);
+          tc::tmem_ld_wait();
+          const uint32_t buf = (uint32_t)(c0 >> 5 & 1) * 4096u;
+          // the store before the previous one, from this buffer, must have finished reading it
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          __syncwarp();
+          uint8_t* row = my_ptr + buf + lane * 128;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)                                     // 16-byte chunks, swizzled as the tensor map expects
+            *reinterpret_cast<uint4*>(row + ((j ^ (lane & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            // rows >= M and columns >= N are clipped; a box that lies beyond the last column is not sent at all
+            if (b_blk * G2_BN + c0 < p.N) g2_tma_store_2d(&tmap_out, my_smem + buf, b_blk * G2_BN + c0, row0);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
+      } else {
 #pragma unroll 1
       for (int c0 = 0; c0 < G2_BN; c0 += 64) {
         // 64 accumulator columns of this thread's row → up to 64 bf16 (32 for SwiGLU) in shared memory
@@ -248,9 +277,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         __syncwarp();
         if (lane == 0) {
           const int out_col = EPI == G2_SWIGLU ? (b_blk * G2_BN + c0) / 2 : b_blk * G2_BN + c0;
-          g2_tma_store_2d(&tmap_out, my_smem, out_col, row0);             // rows >= M are clipped by the tensor map
+          if (b_blk * G2_BN + c0 < p.N) g2_tma_store_2d(&tmap_out, my_smem, out_col, row0);     // rows >= M are clipped by the tensor map
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
+      }
       }
       tc::fence_before_sync();
       __syncwarp();
@@ -276,29 +306,54 @@ using namespace jl;
 static int g2_pairs_used = 0;
 extern "C" JL_API int jl_gemm_2cta_pairs(void) { return g2_pairs_used; }
 
+namespace jl {
+int gemm_2cta_f32(const void* x, const void* w, void* out, int M, int N, int K, int num_sms, void* stream);
+}
+static int gemm_2cta(const void* x, const void* w, const void* residual, void* out, int M, int N, int K, int mode, int num_sms, void* stream);
+
 extern "C" JL_API int jl_gemm_2cta(const void* x, const void* w, const void* residual, void* out, int M, int N, int K,
                                    int mode, int num_sms, void* stream) {
-  if (M < 256 || N % G2_BN != 0 || K % G2_BK != 0 || mode < 0 || mode > 2) return JL_ERR_UNSUPPORTED;
+  if (mode < 0 || mode > 2) return JL_ERR_UNSUPPORTED;
+  return gemm_2cta(x, w, residual, out, M, N, K, mode, num_sms, stream);
+}
+
+// fp32 result [M, N]
+int jl::gemm_2cta_f32(const void* x, const void* w, void* out, int M, int N, int K, int num_sms, void* stream) {
+  return gemm_2cta(x, w, nullptr, out, M, N, K, G2_F32, num_sms, stream);
+}
+
+static int gemm_2cta(const void* x, const void* w, const void* residual, void* out, int M, int N, int K, int mode, int num_sms, void* stream) {
+  const bool ragged = mode == G2_PLAIN || mode == G2_F32;
+  if (M < 256 || N % (ragged ? 8 : G2_BN) != 0 || N < G2_BN || K % (ragged ? 8 : G2_BK) != 0 || K < G2_BK) return JL_ERR_UNSUPPORTED;
   if (mode == G2_RESIDUAL && residual == nullptr) return JL_ERR_UNSUPPORTED;
+  if (mode == G2_F32 || N % G2_BN != 0 || K % G2_BK != 0) {
+    // A pair takes a 256 x 256 tile in about four fifths of the time in which a single CTA takes its 128 x 256 tile (2048 x 6160 x 2048, three
+    // rounds of either: 45.6 against 57.3 us), but its tiles are twice as high: 600 x 6160 x 2048 is two rounds of pairs (27.6 us) and one
+    // of single CTAs (23.2 us).
+    const int sms = num_sms > 0 ? num_sms : 148, cols = (N + G2_BN - 1) / G2_BN;
+    const int pair_rounds = ((M + 255) / 256 * cols + sms / 2 - 1) / (sms / 2), single_rounds = ((M + 127) / 128 * cols + sms - 1) / sms;
+    if (4 * pair_rounds > 5 * single_rounds) return JL_ERR_UNSUPPORTED;
+  }
   if (num_sms <= 0) num_sms = 148;
   const int odim = mode == G2_SWIGLU ? N / 2 : N;
   Gemm2Params p{};
   p.residual = (const __nv_bfloat16*)residual; p.M = M; p.N = N; p.K = K; p.ldo = odim;
   p.a_blocks = (M + 2 * G2_BM - 1) / (2 * G2_BM);
-  p.b_blocks = N / G2_BN;
+  p.b_blocks = (N + G2_BN - 1) / G2_BN;
   CUtensorMap ta, tb, to;
   int rc;
   if ((rc = make_tmap_2d_bf16(&ta, x, M, K, K, G2_BM))) return rc;
   if ((rc = make_tmap_2d_bf16(&tb, w, N, K, K, G2_BN / 2))) return rc;
-  if ((rc = make_tmap_2d_bf16_plain(&to, out, M, odim, odim, mode == G2_SWIGLU ? 32 : 64, 32))) return rc;
+  rc = mode == G2_F32 ? make_tmap_2d_f32(&to, out, M, odim, odim, 32) : make_tmap_2d_bf16_plain(&to, out, M, odim, odim, mode == G2_SWIGLU ? 32 : 64, 32);
+  if (rc) return rc;
   int stages = (int)((200 * 1024) / G2_STAGE_BYTES);
   if (stages > 6) stages = 6;
-  const int num_kb = K / G2_BK;
+  const int num_kb = (K + G2_BK - 1) / G2_BK;
   if (stages > num_kb * 2) stages = num_kb * 2 < 2 ? 2 : num_kb * 2;
   p.stages = stages;
-  const size_t smem = (size_t)stages * G2_STAGE_BYTES + G2_EPI_BYTES + 8 * (2 * stages + 4) + 16 + 1024;
+  const size_t smem = (size_t)stages * G2_STAGE_BYTES + g2_epi_bytes(mode) + 8 * (2 * stages + 4) + 16 + 1024;
   void (*kern)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const Gemm2Params) =
-      mode == G2_SWIGLU ? gemm2_kernel<G2_SWIGLU> : (mode == G2_RESIDUAL ? gemm2_kernel<G2_RESIDUAL> : gemm2_kernel<G2_PLAIN>);
+      mode == G2_F32 ? gemm2_kernel<G2_F32> : mode == G2_SWIGLU ? gemm2_kernel<G2_SWIGLU> : (mode == G2_RESIDUAL ? gemm2_kernel<G2_RESIDUAL> : gemm2_kernel<G2_PLAIN>);
   JL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(G2_THREADS);
@@ -307,7 +362,7 @@ extern "C" JL_API int jl_gemm_2cta(const void* x, const void* w, const void* res
   // The tile loop is persistent, so every cluster of the grid must be resident at once: a pair that only starts when
   // another one has finished doubles the run time.  Not every TPC can host a 2-CTA cluster of this size on every part
   // (measured here: fewer than num_sms / 2), so ask the runtime how many fit.
-  static int max_pairs[3] = {0, 0, 0};
+  static int max_pairs[4] = {0, 0, 0, 0};
   if (max_pairs[mode] == 0) {
     cfg.gridDim = dim3((num_sms / 2) * 2);
     cudaLaunchAttribute cattr[1];

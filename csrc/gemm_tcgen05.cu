@@ -22,6 +22,8 @@
 
 namespace jl {
 
+int gemm_2cta_f32(const void* x, const void* w, void* out, int M, int N, int K, int num_sms, void* stream);      // gemm_2cta.cu
+
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;
 constexpr int GEMM_THREADS = 256;   // warp0 TMA, warp1 MMA, warp2 TMEM alloc, warp3 idle, warps 4-7 epilogue
@@ -527,6 +529,10 @@ extern "C" JL_API int jl_gemm(const void* x, const void* w, const void* residual
   // token-major tiles of the prefill shapes go to the CTA-pair kernel (cta_group::2, gemm_2cta.cu); JLLAMA_GEMM_2CTA=0
   // keeps everything on the single-CTA kernel below (A/B measurements)
   static const bool pair_on = [] { const char* e = getenv("JLLAMA_GEMM_2CTA"); return !(e && e[0] == '0'); }();
+  if (pair_on && out_f32 && M >= 256) {
+    const int rc = gemm_2cta_f32(x, w, out, M, N, K, num_sms, stream);
+    if (rc != JL_ERR_UNSUPPORTED) return rc;
+  }
   if (pair_on && !out_f32 && M >= 256) {
     const int rc = jl_gemm_2cta(x, w, residual, out, M, N, K, mode, num_sms, stream);
     if (rc != JL_ERR_UNSUPPORTED) return rc;

@@ -238,6 +238,8 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 // and 128-byte swizzle.  Returns 0 on success (tensormap.cu).
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                       uint32_t box_rows);
+// fp32 matrix with a {32, box_rows} box (128-byte rows) and 128-byte swizzle.
+int make_tmap_2d_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
 // Un-swizzled variant with a {box_cols <= 256, box_rows <= 256} box: the tile lands row-major in smem.
 int make_tmap_2d_bf16_plain(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                             uint32_t box_cols, uint32_t box_rows);

@@ -93,3 +93,20 @@ def test_float32_infinities_and_nan_stay_what_they_are():
     assert torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
     keep = same & (torch.arange(20, device="cuda")[:, None] != 6)
     assert float((got - want)[keep].abs().max()) < 1e-3
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (257, 264, 72), (300, 2048, 5464), (511, 520, 128), (600, 1032, 264), (1000, 776, 2048)])
+def test_prompt_rows_bfloat16_on_cta_pairs(M, N, K):
+    """fp32 and bfloat16 results of ragged sizes (the last tile of rows, columns and K is cut off by the tensor maps): nothing beyond them is
+    written.  Sums of K products by a tensor core that cuts off: 2^-17 Σ |x w| is four times what 5464 terms give."""
+    g = torch.Generator().manual_seed(M + N)
+    x, w = torch.randn(M, K, generator=g).bfloat16().cuda(), torch.randn(N, K, generator=g).bfloat16().cuda()
+    room = torch.full((M * N + 4096,), 7.0, device="cuda")
+    got = SK.linear(x, w, out=room[:M * N].view(M, N))
+    ref, scale = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert bool(((got.double() - ref).abs() <= 2.0 ** -17 * scale + 1e-30).all())
+    assert bool((room[M * N:] == 7.0).all())
+    room = torch.full((M * N + 4096,), 7.0, dtype=torch.bfloat16, device="cuda")
+    got = SK.linear(x, w, out_f32=False, out=room[:M * N].view(M, N))
+    assert bool(((got.double() - ref).abs() <= 2.0 ** -17 * scale + 2.0 ** -8 * ref.abs() + 1e-30).all())
+    assert bool((room[M * N:] == 7.0).all())

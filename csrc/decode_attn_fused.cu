@@ -7,11 +7,14 @@
 //     in registers from the fp32 cos/sin table (position = cache_len − pad_left[b]);
 //   * the new token is appended to the cache by split 0 and folded into its online softmax from registers,
 //     so the streamed range is [pad_left, cache_len) and nothing written in this launch is re-read;
-//   * many more, shorter splits (64 keys each at 2k context) to cover the load latency with parallelism;
+//   * splits of the cache are chosen for the shape (see the dispatch), to cover load latency with parallelism;
 //   * the last CTA of each (batch, kv-head) to finish — found with an atomic ticket — merges the partial
 //     (m, l, o) triples, so there is no separate combine kernel.  The ticket counter is reset by that CTA.
 // Reference semantics: /root/reference/jax_llama/model.py:201-300 at S = 1.
+#include <atomic>
+
 #include "common.cuh"
+#include "tcgen05.cuh"
 #include "jllama_b200.h"
 
 namespace jl {
@@ -40,7 +43,8 @@ struct FusedAttnParams {
 // partial triples of all splits.  The ticket counter is reset by that CTA.
 template <int NG, int G, int HD>
 __device__ __forceinline__ void df_fold_and_merge(const FusedAttnParams& p, float (*s_o)[G][HD], float (*s_ml)[G][2],
-                                                  int* s_last_p, const int b, const int kvh, const int split) {
+                                                  int* s_last_p, const int b, const int kvh, const int split,
+                                                  const int active) {
   const int nh = p.nkv * G;
   int& s_last = *s_last_p;
   __syncthreads();
@@ -58,7 +62,7 @@ __device__ __forceinline__ void df_fold_and_merge(const FusedAttnParams& p, floa
       L += w * s_ml[j][g][1];
     }
     const int h = kvh * G + g;
-    if (p.splits == 1) {
+    if (active == 1) {
       p.out[((size_t)b * nh + h) * HD + d] = __float2bfloat16(L > 0.f ? acc / L : 0.f);
     } else {
       const size_t pi = ((size_t)b * nh + h) * p.splits + split;
@@ -66,7 +70,7 @@ __device__ __forceinline__ void df_fold_and_merge(const FusedAttnParams& p, floa
       if (d == 0) { p.ml_part[pi * 2] = M; p.ml_part[pi * 2 + 1] = L; }
     }
   }
-  if (p.splits == 1) return;
+  if (active == 1) return;
 
   // ---- ticket: the last CTA of this (b, kv head) merges all splits
   __threadfence();
@@ -74,7 +78,7 @@ __device__ __forceinline__ void df_fold_and_merge(const FusedAttnParams& p, floa
   if (threadIdx.x == 0) {
     int* t = p.tickets + b * p.nkv + kvh;
     const int prev = atomicAdd(t, 1);
-    s_last = prev == p.splits - 1;
+    s_last = prev == active - 1;
     if (s_last) *t = 0;                                  // everyone has arrived: safe to re-arm for the next launch
   }
   __syncthreads();
@@ -85,29 +89,39 @@ __device__ __forceinline__ void df_fold_and_merge(const FusedAttnParams& p, floa
   float* s_m = &s_o[0][0][0];                       // reuse: G*splits floats each, far below NG*G*HD
   float* s_l = s_m + G * 64;
   __syncthreads();
-  for (int i = threadIdx.x; i < G * p.splits; i += (int)blockDim.x) {
-    const int g = i / p.splits, sp = i - g * p.splits;
+  for (int i = threadIdx.x; i < G * active; i += (int)blockDim.x) {
+    const int g = i / active, sp = i - g * active;
     const size_t bh = (size_t)b * nh + kvh * G + g;
     s_m[g * 64 + sp] = __ldcg(p.ml_part + (bh * p.splits + sp) * 2);
     s_l[g * 64 + sp] = __ldcg(p.ml_part + (bh * p.splits + sp) * 2 + 1);
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < G * HD; idx += (int)blockDim.x) {
-    const int g = idx / HD, d = idx - g * HD;
+  // four columns per thread, the partial rows of 16 splits requested before the first is used (one memory round trip
+  // for up to 16 splits: a loop with a remainder took one per remaining split, 15.2 us at 12 splits against 12.1 at 8)
+  for (int idx = threadIdx.x; idx < G * (HD / 4); idx += (int)blockDim.x) {
+    const int g = idx / (HD / 4), d = 4 * (idx - g * (HD / 4));
     const size_t bh = (size_t)b * nh + kvh * G + g;
     float M = -INFINITY;
-    for (int sp = 0; sp < p.splits; ++sp) M = fmaxf(M, s_m[g * 64 + sp]);
+    for (int sp = 0; sp < active; ++sp) M = fmaxf(M, s_m[g * 64 + sp]);
     const float Ms = M == -INFINITY ? 0.f : M;
-    float acc = 0.f, L = 0.f;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f}, L = 0.f;
     const float* op = p.o_part + bh * p.splits * HD + d;
-#pragma unroll 8
-    for (int sp = 0; sp < p.splits; ++sp) {
-      const float w = exp2f(s_m[g * 64 + sp] - Ms);
-      const float ov = __ldcg(op + (size_t)sp * HD);
-      acc += w > 0.f ? w * ov : 0.f;
-      L += w * s_l[g * 64 + sp];
+    for (int sp0 = 0; sp0 < active; sp0 += 16) {
+      float4 ov[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        ov[i] = sp0 + i < active ? __ldcg(reinterpret_cast<const float4*>(op + (size_t)(sp0 + i) * HD)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (sp0 + i < active) {
+          const float w = exp2f(s_m[g * 64 + sp0 + i] - Ms);
+          if (w > 0.f) { acc[0] += w * ov[i].x; acc[1] += w * ov[i].y; acc[2] += w * ov[i].z; acc[3] += w * ov[i].w; }
+          L += w * s_l[g * 64 + sp0 + i];
+        }
+      }
     }
-    p.out[bh * HD + d] = __float2bfloat16(L > 0.f ? acc / L : 0.f);
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    *reinterpret_cast<uint2*>(p.out + bh * HD + d) = make_uint2(pack_bf16(acc[0] * inv, acc[1] * inv), pack_bf16(acc[2] * inv, acc[3] * inv));
   }
 }
 
@@ -298,41 +312,51 @@ __global__ void __launch_bounds__(DF_WARPS * 32) decode_attn_fused_kernel(const 
     for (int e = 0; e < 8; ++e) s_o[gid][g][lig * 8 + e] = o[g][e];
     if (lig == 0) { s_ml[gid][g][0] = m[g]; s_ml[gid][g][1] = l[g]; }
   }
-  df_fold_and_merge<NG, G, HD>(p, s_o, s_ml, &s_last, b, kvh, split);
+  df_fold_and_merge<NG, G, HD>(p, s_o, s_ml, &s_last, b, kvh, split, p.splits);
 }
 
 // =====================================================================================================================
-// Tensor-core variant for batched decode (batch x kv-heads large enough to fill the GPU; head_dim 128).
+// Tensor-core variant (the shapes that take it: rule at the dispatch below).
 //
 // Why: at batch 32 / 2k context the kernel above moves 268 MB per layer in 133 µs (2 TB/s) — ncu shows ~1 issued
 // instruction per cycle and no memory stall: the bf16 → fp32 unpacking and the G x 256 FMAs per key are the limit,
 // not HBM.  Here both products go through mma.sync.m16n8k16 (bf16 in, fp32 accumulate) with the G query heads of
-// the kv head as rows 0..G-1 of the 16-row operand, and K / V travel global memory → registers → MMA with no
-// shared memory, no ldmatrix and no barrier in the loop; every warp runs an independent online softmax over its
-// own 32-key blocks.
-//   S = Q Kᵀ: the contraction index d may be permuted freely as long as Q and K use the same permutation, so thread
-//     (g = lane / 4, t = lane % 4) loads the 16-byte chunks t, t + 4, t + 8, t + 12 of K[key g] (four LDG.128, each
-//     one 64 contiguous bytes per quad = whole sectors) and k-step s = 2u + v uses words (2v, 2v+1) of chunk u as
-//     (b0, b1); Q is held the same way.  Blocks two iterations ahead are requested into L2 with
-//     cp.async.bulk.prefetch (no registers), so the register loads mostly hit L2.
-//   O = P V: the C fragment of S (row g, keys 2t, 2t+1) is already the A fragment of P.  The B operand needs two
-//     KEYS of one d packed per register: thread (g, t) loads V[key][8 g .. 8 g + 7] and V[key][64 + 8 g ..] for its
-//     four keys (2t, 2t+1, 2t+8, 2t+9) and pairs them with PRMT; output tile (h, e) column n is d = 64 h + 8 n + e.
-// The new token is folded in by the same code as a block whose only valid key is slot 0.
+// the kv head as rows 0..G-1 of the 16-row operand.
+//   * Every warp is a stream of its own: one lane keeps DM_STAGES blocks of KPI keys (K and V, 128-byte swizzled TMA
+//     boxes) in flight into the warp's ring in shared memory, the warp reads them with ldmatrix and runs its own online
+//     softmax.  No barrier between warps until the fold.  Keeping the blocks in registers instead (fragments loaded
+//     from an L2 prefetched two blocks ahead) left one memory round trip exposed per block:
+//     24 rows x 8 heads, 3500 keys, 80 us (4.6 TB/s) before and 64 (5.7) with the rings, 16 x 8 heads 18.4 and 13.9.
+//   * P goes into the second product as high + low bfloat16 parts, in the two halves of the 16-row operand: rows
+//     0..7 hold the high parts and rows 8..15 the low ones, so that 16 bits of P cost no instruction more than 8 would;
+//     the two halves of the accumulator are added at the end.
+// The new token is folded in by the same code as a block whose only valid key is slot 0.  One CTA alone runs at the latency of
+// its dependent steps (ldmatrix → S → maximum → exponentials → P·V, ~0.6 us per 16 keys of a warp), many at HBM's rate.
 constexpr int DM_WARPS = 4;
+constexpr int DM_STAGES = 3;
+template <int HD> struct DmTile {
+  static constexpr int KPI = HD == 128 ? 16 : 32;            // keys of a block: 8 KB of K and V at either width
+  static constexpr int ONE_SPLIT = 40960 / HD;               // keys that one CTA takes rather than split (320, 640)
+  static constexpr int HALVES = HD / 64;                     // 64-column boxes of a row
+  static constexpr int BOX = KPI * 128;                      // bytes
+  static constexpr int STAGE = 2 * HALVES * BOX;
+  static constexpr int SMEM = DM_WARPS * DM_STAGES * STAGE + 1024;
+};
 
-__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-  return r;
+__device__ __forceinline__ void dm_ldsm(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-__device__ __forceinline__ uint32_t u4w(const uint4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
+__device__ __forceinline__ void dm_ldsm_t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
 
 // rotate the four (re, im) pairs of one 16-byte chunk; pair j uses cos/sin entry j of cs / sn
 __device__ __forceinline__ uint4 rope_chunk(const uint4 a, const float4 cs, const float4 sn) {
@@ -347,22 +371,38 @@ __device__ __forceinline__ uint4 rope_chunk(const uint4 a, const float4 cs, cons
   return make_uint4(r[0], r[1], r[2], r[3]);
 }
 
-template <int G, int KPI>
-__global__ void __launch_bounds__(DM_WARPS * 32, KPI == 32 ? 2 : 3) decode_attn_mma_kernel(const FusedAttnParams p) {
-  constexpr int HD = 128;
+template <int G, int HD>
+__global__ void __launch_bounds__(DM_WARPS * 32, 2)
+    decode_attn_mma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const FusedAttnParams p) {
+  using Tile = DmTile<HD>;
+  constexpr int KPI = Tile::KPI, HALVES = Tile::HALVES;
   constexpr int NT = KPI / 8;                  // 8-key S tiles per block
   constexpr int NB = KPI / 16;                 // 16-key P·V steps per block
-  __shared__ float s_o[DM_WARPS][G][HD];
+  constexpr int KS = HD / 16;                  // k-steps of S
+  extern __shared__ uint8_t dm_smem[];
   __shared__ float s_ml[DM_WARPS][G][2];
+  __shared__ __align__(8) uint64_t s_bar[DM_WARPS][DM_STAGES];
   __shared__ int s_last;
+  static_assert(DM_WARPS * G * HD * 4 <= Tile::SMEM - 1024, "the partial outputs take the ring's place");
+
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const uint32_t raw = tc::smem_u32(dm_smem);
+  const uint32_t ring0 = (raw + 1023u) & ~1023u;
+  const uint32_t ring = ring0 + warp * (DM_STAGES * Tile::STAGE);
+  const uint32_t bar0 = tc::smem_u32(&s_bar[warp][0]);
+  if (lane == 0) {
+#pragma unroll
+    for (int i = 0; i < DM_STAGES; ++i) tc::mbar_init(bar0 + 8 * i, 1);
+    tc::fence_barrier_init();
+  }
+  __syncwarp();
 
   pdl_wait();
   pdl_launch_dependents();
 
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int nh = p.nkv * G;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
 
   int len = *p.cache_len_ptr;
   len = len > p.T ? p.T : len;
@@ -372,58 +412,86 @@ __global__ void __launch_bounds__(DM_WARPS * 32, KPI == 32 ? 2 : 3) decode_attn_
   pos = pos < 0 ? 0 : (pos >= p.max_pos ? p.max_pos - 1 : pos);
   int chunk = (valid + p.splits - 1) / p.splits;
   chunk = ((chunk + DM_WARPS * KPI - 1) / (DM_WARPS * KPI)) * (DM_WARPS * KPI);
+  if (valid <= Tile::ONE_SPLIT) chunk = valid;            // the merge would cost more than the keys
+  const int active = valid > 0 ? (valid + chunk - 1) / chunk : 1;
+  if (split >= active) return;
   const int lo = first + split * chunk;
   const int hi = lo + chunk < len ? lo + chunk : len;
 
-  // K and V rows of a block are contiguous (KPI x 256 bytes each): one lane asks for them to be brought into L2
-  const size_t head_off = ((size_t)b * p.nkv + kvh) * (size_t)p.T * HD;
-  auto prefetch_block = [&](const int base) {
+  const int row0 = (b * p.nkv + kvh) * p.T;              // first cache row of this head in the [B·nkv·T, HD] view
+  // one lane asks for a block; a box may run past the last key (next head's rows, or zeros past the cache): those keys
+  // are masked below
+  auto request = [&](const int base, const int st) {
     if (lane == 0 && base < hi) {
-      const int n = hi - base < KPI ? hi - base : KPI;
-      const size_t off = head_off + (size_t)base * HD;
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.kc + off), "r"(n * HD * 2) : "memory");
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.vc + off), "r"(n * HD * 2) : "memory");
+      const uint32_t dst = ring + st * Tile::STAGE, bar = bar0 + 8 * st;
+      tc::mbar_expect_tx(bar, Tile::STAGE);
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) {
+        tc::tma_load_2d(dst + h * Tile::BOX, &tm_k, bar, 64 * h, row0 + base, tc::EVICT_FIRST);
+        tc::tma_load_2d(dst + (HALVES + h) * Tile::BOX, &tm_v, bar, 64 * h, row0 + base, tc::EVICT_FIRST);
+      }
     }
   };
-  prefetch_block(lo + warp * KPI);                       // overlaps the position → cos/sin → q dependency chain below
-  prefetch_block(lo + warp * KPI + DM_WARPS * KPI);
+#pragma unroll
+  for (int i = 0; i < DM_STAGES; ++i) request(lo + (i * DM_WARPS + warp) * KPI, i);
 
+  // the new token belongs to the last warp of the last working split, which has the fewest keys
+  const bool newest = split == active - 1 && warp == DM_WARPS - 1;
   const __nv_bfloat16* row = p.qkv + (size_t)b * (nh + 2 * p.nkv) * HD;
-  const float4* cos4 = reinterpret_cast<const float4*>(p.cos_t) + (size_t)pos * (HD / 8) + t;   // chunk t + 4u: entry 4u
-  const float4* sin4 = reinterpret_cast<const float4*>(p.sin_t) + (size_t)pos * (HD / 8) + t;
+  uint4 kn = make_uint4(0, 0, 0, 0), vn = kn;             // chunk `lane` of its rows, asked for ahead of the loop
+  if (newest && lane < HD / 8) {
+    kn = *reinterpret_cast<const uint4*>(row + (size_t)(nh + kvh) * HD + 8 * lane);
+    vn = *reinterpret_cast<const uint4*>(row + (size_t)(nh + p.nkv + kvh) * HD + 8 * lane);
+  }
+  const float* cos_p = p.cos_t + (size_t)pos * (HD / 2);
+  const float* sin_p = p.sin_t + (size_t)pos * (HD / 2);
 
   // Q of head kvh·G + g, rotated and rounded to bf16 (as the unfused path does): qa[s] = (a0, a2) of k-step s
-  uint32_t qa[8][2];
+  uint32_t qa[KS][2];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    uint4 r = make_uint4(0, 0, 0, 0);
-    if (g < G)
-      r = rope_chunk(*reinterpret_cast<const uint4*>(row + (size_t)(kvh * G + g) * HD + 8 * t + 32 * u),
-                     __ldg(cos4 + 4 * u), __ldg(sin4 + 4 * u));
-    qa[2 * u][0] = r.x; qa[2 * u][1] = r.y; qa[2 * u + 1][0] = r.z; qa[2 * u + 1][1] = r.w;
-  }
+  for (int s = 0; s < KS; ++s)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      qa[s][i] = 0;
+      if (g < G) {
+        const int pair = 8 * s + 4 * i + t;
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(row + (size_t)(kvh * G + g) * HD + 2 * pair);
+        const float c = __ldg(cos_p + pair), sn = __ldg(sin_p + pair), re = bf16_lo(w), im = bf16_hi(w);
+        qa[s][i] = pack_bf16(re * c - im * sn, re * sn + im * c);
+      }
+    }
 
   float m = -INFINITY, l = 0.f;                // row g: m is quad-uniform, l is this thread's share of the sum
-  float o[2][8][4];
+  float o[HD / 8][4];                          // [0..1]: row g against P's high parts, [2..3]: against the low parts
 #pragma unroll
-  for (int h = 0; h < 2; ++h)
+  for (int e = 0; e < HD / 8; ++e)
 #pragma unroll
-    for (int e = 0; e < 8; ++e)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) o[h][e][i] = 0.f;
+    for (int i = 0; i < 4; ++i) o[e][i] = 0.f;
 
-  const __nv_bfloat16* kbase = p.kc + head_off + 8 * t;
-  const __nv_bfloat16* vbase = p.vc + head_off + 8 * g;
+  // ldmatrix addresses within a 64-column box: row r's 16-byte chunk c lies at r * 128 + ((c ^ (r & 7)) << 4)
+  const int l7 = lane & 7, q8 = lane >> 3;
+  uint32_t koff[2], voff[4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) koff[i] = l7 * 128 + (((4 * i + q8) ^ l7) << 4);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) voff[i] = ((q8 & 1) * 8 + l7) * 128 + (((2 * i + (q8 >> 1)) ^ l7) << 4);
 
-  // one online-softmax update with a KPI-key block whose K / V fragments are in registers; keys >= limit are masked
-  auto process = [&](const uint4 (&kr)[NT][4], const uint4 (&vr)[NB][4][2], const int base, const int limit) {
-    float c[NT][4];
+  // one online-softmax update with the block in stage `st`; keys >= limit are masked
+  auto process = [&](const int st, const int base, const int limit) {
+    const uint32_t ks = ring + st * Tile::STAGE, vs = ks + HALVES * Tile::BOX;
+    float c[NT][2];
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
-      c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
+      float d[2][4] = {};                                  // two chains: half the latency of the dependent products
 #pragma unroll
-      for (int s = 0; s < 8; ++s)
-        mma_16816(c[j], qa[s][0], qa[s][1], u4w(kr[j][s >> 1], (s & 1) * 2), u4w(kr[j][s >> 1], (s & 1) * 2 + 1));
+      for (int i = 0; i < KS / 2; ++i) {
+        uint32_t r[4];
+        dm_ldsm(ks + (i >> 1) * Tile::BOX + j * 1024 + koff[i & 1], r);
+        mma_16816(d[0], qa[2 * i][0], 0u, qa[2 * i][1], 0u, r[0], r[1]);
+        mma_16816(d[1], qa[2 * i + 1][0], 0u, qa[2 * i + 1][1], 0u, r[2], r[3]);
+      }
+      c[j][0] = d[0][0] + d[1][0];
+      c[j][1] = d[0][1] + d[1][1];
     }
     float mx = -INFINITY;
 #pragma unroll
@@ -447,99 +515,107 @@ __global__ void __launch_bounds__(DM_WARPS * 32, KPI == 32 ? 2 : 3) decode_attn_
       psum += c[j][0] + c[j][1];
     }
     l = l * corr + psum;
+    if (__any_sync(0xffffffffu, corr != 1.f)) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+      for (int e = 0; e < HD / 8; ++e)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) { o[h][e][0] *= corr; o[h][e][1] *= corr; }
+        for (int i = 0; i < 4; ++i) o[e][i] *= corr;
+    }
 #pragma unroll
     for (int kb = 0; kb < NB; ++kb) {
-      const uint32_t a0 = pack_bf16(c[2 * kb][0], c[2 * kb][1]), a2 = pack_bf16(c[2 * kb + 1][0], c[2 * kb + 1][1]);
+      const float(&c0)[2] = c[2 * kb];
+      const float(&c1)[2] = c[2 * kb + 1];
+      const uint32_t h0 = pack_bf16(c0[0], c0[1]), h2 = pack_bf16(c1[0], c1[1]);
+      const uint32_t l0 = pack_bf16(c0[0] - bf16_lo(h0), c0[1] - bf16_hi(h0));
+      const uint32_t l2 = pack_bf16(c1[0] - bf16_lo(h2), c1[1] - bf16_hi(h2));
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const uint32_t sel = (e & 1) ? 0x7632u : 0x5410u;
-          const uint32_t b0 = prmt(u4w(vr[kb][0][h], e >> 1), u4w(vr[kb][1][h], e >> 1), sel);
-          const uint32_t b1 = prmt(u4w(vr[kb][2][h], e >> 1), u4w(vr[kb][3][h], e >> 1), sel);
-          mma_16816(o[h][e], a0, a2, b0, b1);
-        }
+      for (int e = 0; e < HD / 16; ++e) {
+        uint32_t r[4];
+        dm_ldsm_t(vs + (e >> 2) * Tile::BOX + kb * 2048 + voff[e & 3], r);
+        mma_16816(o[2 * e], h0, l0, h2, l2, r[0], r[1]);
+        mma_16816(o[2 * e + 1], h0, l0, h2, l2, r[2], r[3]);
+      }
     }
   };
+  // V rows [n, KPI) of a stage hold no key: zero them, a weight of zero times an unused slot's NaN would be NaN
+  auto zero_v_rows = [&](const int st, const int n) {
+    for (int i = lane; i < (KPI - n) * 8 * HALVES; i += 32) {
+      const int r = n + i / (8 * HALVES), c = i % (8 * HALVES);
+      const uint32_t a = ring + st * Tile::STAGE + (HALVES + (c >> 3)) * Tile::BOX + r * 128 + (c & 7) * 16;
+      asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(a), "r"(0) : "memory");
+    }
+    __syncwarp();
+  };
 
+  int st = 0;
+  uint32_t phase = 0;
   for (int base = lo + warp * KPI; base < hi; base += DM_WARPS * KPI) {
-    prefetch_block(base + 2 * DM_WARPS * KPI);
-    uint4 kr[NT][4], vr[NB][4][2];
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      const int key = base + 8 * j + g;
-      const __nv_bfloat16* src = kbase + (size_t)key * HD;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) kr[j][u] = key < hi ? ldg_stream(src + 32 * u) : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int kb = 0; kb < NB; ++kb)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int key = base + 16 * kb + 2 * t + (q & 1) + (q >> 1) * 8;
-        const __nv_bfloat16* src = vbase + (size_t)key * HD;
-        vr[kb][q][0] = key < hi ? ldg_stream(src) : make_uint4(0, 0, 0, 0);
-        vr[kb][q][1] = key < hi ? ldg_stream(src + 64) : make_uint4(0, 0, 0, 0);
-      }
-    process(kr, vr, base, hi);
+    tc::mbar_wait(bar0 + 8 * st, phase);
+    if (base + KPI > hi) zero_v_rows(st, hi - base);
+    process(st, base, hi);
+    __syncwarp();                                          // every lane has read the stage: it may be filled again
+    request(base + DM_STAGES * DM_WARPS * KPI, st);
+    if (++st == DM_STAGES) { st = 0; phase ^= 1; }
   }
 
-  // ---- the new token (split 0, warp 0): rotate k, append k and v to the cache, fold it in as key 0 of a block
-  if (split == 0 && warp == 0) {
-    uint4 kr[NT][4], vr[NB][4][2];
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int u = 0; u < 4; ++u) kr[j][u] = make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (int kb = 0; kb < NB; ++kb)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) vr[kb][q][0] = vr[kb][q][1] = make_uint4(0, 0, 0, 0);
-    if (g == 0) {                                          // K fragment of key 0 lives in the quad g == 0
-      const __nv_bfloat16* src = row + (size_t)(nh + kvh) * HD + 8 * t;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        kr[0][u] = rope_chunk(*reinterpret_cast<const uint4*>(src + 32 * u), __ldg(cos4 + 4 * u), __ldg(sin4 + 4 * u));
-        if (len < p.T) *reinterpret_cast<uint4*>(p.kc + head_off + (size_t)len * HD + 8 * t + 32 * u) = kr[0][u];
-      }
-    }
-    if (t == 0) {                                          // V fragments of key 0 = key slot 2t, t == 0
-      const __nv_bfloat16* src = row + (size_t)(nh + p.nkv + kvh) * HD + 8 * g;
-      vr[0][0][0] = *reinterpret_cast<const uint4*>(src);
-      vr[0][0][1] = *reinterpret_cast<const uint4*>(src + 64);
+  // ---- the new token: rotate k, append k and v to the cache, fold it in as key 0 of a block
+  if (newest) {                                            // all copies into this warp's ring have been waited for
+    const size_t slot = ((size_t)row0 + len) * HD;
+    if (lane < HD / 8) {                                   // row 0 of a box is not permuted
+      kn = rope_chunk(kn, __ldg(reinterpret_cast<const float4*>(cos_p) + lane), __ldg(reinterpret_cast<const float4*>(sin_p) + lane));
       if (len < p.T) {
-        *reinterpret_cast<uint4*>(p.vc + head_off + (size_t)len * HD + 8 * g) = vr[0][0][0];
-        *reinterpret_cast<uint4*>(p.vc + head_off + (size_t)len * HD + 64 + 8 * g) = vr[0][0][1];
+        *reinterpret_cast<uint4*>(p.kc + slot + 8 * lane) = kn;
+        *reinterpret_cast<uint4*>(p.vc + slot + 8 * lane) = vn;
       }
+      const uint32_t a = ring + (lane >> 3) * Tile::BOX + (lane & 7) * 16;
+      asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(kn.x), "r"(kn.y), "r"(kn.z), "r"(kn.w) : "memory");
+      asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a + HALVES * Tile::BOX), "r"(vn.x), "r"(vn.y), "r"(vn.z), "r"(vn.w)
+                   : "memory");
     }
-    process(kr, vr, 0, 1);
+    zero_v_rows(0, 1);
+    process(0, 0, 1);
   }
 
-  // ---- this warp's triple → shared memory; tile (h, e) holds columns d = 64 h + 8 n + e, n = 2t (c0), 2t + 1 (c1)
+  // ---- this warp's triple → shared memory, over the rings once every warp is done with its own
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
+  __syncthreads();
+  float(*s_o)[G][HD] = reinterpret_cast<float(*)[G][HD]>(dm_smem + (ring0 - raw));
   if (g < G) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        s_o[warp][g][64 * h + 16 * t + e] = o[h][e][0];
-        s_o[warp][g][64 * h + 16 * t + 8 + e] = o[h][e][1];
-      }
+    for (int e = 0; e < HD / 8; ++e)
+      *reinterpret_cast<float2*>(&s_o[warp][g][8 * e + 2 * t]) = make_float2(o[e][0] + o[e][2], o[e][1] + o[e][3]);
     if (t == 0) { s_ml[warp][g][0] = m; s_ml[warp][g][1] = l; }
   }
-  df_fold_and_merge<DM_WARPS, G, HD>(p, s_o, s_ml, &s_last, b, kvh, split);
+  df_fold_and_merge<DM_WARPS, G, HD>(p, s_o, s_ml, &s_last, b, kvh, split, active);
+}
+
+template <int G, int HD>
+static int launch_decode_mma(const FusedAttnParams& p, int B, cudaStream_t s) {
+  CUtensorMap tk, tv;
+  const uint64_t rows = (uint64_t)B * p.nkv * p.T;
+  int rc = make_tmap_2d_bf16(&tk, p.kc, rows, HD, HD, DmTile<HD>::KPI);
+  if (rc == JL_OK) rc = make_tmap_2d_bf16(&tv, p.vc, rows, HD, HD, DmTile<HD>::KPI);
+  if (rc != JL_OK) return rc;
+  // attributes belong to the device's context: set at the first call on each (bit per device; setting them twice is harmless)
+  static std::atomic<uint64_t> set{0};
+  int dev = 0;
+  JL_CUDA(cudaGetDevice(&dev));
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (bit == 0 || !(set.load(std::memory_order_acquire) & bit)) {
+    JL_CUDA(cudaFuncSetAttribute(decode_attn_mma_kernel<G, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, DmTile<HD>::SMEM));
+    JL_CUDA(cudaFuncSetAttribute(decode_attn_mma_kernel<G, HD>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    set.fetch_or(bit, std::memory_order_release);
+  }
+  JL_CUDA(launch_pdl(decode_attn_mma_kernel<G, HD>, dim3(p.splits, p.nkv, B), dim3(DM_WARPS * 32), DmTile<HD>::SMEM, s, tk, tv, p));
+  return JL_OK;
 }
 
 }  // namespace jl
 
 using namespace jl;
 
-static int g_attn_variant = 0;      // 0 = by shape, 1 = SIMT kernel, 2 = tensor-core kernel (head_dim 128 only)
+static int g_attn_variant = 0;      // 0 = by shape, 1 = SIMT kernel, 2 = tensor-core kernel
 
 // Pins the kernel behind jl_decode_attn_fused (tests and A/B measurements); 0 restores the shape-based choice.
 extern "C" JL_API int jl_decode_attn_fused_set_variant(int variant) {
@@ -582,36 +658,38 @@ extern "C" JL_API int jl_decode_attn_fused(const void* qkv, void* k_cache, void*
   p.scale_log2 = scale * 1.4426950408889634f;
   auto s = (cudaStream_t)stream;
   cudaError_t e = cudaErrorInvalidValue;
-  // 16 or more (batch, kv-head) pairs: the tensor-core kernel (see its header; measured faster from 2 x 8 pairs up:
-  // 19.5 vs 27.6 us at 2k context, 55 vs 162 us at batch 32); below that the SIMT kernel with many short splits
-  const bool use_mma = hd == 128 && (g_attn_variant == 2 || (g_attn_variant == 0 && B * nkv >= 16));
+  // The tensor-core kernel, but for one query head per kv head over a cache of at most 128 slots, where the ring and the
+  // 16-row products have nothing to share and the SIMT kernel's shorter start wins (2.8 vs 3.7 us at 4 heads of 128 and 128 slots, 5.1 vs 3.7
+  // at 160).  Everywhere else it
+  // was the slower one of the two: 20 vs 9.1 us (1 x 8 heads, 4000 keys), 3.4 vs 4.8 (3 x 4 heads of 64, 100 keys), 52
+  // vs 15.7 (16 x 8 heads of 64, 2500 keys), 193 vs 64 (24 x 8 heads, 4000 keys).
+  const bool use_mma = (hd == 128 || hd == 64) && (g_attn_variant == 2 || (g_attn_variant == 0 && !(G == 1 && T <= 128)));
   if (use_mma) {
-    // one resident wave (2 CTAs per SM) of long CTAs: every CTA pays the position → q → first-block latency chain and
-    // the fold / ticket / merge tail once, and with 2.6 waves of short CTAs that fixed cost was ~25 of 72 us at
-    // batch 32.  The scratch layout (ticket offset) still follows the caller's `splits`.
     static int sms = 0;
     if (sms == 0) {
       int dev = 0;
       if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         sms = 148;
     }
-    // fewest splits whose CTA count fills whole waves of the 2 x sms resident slots best (e.g. 192 pairs x 3 = 576 of
-    // 592 slots); at equal fill the smaller count wins (less fixed cost, no merge at 1)
-    const int slots = 2 * sms, pairs = B * nkv;
+    // Splits by estimate, the caller's count (which sizes the scratch) being the most there may be.  A call costs the
+    // larger of its bytes and of the waves of CTAs (2 per SM) times the keys of one CTA at the pace of its dependent
+    // blocks; each wave adds the way from the position to the first block, splitting adds the merge.  The five constants are
+    // fits to 31 shapes swept over 1 to 32 splits; the choice was within 5 % of the best count in all but two of them (8 %).
+    const int slots = 2 * sms, pairs = B * nkv, step = hd == 128 ? 64 : 128;
+    const float key_us = hd == 128 ? 0.0091f : 0.0039f, bw_us = (float)pairs * (float)T * (float)hd * 4.f / 6.0e6f;
     int ms = 1;
     float best = 0.f;
-    for (int c = 1; c <= splits && c <= 16; ++c) {
-      const int n = pairs * c;
-      const float fill = (float)n / (float)(((n + slots - 1) / slots) * slots);
-      if (fill > best + 0.02f) { best = fill; ms = c; }
+    for (int c = 1; c <= splits && c <= 32; ++c) {
+      const float waves = (float)((pairs * c + slots - 1) / slots);
+      const float chunk = (float)(((T + c - 1) / c + step - 1) / step * step);
+      const float us = fmaxf(bw_us, waves * chunk * key_us) + 3.4f * waves + (c > 1 ? 2.5f + 0.12f * c : 0.f);
+      if (c == 1 || us < best) { best = us; ms = c; }
     }
     p.splits = ms;
-    splits = ms;
-#define JL_DM(G_) \
-    if (G == G_) e = launch_pdl(decode_attn_mma_kernel<G_, 32>, dim3(splits, nkv, B), dim3(DM_WARPS * 32), 0, s, p);
-    JL_DM(1) else JL_DM(2) else JL_DM(4) else JL_DM(8)
+#define JL_DM(G_, HD_) if (G == G_ && hd == HD_) return launch_decode_mma<G_, HD_>(p, B, s);
+    JL_DM(1, 128) JL_DM(2, 128) JL_DM(4, 128) JL_DM(8, 128)
+    JL_DM(1, 64) JL_DM(2, 64) JL_DM(4, 64) JL_DM(8, 64)
 #undef JL_DM
-    if (e != cudaErrorInvalidValue) { JL_CUDA(e); return JL_OK; }
   }
 #define JL_DF(G_, HD_) \
   if (G == G_ && hd == HD_) e = launch_pdl(decode_attn_fused_kernel<G_, HD_>, dim3(splits, nkv, B), dim3(DF_WARPS * 32), 0, s, p);

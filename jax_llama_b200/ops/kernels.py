@@ -268,7 +268,7 @@ def decode_attn_fused_plan(B: int, nh: int, nkv: int, hd: int, max_len: int, dev
 
 
 def set_decode_attn_variant(variant: int) -> None:
-    """Pins the kernel behind `decode_attn_fused`: 0 = by shape (default), 1 = SIMT, 2 = tensor-core (head_dim 128).
+    """Pins the kernel behind `decode_attn_fused`: 0 = by shape (default), 1 = SIMT, 2 = tensor-core.
     Process-wide; for tests and A/B timing."""
     _lib.check(_lib.lib().jl_decode_attn_fused_set_variant(int(variant)), "jl_decode_attn_fused_set_variant")
 

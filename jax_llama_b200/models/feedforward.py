@@ -175,8 +175,7 @@ class MoeFeedForward:
             xs = SK.moe_gather(h, row_src)
             if s.gated:
                 gu = SK.gemm_grouped(xs, self.up, tile_group, tiles_used=used)
-                t = _gated_act(gu, self.u_off, s.ff, s.act, s.limit, h.dtype, rows_used=used, rows_mult=SK.GEMM_TILE_ROWS,
-                               zero=True)
+                t = _gated_act(gu, self.u_off, s.ff, s.act, s.limit, h.dtype, rows_used=used, rows_mult=SK.GEMM_TILE_ROWS)
             else:
                 t = SK.gemm_grouped(xs, self.up, tile_group, act=self.act, out_f32=False, tiles_used=used)
             y = SK.gemm_grouped(t, self.down, tile_group, tiles_used=used)

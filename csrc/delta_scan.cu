@@ -220,68 +220,61 @@ struct DeltaHeadParams {
 
 __device__ __forceinline__ float delta_head_decay(float z, float a_log) { return expf(-expf(a_log) * delta_softplus(z)); }
 
-// A warp takes one token of one q / k head: dot products with the DH_NB - 1 tokens before it, norms, the normalised rows, gates and values.
-// (One CTA of four warps per token and head, a warp per lag: 66 us for 2000 tokens x 16 heads of 64 x 128 against 50 us.)
-constexpr int DH_PREP_WARPS = 4;
-
+// grid (tokens, q / k heads), 128 threads: warp l forms the dot products at lag l.  (One warp per token with all lags in registers is
+// the faster kernel alone, 50 us against 66 for 2000 tokens x 16 heads of 64 x 128, but as a link of the launch chain it made the
+// layer slower: 452 us a pass against 385.)
 template <typename T, int DP>
-__global__ void __launch_bounds__(32 * DH_PREP_WARPS) delta_head_prep_kernel(DeltaHeadParams p, const T* __restrict__ a_bias, const T* __restrict__ a_log) {
+__global__ void __launch_bounds__(32 * DH_NB) delta_head_prep_kernel(DeltaHeadParams p, const T* __restrict__ a_bias, const T* __restrict__ a_log) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
   pdl_launch_dependents();
+  __shared__ float hs[3][DH_NB];                               // per lag: q.k, k.k, |k| factor of the earlier token
+  __shared__ float rq_s;
   constexpr int PITCH = DP + 4;
-  const int g = blockIdx.y, lane = threadIdx.x & 31;
-  const size_t m = (size_t)blockIdx.x * DH_PREP_WARPS + (threadIdx.x >> 5);
-  if (m >= (size_t)p.B * p.S) return;
+  const int g = blockIdx.y, lane = threadIdx.x & 31, lag = threadIdx.x >> 5;
+  const size_t m = blockIdx.x;
   const int b = (int)(m / p.S), s = (int)(m % p.S);
   const float* ur = p.u + m * p.ldu;
   const float* q = ur + p.q_off + g * p.D;
   const float* k = ur + p.k_off + g * p.D;
-  float qq = 0.0f, ll[DH_NB], ql[DH_NB], kk[DH_NB];
-#pragma unroll
-  for (int l = 0; l < DH_NB; ++l) ll[l] = ql[l] = kk[l] = 0.0f;
-  for (int d = lane; d < p.D; d += 32) {
-    const float qv = q[d], kv = k[d];
-    qq = fmaf(qv, qv, qq);
-#pragma unroll
-    for (int l = 0; l < DH_NB; ++l) {
-      if (l > s) break;                                        // a token of an earlier call is never in a block with this one
-      const float lv = l == 0 ? kv : k[d - (ptrdiff_t)l * p.ldu];
-      ll[l] = fmaf(lv, lv, ll[l]); ql[l] = fmaf(qv, lv, ql[l]); kk[l] = fmaf(kv, lv, kk[l]);
+  if (lag <= s) {
+    const float* kl = k - (size_t)lag * p.ldu;
+    float qq = 0.0f, ll = 0.0f, ql = 0.0f, kk = 0.0f;
+    for (int d = lane; d < p.D; d += 32) {
+      const float qv = q[d], kv = k[d], lv = kl[d];
+      qq = fmaf(qv, qv, qq); ll = fmaf(lv, lv, ll); ql = fmaf(qv, lv, ql); kk = fmaf(kv, lv, kk);
     }
-  }
-  const float rq = 1.0f / sqrtf(warp_sum(qq) + 1e-6f) / sqrtf((float)p.D);
-  float rl[DH_NB];                                             // per lag: |k| factor of the earlier token
-#pragma unroll
-  for (int l = 0; l < DH_NB; ++l) {
-    rl[l] = l <= s ? 1.0f / sqrtf(warp_sum(ll[l]) + 1e-6f) : 0.0f;
-    ql[l] = warp_sum(ql[l]);
-    if (l > 0) kk[l] = warp_sum(kk[l]);
-  }
-  const float rk = rl[0];
+    qq = warp_sum(qq); ll = warp_sum(ll); ql = warp_sum(ql); kk = warp_sum(kk);
+    if (lane == 0) {
+      hs[0][lag] = ql; hs[1][lag] = kk; hs[2][lag] = 1.0f / sqrtf(ll + 1e-6f);
+      if (lag == 0) rq_s = 1.0f / sqrtf(qq + 1e-6f) / sqrtf((float)p.D);
+    }
+  } else if (lane == 0) { hs[0][lag] = hs[1][lag] = hs[2][lag] = 0.0f; }       // a token of an earlier call is never in a block with this one
+  __syncthreads();
+  const float rq = rq_s, rk = hs[2][0];
   const int P = p.P;
   const size_t row = ((size_t)b * p.G + g) * p.S + s;
   float* dst = p.qk + row * (2 * P * PITCH);
-  for (int d = lane; d < P * DP; d += 32) {
+  for (int d = threadIdx.x; d < P * DP; d += blockDim.x) {
     float* o = dst + (d / DP) * PITCH + d % DP;
     o[0] = d < p.D ? q[d] * rq : 0.0f;
     o[P * PITCH] = d < p.D ? k[d] * rk : 0.0f;
   }
-  float pv = 0.0f;
-#pragma unroll
-  for (int l = 0; l < DH_NB; ++l) {
-    if (lane == l) pv = ql[l] * rq * rl[l];
-    if (l > 0 && lane == DH_NB + l - 1) pv = kk[l] * rk * rl[l];
+  if (threadIdx.x < DH_PAIR) {
+    const int i = threadIdx.x;
+    float v = 0.0f;
+    if (i < DH_NB) v = hs[0][i] * rq * hs[2][i];
+    else if (i < 2 * DH_NB - 1) v = hs[1][i - DH_NB + 1] * rk * hs[2][i - DH_NB + 1];
+    p.pair[row * DH_PAIR + i] = v;
   }
-  if (lane < DH_PAIR) p.pair[row * DH_PAIR + lane] = pv;
   const int per = p.H / p.G, ns = (p.Dv + p.cols - 1) / p.cols, width = ns * p.cols;
-  for (int i = lane; i < per; i += 32) {
+  for (int i = threadIdx.x; i < per; i += blockDim.x) {
     const int h = g * per + i;
     float* gt = p.gate + (((size_t)b * p.H + h) * p.S + s) * DH_GATE;
     gt[0] = sigmoid_f(p.y[m * p.ldy + p.b_off + h]);
     gt[1] = delta_head_decay(p.y[m * p.ldy + p.a_off + h] + to_f(a_bias[h]), to_f(a_log[h]));
     gt[2] = gt[3] = 0.0f;
   }
-  for (int i = lane; i < per * width; i += 32) {
+  for (int i = threadIdx.x; i < per * width; i += blockDim.x) {
     const int h = g * per + i / width, c = i % width;
     p.val[((((size_t)b * p.H + h) * ns + c / p.cols) * p.S + s) * p.cols + c % p.cols] = c < p.Dv ? ur[p.v_off + h * p.Dv + c] : 0.0f;
   }
@@ -563,7 +556,7 @@ static int delta_head_launch(DeltaHeadParams p, const DeltaHeadPlan& plan, const
     JL_CUDA(cudaGetLastError());
     return JL_OK;
   }
-  JL_LAUNCH_PDL((delta_head_prep_kernel<T, DP>), dim3((p.B * p.S + DH_PREP_WARPS - 1) / DH_PREP_WARPS, p.G), dim3(32 * DH_PREP_WARPS), 0, stream, p, (const T*)a_bias, (const T*)a_log);
+  JL_LAUNCH_PDL((delta_head_prep_kernel<T, DP>), dim3(p.B * p.S, p.G), dim3(32 * DH_NB), 0, stream, p, (const T*)a_bias, (const T*)a_log);
   JL_CUDA(cudaGetLastError());
   int tc = DS_TC;                                               // tokens per pipeline stage: two stages have to fit
   while (tc > DH_NB && (size_t)2 * tc * SF * sizeof(float) > 100 * 1024) tc /= 2;

@@ -289,6 +289,10 @@ __device__ __forceinline__ void sf_sync(cg::cluster_group& cl, int size) {
   if (size > 1) cl.sync(); else __syncthreads();
 }
 
+// "I have started" without an order of memory: the barrier's wait comes after the pass over the slice, which hides it
+__device__ __forceinline__ void sf_cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void sf_cluster_wait() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
+
 // One row as its cluster sees it.
 struct SfCluster {
   SfShared* s;
@@ -539,6 +543,7 @@ __global__ void __launch_bounds__(SF_THREADS, GREEDY ? 2 : 1) sample_full_kernel
   cg::cluster_group cl = cg::this_cluster();
   const int csize = (int)cl.num_blocks(), crank = (int)cl.block_rank();
   const int row = blockIdx.x / csize;
+  if (csize > 1) sf_cluster_arrive();                       // waited for before the first store into another CTA's shared memory
   if (p.cand != nullptr) {
     // every (rank, CTA) of the decode kernel has published its candidate for this row ⇒ its logits stores landed
     const unsigned int gen_now = *reinterpret_cast<const volatile unsigned int*>(p.gen);
@@ -593,6 +598,7 @@ __global__ void __launch_bounds__(SF_THREADS, GREEDY ? 2 : 1) sample_full_kernel
     if ((threadIdx.x & 31) == 0) { atomicMax(&sb.best_local, best); if (any_nan) sb.odd_local = 1; }
   }
   __syncthreads();
+  if (csize > 1) sf_cluster_wait();                         // every CTA of the cluster runs: its shared memory exists
   if ((int)threadIdx.x < csize) {
     SfBest* o = cl.map_shared_rank(&sb, (int)threadIdx.x);
     o->best[crank] = sb.best_local; o->odd[crank] = sb.odd_local;

@@ -142,3 +142,20 @@ def test_rows_without_probabilities_still_give_a_token(bad):
     assert bool(((y >= 0) & (y < 20000)).all())
     clean = K.sample_full(x[[0, 0, 2]].contiguous(), temperature=0.9, top_p=0.9, seed=3)
     assert y[0] == clean[0] and y[2] == clean[2]
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 8192), (2, 8192), (1, 16385), (7, 32771), (12, 131072), (18, 8200)])
+def test_clusters_exchange_their_best_after_all_of_them_have_started(rows, vocab):
+    """Launches back to back, each starting under the tail of the one before it: the maximum moves through the slices of a row's CTAs, so a
+    store into a CTA that has not begun, or a read before it, would give the token of an earlier launch."""
+    x = torch.randn(rows, vocab, generator=torch.Generator().manual_seed(vocab)).cuda()
+    at = [(i * vocab // 24 + 5 * i) % vocab for i in range(24)]
+    inputs = []
+    for a in at:
+        y = x.clone()
+        y[:, a] = 200.0
+        inputs.append(y)
+    greedy = [K.sample_full(y, temperature=0.0) for y in inputs]
+    drawn = [K.sample_full(y, temperature=0.8, top_p=0.9, seed=1) for y in inputs]
+    for a, t, u in zip(at, greedy, drawn):
+        assert (t == a).all() and (u == a).all()

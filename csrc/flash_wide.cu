@@ -12,6 +12,8 @@
 //              in TMEM only when the maximum has grown by 2^8; the 64 score columns are overwritten by hi (32 columns of packed pairs) and
 //              lo (32 columns);
 //   O += P·V   eight MMAs per tile, A from TMEM.
+// Slots that no query of the CTA sees (behind the last key, before the first one) may hold anything: their scores are masked, and the softmax
+// warps clear their value rows in shared memory, because a weight of zero times a NaN is a NaN.
 // Bound: per tile 64 · D + 2 · 64 · Dv MACs of a row against 64 exponentials; at D 192, Dv 128 the tensor work is 900 cycles, the
 // softmax warps need about as many.  2048 tokens, 16 heads, D 192, Dv 128, window 1024 on one B200: 41 us; attn_rows_kernel 1173 us
 // (fp32 FMAs from shared memory).
@@ -169,7 +171,17 @@ flash_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     const int slot = start + q0 + r;                       // cache slot (= causal limit) of this query
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     const int lo_row = first_seen(slot), lo_warp = first_seen(start + q0 + quarter * 32 + 31);     // the largest bound of the warp
+    const int lo_cta = first_seen(start + q0), hi_cta = start + q_hi;
     float m_ref = -INFINITY, l_run = 0.f;
+    // rows [r0, r1) of a value tile (the swizzle moves 16-byte pieces within a row), the four warps together
+    auto zero_rows = [&](uint32_t tile, int r0, int r1) {
+      r0 = max(r0, 0);
+      r1 = min(r1, FW_BN);
+      for (int i = r0 * 8 + quarter * 32 + lane; i < r1 * 8; i += 128)
+#pragma unroll
+        for (int c = 0; c < VC; ++c)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(tile + c * FW_KV_CHUNK + i * 16), "r"(0) : "memory");
+    };
 
     for (int j = 0; j < n_tiles; ++j) {
       const int key0 = (first_tile + j) * FW_BN;
@@ -231,6 +243,12 @@ flash_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       split(v1, 16);
       tc::tmem_st_wait();
       l_run += psum0 + psum1;
+      if (key0 < lo_cta || key0 + FW_BN - 1 > hi_cta) {          // (uniform) the first or the last tile: slots that no query of the CTA sees
+        tc::mbar_wait(v_full(j & 1), (j >> 1) & 1);
+        zero_rows(sV(j & 1), 0, lo_cta - key0);
+        zero_rows(sV(j & 1), hi_cta + 1 - key0, FW_BN);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");         // before the product that reads them
+      }
       // at most one phase of p_full may be outstanding: P·V_{j-1} complete proves that the MMA warp consumed phase j-1 (flash_prefill.cu)
       if (j > 0) tc::mbar_wait(o_full, (j - 1) & 1);
       tc::fence_before_sync();

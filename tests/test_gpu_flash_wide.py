@@ -83,3 +83,37 @@ def test_probabilities_keep_more_than_one_bfloat16():
     got = SK.attn_windowed(q.view(S, D).cuda(), k.transpose(1, 2).contiguous().cuda(), v.transpose(1, 2).contiguous().cuda(),
                            torch.zeros(1, dtype=torch.int32, device="cuda"), None, 1, S, 1, 1, D, 128, S, D, 128, 0, 1.0)
     assert abs(float(got[1, 0]) - want) <= 2 ** -6 * want   # one bfloat16 would give 0 or 2^-9, off by all of it
+
+
+@pytest.mark.parametrize("D,Dv,B,S,start,T,H,G,window,chunk,token_major", [
+    (192, 128, 1, 130, 0, 200, 2, 2, 0, 0, True), (192, 64, 2, 2, 126, 260, 4, 2, 0, 0, False), (128, 128, 2, 64, 0, 65, 4, 1, 0, 0, False),
+    (128, 64, 1, 65, 70, 300, 2, 1, 7, 0, False), (64, 128, 3, 63, 0, 64, 3, 3, 0, 50, True), (64, 64, 1, 100, 3, 500, 2, 2, 64, 0, False),
+    (256, 128, 1, 200, 57, 320, 2, 1, 0, 64, False), (256, 64, 2, 31, 0, 96, 2, 2, 0, 0, True)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_slots_without_a_key_may_hold_anything(D, Dv, B, S, start, T, H, G, window, chunk, token_major, bad):
+    """Behind the last key, before a row's first one, and before the first key that a window or chunk of the first tile reaches (64 slots of
+    the tile at most): nothing of it reaches a result, which is bit for bit that of a clean cache."""
+    g = torch.Generator().manual_seed(D + S)
+    bf = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16)              # noqa: E731
+    q, k, v = bf(B, S, H, D).cuda(), bf(B, T, G, D).cuda(), bf(B, T, G, Dv).cuda()
+    pads = torch.tensor([2 + b for b in range(B)], dtype=torch.int32)
+    lo = pads.clone()                                       # first key that any query of the row sees
+    if window:
+        lo = torch.maximum(lo, torch.tensor(start - window + 1))
+    if chunk:
+        lo = torch.where(torch.tensor(start) >= pads, torch.maximum(lo, pads + (start - pads) // chunk * chunk), lo)
+    lens = torch.tensor([start], dtype=torch.int32, device="cuda")
+
+    def attend(k, v):
+        layout = {}
+        if token_major:
+            layout = dict(T_cap=T, ldk=G * D, ldv=G * Dv, strides=(T * G * D, D, T * G * Dv, Dv))
+        else:
+            k, v = k.transpose(1, 2).contiguous(), v.transpose(1, 2).contiguous()
+        return SK.attn_masked(q.reshape(B * S, H * D).contiguous(), k, v, lens, pads.cuda(), B, S, H, G, D, Dv, D ** -0.5, window=window, chunk=chunk,
+                              **layout)
+    clean = attend(k, v)
+    slot = torch.arange(T)[None, :]
+    dead = ((slot < lo[:, None]) | (slot >= start + S)).cuda()[:, :, None, None]
+    got = attend(torch.where(dead, bad, k), torch.where(dead, bad, v))
+    assert bool(torch.isfinite(clean).all()) and torch.equal(got, clean)

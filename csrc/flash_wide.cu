@@ -260,8 +260,9 @@ flash_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       tc::fence_after_sync();
     }
     const bool row_on = q0 + r < p.S;
+    const bool seen = !(l_run == 0.f);                       // (a sum that is NaN belongs to a query with a NaN or an infinite score: it stays NaN)
     float inv = 0.f;                                         // a query that sees nothing: its row is zero
-    if (l_run > 0.f) inv = 1.0f / (l_run + (p.sink ? exp2f((p.sink_logit ? p.sink_logit[h] : 0.f) * 1.4426950408889634f - m_ref) : 0.f));
+    if (seen) inv = 1.0f / (l_run + (p.sink ? exp2f((p.sink_logit ? p.sink_logit[h] : 0.f) * 1.4426950408889634f - m_ref) : 0.f));
     if (p.gate != nullptr && row_on) inv *= 1.0f / (1.0f + __expf(-p.gate[(size_t)(b * p.S + q0 + r) * p.ldg + h]));
     uint4* dst = reinterpret_cast<uint4*>(p.out + ((size_t)(b * p.S + q0 + r) * p.H + h) * (VC * 64));
 #pragma unroll 1
@@ -277,7 +278,7 @@ flash_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         uint32_t w[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          w[e] = l_run > 0.f ? pack_bf16(__uint_as_float(o[8 * i + 2 * e]) * inv, __uint_as_float(o[8 * i + 2 * e + 1]) * inv) : 0u;
+          w[e] = seen ? pack_bf16(__uint_as_float(o[8 * i + 2 * e]) * inv, __uint_as_float(o[8 * i + 2 * e + 1]) * inv) : 0u;
         dst[c * 4 + i] = make_uint4(w[0], w[1], w[2], w[3]);
       }
     }

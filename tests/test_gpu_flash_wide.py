@@ -117,3 +117,24 @@ def test_slots_without_a_key_may_hold_anything(D, Dv, B, S, start, T, H, G, wind
     dead = ((slot < lo[:, None]) | (slot >= start + S)).cuda()[:, :, None, None]
     got = attend(torch.where(dead, bad, k), torch.where(dead, bad, v))
     assert bool(torch.isfinite(clean).all()) and torch.equal(got, clean)
+
+
+@pytest.mark.parametrize("D,Dv", [(64, 64), (128, 128), (192, 128), (256, 64)])
+def test_a_nan_stays_visible(D, Dv):
+    """A NaN or an infinite score is in the results of its own query and of no other; a query that sees no key stays zero."""
+    B, S, H, T = 1, 150, 2, 150
+    g = torch.Generator().manual_seed(D)
+    q, k, v = (torch.randn(S, H, d, generator=g).to(torch.bfloat16).cuda() for d in (D, D, Dv))
+    pads, lens = torch.tensor([3], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def attend(q):
+        return SK.attn_masked(q.reshape(S, H * D), k, v, lens, pads, B, S, H, H, D, Dv, D ** -0.5, T_cap=T, ldk=H * D, ldv=H * Dv,
+                              strides=(T * H * D, D, T * H * Dv, Dv)).view(S, H, Dv)
+    clean = attend(q)
+    q[40, 1, 5] = float("nan")
+    q[77, 0] = 3e38 * torch.sign(k[60, 0].float()).to(torch.bfloat16)              # its score with key 60 is +inf
+    got = attend(q)
+    assert bool(torch.isnan(got[40, 1]).all()) and bool(torch.isnan(got[77, 0]).all())
+    same = torch.ones(S, H, dtype=torch.bool)
+    same[40, 1] = same[77, 0] = False
+    assert torch.equal(got[same.cuda()], clean[same.cuda()]) and bool((clean[:3] == 0).all())

@@ -17,10 +17,9 @@
 // Bound: per tile 64 · D + 2 · 64 · Dv MACs of a row against 64 exponentials; at D 192, Dv 128 the tensor work is 900 cycles, the
 // softmax warps need about as many.  2048 tokens, 16 heads, D 192, Dv 128, window 1024 on one B200: 41 us; attn_rows_kernel 1173 us
 // (fp32 FMAs from shared memory).
-#include <stdlib.h>
-
 #include "flash_wide.cuh"
 #include "jllama_b200.h"
+#include "seq_types.cuh"
 #include "tcgen05.cuh"
 
 namespace jl {
@@ -303,9 +302,7 @@ bool flash_wide_takes(int S, int D, int Dv, int T_cap, int ldk, int ldv, long lo
                       const void* q, const void* k, const void* v, const void* out) {
   // TMA: 16-byte bases and strides; the tensor maps of a tile of 64 keys want a value row that is not shared with other channels
   auto stride_ok = [](long long s) { return s > 0 && s % 8 == 0; };
-  const char* e = getenv("JLLAMA_HYBRID_TC");
-  if (e && e[0] == '0') return false;                        // the exact SIMT kernels were asked for
-  return S > 1 && T_cap >= 1 && D % 64 == 0 && D <= 256 && (Dv == 64 || Dv == 128) && ldk % 8 == 0 && ldv % 8 == 0 && stride_ok(k_bs) &&
+  return hybrid_tensor_cores() && S > 1 && T_cap >= 1 && D % 64 == 0 && D <= 256 && (Dv == 64 || Dv == 128) && ldk % 8 == 0 && ldv % 8 == 0 && stride_ok(k_bs) &&
          stride_ok(k_hs) && stride_ok(v_bs) && stride_ok(v_hs) && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) == 0;
 }
 

@@ -273,13 +273,14 @@ __global__ void __launch_bounds__(256) linear_tiled_kernel(const T* __restrict__
 
 template <typename T, typename OutT>
 static int launch_linear(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0,
-                         float p1, cudaStream_t st, LinearGroup g = LinearGroup{0, 0, 0, 1, nullptr, nullptr, nullptr}, int nbatch = 1) {
+                         float p1, cudaStream_t st, bool tensor_cores, LinearGroup g = LinearGroup{0, 0, 0, 1, nullptr, nullptr, nullptr},
+                         int nbatch = 1) {
   if (M <= LR_MAXM && g.tile_group == nullptr) {
     constexpr int VN = Vec<T>::N;
     const int vec_ok = (K % VN == 0) && (ldx % VN == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) &&
                        (g.x_bs % VN == 0) && (g.w_bs % VN == 0);
     if constexpr (sizeof(T) == 2) {
-      if (vec_ok && M > 4 && (long)((N + 15) / 16) * nbatch >= 96) {
+      if (tensor_cores && vec_ok && M > 4 && (long)((N + 15) / 16) * nbatch >= 96) {
         lm_launch<OutT>((const T*)x, ldx, (const T*)w, (OutT*)out, ldo, M, N, K, act, p0, p1, st, g, nbatch);
         return cudaGetLastError() == cudaSuccess ? JL_OK : JL_ERR_CUDA;
       }
@@ -294,7 +295,7 @@ static int launch_linear(const void* x, int ldx, const void* w, void* out, int l
 #undef JL_LR
   } else {
     if constexpr (sizeof(T) == 4 && sizeof(OutT) == 4) {
-      if (linear_f32_takes(M, K, ldx, g, x, w))
+      if (tensor_cores && linear_f32_takes(M, K, ldx, g, x, w))
         return linear_f32_launch((const float*)x, ldx, (const float*)w, (float*)out, ldo, M, N, K, act, p0, p1, st, g, nbatch) == cudaSuccess
                    ? JL_OK : JL_ERR_CUDA;
     }
@@ -308,20 +309,30 @@ static int launch_linear(const void* x, int ldx, const void* w, void* out, int l
 
 using namespace jl;
 
-extern "C" JL_API int jl_linear_any(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act,
-                                    float p0, float p1, int dtype, int out_f32, void* stream) {
+static int linear_any(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1, int dtype,
+                      int out_f32, void* stream, bool tensor_cores) {
   JL_CHECK_ARG(M >= 1 && N >= 1 && K >= 1 && ldx >= K && ldo >= N, "jl_linear_any: bad shape M=%d N=%d K=%d ldx=%d ldo=%d", M, N,
                K, ldx, ldo);
   JL_CHECK_ARG(act >= 0 && act <= ACT_LAST, "jl_linear_any: bad activation %d", act);
   cudaStream_t st = (cudaStream_t)stream;
   int rc;
   if (dtype == DT_BF16)
-    rc = out_f32 ? launch_linear<__nv_bfloat16, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st)
-                 : launch_linear<__nv_bfloat16, __nv_bfloat16>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st);
+    rc = out_f32 ? launch_linear<__nv_bfloat16, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tensor_cores)
+                 : launch_linear<__nv_bfloat16, __nv_bfloat16>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tensor_cores);
   else
-    rc = launch_linear<float, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st);
+    rc = launch_linear<float, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tensor_cores);
   if (rc != JL_OK) return cuda_fail(cudaGetLastError(), "jl_linear_any launch");
   return JL_OK;
+}
+
+extern "C" JL_API int jl_linear_any(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act,
+                                    float p0, float p1, int dtype, int out_f32, void* stream) {
+  return linear_any(x, ldx, w, out, ldo, M, N, K, act, p0, p1, dtype, out_f32, stream, hybrid_tensor_cores());
+}
+
+extern "C" JL_API int jl_linear_exact(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act,
+                                      float p0, float p1, int dtype, int out_f32, void* stream) {
+  return linear_any(x, ldx, w, out, ldo, M, N, K, act, p0, p1, dtype, out_f32, stream, false);
 }
 
 extern "C" JL_API int jl_linear_tile_rows(void) { return LT_BM; }
@@ -337,12 +348,13 @@ extern "C" JL_API int jl_linear_grouped(const void* x, int ldx, long long x_bs, 
   JL_CHECK_ARG(nbatch <= 65535, "jl_linear_grouped: %d batches above the grid limit", nbatch);
   cudaStream_t st = (cudaStream_t)stream;
   const LinearGroup g{x_bs, w_bs, o_bs, x_div, w_index, tile_group, row_src};
+  const bool tc = hybrid_tensor_cores();
   int rc;
   if (dtype == DT_BF16)
-    rc = out_f32 ? launch_linear<__nv_bfloat16, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, g, nbatch)
-                 : launch_linear<__nv_bfloat16, __nv_bfloat16>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, g, nbatch);
+    rc = out_f32 ? launch_linear<__nv_bfloat16, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tc, g, nbatch)
+                 : launch_linear<__nv_bfloat16, __nv_bfloat16>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tc, g, nbatch);
   else
-    rc = launch_linear<float, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, g, nbatch);
+    rc = launch_linear<float, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tc, g, nbatch);
   if (rc != JL_OK) return cuda_fail(cudaGetLastError(), "jl_linear_grouped launch");
   return JL_OK;
 }

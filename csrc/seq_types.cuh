@@ -4,10 +4,18 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stdlib.h>
+#include <string.h>
 
 #include "common.cuh"
 
 namespace jl {
+
+// JLLAMA_HYBRID_TC=0 keeps the hybrid family on the exact SIMT kernels (A/B and debugging); asked at every call
+inline bool hybrid_tensor_cores() {
+  const char* e = getenv("JLLAMA_HYBRID_TC");
+  return e == nullptr || strcmp(e, "0") != 0;
+}
 
 enum { DT_BF16 = 0, DT_F32 = 1 };
 // epilogue / activation codes shared by the generic linears and jl_act_cast

@@ -278,6 +278,9 @@ int jl_act_inplace(void* data, int ld, int M, int N, int act, float p0, float p1
 /* out[:, 0:N] (pitch ldo; fp32 if out_f32 else dtype) = act(x W^T): x [M, K] (pitch ldx), W [N, K]; any M, N, K. */
 int jl_linear_any(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1,
                   int dtype, int out_f32, void* stream);
+/* The same on the SIMT kernels whatever the sizes (fp32 FMAs in order of k within a thread): what JLLAMA_HYBRID_TC=0 gives every call. */
+int jl_linear_exact(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1,
+                    int dtype, int out_f32, void* stream);
 /* Rotary embedding (first `rot` channels, interleaved pairs), optional unit-RMS per head, cache append.  y fp32 [B*S, ldy] holds
  * q at q_off ([H*D]), k at k_off ([G*D]; < 0: queries only), v at v_off ([G*Dv]); caches [B][G][T_cap][D|Dv] of dtype. */
 int jl_attn_prep(const float* y, int ldy, int q_off, int k_off, int v_off, void* q_out, void* k_cache, void* v_cache,

@@ -115,8 +115,9 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
     """act(x Wᵀ): x [M, K] and W [N, K] of one dtype (bf16 or fp32) → fp32 (or the operand dtype) [M, N].
 
     bfloat16 with more than 8 rows and 16-byte pitches runs the tcgen05 GEMM (fp32 accumulate; the activation is
-    then an in-place pass over the stored result); 8 rows or fewer the weight-streaming kernel; everything else — true
-    float32 in particular — the exact tiled SIMT kernel."""
+    then an in-place pass over the stored result), float32 with more than 8 rows the three-part tcgen05 kernel (csrc/linear_f32.cu),
+    8 rows or fewer a weight-streaming kernel (bfloat16 from 5 rows on: mma.sync); everything else — and every size with
+    `tensor_cores=False` or JLLAMA_HYBRID_TC=0 — the exact SIMT kernels."""
     if not x.is_cuda:
         raise ValueError("linear: CUDA tensors only")
     _need(w, x.dtype, "w")
@@ -140,9 +141,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
             _lib.check(L.jl_act_inplace(out.data_ptr(), out.stride(0), M, N, act, float(p0), float(p1),
                                         dtype_code(out.dtype), _stream()), "jl_act_inplace")
         return out
-    _lib.check(L.jl_linear_any(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), M, N, K, act,
-                               float(p0), float(p1), dtype_code(x.dtype), int(out.dtype == torch.float32), _stream()),
-               "jl_linear_any")
+    call = L.jl_linear_any if use_tc else L.jl_linear_exact
+    _lib.check(call(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), M, N, K, act,
+                    float(p0), float(p1), dtype_code(x.dtype), int(out.dtype == torch.float32), _stream()),
+               "jl_linear_any" if use_tc else "jl_linear_exact")
     return out
 
 

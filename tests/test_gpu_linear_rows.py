@@ -22,7 +22,7 @@ def check(got, x, w, act=lambda z: z):
 def test_decode_rows_bfloat16(M, N, K):
     g = torch.Generator().manual_seed(N + K + M)
     x, w = torch.randn(M, K, generator=g).bfloat16().cuda(), torch.randn(N, K, generator=g).bfloat16().cuda()
-    check(SK.linear(x, w, tensor_cores=False), x, w)
+    check(SK.linear(x, w), x, w)
     check(SK.linear(x, w, act=SK.ACT_RELU, out_f32=False), x, w, torch.relu)
 
 
@@ -110,3 +110,28 @@ def test_prompt_rows_bfloat16_on_cta_pairs(M, N, K):
     got = SK.linear(x, w, out_f32=False, out=room[:M * N].view(M, N))
     assert bool(((got.double() - ref).abs() <= 2.0 ** -17 * scale + 2.0 ** -8 * ref.abs() + 1e-30).all())
     assert bool((room[M * N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("how", ["argument", "environment"])
+def test_exact_kernels_are_still_there(how, monkeypatch):
+    """`tensor_cores=False` and JLLAMA_HYBRID_TC=0: the SIMT kernels, shown bit for bit by the same rows in calls that no tensor-core kernel
+    takes (four rows at a time in bfloat16, rows off the 16-byte boundary in float32).  The tensor-core kernels order their sums in another way."""
+    g = torch.Generator().manual_seed(8)
+    x, w = torch.randn(8, 2048, generator=g).bfloat16().cuda(), torch.randn(2048, 2048, generator=g).bfloat16().cuda()
+    exact = torch.cat([SK.linear(x[:4], w), SK.linear(x[4:], w)])
+    xf, wf = torch.randn(100, 2048, generator=g).cuda(), torch.randn(500, 2048, generator=g).cuda()
+    odd = torch.empty(100, 2049, device="cuda")
+    odd[:, :2048] = xf
+    exact_f = SK.linear(odd[:, :2048], wf)
+    fast, fast_f = SK.linear(x, w), SK.linear(xf, wf)
+    kw = {}
+    if how == "argument":
+        kw = dict(tensor_cores=False)
+    else:
+        monkeypatch.setenv("JLLAMA_HYBRID_TC", "0")
+        out = torch.empty(8, 2048, device="cuda")
+        assert torch.equal(SK.linear_batched(x, w[None], out, nbatch=1, rows=8, x_bs=0, o_bs=0), exact)
+        out = torch.empty(100, 500, device="cuda")
+        assert torch.equal(SK.linear_batched(xf, wf[None], out, nbatch=1, rows=100, x_bs=0, o_bs=0), exact_f)
+    assert torch.equal(SK.linear(x, w, **kw), exact) and torch.equal(SK.linear(xf, wf, **kw), exact_f)
+    assert not torch.equal(fast, exact) and not torch.equal(fast_f, exact_f)

@@ -585,8 +585,10 @@ static int launch_scan(GlaParams p, const void* a2, const void* a2_bias, float* 
     p.P = gla_lanes(D);
     const int slots = H * (p.P * GT_DP + ((Dv + 3) & ~3));
     const dim3 pgrid((B * S + GP_TOK - 1) / GP_TOK, (slots + GP_THREADS - 1) / GP_THREADS);
-    JL_CHECK_ARG(GP_TOK * R * sizeof(float) <= 48 * 1024, "jl_gla_scan: rank %d does not fit the staging buffer", R);
-    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(gla_prep_kernel<T>, pgrid, dim3(GP_THREADS), GP_TOK * R * sizeof(float), st, p, (const T*)a2, (const T*)a2_bias, ws));
+    const size_t zsm = (size_t)GP_TOK * R * sizeof(float);     // (the check above leaves at most 200 KB)
+    if (zsm > 48 * 1024)
+      JL_DISPATCH_DTYPE(dtype, JL_CUDA(cudaFuncSetAttribute(gla_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm)));
+    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(gla_prep_kernel<T>, pgrid, dim3(GP_THREADS), zsm, st, p, (const T*)a2, (const T*)a2_bias, ws));
     JL_CUDA(cudaGetLastError());
     switch (p.P) {
       case 1: return launch_stream<1>(p, ws, st);

@@ -39,3 +39,23 @@ def test_projected_decays_over_a_prompt(B, S, H, D, Dv):
     tol = 2.0 ** -23 * (S + D)
     assert float((got - want).abs().max()) <= tol * float(want.abs().max())
     assert float((got_state.double().cpu() - end).abs().max()) <= tol * float(end.abs().max())
+
+
+@pytest.mark.parametrize("R", [1536, 1537, 4000, 5900])
+def test_wide_decay_projections(R):
+    """Ranks whose rows of eight tokens outgrow the default shared memory (48 KB: 1536), up to what the staging check of the entry point
+    leaves; the decays of a rank of thousands are summed in fp32 (2^-23 · R of their scale), everything after them as above."""
+    B, S, H, D, Dv = 1, 21, 1, 16, 8
+    g = torch.Generator().manual_seed(R)
+    y = torch.randn(S, 2 * D + Dv + R, generator=g)
+    a2, bias = torch.randn(D, R, generator=g) * R ** -0.5, torch.randn(D, generator=g)
+    alpha = torch.sigmoid(y[:, -R:].double() @ a2.double().T + bias.double()).pow(0.25)
+    state, want = torch.zeros(D, Dv, dtype=torch.float64), []
+    for t in range(S):
+        state = alpha[t][:, None] * state + y[t, D:2 * D].double()[:, None] * y[t, 2 * D:2 * D + Dv].double()
+        want.append(state.T @ y[t, :D].double())
+    want = torch.stack(want)
+    end = torch.zeros(1, 1, D, Dv, device="cuda")
+    got = SK.gla_scan(y.cuda(), 0, D, 2 * D, 2 * D + Dv, a2.cuda(), bias.cuda(), end, None, None, B, S, H, D, Dv, 1.0, 4.0).double().cpu()
+    assert float((got - want).abs().max()) <= 2.0 ** -23 * (R + S + D) * float(want.abs().max())
+    assert float((end.double().cpu()[0, 0] - state).abs().max()) <= 2.0 ** -23 * (R + S + D) * float(state.abs().max())

@@ -1,13 +1,15 @@
 // float32 linears of more than a few rows on tcgen05 tensor cores, with the accuracy of fp32 FMAs.
 //
-// A float32 number is the sum of three bfloat16 numbers, x = x1 + x2 + x3 exactly: x1 its upper 16 bits, x2 the upper 16 bits of x - x1,
-// x3 the rest (8 significant bits each, cut off rather than rounded).  Six of the nine products reach 2^-24 of x·w:
+// A float32 number is the sum of three bfloat16 numbers, x = x1 + x2 + x3 exactly (Henry, Tang, Heinecke, "Leveraging the bfloat16 Artificial
+// Intelligence Datatype For Higher-Precision Computations", 2019): x1 is x rounded to nearest, x2 the rest rounded to nearest, |x2| <= 2^-8 |x|,
+// x3 what then remains, |x3| <= 2^-17 |x|.  Six of the nine products leave out less than 2^-24 of x·w, of either sign:
 //     x1 w1 + (x1 w2 + x2 w1) + (x1 w3 + x2 w2 + x3 w1),
-// each exact in the tensor core's fp32 sums.  The tensor core cuts off when it adds (measured: 6e-8 of a sum of 64 products, 2e-6 of one of
+// each exact in the tensor core's fp32 sums.  (Parts that are cut off instead of rounded leave out up to 2^-21, always towards zero.)  The tensor core cuts off when it adds (measured: 6e-8 of a sum of 64 products, 2e-6 of one of
 // 2048), so a sum runs over 64 k only, small products first, and the sums of 64 meet in registers in rounded fp32 additions.
 // Error against float64 (2-norm, normal operands), FMA kernel -> this one: K 256 2.8e-7 -> 1.3e-7, 1024 5.7e-7 -> 1.4e-7, 2048 8.1e-7 -> 1.6e-7,
 // 5464 1.3e-6 -> 1.6e-7.
-// An output that comes out infinite or NaN is formed again with FMAs in order of k: an infinite operand has no such parts.
+// An output that comes out infinite or NaN is formed again with FMAs in order of k: an infinite operand has no such parts, and a finite one
+// above the largest bfloat16 number rounds to infinity.
 //
 //   * 8 producer warps read float32 tiles (128 features and BN rows of 64 k), cut them and write the six bfloat16 tiles in the
 //     128-byte-swizzled K-major layout; the next tile's loads are in flight meanwhile;
@@ -45,20 +47,18 @@ struct LinearF32 {
 // eight consecutive floats -> the 16 bytes of each part
 __device__ __forceinline__ void lf_split8(const float4& a, const float4& b, uint4 (&part)[3]) {
   const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-  uint32_t h[3][8];
+  uint32_t h[3][4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t b1 = __float_as_uint(v[i]) & 0xffff0000u;
-    const float r = v[i] - __uint_as_float(b1);
-    const uint32_t b2 = __float_as_uint(r) & 0xffff0000u;
-    h[0][i] = b1;
-    h[1][i] = b2;
-    h[2][i] = __float_as_uint(r - __uint_as_float(b2));              // at most 8 significant bits: its lower half is zero
+  for (int i = 0; i < 4; ++i) {
+    float r0 = v[2 * i], r1 = v[2 * i + 1];
+    h[0][i] = pack_bf16(r0, r1);
+    r0 -= bf16_lo(h[0][i]);
+    r1 -= bf16_hi(h[0][i]);
+    h[1][i] = pack_bf16(r0, r1);
+    h[2][i] = pack_bf16(r0 - bf16_lo(h[1][i]), r1 - bf16_hi(h[1][i]));            // at most 8 significant bits: exact
   }
 #pragma unroll
-  for (int p = 0; p < 3; ++p)
-    part[p] = make_uint4(__byte_perm(h[p][0], h[p][1], 0x7632), __byte_perm(h[p][2], h[p][3], 0x7632),
-                         __byte_perm(h[p][4], h[p][5], 0x7632), __byte_perm(h[p][6], h[p][7], 0x7632));
+  for (int p = 0; p < 3; ++p) part[p] = make_uint4(h[p][0], h[p][1], h[p][2], h[p][3]);
 }
 
 template <int BN>

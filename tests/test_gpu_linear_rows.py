@@ -135,3 +135,18 @@ def test_exact_kernels_are_still_there(how, monkeypatch):
         assert torch.equal(SK.linear_batched(xf, wf[None], out, nbatch=1, rows=100, x_bs=0, o_bs=0), exact_f)
     assert torch.equal(SK.linear(x, w, **kw), exact) and torch.equal(SK.linear(xf, wf, **kw), exact_f)
     assert not torch.equal(fast, exact) and not torch.equal(fast_f, exact_f)
+
+
+@pytest.mark.parametrize("M,N,K", [(20, 64, 256), (100, 500, 2048)])
+def test_float32_of_one_sign_is_not_biased(M, N, K):
+    """Operands of one sign whose lower parts are as large as they get: products left out would all pull the same way.  Rounded parts leave out
+    less than 2^-24 of a product; the tensor core cuts off some thirty times per 64 products, most of it in the last four (2^-23 of the sum
+    each at most), and the sums of 64 round once each: 2^-21 holds with room, parts cut off instead of rounded miss it (2^-21 alone)."""
+    worst = 1 + 2.0 ** -7 - 2.0 ** -23
+    x, w = torch.full((M, K), worst, device="cuda"), torch.full((N, K), worst, device="cuda")
+    ref = x.double() @ w.double().T
+    assert float(((SK.linear(x, w).double() - ref) / ref).abs().max()) < 2.0 ** -21
+    g = torch.Generator().manual_seed(K)
+    x, w = torch.rand(M, K, generator=g).cuda(), torch.rand(N, K, generator=g).cuda()
+    ref = x.double() @ w.double().T
+    assert float(((SK.linear(x, w).double() - ref) / ref).mean().abs()) < 2.0 ** -22

@@ -24,6 +24,8 @@
 // /root/reference/jax_llama/model.py:119-150 (wq/wk/wv/wo) and :311-338 (w1/w2/w3).
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "jllama_b200.h"
 #include "tcgen05.cuh"
 
@@ -37,6 +39,7 @@ constexpr uint32_t G2_A_BYTES = G2_BM * G2_BK * 2;                 // 16 KB
 constexpr uint32_t G2_B_BYTES = (G2_BN / 2) * G2_BK * 2;           // 16 KB
 constexpr uint32_t G2_STAGE_BYTES = G2_A_BYTES + G2_B_BYTES;
 constexpr uint32_t G2_EPI_BYTES = 4 * 32 * 64 * 2;                 // per CTA: 4 warps x [32 rows][64 cols] bf16 (fp32: [32][32], twice)
+constexpr int G2_MAX_STAGES = 6;
 constexpr uint32_t G2_PEER_MASK = 0xFEFFFFFFu;                     // shared::cluster address of the same offset in CTA 0
 
 enum { G2_PLAIN = 0, G2_RESIDUAL = 1, G2_SWIGLU = 2, G2_F32 = 3 };
@@ -322,19 +325,55 @@ int jl::gemm_2cta_f32(const void* x, const void* w, void* out, int M, int N, int
   return gemm_2cta(x, w, nullptr, out, M, N, K, G2_F32, num_sms, stream);
 }
 
+using Gemm2Kernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const Gemm2Params);
+
+// The tile loop is persistent, so every cluster of the grid must be resident at once: a pair that only starts when another one has finished
+// doubles the run time.  Not every TPC can host a 2-CTA cluster of this size on every part (measured here: fewer than num_sms / 2), so the
+// runtime is asked how many fit, once per device, epilogue and ring depth (a short K has a small ring, of which more may fit).
+static int g2_resident_pairs(Gemm2Kernel kern, int mode, int stages, size_t smem, int num_sms) {
+  constexpr int DEVICES = 16;
+  static std::atomic<int> known[DEVICES][4][G2_MAX_STAGES + 1];
+  int dev = 0, n = 0;
+  const bool cached = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < DEVICES;
+  if (cached) n = known[dev][mode][stages].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(G2_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3((num_sms / 2) * 2);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = num_sms / 2; }
+    if (const char* e = getenv("JLLAMA_GEMM_PAIRS")) { const int v = atoi(e); if (v >= 1) n = v; }
+    if (cached) known[dev][mode][stages].store(n, std::memory_order_relaxed);
+  }
+  return n < num_sms / 2 ? n : num_sms / 2;
+}
+
 static int gemm_2cta(const void* x, const void* w, const void* residual, void* out, int M, int N, int K, int mode, int num_sms, void* stream) {
   const bool ragged = mode == G2_PLAIN || mode == G2_F32;
   if (M < 256 || N % (ragged ? 8 : G2_BN) != 0 || N < G2_BN || K % (ragged ? 8 : G2_BK) != 0 || K < G2_BK) return JL_ERR_UNSUPPORTED;
   if (mode == G2_RESIDUAL && residual == nullptr) return JL_ERR_UNSUPPORTED;
+  if (num_sms <= 0) num_sms = 148;
+  const int num_kb = (K + G2_BK - 1) / G2_BK;
+  int stages = (int)((200 * 1024) / G2_STAGE_BYTES);
+  if (stages > G2_MAX_STAGES) stages = G2_MAX_STAGES;
+  if (stages > num_kb * 2) stages = num_kb * 2 < 2 ? 2 : num_kb * 2;
+  const size_t smem = (size_t)stages * G2_STAGE_BYTES + g2_epi_bytes(mode) + 8 * (2 * stages + 4) + 16 + 1024;
+  const Gemm2Kernel kern =
+      mode == G2_F32 ? gemm2_kernel<G2_F32> : mode == G2_SWIGLU ? gemm2_kernel<G2_SWIGLU> : (mode == G2_RESIDUAL ? gemm2_kernel<G2_RESIDUAL> : gemm2_kernel<G2_PLAIN>);
+  JL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int pairs = g2_resident_pairs(kern, mode, stages, smem, num_sms);
   if (mode == G2_F32 || N % G2_BN != 0 || K % G2_BK != 0) {
     // A pair takes a 256 x 256 tile in about four fifths of the time in which a single CTA takes its 128 x 256 tile (2048 x 6160 x 2048, three
     // rounds of either: 45.6 against 57.3 us), but its tiles are twice as high: 600 x 6160 x 2048 is two rounds of pairs (27.6 us) and one
     // of single CTAs (23.2 us).
-    const int sms = num_sms > 0 ? num_sms : 148, cols = (N + G2_BN - 1) / G2_BN;
-    const int pair_rounds = ((M + 255) / 256 * cols + sms / 2 - 1) / (sms / 2), single_rounds = ((M + 127) / 128 * cols + sms - 1) / sms;
+    const int cols = (N + G2_BN - 1) / G2_BN;
+    const int pair_rounds = ((M + 255) / 256 * cols + pairs - 1) / pairs, single_rounds = ((M + 127) / 128 * cols + num_sms - 1) / num_sms;
     if (4 * pair_rounds > 5 * single_rounds) return JL_ERR_UNSUPPORTED;
   }
-  if (num_sms <= 0) num_sms = 148;
   const int odim = mode == G2_SWIGLU ? N / 2 : N;
   Gemm2Params p{};
   p.residual = (const __nv_bfloat16*)residual; p.M = M; p.N = N; p.K = K; p.ldo = odim;
@@ -346,38 +385,15 @@ static int gemm_2cta(const void* x, const void* w, const void* residual, void* o
   if ((rc = make_tmap_2d_bf16(&tb, w, N, K, K, G2_BN / 2))) return rc;
   rc = mode == G2_F32 ? make_tmap_2d_f32(&to, out, M, odim, odim, 32) : make_tmap_2d_bf16_plain(&to, out, M, odim, odim, mode == G2_SWIGLU ? 32 : 64, 32);
   if (rc) return rc;
-  int stages = (int)((200 * 1024) / G2_STAGE_BYTES);
-  if (stages > 6) stages = 6;
-  const int num_kb = (K + G2_BK - 1) / G2_BK;
-  if (stages > num_kb * 2) stages = num_kb * 2 < 2 ? 2 : num_kb * 2;
   p.stages = stages;
-  const size_t smem = (size_t)stages * G2_STAGE_BYTES + g2_epi_bytes(mode) + 8 * (2 * stages + 4) + 16 + 1024;
-  void (*kern)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const Gemm2Params) =
-      mode == G2_F32 ? gemm2_kernel<G2_F32> : mode == G2_SWIGLU ? gemm2_kernel<G2_SWIGLU> : (mode == G2_RESIDUAL ? gemm2_kernel<G2_RESIDUAL> : gemm2_kernel<G2_PLAIN>);
-  JL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(G2_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = (cudaStream_t)stream;
-  // The tile loop is persistent, so every cluster of the grid must be resident at once: a pair that only starts when
-  // another one has finished doubles the run time.  Not every TPC can host a 2-CTA cluster of this size on every part
-  // (measured here: fewer than num_sms / 2), so ask the runtime how many fit.
-  static int max_pairs[4] = {0, 0, 0, 0};
-  if (max_pairs[mode] == 0) {
-    cfg.gridDim = dim3((num_sms / 2) * 2);
-    cudaLaunchAttribute cattr[1];
-    cattr[0].id = cudaLaunchAttributeClusterDimension;
-    cattr[0].val.clusterDim.x = 2; cattr[0].val.clusterDim.y = 1; cattr[0].val.clusterDim.z = 1;
-    cfg.attrs = cattr; cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = num_sms / 2; }
-    if (const char* e = getenv("JLLAMA_GEMM_PAIRS")) { const int v = atoi(e); if (v >= 1) n = v; }
-    max_pairs[mode] = n < num_sms / 2 ? n : num_sms / 2;
-  }
   int grid = p.a_blocks * p.b_blocks * 2;
-  if (grid > 2 * max_pairs[mode]) grid = 2 * max_pairs[mode];
+  if (grid > 2 * pairs) grid = 2 * pairs;
   cfg.gridDim = dim3(grid);
-  g2_pairs_used = max_pairs[mode];
+  g2_pairs_used = pairs;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;

@@ -2,6 +2,9 @@
 
 Products of the operands are formed exactly or in fp32 and summed in fp32: with K terms an error of a few 2^-24 of Σ |x w| per level of the
 sum; 2^-20 Σ |x w| bounds every kernel here.  bfloat16 results add one rounding (2^-9)."""
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -150,3 +153,15 @@ def test_float32_of_one_sign_is_not_biased(M, N, K):
     x, w = torch.rand(M, K, generator=g).cuda(), torch.rand(N, K, generator=g).cuda()
     ref = x.double() @ w.double().T
     assert float(((SK.linear(x, w).double() - ref) / ref).mean().abs()) < 2.0 ** -22
+
+
+def test_a_short_k_first_does_not_set_the_number_of_resident_pairs():
+    """The persistent grid of the CTA-pair kernel is as wide as what fits at its own ring depth, whatever ran before it in the process."""
+    code = ("import sys, torch\n"
+            "from jax_llama_b200.ops import _lib, seq_kernels as SK\n"
+            "for K in map(int, sys.argv[1:]):\n"
+            "    SK.linear(torch.zeros(2048, K, dtype=torch.bfloat16, device='cuda'), torch.zeros(2048, K, dtype=torch.bfloat16, device='cuda'))\n"
+            "print(_lib.lib().jl_gemm_2cta_pairs())\n")
+    last = [subprocess.run([sys.executable, "-c", code, *ks], capture_output=True, text=True, timeout=120, check=True).stdout.split()[-1]
+            for ks in (["512"], ["64", "512"])]
+    assert last[0] == last[1] and int(last[0]) > 0

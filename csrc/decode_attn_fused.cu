@@ -36,6 +36,7 @@ struct FusedAttnParams {
   __nv_bfloat16* out;            // [B, nh·hd]
   int nkv, T, max_pos, splits;
   float scale_log2;
+  int vec;                       // o_part on 16-byte and out on 8-byte boundaries
 };
 
 // Shared tail of both kernels: s_o / s_ml hold the (m, l, o) triples of the CTA's NG independent streams.  Folds them,
@@ -96,6 +97,23 @@ __device__ __forceinline__ void df_fold_and_merge(const FusedAttnParams& p, floa
     s_l[g * 64 + sp] = __ldcg(p.ml_part + (bh * p.splits + sp) * 2 + 1);
   }
   __syncthreads();
+  if (!p.vec) {                                     // scratch or output off those boundaries: one column per thread
+    for (int idx = threadIdx.x; idx < G * HD; idx += (int)blockDim.x) {
+      const int g = idx / HD, d = idx - g * HD;
+      const size_t bh = (size_t)b * nh + kvh * G + g;
+      float M = -INFINITY;
+      for (int sp = 0; sp < active; ++sp) M = fmaxf(M, s_m[g * 64 + sp]);
+      const float Ms = M == -INFINITY ? 0.f : M;
+      float acc = 0.f, L = 0.f;
+      for (int sp = 0; sp < active; ++sp) {
+        const float w = exp2f(s_m[g * 64 + sp] - Ms);
+        if (w > 0.f) acc += w * __ldcg(p.o_part + (bh * p.splits + sp) * HD + d);
+        L += w * s_l[g * 64 + sp];
+      }
+      p.out[bh * HD + d] = __float2bfloat16(acc * (L > 0.f ? 1.f / L : 0.f));
+    }
+    return;
+  }
   // four columns per thread, the partial rows of 16 splits requested before the first is used (one memory round trip
   // for up to 16 splits: a loop with a remainder took one per remaining split, 15.2 us at 12 splits against 12.1 at 8)
   for (int idx = threadIdx.x; idx < G * (HD / 4); idx += (int)blockDim.x) {
@@ -656,6 +674,7 @@ extern "C" JL_API int jl_decode_attn_fused(const void* qkv, void* k_cache, void*
   p.out = (__nv_bfloat16*)out;
   p.nkv = nkv; p.T = T; p.max_pos = max_pos; p.splits = splits;
   p.scale_log2 = scale * 1.4426950408889634f;
+  p.vec = (uintptr_t)scratch % 16 == 0 && (uintptr_t)out % 8 == 0;
   auto s = (cudaStream_t)stream;
   cudaError_t e = cudaErrorInvalidValue;
   // The tensor-core kernel, but for one query head per kv head over a cache of at most 128 slots, where the ring and the

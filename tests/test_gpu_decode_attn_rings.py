@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from jax_llama_b200.models import reference as ref
-from jax_llama_b200.ops import kernels as K
+from jax_llama_b200.ops import _lib, kernels as K
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -45,3 +45,33 @@ def test_blocks_splits_and_cache_edges(B, nkv, G, hd, filled, T):
     for now, was in zip((gk, gv), before):                    # nothing but the new slot was written
         assert torch.equal(now[:, :, keep.to(DEV)].view(torch.int16), was[:, :, keep.to(DEV)].view(torch.int16))
     assert torch.equal(gv[:, :, filled].cpu(), qkv.view(B, nh + 2 * nkv, hd)[:, nh + nkv:]) and (scratch[-B * nkv:] == 0).all()
+
+
+@pytest.mark.parametrize("variant", [1, 2])
+@pytest.mark.parametrize("hd,G", [(128, 4), (64, 1)])
+@pytest.mark.parametrize("out_off,scratch_off", [(0, 0), (1, 0), (0, 1), (2, 3)])
+def test_buffers_at_any_element(hd, G, out_off, scratch_off, variant):
+    """The C entry takes an output and a scratch that start at any element; the merge uses wide accesses only where both allow it."""
+    B, nkv, T, filled = 2, 4, 2048, 2000
+    nh = nkv * G
+    g = torch.Generator().manual_seed(hd)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).to(DEV)
+    qkv, kc, vc = rnd(B, (nh + 2 * nkv) * hd), rnd(B, nkv, T, hd), rnd(B, nkv, T, hd)
+    cos, sin = (t.to(DEV) for t in ref.rope_cos_sin(hd, T, 500000.0))
+    clen, pad = torch.tensor([filled], dtype=torch.int32, device=DEV), torch.zeros(B, dtype=torch.int32, device=DEV)
+    splits, scratch = K.decode_attn_fused_plan(B, nh, nkv, hd, T, torch.device(DEV))
+    assert splits > 1
+    K.set_decode_attn_variant(variant)
+    try:
+        want = K.decode_attn_fused(qkv, kc.clone(), vc.clone(), cos, sin, clen, pad, nh, nkv, hd, splits, scratch)
+        room = torch.zeros(scratch.numel() + 4, dtype=scratch.dtype, device=DEV)[scratch_off:scratch_off + scratch.numel()]
+        out = torch.full((B * nh * hd + 8,), 7.0, dtype=torch.bfloat16, device=DEV)
+        got = out[out_off:out_off + B * nh * hd].view(B, nh * hd)
+        _lib.check(_lib.lib().jl_decode_attn_fused(qkv.data_ptr(), kc.data_ptr(), vc.data_ptr(), cos.data_ptr(), sin.data_ptr(), clen.data_ptr(),
+                                                   pad.data_ptr(), room.data_ptr(), got.data_ptr(), B, nh, nkv, hd, T, T, hd ** -0.5, splits,
+                                                   torch.cuda.current_stream().cuda_stream), "jl_decode_attn_fused")
+    finally:
+        K.set_decode_attn_variant(0)
+    # the sums of the two merges run in the same order; a contraction may differ in the last bit of fp32, so one bfloat16 step at most
+    torch.testing.assert_close(got.float(), want.float().view(B, nh * hd), rtol=2.0 ** -8, atol=2.0 ** -20)
+    assert (out[:out_off] == 7.0).all() and (out[out_off + B * nh * hd:] == 7.0).all()

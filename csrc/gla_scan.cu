@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(GS_THREADS, 3) gla_stream_kernel(GlaParams p, 
   constexpr int QKA = 3 * P * GT_PITCH;                                 // floats of q | k | alpha per token
   const int SF = QKA + cols;                                            // floats per token in a stage
   const int RF = gla_record_floats(P, p.Dv);
-  const bool vec = p.Dv % 4 == 0;
+  const bool vec = p.Dv % 4 == 0 && ((uintptr_t)(MODE == 0 ? p.state : p.cstate) & 15) == 0;      // rows of the state on 16-byte boundaries
   unsigned long long st[GT_DP / 2][GT_C];                               // pairs of channels
   const int d0 = part * GT_DP;
   float* sbase = MODE == 0 ? p.state + (((size_t)b * p.H + h) * p.D) * p.Dv

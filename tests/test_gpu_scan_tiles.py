@@ -59,3 +59,20 @@ def test_wide_decay_projections(R):
     got = SK.gla_scan(y.cuda(), 0, D, 2 * D, 2 * D + Dv, a2.cuda(), bias.cuda(), end, None, None, B, S, H, D, Dv, 1.0, 4.0).double().cpu()
     assert float((got - want).abs().max()) <= 2.0 ** -23 * (R + S + D) * float(want.abs().max())
     assert float((end.double().cpu()[0, 0] - state).abs().max()) <= 2.0 ** -23 * (R + S + D) * float(state.abs().max())
+
+
+@pytest.mark.parametrize("S", [20, 700])                    # one chunk (the caller's state), several (the scratch)
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_state_at_any_element(S, offset):
+    """A state that starts off the 16-byte boundary gives the same numbers bit for bit."""
+    B, H, D, Dv, R = 1, 2, 32, 64, 4
+    g = torch.Generator().manual_seed(S + offset)
+    y, a2, bias = torch.randn(S, 2 * H * D + H * Dv + R, generator=g).cuda(), torch.randn(H * D, R, generator=g).cuda(), torch.randn(H * D, generator=g).cuda()
+    first = torch.randn(B, H, D, Dv, generator=g).cuda()
+    room = torch.full((first.numel() + 8,), 7.0, device="cuda")
+    moved = room[offset:offset + first.numel()].view_as(first)
+    moved.copy_(first)
+    scan = lambda state: SK.gla_scan(y, 0, H * D, 2 * H * D, 2 * H * D + H * Dv, a2, bias, state, None, None, B, S, H, D, Dv, 0.25, 4.0)
+    want, got = scan(first), scan(moved)
+    assert torch.equal(got, want) and torch.equal(moved, first)
+    assert bool((room[:offset] == 7.0).all()) and bool((room[offset + first.numel():] == 7.0).all())

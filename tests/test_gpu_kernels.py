@@ -213,6 +213,27 @@ def test_gemm_small_batch_split_k(M, N, K_, mode):
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[1], outs[2])
 
 
+@pytest.mark.parametrize("N,parts", [(2048, 8), (2560, 7), (3072, 6), (3712, 5), (4736, 4), (6144, 3), (9472, 2)])
+@pytest.mark.parametrize("M,mode", [(9, "residual"), (33, "swiglu"), (128, "f32")])
+def test_gemm_split_k_of_every_cluster_size(N, parts, M, mode):
+    """One CTA of a cluster per part of K, as many parts as leave every SM at most one CTA; against fp32, and bit for bit again and again."""
+    K_ = 2112                                               # 33 blocks of 64: parts of unequal length
+    assert min(148 // (N // 128), 33 // 4, 8) == parts
+    x, w = rnd(M, K_, seed=63), rnd(N, K_, scale=0.03, seed=64)
+    xd, wd = x.to(DEV), w.to(DEV)
+    K.ensure_gemm_workspace(torch.device(DEV))
+    if mode == "residual":
+        res = rnd(M, N, seed=65)
+        want, call = K.linear(x, w, residual=res, mode=K.RESIDUAL), dict(residual=res.to(DEV), mode=K.RESIDUAL)
+    elif mode == "swiglu":
+        want, call = K.linear(x, w, mode=K.SWIGLU), dict(mode=K.SWIGLU)
+    else:
+        want, call = x.float() @ w.float().t(), dict(out_f32=True)
+    outs = [K.linear(xd, wd, force="gemm", **call) for _ in range(3)]
+    assert_close(outs[0], want, 2e-2)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[1], outs[2])
+
+
 @pytest.mark.parametrize("M", [24, 384])
 def test_gemm_epilogues(M):
     N, K_ = 1024, 512

@@ -2,6 +2,8 @@
 import pytest
 import torch
 
+from jax_llama_b200.config import MoeMlpSpec
+from jax_llama_b200.models.feedforward import MoeFeedForward
 from jax_llama_b200.ops import seq_kernels as SK
 
 pytestmark = pytest.mark.gpu
@@ -37,3 +39,28 @@ def test_combine(W, pitch, shift, top, dtype, extras):
     got = SK.moe_combine(z, pos, wt, shared, gate, W, **kw)
     # top + 2 rounded additions and the gate's few roundings: (top + 2 + 4) * 2^-24 of the sum of magnitudes
     assert ((got.double() - want).abs() <= (top + 6) * 2.0 ** -24 * scale + 1e-30).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,experts,top", [(17, 32, 2), (40, 8, 1), (129, 32, 4), (300, 4, 2)])
+def test_buffers_that_nobody_cleared_reach_no_result(M, experts, top, dtype, monkeypatch):
+    """Few tokens and experts without any: whatever the uncleared buffers of the prompt path hold, the layer's output is the same bit for bit."""
+    g = torch.Generator(device=DEV).manual_seed(M)
+    W, F = 256, 136
+    rnd = lambda *s: (torch.randn(*s, generator=g, device=DEV) * s[-1] ** -0.5).to(dtype)
+    w = {"router": rnd(experts, W)}
+    w["router"][experts // 2:] -= 1.0                          # positive inputs: the second half of the experts gets no token
+    for e in range(experts):
+        w[f"e{e}.gate"], w[f"e{e}.up"], w[f"e{e}.down"] = rnd(F, W), rnd(F, W), rnd(W, F)
+    spec = MoeMlpSpec(experts=experts, top=top, ff=F, act="silu", score="softmax", gated=True, shared_ff=0, shared_gate=False)
+    layer = MoeFeedForward(spec, w)
+    h = torch.rand(M, W, generator=g, device=DEV).to(dtype)
+    want = layer.run(h).clone()
+    plain = torch.empty
+
+    def poisoned(*a, **kw):
+        t = plain(*a, **kw)
+        return t.fill_(float("nan")) if t.is_floating_point() else t
+    monkeypatch.setattr(torch, "empty", poisoned)
+    got = layer.run(h)
+    assert bool(torch.isfinite(want).all()) and torch.equal(got, want)

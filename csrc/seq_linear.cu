@@ -110,14 +110,18 @@ __global__ void __launch_bounds__(LR_WARPS * 32) linear_rows_kernel(const T* __r
 // 16-byte chunks t, t + 4, ... of rows g and g + 8 straight into A fragments, and the same chunks of token g into B fragments (the order of
 // k inside a product is free as long as both agree: MMA v of chunk u uses words 2v, 2v + 1), so a batch is 16 weight loads in flight
 // per lane, 8 token loads (L1) and 16 MMAs.  The FMA kernel is bound by issue there: it unpacks every weight and multiplies it once per token.
-// The tensor core truncates when it adds, so a chain of sums is two MMAs long (32 k) and meets the rest in rounded fp32 additions:
-// fp32 results are 0.8 to 1.0e-7 off float64, those of the FMA kernel 0.8 to 0.9e-7, and a layer's or a model's output is not further
-// off than before.  The KS warps of a CTA meet in shared memory, neighbours first.
-// 8 tokens on one B200, FMA kernel -> this one (features x K): 32000 x 2048 83.5 -> 26.2 us, 8192 x 2048 23.8 -> 10.5, 2048 x 8192
-// 16.2 -> 10.6, 2048 x 2048 7.9 -> 4.4.  Up to 4 tokens the FMA kernel, whose loads run along a row (512 contiguous bytes against 64), is
+// The tensor core truncates when it adds, so every MMA (16 k) starts from zero and its sums meet the rest in rounded fp32 additions; the KS
+// warps of a CTA meet in shared memory, neighbours first.  Error against float64 (2-norm; features x K), FMA kernel -> this one, normal
+// operands | of one sign: 2048 x 1536 7.4e-8 -> 7.2e-8 | 4.6e-8 -> 3.9e-8, 2048 x 2048 7.9e-8 -> 7.5e-8 | 4.8e-8 -> 4.4e-8, 8192 x 11008 9.3e-8 ->
+// 9.0e-8 | 5.4e-8 -> 4.4e-8.  It is kept where it is the more exact one: from LM_MIN_K on (2048 x 1024: 6.8e-8 -> 7.0e-8 | 4.3e-8 -> 4.4e-8), and
+// with at most LM_MAX_SEG k to a warp, whose batches are added one after the other (32000 features in parts of 2048 k 8.4e-8 -> 8.5e-8, of 4096 8.9e-8
+// -> 10.0e-8).  (Chains of two MMAs: 5 % faster, but 5.4e-8 with operands of one sign at 2048 x 2048.)
+// 8 tokens on one B200, FMA kernel -> this one (features x K; cold L2, launch included): 32000 x 2048 90 -> 37 us, 8192 x 2048 29.5 -> 18.4,
+// 2048 x 8192 22.6 -> 18.3, 2048 x 2048 14.2 -> 10.1.  Up to 4 tokens the FMA kernel, whose loads run along a row (512 contiguous bytes against 64), is
 // as fast or faster (2 tokens: 2048 x 8192 7.9 against 10.5), and with fewer than 96 groups of 16 features too (8 tokens, 1024 x 5464:
 // 7.4 against 8.9: a warp's batches run one after the other).
 constexpr int LM_U = 8, LM_BATCH = 32 * LM_U;        // chunk groups of 32 k in flight; k of a batch
+constexpr int LM_MIN_K = 1536, LM_MAX_SEG = 1536;
 
 __device__ __forceinline__ uint4 lm_load(const void* p) {      // touched once: no line in L1 (the tokens live there)
   uint4 r;
@@ -167,11 +171,14 @@ __global__ void __launch_bounds__((KS > 4 ? KS : 4) * 32) linear_mma_rows_kernel
         const int k = kb + 32 * u + 8 * t;
         c[u] = tok && k < k1 ? *reinterpret_cast<const uint4*>(xr + k) : make_uint4(0u, 0u, 0u, 0u);
       }
-      float d[LM_U][4] = {};
+      float d[LM_U][4];
 #pragma unroll
       for (int u = 0; u < LM_U; ++u) {
-        lm_mma(d[u], a[u].x, b[u].x, a[u].y, b[u].y, c[u].x, c[u].y);
-        lm_mma(d[u], a[u].z, b[u].z, a[u].w, b[u].w, c[u].z, c[u].w);
+        float e[2][4] = {};
+        lm_mma(e[0], a[u].x, b[u].x, a[u].y, b[u].y, c[u].x, c[u].y);
+        lm_mma(e[1], a[u].z, b[u].z, a[u].w, b[u].w, c[u].z, c[u].w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[u][i] = e[0][i] + e[1][i];
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -198,10 +205,10 @@ __global__ void __launch_bounds__((KS > 4 ? KS : 4) * 32) linear_mma_rows_kernel
 template <typename OutT>
 static void lm_launch(const __nv_bfloat16* x, int ldx, const __nv_bfloat16* w, OutT* out, int ldo, int M, int N, int K, int act, float p0,
                       float p1, cudaStream_t st, const LinearGroup& g, int nbatch) {
-  // parts of K: some 14 warps on every SM (8 KB in flight each), each part at least half a batch long
+  // parts of K: some 14 warps on every SM (8 KB in flight each), each part at least half a batch long, at most LM_MAX_SEG
   const long groups = (long)((N + 15) / 16) * nbatch;
   int ks = 1;
-  while (ks < 16 && groups * ks < 148 * 14 && K >= 2 * ks * (LM_BATCH / 2)) ks *= 2;
+  while (ks < 16 && (K > ks * LM_MAX_SEG || (groups * ks < 148 * 14 && K >= 2 * ks * (LM_BATCH / 2)))) ks *= 2;
   const int per = (ks > 4 ? 1 : 4 / ks) * 16;
   const dim3 grid((N + per - 1) / per, nbatch), block((ks > 4 ? ks : 4) * 32);
 #define JL_LM(KS_) case KS_: JL_LAUNCH_PDL((linear_mma_rows_kernel<OutT, KS_>), grid, block, 0, st, x, ldx, w, out, ldo, M, N, K, act, p0, p1, g); break;
@@ -280,7 +287,7 @@ static int launch_linear(const void* x, int ldx, const void* w, void* out, int l
     const int vec_ok = (K % VN == 0) && (ldx % VN == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) &&
                        (g.x_bs % VN == 0) && (g.w_bs % VN == 0);
     if constexpr (sizeof(T) == 2) {
-      if (tensor_cores && vec_ok && M > 4 && (long)((N + 15) / 16) * nbatch >= 96) {
+      if (tensor_cores && vec_ok && M > 4 && K >= LM_MIN_K && K <= 16 * LM_MAX_SEG && (long)((N + 15) / 16) * nbatch >= 96) {
         lm_launch<OutT>((const T*)x, ldx, (const T*)w, (OutT*)out, ldo, M, N, K, act, p0, p1, st, g, nbatch);
         return cudaGetLastError() == cudaSuccess ? JL_OK : JL_ERR_CUDA;
       }

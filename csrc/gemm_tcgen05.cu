@@ -17,6 +17,8 @@
 // :311-338 (w1/w2/w3) and :699-706 (lm_head).
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "jllama_b200.h"
 #include "tcgen05.cuh"
 
@@ -356,20 +358,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
                 if (tok < p.Rb && ra < p.Ra) rr[u] = __bfloat162float(p.residual[(size_t)tok * p.ldo + ra]);
               }
             }
-            float q[8][4];                                // all ranks' four tokens in flight; a warp reads 128 bytes of a rank
+            float x[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+            for (int sp0 = 0; sp0 < ksplit; sp0 += 8) {   // eight ranks' four tokens in flight; a warp reads 128 bytes of a rank
+              float q[8][4];
 #pragma unroll
-            for (int sp = 0; sp < 8; ++sp)
-              if (sp < ksplit) {
-                const uint32_t at = gemm_mapa(part + j0 * (GEMM_BM * 4), sp);
+              for (int sp = 0; sp < 8; ++sp)
+                if (sp0 + sp < ksplit) {
+                  const uint32_t at = gemm_mapa(part + j0 * (GEMM_BM * 4), sp0 + sp);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) q[sp][u] = gemm_ld_cluster(at + u * (GEMM_BM * 4));
-              }
-            float x[4];
+                  for (int u = 0; u < 4; ++u) q[sp][u] = gemm_ld_cluster(at + u * (GEMM_BM * 4));
+                }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              x[u] = q[0][u];
+              for (int u = 0; u < 4; ++u)
 #pragma unroll
-              for (int sp = 1; sp < 8; ++sp) if (sp < ksplit) x[u] += q[sp][u];
+                for (int sp = 0; sp < 8; ++sp) if (sp0 + sp < ksplit) x[u] += q[sp][u];
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) swap_emit(b_blk * BN + j0 + u, x[u], true, rr[u]);
@@ -402,6 +405,40 @@ static bool splitk_allowed() {
   return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 16 && g_splitk[dev];
 }
 
+constexpr uint32_t gemm_stage_bytes(int bn) { return GEMM_BM * GEMM_BK * 2 + (bn * GEMM_BK * 2 < 1024 ? 1024 : bn * GEMM_BK * 2); }
+constexpr int GEMM_SPLIT_RING = 100 * 1024;               // ring of a split-K launch: two CTAs of neighbouring kernels fit an SM
+constexpr size_t gemm_smem(int stages, int bn) { return (size_t)stages * gemm_stage_bytes(bn) + 8 * (2 * stages + 4) + 16 + 1024; }
+
+// whether the device holds clusters of `ks` > 8 CTAs of the split-K kernel (asked once per device, kernel and size)
+template <int BN, int EPI, bool OUT_F32>
+static bool wide_clusters(int ks, int num_sms) {
+  static std::atomic<signed char> known[16][17];          // 0: not asked yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return false;
+  signed char v = known[dev][ks].load(std::memory_order_relaxed);
+  if (v == 0) {
+    auto kern = gemm_kernel<BN, EPI, true, OUT_F32>;
+    int n = 0, stages = (int)(GEMM_SPLIT_RING / gemm_stage_bytes(BN));
+    if (stages > 10) stages = 10;
+    const size_t smem = gemm_smem(stages, BN);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(num_sms / ks * ks);
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+                    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1;
+    if (!ok) cudaGetLastError();
+    v = ok ? 1 : -1;
+    known[dev][ks].store(v, std::memory_order_relaxed);
+  }
+  return v > 0;
+}
+
 template <int BN, int EPI, bool SWAP, bool OUT_F32>
 static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int Ra, int Rb, int K, int num_sms,
                        cudaStream_t stream, int b_matrices = 1) {
@@ -412,9 +449,7 @@ static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int R
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, b, Rb * b_matrices, K, K, BN);
   if (rc) return rc;
-  constexpr uint32_t A_BYTES = GEMM_BM * GEMM_BK * 2;
-  constexpr uint32_t B_BYTES = BN * GEMM_BK * 2;
-  constexpr uint32_t STAGE_BYTES = A_BYTES + (B_BYTES < 1024 ? 1024 : B_BYTES);
+  constexpr uint32_t STAGE_BYTES = gemm_stage_bytes(BN);
   const int num_kb = (K + GEMM_BK - 1) / GEMM_BK;
   p.a_blocks = (Ra + GEMM_BM - 1) / GEMM_BM;
   p.b_blocks = (Rb + BN - 1) / BN;
@@ -425,7 +460,11 @@ static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int R
     if (grid * 2 <= num_sms && splitk_allowed()) {
       int ks = num_sms / grid;
       if (ks > num_kb / 4) ks = num_kb / 4;
-      if (ks > 8) ks = 8;                                  // portable cluster size
+      // Eight CTAs are what every GPU takes as a cluster.  More pay with a long K over few weight tiles (9 to 16 rows of 1024 x 14336: 8 parts
+      // 11.8 us, 16 parts 10.1; 1536 x 14336 12.8 and 12.0 in 12 parts); at K 8192 and below, and with less than half as many again, the
+      // wider meeting costs what it gives or more (1024 x 4096 5.8 and 5.9 us, 64 rows 7.8 and 8.5; 2048 x 14336, 9 parts, 13.7 and 14.1).
+      if (ks > 16) ks = 16;
+      if (ks > 8 && (ks < 12 || num_kb <= 128 || !wide_clusters<BN, EPI, OUT_F32>(ks, num_sms))) ks = 8;
       if (ks > 1) {
         p.ksplit = ks;
         grid *= ks;
@@ -439,12 +478,12 @@ static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int R
   // grid — runs under our epilogue and split-K finish; those prologue / tail latencies were most of a 25 us GEMM.
   // A split-K launch always takes the small ring too (its partial tile, at most 64 KB, fits).
   int budget = 200 * 1024;
-  if (SWAP && (p.ksplit > 1 || (size_t)Ra * K * 2 / grid <= (size_t)1280 * 1024)) budget = 100 * 1024;
+  if (SWAP && (p.ksplit > 1 || (size_t)Ra * K * 2 / grid <= (size_t)1280 * 1024)) budget = GEMM_SPLIT_RING;
   int stages = (int)(budget / STAGE_BYTES);
   if (stages > 10) stages = 10;
   if (stages > num_kb * 2) stages = num_kb * 2 < 2 ? 2 : num_kb * 2;
   p.stages = stages;
-  const size_t smem = (size_t)stages * STAGE_BYTES + 8 * (2 * stages + 4) + 16 + 1024;
+  const size_t smem = gemm_smem(stages, BN);
   auto kern = gemm_kernel<BN, EPI, SWAP, OUT_F32>;
   JL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (p.ksplit == 1) {

@@ -220,9 +220,10 @@ struct DeltaHeadParams {
 
 __device__ __forceinline__ float delta_head_decay(float z, float a_log) { return expf(-expf(a_log) * delta_softplus(z)); }
 
-// grid (tokens, q / k heads), 128 threads: warp l forms the dot products at lag l.  (One warp per token with all lags in registers is
-// the faster kernel alone, 50 us against 66 for 2000 tokens x 16 heads of 64 x 128, but as a link of the launch chain it made the
-// layer slower: 452 us a pass against 385.)
+// grid (tokens, q / k heads), 128 threads: warp l forms the dot products at lag l.  One warp per token with all lags in registers is
+// the faster kernel, 50 us against 66 for 2000 tokens x 16 heads of 64 x 128, and without programmatic dependent launch the faster layer, 377 us
+// a pass against 391.  With it the layer is slower, 450 against 385, presumably by placement: the scan's few long CTAs come in as soon as the last CTAs of this
+// kernel have started, and a quarter as many, four times as long CTAs leave them the room of a few SMs, where they then share.
 template <typename T, int DP>
 __global__ void __launch_bounds__(32 * DH_NB) delta_head_prep_kernel(DeltaHeadParams p, const T* __restrict__ a_bias, const T* __restrict__ a_log) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done

@@ -1,9 +1,9 @@
 """Reference arm of bench.py: the UNMODIFIED reference (installed under baseline/_ref) driven through its own public
 API and stock code path, for the same metric and config as our arm.
 
-What it runs is the reference's `jax_example.load` flow (/root/reference/jax_example.py:10-31) with random-init
+What it runs is the reference's `jax_example.load` flow (jax_example.py:10-31) with random-init
 parameters in place of a checkpoint (there are none on the box) and then `LLaMA.generate`
-(/root/reference/jax_llama/generation.py:22-45):
+(jax_llama/generation.py:22-45):
 
     mesh (1, n_devices) over ('dp', 'mp')  →  FlaxLLaMAForCausalLM(config, _do_init=False)
     →  params = model.init_weights(...) placed with get_llama_param_partition_spec(params, fsdp=False)

@@ -97,7 +97,7 @@ class SyntheticTokenizer:
 
 def tp_check(args, cfg, eng, dev, rank: int, world: int) -> dict:
     """Correctness of the tensor-parallel engine, measured before the timed region and printed in the JSON line
-    (the reference trusts its sharded model only after /root/reference/jax_test.py:427-522 compared logits and
+    (the reference trusts its sharded model only after jax_test.py:427-522 compared logits and
     greedy generations over all GPUs).  The single-GPU engine built from the same seed is the same model
     (`B200Engine.random_init` slices full matrices), so on every rank we compare
       * last-token prefill logits, TP vs single GPU (max error relative to the largest logit);

@@ -3,7 +3,7 @@
 //
 // The reference has no explicit collective: GSPMD inserts NCCL all-reduces after the row-parallel `wo`
 // and `w2` matmuls and an all-gather of the vocab-sharded logits (SURVEY §2.5, K2-K4;
-// /root/reference/jax_llama/partition.py:62-78).  Here every rank maps every peer's "inbox" buffer
+// jax_llama/partition.py:62-78).  Here every rank maps every peer's "inbox" buffer
 // (CUDA IPC) and:
 //   * `gemv_ar_kernel`  — row-parallel linear at decode batch sizes + ONE-SHOT all-reduce + residual add:
 //     each CTA computes a 32-row slice of the partial product, stores it (fp32) straight into every

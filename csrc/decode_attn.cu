@@ -1,7 +1,7 @@
 // Single-token (decode) attention over the KV cache with GQA: split-KV "flash decoding".
 //
 // The reference attends over all `max_length` cache slots with a mask every step
-// (/root/reference/jax_llama/model.py:194-198,263-288); here only the filled, non-padding prefix
+// (jax_llama/model.py:194-198,263-288); here only the filled, non-padding prefix
 // [pad_left[b], cache_len + n_new) is streamed, once, at HBM rate, and no mask tensor or repeated KV
 // heads are ever materialised: the G query heads of a KV group share every K/V byte loaded.
 //

@@ -14,7 +14,7 @@
 //     per CTA, merge spread over the grid), final norm + LM head with a running arg-max.
 //   * rows of each GEMV are cut into 148 contiguous, near-equal ranges (±1 group of 8 rows).
 //
-// DATA-FLOW SYNCHRONISATION (round 2).  The first version separated the ops with 5-6 grid-wide barriers per
+// DATA-FLOW SYNCHRONISATION.  The first version separated the ops with 5-6 grid-wide barriers per
 // layer plus two all-reduce waits; the %globaltimer trace put ≈ 12 of 44 µs per layer into them at TP=4, which
 // is why 8 GPUs bought only 2.07x one GPU.  Now there is NO grid barrier.  Every activation that crosses CTAs
 // travels as an 8-byte TAGGED PACKET {payload, tag}: the producer's plain store is data and flag at once (an
@@ -50,9 +50,9 @@
 //
 // Weights of all layers are stacked per op ([L·N, K]) so five tensor maps describe the whole model.
 // Math is identical to the unfused kernels (gemv.cu, decode_attn_fused.cu); the tests compare the two.
-// Reference: the body of HF Flax `_sample`'s while-loop that /root/reference/jax_llama/generation.py:28-41
+// Reference: the body of HF Flax `_sample`'s while-loop that jax_llama/generation.py:28-41
 // runs as one compiled XLA program — this is the hand-written equivalent; the all-reduces are the ones GSPMD
-// inserts for /root/reference/jax_llama/partition.py:67,70.
+// inserts for jax_llama/partition.py:67,70.
 #include <stdlib.h>
 
 #include "jllama_b200.h"
@@ -349,7 +349,7 @@ __device__ __forceinline__ void mg_attention_item(const MegaParams& p, const Meg
   const bool owns_new = split == 0 && warp == 0;      // consumes the new k, v after the KV loop
   // The K/V cache rows of this item's first load batch do not depend on q: request them BEFORE polling for q, so the
   // HBM round trip of the cache overlaps the wait for the qkv GEMV of the other CTAs (needs the 224-register
-  // consumers: at 168 registers the held rows spilled and this lost, round 1).
+  // consumers: at 168 registers the held rows spilled and this lost).
   constexpr int UNR = G <= 4 ? 2 : 1;
   const size_t head_off = (((size_t)layer * M + b) * p.nkv + kvh) * (size_t)p.T * HD;
   const __nv_bfloat16* kbase = p.kc + head_off + lig * 8;

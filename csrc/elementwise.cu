@@ -1,7 +1,7 @@
 // Memory-bound building blocks: embedding gather, RMSNorm (+ fused residual add), RoPE fused with the
 // KV-cache append, stand-alone SwiGLU.  All bf16 in/out, fp32 math, 16-byte vector accesses.
 //
-// Reference ops: /root/reference/jax_llama/model.py:42-48 (RMSNorm), :58-92 (interleaved RoPE),
+// Reference ops: jax_llama/model.py:42-48 (RMSNorm), :58-92 (interleaved RoPE),
 // :177-199 (cache append), :338 (SwiGLU), :611-617,638 (embedding).
 #include "common.cuh"
 #include "jllama_b200.h"

@@ -1,7 +1,7 @@
 // Causal flash attention for prefill on tcgen05 tensor cores (head_dim 128, GQA, left padding).
 //
 // The reference materialises softmax(QKᵀ/√d + bias) as a [B, nh, Q, K] tensor with an explicit mask
-// (/root/reference/jax_llama/model.py:236-288).  Here one CTA owns a 128-query tile of one head and walks
+// (jax_llama/model.py:236-288).  Here one CTA owns a 128-query tile of one head and walks
 // the visible keys in tiles of 64; two such CTAs share an SM so that one CTA's softmax runs under the other's
 // MMAs (each SM sub-partition then has two softmax warps to switch between):
 //   S = Q·Kᵀ   tcgen05.mma (A = Q, B = K tile, both K-major in smem via TMA) → TMEM, double-buffered;

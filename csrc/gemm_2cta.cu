@@ -21,7 +21,7 @@
 // Used for token-major GEMMs with M >= 256 and N and K multiples of 256 and 64 (every prefill GEMM of the LLaMA shapes); plain bf16 and
 // fp32 results with any N and K that are multiples of 8 (the tensor maps read zeros and clip beyond the matrix).  Other shapes take the
 // single-CTA kernel (gemm_tcgen05.cu).  Replaces the cuBLAS GEMMs XLA emitted for
-// /root/reference/jax_llama/model.py:119-150 (wq/wk/wv/wo) and :311-338 (w1/w2/w3).
+// jax_llama/model.py:119-150 (wq/wk/wv/wo) and :311-338 (w1/w2/w3).
 #include <stdlib.h>
 
 #include <atomic>

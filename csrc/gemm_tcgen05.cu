@@ -13,7 +13,7 @@
 //           [M,K] (MMA N = padded batch); the D tile is transposed on the way out.
 // Epilogues: plain bf16 / fp32, residual add, SwiGLU over interleaved (w1,w3) output columns.
 //
-// Replaces the cuBLAS GEMMs XLA emitted for /root/reference/jax_llama/model.py:119-150 (wq/wk/wv/wo),
+// Replaces the cuBLAS GEMMs XLA emitted for jax_llama/model.py:119-150 (wq/wk/wv/wo),
 // :311-338 (w1/w2/w3) and :699-706 (lm_head).
 #include <stdlib.h>
 
@@ -215,7 +215,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     // ===================================================== epilogue: TMEM → registers → global
     const int quarter = warp & 3;                           // TMEM lanes [32·quarter, 32·quarter+32)
     int it = 0;
-    if constexpr (SWAP) pdl_wait();                         // residual, output, split-K scratch: after the previous kernel
+    if constexpr (SWAP) pdl_wait();                         // residual, output: after the previous kernel
     for (int wi = blockIdx.x; wi < num_work; wi += gridDim.x, ++it) {
       const int t = wi / ksplit, split = wi % ksplit;
       const int b_blk = t / a_blocks;

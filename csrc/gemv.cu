@@ -7,7 +7,7 @@
 // mma.sync and reaches the HBM roofline.  M > 8 goes to the tcgen05 swap-AB kernel in gemm_tcgen05.cu.
 //
 // Covers the reference's wq/wk/wv (fused), wo, w1/w3 (fused, interleaved), w2 and lm_head at decode
-// (/root/reference/jax_llama/model.py:119-150,311-338,699-706).
+// (jax_llama/model.py:119-150,311-338,699-706).
 #include "common.cuh"
 #include "jllama_b200.h"
 

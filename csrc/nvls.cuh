@@ -4,7 +4,7 @@
 // (`multimem.red`).  The multicast mapping itself is created by parallel/symm.py.
 //
 // What these replace: the reference's collectives are whatever NCCL call GSPMD emits for the shardings of
-// /root/reference/jax_llama/partition.py:62-78; here the same traffic is issued from inside the compute kernels.
+// jax_llama/partition.py:62-78; here the same traffic is issued from inside the compute kernels.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

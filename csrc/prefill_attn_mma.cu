@@ -2,7 +2,7 @@
 //
 // Why it exists: the tcgen05 flash kernel (flash_prefill.cu) is built for head_dim 128, the width of every LLaMA-1/2/3
 // checkpoint the reference names.  LLaMA-architecture models with 64-wide heads (hidden 2048 / 32 heads: the 1B class)
-// are loadable by the reference as well (/root/reference/jax_llama/model.py:115 takes any hidden / heads), so they get
+// are loadable by the reference as well (jax_llama/model.py:115 takes any hidden / heads), so they get
 // a kernel here instead of a refusal.  Same contract as jl_flash_prefill; reference semantics model.py:201-300 (S > 1).
 //
 // Shape of the kernel: one warp owns 16 query rows of one head and walks the visible keys in blocks of 32 (16 at head_dim

@@ -1,9 +1,9 @@
 // Exact temperature / top-k / top-p / categorical selection over the WHOLE vocabulary, a cluster of CTAs per row, plus the
 // sequence bookkeeping of the step — the second (and last) launch of a sampling decode step at any tp.
 //
-// Reference behaviour: the HF Flax warpers as configured by /root/reference/jax_llama/generation.py:28-41 —
+// Reference behaviour: the HF Flax warpers as configured by jax_llama/generation.py:28-41 —
 // logits / T → top-k (if set) → top-p with min_tokens_to_keep = 1 (sorted descending, a token is kept while the
-// probability mass before it is < top_p) → categorical; temperature 0 = arg-max.  Round 1 ran this on at most 64
+// probability mass before it is < top_p) → categorical; temperature 0 = arg-max.  A first form ran this on at most 64
 // candidates per row, so `top_k=None` silently meant "nucleus over the 64 most likely tokens" on the GPU and a
 // plateau of equal logits could overflow the candidate list.  This kernel has no candidate budget:
 //

@@ -3,7 +3,7 @@
 // the decode loop free of host synchronisation.
 //
 // Reference behaviour: HF Flax logits warpers + `_sample/_greedy_search` as configured by
-// /root/reference/jax_llama/generation.py:28-41 (temperature → top-k → top-p(min_keep=1) → categorical;
+// jax_llama/generation.py:28-41 (temperature → top-k → top-p(min_keep=1) → categorical;
 // finished rows emit pad; EOS marks a row finished).  The candidate representation is what makes the
 // vocab-parallel head exact without gathering [B, V] logits: each rank extracts its local top-k
 // (value, global index) pairs, ranks exchange tp·k pairs, and every rank runs the identical final

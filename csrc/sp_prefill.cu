@@ -1,6 +1,6 @@
 // Owner-side step of the sequence-parallel prefill and the all-reduce of a row-parallel GEMM, over NVLS.
 // What XLA/GSPMD emitted here for the reference: an NCCL all-reduce of the whole [M, H] activation after wo / w2
-// (/root/reference/jax_llama/partition.py:67,70), then replicated norms (:73-76).  (Round 1 scattered the GEMM's
+// (jax_llama/partition.py:67,70), then replicated norms (:73-76).  (A first form scattered the GEMM's
 // partial tiles into the row owners' buffers with per-thread remote stores and pushed the normalised rows with tp
 // unicast stores; it lost to NCCL by 8-19 % and is gone.)
 #include "common.cuh"
@@ -10,7 +10,7 @@
 namespace jl {
 
 // ------------------------------------------------------------------------------------------------------------------
-// NVLS form of the owner-side reduction (round 2).  The row-parallel GEMM no longer scatters anything: it stores its
+// NVLS form of the owner-side reduction.  The row-parallel GEMM no longer scatters anything: it stores its
 // bf16 partial product [M, H] into ITS OWN copy of a symmetric buffer with ordinary coalesced stores and runs at full
 // speed.  The reduce-scatter is one `multimem.ld_reduce` per 16 bytes on the multicast address of that buffer: the
 // NVSwitch fetches the tp partials, sums them in fp32 and returns 8 reduced bf16 — 1/tp of the bytes per rank that
@@ -134,7 +134,7 @@ using namespace jl;
 //   * sequence-parallel owner step: rows = mloc, xn_mc != NULL (normalised rows broadcast, "ready" flag published);
 //   * plain all-reduce of a row-parallel GEMM (any token count): rows = M, xn_mc = NULL — every rank pulls the sum of
 //     all rows and adds it to its replicated residual stream (what GSPMD's all-reduce did for
-//     /root/reference/jax_llama/partition.py:67,70).
+//     jax_llama/partition.py:67,70).
 // has_partials = 0 skips the reduction (chain start on the embedding rows).
 //   * batched decode under TP: rows = batch, has_partials = 1 (the "GEMM done" exchange happens inside: the grid is a
 //     few dozen resident CTAs), xn_mc = NULL, xn_local = where the rows normalised with `norm_w` go — all-reduce,

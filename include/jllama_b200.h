@@ -7,7 +7,7 @@
  *  - activations / weights are bf16, row-major; linear weights are [N, K] (out, in) i.e. K-major;
  *  - kernels are launched with Programmatic Dependent Launch enabled and are safe in PDL chains.
  *
- * Each declaration cites the reference op it replaces (paths under /root/reference/jax_llama/).
+ * Each declaration cites the reference op it replaces (paths under jax_llama/).
  */
 #ifndef JLLAMA_B200_H
 #define JLLAMA_B200_H

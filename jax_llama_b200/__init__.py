@@ -1,6 +1,6 @@
 """jax_llama_b200 — a B200-native LLaMA inference framework with the capabilities of LSaldyt/JAX_llama.
 
-Public surface mirrors /root/reference/jax_llama/__init__.py:4-10 (plus torch-flavoured names).
+Public surface mirrors jax_llama/__init__.py:4-10 (plus torch-flavoured names).
 """
 from .config import LLaMAConfig, ModelArgs, config_from_params, preset
 from .convert_weights import convert_llama_weights, convert_llama_weights_for_rank, write_meta_checkpoint

@@ -2,7 +2,7 @@
 
 The reference only knows how to load Meta ``consolidated.*.pth`` files — every start pays the
 "load all shards, concatenate, cast to fp32" cost, ~3× the model in host RAM
-(/root/reference/jax_llama/convert_weights.py:55-89; its ``convert.sh --out_dir`` is stale and writes
+(jax_llama/convert_weights.py:55-89; its ``convert.sh --out_dir`` is stale and writes
 nothing).  This module adds the missing persistence layer:
 
     cache_dir/

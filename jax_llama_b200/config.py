@@ -1,11 +1,11 @@
 """Model configuration.
 
 `LLaMAConfig` keeps the field names, defaults and JSON schema of the reference's HF-style config
-(/root/reference/jax_llama/config.py:72-116) but is a free-standing class: it does not depend on
+(jax_llama/config.py:72-116) but is a free-standing class: it does not depend on
 `transformers`, so it loads in every process of a torchrun job without importing HF.
 
 `ModelArgs` / `config_from_params` mirror Meta's ``params.json`` schema and the SwiGLU width formula
-(/root/reference/jax_llama/convert_weights.py:13-50).  Unlike the reference, unknown ``params.json``
+(jax_llama/convert_weights.py:13-50).  Unlike the reference, unknown ``params.json``
 keys (e.g. LLaMA-3.1's ``use_scaled_rope``) are tolerated and reported instead of raising.
 """
 from __future__ import annotations
@@ -152,7 +152,7 @@ class LLaMAConfig:
 
 @dataclass
 class ModelArgs:
-    """Meta ``params.json`` schema (/root/reference/jax_llama/convert_weights.py:13-26)."""
+    """Meta ``params.json`` schema (jax_llama/convert_weights.py:13-26)."""
 
     dim: int = 512
     n_layers: int = 8

@@ -1,6 +1,6 @@
 """Meta checkpoint (``consolidated.NN.pth`` + ``params.json``) → canonical parameter tree.
 
-Same contract as /root/reference/jax_llama/convert_weights.py:52-92: the result is the tree of
+Same contract as jax_llama/convert_weights.py:52-92: the result is the tree of
 SURVEY §2.2 (``transformer/h/{i}/attention/wq/kernel`` …) with linear kernels in ``[in, out]``
 layout, plus a `LLaMAConfig` whose ``vocab_size`` comes from the tokenizer.  Differences, on purpose:
 
@@ -252,7 +252,7 @@ test_intermediate_size.__test__ = False                  # a helper with a refer
 
 def main(argv: Optional[Sequence[str]] = None) -> int:
     """``python -m jax_llama_b200.convert_weights --ckpt_dir D --out_dir O [--tp N]`` — the command the
-    reference's convert.sh calls but never shipped (/root/reference/convert.sh:10): Meta shards → the sharded
+    reference's convert.sh calls but never shipped (convert.sh:10): Meta shards → the sharded
     safetensors cache of `checkpoint.py`, one rank slice at a time."""
     import argparse
 

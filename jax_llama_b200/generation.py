@@ -1,6 +1,6 @@
 """Generation front-end: `LLaMA(params, model, tokenizer, mesh).generate / generate_from_str`.
 
-Same call signatures and post-processing as /root/reference/jax_llama/generation.py:15-79: prompts
+Same call signatures and post-processing as jax_llama/generation.py:15-79: prompts
 are encoded with BOS, left-padded with ``eos_id`` to the longest prompt, the attention mask is
 ``tokens != eos_id``, sampling is on iff ``temperature != 0``, and the returned strings include the
 prompt, start at the first BOS and stop before the first EOS.  Added knobs (`top_k`, `seed`) default

@@ -12,7 +12,7 @@ What XLA/GSPMD did implicitly for the reference (fused elementwise kernels, cuBL
 * the step's moving parts (``cache_len``, ``cur_len``, RNG step, finished flags) live in device memory so
   the same graph serves every position.
 
-Model math: /root/reference/jax_llama/model.py:201-300 (attention), :337-340 (MLP), :374-398 (block),
+Model math: jax_llama/model.py:201-300 (attention), :337-340 (MLP), :374-398 (block),
 :622-741 (backbone + head); decode loop semantics: HF Flax `_sample` as configured by generation.py:28-41.
 """
 from __future__ import annotations

@@ -1,6 +1,6 @@
 """HF-style model classes: `LLaMAModel`, `LLaMAForCausalLM` (+ `FlaxLLaMA*` aliases).
 
-API surface of /root/reference/jax_llama/model.py:402-546,680-772: ctor ``(config, input_shape, seed,
+API surface of jax_llama/model.py:402-546,680-772: ctor ``(config, input_shape, seed,
 dtype, _do_init)``, ``__call__(input_ids, attention_mask, position_ids, params, past_key_values, …,
 output_attentions, output_hidden_states, return_dict)``, ``init_cache``, the two generation hooks,
 ``generate`` (inherited from HF in the reference; implemented here), ``save_pretrained`` /

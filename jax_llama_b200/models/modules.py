@@ -2,8 +2,8 @@
 
 The reference exposes its layers as `flax.linen` modules (`RMSNorm`, `FlaxLLaMAAttention`, `FlaxLLaMAMLP`,
 `FlaxLLaMABlock`, `FlaxLLaMABlockCollection`, `FlaxLLaMAModule`, `FlaxLLaMAForCausalLMModule`;
-/root/reference/jax_llama/model.py:28-48, 105-300, 302-340, 342-400, 548-600, 602-677, 691-741) and its own
-parity harness drives them with ``module.apply({"params": subtree}, ...)`` (/root/reference/jax_test.py:73-413).
+jax_llama/model.py:28-48, 105-300, 302-340, 342-400, 548-600, 602-677, 691-741) and its own
+parity harness drives them with ``module.apply({"params": subtree}, ...)`` (jax_test.py:73-413).
 Here the math lives in plain functions (`models/reference.py`, the fp32 oracle) and in CUDA kernels
 (`models/engine.py`); these classes give the same call shape over the same parameter sub-trees so that such
 code keeps working.  They are stateless: all weights come in through `variables["params"]`.

@@ -1,7 +1,7 @@
 """Plain-PyTorch LLaMA forward pass: the numerical oracle and the CPU execution path.
 
 This is a deliberately un-fused restatement of the model math the reference implements in Flax
-(/root/reference/jax_llama/model.py:28-300 RMSNorm / RoPE / GQA attention with KV cache,
+(jax_llama/model.py:28-300 RMSNorm / RoPE / GQA attention with KV cache,
 :302-400 SwiGLU MLP and pre-norm block, :602-741 backbone and LM head).  It works on the canonical
 parameter tree (kernels ``[in, out]``), supports arbitrary key-padding masks, ``output_attentions`` /
 ``output_hidden_states``, and is what every CUDA kernel in ``csrc/`` is tested against.

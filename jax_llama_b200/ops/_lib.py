@@ -150,7 +150,7 @@ def lib() -> C.CDLL:
     from .build import is_fresh
     path = LIB_PATH
     partial = False
-    if os.environ.get("JLLAMA_LIB"):           # A/B of two builds on one box (scripts/sweep_env.sh JLLAMA_LIB "a.so b.so")
+    if os.environ.get("JLLAMA_LIB"):           # A/B of two builds on one box
         from pathlib import Path
         path = Path(os.environ["JLLAMA_LIB"])
     elif _subset is not None and not is_fresh():

@@ -1,7 +1,7 @@
 """Logit processing and token selection: temperature → top-k → top-p → categorical / argmax.
 
 The reference gets this pipeline from HF's Flax generation mixin, configured at
-/root/reference/jax_llama/generation.py:32-40 (`do_sample = temperature != 0`, nucleus `top_p`,
+jax_llama/generation.py:32-40 (`do_sample = temperature != 0`, nucleus `top_p`,
 HF-4.x default `top_k=50`, `min_tokens_to_keep=1`).  This module is the fp32 PyTorch statement of that
 pipeline (CPU path and oracle); the CUDA path (`csrc/sampling.cu`) implements the same selection on
 candidates gathered across tensor-parallel ranks.

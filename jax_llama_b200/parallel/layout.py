@@ -1,7 +1,7 @@
 """Tensor-parallel layout: partition rules, mesh, shard / unshard of the canonical parameter tree.
 
 The reference describes its layout as regex rules that map parameter paths to `PartitionSpec`s and
-lets XLA/GSPMD do the rest (/root/reference/jax_llama/partition.py:16-81).  Here the same rule table
+lets XLA/GSPMD do the rest (jax_llama/partition.py:16-81).  Here the same rule table
 is the single source of truth, but it is *executed* explicitly: `shard_tree` cuts the canonical tree
 (SURVEY §2.2 names, kernels in `[in, out]` layout) into the per-rank slices a Megatron-style TP engine
 loads on one GPU each, and `unshard_tree` is its inverse (used by tests and checkpoint export).

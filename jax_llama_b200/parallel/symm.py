@@ -8,7 +8,7 @@
 The mapping (``cuMemCreate`` + ``cuMulticastCreate/BindMem`` + handle exchange) is done by
 ``torch.distributed._symmetric_memory``; every instruction that touches it is ours.  When the platform has no
 multicast support ``mc_ptr`` is 0 and the kernels fall back to one unicast store per peer.  What this replaces:
-the placement XLA/GSPMD derives from /root/reference/jax_llama/partition.py:62-78 plus the NCCL buffers it
+the placement XLA/GSPMD derives from jax_llama/partition.py:62-78 plus the NCCL buffers it
 allocates behind the scenes.
 """
 from __future__ import annotations

@@ -1,7 +1,7 @@
 """Tensor-parallel forward pass in plain PyTorch + torch.distributed (gloo on CPU, NCCL on GPU).
 
 Executes the Megatron layout that the partition rules describe (column-parallel wq/wk/wv/w1/w3, row-parallel
-wo/w2 followed by an all-reduce, vocab-parallel embedding and LM head — /root/reference/jax_llama/
+wo/w2 followed by an all-reduce, vocab-parallel embedding and LM head — jax_llama/
 partition.py:62-78) with explicit collectives.  It is the host-side oracle for the fused NVLink kernels and
 the way the layout is tested without GPUs (2-process gloo runs in tests/test_tp_cpu.py).
 """

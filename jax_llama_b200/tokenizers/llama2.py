@@ -1,6 +1,6 @@
 """LLaMA-1/2 tokenizer: a thin shell over the sentencepiece C++ library.
 
-Capability parity with /root/reference/jax_llama/llama2_tokenizer.py:14-71 (`encode(s, bos, eos)`,
+Capability parity with jax_llama/llama2_tokenizer.py:14-71 (`encode(s, bos, eos)`,
 `decode`, `len()`, `n_words/bos_id/eos_id/pad_id`).  Tokenisation is host-side and off the measured
 path, so the native dependency is kept.
 """

@@ -1,6 +1,6 @@
 """LLaMA-3 tokenizer (tiktoken BPE + 256 reserved specials) and chat prompt format.
 
-Capability parity with /root/reference/jax_llama/llama3_tokenizer.py:38-232.  The special-token
+Capability parity with jax_llama/llama3_tokenizer.py:38-232.  The special-token
 table, its order and the split regex are part of Meta's published LLaMA-3 vocabulary definition (an
 interchange format), so they are reproduced as data; the code around them is ours.
 """

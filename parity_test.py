@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Parity harness — the counterpart of the reference's jax_test.py (/root/reference/jax_test.py:524-649).
+"""Parity harness — the counterpart of the reference's jax_test.py (jax_test.py:524-649).
 
     python parity_test.py                                   # unit parity, CPU, synthetic tiny model
     python parity_test.py --ckpt_dir D --tokenizer_path T [--is_llama3 true]

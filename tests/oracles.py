@@ -2,7 +2,7 @@
 
 HF uses the half-split rotary convention, Meta/ours the interleaved one, so wq/wk rows are permuted
 (the standard Meta→HF conversion).  Two independent implementations agreeing stands in for the Meta
-repository the reference's own harness compared against (/root/reference/jax_test.py:316-413).
+repository the reference's own harness compared against (jax_test.py:316-413).
 """
 import torch
 

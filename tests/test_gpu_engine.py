@@ -118,7 +118,7 @@ def test_generate_eos_and_sampling_on_device():
 def test_left_pad_counts_do_not_leak_into_the_next_request():
     """generate(mask with left padding) followed by generate(no mask) on the same (B, max_length) reuses the
     cached KV object: the second request must run with zero left padding (reference: every call of
-    /root/reference/jax_llama/model.py:748-767 builds its positions from that call's mask alone)."""
+    jax_llama/model.py:748-767 builds its positions from that call's mask alone)."""
     cfg, tree, tree32 = make("gqa128")
     eng = B200Engine.from_tree(cfg, tree_to(tree, device="cuda"))
     ids = torch.randint(3, cfg.vocab_size, (2, 10), generator=torch.Generator().manual_seed(11)).cuda()
@@ -308,7 +308,7 @@ def test_megakernel_matches_fp32_oracle_at_benchmark_shapes(shape, B, ctx):
     """Decode-kernel logits against the fp32 reference model (not against other kernels), teacher-forced, for the
     GQA groups / hidden sizes / FFN widths of the benchmarked configurations; ctx = 300 exercises more than one
     split-KV chunk per head and the split merge.  Reference: last-token logits within tolerance, as
-    /root/reference/jax_test.py:427-490 does for the real checkpoints."""
+    jax_test.py:427-490 does for the real checkpoints."""
     kw = MEGA_SHAPES[shape]
     cfg = LLaMAConfig(vocab_size=2048, num_hidden_layers=2, max_sequence_length=512, initializer_range=0.02,
                       head_dim=128, **kw)

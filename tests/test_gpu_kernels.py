@@ -195,8 +195,8 @@ def test_gemm_cta_pair(M, N, K_, mode, monkeypatch):
 @pytest.mark.parametrize("M,N,K_,mode", [(16, 4096, 14336, "residual"), (64, 4096, 4096, "plain"),
                                          (9, 6144, 4096, "f32"), (100, 2048, 2048, "swiglu")])
 def test_gemm_small_batch_split_k(M, N, K_, mode):
-    """Few weight-row tiles → the K range is split over the idle SMs; partials are summed in split order by
-    the last arriving split (tickets re-arm themselves), so repeated calls agree bit for bit."""
+    """Few weight-row tiles → the K range is split over the CTAs of a cluster; each sums its share of the partials in rank order, so
+    repeated calls agree bit for bit."""
     x, w = rnd(M, K_, seed=60), rnd(N, K_, scale=0.03, seed=61)
     xd, wd = x.to(DEV), w.to(DEV)
     if mode == "residual":

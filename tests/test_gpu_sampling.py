@@ -1,5 +1,5 @@
 """Exact full-vocabulary sampler (csrc/sample_full.cu) against the fp32 statement of the HF warper pipeline the
-reference configures in /root/reference/jax_llama/generation.py:28-41 (temperature → top-k → top-p → categorical)."""
+reference configures in jax_llama/generation.py:28-41 (temperature → top-k → top-p → categorical)."""
 import pytest
 import torch
 
@@ -43,7 +43,7 @@ def test_constant_logits_top_k_keeps_the_lowest_indices():
                                                            (0, 0.5, 1.0, 0.3)])
 def test_samples_stay_inside_the_exact_nucleus_and_follow_its_distribution(top_k, top_p, temperature, scale):
     """No candidate budget: `top_k=None` is the nucleus over the whole vocabulary (flat logits keep tens of thousands of
-    tokens), top_k = 100 / 1000 exceed round 1's 64-candidate limit."""
+    tokens), top_k = 100 / 1000 exceed any small candidate list."""
     g = torch.Generator().manual_seed(2)
     x = torch.randn(V, generator=g) * scale
     order, p = kept_set(x, temperature, top_k, top_p)

@@ -91,7 +91,7 @@ def test_example_cli_end_to_end_on_cpu(tmp_path, spm_model):
 
 def test_reference_arm_runner_with_a_stubbed_reference(tmp_path, monkeypatch):
     """The runner drives the reference's own API (mesh → FlaxLLaMAForCausalLM(_do_init=False) → partition spec →
-    LLaMA.generate, /root/reference/jax_example.py:10-31).  jax and flax are not installable here, so the API is stubbed:
+    LLaMA.generate, jax_example.py:10-31).  jax and flax are not installable here, so the API is stubbed:
     the test pins the call sequence and the JSON contract, and that decode time is the difference of two generate calls."""
     import textwrap
     import types

@@ -1,4 +1,4 @@
-"""Unit parity tests mirroring /root/reference/jax_test.py:73-413 (same tiny config, random trials,
+"""Unit parity tests mirroring jax_test.py:73-413 (same tiny config, random trials,
 atol 1e-2 — we hold 1e-4 because both sides are fp32 PyTorch) plus the gaps SURVEY §4 lists."""
 import math
 

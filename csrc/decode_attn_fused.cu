@@ -679,11 +679,11 @@ extern "C" JL_API int jl_decode_attn_fused(const void* qkv, void* k_cache, void*
   p.vec = (uintptr_t)scratch % 16 == 0 && (uintptr_t)out % 8 == 0;
   auto s = (cudaStream_t)stream;
   cudaError_t e = cudaErrorInvalidValue;
-  // The tensor-core kernel, but for one query head per kv head over a cache of at most 128 slots, where the ring and the
-  // 16-row products have nothing to share and the SIMT kernel's shorter start wins (2.8 vs 3.7 us at 4 heads of 128 and 128 slots, 5.1 vs 3.7
-  // at 160).  Everywhere else it
-  // was the slower one of the two: 20 vs 9.1 us (1 x 8 heads, 4000 keys), 3.4 vs 4.8 (3 x 4 heads of 64, 100 keys), 52
-  // vs 15.7 (16 x 8 heads of 64, 2500 keys), 193 vs 64 (24 x 8 heads, 4000 keys).
+  // The tensor-core kernel, but for one query head per kv head over a cache of at most 128 slots, where the ring and the 16-row products have
+  // nothing to share and the SIMT kernel's shorter start wins (SIMT and this one, us in a graph: 4 heads of 128, 128 slots 2.8 and 3.7, of 64
+  // 2.3 and 2.8; at 160 slots 5.3 and 3.7, 4.9 and 2.9).  Everywhere else it is the faster one: 3 x 4 heads of 64, 100 keys, two query heads
+  // each 3.1 and 2.8, four 3.4 and 3.0; 1 x 8 heads, 4000 keys 20 and 9.1; 16 x 8 heads of 64, 2500 keys 52 and 15.7; 24 x 8 heads, 4000 keys 193
+  // and 64.
   const bool use_mma = (hd == 128 || hd == 64) && (g_attn_variant == 2 || (g_attn_variant == 0 && !(G == 1 && T <= 128)));
   if (use_mma) {
     static int sms = 0;

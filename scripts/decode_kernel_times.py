@@ -2,9 +2,9 @@
 `ncu --metrics gpu__time_duration.sum --csv` so that every kernel of a decode step gets its own duration:
 
     python scripts/decode_kernel_times.py                       # plain run (must exit 0 first)
-    ncu --metrics gpu__time_duration.sum --clock-control none --csv --log-file gpurun_out/kt.csv \
+    ncu --metrics gpu__time_duration.sum --clock-control none --csv --log-file kt.csv \
         python scripts/decode_kernel_times.py
-    python scripts/decode_kernel_times.py --summarise gpurun_out/kt.csv
+    python scripts/decode_kernel_times.py --summarise kt.csv
 
 The prompt is short (the prefill is not the subject); the cache length is set with --context so that the attention
 kernel reads as much K/V as in the benchmark.  ncu serialises the kernels: the sum is an upper bound of the step."""

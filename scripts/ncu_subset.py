@@ -1,6 +1,6 @@
 """`ncu -i REPORT --page raw --csv` → a small CSV with the columns the profiles/ summaries quote.
 
-usage: python scripts/ncu_subset.py gpurun_out/x.ncu-rep profiles/r2/ncu/x_raw_subset.csv [kernel-name-substring]
+usage: python scripts/ncu_subset.py x.ncu-rep profiles/r2/ncu/x_raw_subset.csv [kernel-name-substring]
 """
 import csv
 import subprocess

@@ -7,18 +7,15 @@
 //   * persistent: one CTA per SM walks the tile list, A-tile index fastest so CTAs that run together
 //     share the same weight tile through L2.
 //
-// Two orientations share the kernel:
-//   normal  (prefill, M >= 128): A = activations [M,K], B = weights [N,K]; D tile rows are tokens;
-//   swap-AB (decode, 8 < M <= 128): A = weights [N,K] (fills the 128-wide MMA M), B = activations
-//           [M,K] (MMA N = padded batch); the D tile is transposed on the way out.
+// A = activations [M,K], B = weights [N,K]; D tile rows are tokens (prefill).  With few tokens the weights take the MMA's rows
+// instead (gemm_swap.cu).
 // Epilogues: plain bf16 / fp32, residual add, SwiGLU over interleaved (w1,w3) output columns.
 //
 // Replaces the cuBLAS GEMMs XLA emitted for jax_llama/model.py:119-150 (wq/wk/wv/wo),
 // :311-338 (w1/w2/w3) and :699-706 (lm_head).
 #include <stdlib.h>
 
-#include <atomic>
-
+#include "gemm_swap.cuh"
 #include "jllama_b200.h"
 #include "tcgen05.cuh"
 
@@ -40,11 +37,6 @@ struct GemmParams {
   int a_blocks, b_blocks;   // tile counts
   int stages;
   uint64_t hint_a, hint_b;
-  // ---- split-K for swap-AB launches with fewer weight-row tiles than SMs (decode and short prompts: N = 4096 gives 32 tiles, i.e. 22 %
-  // of the SMs streaming): the CTAs of a cluster of `ksplit` share a tile, each takes a part of its K, the fp32 partials meet in
-  // distributed shared memory and each CTA sums its share of the tokens in rank order — deterministic, no scratch in global memory and
-  // nothing that launches on other streams could share — and runs the epilogue.  ksplit == 1: off.
-  int ksplit;
   unsigned long long* trace;         // optional [grid][16] %globaltimer stamps (jl_gemm_set_trace), NULL = off
   // ---- grouped B operand (normal orientation only): the B tensor holds `groups` matrices of group_rows rows one after
   // the other and A-tile a uses matrix tile_group[a] (< 0: a padding tile, any matrix will do — nobody reads its rows).
@@ -67,21 +59,8 @@ __device__ __forceinline__ void gemm_stamp(const GemmParams& p, int ev) {
   }
 }
 
-__device__ __forceinline__ void gemm_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void gemm_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ uint32_t gemm_mapa(uint32_t local_addr, int rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ float gemm_ld_cluster(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-
-template <int BN, int EPI, bool SWAP, bool OUT_F32>
-__global__ void __launch_bounds__(GEMM_THREADS, SWAP ? 2 : 1)
+template <int BN, int EPI, bool OUT_F32>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   constexpr uint32_t A_BYTES = GEMM_BM * GEMM_BK * 2;
@@ -103,11 +82,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_kb = (p.K + GEMM_BK - 1) / GEMM_BK;
-  const int ksplit = SWAP ? p.ksplit : 1;
 
-  // swap-AB (decode): the next kernel of the chain may start right away — it waits for this grid itself before it
-  // touches anything this grid writes — so that ITS weight prefetch (below) overlaps our epilogue
-  if constexpr (SWAP) pdl_launch_dependents();
   if (threadIdx.x == 0) gemm_stamp(p, 0);
   if (warp == 0 && lane == 0) {
     tc::prefetch_tensormap(&tmap_a);
@@ -126,59 +101,32 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   if (threadIdx.x == 0) gemm_stamp(p, 1);
 
   int a_blocks = p.a_blocks;
-  if constexpr (!SWAP) {
-    pdl_wait();               // everything above overlapped the previous kernel's tail
-    pdl_launch_dependents();
-    if (p.a_blocks_used != nullptr) {                     // one value for every thread of the grid: all roles walk the same list
-      const int used = *p.a_blocks_used;
-      a_blocks = used < 1 ? 1 : (used < a_blocks ? used : a_blocks);
-    }
+  pdl_wait();                 // everything above overlapped the previous kernel's tail
+  pdl_launch_dependents();
+  if (p.a_blocks_used != nullptr) {                       // one value for every thread of the grid: all roles walk the same list
+    const int used = *p.a_blocks_used;
+    a_blocks = used < 1 ? 1 : (used < a_blocks ? used : a_blocks);
   }
   const int num_tiles = a_blocks * p.b_blocks;
-  const int num_work = num_tiles * ksplit;              // (tile, K split) items; the splits of a tile are the CTAs of a cluster
 
   if (warp == 0) {
     // ===================================================== TMA producer
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
-      int pre = 0;            // leading k-blocks of the first item whose weight tile is already on its way
-      if constexpr (SWAP) {
-        // the weights do not depend on the previous kernel: fill the ring with A tiles NOW — they stream from HBM
-        // while that kernel runs its tail — and only then wait for it; the activation tiles follow after the wait
-        if ((int)blockIdx.x < num_work) {
-          const int t = blockIdx.x / ksplit, split = blockIdx.x % ksplit;
-          const int kb0 = split * num_kb / ksplit, kb1 = (split + 1) * num_kb / ksplit;
-          const int a_blk = t % a_blocks;
-          pre = kb1 - kb0 < stages ? kb1 - kb0 : stages;
-          for (int i = 0; i < pre; ++i) {
-            tc::mbar_expect_tx(full_bar(i), A_BYTES + B_BYTES);
-            tc::tma_load_2d(smem_base + i * STAGE_BYTES, &tmap_a, full_bar(i), (kb0 + i) * GEMM_BK, a_blk * GEMM_BM, p.hint_a);
-          }
-        }
-        pdl_wait();
-      }
       gemm_stamp(p, 2);
-      for (int wi = blockIdx.x; wi < num_work; wi += gridDim.x) {
-        const int t = wi / ksplit, split = wi % ksplit;
-        const int kb0 = split * num_kb / ksplit, kb1 = (split + 1) * num_kb / ksplit;
+      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const int b_blk = t / a_blocks;
         const int a_blk = t % a_blocks;
         int b_row = b_blk * BN;
-        if constexpr (!SWAP) {
-          if (p.tile_group != nullptr) {
-            const int e = p.tile_group[a_blk];
-            b_row += (e < 0 ? 0 : e) * p.group_rows;
-          }
+        if (p.tile_group != nullptr) {
+          const int e = p.tile_group[a_blk];
+          b_row += (e < 0 ? 0 : e) * p.group_rows;
         }
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           const uint32_t sa = smem_base + stage * STAGE_BYTES, sb = sa + A_BYTES;
-          if (pre > 0) {
-            --pre;
-          } else {
-            tc::mbar_wait(empty_bar(stage), phase ^ 1);
-            tc::mbar_expect_tx(full_bar(stage), A_BYTES + B_BYTES);
-            tc::tma_load_2d(sa, &tmap_a, full_bar(stage), kb * GEMM_BK, a_blk * GEMM_BM, p.hint_a);
-          }
+          tc::mbar_wait(empty_bar(stage), phase ^ 1);
+          tc::mbar_expect_tx(full_bar(stage), A_BYTES + B_BYTES);
+          tc::tma_load_2d(sa, &tmap_a, full_bar(stage), kb * GEMM_BK, a_blk * GEMM_BM, p.hint_a);
           tc::tma_load_2d(sb, &tmap_b, full_bar(stage), kb * GEMM_BK, b_row, p.hint_b);
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
@@ -188,22 +136,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     // ===================================================== MMA issuer (single thread)
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0; int it = 0;
-      for (int wi = blockIdx.x; wi < num_work; wi += gridDim.x, ++it) {
-        const int split = wi % ksplit;
-        const int kb0 = split * num_kb / ksplit, kb1 = (split + 1) * num_kb / ksplit;
+      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
         const int as = it & 1; const uint32_t aphase = (it >> 1) & 1;
         tc::mbar_wait(tempty_bar(as), aphase ^ 1);          // epilogue has drained this accumulator
         tc::fence_after_sync();
         const uint32_t d_tmem = tmem_base + as * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           tc::mbar_wait(full_bar(stage), phase);
           tc::fence_after_sync();
-          if (it == 0 && kb == kb0) gemm_stamp(p, 3);
+          if (it == 0 && kb == 0) gemm_stamp(p, 3);
           const uint32_t sa = smem_base + stage * STAGE_BYTES, sb = sa + A_BYTES;
           const uint64_t da = tc::smem_desc_kmajor_sw128(sa), db = tc::smem_desc_kmajor_sw128(sb);
 #pragma unroll
           for (int k = 0; k < GEMM_BK / 16; ++k)            // +32 bytes per UMMA_K inside the swizzle span
-            tc::mma_ss(d_tmem, da + 2 * k, db + 2 * k, IDESC, kb != kb0 || k != 0);
+            tc::mma_ss(d_tmem, da + 2 * k, db + 2 * k, IDESC, kb != 0 || k != 0);
           tc::mma_commit(empty_bar(stage));                 // frees the smem slot when these MMAs retire
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
@@ -215,9 +161,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     // ===================================================== epilogue: TMEM → registers → global
     const int quarter = warp & 3;                           // TMEM lanes [32·quarter, 32·quarter+32)
     int it = 0;
-    if constexpr (SWAP) pdl_wait();                         // residual, output: after the previous kernel
-    for (int wi = blockIdx.x; wi < num_work; wi += gridDim.x, ++it) {
-      const int t = wi / ksplit, split = wi % ksplit;
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
       const int b_blk = t / a_blocks;
       const int a_blk = t % a_blocks;
       const int as = it & 1; const uint32_t aphase = (it >> 1) & 1;
@@ -227,26 +171,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int ra = a_blk * GEMM_BM + quarter * 32 + lane;  // A-side row of this thread
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + as * BN;
       constexpr int CH = BN >= 32 ? 32 : 16;
-      // swap-AB epilogue of one (token, feature = this lane's weight row) value; whole warps call it together
-      // rpre: the residual value when the caller already holds it (split-K finish), else it is loaded here
-      auto swap_emit = [&](const int tok, float x, const bool pre = false, const float rpre = 0.f) {
-        if constexpr (EPI == EPI_SWIGLU) {
-          // (gate, up) sit in adjacent lanes: even lane gets its neighbour's value
-          const float xb = __bfloat162float(__float2bfloat16(x));
-          const float up = __shfl_down_sync(0xffffffffu, xb, 1);
-          if ((lane & 1) == 0 && tok < p.Rb && ra + 1 < p.Ra)
-            reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)tok * p.ldo + ra / 2] = __float2bfloat16(silu(xb) * up);
-        } else if (tok < p.Rb && ra < p.Ra) {
-          if constexpr (OUT_F32) {
-            reinterpret_cast<float*>(p.out)[(size_t)tok * p.ldo + ra] = x;
-          } else {
-            if constexpr (EPI == EPI_RESIDUAL)
-              x = __bfloat162float(__float2bfloat16(x)) +
-                  (pre ? rpre : __bfloat162float(p.residual[(size_t)tok * p.ldo + ra]));
-            reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)tok * p.ldo + ra] = __float2bfloat16(x);
-          }
-        }
-      };
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += CH) {
         uint32_t v[CH];
@@ -254,7 +178,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         else tc::tmem_ld16(t_row + c0, reinterpret_cast<uint32_t(&)[16]>(v));
         tc::tmem_ld_wait();
         const int cb0 = b_blk * BN + c0;                    // first B-side row of this chunk
-        if constexpr (!SWAP) {
+        {
           // thread owns one token row, CH consecutive output columns
           if (ra < p.Ra) {
             if constexpr (EPI == EPI_SWIGLU) {
@@ -323,73 +247,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
               }
             }
           }
-        } else {
-          // swap-AB: lanes are weight rows (output features), columns are tokens
-          if (ksplit > 1) {
-            // fp32 partial of this K split, [token][feature] in shared memory: the ring is free (one work item per CTA, all its MMAs done)
-            const uint32_t part = smem_base + (uint32_t)(c0 * GEMM_BM + quarter * 32 + lane) * 4;
-#pragma unroll
-            for (int j = 0; j < CH; ++j) asm volatile("st.shared.b32 [%0], %1;" ::"r"(part + j * (GEMM_BM * 4)), "r"(v[j]) : "memory");
-          } else {
-            // transposed store: for a fixed token the 32 lanes write 32 consecutive features (coalesced)
-#pragma unroll
-            for (int j = 0; j < CH; ++j) swap_emit(cb0 + j, __uint_as_float(v[j]));
-          }
         }
       }
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(tempty_bar(as));
-      if constexpr (SWAP) {
-        if (ksplit > 1) {
-          // ---- split-K finish: once all partials of the cluster are there, every CTA sums and emits ITS share of the tile's tokens
-          if (threadIdx.x == 128) gemm_stamp(p, 6);
-          gemm_cluster_arrive();
-          gemm_cluster_wait();
-          if (threadIdx.x == 128) gemm_stamp(p, 7);
-          const uint32_t part = smem_base + (uint32_t)(quarter * 32 + lane) * 4;
-          const int per = ((BN + ksplit - 1) / ksplit + 3) & ~3, j_hi = split * per + per < BN ? split * per + per : BN;
-          for (int j0 = split * per; j0 < j_hi; j0 += 4) {
-            float rr[4] = {0.f, 0.f, 0.f, 0.f};
-            if constexpr (EPI == EPI_RESIDUAL) {
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const int tok = b_blk * BN + j0 + u;
-                if (tok < p.Rb && ra < p.Ra) rr[u] = __bfloat162float(p.residual[(size_t)tok * p.ldo + ra]);
-              }
-            }
-            float x[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-            for (int sp0 = 0; sp0 < ksplit; sp0 += 8) {   // eight ranks' four tokens in flight; a warp reads 128 bytes of a rank
-              float q[8][4];
-#pragma unroll
-              for (int sp = 0; sp < 8; ++sp)
-                if (sp0 + sp < ksplit) {
-                  const uint32_t at = gemm_mapa(part + j0 * (GEMM_BM * 4), sp0 + sp);
-#pragma unroll
-                  for (int u = 0; u < 4; ++u) q[sp][u] = gemm_ld_cluster(at + u * (GEMM_BM * 4));
-                }
-#pragma unroll
-              for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int sp = 0; sp < 8; ++sp) if (sp0 + sp < ksplit) x[u] += q[sp][u];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) swap_emit(b_blk * BN + j0 + u, x[u], true, rr[u]);
-          }
-          if (threadIdx.x == 128) gemm_stamp(p, 8);
-        }
-      }
     }
   }
 
-  if constexpr (SWAP) {
-    if (ksplit > 1) {
-      if (warp < 4) { gemm_cluster_arrive(); gemm_cluster_wait(); }     // (the epilogue warps passed this barrier above)
-      gemm_cluster_arrive();                              // no CTA leaves while its partial may still be read
-      gemm_cluster_wait();
-    }
-  }
   tc::fence_before_sync();
   __syncthreads();
   if (threadIdx.x == 0) gemm_stamp(p, 9);
@@ -398,48 +263,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
 static unsigned long long* g_gemm_trace = nullptr;
 
-// whether the caller allows split-K on a device (jl_gemm_set_workspace)
-static bool g_splitk[16] = {};
-static bool splitk_allowed() {
-  int dev = 0;
-  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 16 && g_splitk[dev];
-}
-
 constexpr uint32_t gemm_stage_bytes(int bn) { return GEMM_BM * GEMM_BK * 2 + (bn * GEMM_BK * 2 < 1024 ? 1024 : bn * GEMM_BK * 2); }
-constexpr int GEMM_SPLIT_RING = 100 * 1024;               // ring of a split-K launch: two CTAs of neighbouring kernels fit an SM
 constexpr size_t gemm_smem(int stages, int bn) { return (size_t)stages * gemm_stage_bytes(bn) + 8 * (2 * stages + 4) + 16 + 1024; }
 
-// whether the device holds clusters of `ks` > 8 CTAs of the split-K kernel (asked once per device, kernel and size)
 template <int BN, int EPI, bool OUT_F32>
-static bool wide_clusters(int ks, int num_sms) {
-  static std::atomic<signed char> known[16][17];          // 0: not asked yet
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return false;
-  signed char v = known[dev][ks].load(std::memory_order_relaxed);
-  if (v == 0) {
-    auto kern = gemm_kernel<BN, EPI, true, OUT_F32>;
-    int n = 0, stages = (int)(GEMM_SPLIT_RING / gemm_stage_bytes(BN));
-    if (stages > 10) stages = 10;
-    const size_t smem = gemm_smem(stages, BN);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(num_sms / ks * ks);
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-                    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                    cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1;
-    if (!ok) cudaGetLastError();
-    v = ok ? 1 : -1;
-    known[dev][ks].store(v, std::memory_order_relaxed);
-  }
-  return v > 0;
-}
-
-template <int BN, int EPI, bool SWAP, bool OUT_F32>
 static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int Ra, int Rb, int K, int num_sms,
                        cudaStream_t stream, int b_matrices = 1) {
   GemmParams p = p0;
@@ -454,80 +281,27 @@ static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int R
   p.a_blocks = (Ra + GEMM_BM - 1) / GEMM_BM;
   p.b_blocks = (Rb + BN - 1) / BN;
   int grid = p.a_blocks * p.b_blocks;
-  p.ksplit = 1;
-  if constexpr (SWAP) {
-    // few weight-row tiles (N <= ~9k): cut K so that (nearly) every SM streams weights, at least 4 k-blocks (256 columns) per CTA
-    if (grid * 2 <= num_sms && splitk_allowed()) {
-      int ks = num_sms / grid;
-      if (ks > num_kb / 4) ks = num_kb / 4;
-      // Eight CTAs are what every GPU takes as a cluster.  More pay with a long K over few weight tiles (9 to 16 rows of 1024 x 14336: 8 parts
-      // 11.8 us, 16 parts 10.1; 1536 x 14336 12.8 and 12.0 in 12 parts); at K 8192 and below, and with less than half as many again, the
-      // wider meeting costs what it gives or more (1024 x 4096 5.8 and 5.9 us, 64 rows 7.8 and 8.5; 2048 x 14336, 9 parts, 13.7 and 14.1).
-      if (ks > 16) ks = 16;
-      if (ks > 8 && (ks < 12 || num_kb <= 128 || !wide_clusters<BN, EPI, OUT_F32>(ks, num_sms))) ks = 8;
-      if (ks > 1) {
-        p.ksplit = ks;
-        grid *= ks;
-      }
-    }
-  }
   if (grid > num_sms) grid = num_sms;
-  // Ring depth.  Token-major GEMMs and long weight streams (> 1.25 MB per CTA: w13, lm_head) take the whole shared
-  // memory (10 stages).  Short decode GEMMs (wqkv, wo, w2 at batch 9..128) stay under half of it, so that the CTAs of
-  // the NEXT kernel of the chain fit on the same SM and their weight prefetch — issued before they wait for this
-  // grid — runs under our epilogue and split-K finish; those prologue / tail latencies were most of a 25 us GEMM.
-  // A split-K launch always takes the small ring too (its partial tile, at most 64 KB, fits).
-  int budget = 200 * 1024;
-  if (SWAP && (p.ksplit > 1 || (size_t)Ra * K * 2 / grid <= (size_t)1280 * 1024)) budget = GEMM_SPLIT_RING;
+  const int budget = 200 * 1024;
   int stages = (int)(budget / STAGE_BYTES);
   if (stages > 10) stages = 10;
   if (stages > num_kb * 2) stages = num_kb * 2 < 2 ? 2 : num_kb * 2;
   p.stages = stages;
   const size_t smem = gemm_smem(stages, BN);
-  auto kern = gemm_kernel<BN, EPI, SWAP, OUT_F32>;
+  auto kern = gemm_kernel<BN, EPI, OUT_F32>;
   JL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (p.ksplit == 1) {
-    JL_CUDA(launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS), smem, stream, ta, tb, p));
-    return JL_OK;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(GEMM_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = p.ksplit;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  count_launch();
-  JL_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
+  JL_CUDA(launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS), smem, stream, ta, tb, p));
   return JL_OK;
 }
 
 template <int EPI, bool OUT_F32>
 static int dispatch_gemm(const void* x, const void* w, const GemmParams& p, int M, int N, int K, int num_sms,
                          cudaStream_t s) {
-  if (M > 128) {
-    // normal orientation: A = activations, B = weights
-    GemmParams q = p;
-    q.Ra = M; q.Rb = N;
-    q.hint_a = tc::EVICT_LAST; q.hint_b = tc::EVICT_NORMAL;
-    if (N >= 256) return launch_gemm<256, EPI, false, OUT_F32>(x, w, q, M, N, K, num_sms, s);
-    return launch_gemm<128, EPI, false, OUT_F32>(x, w, q, M, N, K, num_sms, s);
-  }
-  // swap-AB: A = weights (streamed once → evict-first), B = activations (re-read by every CTA)
   GemmParams q = p;
-  q.Ra = N; q.Rb = M;
-  q.hint_a = tc::EVICT_FIRST; q.hint_b = tc::EVICT_LAST;
-  if (M <= 16) return launch_gemm<16, EPI, true, OUT_F32>(w, x, q, N, M, K, num_sms, s);
-  if (M <= 32) return launch_gemm<32, EPI, true, OUT_F32>(w, x, q, N, M, K, num_sms, s);
-  if (M <= 64) return launch_gemm<64, EPI, true, OUT_F32>(w, x, q, N, M, K, num_sms, s);
-  return launch_gemm<128, EPI, true, OUT_F32>(w, x, q, N, M, K, num_sms, s);
+  q.Ra = M; q.Rb = N;
+  q.hint_a = tc::EVICT_LAST; q.hint_b = tc::EVICT_NORMAL;
+  if (N >= 256) return launch_gemm<256, EPI, OUT_F32>(x, w, q, M, N, K, num_sms, s);
+  return launch_gemm<128, EPI, OUT_F32>(x, w, q, M, N, K, num_sms, s);
 }
 
 }  // namespace jl
@@ -546,7 +320,7 @@ extern "C" JL_API int jl_gemm_set_workspace(void* ws, size_t ws_bytes, int* tick
   JL_CUDA(cudaGetDevice(&dev));
   JL_CHECK_ARG(dev >= 0 && dev < 16, "jl_gemm_set_workspace: device %d out of range", dev);
   (void)ws_bytes; (void)tickets; (void)n_tickets;
-  g_splitk[dev] = ws != nullptr;
+  gemm_swap_allow_split(dev, ws != nullptr);
   return JL_OK;
 }
 
@@ -565,6 +339,7 @@ extern "C" JL_API int jl_gemm(const void* x, const void* w, const void* residual
   p.K = K;
   p.ldo = mode == EPI_SWIGLU ? N / 2 : N;
   auto s = (cudaStream_t)stream;
+  if (gemm_swap_takes(M, N, K, num_sms)) return gemm_swap(x, w, residual, out, M, N, K, mode, out_f32 != 0, num_sms, g_gemm_trace, s);
   // token-major tiles of the prefill shapes go to the CTA-pair kernel (cta_group::2, gemm_2cta.cu); JLLAMA_GEMM_2CTA=0
   // keeps everything on the single-CTA kernel below (A/B measurements)
   static const bool pair_on = [] { const char* e = getenv("JLLAMA_GEMM_2CTA"); return !(e && e[0] == '0'); }();
@@ -602,9 +377,9 @@ extern "C" JL_API int jl_gemm_grouped(const void* x, const void* w, void* out, i
   p.a_blocks_used = tiles_used;
   auto s = (cudaStream_t)stream;
   if (out_f32) {
-    if (N >= 256) return launch_gemm<256, EPI_PLAIN, false, true>(x, w, p, M, N, K, num_sms, s, groups);
-    return launch_gemm<128, EPI_PLAIN, false, true>(x, w, p, M, N, K, num_sms, s, groups);
+    if (N >= 256) return launch_gemm<256, EPI_PLAIN, true>(x, w, p, M, N, K, num_sms, s, groups);
+    return launch_gemm<128, EPI_PLAIN, true>(x, w, p, M, N, K, num_sms, s, groups);
   }
-  if (N >= 256) return launch_gemm<256, EPI_PLAIN, false, false>(x, w, p, M, N, K, num_sms, s, groups);
-  return launch_gemm<128, EPI_PLAIN, false, false>(x, w, p, M, N, K, num_sms, s, groups);
+  if (N >= 256) return launch_gemm<256, EPI_PLAIN, false>(x, w, p, M, N, K, num_sms, s, groups);
+  return launch_gemm<128, EPI_PLAIN, false>(x, w, p, M, N, K, num_sms, s, groups);
 }

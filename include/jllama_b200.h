@@ -56,18 +56,18 @@ int jl_gemv_tma(const void* x, const void* w, const void* norm_w, const void* re
                 int K, float eps, int mode, int out_f32, int num_sms, void* stream);
 
 /* Same linear layers for any M on the tcgen05 tensor cores (TMA-fed, TMEM accumulators).  M > 128 runs
- * token-major tiles (prefill); M <= 128 runs swap-AB so the weight rows fill the 128-wide MMA and the
- * batch is the MMA N (decode at batch 9..128).  Modes / out_f32 as in jl_gemv.  N % 8 == 0, K % 8 == 0;
+ * token-major tiles (prefill); M <= 128, and M <= 256 with few weight rows, runs swap-AB so the weight rows fill the
+ * 128-wide MMA and the batch is the MMA N (decode, short prompts).  Modes / out_f32 as in jl_gemv.  N % 8 == 0, K % 8 == 0;
  * SwiGLU needs N % 16 == 0. */
 int jl_gemm(const void* x, const void* w, const void* residual, void* out, int M, int N, int K, int mode,
             int out_f32, int num_sms, void* stream);
-/* Allows split-K in jl_gemm on the CURRENT device (ws != NULL; NULL forbids it): small-batch (M <= 128) launches that have fewer
- * 128-row weight tiles than half the SMs (N = 4096: 32 tiles) then split K over the CTAs of a cluster; partial sums meet in
+/* Allows split-K in jl_gemm on the CURRENT device (ws != NULL; NULL forbids it): launches of few tokens with fewer
+ * 128-row weight tiles than SMs (N = 4096: 32 tiles) then split K over the CTAs of a cluster; partial sums meet in
  * distributed shared memory, each CTA adds the partials of its share of the tokens in rank order and runs the epilogue —
  * results do not depend on timing.  The buffers themselves are not used. */
 int jl_gemm_set_workspace(void* ws, size_t ws_bytes, int* tickets, int n_tickets);
-/* Timeline hook of the single-CTA GEMM kernel for scripts/gemm_trace.py: [grid][16] u64 device buffer of
- * %globaltimer stamps, NULL = off (default). */
+/* Timeline hook of the few-token and the single-CTA GEMM kernel for scripts/gemm_trace.py: [num_sms][16] u64 device buffer of
+ * %globaltimer stamps of the first num_sms CTAs, NULL = off (default). */
 void jl_gemm_set_trace(void* buf);
 
 /* model.py:194-198,263-288 at S=1 — split-KV GQA decode attention over [pad_left[b], *cache_len+n_new).

@@ -1,0 +1,59 @@
+"""The few-token GEMM (weights as the MMA's rows) at the edges of its tiles: token counts around multiples of 16 and its limits, ragged weight
+rows and K, one tile, more tiles than two CTAs per SM hold at once, split and unsplit, outputs at any element."""
+import pytest
+import torch
+
+from jax_llama_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _inputs(M, N, Kd, seed):
+    g = torch.Generator().manual_seed(seed)
+    x, w, r = (torch.randn(s, generator=g).bfloat16() for s in ((M, Kd), (N, Kd), (M, N)))
+    return x, (w.float() * Kd ** -0.5).bfloat16(), r
+
+
+def _check(M, N, Kd, mode, shift=0):
+    """Sums of K products in fp32, one rounding to bfloat16 per stored or intermediate value (2^-9 of it each, at most three in a row)."""
+    K.ensure_gemm_workspace(torch.device(DEV))
+    x, w, r = _inputs(M, N, Kd, M + N + Kd)
+    xd, wd, rd = x.to(DEV), w.to(DEV), r.to(DEV)
+    want = K.linear(xd.float().cpu().bfloat16(), w, residual=r if mode == "residual" else None, out_f32=mode == "f32",
+                    mode={"residual": K.RESIDUAL, "swiglu": K.SWIGLU}.get(mode, K.PLAIN)).float()
+    cols, dt = N // 2 if mode == "swiglu" else N, torch.float32 if mode == "f32" else torch.bfloat16
+    buf = torch.full((M * cols + shift + 64,), 7.0, dtype=dt, device=DEV)
+    out = buf[shift:shift + M * cols].view(M, cols)
+    args = dict(out_f32=mode == "f32", out=out, force="gemm", mode={"residual": K.RESIDUAL, "swiglu": K.SWIGLU}.get(mode, K.PLAIN))
+    if mode == "residual":
+        args["residual"] = rd
+    K.linear(xd, wd, **args)
+    got = out.float().cpu()
+    bound = 1e-5 + (0.0 if mode == "f32" else 3 * 2.0 ** -8) * want.abs() + (2e-5 if mode == "f32" else 3 * 2.0 ** -8)
+    assert bool(((got - want).abs() <= bound).all()), float((got - want).abs().max())
+    assert bool((buf[:shift] == 7.0).all()) and bool((buf[shift + M * cols:] == 7.0).all())
+    first = out.clone()
+    K.linear(xd, wd, **args)
+    assert torch.equal(first, out)
+
+
+@pytest.mark.parametrize("M", [5, 16, 17, 48, 49, 100, 112, 113, 128, 129, 160, 255, 256])
+@pytest.mark.parametrize("N,Kd,mode", [(1000, 520, "plain"), (2048, 1024, "residual"), (4096, 2112, "swiglu"), (136, 256, "f32"),
+                                       (11008, 4096, "plain")])
+def test_token_counts(M, N, Kd, mode):
+    _check(M, N, Kd, mode)
+
+
+@pytest.mark.parametrize("M", [9, 33, 128])
+@pytest.mark.parametrize("N,Kd,mode", [(128, 64, "plain"), (8, 8, "f32"), (18944, 192, "swiglu"), (19072, 320, "residual"), (37888, 128, "f32"),
+                                       (38016, 200, "plain"), (50000, 128, "swiglu"), (4096, 16384, "residual"), (14336, 2048, "swiglu")])
+def test_tile_counts(M, N, Kd, mode):
+    _check(M, N, Kd, mode)
+
+
+@pytest.mark.parametrize("shift", [1, 2, 3])
+@pytest.mark.parametrize("M,N,Kd", [(20, 1024, 2048), (20, 40000, 64)])
+@pytest.mark.parametrize("mode", ["plain", "residual", "swiglu", "f32"])
+def test_output_at_any_element(M, N, Kd, mode, shift):
+    _check(M, N, Kd, mode, shift)

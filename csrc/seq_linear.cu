@@ -1,7 +1,8 @@
 // Linear layers for any shape and for bfloat16 or true float32 operands: y = act(x W^T) with W [N, K] (out, in).
 //
-//  * linear_mma_rows_kernel (bfloat16, M = 5 .. 8: decode) — weight-streaming through mma.sync: see there.
-//  * linear_rows_kernel  (M <= 8: fewer tokens, float32, pitches without 16-byte rows) — weight-streaming: a CTA owns ROWS output features, its 8 warps split K, each
+//  * linear_mma_rows_kernel (bfloat16, M = 3 .. 8: decode) — weight-streaming through mma.sync: see there.
+//  * linear_flow_kernel  (bfloat16, M <= 4) — the sums of the next one by CTAs that stay: see there.
+//  * linear_rows_kernel  (M <= 8: float32, pitches without 16-byte rows) — weight-streaming: a CTA owns ROWS output features, its 8 warps split K, each
 //    lane reads 16 bytes of every row per step (all loads issued before the first use) and keeps ROWS x M fp32
 //    accumulators; activations come from L1; the warps' sums meet in shared memory in a fixed order.
 //  * linear_f32_kernel   (float32, M > 8, linear_f32.cu) — tensor cores with the accuracy of fp32 FMAs.
@@ -32,6 +33,16 @@ template <> __device__ __forceinline__ void load_vec<__nv_bfloat16>(const __nv_b
   uint4 t = *reinterpret_cast<const uint4*>(p);
   v[0] = bf16_lo(t.x); v[1] = bf16_hi(t.x); v[2] = bf16_lo(t.y); v[3] = bf16_hi(t.y);
   v[4] = bf16_lo(t.z); v[5] = bf16_hi(t.z); v[6] = bf16_lo(t.w); v[7] = bf16_hi(t.w);
+}
+
+__device__ __forceinline__ void unpack8(const uint4& t, float (&v)[8]) {
+  v[0] = bf16_lo(t.x); v[1] = bf16_hi(t.x); v[2] = bf16_lo(t.y); v[3] = bf16_hi(t.y);
+  v[4] = bf16_lo(t.z); v[5] = bf16_hi(t.z); v[6] = bf16_lo(t.w); v[7] = bf16_hi(t.w);
+}
+__device__ __forceinline__ uint4 ldg_weights(const void* p) {     // touched once: no line in L1 (the tokens live there)
+  uint4 r;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  return r;
 }
 
 constexpr int LR_WARPS = 8;     // warps of a CTA: they split K for the same LR_ROWS output features
@@ -105,7 +116,118 @@ __global__ void __launch_bounds__(LR_WARPS * 32) linear_rows_kernel(const T* __r
   }
 }
 
-// bfloat16 weights of a decode step of 5 to 8 tokens, streamed once, tokens as the 8 columns of mma.sync.m16n8k16 (products exact,
+// bfloat16, up to 4 tokens, one matrix: the same sums in the same order, but the CTAs stay (FL_CTAS per SM) and walk the groups of four output
+// features, the next group's (or next 2048 k's) weights already on their way into registers while this one is multiplied; and where the
+// weights are known to be a parameter the first ones are requested BEFORE the wait for the kernels ahead.  Bound: the weights' way from
+// memory; a CTA per group spends itself on coming and going where K is short (one load round each).
+// One B200, us in a chain of cold weights, linear_rows_kernel -> this -> this with the early request (features x K): 1 token 2048 x 2048 3.9 -> 3.4 ->
+// 2.4, 8192 x 2048 9.1 -> 8.6 -> 7.6, 32000 x 2048 27.4 -> 26.1 -> 25.0, 2048 x 8192 8.7 -> 7.8 -> 6.9, 4096 x 14336 24.9 -> 22.1 -> 21.2 (5.5 TB/s); 2 tokens 2048 x 2048
+// 3.9 -> 4.0 -> 2.8, 8192 x 2048 9.8 -> 10.5 -> 9.2; 2 tokens with more k stay with linear_rows_kernel (4096 x 14336 21.4 against 25.5: more CTAs to hide a
+// round behind).  3 and 4 tokens: what linear_mma_rows_kernel leaves (4 tokens 2048 x 2048 5.8 -> 5.4 -> 4.2,
+// 2048 x 1024 4.6 -> 4.4 -> 3.6).
+constexpr int fl_ctas(int m) { return m <= 2 ? 4 : 3; }          // per SM
+
+template <typename OutT, int M>
+__global__ void __launch_bounds__(LR_WARPS * 32, fl_ctas(M)) linear_flow_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
+                                                                    const __nv_bfloat16* __restrict__ w, OutT* __restrict__ out, int ldo,
+                                                                    int N, int K, int act, float p0, float p1, int early) {
+  constexpr int NV = M == 3 ? 16 : 4 * M, STEP = LR_WARPS * 32 * 8;       // sums of a thread, to a power of two; k of a round
+  __shared__ float red[2][LR_WARPS][NV];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int groups = (N + LR_ROWS - 1) / LR_ROWS, steps = (K + STEP - 1) / STEP;
+  int g = blockIdx.x, s = 0;                               // the round that is loaded
+  uint4 wv[LR_ROWS];
+  auto load = [&](int gl, int sl) {
+    const int k = sl * STEP + (int)threadIdx.x * 8;
+    const __nv_bfloat16* row = w + (size_t)gl * LR_ROWS * K + k;
+#pragma unroll
+    for (int r = 0; r < LR_ROWS; ++r)
+      wv[r] = k < K && gl < groups ? ldg_weights(row + (size_t)min(r, N - 1 - gl * LR_ROWS) * K) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  if (early) load(g, 0);
+  pdl_wait();
+  pdl_launch_dependents();
+  if (!early) load(g, 0);
+  float acc[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) acc[i] = 0.0f;
+  int buf = 0;
+  while (g < groups) {
+    const int k = s * STEP + (int)threadIdx.x * 8;
+    uint4 xv[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) xv[m] = k < K ? *reinterpret_cast<const uint4*>(x + (size_t)m * ldx + k) : make_uint4(0u, 0u, 0u, 0u);
+    float wf[LR_ROWS][8];
+#pragma unroll
+    for (int r = 0; r < LR_ROWS; ++r) unpack8(wv[r], wf[r]);
+    const int g0 = g;
+    const bool last = s + 1 == steps;
+    s = last ? 0 : s + 1;
+    if (last) g += gridDim.x;
+    load(g, s);                                            // in flight during everything below
+    if (k < K) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        float xf[8];
+        unpack8(xv[m], xf);
+#pragma unroll
+        for (int r = 0; r < LR_ROWS; ++r)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[r * M + m] = fmaf(wf[r][j], xf[j], acc[r * M + m]);
+      }
+    }
+    if (last) {
+      // fold: at each step a lane keeps half of its sums and gives the other half to its partner (the additions of warp_sum)
+      int idx = 0;
+#pragma unroll
+      for (int o = 16, n = NV; o > 0; o >>= 1) {
+        if (n > 1) {
+          const bool up = (lane & o) != 0;
+          n >>= 1;
+          idx = idx * 2 + (up ? 1 : 0);
+#pragma unroll
+          for (int i = 0; i < NV / 2; ++i)
+            if (i < n) {
+              const float keep = up ? acc[i + n] : acc[i], give = up ? acc[i] : acc[i + n];
+              acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        } else {
+          acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+        }
+      }
+      if ((lane & (32 / NV - 1)) == 0) red[buf][warp][idx] = acc[0];
+      __syncthreads();                                     // (a buffer is written again only after the next one of these)
+      if (threadIdx.x < LR_ROWS * M) {
+        const int r = threadIdx.x / M, m = threadIdx.x % M;
+        float t = 0.0f;
+#pragma unroll
+        for (int wq = 0; wq < LR_WARPS; ++wq) t += red[buf][wq][threadIdx.x];
+        if (g0 * LR_ROWS + r < N) out[(size_t)m * ldo + g0 * LR_ROWS + r] = from_f<OutT>(apply_act(t, act, p0, p1));
+      }
+      buf ^= 1;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) acc[i] = 0.0f;
+    }
+  }
+}
+
+template <typename OutT>
+static int flow_launch(const __nv_bfloat16* x, int ldx, const __nv_bfloat16* w, OutT* out, int ldo, int M, int N, int K, int act, float p0,
+                       float p1, bool early, cudaStream_t st) {
+  const int groups = (N + LR_ROWS - 1) / LR_ROWS;
+#define JL_FL(MM)                                                                                                        \
+  case MM: {                                                                                                             \
+    const int most = 148 * fl_ctas(MM);                                                                          \
+    JL_LAUNCH_PDL((linear_flow_kernel<OutT, MM>), dim3(groups < most ? groups : most), dim3(LR_WARPS * 32), 0, st, x, ldx, w, out, ldo, N, K, act, \
+                  p0, p1, early ? 1 : 0);                                                                                \
+    break;                                                                                                               \
+  }
+  switch (M) { JL_FL(1) JL_FL(2) JL_FL(3) JL_FL(4) }
+#undef JL_FL
+  return cudaGetLastError() == cudaSuccess ? JL_OK : JL_ERR_CUDA;
+}
+
+// bfloat16 weights of a decode step of 3 to 8 tokens, streamed once, tokens as the 8 columns of mma.sync.m16n8k16 (products exact,
 // fp32 sums).  A warp takes 16 output features and one of KS parts of K in batches of 256 k: lane (g = lane / 4, t = lane % 4) loads the
 // 16-byte chunks t, t + 4, ... of rows g and g + 8 straight into A fragments, and the same chunks of token g into B fragments (the order of
 // k inside a product is free as long as both agree: MMA v of chunk u uses words 2v, 2v + 1), so a batch is 16 weight loads in flight
@@ -117,17 +239,14 @@ __global__ void __launch_bounds__(LR_WARPS * 32) linear_rows_kernel(const T* __r
 // with at most LM_MAX_SEG k to a warp, whose batches are added one after the other (32000 features in parts of 2048 k 8.4e-8 -> 8.5e-8, of 4096 8.9e-8
 // -> 10.0e-8).  (Chains of two MMAs: 5 % faster, but 5.4e-8 with operands of one sign at 2048 x 2048.)
 // 8 tokens on one B200, FMA kernel -> this one (features x K; cold L2, launch included): 32000 x 2048 90 -> 37 us, 8192 x 2048 29.5 -> 18.4,
-// 2048 x 8192 22.6 -> 18.3, 2048 x 2048 14.2 -> 10.1.  Up to 4 tokens the FMA kernel, whose loads run along a row (512 contiguous bytes against 64), is
-// as fast or faster (2 tokens: 2048 x 8192 7.9 against 10.5), and with fewer than 96 groups of 16 features too (8 tokens, 1024 x 5464:
-// 7.4 against 8.9: a warp's batches run one after the other).
+// 2048 x 8192 22.6 -> 18.3, 2048 x 2048 14.2 -> 10.1; 4 tokens, in a chain of cold weights: 32000 x 2048 50 -> 26.5, 28672 x 4096 65 -> 44, 8192 x 2048 14.6 -> 10.7,
+// 2048 x 8192 12.8 -> 10.6, 6160 x 2048 11.7 -> 6.8 (3 tokens: 42.5, 57.8, 12.9, 12.9, 10.4 before).  With 1 or 2 tokens the FMA kernels, whose loads run along a row (512
+// contiguous bytes against 64), are as fast or faster (2 tokens: 2048 x 8192 7.9 against 10.5), and with fewer than 96 groups of 16 features too (8 tokens, 1024 x 5464:
+// 7.4 against 8.9: a warp's batches run one after the other), with 3 or 4 tokens 192 (2048 x 2048: linear_flow_kernel, its weights asked for early, 4.2 against
+// 4.6; 4096 x 2048: 7.0 against 5.9).
 constexpr int LM_U = 8, LM_BATCH = 32 * LM_U;        // chunk groups of 32 k in flight; k of a batch
 constexpr int LM_MIN_K = 1536, LM_MAX_SEG = 1536;
 
-__device__ __forceinline__ uint4 lm_load(const void* p) {      // touched once: no line in L1 (the tokens live there)
-  uint4 r;
-  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
-  return r;
-}
 __device__ __forceinline__ void lm_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -163,8 +282,8 @@ __global__ void __launch_bounds__((KS > 4 ? KS : 4) * 32) linear_mma_rows_kernel
       for (int u = 0; u < LM_U; ++u) {                     // all loads of the batch before the first use
         const int k = kb + 32 * u + 8 * t;
         const bool on = k < k1;                            // K is a multiple of 8
-        a[u] = on ? lm_load(w0 + k) : make_uint4(0u, 0u, 0u, 0u);
-        b[u] = on ? lm_load(w1 + k) : make_uint4(0u, 0u, 0u, 0u);
+        a[u] = on ? ldg_weights(w0 + k) : make_uint4(0u, 0u, 0u, 0u);
+        b[u] = on ? ldg_weights(w1 + k) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
       for (int u = 0; u < LM_U; ++u) {
@@ -281,16 +400,18 @@ __global__ void __launch_bounds__(256) linear_tiled_kernel(const T* __restrict__
 template <typename T, typename OutT>
 static int launch_linear(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0,
                          float p1, cudaStream_t st, bool tensor_cores, LinearGroup g = LinearGroup{0, 0, 0, 1, nullptr, nullptr, nullptr},
-                         int nbatch = 1) {
+                         int nbatch = 1, bool early = false) {
   if (M <= LR_MAXM && g.tile_group == nullptr) {
     constexpr int VN = Vec<T>::N;
     const int vec_ok = (K % VN == 0) && (ldx % VN == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) &&
                        (g.x_bs % VN == 0) && (g.w_bs % VN == 0);
     if constexpr (sizeof(T) == 2) {
-      if (tensor_cores && vec_ok && M > 4 && K >= LM_MIN_K && K <= 16 * LM_MAX_SEG && (long)((N + 15) / 16) * nbatch >= 96) {
+      if (tensor_cores && vec_ok && M > 2 && K >= LM_MIN_K && K <= 16 * LM_MAX_SEG && (long)((N + 15) / 16) * nbatch >= (M > 4 ? 96 : 192)) {
         lm_launch<OutT>((const T*)x, ldx, (const T*)w, (OutT*)out, ldo, M, N, K, act, p0, p1, st, g, nbatch);
         return cudaGetLastError() == cudaSuccess ? JL_OK : JL_ERR_CUDA;
       }
+      if (vec_ok && (M == 1 || (M <= 4 && K <= 4096)) && nbatch == 1 && g.w_index == nullptr)
+        return flow_launch<OutT>((const T*)x, ldx, (const T*)w, (OutT*)out, ldo, M, N, K, act, p0, p1, early, st);
     }
     const dim3 blocks((N + LR_ROWS - 1) / LR_ROWS, nbatch);
 #define JL_LR(MM)                                                                                                       \
@@ -317,15 +438,22 @@ static int launch_linear(const void* x, int ldx, const void* w, void* out, int l
 using namespace jl;
 
 static int linear_any(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1, int dtype,
-                      int out_f32, void* stream, bool tensor_cores) {
+                      int out_f32, void* stream, bool tensor_cores, bool early = false) {
   JL_CHECK_ARG(M >= 1 && N >= 1 && K >= 1 && ldx >= K && ldo >= N, "jl_linear_any: bad shape M=%d N=%d K=%d ldx=%d ldo=%d", M, N,
                K, ldx, ldo);
   JL_CHECK_ARG(act >= 0 && act <= ACT_LAST, "jl_linear_any: bad activation %d", act);
   cudaStream_t st = (cudaStream_t)stream;
+  const LinearGroup plain{0, 0, 0, 1, nullptr, nullptr, nullptr};
+  if (early) {
+    // inside one captured graph everything before the graph is complete, whatever wrote the weights included; outside, the kernel just
+    // ahead in the stream may have written them
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    early = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusActive;
+  }
   int rc;
   if (dtype == DT_BF16)
-    rc = out_f32 ? launch_linear<__nv_bfloat16, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tensor_cores)
-                 : launch_linear<__nv_bfloat16, __nv_bfloat16>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tensor_cores);
+    rc = out_f32 ? launch_linear<__nv_bfloat16, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tensor_cores, plain, 1, early)
+                 : launch_linear<__nv_bfloat16, __nv_bfloat16>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tensor_cores, plain, 1, early);
   else
     rc = launch_linear<float, float>(x, ldx, w, out, ldo, M, N, K, act, p0, p1, st, tensor_cores);
   if (rc != JL_OK) return cuda_fail(cudaGetLastError(), "jl_linear_any launch");
@@ -335,6 +463,11 @@ static int linear_any(const void* x, int ldx, const void* w, void* out, int ldo,
 extern "C" JL_API int jl_linear_any(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act,
                                     float p0, float p1, int dtype, int out_f32, void* stream) {
   return linear_any(x, ldx, w, out, ldo, M, N, K, act, p0, p1, dtype, out_f32, stream, hybrid_tensor_cores());
+}
+
+extern "C" JL_API int jl_linear_resident(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act,
+                                         float p0, float p1, int dtype, int out_f32, void* stream) {
+  return linear_any(x, ldx, w, out, ldo, M, N, K, act, p0, p1, dtype, out_f32, stream, hybrid_tensor_cores(), true);
 }
 
 extern "C" JL_API int jl_linear_exact(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act,

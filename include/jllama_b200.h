@@ -278,6 +278,10 @@ int jl_act_inplace(void* data, int ld, int M, int N, int act, float p0, float p1
 /* out[:, 0:N] (pitch ldo; fp32 if out_f32 else dtype) = act(x W^T): x [M, K] (pitch ldx), W [N, K]; any M, N, K. */
 int jl_linear_any(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1,
                   int dtype, int out_f32, void* stream);
+/* The same where W is a parameter: in a captured graph no kernel of which writes W, a decode step's kernel reads W ahead of its wait for the
+ * kernels before it. */
+int jl_linear_resident(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1,
+                       int dtype, int out_f32, void* stream);
 /* The same on the SIMT kernels whatever the sizes (fp32 FMAs in order of k within a thread): what JLLAMA_HYBRID_TC=0 gives every call. */
 int jl_linear_exact(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1,
                     int dtype, int out_f32, void* stream);

@@ -73,10 +73,10 @@ class DenseFeedForward:
 
     def run(self, h: torch.Tensor) -> torch.Tensor:
         if self.spec.gated:
-            t = _gated_act(SK.linear(h, self.up), self.u_off, self.spec.ff, self.spec.act, 0.0, h.dtype)
+            t = _gated_act(SK.linear(h, self.up, resident=True), self.u_off, self.spec.ff, self.spec.act, 0.0, h.dtype)
         else:
-            t = SK.linear(h, self.up, act=self.act, p0=self.p0, p1=self.p1, out_f32=False)
-        return SK.linear(t, self.down)
+            t = SK.linear(h, self.up, act=self.act, p0=self.p0, p1=self.p1, out_f32=False, resident=True)
+        return SK.linear(t, self.down, resident=True)
 
 
 class MoeFeedForward:
@@ -150,7 +150,7 @@ class MoeFeedForward:
     def run(self, h: torch.Tensor) -> torch.Tensor:
         s = self.spec
         M, W = h.shape
-        z = SK.linear(h, self.w_route)                                             # fp32 [M, router logits | gate logit]
+        z = SK.linear(h, self.w_route, resident=True)                                             # fp32 [M, router logits | gate logit]
         ident_w = torch.empty(M, dtype=torch.float32, device=h.device) if s.identity else None
         idx, wt = SK.moe_route(z, self.n_route, s.top, s.groups, s.keep, s.group_top, self.score, s.normalise, s.scale,
                                bias=self.router_bias, choice_bias=self.choice_bias, n_real=s.experts, ident_w=ident_w)
@@ -195,10 +195,10 @@ class MoeFeedForward:
         gate = None
         if self.has_shared:
             if s.gated:
-                u = _gated_act(SK.linear(h, self.shared_up), self.shared_u_off, s.shared_ff, s.act, s.shared_limit, h.dtype)
+                u = _gated_act(SK.linear(h, self.shared_up, resident=True), self.shared_u_off, s.shared_ff, s.act, s.shared_limit, h.dtype)
             else:
-                u = SK.linear(h, self.shared_up, act=self.act, out_f32=False)
-            shared = SK.linear(u, self.shared_down)
+                u = SK.linear(h, self.shared_up, act=self.act, out_f32=False, resident=True)
+            shared = SK.linear(u, self.shared_down, resident=True)
             if self.gate_off >= 0:
                 gate = z[:, self.gate_off:self.gate_off + 1]
         if s.identity:                                     # pairs that chose an identity expert ran nothing: weight · input instead

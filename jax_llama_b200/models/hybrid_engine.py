@@ -112,9 +112,9 @@ class TokenSide:
             g = SK.side_gate_rows(x, ids, self.table, self.col0, self.gate)
         else:
             xc = x_cast if x_cast is not None else (x if self.gate.dtype == torch.float32 else SK.act_cast(x, self.gate.dtype))
-            t = SK.linear(xc, self.gate)                                      # fp32 [M, dim]
+            t = SK.linear(xc, self.gate, resident=True)                                      # fp32 [M, dim]
             g = SK.side_gate(t, ids, self.table, self.col0, self.dim, self.gate.dtype)
-        y = SK.linear(g, self.proj)                                           # fp32 [M, width]
+        y = SK.linear(g, self.proj, resident=True)                                           # fp32 [M, width]
         return SK.postnorm_add(y, self.norm, x, eps, 0.0, w_next=w_next)
 
 
@@ -378,8 +378,8 @@ class HybridEngine(B200Engine):
         c = self.config
         h = SK.norm_f32(x, self.final_norm, self.eps, self.norm_offset)
         if c.logit_scale == 1.0 and c.logit_softcap == 0.0:
-            return SK.linear(h, self.lm_head, out=out)
-        return SK.linear(h, self.lm_head, act=SK.ACT_SCALE_SOFTCAP, p0=c.logit_scale, p1=c.logit_softcap, out=out)
+            return SK.linear(h, self.lm_head, out=out, resident=True)
+        return SK.linear(h, self.lm_head, act=SK.ACT_SCALE_SOFTCAP, p0=c.logit_scale, p1=c.logit_softcap, out=out, resident=True)
 
     def _layers(self, x: torch.Tensor, B: int, S: int, cache: HybridCache, positions: Optional[torch.Tensor],
                 ws: Optional[DecodeState] = None) -> torch.Tensor:

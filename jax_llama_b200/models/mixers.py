@@ -94,7 +94,7 @@ class Mixer:
         return p.y1 if p.bias is None and p.y2 is None and p.c1 == 1.0 else SK.weighted_sum2(*p)
 
     def parts(self, h: torch.Tensor, B: int, S: int, cache: "object", layer: int, rope: Optional[Tuple] = None) -> MixerParts:
-        return MixerParts(SK.linear(self.run(h, B, S, cache, layer, rope), self.wo), bias=self.out_bias)
+        return MixerParts(SK.linear(self.run(h, B, S, cache, layer, rope), self.wo, resident=True), bias=self.out_bias)
 
     out_bias: Optional[torch.Tensor] = None        # bias of the output projection
 
@@ -264,7 +264,7 @@ class AttentionMixer(Mixer):
     def run(self, h: torch.Tensor, B: int, S: int, cache: "object", layer: int, rope: Tuple[torch.Tensor, torch.Tensor]
             ) -> torch.Tensor:
         s = self.spec
-        y = SK.linear(h, self.w_in)                                   # fp32 [M, q | k | v | gate]
+        y = SK.linear(h, self.w_in, resident=True)                                   # fp32 [M, q | k | v | gate]
         q = torch.empty((B * S, s.heads * s.dim), dtype=self.dtype, device=h.device)
         src = layer if not self.shares_kv else s.kv_from
         kc, vc = cache.ks[src], cache.vs[src]
@@ -394,7 +394,7 @@ class GlaMixer(Mixer):
     def run(self, h: torch.Tensor, B: int, S: int, cache: "object", layer: int, rope: Optional[Tuple] = None
             ) -> torch.Tensor:
         s = self.spec
-        y = SK.linear(h, self.w_in)                                   # fp32 [M, q | k | v | gate | low-rank decay input]
+        y = SK.linear(h, self.w_in, resident=True)                                   # fp32 [M, q | k | v | gate | low-rank decay input]
         o = SK.gla_scan(y, self.q_off, self.k_off, self.v_off, self.a_off, self.a2, self.a2_bias, cache.states[layer],
                         cache.len_dev, cache.pad_left, B, S, s.heads, s.dim, s.vdim, s.dim ** -0.5, s.tau)
         gate = y[:, self.g_off:self.g_off + s.heads * s.vdim]
@@ -489,12 +489,12 @@ class LatentAttentionMixer(Mixer):
         layout = SK.ROT_LAYOUTS[s.rot.layout] if s.rot is not None else 0
         kc = cache.ks[layer]                                                   # [B, T, kv_rank + rot_dim]
         starts = S > 1 and int(cache.index) == 0                               # a prompt from an empty cache
-        y = SK.linear(h, self.w_in)                                            # fp32 [M, queries (or latent) | kv latent | key part | gate]
+        y = SK.linear(h, self.w_in, resident=True)                                            # fp32 [M, queries (or latent) | kv latent | key part | gate]
         gate = y[:, self.g_off:self.g_off + H] if s.head_gate else None
         cq, c_new, kr_new = SK.latent_prep(y, self.q_off, self.q_cols, self.kv_off, s.kv_rank, s.rot_dim, rot, layout,
                                            self.q_norm, self.kv_norm, kc, rope[0], rope[1], self.eps, cache.len_dev,
                                            cache.pad_left, B, S, token_major=starts)
-        q = SK.linear(cq, self.uq, out_f32=False) if s.q_rank else cq          # [M, H·(rot_dim + dim)]
+        q = SK.linear(cq, self.uq, out_f32=False, resident=True) if s.q_rank else cq          # [M, H·(rot_dim + dim)]
         if starts:
             return self._attend_projected(q, c_new, kr_new, cache, B, S, rot, layout, rope, gate)
         qa = torch.empty((M, H * self.row), dtype=self.dtype, device=h.device)
@@ -513,7 +513,7 @@ class LatentAttentionMixer(Mixer):
         """Per-head keys and values of the S new tokens of every row, token-major; slot == index within the prompt."""
         s = self.spec
         M, H, qd = B * S, s.heads, s.dim + s.rot_dim
-        kv = SK.linear(c_new, self.w_kv, out_f32=False)                        # [M, H·dim | H·vdim (| padding)]
+        kv = SK.linear(c_new, self.w_kv, out_f32=False, resident=True)                        # [M, H·dim | H·vdim (| padding)]
         qf = torch.empty_like(q)
         SK.rotary_slice(q, qd, 0, qf, qd, 0, H, qd, rot, layout, rope[0], rope[1], cache.len_dev, cache.pad_left, B, S)
         kf = torch.empty((M, H * qd), dtype=self.dtype, device=q.device)       # [M, H, rot_dim | dim]
@@ -555,7 +555,7 @@ class RetentionMixer(Mixer):
         s = self.spec
         rot = s.rot.dims if s.rot is not None else 0
         layout = SK.ROT_LAYOUTS[s.rot.layout] if s.rot is not None else 0
-        y = SK.linear(h, self.w_in)                                   # fp32 [M, q | k | v | gate]
+        y = SK.linear(h, self.w_in, resident=True)                                   # fp32 [M, q | k | v | gate]
         o = SK.retention_scan(y, self.q_off, self.k_off, self.v_off, self.decay, rope[0], rope[1], rot, layout,
                               s.dim ** -0.5, cache.states[layer], cache.len_dev, cache.pad_left, B, S, s.heads, s.dim,
                               s.vdim)
@@ -607,7 +607,7 @@ class StateSpaceMixer(Mixer):
             ) -> torch.Tensor:
         s = self.spec
         state, conv_state = cache.states[layer]
-        y = SK.linear(h, self.w_in)                                   # fp32 [M, z | x | B | C | dt]
+        y = SK.linear(h, self.w_in, resident=True)                                   # fp32 [M, z | x | B | C | dt]
         u = SK.causal_conv(y, self.x_off, self.conv_w, self.conv_b, conv_state, cache.len_dev, cache.pad_left, B, S,
                            act=SK.ACT_SILU)                           # fp32 [M, x | B | C]
         o = SK.ssd_scan(y, self.dt_off, self.dt_bias, self.a_log, u, self.inner + self.gn, self.inner, 0, s.groups, state,
@@ -671,7 +671,7 @@ class DeltaRuleMixer(Mixer):
             ) -> torch.Tensor:
         s = self.spec
         state, conv_state = cache.states[layer]
-        y = SK.linear(h, self.w_in)                                   # fp32, the stacked projection
+        y = SK.linear(h, self.w_in, resident=True)                                   # fp32, the stacked projection
         u = SK.causal_conv(y, self.q_off, self.conv_w, None, conv_state, cache.len_dev, cache.pad_left, B, S, act=SK.ACT_SILU)
         if s.head_decay:
             o = SK.delta_head_scan(u, 0, self.nq, 2 * self.nq, s.kv_heads, y, self.b_off, self.a_off, self.a_bias, self.a_log, state,
@@ -680,7 +680,7 @@ class DeltaRuleMixer(Mixer):
         o = SK.delta_scan(u, 0, self.nq, 2 * self.nq, s.kv_heads, y, self.b_off, self.a_off, self.a2, self.a_bias,
                           self.a_log, state, cache.len_dev, cache.pad_left, B, S, s.heads, s.dim, s.vdim)
         g_in = SK.act_cast(y[:, self.g_off:self.g_off + self.gate_rank], self.dtype)
-        gate = SK.linear(g_in, self.g2)                               # fp32 [M, heads · vdim]
+        gate = SK.linear(g_in, self.g2, resident=True)                               # fp32 [M, heads · vdim]
         return SK.headnorm_gate(o, self.norm, gate, s.heads, s.vdim, self.eps, SK.ACT_SIGMOID)
 
 
@@ -797,7 +797,7 @@ class LightningMixer(Mixer):
 
     def run(self, h: torch.Tensor, B: int, S: int, cache: "object", layer: int, rope: Optional[Tuple] = None) -> torch.Tensor:
         s = self.spec
-        y = SK.linear(h, self.w_in)                                   # fp32 [M, q | k | v | gate]
+        y = SK.linear(h, self.w_in, resident=True)                                   # fp32 [M, q | k | v | gate]
         o = SK.activated_scan(y, self.q_off, self.k_off, self.v_off, self.decay, SK.ACT_SILU, cache.states[layer], cache.len_dev,
                               cache.pad_left, B, S, s.heads, s.dim, s.vdim)
         return SK.rownorm_gate(o, self.norm, y[:, self.g_off:self.g_off + s.heads * s.vdim], self.eps, SK.ACT_SIGMOID)
@@ -841,7 +841,7 @@ class MlstmMixer(Mixer):
     def run(self, h: torch.Tensor, B: int, S: int, cache: "object", layer: int, rope: Optional[Tuple] = None) -> torch.Tensor:
         s = self.spec
         state, m_state = cache.states[layer]
-        y = SK.linear(h, self.w_in)                                   # fp32 [M, q | k | v | gate | i | f]
+        y = SK.linear(h, self.w_in, resident=True)                                   # fp32 [M, q | k | v | gate | i | f]
         o, aux = SK.mlstm_scan(y, self.q_off, self.k_off, self.v_off, self.i_off, self.f_off, self.i_bias, self.f_bias, s.gate_cap,
                                s.dim ** -0.5, state, m_state, cache.len_dev, cache.pad_left, B, S, s.heads, s.dim, s.vdim)
         return SK.mlstm_finish(o, aux, self.norm, y[:, self.g_off:self.g_off + s.heads * s.vdim], s.heads, s.vdim, self.eps,

@@ -111,13 +111,15 @@ def act_cast(y: torch.Tensor, out_dtype: torch.dtype, act: int = ACT_NONE, p0: f
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float = 0.0, p1: float = 0.0,
-           out_f32: bool = True, out: Optional[torch.Tensor] = None, tensor_cores: Optional[bool] = None) -> torch.Tensor:
+           out_f32: bool = True, out: Optional[torch.Tensor] = None, tensor_cores: Optional[bool] = None,
+           resident: bool = False) -> torch.Tensor:
     """act(x Wᵀ): x [M, K] and W [N, K] of one dtype (bf16 or fp32) → fp32 (or the operand dtype) [M, N].
 
     bfloat16 with more than 8 rows and 16-byte pitches runs the tcgen05 GEMM (fp32 accumulate; the activation is
     then an in-place pass over the stored result), float32 with more than 8 rows the three-part tcgen05 kernel (csrc/linear_f32.cu),
-    8 rows or fewer a weight-streaming kernel (bfloat16 from 5 rows on: mma.sync); everything else — and every size with
-    `tensor_cores=False` or JLLAMA_HYBRID_TC=0 — the exact SIMT kernels."""
+    8 rows or fewer a weight-streaming kernel (bfloat16 from 3 rows on: mma.sync); everything else — and every size with
+    `tensor_cores=False` or JLLAMA_HYBRID_TC=0 — the exact SIMT kernels.  `resident`: W is a parameter, written by no kernel of the
+    graph a call is captured in; a decode step then reads it ahead of the kernels before."""
     if not x.is_cuda:
         raise ValueError("linear: CUDA tensors only")
     _need(w, x.dtype, "w")
@@ -141,7 +143,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
             _lib.check(L.jl_act_inplace(out.data_ptr(), out.stride(0), M, N, act, float(p0), float(p1),
                                         dtype_code(out.dtype), _stream()), "jl_act_inplace")
         return out
-    call = L.jl_linear_any if use_tc else L.jl_linear_exact
+    call = (L.jl_linear_resident if resident else L.jl_linear_any) if use_tc else L.jl_linear_exact
     _lib.check(call(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), M, N, K, act,
                     float(p0), float(p1), dtype_code(x.dtype), int(out.dtype == torch.float32), _stream()),
                "jl_linear_any" if use_tc else "jl_linear_exact")

@@ -181,3 +181,38 @@ def test_decode_rows_are_not_further_from_float64_than_the_exact_kernel(N, K, dr
         fast += float((SK.linear(x, w).double() - ref).norm() / ref.norm()) ** 2
         exact += float((SK.linear(x, w, tensor_cores=False).double() - ref).norm() / ref.norm()) ** 2
     assert fast <= exact
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K", [(1, 8), (3, 2048), (130, 2056), (2371, 1024), (2371, 4096), (9481, 264), (600, 1528)])
+def test_decode_rows_that_stay_give_the_same_bits(M, N, K, monkeypatch):
+    """The kernel whose CTAs walk the features forms every sum in the order of the one with a CTA per four features (which batches take)."""
+    g = torch.Generator().manual_seed(N + K + M)
+    x, w = torch.randn(M, K, generator=g).bfloat16().cuda(), torch.randn(2, N, K, generator=g).bfloat16().cuda()
+    want = torch.full((2 * M, N), 7.0, device="cuda")
+    monkeypatch.setenv("JLLAMA_HYBRID_TC", "0")
+    SK.linear_batched(torch.cat([x, x]), w, want, nbatch=2, rows=M, x_bs=M * K, o_bs=M * N)
+    room = torch.full((M * N + 64,), 7.0, device="cuda")
+    assert torch.equal(SK.linear(x, w[1], out=room[:M * N].view(M, N)), want[M:]) and bool((room[M * N:] == 7.0).all())
+    check(SK.linear(x, w[0], act=SK.ACT_RELU, out_f32=False), x, w[0], torch.relu)
+
+
+@pytest.mark.parametrize("M,K", [(1, 2048), (2, 1024), (4, 512)])
+def test_decode_rows_of_a_parameter_in_a_graph(M, K):
+    """A captured chain that asks for its weights ahead of the kernels before it sees the weights and tokens of every replay."""
+    g = torch.Generator().manual_seed(K)
+    x, w1, w2 = (torch.randn(s, K, generator=g).bfloat16().cuda() for s in (M, K, 777))
+
+    def chain():
+        return SK.linear(SK.linear(x, w1, out_f32=False, resident=True), w2, resident=True)
+
+    chain()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain()
+    for _ in range(3):
+        graph.replay()
+        y = SK.linear(x, w1, out_f32=False)
+        assert torch.equal(out, SK.linear(y, w2))
+        for t in (x, w1, w2):
+            t.copy_(torch.randn(t.shape, generator=g).bfloat16())

@@ -11,6 +11,7 @@
 // itself.  delta_scan_kernel walks the tokens: a thread owns DP key channels of one value column in registers, the
 // P = ceil(D / DP) lanes of a column are adjacent.  With c = a ⊙ s the two dot products k·c and q·c are formed in one pass and reduced together, and
 // o = q·c + (q·k) e needs no second reduction; the second pass adds k e to the state.
+#include "delta_chunk.cuh"
 #include "jllama_b200.h"
 #include "seq_types.cuh"
 
@@ -24,7 +25,6 @@ namespace jl {
 constexpr int DS_TC = 32;            // tokens per pipeline stage (fewer when two stages of wide keys would not fit)
 constexpr int DS_THREADS = 128;
 
-__device__ __forceinline__ float delta_softplus(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
 __host__ __device__ inline int delta_record_floats(int P, int DP, int Dv) { return 3 * P * (DP + 4) + ((Dv + 3) & ~3) + 4; }
 
 struct DeltaParams {
@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(DS_THREADS) delta_scan_kernel(DeltaParams p, i
 }
 
 // ------------------------------------------------------------------------------------------------ one decay per head
+// A few tokens per row, and keys above 128 channels (prompts of narrower keys: delta_chunk.cu).
 // With one decay a per (token, head) the decay commutes with every product over key channels, so DH_NB consecutive tokens are
 // taken together: their 2 DH_NB dot products with the state as it stands (k_i . S, q_i . S) are formed in one pass and reduced
 // together, and what the tokens of a block do to one another is scalar work with the dot products of their keys and queries
@@ -207,23 +208,7 @@ constexpr int DH_NB = 4;
 constexpr int DH_PAIR = 8;           // q.k at lags 0 .. 3 | k.k at lags 1 .. 3 | unused
 constexpr int DH_GATE = 4;           // beta, a, two unused (16-byte rows)
 
-struct DeltaHeadParams {
-  const float* u; int ldu;           // q | k | v after their convolutions
-  int q_off, k_off, v_off, G;
-  const float* y; int ldy;           // projection row: beta logits and decay inputs, one of each per head
-  int b_off, a_off;
-  int B, S, H, D, Dv, P, cols;
-  const int* cache_len; const int* pad_left;
-  float* state; float* o;
-  float* qk; float* pair; float* gate; float* val;       // workspace parts (prompts)
-};
-
-__device__ __forceinline__ float delta_head_decay(float z, float a_log) { return expf(-expf(a_log) * delta_softplus(z)); }
-
-// grid (tokens, q / k heads), 128 threads: warp l forms the dot products at lag l.  One warp per token with all lags in registers is
-// the faster kernel, 50 us against 66 for 2000 tokens x 16 heads of 64 x 128, and without programmatic dependent launch the faster layer, 377 us
-// a pass against 391.  With it the layer is slower, 450 against 385, presumably by placement: the scan's few long CTAs come in as soon as the last CTAs of this
-// kernel have started, and a quarter as many, four times as long CTAs leave them the room of a few SMs, where they then share.
+// grid (tokens, q / k heads), 128 threads: warp l forms the dot products at lag l.
 template <typename T, int DP>
 __global__ void __launch_bounds__(32 * DH_NB) delta_head_prep_kernel(DeltaHeadParams p, const T* __restrict__ a_bias, const T* __restrict__ a_log) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
@@ -543,6 +528,7 @@ extern "C" JL_API int jl_delta_scan(const float* u, int ldu, int q_off, int k_of
 }
 
 extern "C" JL_API size_t jl_delta_head_scan_ws_floats(int B, int S, int H, int G, int D, int Dv) {
+  if (delta_chunk_takes(D)) return delta_chunk_ws_floats(B, S, H, D);
   size_t off[4];
   return delta_head_ws(delta_head_plan(B, H, D, Dv), B, S, H, G, off);
 }
@@ -557,6 +543,9 @@ static int delta_head_launch(DeltaHeadParams p, const DeltaHeadPlan& plan, const
     JL_CUDA(cudaGetLastError());
     return JL_OK;
   }
+  if constexpr (DP < 32) {
+    return JL_ERR_UNSUPPORTED;                                  // (prompts of up to 128 channels go in chunks: delta_chunk.cu)
+  } else {
   JL_LAUNCH_PDL((delta_head_prep_kernel<T, DP>), dim3(p.B * p.S, p.G), dim3(32 * DH_NB), 0, stream, p, (const T*)a_bias, (const T*)a_log);
   JL_CUDA(cudaGetLastError());
   int tc = DS_TC;                                               // tokens per pipeline stage: two stages have to fit
@@ -568,6 +557,7 @@ static int delta_head_launch(DeltaHeadParams p, const DeltaHeadPlan& plan, const
   JL_LAUNCH_PDL((delta_head_scan_kernel<T, DP, false>), grid, block, smem, stream, p, tc, (const T*)a_bias, (const T*)a_log);
   JL_CUDA(cudaGetLastError());
   return JL_OK;
+  }
 }
 
 // The delta rule with one decay per head: a_t = exp(-exp(a_log[h]) * softplus(y[m, a_off + h] + a_bias[h])); otherwise as jl_delta_scan.
@@ -585,6 +575,7 @@ extern "C" JL_API int jl_delta_head_scan(const float* u, int ldu, int q_off, int
   delta_head_ws(plan, B, S, H, G, off);
   DeltaHeadParams p{u, ldu, q_off, k_off, v_off, G, y, ldy, b_off, a_off, B, S, H, D, Dv, plan.P, plan.cols, cache_len, pad_left, state, o,
                     ws ? ws + off[0] : nullptr, ws ? ws + off[1] : nullptr, ws ? ws + off[2] : nullptr, ws ? ws + off[3] : nullptr};
+  if (S > DS_FUSED_MAX_TOKENS && delta_chunk_takes(D)) return delta_chunk_launch(p, ws, a_bias, a_log, dtype, (cudaStream_t)stream);
   if (plan.DP == 8) JL_DISPATCH_DTYPE(dtype, return (delta_head_launch<T, 8>(p, plan, a_bias, a_log, stream)));
   if (plan.DP == 16) JL_DISPATCH_DTYPE(dtype, return (delta_head_launch<T, 16>(p, plan, a_bias, a_log, stream)));
   JL_DISPATCH_DTYPE(dtype, return (delta_head_launch<T, 32>(p, plan, a_bias, a_log, stream)));

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(128) embed_pair_norm_kernel(const int* __restr
 }
 
 constexpr int CC_MAX_TAPS = 32;      // instances of 4, 8 and 32: the history and the taps of a channel live in registers
-constexpr int CC_CHUNK = 64;       // tokens per CTA along time
+constexpr int CC_CHUNK = 64;       // tokens per CTA along time (or half of it)
 constexpr int CC_AHEAD = 8;        // inputs requested at once: a walk token by token paid a memory latency for each
 
 // grid (channel blocks, rows, time chunks); a thread owns one channel and walks its chunk with the last taps-1 inputs in
@@ -423,7 +423,8 @@ extern "C" JL_API int jl_causal_conv(const float* y, int ldy, int col0, int C, c
   JL_CHECK_ARG(B >= 1 && S >= 1 && C >= 1 && ldo >= C, "jl_causal_conv: bad shape");
   JL_CHECK_ARG(taps >= 1 && taps <= CC_MAX_TAPS, "jl_causal_conv: %d taps (1 .. %d)", taps, CC_MAX_TAPS);
   JL_CHECK_ARG(taps == 1 || state != nullptr, "jl_causal_conv: no state for %d taps", taps);
-  const int chunk = CC_CHUNK;
+  // half the tokens per CTA where that many CTAs leave room (2048 tokens x 2048 channels 33 -> 22 us a cold launch; at least taps - 1 tokens: 31)
+  const int chunk = (long)((C + 127) / 128) * B * ((S + CC_CHUNK - 1) / CC_CHUNK) < 148 * 6 ? CC_CHUNK / 2 : CC_CHUNK;
   dim3 grid((C + 127) / 128, B, (S + chunk - 1) / chunk);
 #define JL_CC(MT_)                                                                                                              \
   JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((causal_conv_kernel<T, MT_>), dim3(grid), dim3(128), 0, stream, y, ldy, col0, C, in_bias, \

@@ -830,3 +830,36 @@ def test_trace_replay_of_batches_that_come_and_go(dtype, tmp_path):
             continue
         got = torch.from_numpy(np.fromfile(path, dtype="<f4").reshape(len(want), 80).copy())
         assert err(got, torch.stack(want)) < bound, s["step"]
+
+
+@pytest.mark.parametrize("H,G,D,Dv,S", [(2, 2, 64, 128, 9), (2, 1, 64, 130, 31), (16, 16, 32, 64, 32), (40, 20, 64, 200, 33), (4, 4, 128, 128, 97), (3, 3, 33, 7, 64),
+                                        (110, 110, 16, 20, 65)])
+def test_delta_rule_in_chunks_of_every_width(H, G, D, Dv, S):
+    """Prompts in chunks of 32 tokens: remainders, padded rows, 8, 16 and 32 value columns per CTA, rows of values off the 16-byte boundary; a token
+    that is not finite reaches itself and the later tokens of its row, no earlier one."""
+    nu = 2 * G * D + H * Dv + (1 if Dv % 4 else 0)
+    g = torch.Generator().manual_seed(H + D + S)
+    u, y = torch.randn(2, S, nu, generator=g), torch.randn(2, S, 2 * H, generator=g)
+    bias, a_log = torch.randn(H, generator=g).to(torch.bfloat16), (torch.randn(H, generator=g) - 2.0).to(torch.bfloat16)
+    first, st0 = [0, min(5, S - 1)], torch.randn(2, H, D, Dv, generator=g)
+
+    def run(u, carry):
+        st = (st0 if carry else torch.zeros_like(st0)).cuda()
+        o = SK.delta_head_scan(u.reshape(2 * S, nu).contiguous().cuda(), 0, G * D, 2 * G * D, G, y.reshape(2 * S, -1).contiguous().cuda(), 0, H, bias.cuda(),
+                               a_log.cuda(), st, i32([0]), i32(first), 2, S, H, D, Dv)
+        return o.view(2, S, H, Dv).double().cpu(), st.cpu()
+
+    got, _ = run(u, False)
+    for b in range(2):
+        want = _delta_rows(u[b, first[b]:, :2 * G * D + H * Dv], y[b, first[b]:], H, G, D, Dv, 0, H, bias, a_log)
+        assert (got[b, first[b]:] - want).abs().max() < 2e-5 * max(1.0, float(want.abs().max())), b
+    clean, _ = run(u, True)
+    at = 2 * S // 3
+    for value, col in ((float("nan"), 2 * G * D), (float("inf"), G * D)):
+        bad = u.clone()
+        bad[0, at, col] = value
+        o, st = run(bad, True)
+        # such a chunk is summed term by term: sums of up to 32 + 128 products in another order, 2^-24 of their largest partial sum per addition
+        near = (o[0, :at] - clean[0, :at]).abs().max() <= 160 * 2.0 ** -24 * max(1.0, float(clean.abs().max()))
+        assert bool(near) and torch.equal(o[1], clean[1])
+        assert bool(torch.isnan(st[0]).any()) and not bool(torch.isfinite(o[0, at:]).all()) and bool(torch.isfinite(st[1]).all())

@@ -235,6 +235,84 @@ __global__ void __launch_bounds__(128) rotary_slice_kernel(const T* __restrict__
   }
 }
 
+// What a prompt of latent attention needs per head before the attention kernel, one launch, a CTA per token: queries rotated in place (the leading rot
+// channels of a head), keys put together as [key part shared by the heads | the head's own projection].  Bound by what it moves: 16 bytes a thread and
+// step where sizes and addresses allow (vec).  2048 tokens, 16 heads of 64 + 128 channels on one B200: 36 us as three rotary_slice_kernel, 7.3 here.
+struct LatentHeads {
+  int ldq, ldkr, ldkv, ldkf;        // row pitches
+  int H, rot_dim, dim, rot, layout, max_pos, S, vec;
+  const float* cos_t; const float* sin_t;
+  const int* cache_len; const int* pad_left;
+};
+template <typename T>
+__global__ void __launch_bounds__(256) latent_heads_kernel(const LatentHeads p, T* __restrict__ q, const T* __restrict__ kr, const T* __restrict__ kv,
+                                                           T* __restrict__ kf) {
+  pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
+  pdl_launch_dependents();
+  const int m = blockIdx.x, b = m / p.S, s = m % p.S, qd = p.rot_dim + p.dim, half = p.rot / 2;
+  int pos = (p.cache_len ? *p.cache_len : 0) + s - (p.pad_left ? p.pad_left[b] : 0);
+  pos = pos < 0 ? 0 : (pos >= p.max_pos ? p.max_pos - 1 : pos);
+  const float* ct = p.cos_t + (size_t)pos * half;
+  const float* st = p.sin_t + (size_t)pos * half;
+  T* qm = q + (size_t)m * p.ldq;
+  const T* krm = kr + (size_t)m * p.ldkr;
+  const T* kvm = kv + (size_t)m * p.ldkv;
+  T* kfm = kf + (size_t)m * p.ldkf;
+  constexpr int N = 16 / sizeof(T);
+  if (p.vec) {
+    // four pairs a thread: rot is a multiple of 8
+    for (int i = threadIdx.x; i < p.H * (half / 4); i += blockDim.x) {
+      const int h = i / (half / 4), i0 = i % (half / 4) * 4;
+      float c[4], sn[4], u[4], v[4];
+      load4(ct + i0, c);
+      load4(st + i0, sn);
+      T* a = qm + h * qd + (p.layout == 0 ? 2 * i0 : i0);
+      T* w = a + (p.layout == 0 ? 4 : half);
+      load4(a, u);
+      load4(w, v);
+      if (p.layout == 0) {         // u0 u1 u2 u3 v0 v1 v2 v3: pairs (2i, 2i + 1)
+        const float x[8] = {u[0], u[1], u[2], u[3], v[0], v[1], v[2], v[3]};
+        float y[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          y[2 * j] = x[2 * j] * c[j] - x[2 * j + 1] * sn[j];
+          y[2 * j + 1] = x[2 * j + 1] * c[j] + x[2 * j] * sn[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { u[j] = y[j]; v[j] = y[4 + j]; }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float x = u[j];
+          u[j] = x * c[j] - v[j] * sn[j];
+          v[j] = v[j] * c[j] + x * sn[j];
+        }
+      }
+      store4(a, u);
+      store4(w, v);
+    }
+    const int per = qd / N, kr_n = p.rot_dim / N;
+    for (int i = threadIdx.x; i < p.H * per; i += blockDim.x) {
+      const int h = i / per, d = i % per;
+      const T* src = d < kr_n ? krm + d * N : kvm + h * p.dim + (d - kr_n) * N;
+      *reinterpret_cast<uint4*>(kfm + (size_t)i * N) = *reinterpret_cast<const uint4*>(src);
+    }
+    return;
+  }
+  for (int i = threadIdx.x; i < p.H * half; i += blockDim.x) {
+    const int h = i / half, j = i % half;
+    T* a = qm + h * qd + (p.layout == 0 ? 2 * j : j);
+    T* w = a + (p.layout == 0 ? 1 : half);
+    const float u = to_f(*a), v = to_f(*w);
+    *a = from_f<T>(u * ct[j] - v * st[j]);
+    *w = from_f<T>(v * ct[j] + u * st[j]);
+  }
+  for (int i = threadIdx.x; i < p.H * qd; i += blockDim.x) {
+    const int h = i / qd, d = i % qd;
+    kfm[i] = d < p.rot_dim ? krm[d] : kvm[h * p.dim + d - p.rot_dim];
+  }
+}
+
 // Preparation of designs whose q / k norm runs over ALL channels of the projection (weights [H*D] / [G*D]) before the rotation,
 // and whose values may be mixed with another layer's values of the same token: v <- (1 - l) v + l v_first.  Two CTAs per
 // token: the queries; the keys and values.  Sums of squares first, then the rows again (L1 hits) with the rotation and the stores.
@@ -1049,6 +1127,20 @@ extern "C" JL_API int jl_rotary_slice(const void* in, int ldi, int in_hs, int in
   JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(rotary_slice_kernel<T>, dim3(B * S), dim3(128), 0, (cudaStream_t)stream, (const T*)in, ldi,
                                          in_hs, in_off, (T*)out, ldo, out_hs, out_off, H, n, rot, layout, cos_t, sin_t, max_pos,
                                          cache_len, pad_left, S));
+  JL_CUDA(cudaGetLastError());
+  return JL_OK;
+}
+
+extern "C" JL_API int jl_latent_heads(void* q, int ldq, const void* kr, int ldkr, const void* kv, int ldkv, void* kf, int ldkf, int H, int rot_dim, int dim,
+                                      int rot, int layout, const float* cos_t, const float* sin_t, int max_pos, const int* cache_len,
+                                      const int* pad_left, int B, int S, int dtype, void* stream) {
+  JL_CHECK_ARG(B >= 1 && S >= 1 && H >= 1 && rot_dim >= 0 && dim >= 1, "jl_latent_heads: bad shape");
+  JL_CHECK_ARG(rot >= 0 && rot <= rot_dim && rot % 2 == 0 && (layout == 0 || layout == 1), "jl_latent_heads: rot=%d of %d, layout %d", rot, rot_dim, layout);
+  const int n = dtype == DT_BF16 ? 8 : 4;
+  const int vec = rot % 8 == 0 && rot_dim % n == 0 && dim % n == 0 && ldq % n == 0 && ldkr % n == 0 && ldkv % n == 0 && ldkf % n == 0 &&
+                  (((uintptr_t)q | (uintptr_t)kr | (uintptr_t)kv | (uintptr_t)kf | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0;
+  const LatentHeads p{ldq, ldkr, ldkv, ldkf, H, rot_dim, dim, rot, layout, max_pos, S, vec, cos_t, sin_t, cache_len, pad_left};
+  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(latent_heads_kernel<T>, dim3(B * S), dim3(256), 0, (cudaStream_t)stream, p, (T*)q, (const T*)kr, (const T*)kv, (T*)kf));
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }

@@ -352,6 +352,11 @@ int jl_latent_prep(const float* y, int ldy, int q_off, int q_rank, int kv_off, i
 int jl_rotary_slice(const void* in, int ldi, int in_hs, int in_off, void* out, int ldo, int out_hs, int out_off, int H, int n,
                     int rot, int layout, const float* cos_t, const float* sin_t, int max_pos, const int* cache_len,
                     const int* pad_left, int B, int S, int dtype, void* stream);
+/* Prompts of latent attention, token-major: the leading rot channels of every head of q [B*S, H*(rot_dim + dim)] rotated in place at the token's position;
+ * kf [B*S, H*(rot_dim + dim)]: per head [kr row (rot_dim, shared by the heads) | its dim columns of kv].  Row pitches in elements. */
+int jl_latent_heads(void* q, int ldq, const void* kr, int ldkr, const void* kv, int ldkv, void* kf, int ldkf, int H, int rot_dim, int dim, int rot,
+                    int layout, const float* cos_t, const float* sin_t, int max_pos, const int* cache_len, const int* pad_left, int B, int S, int dtype,
+                    void* stream);
 /* Mixture-of-experts routing.  z fp32 [M, ldz]: router logits in columns 0 .. E-1.  score 0: sigmoid, 1: softmax.  groups > 1:
  * experts form `groups` equal groups of neighbours, a group scores the sum of its group_top largest scores, and only experts
  * of the `keep` best groups can be chosen.  idx int32 / wt fp32 [M, top]: the top largest, weights = scores (over their sum

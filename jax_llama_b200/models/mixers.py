@@ -514,15 +514,10 @@ class LatentAttentionMixer(Mixer):
         s = self.spec
         M, H, qd = B * S, s.heads, s.dim + s.rot_dim
         kv = SK.linear(c_new, self.w_kv, out_f32=False, resident=True)                        # [M, H·dim | H·vdim (| padding)]
-        qf = torch.empty_like(q)
-        SK.rotary_slice(q, qd, 0, qf, qd, 0, H, qd, rot, layout, rope[0], rope[1], cache.len_dev, cache.pad_left, B, S)
-        kf = torch.empty((M, H * qd), dtype=self.dtype, device=q.device)       # [M, H, rot_dim | dim]
-        if s.rot_dim:
-            SK.rotary_slice(kr_new, 0, 0, kf, qd, 0, H, s.rot_dim, 0, 0, rope[0], rope[1], cache.len_dev, cache.pad_left, B, S)
-        SK.rotary_slice(kv, s.dim, 0, kf, qd, s.rot_dim, H, s.dim, 0, 0, rope[0], rope[1], cache.len_dev, cache.pad_left, B, S)
+        kf = SK.latent_heads(q, kr_new, kv, H, s.rot_dim, s.dim, rot, layout, rope[0], rope[1], cache.len_dev, cache.pad_left, B, S)
         v = kv[:, self.v_col:]
         ldv = kv.stride(0)
-        return self._attend(qf, kf, v, cache, B, S, H, H, qd, s.vdim, S, H * qd, ldv, gate, strides=(S * H * qd, qd, S * ldv, s.vdim))
+        return self._attend(q, kf, v, cache, B, S, H, H, qd, s.vdim, S, H * qd, ldv, gate, strides=(S * H * qd, qd, S * ldv, s.vdim))
 
 
 class RetentionMixer(Mixer):

@@ -315,6 +315,20 @@ def rotary_slice(src: torch.Tensor, in_hs: int, in_off: int, out: torch.Tensor, 
     return out
 
 
+def latent_heads(q: torch.Tensor, kr: torch.Tensor, kv: torch.Tensor, H: int, rot_dim: int, dim: int, rot: int, layout: int, cos: torch.Tensor,
+                 sin: torch.Tensor, cache_len: torch.Tensor, pad_left: Optional[torch.Tensor], B: int, S: int) -> torch.Tensor:
+    """Rotates the leading `rot` channels of every head of q [B·S, H·(rot_dim + dim)] IN PLACE at the token's position and returns the keys in the
+    same layout: per head [kr [B·S, rot_dim], shared by the heads | its `dim` columns of kv [B·S, ≥ H·dim]]."""
+    _need(kr, q.dtype, "kr")
+    _need(kv, q.dtype, "kv")
+    kf = torch.empty((B * S, H * (rot_dim + dim)), dtype=q.dtype, device=q.device)
+    _lib.check(_lib.lib().jl_latent_heads(
+        q.data_ptr(), q.stride(0), kr.data_ptr(), kr.stride(0), kv.data_ptr(), kv.stride(0), kf.data_ptr(), kf.stride(0), H, rot_dim, dim, rot,
+        layout, cos.data_ptr(), sin.data_ptr(), cos.shape[0], _p(cache_len), _p(pad_left), B, S, dtype_code(q.dtype), _stream()),
+        "jl_latent_heads")
+    return kf
+
+
 def attn_windowed(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, cache_len: torch.Tensor,
                   pad_left: Optional[torch.Tensor], B: int, S: int, H: int, G: int, D: int, Dv: int, T_cap: int, ldk: int,
                   ldv: int, window: int, scale: float, out: Optional[torch.Tensor] = None,

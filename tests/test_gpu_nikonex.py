@@ -139,6 +139,29 @@ def test_rotation_of_a_head_slice(dtype, layout, n, rot):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("layout", ["interleaved", "half"])
+@pytest.mark.parametrize("H,rot_dim,dim,rot", [(16, 64, 128, 64), (3, 16, 24, 8), (5, 8, 8, 0), (2, 0, 40, 0), (3, 6, 7, 4), (2, 64, 128, 60)])
+def test_heads_of_latent_attention(dtype, layout, H, rot_dim, dim, rot):
+    """Queries rotated in place and keys put together in one launch: what the slices one by one give (the same products, at most fused otherwise:
+    one rounding of the operand type), 16-byte and single-element forms, keys as columns of a wider projection."""
+    B, S, qd = 2, 9, rot_dim + dim
+    g = torch.Generator(device="cuda").manual_seed(H + dim)
+    q = torch.randn(B * S, H * qd, device="cuda", generator=g).to(dtype)
+    kr = torch.randn(B * S, max(rot_dim, 1), device="cuda", generator=g).to(dtype)
+    kv = torch.randn(B * S, H * dim + 16, device="cuda", generator=g).to(dtype)
+    cos, sin = rotary_table(max(rot, 2), 100.0, 64, torch.device("cuda"))
+    base, pad, lay = torch.tensor([3], dtype=torch.int32, device="cuda"), torch.tensor([0, 5], dtype=torch.int32, device="cuda"), SK.ROT_LAYOUTS[layout]
+    want = torch.empty_like(q)
+    SK.rotary_slice(q, qd, 0, want, qd, 0, H, qd, rot, lay, cos, sin, base, pad, B, S)
+    kf = SK.latent_heads(q, kr, kv, H, rot_dim, dim, rot, lay, cos, sin, base, pad, B, S)
+    bound = (2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -21) * (1.0 + want.double().abs())
+    assert bool(((q.double() - want.double()).abs() <= bound).all())
+    k = kf.view(B * S, H, qd)
+    assert torch.equal(k[:, :, rot_dim:], kv[:, :H * dim].view(B * S, H, dim))
+    assert torch.equal(k[:, :, :rot_dim], kr[:, None, :rot_dim].expand(-1, H, -1))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("width", [72, 90, 100, 1100])
 def test_branch_sum_and_two_norms(dtype, width):
     g = torch.Generator(device="cuda").manual_seed(width)

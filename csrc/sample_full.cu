@@ -648,6 +648,7 @@ __global__ void __launch_bounds__(SF_THREADS, GREEDY ? 2 : 1) sample_full_kernel
     if (token < 0 || token >= p.V) token = 0;
     p.tok[row] = token;
   }
+  if (p.next_ids == nullptr) return;
   // ---- last CTA: sequence bookkeeping of all rows
   __threadfence();
   __syncthreads();
@@ -657,7 +658,7 @@ __global__ void __launch_bounds__(SF_THREADS, GREEDY ? 2 : 1) sample_full_kernel
     if (s_last) *p.ticket = 0;
   }
   __syncthreads();
-  if (s_last && p.next_ids != nullptr) {
+  if (s_last) {
     __threadfence();
     __shared__ int alive;
     if (threadIdx.x == 0) alive = 0;

@@ -212,7 +212,7 @@ int jl_memcpy_d2d(void* dst, const void* src, size_t bytes, void* stream);
  * for any top_k / top_p (no candidate budget), deterministic ties (lower index), identical on every rank: see
  * csrc/sample_full.cu.  logits fp32 [B, ld] with V valid columns; temperature 0 = arg-max; top_k <= 0 or >= V and
  * top_p >= 1 disable the filters.  `cand`/`gen` (may be NULL) = candidate packets / step counter of jl_decode_mega: wait
- * for every rank's logits shard first.  `next_ids` == NULL: selection only (tok[B]).  `ticket` = one zero int. */
+ * for every rank's logits shard first.  `next_ids` == NULL: selection only (tok[B]), the ticket is not touched.  `ticket` = one zero int. */
 int jl_sample_full(const float* logits, int B, int V, int ld, float temperature, int top_k, float top_p,
                    unsigned long long seed, const int* step, int* tok, const void* cand, const unsigned int* gen, int tp,
                    int rank, int num_sms, int L, int* ticket, int* next_ids, int* finished, int* sequences, int max_len,

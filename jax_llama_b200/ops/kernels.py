@@ -21,8 +21,16 @@ _NUM_SMS = {}
 _SMALL_M_PATH = os.environ.get("JLLAMA_SMALL_M", "gemv")    # measured faster in the graph-replayed step than "gemv_tma"
 
 
+_get_device = getattr(torch._C, "_cuda_getDevice", None)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle (the callers hold CUDA tensors: CUDA is initialised).  torch.cuda.current_stream() builds a Stream object
+    first: 3.2 us a call, a quarter of what a small linear costs the host; these two 0.2."""
+    if _raw_stream is None or _get_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_get_device())
 
 
 def num_sms(device: Optional[torch.device] = None) -> int:
@@ -182,7 +190,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, norm_w: Optional[torch.Tensor] =
     m = x.numel() // k
     odim = n // 2 if mode == SWIGLU else n
     if out is None:
-        out = torch.empty((m, odim), dtype=torch.float32 if out_f32 else x.dtype, device=x.device)
+        out = x.new_empty((m, odim), dtype=torch.float32 if out_f32 else x.dtype)
     sms = num_sms(x.device)
     if force is None:
         path = ("gemv_tma" if _SMALL_M_PATH == "gemv_tma" else "gemv") if m <= 4 else "gemm"
@@ -396,10 +404,9 @@ def sample_full(logits: torch.Tensor, *, temperature: float, top_k: int = 0, top
         B, V, ld = int(rows or 1), logits.shape[0], 0
     else:
         B, V, ld = logits.shape[0], logits.shape[1], logits.stride(0)
-    tok = torch.empty(B, dtype=torch.int32, device=logits.device)
-    ticket = torch.zeros(1, dtype=torch.int32, device=logits.device)
+    tok = logits.new_empty(B, dtype=torch.int32)
     _lib.check(_lib.lib().jl_sample_full(
         logits.data_ptr(), B, V, ld, float(temperature), int(top_k or 0), float(top_p), int(seed), _p(step), tok.data_ptr(),
-        None, None, 1, 0, 0, 0, ticket.data_ptr(), None, None, None, 0, 0, 0, None, None, None, None, _stream()),
+        None, None, 1, 0, 0, 0, tok.data_ptr(), None, None, None, 0, 0, 0, None, None, None, None, _stream()),    # (no bookkeeping: no ticket)
         "jl_sample_full")
     return tok

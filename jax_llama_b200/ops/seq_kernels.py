@@ -128,7 +128,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
     x = x.view(M, K) if x.is_contiguous() else x
     odt = torch.float32 if out_f32 else x.dtype
     if out is None:
-        out = torch.empty((M, N), dtype=odt, device=x.device)
+        out = x.new_empty((M, N), dtype=odt)
     L = _lib.lib()
     use_tc = tensor_cores_enabled() if tensor_cores is None else tensor_cores
     if (use_tc and x.dtype == torch.bfloat16 and M > 8 and K % 8 == 0 and N % 8 == 0 and x.is_contiguous()

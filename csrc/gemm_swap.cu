@@ -32,6 +32,7 @@ struct SwapParams {
   const __nv_bfloat16* residual;
   int N, M, K, nb;          // weight rows, tokens, reduction length, tokens padded to a multiple of 16
   int ldo, stages, ksplit, wide;   // wide: out and residual take 4-feature accesses
+  int turned;                      // the result's rows are the A operand's (fp32): out[feature * ldo + token]
   uint32_t cols, idesc;
   unsigned long long* trace;       // optional [trace_rows][16] %globaltimer stamps (jl_gemm_set_trace), NULL = off
   int trace_rows;
@@ -70,6 +71,13 @@ __device__ __forceinline__ uint2 swap_residual(const SwapParams& p, int tok, int
 template <int EPI, bool OUT_F32>
 __device__ __forceinline__ void swap_emit(const SwapParams& p, int tok, int f0, const float (&x)[4], uint2 res) {
   if constexpr (OUT_F32) {
+    if (p.turned) {
+      float* o = reinterpret_cast<float*>(p.out) + (size_t)f0 * p.ldo + tok;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (f0 + i < p.N) o[(size_t)i * p.ldo] = x[i];
+      return;
+    }
     float* o = reinterpret_cast<float*>(p.out) + (size_t)tok * p.ldo + f0;
     if (p.wide) *reinterpret_cast<float4*>(o) = make_float4(x[0], x[1], x[2], x[3]);
     else { o[0] = x[0]; o[1] = x[1]; o[2] = x[2]; o[3] = x[3]; }
@@ -381,13 +389,14 @@ static int swap_parts(int nb, int tiles, int num_kb, int num_sms) {
 
 template <int EPI, bool OUT_F32>
 static int launch_swap(const void* x, const void* w, const void* residual, void* out, int M, int N, int K, int num_sms,
-                       unsigned long long* trace, cudaStream_t stream) {
+                       unsigned long long* trace, cudaStream_t stream, bool turned = false) {
   SwapParams p{};
   p.out = out;
   p.residual = (const __nv_bfloat16*)residual;
   p.N = N; p.M = M; p.K = K;
   p.nb = (M + 15) / 16 * 16;
-  p.ldo = EPI == SWAP_SWIGLU ? N / 2 : N;
+  p.ldo = turned ? M : EPI == SWAP_SWIGLU ? N / 2 : N;
+  p.turned = turned;
   const uintptr_t step = OUT_F32 ? 16 : EPI == SWAP_SWIGLU ? 4 : 8;
   p.wide = (((uintptr_t)out | (uintptr_t)residual) & (step - 1)) == 0;
   p.cols = p.nb <= 32 ? 32 : p.nb <= 64 ? 64 : p.nb <= 128 ? 128 : 256;
@@ -436,6 +445,16 @@ static int launch_swap(const void* x, const void* w, const void* residual, void*
 // weights the two are equal (28672 x 4096: 62 us).
 bool gemm_swap_takes(int M, int N, int K, int num_sms) {
   return M <= 128 || (M <= 256 && (N + GS_BM - 1) / GS_BM * 2 <= num_sms && K >= 8 * GS_BK && splitk_allowed());
+}
+
+// Few output features over many tokens (a router): the tokens take the MMA's rows, 128 to a tile, and K is split over clusters, where the token-major kernel has a
+// tile, i.e. a CTA, per 128 tokens (32 features, K 2048: 512 tokens 12.3 -> 6.0 us, 2048 12.2 -> 6.6,
+// 4096 12.3 -> 8.0; 64 features, K 4096, 2048 tokens 21.5 -> 9.8; 8192 x 64 x 2048 13.5 and 14.6).
+bool gemm_turned_takes(int M, int N, int K, int num_sms) {
+  return N <= 64 && M > 128 && (M + GS_BM - 1) / GS_BM * 4 <= num_sms && K >= 8 * GS_BK && splitk_allowed();
+}
+int gemm_turned_f32(const void* x, const void* w, void* out, int M, int N, int K, int num_sms, unsigned long long* trace, cudaStream_t s) {
+  return launch_swap<SWAP_PLAIN, true>(w, x, nullptr, out, N, M, K, num_sms, trace, s, true);
 }
 
 int gemm_swap(const void* x, const void* w, const void* residual, void* out, int M, int N, int K, int mode, bool out_f32, int num_sms,

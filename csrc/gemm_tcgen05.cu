@@ -38,12 +38,6 @@ struct GemmParams {
   int stages;
   uint64_t hint_a, hint_b;
   unsigned long long* trace;         // optional [grid][16] %globaltimer stamps (jl_gemm_set_trace), NULL = off
-  // ---- grouped B operand (normal orientation only): the B tensor holds `groups` matrices of group_rows rows one after
-  // the other and A-tile a uses matrix tile_group[a] (< 0: a padding tile, any matrix will do — nobody reads its rows).
-  // The rows of A were ordered beforehand so that every 128-row tile belongs to one matrix (a mixture of experts).
-  const int* tile_group;
-  int group_rows;
-  const int* a_blocks_used;          // optional device count of leading A tiles that hold rows: the tiles after them are skipped
 };
 
 __host__ __device__ constexpr int tmem_cols_for(int bn) {
@@ -100,13 +94,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const uint32_t tmem_base = *tmem_slot_ptr;
   if (threadIdx.x == 0) gemm_stamp(p, 1);
 
-  int a_blocks = p.a_blocks;
   pdl_wait();                 // everything above overlapped the previous kernel's tail
   pdl_launch_dependents();
-  if (p.a_blocks_used != nullptr) {                       // one value for every thread of the grid: all roles walk the same list
-    const int used = *p.a_blocks_used;
-    a_blocks = used < 1 ? 1 : (used < a_blocks ? used : a_blocks);
-  }
+  const int a_blocks = p.a_blocks;
   const int num_tiles = a_blocks * p.b_blocks;
 
   if (warp == 0) {
@@ -117,11 +107,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const int b_blk = t / a_blocks;
         const int a_blk = t % a_blocks;
-        int b_row = b_blk * BN;
-        if (p.tile_group != nullptr) {
-          const int e = p.tile_group[a_blk];
-          b_row += (e < 0 ? 0 : e) * p.group_rows;
-        }
+        const int b_row = b_blk * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
           const uint32_t sa = smem_base + stage * STAGE_BYTES, sb = sa + A_BYTES;
           tc::mbar_wait(empty_bar(stage), phase ^ 1);
@@ -268,13 +254,13 @@ constexpr size_t gemm_smem(int stages, int bn) { return (size_t)stages * gemm_st
 
 template <int BN, int EPI, bool OUT_F32>
 static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int Ra, int Rb, int K, int num_sms,
-                       cudaStream_t stream, int b_matrices = 1) {
+                       cudaStream_t stream) {
   GemmParams p = p0;
   p.trace = g_gemm_trace;
   CUtensorMap ta, tb;
   int rc = make_tmap_2d_bf16(&ta, a, Ra, K, K, GEMM_BM);
   if (rc) return rc;
-  rc = make_tmap_2d_bf16(&tb, b, Rb * b_matrices, K, K, BN);
+  rc = make_tmap_2d_bf16(&tb, b, Rb, K, K, BN);
   if (rc) return rc;
   constexpr uint32_t STAGE_BYTES = gemm_stage_bytes(BN);
   const int num_kb = (K + GEMM_BK - 1) / GEMM_BK;
@@ -339,6 +325,7 @@ extern "C" JL_API int jl_gemm(const void* x, const void* w, const void* residual
   p.K = K;
   p.ldo = mode == EPI_SWIGLU ? N / 2 : N;
   auto s = (cudaStream_t)stream;
+  if (out_f32 && gemm_turned_takes(M, N, K, num_sms)) return gemm_turned_f32(x, w, out, M, N, K, num_sms, g_gemm_trace, s);
   if (gemm_swap_takes(M, N, K, num_sms)) return gemm_swap(x, w, residual, out, M, N, K, mode, out_f32 != 0, num_sms, g_gemm_trace, s);
   // token-major tiles of the prefill shapes go to the CTA-pair kernel (cta_group::2, gemm_2cta.cu); JLLAMA_GEMM_2CTA=0
   // keeps everything on the single-CTA kernel below (A/B measurements)
@@ -355,31 +342,4 @@ extern "C" JL_API int jl_gemm(const void* x, const void* w, const void* residual
   if (mode == EPI_PLAIN) return dispatch_gemm<EPI_PLAIN, false>(x, w, p, M, N, K, num_sms, s);
   if (mode == EPI_RESIDUAL) return dispatch_gemm<EPI_RESIDUAL, false>(x, w, p, M, N, K, num_sms, s);
   return dispatch_gemm<EPI_SWIGLU, false>(x, w, p, M, N, K, num_sms, s);
-}
-
-// Grouped form of the token-major GEMM: x [M, K] with M a multiple of 128 and every 128-row tile belonging to one of
-// `groups` weight matrices w [groups][N, K]; out[m] = W_(tile_group[m / 128]) x[m] (bf16 or fp32, row pitch N).  tiles_used
-// (optional, device): how many leading 128-row tiles hold rows; the rest are not computed.
-extern "C" JL_API int jl_gemm_grouped(const void* x, const void* w, void* out, int M, int N, int K, int groups,
-                                      const int* tile_group, const int* tiles_used, int out_f32, int num_sms, void* stream) {
-  JL_CHECK_ARG(M >= GEMM_BM && M % GEMM_BM == 0, "jl_gemm_grouped: M=%d must be a multiple of %d", M, GEMM_BM);
-  JL_CHECK_ARG(N >= 8 && N % 8 == 0 && K >= 8 && K % 8 == 0 && groups >= 1 && tile_group != nullptr,
-               "jl_gemm_grouped: bad shape N=%d K=%d groups=%d", N, K, groups);
-  if (num_sms <= 0) num_sms = 148;
-  GemmParams p{};
-  p.out = out;
-  p.K = K;
-  p.ldo = N;
-  p.Ra = M; p.Rb = N;
-  p.hint_a = tc::EVICT_NORMAL; p.hint_b = tc::EVICT_LAST;
-  p.tile_group = tile_group;
-  p.group_rows = N;
-  p.a_blocks_used = tiles_used;
-  auto s = (cudaStream_t)stream;
-  if (out_f32) {
-    if (N >= 256) return launch_gemm<256, EPI_PLAIN, true>(x, w, p, M, N, K, num_sms, s, groups);
-    return launch_gemm<128, EPI_PLAIN, true>(x, w, p, M, N, K, num_sms, s, groups);
-  }
-  if (N >= 256) return launch_gemm<256, EPI_PLAIN, false>(x, w, p, M, N, K, num_sms, s, groups);
-  return launch_gemm<128, EPI_PLAIN, false>(x, w, p, M, N, K, num_sms, s, groups);
 }

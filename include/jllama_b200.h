@@ -380,6 +380,13 @@ int jl_moe_gather(const void* x, int ldx, const int* row_src, void* xs, int rows
  * tiles_used (optional, device int): only that many leading tiles are computed. */
 int jl_gemm_grouped(const void* x, const void* w, void* out, int M, int N, int K, int groups, const int* tile_group,
                     const int* tiles_used, int out_f32, int num_sms, void* stream);
+/* The same with bf16 results and an activation on the rounded value. */
+int jl_gemm_grouped_act(const void* x, const void* w, void* out, int M, int N, int K, int groups, const int* tile_group, const int* tiles_used, int act,
+                        int num_sms, void* stream);
+/* Gated activation behind the product: out [M, F] (bf16) = glu(gate, up), the fp32 products of x [M, K] with F weight rows from g_off and F from u_off of
+ * w [groups][w_rows, K]; kind, act, limit, alpha as in jl_glu_act.  tile_group NULL: one matrix, any M; else as in jl_gemm_grouped.  F % 8 == 0, K % 8 == 0. */
+int jl_gemm_glu(const void* x, const void* w, void* out, int M, int F, int K, int w_rows, int g_off, int u_off, int groups, const int* tile_group,
+                const int* tiles_used, int kind, int act, float limit, float alpha, int num_sms, void* stream);
 
 /* ---- token embedding with a hashed pair table, short convolutions with state, delta-rule and state-space scans,
  *      gated activations and the norms around mixers that run side by side (csrc/seq_mix.cu, delta_scan.cu, gla_scan.cu) */

@@ -28,6 +28,25 @@ def _gated_act(y: torch.Tensor, u_off: int, F: int, act: str, limit: float, dtyp
     return SK.glu_act(y, 0, u_off, F, dtype, kind=SK.GLU_PRODUCT, act=SK.ACTIVATIONS[act], **kw)
 
 
+def _gated_product(h: torch.Tensor, w: torch.Tensor, u_off: int, F: int, act: str, limit: float, **kw) -> torch.Tensor:
+    """act(gate h) · (up h) in one tensor-core kernel (bfloat16 prompts)."""
+    if act == "glu_clamped":
+        return SK.gemm_glu(h, w, u_off, F, kind=SK.GLU_CLAMPED, limit=limit, alpha=GLU_ALPHA, **kw)
+    return SK.gemm_glu(h, w, u_off, F, kind=SK.GLU_PRODUCT, act=SK.ACTIVATIONS[act], **kw)
+
+
+def _takes_gated_product(h: torch.Tensor, F: int) -> bool:
+    return (SK.tensor_cores_enabled() and h.dtype == torch.bfloat16 and h.shape[0] > 128 and h.shape[1] % 8 == 0 and F % 8 == 0
+            and h.is_contiguous() and h.data_ptr() % 16 == 0)
+
+
+def _gated_layer(h: torch.Tensor, w: torch.Tensor, u_off: int, F: int, act: str, limit: float) -> torch.Tensor:
+    """act(gate h) · (up h) of a dense layer whose gate and up rows are stacked in w, in h's type."""
+    if _takes_gated_product(h, F):
+        return _gated_product(h, w, u_off, F, act, limit)
+    return _gated_act(SK.linear(h, w, resident=True), u_off, F, act, limit, h.dtype)
+
+
 def _softplus(z: float) -> float:
     return z if z > 30.0 else math.log1p(math.exp(z))
 
@@ -73,7 +92,7 @@ class DenseFeedForward:
 
     def run(self, h: torch.Tensor) -> torch.Tensor:
         if self.spec.gated:
-            t = _gated_act(SK.linear(h, self.up, resident=True), self.u_off, self.spec.ff, self.spec.act, 0.0, h.dtype)
+            t = _gated_layer(h, self.up, self.u_off, self.spec.ff, self.spec.act, 0.0)
         else:
             t = SK.linear(h, self.up, act=self.act, p0=self.p0, p1=self.p1, out_f32=False, resident=True)
         return SK.linear(t, self.down, resident=True)
@@ -174,8 +193,7 @@ class MoeFeedForward:
             pos, row_src, tile_group, used = SK.moe_sort(idx, s.experts, tile=SK.GEMM_TILE_ROWS)
             xs = SK.moe_gather(h, row_src)
             if s.gated:
-                gu = SK.gemm_grouped(xs, self.up, tile_group, tiles_used=used)
-                t = _gated_act(gu, self.u_off, s.ff, s.act, s.limit, h.dtype, rows_used=used, rows_mult=SK.GEMM_TILE_ROWS)
+                t = _gated_product(xs, self.up, self.u_off, s.ff, s.act, s.limit, tile_group=tile_group, tiles_used=used)
             else:
                 t = SK.gemm_grouped(xs, self.up, tile_group, act=self.act, out_f32=False, tiles_used=used)
             y = SK.gemm_grouped(t, self.down, tile_group, tiles_used=used)
@@ -195,7 +213,7 @@ class MoeFeedForward:
         gate = None
         if self.has_shared:
             if s.gated:
-                u = _gated_act(SK.linear(h, self.shared_up, resident=True), self.shared_u_off, s.shared_ff, s.act, s.shared_limit, h.dtype)
+                u = _gated_layer(h, self.shared_up, self.shared_u_off, s.shared_ff, s.act, s.shared_limit)
             else:
                 u = SK.linear(h, self.shared_up, act=self.act, out_f32=False, resident=True)
             shared = SK.linear(u, self.shared_down, resident=True)

@@ -84,6 +84,8 @@ _HYBRID = {
     "jl_moe_sort": (i32, [ip] + [i32] * 5 + [ip, ip, ip, ip, vp]),
     "jl_moe_gather": (i32, [vp, i32, ip, vp, i32, i32, i32, vp]),
     "jl_gemm_grouped": (i32, [vp, vp, vp, i32, i32, i32, i32, ip, ip, i32, i32, vp]),
+    "jl_gemm_grouped_act": (i32, [vp, vp, vp, i32, i32, i32, i32, ip, ip, i32, i32, vp]),
+    "jl_gemm_glu": (i32, [vp, vp, vp] + [i32] * 7 + [ip, ip, i32, i32, f32, f32, i32, vp]),
     "jl_moe_combine": (i32, [fp, i32, ip, fp, i32, fp, i32, fp, i32, fp, i32, i32, vp]),
     "jl_embed_pair_norm": (i32, [ip, vp, vp, vp, fp, ip, ip, ip] + [i32] * 5 + [i64, i64, f32, i32, vp]),
     "jl_causal_conv": (i32, [fp, i32, i32, i32, fp, vp, vp, fp, fp, i32, ip, ip] + [i32] * 5 + [vp]),

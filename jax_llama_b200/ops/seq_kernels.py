@@ -465,18 +465,39 @@ def gemm_grouped(x: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, *, 
                  tiles_used: Optional[torch.Tensor] = None) -> torch.Tensor:
     """tcgen05 GEMM over sorted rows: x bf16 [rows, K] (rows a multiple of 128, contiguous), w bf16 [n, N, K]; 128-row
     tile t runs against w[tile_group[t]]; with `tiles_used` (device int) only that many leading tiles are computed
-    (the rows after them are left as they are).  The activation is an in-place pass over the stored result."""
+    (the rows after them are left as they are).  The activation acts on the stored result, bf16 results on the rounded value: in the kernel
+    (bf16) or in place behind it (fp32)."""
     _need(x, torch.bfloat16, "x")
     _need(w, torch.bfloat16, "w")
     n, N, K = w.shape
     rows = x.shape[0]
     out = torch.empty((rows, N), dtype=torch.float32 if out_f32 else torch.bfloat16, device=x.device)
     L = _lib.lib()
+    if act != ACT_NONE and not out_f32:
+        _lib.check(L.jl_gemm_grouped_act(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, N, K, n, tile_group.data_ptr(), _p(tiles_used),
+                                         act, num_sms(x.device), _stream()), "jl_gemm_grouped_act")
+        return out
     _lib.check(L.jl_gemm_grouped(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, N, K, n, tile_group.data_ptr(), _p(tiles_used),
                                  int(out_f32), num_sms(x.device), _stream()), "jl_gemm_grouped")
     if act != ACT_NONE:
         _lib.check(L.jl_act_inplace(out.data_ptr(), out.stride(0), rows, N, act, 0.0, 0.0, dtype_code(out.dtype), _stream()),
                    "jl_act_inplace")
+    return out
+
+
+def gemm_glu(x: torch.Tensor, w: torch.Tensor, u_off: int, F: int, *, kind: int = GLU_PRODUCT, act: int = ACT_GELU_TANH, limit: float = 0.0,
+             alpha: float = 1.0, tile_group: Optional[torch.Tensor] = None, tiles_used: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """glu(x Wgᵀ, x Wuᵀ) in bf16 [rows, F] without the fp32 product in memory: Wg the first F rows of w, Wu the F rows from u_off.  w [N, K], or
+    [n, N, K] over sorted rows as in `gemm_grouped`.  The activation acts on the fp32 sums, as `glu_act` does."""
+    _need(x, torch.bfloat16, "x")
+    _need(w, torch.bfloat16, "w")
+    if not (x.is_contiguous() and w.is_contiguous()):
+        raise ValueError("gemm_glu: contiguous operands")
+    n, N, K = w.shape if w.dim() == 3 else (1, *w.shape)
+    rows = x.shape[0]
+    out = x.new_empty((rows, F))
+    _lib.check(_lib.lib().jl_gemm_glu(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, F, K, N, 0, int(u_off), n, _p(tile_group), _p(tiles_used), kind,
+                                      act, float(limit), float(alpha), num_sms(x.device), _stream()), "jl_gemm_glu")
     return out
 
 

@@ -1,0 +1,59 @@
+"""Gated activations behind the tensor-core product, at the edges of its tiles, against float64."""
+import pytest
+import torch
+
+from jax_llama_b200.ops import seq_kernels as SK
+
+pytestmark = pytest.mark.gpu
+
+ACTS = {"silu": lambda z: z * torch.sigmoid(z), "relu": torch.relu, "relu2": lambda z: torch.relu(z) ** 2,
+        "gelu_tanh": lambda z: torch.nn.functional.gelu(z, approximate="tanh")}
+
+
+@pytest.mark.parametrize("M", [1, 127, 128, 129, 300])
+@pytest.mark.parametrize("F,Kd,gap", [(8, 8, 0), (120, 72, 16), (128, 64, 0), (136, 520, 8), (1000, 256, 0)])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "relu", "relu2", "clamped"])
+def test_gated_product(M, F, Kd, gap, act):
+    """fp32 sums of K products (2^-17 of the sum of their sizes, tensor cores cut off when they add), fp32 activations, one rounding to bfloat16; nothing
+    beyond the result is written."""
+    g = torch.Generator().manual_seed(M + F + Kd)
+    x, w = torch.randn(M, Kd, generator=g).bfloat16(), torch.randn(2 * F + gap, Kd, generator=g).bfloat16()
+    gate, up = (x.double() @ w[o:o + F].double().T for o in (0, F + gap))
+    size = [x.double().abs() @ w[o:o + F].double().abs().T for o in (0, F + gap)]
+    if act == "clamped":
+        a, b = gate.clamp(max=7.0), up.clamp(-7.0, 7.0)
+        want = a * torch.sigmoid(1.702 * a) * (b + 1.0)
+        kw, slope, outer = dict(kind=SK.GLU_CLAMPED, limit=7.0, alpha=1.702), 1.2, b.abs() + 1.0
+        inner = a.abs()
+    else:
+        want = ACTS[act](gate) * up
+        kw, slope, outer = dict(act=SK.ACTIVATIONS[act]), 1.2 if act != "relu2" else 2.0 * gate.abs().clamp(min=1.0), up.abs()
+        inner = ACTS[act](gate).abs()
+    got = SK.gemm_glu(x.cuda(), w.cuda(), F + gap, F, **kw).double().cpu()
+    bound = 2.0 ** -8 * want.abs() + 2.0 ** -17 * (slope * size[0] * outer + size[1] * inner) + 1e-6
+    assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() - bound).max())
+
+
+@pytest.mark.parametrize("act", [SK.ACT_NONE, SK.ACT_RELU2, SK.ACT_SILU])
+@pytest.mark.parametrize("N,Kd", [(8, 64), (264, 136), (512, 1024)])
+def test_sorted_rows(N, Kd, act):
+    """Tiles of several matrices, padding tiles, a device count that leaves the last tiles alone; the gated form over the same rows."""
+    g = torch.Generator().manual_seed(N)
+    x, w = torch.randn(640, Kd, generator=g).bfloat16().cuda(), (torch.randn(3, 2 * N, Kd, generator=g) * Kd ** -0.5).bfloat16().cuda()
+    group, used = torch.tensor([2, 0, -1, 1, 1], dtype=torch.int32, device="cuda"), torch.tensor([4], dtype=torch.int32, device="cuda")
+    for out_f32 in ((False, True) if act == SK.ACT_NONE else (False,)):
+        got = SK.gemm_grouped(x, w, group, act=act, out_f32=out_f32, tiles_used=used)
+        for t in (0, 1, 3):
+            want = x[t * 128:(t + 1) * 128].double() @ w[int(group[t])].double().T
+            if not out_f32:
+                want = want.bfloat16().double()
+                want = {SK.ACT_NONE: want, SK.ACT_RELU2: torch.relu(want) ** 2, SK.ACT_SILU: want * torch.sigmoid(want)}[act]
+            err = (got[t * 128:(t + 1) * 128].double() - want).abs()
+            # a value that rounds the other way before the activation: two roundings, slope at most 2 max(1, |value|)
+            assert bool((err <= (1e-4 if out_f32 else 2.0 ** -6 * (1.0 + want.abs()))).all())
+    glu = SK.gemm_glu(x, w, N, N, act=SK.ACT_SILU, tile_group=group, tiles_used=used)
+    for t in (0, 1, 3):
+        a = x[t * 128:(t + 1) * 128].double()
+        gate, up = a @ w[int(group[t]), :N].double().T, a @ w[int(group[t]), N:].double().T
+        want = gate * torch.sigmoid(gate) * up
+        assert bool(((glu[t * 128:(t + 1) * 128].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all())

@@ -52,6 +52,13 @@ def test_tile_counts(M, N, Kd, mode):
     _check(M, N, Kd, mode)
 
 
+@pytest.mark.parametrize("M", [129, 130, 1000, 2048, 9472])
+@pytest.mark.parametrize("N,Kd", [(8, 512), (32, 2048), (40, 520), (64, 1032)])
+def test_few_features_over_many_tokens(M, N, Kd):
+    _check(M, N, Kd, "f32")
+    _check(M, N, Kd, "f32", shift=1)
+
+
 @pytest.mark.parametrize("shift", [1, 2, 3])
 @pytest.mark.parametrize("M,N,Kd", [(20, 1024, 2048), (20, 40000, 64)])
 @pytest.mark.parametrize("mode", ["plain", "residual", "swiglu", "f32"])

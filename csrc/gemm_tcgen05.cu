@@ -257,6 +257,7 @@ static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int R
                        cudaStream_t stream) {
   GemmParams p = p0;
   p.trace = g_gemm_trace;
+  JL_CHECK_ARG((((uintptr_t)p.out | (uintptr_t)p.residual) & 15) == 0, "jl_gemm: result and residual of the token-major kernel start on a 16-byte boundary");
   CUtensorMap ta, tb;
   int rc = make_tmap_2d_bf16(&ta, a, Ra, K, K, GEMM_BM);
   if (rc) return rc;

@@ -15,11 +15,11 @@
 //     associative, hence bit-identical on every rank and every run (float atomics are not);
 //   * a cluster of up to 8 CTAs shares a row.  ONE pass over the logits fills a histogram (counts and masses) over equal steps of
 //     z below the row's maximum; its prefix sums answer all three questions down to a bin, because top-k and top-p only cut the
-//     same cumulative sum off at an earlier point.  The few elements of the bin are then gathered and ranked exactly; a bin with
+//     same cumulative sum off at an earlier point.  The few elements of all their bins are then gathered and ranked exactly; a bin with
 //     more than SF_CAND elements (plateaus, coarse logits) is first narrowed by histograms over its own (key, ~index) range.
 //     What bounds it is the chain of cluster barriers and short passes, not the 0.5 MB of a row: 4 rows of 128256, top-p 0.95, on
 //     one B200: 632 us with one CTA per row and three radix passes per question (the top bits of normal logits fall into a few
-//     dozen bins, so its 64-bit shared-memory atomics serialised), 30 us now;
+//     dozen bins, so its 64-bit shared-memory atomics serialised), 30 us with one gather per question, 25 us with one gather for all;
 //   * rows that hold a NaN or whose maximum is not finite take the radix select that the first form of this kernel ran for every
 //     row (sf_select): their masses are not sums of probabilities, and what they return stays what it was.
 //   * tensor parallelism: the decode kernel stores every rank's logits shard into every rank's [B, V] buffer with
@@ -275,6 +275,11 @@ struct SfShared {
   unsigned long long rlo[SF_MAX_CLUSTER], rhi[SF_MAX_CLUSTER];
   unsigned long long base_m; unsigned int base_c;
   unsigned long long res_comp, res_before, res_mass;
+  // all questions at once: ranges of bins to gather (rank 0's decision, written into every CTA), per candidate its bin and the sums before it
+  int ranges, range_lo[3], range_hi[3], at[2];
+  int cbin[SF_CAND];
+  unsigned long long cbefore[SF_CAND];
+  unsigned int crank_of[SF_CAND];
 };
 
 struct SfBest {
@@ -304,14 +309,23 @@ struct SfCluster {
   bool count_all;               // elements without mass count too (a top-k question will be asked)
   SfRow row;
 
-  template <typename F> __device__ __forceinline__ void for_slice(F f) const {
+  template <int N = 4, typename F> __device__ __forceinline__ void for_slice(F f) const {
     if (vec) {                                              // lo is a multiple of four
-      for (int i = lo + 4 * (int)threadIdx.x; i < hi; i += 4 * SF_THREADS) {
-        if (i + 4 <= hi) {
-          const float4 v = *reinterpret_cast<const float4*>(x + i);
-          f(v.x, i); f(v.y, i + 1); f(v.z, i + 2); f(v.w, i + 3);
-        } else {
-          for (int j = i; j < hi; ++j) f(x[j], j);
+      // N loads in flight: a slice of a 128 k row is four rounds, each a memory latency when they follow one another (two for the arg-max
+      // alone, whose two CTAs per SM have 32 registers a thread: 64 rows of 128256 24 -> 18 us)
+      for (int i0 = lo + 4 * (int)threadIdx.x; i0 < hi; i0 += 4 * N * SF_THREADS) {
+        float4 v[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u)
+          if (i0 + 4 * SF_THREADS * u + 4 <= hi) v[u] = *reinterpret_cast<const float4*>(x + i0 + 4 * SF_THREADS * u);
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+          const int i = i0 + 4 * SF_THREADS * u;
+          if (i + 4 <= hi) {
+            f(v[u].x, i); f(v[u].y, i + 1); f(v[u].z, i + 2); f(v[u].w, i + 3);
+          } else {
+            for (int j = i; j < hi; ++j) f(x[j], j);
+          }
         }
       }
     } else {
@@ -354,7 +368,9 @@ struct SfCluster {
     for (int b = rank * share + threadIdx.x; b < (rank + 1) * share; b += SF_THREADS) {
       unsigned long long m = 0;
       unsigned int c = 0;
-      for (int r = 0; r < size; ++r) {
+#pragma unroll
+      for (int r = 0; r < SF_MAX_CLUSTER; ++r) {                    // (unrolled: all CTAs' numbers on their way at once)
+        if (r >= size) continue;
         const SfShared* o = cl.map_shared_rank(s, r);
         c += o->cnt[b];
         m += (unsigned long long)o->m0[b] + ((unsigned long long)o->m1[b] << 14) + ((unsigned long long)o->m2[b] << 28);
@@ -529,6 +545,108 @@ struct SfCluster {
     }
     __syncthreads();
   }
+
+  // rank 0: the bins that hold lo and hi (masses, below the total) -> s->at
+  __device__ __forceinline__ void find_two(unsigned long long lo_t, unsigned long long hi_t) const {
+    for (int b = threadIdx.x; b < SF_BINS; b += SF_THREADS) {
+      const unsigned long long a = s->pm[b], e = s->pm[b + 1];
+      if (a <= lo_t && lo_t < e) s->at[0] = b;
+      if (a <= hi_t && hi_t < e) s->at[1] = b;
+    }
+    __syncthreads();
+  }
+  // Every question of the row from one gather.  What top-k keeps lies between the sums before and behind the bin of its boundary, so the
+  // next target lies in a range of bins, almost always one, and so on: the bins of all answers are known before any answer is, and when they
+  // hold few enough elements these are gathered together and the questions answered one after the other by rank 0 alone.  The sums are the
+  // same integers that select() forms.  False (in every CTA): more than SF_CAND elements, nothing was answered, select() goes on.
+  // It saves a pass over the slice and two cluster barriers per question: 4 rows of 128256, top-k 50 and top-p 0.9, 36 -> 27 us from one
+  // event to the next; top-p 0.95 alone 32 -> 27; 200 rows, both, 222 -> 135.
+  template <typename Target>
+  __device__ bool all_at_once(int top_k, float top_p, float u01, unsigned long long total, Target target_of, int* token) const {
+    cg::cluster_group cl = cg::this_cluster();
+    SfShared* lead = cl.map_shared_rank(s, 0);
+    if (rank == 0) {
+      int nr = 0, n = 0, lo_b[3], hi_b[3];
+      unsigned long long t_lo = total, t_hi = total;                // bounds of the kept set's mass
+      auto range = [&](int a, int b) {
+        if (nr == 0 || lo_b[nr - 1] != a || hi_b[nr - 1] != b) {    // (the same bins again: gathered once)
+          n += (int)(s->pc[b + 1] - s->pc[a]);
+          lo_b[nr] = a; hi_b[nr] = b; ++nr;
+        }
+        t_lo = s->pm[a]; t_hi = s->pm[b + 1];
+      };
+      if (count_all) {
+        find(s->pm, s->pc, true, (unsigned long long)(top_k - 1));
+        range(s->bin, s->bin);
+      }
+      if (top_p < 1.0f) {
+        find_two(target_of(t_lo, (double)top_p), target_of(t_hi, (double)top_p));
+        range(s->at[0], s->at[1]);
+        __syncthreads();                                            // (s->at is written again)
+      }
+      find_two(target_of(t_lo, (double)u01), target_of(t_hi, (double)u01));
+      range(s->at[0], s->at[1]);
+      if (n > SF_CAND) nr = 0;
+      if ((int)threadIdx.x < size) {
+        SfShared* o = cl.map_shared_rank(s, (int)threadIdx.x);
+        o->ranges = nr;
+        for (int k = 0; k < nr; ++k) { o->range_lo[k] = lo_b[k]; o->range_hi[k] = hi_b[k]; }
+      }
+      if (threadIdx.x == 0) s->n_cand = 0;
+    }
+    sf_sync(cl, size);
+    const int nr = s->ranges;
+    if (nr == 0) return false;
+    int lo_b[3], hi_b[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { lo_b[k] = k < nr ? s->range_lo[k] : 1; hi_b[k] = k < nr ? s->range_hi[k] : 0; }
+    for_slice([&](float v, int i) {
+      const float z = sf_scaled(v, inv_temp);
+      const int b = bin_of(z);
+      if (!((b >= lo_b[0] && b <= hi_b[0]) || (b >= lo_b[1] && b <= hi_b[1]) || (b >= lo_b[2] && b <= hi_b[2]))) return;
+      if (!count_all && sf_mass(row, z) == 0) return;
+      const unsigned slot = atomicAdd(&lead->n_cand, 1u);
+      if (slot < SF_CAND) lead->cand[slot] = comp(sf_key(z), i);
+    });
+    sf_sync(cl, size);
+    if (rank != 0) return true;
+    const int nc = min((int)s->n_cand, SF_CAND), t = threadIdx.x;
+    if (t < nc) {
+      const float z = z_of(s->cand[t]);
+      s->cmass[t] = sf_mass(row, z);
+      s->cbin[t] = bin_of(z);
+    }
+    __syncthreads();
+    const int c = t >> 2;
+    const unsigned long long mine = c < nc ? s->cand[c] : 0ull;
+    const int my_bin = c < nc ? s->cbin[c] : -1;
+    unsigned long long bm = 0;
+    unsigned int bc = 0;
+    for (int j = t & 3; j < nc; j += 4)
+      if (s->cand[j] > mine && s->cbin[j] == my_bin) { bm += s->cmass[j]; ++bc; }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) { bm += __shfl_xor_sync(0xffffffffu, bm, o); bc += __shfl_xor_sync(0xffffffffu, bc, o); }
+    if (c < nc && (t & 3) == 0) { s->cbefore[c] = bm + s->pm[my_bin]; s->crank_of[c] = bc + s->pc[my_bin]; }
+    if (t == 0) { s->res_comp = 0x7fffffffull; s->res_before = 0; s->res_mass = 0; }
+    __syncthreads();
+    auto answer = [&](bool by_count, unsigned long long target) {
+      if (t < nc) {
+        const unsigned long long a = s->cbefore[t], m = s->cmass[t];
+        if (by_count ? (unsigned long long)s->crank_of[t] == target : a <= target && target - a < m) {
+          s->res_comp = s->cand[t]; s->res_before = a; s->res_mass = m;
+        }
+      }
+      __syncthreads();
+      const unsigned long long kept = s->res_before + s->res_mass;
+      __syncthreads();
+      return kept;
+    };
+    if (count_all) total = answer(true, (unsigned long long)(top_k - 1));
+    if (top_p < 1.0f) total = answer(false, target_of(total, (double)top_p));
+    answer(false, target_of(total, (double)u01));
+    *token = 0x7fffffff - (int)(s->res_comp & 0xffffffffu);
+    return true;
+  }
 };
 
 // GREEDY (temperature 0): the arg-max alone, without the histograms' shared memory and registers (two CTAs fit an SM).
@@ -582,7 +700,7 @@ __global__ void __launch_bounds__(SF_THREADS, GREEDY ? 2 : 1) sample_full_kernel
     uint32_t bk = 0;                                        // a thread's indices ascend: the first of equal keys stays
     int bi = 0x7fffffff;
     bool nan = false;
-    q.for_slice([&](float v, int i) {
+    q.for_slice<GREEDY ? 2 : 4>([&](float v, int i) {
       const float z = sf_scaled(v, p.inv_temp);
       const uint32_t key = sf_key(z);
       if (key > bk || bi == 0x7fffffff) { bk = key; bi = i; }
@@ -625,21 +743,23 @@ __global__ void __launch_bounds__(SF_THREADS, GREEDY ? 2 : 1) sample_full_kernel
       q.merge(false);
       unsigned long long total = crank == 0 ? sh.pm[SF_BINS] : 0;
       // target of a fraction of the kept set's mass Z: max(fraction·Z, 1) − 1 (a token is kept while the mass before it is < fraction·Z)
-      auto target_of = [&](double fraction) {
-        unsigned long long t = (unsigned long long)((double)total * fraction);
-        if (t > total) t = total;
+      auto target_of = [](unsigned long long z, double fraction) -> unsigned long long {
+        unsigned long long t = (unsigned long long)((double)z * fraction);
+        if (t > z) t = z;
         return t > 0 ? t - 1 : 0;
       };
-      if (q.count_all) {
-        q.select(true, (unsigned long long)(p.top_k - 1));
-        if (crank == 0) total = sh.res_before + sh.res_mass;
+      if (!q.all_at_once(p.top_k, p.top_p, u01, total, target_of, &token)) {
+        if (q.count_all) {
+          q.select(true, (unsigned long long)(p.top_k - 1));
+          if (crank == 0) total = sh.res_before + sh.res_mass;
+        }
+        if (p.top_p < 1.0f) {
+          q.select(false, target_of(total, (double)p.top_p));
+          if (crank == 0) total = sh.res_before + sh.res_mass;
+        }
+        q.select(false, target_of(total, (double)u01));
+        if (crank == 0) token = 0x7fffffff - (int)(sh.res_comp & 0xffffffffu);
       }
-      if (p.top_p < 1.0f) {
-        q.select(false, target_of((double)p.top_p));
-        if (crank == 0) total = sh.res_before + sh.res_mass;
-      }
-      q.select(false, target_of((double)u01));
-      if (crank == 0) token = 0x7fffffff - (int)(sh.res_comp & 0xffffffffu);
     }
   }
   sf_sync(cl, csize);                                                // no CTA leaves while another may still write into its shared memory
@@ -711,8 +831,8 @@ extern "C" JL_API int jl_sample_full(const float* logits, int B, int V, int ld, 
   // CTAs per row: as many as leave every CTA a slice of at least 4096 logits (below that the barriers cost more than the slice) and
   // all rows' CTAs resident at once, one per SM.  Clusters of eight only where two thirds of the SMs hold them: a cluster stays within
   // one GPC, and 16 of eight did not all fit (16 rows of 128256: 51 us in clusters of eight, 38 us of four).
-  // Measured, nucleus 0.95, one CTA with radix passes -> now: 1 x 8000 78 -> 19 us, 1 x 32000 177 -> 25, 4 x 128256 632 -> 29,
-  // 24 x 128256 650 -> 39, 64 x 128256 645 -> 59, 200 x 128256 1062 -> 180, 2000 x 8000 685 -> 191; equal logits 27.4 ms -> 70 us.
+  // Measured, nucleus 0.95, one CTA with radix passes -> now: 1 x 8000 78 -> 18 us, 1 x 32000 177 -> 21, 4 x 128256 632 -> 27,
+  // 24 x 128256 650 -> 35, 64 x 128256 645 -> 47, 200 x 128256 1062 -> 135; equal logits 27.4 ms -> 70 us.
   int C = 1;
   while (C < SF_MAX_CLUSTER && V / (2 * C) >= 4096 && (long)B * 2 * C <= (2 * C < SF_MAX_CLUSTER ? num_sms : num_sms * 2 / 3)) C *= 2;
   auto* kernel = greedy ? sample_full_kernel<true> : sample_full_kernel<false>;

@@ -1,5 +1,8 @@
 """Exact full-vocabulary sampler (csrc/sample_full.cu) against the fp32 statement of the HF warper pipeline the
 reference configures in jax_llama/generation.py:28-41 (temperature → top-k → top-p → categorical)."""
+import itertools
+import math
+
 import pytest
 import torch
 
@@ -159,3 +162,31 @@ def test_clusters_exchange_their_best_after_all_of_them_have_started(rows, vocab
     drawn = [K.sample_full(y, temperature=0.8, top_p=0.9, seed=1) for y in inputs]
     for a, t, u in zip(at, greedy, drawn):
         assert (t == a).all() and (u == a).all()
+
+
+@pytest.mark.parametrize("first,second", [(1, 0), (255, 1), (128, 128), (128, 129), (256, 300), (257, 0), (90, 200)])
+@pytest.mark.parametrize("vocab,skew", [(5000, 0), (20000, 3), (131072, 0)])
+def test_answers_from_one_gather_and_from_several_agree_at_its_limit(first, second, vocab, skew):
+    """Two plateaus one apart and nothing else: the boundaries of top-k, top-p and the draw fall into one bin or two, which hold up to 256 elements
+    (one gather for all three) or more.  Within the plateaus every mass is known to 2^-21 of itself, so over at most 556 elements a sum is
+    out by less than a thousandth of the smallest mass: the token's place in the order is the computed one or, next to an edge, its neighbour."""
+    g = torch.Generator().manual_seed(first * 1000 + second)
+    x = torch.full((3, vocab + skew), float("-inf"))
+    orders = []
+    for r in range(3):
+        place = torch.randperm(vocab, generator=g)[:first + second]
+        top, low = place[:first].sort().values, place[first:].sort().values
+        x[r, top], x[r, low] = 2.0, 1.0
+        orders.append(torch.cat([top, low]).tolist())
+    dev = x.cuda()[:, :vocab]
+    mass = [1.0] * first + [math.exp(-1.0)] * second
+    for top_k, top_p in ((0, 1.0), (0, 0.6), (first + second // 2, 1.0), (first + second // 2, 0.9), (max(first // 2, 1), 0.3)):
+        for seed in range(4):
+            tok = K.sample_full(dev, temperature=1.0, top_k=top_k, top_p=top_p, seed=seed, step=torch.tensor([seed], dtype=torch.int32, device="cuda")).tolist()
+            for r in range(3):
+                kept = mass[:top_k] if top_k else mass
+                edge = list(itertools.accumulate(kept))
+                if top_p < 1.0:
+                    edge = edge[:1 + sum(e < top_p * edge[-1] for e in edge)]
+                want = sum(e <= uniform_of(seed, seed, r) * edge[-1] for e in edge)
+                assert abs(orders[r].index(tok[r]) - want) <= 1, (top_k, top_p, seed, r)

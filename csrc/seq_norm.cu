@@ -7,27 +7,61 @@
 
 namespace jl {
 
+// Bound: one row's latency, not its bytes.  16 bytes of float32 a thread and round (vec), every round's loads in flight together: 2 rows of 2048 9.3 ->
+// 2.4 us a launch in a decode step, whose rows come from memory.
 template <typename T>
-__global__ void embed_f32_kernel(const int* __restrict__ ids, const T* __restrict__ table, float* __restrict__ out, int W,
-                                 int V, float scale) {
+__global__ void __launch_bounds__(256) embed_f32_kernel(const int* __restrict__ ids, const T* __restrict__ table, float* __restrict__ out, int W,
+                                 int V, float scale, int vec) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
   pdl_launch_dependents();
   const int m = blockIdx.x;
   int id = ids[m];
   id = id < 0 ? 0 : (id >= V ? V - 1 : id);
   const T* row = table + (size_t)id * W;
+  if (vec) {                       // W % 4 == 0, all rows on the access's boundary
+#pragma unroll 4
+    for (int i = 4 * threadIdx.x; i < W; i += 4 * blockDim.x) {
+      float v[4];
+      load4(row + i, v);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] *= scale;
+      store4(out + (size_t)m * W + i, v);
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < W; i += blockDim.x) out[(size_t)m * W + i] = to_f(row[i]) * scale;
 }
 
 // out[m, :] = x[m, :] / sqrt(mean(x^2) + eps) * (offset + w)
-template <typename T>
-__global__ void norm_f32_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restrict__ out, int W, float eps,
+// Rows of up to 256 * VPT elements stay in registers, the weights beside them: one memory latency per launch where the loop (VPT 0) has one per
+// group of unrolled loads and another for the weights behind the sum.  The additions are the loop's.  2 rows of 2048 in a decode step: 6.3 -> 2.0 us.
+template <typename T, int VPT>
+__global__ void __launch_bounds__(256) norm_f32_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restrict__ out, int W, float eps,
                                 float offset) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
   pdl_launch_dependents();
   __shared__ float red[33];
   const float* xr = x + (size_t)blockIdx.x * W;
   float ss = 0.0f;
+  if constexpr (VPT > 0) {
+    float xv[VPT];
+    T wv[VPT];
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) {
+      const int i = threadIdx.x + 256 * u;
+      xv[u] = i < W ? xr[i] : 0.0f;
+      if (i < W) wv[u] = w[i];
+    }
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) ss += xv[u] * xv[u];
+    const float r = 1.0f / sqrtf(block_sum(ss, red) / (float)W + eps);
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) {
+      const int i = threadIdx.x + 256 * u;
+      if (i < W) out[(size_t)blockIdx.x * W + i] = from_f<T>(xv[u] * r * (offset + to_f(wv[u])));
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < W; i += blockDim.x) { float v = xr[i]; ss += v * v; }
   const float r = 1.0f / sqrtf(block_sum(ss, red) / (float)W + eps);
   for (int i = threadIdx.x; i < W; i += blockDim.x)
@@ -59,7 +93,8 @@ __global__ void postnorm_add_kernel(const float* __restrict__ y, int ldy, const 
 }
 
 // The same step with the row held in registers: 16-byte loads, x and y read once, x and h written once.
-// W % 4 == 0, ldy % 4 == 0, W <= 256 * 4 * VPT.
+// W % 4 == 0, ldy % 4 == 0, W <= 256 * 4 * VPT.  The weights of rows of up to 4096 are asked for with the row itself: behind the two sums each cost a
+// memory latency of its own (2 rows of 2048 in a decode step, where they come from memory: 4.2 -> 2.5 us).
 template <typename T, int VPT>
 __global__ void __launch_bounds__(256) postnorm_add_vec_kernel(const float* __restrict__ y, int ldy, const T* __restrict__ w_post,
                                                                float* __restrict__ x, const T* __restrict__ w_next,
@@ -70,7 +105,9 @@ __global__ void __launch_bounds__(256) postnorm_add_vec_kernel(const float* __re
   const float* yr = y + (size_t)blockIdx.x * ldy;
   float* xr = x + (size_t)blockIdx.x * W;
   const int nv = W / 4;
+  constexpr bool AHEAD = VPT <= 4;
   float yv[VPT][4], xv[VPT][4];
+  Raw4<T> wp[AHEAD ? VPT : 1], wn[AHEAD ? VPT : 1];
   float ss = 0.0f;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
@@ -78,6 +115,16 @@ __global__ void __launch_bounds__(256) postnorm_add_vec_kernel(const float* __re
     if (idx < nv) {
       load4(yr + 4 * idx, yv[i]);
       load4(xr + 4 * idx, xv[i]);
+      if constexpr (AHEAD) {
+        wp[i].load(w_post + 4 * idx);
+        if (w_next != nullptr) wn[i].load(w_next + 4 * idx);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int idx = threadIdx.x + i * 256;
+    if (idx < nv) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) ss += yv[i][j] * yv[i][j];
     }
@@ -89,7 +136,7 @@ __global__ void __launch_bounds__(256) postnorm_add_vec_kernel(const float* __re
     const int idx = threadIdx.x + i * 256;
     if (idx < nv) {
       float wv[4];
-      load4(w_post + 4 * idx, wv);
+      if constexpr (AHEAD) wp[i].get(wv); else load4(w_post + 4 * idx, wv);
 #pragma unroll
       for (int j = 0; j < 4; ++j) { xv[i][j] += yv[i][j] * r * (offset + wv[j]); s2 += xv[i][j] * xv[i][j]; }
       store4(xr + 4 * idx, xv[i]);
@@ -102,7 +149,7 @@ __global__ void __launch_bounds__(256) postnorm_add_vec_kernel(const float* __re
     const int idx = threadIdx.x + i * 256;
     if (idx < nv) {
       float wv[4], hv[4];
-      load4(w_next + 4 * idx, wv);
+      if constexpr (AHEAD) wn[i].get(wv); else load4(w_next + 4 * idx, wv);
 #pragma unroll
       for (int j = 0; j < 4; ++j) hv[j] = xv[i][j] * r2 * (offset + wv[j]);
       store4(h + (size_t)blockIdx.x * W + 4 * idx, hv);
@@ -130,12 +177,18 @@ __global__ void __launch_bounds__(256) branch_add_norm_kernel(const float* __res
   float ss = 0.0f;
   if (vec) {
     const int nv = W / 4;
+    constexpr bool AHEAD = VPT <= 4;                        // the weights with the row, not behind the sum (see postnorm_add_vec_kernel)
     float xv[VPT][4];
+    Raw4<T> r1[AHEAD ? VPT : 1], r2[AHEAD ? VPT : 1];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int idx = threadIdx.x + i * 256;
       if (idx < nv) {
         load4(xr + 4 * idx, xv[i]);
+        if constexpr (AHEAD) {
+          if (w1) r1[i].load(w1 + 4 * idx);
+          if (w2) r2[i].load(w2 + 4 * idx);
+        }
         if (a || b) {
           float s[4] = {0.f, 0.f, 0.f, 0.f}, t[4];
           if (a) load4(a + 4 * idx, s);
@@ -158,13 +211,13 @@ __global__ void __launch_bounds__(256) branch_add_norm_kernel(const float* __res
       if (idx < nv) {
         float wv[4], hv[4];
         if (w1) {
-          load4(w1 + 4 * idx, wv);
+          if constexpr (AHEAD) r1[i].get(wv); else load4(w1 + 4 * idx, wv);
 #pragma unroll
           for (int j = 0; j < 4; ++j) hv[j] = xv[i][j] * r * wv[j];
           store4(h1 + m * W + 4 * idx, hv);
         }
         if (w2) {
-          load4(w2 + 4 * idx, wv);
+          if constexpr (AHEAD) r2[i].get(wv); else load4(w2 + 4 * idx, wv);
 #pragma unroll
           for (int j = 0; j < 4; ++j) hv[j] = xv[i][j] * r * wv[j];
           store4(h2 + m * W + 4 * idx, hv);
@@ -209,12 +262,15 @@ __global__ void __launch_bounds__(THREADS) postnorm_cast_kernel(const float* __r
   float ss = 0.0f;
   if (vec) {
     const int nv = W / 4;
+    constexpr bool AHEAD = VPT <= 4;
     float yv[VPT][4], xv[VPT][4];
+    Raw4<T> wr[AHEAD ? VPT : 1];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int idx = threadIdx.x + i * THREADS;
       if (idx < nv) {
         float t[4];
+        if constexpr (AHEAD) wr[i].load(w + 4 * idx);
         load4(a + 4 * idx, yv[i]);
         load4(xr + 4 * idx, xv[i]);
         if (bias) {
@@ -240,7 +296,7 @@ __global__ void __launch_bounds__(THREADS) postnorm_cast_kernel(const float* __r
       const int idx = threadIdx.x + i * THREADS;
       if (idx < nv) {
         float wv[4];
-        load4(w + 4 * idx, wv);
+        if constexpr (AHEAD) wr[i].get(wv); else load4(w + 4 * idx, wv);
 #pragma unroll
         for (int j = 0; j < 4; ++j) xv[i][j] += yv[i][j] * r * wv[j];
         store4(xr + 4 * idx, xv[i]);
@@ -329,12 +385,14 @@ __global__ void headnorm_gate_kernel(const float* __restrict__ o, const T* __res
   if (vec) {                                              // read-outs and gate in registers, 16 bytes per access
     const float* grow = gate + (size_t)m * ldg + (size_t)hh * V;
     float ov[HG_VEC][4], gv[HG_VEC][4];
+    Raw4<T> wr[HG_VEC];
 #pragma unroll
     for (int u = 0; u < HG_VEC; ++u) {
       const int i = 4 * lane + 128 * u;
       if (i < V) {
         load4(orow + i, ov[u]);
         load4(grow + i, gv[u]);
+        if (w) wr[u].load(w + i);
 #pragma unroll
         for (int e = 0; e < 4; ++e) ss += ov[u][e] * ov[u][e];
       }
@@ -345,7 +403,7 @@ __global__ void headnorm_gate_kernel(const float* __restrict__ o, const T* __res
       const int i = 4 * lane + 128 * u;
       if (i < V) {
         float wv[4] = {1.0f, 1.0f, 1.0f, 1.0f};
-        if (w) load4(w + i, wv);
+        if (w) wr[u].get(wv);
 #pragma unroll
         for (int e = 0; e < 4; ++e) ov[u][e] = ov[u][e] * r * wv[e] * apply_act(gv[u][e], gate_act, 0.f, 0.f);
         store4(out + ((size_t)m * H + hh) * V + i, ov[u]);
@@ -415,7 +473,8 @@ extern "C" JL_API int jl_act_inplace(void* data, int ld, int M, int N, int act, 
 
 extern "C" JL_API int jl_embed_f32(const int* ids, const void* table, float* out, int M, int W, int V, float scale, int dtype, void* stream) {
   JL_CHECK_ARG(M >= 1 && W >= 1 && V >= 1, "jl_embed_f32: bad shape M=%d W=%d V=%d", M, W, V);
-  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(embed_f32_kernel<T>, dim3(M), dim3(128), 0, (cudaStream_t)stream, ids, (const T*)table, out, W, V, scale));
+  const int vec = W % 4 == 0 && (uintptr_t)table % 16 == 0 && (uintptr_t)out % 16 == 0;
+  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(embed_f32_kernel<T>, dim3(M), dim3(256), 0, (cudaStream_t)stream, ids, (const T*)table, out, W, V, scale, vec));
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }
@@ -423,7 +482,10 @@ extern "C" JL_API int jl_embed_f32(const int* ids, const void* table, float* out
 extern "C" JL_API int jl_norm_f32(const float* x, const void* w, void* out, int M, int W, float eps, float offset, int dtype,
                                   void* stream) {
   JL_CHECK_ARG(M >= 1 && W >= 1, "jl_norm_f32: bad shape M=%d W=%d", M, W);
-  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(norm_f32_kernel<T>, dim3(M), dim3(256), 0, (cudaStream_t)stream, x, (const T*)w, (T*)out, W, eps, offset));
+#define JL_NF(V) \
+  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((norm_f32_kernel<T, V>), dim3(M), dim3(256), 0, (cudaStream_t)stream, x, (const T*)w, (T*)out, W, eps, offset))
+  if (W <= 1024) JL_NF(4); else if (W <= 2048) JL_NF(8); else if (W <= 4096) JL_NF(16); else JL_NF(0);
+#undef JL_NF
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }

@@ -75,6 +75,19 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
   *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
 }
 
+// four elements as they lie in memory: asked for early, unpacked where they are used
+template <typename T> struct Raw4;
+template <> struct Raw4<float> {
+  float4 t;
+  __device__ __forceinline__ void load(const float* p) { t = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ void get(float (&v)[4]) const { v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w; }
+};
+template <> struct Raw4<__nv_bfloat16> {
+  uint2 t;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { t = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ void get(float (&v)[4]) const { v[0] = bf16_lo(t.x); v[1] = bf16_hi(t.x); v[2] = bf16_lo(t.y); v[3] = bf16_hi(t.y); }
+};
+
 __device__ __forceinline__ float block_sum(float v, float* red /* >= 33 floats of shared memory */) {
   v = warp_sum(v);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;

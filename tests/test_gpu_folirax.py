@@ -96,6 +96,38 @@ def test_norms(dtype, width):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [4, 1023, 1024, 1028, 2048, 2052, 4095, 4096, 4100])
+@pytest.mark.parametrize("skew", [0, 1])
+def test_norms_and_embedding_at_the_edges_of_their_rows_in_registers(dtype, width, skew):
+    """Widths around the rows that fit a number of registers, on and off the wide accesses' boundary.  fp32 throughout: sums of `width` squares in any
+    order and a handful of operations behind them (2^-23 · (width + 8) of the result, far above what they leave), then the operand type's rounding."""
+    g = torch.Generator().manual_seed(width)
+    x, y = torch.randn(3, width, generator=g) * 3, torch.randn(3, width, generator=g)
+    w1, w2 = (0.2 * torch.randn(width, generator=g)).to(dtype), (0.2 * torch.randn(width, generator=g)).to(dtype)
+    table = torch.randn(11, width, generator=g).to(dtype)
+
+    def place(t):
+        room = torch.zeros(t.numel() + skew, dtype=t.dtype, device="cuda")
+        room[skew:] = t.flatten().cuda()
+        return room[skew:].view(t.shape)
+
+    tol = 2.0 ** -23 * (width + 8)
+    half = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0      # bfloat16: 8 significant bits, so neighbours in [1, 2) are 2^-7 apart and rounding is out by half
+    h = SK.norm_f32(place(x), place(w1), 1e-5, 1.0)
+    want = O.norm_zero_centred(x.double(), w1, 1e-5)
+    assert bool(((h.double().cpu() - want).abs() <= (tol + half) * want.abs()).all())
+    stream = place(x)
+    hn = SK.postnorm_add(place(y), place(w1), stream, 1e-5, 1.0, w_next=place(w2))
+    want_x = x.double() + O.norm_zero_centred(y.double(), w1, 1e-5)
+    assert (stream.double().cpu() - want_x).abs().max() <= tol * want_x.abs().max()
+    want_h = O.norm_zero_centred(want_x, w2, 1e-5)
+    assert bool(((hn.double().cpu() - want_h).abs() <= half * want_h.abs() + tol * want_h.abs().max()).all())
+    ids = [0, 10, 3]
+    got = SK.embed_f32(torch.tensor(ids, dtype=torch.int32, device="cuda"), place(table), scale=0.75)
+    assert torch.equal(got.cpu(), table[ids].float() * 0.75)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("shape", [(1, 40, 72), (3, 33, 100), (8, 96, 64), (9, 104, 72), (70, 56, 328), (200, 264, 136),
                                    (130, 50, 72)])
 def test_linear_paths(dtype, shape):

@@ -25,7 +25,7 @@ constexpr int GS_THREADS = 128;
 constexpr int GS_PITCH = GS_DP + 4;   // floats per 32 channels in shared memory: 16-byte aligned rows, distinct banks per lane group
 
 __device__ __forceinline__ float log_sigmoid(float z) {
-  return z >= 0.0f ? -log1pf(expf(-z)) : z - log1pf(expf(z));
+  return fminf(z, 0.0f) - log1pf(expf(-fabsf(z)));           // (no branch: lanes of either sign took both sides one after the other)
 }
 
 struct GlaParams {
@@ -212,18 +212,91 @@ inline int gla_threads(int P, int Dv) {
 }
 __host__ __device__ inline int gla_record_floats(int P, int Dv) { return 3 * P * GT_PITCH + ((Dv + 3) & ~3); }
 
+// Whether the preparation's options are all off: q, k and v as they lie in y, the decay projected, its rows of A2 in whole pieces of 16 bytes (at
+// most GP_PIECES).  The instance for these calls (PLAIN) is a small part of the general one's code and asks for all that a thread needs at once, before the
+// barrier: 2048 tokens of 16 heads (64 / 128, rank 16) 42 -> 25 us, where 100 MB read and written take 15.
+constexpr int GP_PIECES = 4;
+inline bool gla_plain(const GlaParams& p, const void* a2, int elem) {
+  return p.rot == 0 && p.act == ACT_NONE && p.aux == nullptr && p.head_decay == nullptr && p.ones == 0 && p.qk_div <= 1 &&
+         p.R * elem % 16 == 0 && p.R * elem <= 16 * GP_PIECES && ((uintptr_t)a2 & 15) == 0;
+}
+
 // A thread forms one slot of the records (a channel of a head, or a value column) for GP_TOK tokens: the channel's row of A2 is read once
 // for all of them.  (One CTA per token, its threads walking all channels, read A2 once per token: 60 us for 2048 tokens of 16 x 64 channels
-// against 42 us.)
+// against 42 us in the general instance.)
 constexpr int GP_TOK = 8, GP_THREADS = 256;
 
-template <typename T>
+template <typename T, bool PLAIN>
 __global__ void __launch_bounds__(GP_THREADS) gla_prep_kernel(GlaParams p, const T* __restrict__ a2, const T* __restrict__ a2b,
                                                               float* __restrict__ rec) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
   pdl_launch_dependents();
-  extern __shared__ float zs[];                                 // [GP_TOK][R]
+  extern __shared__ float4 zs4[];                               // [GP_TOK][R]
+  float* zs = reinterpret_cast<float*>(zs4);
   const int M = p.B * p.S, m0 = blockIdx.x * GP_TOK, nt = min(GP_TOK, M - m0);
+  if constexpr (PLAIN) {
+    const int P = p.P, RF = gla_record_floats(P, p.Dv), per_head = P * GT_DP, dvp = (p.Dv + 3) & ~3;
+    const int i = blockIdx.y * GP_THREADS + threadIdx.x, nq = p.H * per_head;
+    const bool value = i >= nq;
+    const int j = value ? i - nq : i, h = value ? j / dvp : j / per_head, d = value ? j % dvp : j % per_head;
+    const bool on = value ? h < p.H && d < p.Dv : d < p.D;
+    const float* src = p.y + (size_t)m0 * p.ldy + (value ? p.v_off + h * p.Dv : p.q_off + h * p.D) + d;
+    const float* ksrc = p.y + (size_t)m0 * p.ldy + p.k_off + h * p.D + d;
+    float qv[GP_TOK], kv[GP_TOK], av[GP_TOK];
+    constexpr int N = 16 / sizeof(T);
+    uint4 row[GP_PIECES];
+    float bias = 0.0f;
+#pragma unroll
+    for (int t = 0; t < GP_TOK; ++t) qv[t] = on && t < nt ? src[(size_t)t * p.ldy] : 0.0f;
+    if (on && !value) {
+#pragma unroll
+      for (int t = 0; t < GP_TOK; ++t) kv[t] = t < nt ? ksrc[(size_t)t * p.ldy] : 0.0f;
+      const int n = h * p.D + d;
+      bias = to_f(a2b[n]);
+#pragma unroll
+      for (int u = 0; u < GP_PIECES; ++u)
+        if (u * N < p.R) row[u] = *reinterpret_cast<const uint4*>(a2 + (size_t)n * p.R + u * N);
+    }
+    for (int e = threadIdx.x; e < GP_TOK * p.R; e += GP_THREADS)
+      zs[e] = e < nt * p.R ? p.y[(size_t)(m0 + e / p.R) * p.ldy + p.a_off + e % p.R] : 0.0f;
+    __syncthreads();
+    if (value) {
+      if (h >= p.H) return;
+      float* out = rec + ((size_t)m0 * p.H + h) * RF + 3 * P * GT_PITCH + d;
+#pragma unroll
+      for (int t = 0; t < GP_TOK; ++t) if (t < nt) out[(size_t)t * p.H * RF] = qv[t];
+      return;
+    }
+#pragma unroll
+    for (int t = 0; t < GP_TOK; ++t) av[t] = bias;
+    if (on) {
+#pragma unroll
+      for (int u = 0; u < GP_PIECES; ++u) {
+        if (u * N >= p.R) break;
+        const T* e = reinterpret_cast<const T*>(&row[u]);
+#pragma unroll
+        for (int c = 0; c < N; c += 4)
+#pragma unroll
+          for (int t = 0; t < GP_TOK; ++t) {
+            const float4 z = zs4[(t * p.R + u * N + c) >> 2];
+            av[t] = fmaf(to_f(e[c]), z.x, av[t]);
+            av[t] = fmaf(to_f(e[c + 1]), z.y, av[t]);
+            av[t] = fmaf(to_f(e[c + 2]), z.z, av[t]);
+            av[t] = fmaf(to_f(e[c + 3]), z.w, av[t]);
+          }
+      }
+#pragma unroll
+      for (int t = 0; t < GP_TOK; ++t) av[t] = expf(log_sigmoid(av[t]) * p.inv_tau);
+    }
+    float* out = rec + ((size_t)m0 * p.H + h) * RF + (d / GT_DP) * GT_PITCH + d % GT_DP;
+#pragma unroll
+    for (int t = 0; t < GP_TOK; ++t) {
+      if (t >= nt) break;
+      float* o = out + (size_t)t * p.H * RF;
+      o[0] = on ? qv[t] * p.q_scale : 0.0f; o[P * GT_PITCH] = on ? kv[t] * p.k_scale : 0.0f; o[2 * P * GT_PITCH] = on ? av[t] : 1.0f;
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < nt * p.R; i += GP_THREADS) zs[i] = p.y[(size_t)(m0 + i / p.R) * p.ldy + p.a_off + i % p.R];
   __syncthreads();
   const int P = p.P, RF = gla_record_floats(P, p.Dv), per_head = P * GT_DP, dvp = (p.Dv + 3) & ~3;
@@ -587,8 +660,11 @@ static int launch_scan(GlaParams p, const void* a2, const void* a2_bias, float* 
     const dim3 pgrid((B * S + GP_TOK - 1) / GP_TOK, (slots + GP_THREADS - 1) / GP_THREADS);
     const size_t zsm = (size_t)GP_TOK * R * sizeof(float);     // (the check above leaves at most 200 KB)
     if (zsm > 48 * 1024)
-      JL_DISPATCH_DTYPE(dtype, JL_CUDA(cudaFuncSetAttribute(gla_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm)));
-    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(gla_prep_kernel<T>, pgrid, dim3(GP_THREADS), zsm, st, p, (const T*)a2, (const T*)a2_bias, ws));
+      JL_DISPATCH_DTYPE(dtype, JL_CUDA(cudaFuncSetAttribute(gla_prep_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm)));
+    if (gla_plain(p, a2, dtype == DT_BF16 ? 2 : 4))
+      JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((gla_prep_kernel<T, true>), pgrid, dim3(GP_THREADS), zsm, st, p, (const T*)a2, (const T*)a2_bias, ws));
+    else
+      JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((gla_prep_kernel<T, false>), pgrid, dim3(GP_THREADS), zsm, st, p, (const T*)a2, (const T*)a2_bias, ws));
     JL_CUDA(cudaGetLastError());
     switch (p.P) {
       case 1: return launch_stream<1>(p, ws, st);

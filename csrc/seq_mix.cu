@@ -72,7 +72,8 @@ constexpr int CC_AHEAD = 8;        // inputs requested at once: a walk token by 
 // grid (channel blocks, rows, time chunks); a thread owns one channel and walks its chunk with the last taps-1 inputs in
 // registers.  Only the first chunk reads the state (chunks are at least taps-1 tokens long) and it is also the one that
 // replaces it, from the read-only inputs and the old values it holds in registers.
-// 2000 tokens x 4096 channels of 4 taps on one B200 (66 MB read and written): 51 us token by token with the taps in local memory, 30 us now.
+// 2000 tokens x 4096 channels of 4 taps on one B200 (66 MB read and written: 10 us): 51 us token by token with the taps in local memory, 30 us with
+// eight inputs asked for at once, 28 with the next eight in flight meanwhile, 24 with the activations of eight tokens side by side.  Bound: instruction issue.
 // in_bias (fp32 per channel) belongs to the projection: it is part of every input, but not of the zeros before the start.
 template <typename T, int MT>
 __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restrict__ y, int ldy, int col0, int C,
@@ -116,22 +117,35 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restric
       st[(size_t)i * C] = v;
     }
   }
+  const float* yp = y + (size_t)(b * S + s0) * ldy + col0 + c;
+  float* op = out + (size_t)(b * S + s0) * ldo + c;
+  float next[CC_AHEAD];
+#pragma unroll
+  for (int u = 0; u < CC_AHEAD; ++u) next[u] = s0 + u < s1 && s0 + u >= first ? yp[(size_t)u * ldy] + ib : 0.0f;
   for (int t0 = s0; t0 < s1; t0 += CC_AHEAD) {
     float xin[CC_AHEAD];
-#pragma unroll
-    for (int u = 0; u < CC_AHEAD; ++u) xin[u] = t0 + u < s1 ? input(t0 + u) : 0.0f;
+    yp += (size_t)CC_AHEAD * ldy;
 #pragma unroll
     for (int u = 0; u < CC_AHEAD; ++u) {
-      const int s = t0 + u;
-      if (s >= s1) break;
-      float acc = fmaf(wv[0], xin[u], bv);
+      xin[u] = next[u];
+      const int s = t0 + CC_AHEAD + u;
+      next[u] = s < s1 && s >= first ? yp[(size_t)u * ldy] + ib : 0.0f;      // in flight while the eight before it are worked on
+    }
+    float acc[CC_AHEAD];
 #pragma unroll
-      for (int j = 0; j < MT - 1; ++j) if (j < nh) acc = fmaf(wv[j + 1], hist[j], acc);
-      out[(size_t)(b * S + s) * ldo + c] = s >= first ? apply_act(acc, act, 0.0f, 0.0f) : 0.0f;
+    for (int u = 0; u < CC_AHEAD; ++u) {
+      acc[u] = fmaf(wv[0], xin[u], bv);
+#pragma unroll
+      for (int j = 0; j < MT - 1; ++j) if (j < nh) acc[u] = fmaf(wv[j + 1], hist[j], acc[u]);
 #pragma unroll
       for (int j = MT - 1; j > 0; --j) hist[j] = hist[j - 1];
       hist[0] = xin[u];
     }
+    apply_act_n(acc, act, 0.0f, 0.0f);
+#pragma unroll
+    for (int u = 0; u < CC_AHEAD; ++u)
+      if (t0 + u < s1) op[(size_t)u * ldo] = t0 + u >= first ? acc[u] : 0.0f;
+    op += (size_t)CC_AHEAD * ldo;
   }
 }
 

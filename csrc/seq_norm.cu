@@ -370,10 +370,13 @@ __global__ void __launch_bounds__(THREADS) rownorm_gate_kernel(const float* __re
 }
 
 // One warp per (token, head): out = o / sqrt(mean_v(o^2) + eps) * w[v] * act(gate)   (w == nullptr: no weight)
-constexpr int HG_VEC = 4;          // heads of up to 512 channels on the 16-byte path (2048 tokens x 16 heads of 128: 17.8 -> 14.8 us)
+// Heads of up to 128 * NV channels on the 16-byte path, NV at most HG_VEC: the instance decides how many rows an SM holds in flight (NV 1 in 32 registers, NV 4
+// in 56).  2048 tokens x 16 heads of 128 (42 MB: 6.4 us): 17.8 us without the wide accesses, 14.8 with NV 4 for all, 12.1 with NV 1, 11.3 with the four gates of
+// a lane side by side.
+constexpr int HG_VEC = 4;
 
-template <typename T>
-__global__ void headnorm_gate_kernel(const float* __restrict__ o, const T* __restrict__ w, const float* __restrict__ gate,
+template <typename T, int NV>
+__global__ void __launch_bounds__(128) headnorm_gate_kernel(const float* __restrict__ o, const T* __restrict__ w, const float* __restrict__ gate,
                                      int ldg, T* __restrict__ out, int M, int H, int V, float eps, int gate_act, int vec) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
   pdl_launch_dependents();
@@ -384,10 +387,10 @@ __global__ void headnorm_gate_kernel(const float* __restrict__ o, const T* __res
   float ss = 0.0f;
   if (vec) {                                              // read-outs and gate in registers, 16 bytes per access
     const float* grow = gate + (size_t)m * ldg + (size_t)hh * V;
-    float ov[HG_VEC][4], gv[HG_VEC][4];
-    Raw4<T> wr[HG_VEC];
+    float ov[NV][4], gv[NV][4];
+    Raw4<T> wr[NV];
 #pragma unroll
-    for (int u = 0; u < HG_VEC; ++u) {
+    for (int u = 0; u < NV; ++u) {
       const int i = 4 * lane + 128 * u;
       if (i < V) {
         load4(orow + i, ov[u]);
@@ -399,13 +402,14 @@ __global__ void headnorm_gate_kernel(const float* __restrict__ o, const T* __res
     }
     const float r = 1.0f / sqrtf(warp_sum(ss) / (float)V + eps);
 #pragma unroll
-    for (int u = 0; u < HG_VEC; ++u) {
+    for (int u = 0; u < NV; ++u) {
       const int i = 4 * lane + 128 * u;
       if (i < V) {
         float wv[4] = {1.0f, 1.0f, 1.0f, 1.0f};
         if (w) wr[u].get(wv);
+        apply_act_n(gv[u], gate_act, 0.f, 0.f);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) ov[u][e] = ov[u][e] * r * wv[e] * apply_act(gv[u][e], gate_act, 0.f, 0.f);
+        for (int e = 0; e < 4; ++e) ov[u][e] = ov[u][e] * r * wv[e] * gv[u][e];
         store4(out + ((size_t)m * H + hh) * V + i, ov[u]);
       }
     }
@@ -574,8 +578,11 @@ extern "C" JL_API int jl_headnorm_gate(const float* o, const void* w, const floa
   JL_CHECK_ARG(M >= 1 && H >= 1 && V >= 1, "jl_headnorm_gate: bad shape M=%d H=%d V=%d", M, H, V);
   const int warps = 4, blocks = (M * H + warps - 1) / warps;
   const int vec = V % 4 == 0 && V <= 128 * HG_VEC && ldg % 4 == 0 && (((uintptr_t)o | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out) & 15) == 0;
-  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(headnorm_gate_kernel<T>, dim3(blocks), dim3(warps * 32), 0, (cudaStream_t)stream, 
-                               o, (const T*)w, gate, ldg, (T*)out, M, H, V, eps, gate_act, vec));
+#define JL_HG(NV_) \
+  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((headnorm_gate_kernel<T, NV_>), dim3(blocks), dim3(warps * 32), 0, (cudaStream_t)stream, o, (const T*)w, \
+                                         gate, ldg, (T*)out, M, H, V, eps, gate_act, vec))
+  if (V <= 128) JL_HG(1); else if (V <= 256) JL_HG(2); else JL_HG(HG_VEC);
+#undef JL_HG
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }

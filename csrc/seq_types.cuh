@@ -43,6 +43,23 @@ __device__ __forceinline__ float apply_act(float z, int act, float p0, float p1)
   }
 }
 
+// N values through one look at the activation: the common ones side by side (their exponentials and quotients overlap), where a switch per value
+// runs them one after the other
+template <int N>
+__device__ __forceinline__ void apply_act_n(float (&v)[N], int act, float p0, float p1) {
+  if (act == ACT_NONE) return;
+  if (act == ACT_SILU) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = apply_act(v[i], ACT_SILU, p0, p1);
+  } else if (act == ACT_SIGMOID) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = apply_act(v[i], ACT_SIGMOID, p0, p1);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = apply_act(v[i], act, p0, p1);
+  }
+}
+
 // Channel d of a head after the rotary embedding of its first `rot` channels (even): the pair (u, v) turns into
 // (u cos - v sin, v cos + u sin).  layout 0 pairs channel 2i with 2i+1, layout 1 pairs channel i with i + rot/2; ct / st are
 // the cos / sin of the token's position for the rot/2 pairs (any factor on them is already in the table).

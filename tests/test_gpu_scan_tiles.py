@@ -76,3 +76,28 @@ def test_state_at_any_element(S, offset):
     want, got = scan(first), scan(moved)
     assert torch.equal(got, want) and torch.equal(moved, first)
     assert bool((room[:offset] == 7.0).all()) and bool((room[offset + first.numel():] == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype,ranks", [(torch.float32, (4, 12, 16, 20)), (torch.bfloat16, (8, 16, 24, 32, 40))])
+@pytest.mark.parametrize("B,S,H,D,Dv", [(1, 9, 1, 10, 7), (2, 17, 3, 16, 64), (1, 130, 2, 33, 129), (3, 43, 5, 64, 30)])
+def test_decay_projections_in_whole_pieces_match_the_general_preparation(dtype, ranks, B, S, H, D, Dv):
+    """Ranks whose rows of A2 are whole 16-byte pieces, up to the instance's four and beyond; the same matrix off the boundary takes the
+    general one.  The additions are the same ones in the same order: equal bit for bit."""
+    for R in ranks:
+        g = torch.Generator().manual_seed(S * D + R)
+        y = torch.randn(B * S, 2 * H * D + H * Dv + R, generator=g).cuda()
+        a2 = (torch.randn(H * D, R, generator=g) * 0.5).to(dtype).cuda()
+        bias = torch.randn(H * D, generator=g).to(dtype).cuda()
+        room = torch.zeros(a2.numel() + 1, dtype=dtype, device="cuda")
+        off = room[1:].view(H * D, R)
+        off.copy_(a2)
+        pads = torch.tensor([0] + [3 + b for b in range(1, B)], dtype=torch.int32, device="cuda")
+        first = torch.randn(B, H, D, Dv, generator=g).cuda()
+        got, want = [], []
+        for matrix, res in ((a2, got), (off, want)):
+            state = first.clone()
+            out = SK.gla_scan(y, 0, H * D, 2 * H * D, 2 * H * D + H * Dv, matrix, bias, state, torch.zeros(1, dtype=torch.int32, device="cuda"), pads,
+                              B, S, H, D, Dv, 0.25, 4.0)
+            res += [out, state]
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), R
+        assert bool(torch.isfinite(got[0]).all())

@@ -212,7 +212,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, norm_w: Optional[torch.Tensor] =
     elif path == "gemm":
         if norm_w is not None:
             x = rmsnorm(x.view(m, k), norm_w, eps)
-        if m <= 128:
+        if m <= 256 or n <= 64:                            # the sizes whose kernel may split K
             ensure_gemm_workspace(x.device)
         _lib.check(L.jl_gemm(x.data_ptr(), w.data_ptr(), _p(residual), out.data_ptr(), m, n, k, mode,
                              int(out_f32), sms, _stream()), "jl_gemm")

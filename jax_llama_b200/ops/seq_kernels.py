@@ -133,7 +133,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
     use_tc = tensor_cores_enabled() if tensor_cores is None else tensor_cores
     if (use_tc and x.dtype == torch.bfloat16 and M > 8 and K % 8 == 0 and N % 8 == 0 and x.is_contiguous()
             and w.is_contiguous() and out.is_contiguous() and out.shape[1] == N):
-        if M <= 128:
+        if M <= 256 or N <= 64:                            # the sizes whose kernel may split K
             ensure_gemm_workspace(x.device)
         f32 = out.dtype == torch.float32
         _lib.check(L.jl_gemm(x.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, 0, int(f32), num_sms(x.device),

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from jax_llama_b200.ops import kernels as K
+from jax_llama_b200.ops import seq_kernels as SK
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -76,3 +77,13 @@ def test_token_major_kernel_refuses_rows_off_the_16_byte_boundary():
 @pytest.mark.parametrize("mode", ["plain", "residual", "swiglu", "f32"])
 def test_output_at_any_element(M, N, Kd, mode, shift):
     _check(M, N, Kd, mode, shift)
+
+
+@pytest.mark.parametrize("M,N", [(16, 4096), (200, 4096), (2048, 32)])
+def test_split_is_allowed_by_the_first_call_that_can_use_it(monkeypatch, M, N):
+    """Whatever a process ran before: the permission is asked for at every size whose kernel may split K."""
+    x, w = torch.zeros(M, 1024, dtype=torch.bfloat16, device=DEV), torch.zeros(N, 1024, dtype=torch.bfloat16, device=DEV)
+    for call in (lambda: K.linear(x, w, out_f32=True), lambda: SK.linear(x, w)):
+        monkeypatch.setattr(K, "_GEMM_WS", {})
+        call()
+        assert K._GEMM_WS

@@ -125,6 +125,8 @@ __global__ void __launch_bounds__(RT_WARPS * 32) moe_route_kernel(RouteParams p)
 }
 
 // One CTA orders the n = M * top pairs by expert.  counts / offsets live in shared memory (E + 1 ints each).
+constexpr int MS_KEEP = 16;
+
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ idx, int n, int top, int E, int tile, int cap,
                                                         int* __restrict__ pos, int* __restrict__ row_src,
                                                         int* __restrict__ tile_group, int* __restrict__ tiles_used) {
@@ -133,22 +135,59 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
   extern __shared__ int si[];
   int* count = si;                 // [E]
   int* start = si + E;             // [E + 1], in rows
+  // One CTA, so what counts is its chain of latencies: up to MS_KEEP pairs a thread stay in registers with their ranks (all their experts
+  // asked for at once), a warp adds up the counts.  2048 tokens x 4 of 32 experts: 11.4 -> 8.7 us.
+  const bool keep = n <= MS_KEEP * (int)blockDim.x;
+  int ex[MS_KEEP], rank[MS_KEEP];
+  if (keep) {
+#pragma unroll
+    for (int u = 0; u < MS_KEEP; ++u) {
+      const int i = threadIdx.x + u * blockDim.x;
+      ex[u] = i < n ? idx[i] : -1;
+    }
+  }
   for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
   for (int i = threadIdx.x; i < cap; i += blockDim.x) row_src[i] = -1;
   for (int i = threadIdx.x; i < cap / tile; i += blockDim.x) tile_group[i] = -1;
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x)               // rank within its expert (expert < 0: a pair that runs no expert)
-    pos[i] = idx[i] >= 0 ? atomicAdd(&count[idx[i]], 1) : -1;
+  if (keep) {                                                      // rank within its expert (expert < 0: a pair that runs no expert)
+#pragma unroll
+    for (int u = 0; u < MS_KEEP; ++u) rank[u] = ex[u] >= 0 ? atomicAdd(&count[ex[u]], 1) : -1;
+  } else {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) pos[i] = idx[i] >= 0 ? atomicAdd(&count[idx[i]], 1) : -1;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0;
-    for (int e = 0; e < E; ++e) { start[e] = at; at += (count[e] + tile - 1) / tile * tile; }
-    start[E] = at;
-    if (tiles_used) *tiles_used = at / tile;
+  if (threadIdx.x < 32) {
+    const int per = (E + 31) / 32, e0 = min(E, (int)threadIdx.x * per), e1 = min(E, e0 + per);
+    int sum = 0;
+    for (int e = e0; e < e1; ++e) sum += (count[e] + tile - 1) / tile * tile;
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((int)threadIdx.x >= o) incl += t;
+    }
+    int at = incl - sum;
+    for (int e = e0; e < e1; ++e) { start[e] = at; at += (count[e] + tile - 1) / tile * tile; }
+    if (threadIdx.x == 31) {
+      start[E] = incl;
+      if (tiles_used) *tiles_used = incl / tile;
+    }
   }
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x)
     for (int t = start[e] / tile; t < start[e + 1] / tile; ++t) tile_group[t] = e;
+  if (keep) {
+#pragma unroll
+    for (int u = 0; u < MS_KEEP; ++u) {
+      const int i = threadIdx.x + u * blockDim.x;
+      if (i >= n) break;
+      const int at = ex[u] >= 0 ? start[ex[u]] + rank[u] : -1;     // (-1: the combine pass skips the pair)
+      pos[i] = at;
+      if (at >= 0) row_src[at] = i / top;
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     if (idx[i] < 0) continue;                                      // pos stays -1: the combine pass skips the pair
     const int at = start[idx[i]] + pos[i];
@@ -218,21 +257,37 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
 }
 
 // xs[p, :] = x[row_src[p], :] (row_src[p] < 0: zeros): the rows of a step in sorted order, for kernels that cannot gather.
+// A CTA takes GR_ROWS of them, a thread a 16-byte column of each: the rows' loads are in flight together (a CTA per row: 14.2 us for 12256 rows of 2048
+// bfloat16, 50 MB written; now 9.2).
+constexpr int GR_ROWS = 4;
+
 template <typename T>
-__global__ void __launch_bounds__(128) moe_gather_kernel(const T* __restrict__ x, int ldx, const int* __restrict__ row_src,
-                                                         T* __restrict__ xs, int W) {
+__global__ void __launch_bounds__(256) moe_gather_kernel(const T* __restrict__ x, int ldx, const int* __restrict__ row_src,
+                                                         T* __restrict__ xs, int rows, int W) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
   pdl_launch_dependents();
-  const size_t p = blockIdx.x;
-  const int src = row_src[p];
+  const size_t p = (size_t)blockIdx.x * GR_ROWS;
+  int src[GR_ROWS];
+#pragma unroll
+  for (int r = 0; r < GR_ROWS; ++r) src[r] = p + r < (size_t)rows ? row_src[p + r] : -1;
   constexpr int VN = 16 / sizeof(T);
   if (W % VN == 0 && ldx % VN == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)xs & 15) == 0) {
-    const uint4* in = src >= 0 ? reinterpret_cast<const uint4*>(x + (size_t)src * ldx) : nullptr;
-    uint4* out = reinterpret_cast<uint4*>(xs + p * W);
-    for (int i = threadIdx.x; i < W / VN; i += blockDim.x) out[i] = in ? in[i] : make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < W / VN; i += blockDim.x) {
+      uint4 v[GR_ROWS];
+#pragma unroll
+      for (int r = 0; r < GR_ROWS; ++r)
+        v[r] = src[r] >= 0 ? reinterpret_cast<const uint4*>(x + (size_t)src[r] * ldx)[i] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int r = 0; r < GR_ROWS; ++r)
+        if (p + r < (size_t)rows) reinterpret_cast<uint4*>(xs + (p + r) * W)[i] = v[r];
+    }
     return;
   }
-  for (int i = threadIdx.x; i < W; i += blockDim.x) xs[p * W + i] = src >= 0 ? x[(size_t)src * ldx + i] : from_f<T>(0.0f);
+#pragma unroll
+  for (int r = 0; r < GR_ROWS; ++r) {
+    if (p + r >= (size_t)rows) break;
+    for (int i = threadIdx.x; i < W; i += blockDim.x) xs[(p + r) * W + i] = src[r] >= 0 ? x[(size_t)src[r] * ldx + i] : from_f<T>(0.0f);
+  }
 }
 
 }  // namespace jl
@@ -315,7 +370,8 @@ extern "C" JL_API int jl_moe_combine_ex(const float* z, int ldz, const int* pos,
 
 extern "C" JL_API int jl_moe_gather(const void* x, int ldx, const int* row_src, void* xs, int rows, int W, int dtype, void* stream) {
   JL_CHECK_ARG(rows >= 1 && W >= 1 && ldx >= W, "jl_moe_gather: bad shape");
-  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(moe_gather_kernel<T>, dim3(rows), dim3(128), 0, stream, (const T*)x, ldx, row_src, (T*)xs, W));
+  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(moe_gather_kernel<T>, dim3((rows + GR_ROWS - 1) / GR_ROWS), dim3(256), 0, stream, (const T*)x, ldx,
+                                         row_src, (T*)xs, rows, W));
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }

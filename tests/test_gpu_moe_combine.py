@@ -64,3 +64,31 @@ def test_buffers_that_nobody_cleared_reach_no_result(M, experts, top, dtype, mon
     monkeypatch.setattr(torch, "empty", poisoned)
     got = layer.run(h)
     assert bool(torch.isfinite(want).all()) and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M,top,E,tile", [(1, 1, 1, 16), (9, 4, 31, 16), (33, 3, 33, 64), (2048, 4, 32, 128), (4096, 4, 300, 128), (4097, 4, 5, 128)])
+@pytest.mark.parametrize("W", [8, 12, 2056])
+def test_sorted_pairs_and_their_rows(M, top, E, tile, W):
+    """Pairs a thread keeps in registers (up to 16384) and more, experts that do not divide among a warp's lanes, pairs without an expert; every
+    pair's place lies in its expert's segment, the places are distinct, and the gathered rows are copies (zeros where no pair is)."""
+    g = torch.Generator().manual_seed(M + E)
+    idx = torch.randint(-1, E, (M, top), generator=g, dtype=torch.int32)
+    pos, row_src, tile_group, used = (t.cpu() for t in SK.moe_sort(idx.cuda(), E, tile))
+    flat = idx.flatten()
+    counts = torch.bincount(flat[flat >= 0].long(), minlength=E)
+    size = (counts + tile - 1) // tile * tile
+    start = torch.cumsum(size, 0) - size
+    assert int(used) == int(size.sum()) // tile
+    assert tile_group[:int(used)].tolist() == torch.repeat_interleave(torch.arange(E), size // tile).tolist() and bool((tile_group[int(used):] == -1).all())
+    real = flat >= 0
+    assert bool((pos[~real] == -1).all())
+    place, expert = pos[real].long(), flat[real].long()
+    assert bool((place >= start[expert]).all()) and bool((place < start[expert] + counts[expert]).all()) and place.unique().numel() == place.numel()
+    want = torch.full_like(row_src, -1)
+    want[place] = (torch.arange(M * top, dtype=torch.int32) // top)[real]
+    assert torch.equal(row_src, want)
+    for dtype in (torch.bfloat16, torch.float32):
+        x = torch.randn(M, W, generator=g).to(dtype)
+        rows = torch.cat([x, torch.zeros(1, W, dtype=dtype)])[want.long()]
+        for n in (len(want), max(1, len(want) - 1), max(1, len(want) - 3)):
+            assert torch.equal(SK.moe_gather(x.cuda(), want[:n].cuda()).cpu(), rows[:n])

@@ -11,7 +11,7 @@
 // Exact float32 activations (this file is compiled without fast math).
 // Bound: the operands' way from L2 (48 KB per 512 cycles of products) and, for few k, the activations of eight warps.  One B200, gate | up product (fp32) and
 // activation pass -> one kernel (tokens x F x K): 2048 x 5464 x 2048 94 -> 68 us (1340 TFLOP/s), 2048 x 1360 x 2048 34 -> 26.5, 512 x 2736 x 2048 20 -> 16, 129 x 1024 x 1024
-// 13.7 -> 10.5, the same bits; 2048 tokens x top 4 of 32 experts of 2048 x 1024 with a shared one: both GEMMs and activations 265 -> 190 us, the layer 343 -> 262.
+// 13.7 -> 10.5, the same bits; 2048 tokens x top 4 of 32 experts of 2048 x 1024 with a shared one: both GEMMs and activations 265 -> 190 us, the layer 337 -> 275 between events.
 #include "jllama_b200.h"
 #include "seq_types.cuh"
 #include "tcgen05.cuh"

@@ -19,7 +19,7 @@
 //     more than SF_CAND elements (plateaus, coarse logits) is first narrowed by histograms over its own (key, ~index) range.
 //     What bounds it is the chain of cluster barriers and short passes, not the 0.5 MB of a row: 4 rows of 128256, top-p 0.95, on
 //     one B200: 632 us with one CTA per row and three radix passes per question (the top bits of normal logits fall into a few
-//     dozen bins, so its 64-bit shared-memory atomics serialised), 30 us with one gather per question, 25 us with one gather for all;
+//     dozen bins, so its 64-bit shared-memory atomics serialised), 29 us with one gather per question, 23 us with one gather for all;
 //   * rows that hold a NaN or whose maximum is not finite take the radix select that the first form of this kernel ran for every
 //     row (sf_select): their masses are not sums of probabilities, and what they return stays what it was.
 //   * tensor parallelism: the decode kernel stores every rank's logits shard into every rank's [B, V] buffer with

@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
   const float g = shared ? (gate ? sigmoid_f(gate[m * ldg]) : 1.0f) : 0.0f;
   // Bounded by the bytes of z: at most eight experts' rows are known before the columns, and a thread asks for 16 bytes of each
   // before it adds the first (same order of sums).  One float at a time behind its row's index took 29 us for 2048 tokens of
-  // 2048 over 4 experts (100 MB, 3.5 TB/s), now 27: the product that wrote z leaves tens of MB in L2 to be written back meanwhile.
+  // 2048 over 4 experts (100 MB, 3.5 TB/s), then 27 (21 with 128 threads a row): the product that wrote z leaves tens of MB in L2 to be written back meanwhile.
   if (vec) {
     size_t r[8];
     float wk[8];
@@ -300,6 +300,11 @@ static int combine_vec(const float* z, int ldz, int top, const float* shared, in
          ((uintptr_t)z | (uintptr_t)shared | (uintptr_t)out | (uintptr_t)x) % 16 == 0;
 }
 
+// Threads of a row: 128 where the rows fill every SM four times over, because a thread's rows then wait behind one look at the indices (2048
+// tokens x 4 experts, 2048 columns: 256 threads 26 us, 128 21, 512 35; 600 x 2 x 4096: 20.5 and 16.4); with fewer rows the columns' parallelism
+// counts (200 x 4 x 2048: 256 threads 10.2, 128 11.2; 64 x 4 x 4096 10.2 and 14.3).
+static int combine_threads(int M, int vec) { return vec && M >= 4 * 148 ? 128 : 256; }
+
 static int moe_route_launch(const float* z, int ldz, int M, int E, int top, int groups, int keep, int group_top, int score,
                             int normalise, float scale, const float* bias, const float* choice_bias, int n_real, float* ident_w,
                             int* idx, float* wt, void* stream) {
@@ -348,9 +353,9 @@ extern "C" JL_API int jl_moe_sort(const int* idx, int M, int top, int E, int til
 extern "C" JL_API int jl_moe_combine(const float* z, int ldz, const int* pos, const float* wt, int top, const float* shared, int lds,
                                      const float* gate, int ldg, float* out, int M, int W, void* stream) {
   JL_CHECK_ARG(M >= 1 && W >= 1 && top >= 1 && ldz >= W, "jl_moe_combine: bad shape");
-  JL_LAUNCH_PDL(moe_combine_kernel<float>, dim3(M), dim3(256), 0, stream, z, ldz, pos, wt, top, shared, lds, gate, ldg, out, W,
-                (const int*)nullptr, (const float*)nullptr, (const float*)nullptr, 0,
-                combine_vec(z, ldz, top, shared, lds, out, W, nullptr, 0));
+  const int vec = combine_vec(z, ldz, top, shared, lds, out, W, nullptr, 0);
+  JL_LAUNCH_PDL(moe_combine_kernel<float>, dim3(M), dim3(combine_threads(M, vec)), 0, stream, z, ldz, pos, wt, top, shared, lds, gate, ldg, out, W,
+                (const int*)nullptr, (const float*)nullptr, (const float*)nullptr, 0, vec);
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }
@@ -362,8 +367,9 @@ extern "C" JL_API int jl_moe_combine_ex(const float* z, int ldz, const int* pos,
                                         const void* x, int ldx, int dtype, void* stream) {
   JL_CHECK_ARG(M >= 1 && W >= 1 && top >= 1 && ldz >= W, "jl_moe_combine: bad shape");
   JL_CHECK_ARG(ident_w == nullptr || (x != nullptr && ldx >= W), "jl_moe_combine: identity weights without the input rows");
-  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(moe_combine_kernel<T>, dim3(M), dim3(256), 0, stream, z, ldz, pos, wt, top, shared, lds, gate,
-                                         ldg, out, W, idx, ident_w, (const T*)x, ldx, combine_vec(z, ldz, top, shared, lds, out, W, x, ldx)));
+  const int vec = combine_vec(z, ldz, top, shared, lds, out, W, x, ldx);
+  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(moe_combine_kernel<T>, dim3(M), dim3(combine_threads(M, vec)), 0, stream, z, ldz, pos, wt, top, shared, lds, gate,
+                                         ldg, out, W, idx, ident_w, (const T*)x, ldx, vec));
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }

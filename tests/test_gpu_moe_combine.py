@@ -92,3 +92,20 @@ def test_sorted_pairs_and_their_rows(M, top, E, tile, W):
         rows = torch.cat([x, torch.zeros(1, W, dtype=dtype)])[want.long()]
         for n in (len(want), max(1, len(want) - 1), max(1, len(want) - 3)):
             assert torch.equal(SK.moe_gather(x.cuda(), want[:n].cuda()).cpu(), rows[:n])
+
+
+@pytest.mark.parametrize("M", [591, 592, 593])
+@pytest.mark.parametrize("W,top", [(4, 1), (508, 3), (512, 8), (2052, 4)])
+def test_threads_of_a_row_change_no_bit(M, W, top):
+    """Rows on either side of the count from which a row has 128 threads: a column's sum is one thread's, in the order of the choices."""
+    g = torch.Generator().manual_seed(M + W)
+    z, wt, sh = torch.randn(M * top, W, generator=g), torch.rand(M, top, generator=g), torch.randn(M, W, generator=g)
+    pos = torch.randperm(M * top, generator=g).int()
+    d = [t.to(DEV) for t in (z, pos, wt, sh)]
+    got = SK.moe_combine(*d, None, W)
+    few = torch.cat([SK.moe_combine(d[0], d[1][i * top:(i + 100) * top], d[2][i:i + 100], d[3][i:i + 100], None, W) for i in range(0, M, 100)])
+    want = (wt.double()[:, :, None] * z.double()[pos.long()].view(M, top, W)).sum(1) + sh.double()
+    assert torch.equal(got, few)
+    # top + 1 products and additions in fp32, each rounded once
+    bound = 2.0 ** -23 * (top + 1) * ((wt[:, :, None] * z[pos.long()].view(M, top, W).abs()).sum(1) + sh.abs()).double()
+    assert bool(((got.double().cpu() - want).abs() <= bound).all())

@@ -9,7 +9,8 @@
 //     persistent CTA per SM took 224 tiles in two rounds, the second half empty.  More tiles: the same CTAs walk the list;
 //   * few tiles: the CTAs of a cluster of `ksplit` share one and take a part of K each; the finished ring takes the fp32 partial, partials
 //     meet in distributed shared memory, each CTA sums its share of the tokens in rank order — deterministic, no scratch in global memory;
-//   * the weights do not depend on the previous kernel: the ring is filled before the wait for it.
+//   * the weights do not depend on the previous kernel: the ring is filled before the wait for it.  (Not in the turned form, whose A operand is the
+//     tokens: the kernels ahead let this one start before they have written a row.)
 // Epilogues: plain bf16 / fp32, residual add, SwiGLU over interleaved (w1, w3) output features.
 // One B200, us in a chain of cold weights, one persistent CTA per SM -> this (tokens x features x K): 16 x 28672 x 4096 45.8 -> 38.3 (6.1 TB/s), 16 x
 // 24000 x 2048 25.0 -> 17.8, 16 x 11008 x 4096 22.5 -> 18.4, 100 x 28672 x 4096 55 -> 44.5, 100 x 4096 x 4096 17.0 -> 14.1, 100 x 4096 x 14336 34.4 -> 27.8, 128 x 14336 x
@@ -32,7 +33,7 @@ struct SwapParams {
   const __nv_bfloat16* residual;
   int N, M, K, nb;          // weight rows, tokens, reduction length, tokens padded to a multiple of 16
   int ldo, stages, ksplit, wide;   // wide: out and residual take 4-feature accesses
-  int turned;                      // the result's rows are the A operand's (fp32): out[feature * ldo + token]
+  int turned;                      // the A operand is the tokens and the result's rows are its rows (fp32): out[feature * ldo + token]; nothing is asked for early
   uint32_t cols, idesc;
   unsigned long long* trace;       // optional [trace_rows][16] %globaltimer stamps (jl_gemm_set_trace), NULL = off
   int trace_rows;
@@ -148,10 +149,11 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     // ===================================================== TMA producer
     if (lane == 0) {
       // weights stream from HBM while the previous kernel runs its tail; the tokens follow after the wait for it
-      int pre = kb1 - kb0 < stages ? kb1 - kb0 : stages;
+      int pre = p.turned ? 0 : kb1 - kb0 < stages ? kb1 - kb0 : stages;
+      const uint64_t hint_a = p.turned ? tc::EVICT_NORMAL : tc::EVICT_FIRST;      // (tokens are read again by the kernels behind)
       for (int i = 0; i < pre; ++i) {
         tc::mbar_expect_tx(full_bar(i), stage_bytes);
-        tc::tma_load_2d(smem_base + i * stage_bytes, &tmap_w, full_bar(i), (kb0 + i) * GS_BK, tile0 * GS_BM, tc::EVICT_FIRST);
+        tc::tma_load_2d(smem_base + i * stage_bytes, &tmap_w, full_bar(i), (kb0 + i) * GS_BK, tile0 * GS_BM, hint_a);
       }
       pdl_wait();
       swap_stamp(p, 2);
@@ -164,7 +166,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           } else {
             tc::mbar_wait(empty_bar(stage), phase ^ 1);
             tc::mbar_expect_tx(full_bar(stage), stage_bytes);
-            tc::tma_load_2d(sa, &tmap_w, full_bar(stage), kb * GS_BK, tile * GS_BM, tc::EVICT_FIRST);
+            tc::tma_load_2d(sa, &tmap_w, full_bar(stage), kb * GS_BK, tile * GS_BM, hint_a);
           }
           tc::tma_load_2d(sa + GS_A_BYTES, &tmap_x, full_bar(stage), kb * GS_BK, 0, tc::EVICT_LAST);
           if (++stage == stages) { stage = 0; phase ^= 1; }
@@ -448,8 +450,9 @@ bool gemm_swap_takes(int M, int N, int K, int num_sms) {
 }
 
 // Few output features over many tokens (a router): the tokens take the MMA's rows, 128 to a tile, and K is split over clusters, where the token-major kernel has a
-// tile, i.e. a CTA, per 128 tokens (32 features, K 2048: 512 tokens 12.3 -> 6.0 us, 2048 12.2 -> 6.6,
-// 4096 12.3 -> 8.0; 64 features, K 4096, 2048 tokens 21.5 -> 9.8; 8192 x 64 x 2048 13.5 and 14.6).
+// tile, i.e. a CTA, per 128 tokens.  Nothing is asked for ahead of the wait.  Token-major -> this, us a launch in a chain of cold tokens (32 features, K 2048): 512 tokens
+// 12.1 -> 6.0, 2048 12.3 -> 7.2, 4096 12.4 -> 8.8; 64 features, K 4096, 2048 tokens 21.6 ->
+// 10.4; what it adds behind the norm that writes its tokens: 2048 tokens 11.7 -> 6.6 us.
 bool gemm_turned_takes(int M, int N, int K, int num_sms) {
   return N <= 64 && M > 128 && (M + GS_BM - 1) / GS_BM * 4 <= num_sms && K >= 8 * GS_BK && splitk_allowed();
 }

@@ -87,3 +87,58 @@ def test_split_is_allowed_by_the_first_call_that_can_use_it(monkeypatch, M, N):
         monkeypatch.setattr(K, "_GEMM_WS", {})
         call()
         assert K._GEMM_WS
+
+
+def _behind_their_writer(M, N, Kd, between, captured, rounds):
+    """A norm writes the tokens, which held NaN, directly ahead of the product that reads them (with `between`, two kernels ahead, behind a
+    product that lets the next kernel start before its own wait)."""
+    K.ensure_gemm_workspace(torch.device(DEV))
+    g = torch.Generator(device=DEV).manual_seed(M + N + Kd)
+    xs = torch.randn(8, M, Kd, generator=g, device=DEV)
+    gain = torch.ones(Kd, dtype=torch.bfloat16, device=DEV)
+    w = (torch.randn(N, Kd, generator=g, device=DEV) * Kd ** -0.5).bfloat16()
+    w2 = (torch.randn(512, Kd, generator=g, device=DEV) * Kd ** -0.5).bfloat16()
+    h, x, out = torch.empty(M, Kd, dtype=torch.bfloat16, device=DEV), xs[0].clone(), torch.empty(M, N, device=DEV)
+    out2 = torch.empty(M, 512, device=DEV)
+    want = []
+    for i in range(8):
+        SK.norm_f32(xs[i], gain, 1e-5, 0.0, out=h)
+        torch.cuda.synchronize()
+        SK.linear(h, w, out=out)
+        torch.cuda.synchronize()
+        want.append(out.clone())
+
+    def chain(src):
+        h.fill_(float("nan"))
+        SK.norm_f32(src, gain, 1e-5, 0.0, out=h)
+        if between:
+            SK.linear(h, w2, out=out2)
+        SK.linear(h, w, out=out)
+
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            chain(x)
+    got = torch.empty(rounds, M, N, device=DEV)
+    for r in range(rounds):
+        if captured:
+            x.copy_(xs[r % 8])
+            graph.replay()
+        else:
+            chain(xs[r % 8])
+        got[r].copy_(out)
+    bad = [r for r in range(rounds) if not torch.equal(got[r], want[r % 8])]
+    assert not bad, (len(bad), bad[:8])
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("M,N,Kd,between", [(129, 32, 2048, False), (200, 64, 512, True), (1000, 32, 2048, False), (2048, 8, 2048, False),
+                                            (2048, 32, 2048, False), (2048, 64, 2048, False), (4096, 32, 1024, False), (4736, 32, 2048, False)])
+def test_few_features_wait_for_the_kernel_that_writes_the_tokens(M, N, Kd, between, captured):
+    _behind_their_writer(M, N, Kd, between, captured, 200)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("M,N,Kd,between", [(100, 2048, 2048, False), (128, 512, 2048, True), (200, 2048, 2048, False), (256, 4096, 1024, True)])
+def test_few_tokens_wait_for_the_kernel_that_writes_them(M, N, Kd, between, captured):
+    _behind_their_writer(M, N, Kd, between, captured, 100)

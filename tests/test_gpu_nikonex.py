@@ -323,6 +323,23 @@ def test_prompt_in_portions(dtype, cuts):
     assert err(torch.cat(got), want) < TOL[dtype]
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_experts_of_wide_layers_over_long_prompts(dtype):
+    """Width, expert and token counts of which the router's product over a prompt takes its few features as columns, right behind the norm that
+    writes the tokens; the same prompt a few times over, the same logits every time."""
+    layers = [ret(heads=4, dim=32, vdim=32, decay=(0.5, 0.9, 0.99, 0.995), rot=32, mlp=moe(experts=16, top=4, ff=64, groups=None, shared=72)) for _ in range(3)]
+    cfg = config(layers, width=512, dtype=dtype)
+    eng, cpu = build(cfg, dtype, seed=23)
+    toks = tokens(150, cfg.vocab_size, 37)
+    want = oracle_logits(cfg, cpu, toks)
+    first = None
+    for _ in range(5):
+        got = eng.forward(torch.tensor([toks], device="cuda"), cache=eng.new_cache(1, 152)).logits[0].clone()
+        assert err(got, want) < TOL[dtype]
+        first = got if first is None else first
+        assert torch.equal(got, first)
+
+
 def run_unequal_batch(cfg, dtype, lens, extra, seed):
     """Left-padded batch of prompts of the given lengths, then `extra` tokens decoded together; every row is compared
     with the oracle run of that request alone."""

@@ -257,7 +257,9 @@ static int launch_gemm(const void* a, const void* b, const GemmParams& p0, int R
                        cudaStream_t stream) {
   GemmParams p = p0;
   p.trace = g_gemm_trace;
-  JL_CHECK_ARG((((uintptr_t)p.out | (uintptr_t)p.residual) & 15) == 0, "jl_gemm: result and residual of the token-major kernel start on a 16-byte boundary");
+  // whole pieces of 32 columns are stored and read 16 bytes at a time; narrower results go element by element and start anywhere
+  JL_CHECK_ARG(Rb < 32 || (((uintptr_t)p.out | (uintptr_t)p.residual) & 15) == 0,
+               "jl_gemm: result and residual of the token-major kernel start on a 16-byte boundary (N=%d)", Rb);
   CUtensorMap ta, tb;
   int rc = make_tmap_2d_bf16(&ta, a, Ra, K, K, GEMM_BM);
   if (rc) return rc;

@@ -65,11 +65,23 @@ def test_few_features_over_many_tokens(M, N, Kd):
         _check(M, N, Kd, "f32", shift=1)
 
 
-def test_token_major_kernel_refuses_rows_off_the_16_byte_boundary():
-    x, w = torch.zeros(300, 64, dtype=torch.bfloat16, device=DEV), torch.zeros(24, 64, dtype=torch.bfloat16, device=DEV)
-    room = torch.zeros(300 * 24 + 8, device=DEV)
+@pytest.mark.parametrize("N,mode", [(32, "f32"), (40, "plain"), (64, "residual"), (264, "swiglu")])
+def test_token_major_kernel_refuses_rows_off_the_16_byte_boundary(N, mode):
+    """Results with a whole piece of 32 columns; narrower ones are stored element by element (below)."""
+    x, w = torch.zeros(300, 64, dtype=torch.bfloat16, device=DEV), torch.zeros(N, 64, dtype=torch.bfloat16, device=DEV)
+    cols, f32 = N // 2 if mode == "swiglu" else N, mode == "f32"
+    room = torch.zeros(300 * cols + 8, dtype=torch.float32 if f32 else torch.bfloat16, device=DEV)
+    out = room[1:1 + 300 * cols].view(300, cols)
     with pytest.raises(RuntimeError, match="16-byte"):
-        K.linear(x, w, out_f32=True, out=room[1:1 + 300 * 24].view(300, 24), force="gemm")
+        K.linear(x, w, out_f32=f32, out=out, force="gemm", residual=torch.zeros_like(out) if mode == "residual" else None,
+                 mode={"residual": K.RESIDUAL, "swiglu": K.SWIGLU}.get(mode, K.PLAIN))
+
+
+@pytest.mark.parametrize("M", [129, 300, 4800])
+@pytest.mark.parametrize("N,mode", [(8, "f32"), (24, "f32"), (16, "plain"), (24, "residual"), (16, "swiglu")])
+def test_token_major_kernel_takes_narrow_results_at_any_element(M, N, mode):
+    for shift in (0, 1):
+        _check(M, N, 64, mode, shift)
 
 
 @pytest.mark.parametrize("shift", [1, 2, 3])

@@ -24,7 +24,7 @@ constexpr uint32_t GG_EPI = 8 * 4096;                          // eight warps x 
 constexpr size_t GG_SMEM = GG_STAGES * GG_STAGE + GG_EPI + 8 * (2 * GG_STAGES + 4) + 16 + 1024;
 
 enum { GG_F32 = 0, GG_BF16 = 1, GG_GLU = 2 };
-constexpr int GG_CLAMPED = -1, GG_ANY = -2;                      // activations of GG_GLU beside ACT_*: the clamped form, one named at run time
+constexpr int GG_CLAMPED = -1, GG_ANY = -2;                      // activations beside ACT_*: the clamped form (GG_GLU), one named at run time
 
 struct GroupGemm {
   int K, N, a_blocks, b_blocks;      // N: columns of the result
@@ -36,8 +36,10 @@ struct GroupGemm {
 };
 
 template <int ACT>
+__device__ __forceinline__ float gg_act(float z, const GroupGemm& p) { return apply_act(z, ACT == GG_ANY ? p.act : ACT, 0.0f, 0.0f); }
+template <int ACT>
 __device__ __forceinline__ float gg_glu(float g, float u, const GroupGemm& p) {
-  if constexpr (ACT != GG_CLAMPED) return apply_act(g, ACT == GG_ANY ? p.act : ACT, 0.0f, 0.0f) * u;
+  if constexpr (ACT != GG_CLAMPED) return gg_act<ACT>(g, p) * u;
   g = fminf(g, p.limit);
   u = fminf(fmaxf(u, -p.limit), p.limit);
   return g * sigmoid_f(p.alpha * g) * (u + 1.0f);
@@ -47,7 +49,9 @@ __device__ __forceinline__ void gg_store(const CUtensorMap* map, uint32_t src, i
                "r"(c1) : "memory");
 }
 
-// ACT: the gated activation, known at compile time (a branch per value instead leaves nothing to overlap: 57 us a tile)
+// ACT: the activation, known at compile time: a switch per value leaves nothing to overlap (whole launches, gated relu
+// 59.7 -> 25.1 us for 2048 x 1360 x 2048 and 152 -> 71 for F 5464; product and activation pass 31.9 and 97).  Only the two activations that take numbers of their
+// own, which no layer puts here, are named at run time (GG_ANY).
 template <int EPI, int ACT>
 __global__ void __launch_bounds__(GG_THREADS, 1)
 gemm_group_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -172,7 +176,7 @@ gemm_group_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
                 r[i] = pack_bf16(__uint_as_float(v[8 * j + 2 * i]), __uint_as_float(v[8 * j + 2 * i + 1]));
-                if (p.act != ACT_NONE) r[i] = pack_bf16(apply_act(bf16_lo(r[i]), p.act, 0.0f, 0.0f), apply_act(bf16_hi(r[i]), p.act, 0.0f, 0.0f));
+                if constexpr (ACT != ACT_NONE) r[i] = pack_bf16(gg_act<ACT>(bf16_lo(r[i]), p), gg_act<ACT>(bf16_hi(r[i]), p));
               }
               w[h * 4 + j] = make_uint4(r[0], r[1], r[2], r[3]);
             }
@@ -207,6 +211,20 @@ gemm_group_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   if (warp == 2) tc::tmem_dealloc(tmem, 512);
 }
 
+using GroupKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const GroupGemm);
+template <int EPI>
+static GroupKernel group_kernel(int act) {
+  switch (act) {
+    case ACT_NONE: return gemm_group_kernel<EPI, ACT_NONE>;
+    case ACT_RELU2: return gemm_group_kernel<EPI, ACT_RELU2>;
+    case ACT_GELU_TANH: return gemm_group_kernel<EPI, ACT_GELU_TANH>;
+    case ACT_SILU: return gemm_group_kernel<EPI, ACT_SILU>;
+    case ACT_SIGMOID: return gemm_group_kernel<EPI, ACT_SIGMOID>;
+    case ACT_RELU: return gemm_group_kernel<EPI, ACT_RELU>;
+    default: return gemm_group_kernel<EPI, GG_ANY>;
+  }
+}
+
 static int group_launch(int epi, const void* x, const void* w, void* out, int M, GroupGemm p, int w_rows, int num_sms, cudaStream_t st) {
   CUtensorMap ta, tb, to;
   int rc;
@@ -218,9 +236,8 @@ static int group_launch(int epi, const void* x, const void* w, void* out, int M,
   p.a_blocks = (M + GG_BM - 1) / GG_BM;
   p.b_blocks = (p.N + cols - 1) / cols;
   const long tiles = (long)p.a_blocks * p.b_blocks;
-  auto* kern = epi == GG_F32 ? gemm_group_kernel<GG_F32, ACT_NONE> : epi == GG_BF16 ? gemm_group_kernel<GG_BF16, ACT_NONE>
-               : p.kind == 1 ? gemm_group_kernel<GG_GLU, GG_CLAMPED> : p.act == ACT_SILU ? gemm_group_kernel<GG_GLU, ACT_SILU>
-               : p.act == ACT_GELU_TANH ? gemm_group_kernel<GG_GLU, ACT_GELU_TANH> : gemm_group_kernel<GG_GLU, GG_ANY>;
+  auto* kern = epi == GG_F32 ? gemm_group_kernel<GG_F32, ACT_NONE> : epi == GG_BF16 ? group_kernel<GG_BF16>(p.act)
+               : p.kind == 1 ? gemm_group_kernel<GG_GLU, GG_CLAMPED> : group_kernel<GG_GLU>(p.act);
   JL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GG_SMEM));
   JL_CUDA(launch_pdl(kern, dim3((unsigned)(tiles < num_sms ? tiles : num_sms)), dim3(GG_THREADS), GG_SMEM, st, ta, tb, to, p));
   return JL_OK;

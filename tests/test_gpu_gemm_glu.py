@@ -7,12 +7,13 @@ from jax_llama_b200.ops import seq_kernels as SK
 pytestmark = pytest.mark.gpu
 
 ACTS = {"silu": lambda z: z * torch.sigmoid(z), "relu": torch.relu, "relu2": lambda z: torch.relu(z) ** 2,
-        "gelu_tanh": lambda z: torch.nn.functional.gelu(z, approximate="tanh")}
+        "gelu_tanh": lambda z: torch.nn.functional.gelu(z, approximate="tanh"), "sigmoid": torch.sigmoid, "none": lambda z: z,
+        "xielu": lambda z: 0.5 * z}                        # (its two numbers are zero here)
 
 
 @pytest.mark.parametrize("M", [1, 127, 128, 129, 300])
 @pytest.mark.parametrize("F,Kd,gap", [(8, 8, 0), (120, 72, 16), (128, 64, 0), (136, 520, 8), (1000, 256, 0)])
-@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "relu", "relu2", "clamped"])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "relu", "relu2", "sigmoid", "none", "xielu", "clamped"])
 def test_gated_product(M, F, Kd, gap, act):
     """fp32 sums of K products (2^-17 of the sum of their sizes, tensor cores cut off when they add), fp32 activations, one rounding to bfloat16; nothing
     beyond the result is written."""
@@ -34,7 +35,7 @@ def test_gated_product(M, F, Kd, gap, act):
     assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() - bound).max())
 
 
-@pytest.mark.parametrize("act", [SK.ACT_NONE, SK.ACT_RELU2, SK.ACT_SILU])
+@pytest.mark.parametrize("act", [SK.ACT_NONE, SK.ACT_RELU2, SK.ACT_SILU, SK.ACT_GELU_TANH, SK.ACT_SIGMOID, SK.ACT_RELU, SK.ACT_XIELU])
 @pytest.mark.parametrize("N,Kd", [(8, 64), (264, 136), (512, 1024)])
 def test_sorted_rows(N, Kd, act):
     """Tiles of several matrices, padding tiles, a device count that leaves the last tiles alone; the gated form over the same rows."""
@@ -47,7 +48,7 @@ def test_sorted_rows(N, Kd, act):
             want = x[t * 128:(t + 1) * 128].double() @ w[int(group[t])].double().T
             if not out_f32:
                 want = want.bfloat16().double()
-                want = {SK.ACT_NONE: want, SK.ACT_RELU2: torch.relu(want) ** 2, SK.ACT_SILU: want * torch.sigmoid(want)}[act]
+                want = ACTS[next(n for n, a in SK.ACTIVATIONS.items() if a == act)](want)
             err = (got[t * 128:(t + 1) * 128].double() - want).abs()
             # a value that rounds the other way before the activation: two roundings, slope at most 2 max(1, |value|)
             assert bool((err <= (1e-4 if out_f32 else 2.0 ** -6 * (1.0 + want.abs()))).all())

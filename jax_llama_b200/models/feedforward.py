@@ -35,14 +35,25 @@ def _gated_product(h: torch.Tensor, w: torch.Tensor, u_off: int, F: int, act: st
     return SK.gemm_glu(h, w, u_off, F, kind=SK.GLU_PRODUCT, act=SK.ACTIVATIONS[act], **kw)
 
 
-def _takes_gated_product(h: torch.Tensor, F: int) -> bool:
-    return (SK.tensor_cores_enabled() and h.dtype == torch.bfloat16 and h.shape[0] > 128 and h.shape[1] % 8 == 0 and F % 8 == 0
+def _takes_gated_product(h: torch.Tensor, w: torch.Tensor, F: int) -> bool:
+    """Whether product and activation go in one kernel.  Not where the product alone can split K over the SMs that the one kernel's few tiles leave idle:
+    up to 256 rows and half as many tiles as SMs, from a K on that pays for the split and the second launch (µs, two kernels | one: 129 × F 1024 × K 2048
+    10.4 | 16.6; 200 × 256 × 512 8.9 | 9.6, 200 × 4736 × 512 11.4 | 10.8, × 768 12.2 | 12.4; 256 × 1024 × 768 10.1 | 11.2; 256 × 2736 × 1024 13.5 | 13.5, × 2048 16.7 | 17.0;
+    beyond the line 200 × 5464 × 2048 24.8 | 18.8, 300 × 256 × 2048 15.3 | 14.2)."""
+    M, K = h.shape
+    tiles, sms = -(-w.shape[0] // 128), SK.num_sms(h.device)
+    if M <= 256 and 2 * tiles <= sms:
+        wide = 4 * tiles > sms
+        few = K >= ((2048 if wide else 768) if M > 200 else (768 if wide else 512))
+    else:
+        few = False
+    return (SK.tensor_cores_enabled() and h.dtype == torch.bfloat16 and M > 128 and not few and K % 8 == 0 and F % 8 == 0
             and h.is_contiguous() and h.data_ptr() % 16 == 0)
 
 
 def _gated_layer(h: torch.Tensor, w: torch.Tensor, u_off: int, F: int, act: str, limit: float) -> torch.Tensor:
     """act(gate h) · (up h) of a dense layer whose gate and up rows are stacked in w, in h's type."""
-    if _takes_gated_product(h, F):
+    if _takes_gated_product(h, w, F):
         return _gated_product(h, w, u_off, F, act, limit)
     return _gated_act(SK.linear(h, w, resident=True), u_off, F, act, limit, h.dtype)
 

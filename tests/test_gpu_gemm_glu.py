@@ -2,6 +2,8 @@
 import pytest
 import torch
 
+from jax_llama_b200.config import DenseMlpSpec
+from jax_llama_b200.models.feedforward import DenseFeedForward, _takes_gated_product
 from jax_llama_b200.ops import seq_kernels as SK
 
 pytestmark = pytest.mark.gpu
@@ -58,3 +60,19 @@ def test_sorted_rows(N, Kd, act):
         gate, up = a @ w[int(group[t]), :N].double().T, a @ w[int(group[t]), N:].double().T
         want = gate * torch.sigmoid(gate) * up
         assert bool(((glu[t * 128:(t + 1) * 128].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all())
+
+
+@pytest.mark.parametrize("M", [128, 129, 200, 256, 257])
+@pytest.mark.parametrize("W,F,one", [(512, 1024, 201), (768, 1024, 257), (1024, 4736, 201), (2048, 2736, 257), (1024, 4744, 129), (504, 256, 129)])
+def test_gated_layers_on_either_side_of_the_line(M, W, F, one):
+    """Where product and activation are one kernel and where they are two: the gated values rounded to bfloat16 (2^-9 each), fp32 sums on both sides of
+    them.  `one`: rows from which it is one."""
+    g = torch.Generator(device="cuda").manual_seed(M + F)
+    w = {n: (torch.randn(s, generator=g, device="cuda") * s[1] ** -0.5).bfloat16() for n, s in (("gate", (F, W)), ("up", (F, W)), ("down", (W, F)))}
+    layer = DenseFeedForward(DenseMlpSpec(ff=F, act="silu", gated=True), w)
+    h = torch.randn(M, W, generator=g, device="cuda").bfloat16()
+    assert _takes_gated_product(h, layer.up, F) == (M >= one)
+    d = {n: v.double() for n, v in w.items()}
+    gate = h.double() @ d["gate"].T
+    want = (gate * torch.sigmoid(gate) * (h.double() @ d["up"].T)) @ d["down"].T
+    assert float((layer.run(h).double() - want).norm() / want.norm()) < 2.0 ** -8

@@ -444,17 +444,24 @@ static int launch_swap(const void* x, const void* w, const void* residual, void*
 
 // Up to 128 tokens always; up to 256 where K can be split over a cluster: the token-major kernel has (M / 128) x (N / 256) tiles there and no
 // split (200 tokens, us: 4096 x 4096 31.1 -> 14.5, 4096 x 14336 90.8 -> 30.6, 6144 x 4096 30.0 -> 18.7, 2048 x 2048 18.9 -> 9.8, 1024 x 1024 8.9 -> 7.7); with more
-// weights the two are equal (28672 x 4096: 62 us).
-bool gemm_swap_takes(int M, int N, int K, int num_sms) {
-  return M <= 128 || (M <= 256 && (N + GS_BM - 1) / GS_BM * 2 <= num_sms && K >= 8 * GS_BK && splitk_allowed());
+// weights the two are equal (28672 x 4096: 62 us).  What a split costs more the tokens and the tile of few features have to earn: of 256 and more features it pays from K 512
+// (200 tokens, K 512: 6.6 and 6.7 us), above 200 tokens from 768 (256 tokens x 256, fp32: K 512 6.9 -> 7.8, 768 8.0 -> 8.1, 1024 9.1 -> 8.5), of fewer from 1024 (200 x 128: K 768
+// 6.2 -> 6.9, 1024 7.3 -> 7.2) or 1536 (256 x 128: K 1024 7.3 -> 8.1, 2048 11.6 -> 9.3).  A result or residual off the 16-byte boundary comes here at every size.
+bool gemm_swap_takes(int M, int N, int K, int num_sms, bool aligned) {
+  if (M <= 128) return true;
+  const int from = !aligned ? 8 * GS_BK : N >= 256 ? (M <= 200 ? 512 : 768) : (M <= 200 ? 1024 : 1536);
+  return M <= 256 && (N + GS_BM - 1) / GS_BM * 2 <= num_sms && K >= from && splitk_allowed();
 }
 
 // Few output features over many tokens (a router): the tokens take the MMA's rows, 128 to a tile, and K is split over clusters, where the token-major kernel has a
 // tile, i.e. a CTA, per 128 tokens.  Nothing is asked for ahead of the wait.  Token-major -> this, us a launch in a chain of cold tokens (32 features, K 2048): 512 tokens
 // 12.1 -> 6.0, 2048 12.3 -> 7.2, 4096 12.4 -> 8.8; 64 features, K 4096, 2048 tokens 21.6 ->
-// 10.4; what it adds behind the norm that writes its tokens: 2048 tokens 11.7 -> 6.6 us.
-bool gemm_turned_takes(int M, int N, int K, int num_sms) {
-  return N <= 64 && M > 128 && (M + GS_BM - 1) / GS_BM * 4 <= num_sms && K >= 8 * GS_BK && splitk_allowed();
+// 10.4; what it adds behind the norm that writes its tokens: 2048 tokens 11.7 -> 6.6 us.  The line in K, norm and product of 512 tokens: 16 features, K 512 7.8 -> 6.8; 32, K 512 7.2
+// -> 7.6, 768 8.7 -> 7.3; 64, K 512 7.6 -> 8.9, 768 9.0 -> 8.9, 1024 10.6 -> 8.4.  (Products of that kind alone, one behind the other, overlap better in the token-major
+// kernel, which leaves SMs free: 4096 tokens, 64 features, K 1024 7.9 and 9.0.)
+bool gemm_turned_takes(int M, int N, int K, int num_sms, bool aligned) {
+  const int from = !aligned || N <= 16 ? 512 : N <= 32 ? 768 : 1024;
+  return N <= 64 && M > 128 && (M + GS_BM - 1) / GS_BM * 4 <= num_sms && K >= from && splitk_allowed();
 }
 int gemm_turned_f32(const void* x, const void* w, void* out, int M, int N, int K, int num_sms, unsigned long long* trace, cudaStream_t s) {
   return launch_swap<SWAP_PLAIN, true>(w, x, nullptr, out, N, M, K, num_sms, trace, s, true);

@@ -328,8 +328,9 @@ extern "C" JL_API int jl_gemm(const void* x, const void* w, const void* residual
   p.K = K;
   p.ldo = mode == EPI_SWIGLU ? N / 2 : N;
   auto s = (cudaStream_t)stream;
-  if (out_f32 && gemm_turned_takes(M, N, K, num_sms)) return gemm_turned_f32(x, w, out, M, N, K, num_sms, g_gemm_trace, s);
-  if (gemm_swap_takes(M, N, K, num_sms)) return gemm_swap(x, w, residual, out, M, N, K, mode, out_f32 != 0, num_sms, g_gemm_trace, s);
+  const bool aligned = (((uintptr_t)out | (uintptr_t)residual) & 15) == 0;      // what the token-major kernel wants
+  if (out_f32 && gemm_turned_takes(M, N, K, num_sms, aligned)) return gemm_turned_f32(x, w, out, M, N, K, num_sms, g_gemm_trace, s);
+  if (gemm_swap_takes(M, N, K, num_sms, aligned)) return gemm_swap(x, w, residual, out, M, N, K, mode, out_f32 != 0, num_sms, g_gemm_trace, s);
   // token-major tiles of the prefill shapes go to the CTA-pair kernel (cta_group::2, gemm_2cta.cu); JLLAMA_GEMM_2CTA=0
   // keeps everything on the single-CTA kernel below (A/B measurements)
   static const bool pair_on = [] { const char* e = getenv("JLLAMA_GEMM_2CTA"); return !(e && e[0] == '0'); }();

@@ -18,6 +18,7 @@
 //
 // The linear layers of jax_llama/model.py:119-150, :311-338 and :699-706 at decode and for short prompts.
 #include <atomic>
+#include <type_traits>
 
 #include "gemm_swap.cuh"
 #include "jllama_b200.h"
@@ -58,6 +59,15 @@ __device__ __forceinline__ uint32_t swap_mapa(uint32_t local_addr, int rank) {
 __device__ __forceinline__ float4 swap_ld_cluster(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+constexpr int GS_LINES = 160;                            // floats of a token's partial as lines: four of 32, 40 apart
+__device__ __forceinline__ float4 swap_ld_lines(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v.x) : "r"(addr) : "memory");
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v.y) : "r"(addr + 160) : "memory");
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v.z) : "r"(addr + 320) : "memory");
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v.w) : "r"(addr + 480) : "memory");
   return v;
 }
 
@@ -255,51 +265,67 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     // ===================================================== all warps: partial sums meet in the cluster
     pdl_wait();
     const int f0 = tile0 * GS_BM + 4 * lane;                // a warp writes 256 (SwiGLU: 128) contiguous bytes of a token
-    const uint32_t put = smem_base + ((warp & 3) * 32 + lane) * 4, get = smem_base + lane * 16;
+    // A token's partial: its features in a row, read 16 bytes a lane, four ranks' four tokens at once; or feature 4 l + j at 40 j + l, read as four lines of
+    // 128 bytes, all ranks' one token at once (the pitch of 40 keeps the writes off one another's banks).  From four ranks on the lines are faster, since a warp's
+    // 512 bytes of another SM's memory come in four pieces either way; with two or three ranks they leave too little in flight.  Rows -> lines, us: 16 x 2048 x 2048, 8
+    // ranks, 5.24 -> 5.08; 5 x 1024 x 2048, 8 ranks, 4.8 -> 4.2; 128 x 3072 x 2048, 6 ranks, 12.3 -> 10.9; 128 x 4096 x 2048, 4 ranks, 11.4 -> 10.5; 128 x 8192 x 2048, 2 ranks,
+    // 12.8 -> 14.2; 256 x 6144 x 2048, 3 ranks, 14.9 -> 18.3; and 128 x 1024 x 14336, 16 ranks, 17.0 -> 17.9 (100 tokens 15.8 and 15.7).
+    const bool lines = ksplit >= 4 && (ksplit <= 8 || p.nb <= 112);
+    const int row = lines ? GS_LINES * 4 : GS_BM * 4;
+    const uint32_t put = smem_base + (lines ? (lane & 3) * 40 + (warp & 3) * 8 + lane / 4 : (warp & 3) * 32 + lane) * 4, get = smem_base + lane * (lines ? 4 : 16);
     const bool on = f0 < p.N;
     const int per = (p.M + ksplit - 1) / ksplit, t_lo = rank * per, t_hi = t_lo + per < p.M ? t_lo + per : p.M;
     uint2 res[4];
-    auto load_res = [&](int tok0) {                         // residual of tokens tok0, tok0 + 8, + 16, + 24
+    auto load_res = [&](int tok0, int n) {                  // residual of n tokens from tok0 in steps of eight
       if constexpr (EPI == SWAP_RESIDUAL) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) res[u] = on && tok0 + 8 * u < t_hi ? swap_residual(p, tok0 + 8 * u, f0) : make_uint2(0u, 0u);
+        for (int u = 0; u < 4; ++u) if (u < n) res[u] = on && tok0 + 8 * u < t_hi ? swap_residual(p, tok0 + 8 * u, f0) : make_uint2(0u, 0u);
       }
     };
-    load_res(t_lo + warp);
+    load_res(t_lo + warp, lines ? 1 : 4);
     tc::mbar_wait(tfull_bar(0), 0);
     tc::fence_after_sync();
     if (threadIdx.x == 128) swap_stamp(p, 5);
     // the ring is free (one tile per CTA, all its MMAs done) and takes the partial
-    for (int c0 = (warp >> 2) * 16; c0 < p.nb; c0 += 32) to_shared(t_lane + c0, put + c0 * (GS_BM * 4), GS_BM * 4);
+    for (int c0 = (warp >> 2) * 16; c0 < p.nb; c0 += 32) to_shared(t_lane + c0, put + c0 * row, row);
     if (threadIdx.x == 128) swap_stamp(p, 6);
     swap_cluster_arrive();
     swap_cluster_wait();
     if (threadIdx.x == 128) swap_stamp(p, 7);
-    for (int tok0 = t_lo + warp; tok0 < t_hi; tok0 += 32) {
-      if (tok0 != t_lo + warp) load_res(tok0);
-      float x[4][4] = {};
-      for (int r0 = 0; r0 < ksplit; r0 += 4) {              // four ranks' four tokens in flight; a warp reads 512 bytes of each
-        float4 q[4][4];
+    auto meet = [&](auto ranks, auto tokens) {              // a warp takes a token at a time of each group of `tokens`
+      constexpr int R = decltype(ranks)::value, U = decltype(tokens)::value;
+      for (int tok0 = t_lo + warp; tok0 < t_hi; tok0 += 8 * U) {
+        if (tok0 != t_lo + warp) load_res(tok0, U);
+        float x[U][4] = {};
+        for (int r0 = 0; r0 < ksplit; r0 += R) {
+          float4 q[R][U];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          if (r0 + r >= ksplit) continue;
-          const uint32_t at = swap_mapa(get, r0 + r);
+          for (int r = 0; r < R; ++r) {
+            if (r0 + r >= ksplit) continue;
+            const uint32_t at = swap_mapa(get, r0 + r);
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (tok0 + 8 * u < t_hi) q[r][u] = swap_ld_cluster(at + (tok0 + 8 * u) * (GS_BM * 4));
+            for (int u = 0; u < U; ++u) {
+              if (tok0 + 8 * u >= t_hi) continue;
+              if constexpr (U == 1) q[r][u] = swap_ld_lines(at + (tok0 + 8 * u) * (GS_LINES * 4));
+              else q[r][u] = swap_ld_cluster(at + (tok0 + 8 * u) * (GS_BM * 4));
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            if (r0 + r >= ksplit) continue;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (tok0 + 8 * u < t_hi) { x[u][0] += q[r][u].x; x[u][1] += q[r][u].y; x[u][2] += q[r][u].z; x[u][3] += q[r][u].w; }
+          }
         }
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          if (r0 + r >= ksplit) continue;
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (tok0 + 8 * u < t_hi) { x[u][0] += q[r][u].x; x[u][1] += q[r][u].y; x[u][2] += q[r][u].z; x[u][3] += q[r][u].w; }
-        }
+        for (int u = 0; u < U; ++u)
+          if (on && tok0 + 8 * u < t_hi) swap_emit<EPI, OUT_F32>(p, tok0 + 8 * u, f0, x[u], res[u]);
       }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (on && tok0 + 8 * u < t_hi) swap_emit<EPI, OUT_F32>(p, tok0 + 8 * u, f0, x[u], res[u]);
-    }
+    };
+    if (lines && ksplit > 8) meet(std::integral_constant<int, 16>{}, std::integral_constant<int, 1>{});
+    else if (lines) meet(std::integral_constant<int, 8>{}, std::integral_constant<int, 1>{});
+    else meet(std::integral_constant<int, 4>{}, std::integral_constant<int, 4>{});
     if (threadIdx.x == 128) swap_stamp(p, 8);
     swap_cluster_arrive();                                  // no CTA leaves while its partial may still be read
     swap_cluster_wait();
@@ -322,12 +348,12 @@ constexpr size_t gs_smem(int stages, int nb, bool split) {
   return (size_t)stages * (GS_A_BYTES + nb * GS_BK * 2) + (split ? 0 : GS_STAGING) + 8 * (2 * stages + 4) + 16 + 1024;
 }
 
-// ring depth: two CTAs per SM up to 128 tokens; the fp32 partial (512 bytes a token) of a split fits the ring in every case
+// ring depth: two CTAs per SM up to 128 tokens; the fp32 partial (up to 640 bytes a token) of a split fits the ring in every case
 static int gs_stages(int nb, int num_kb, bool split) {
   const int stage = (int)(GS_A_BYTES + nb * GS_BK * 2), budget = nb > 128 ? 200 * 1024 : 111 * 1024 - (split ? 0 : (int)GS_STAGING);
   int stages = budget / stage;
   if (stages > 10) stages = 10;
-  const int tile = split ? (nb * GS_BM * 4 + stage - 1) / stage : 2;
+  const int tile = split ? (nb * GS_LINES * 4 + stage - 1) / stage : 2;
   if (stages > num_kb) stages = num_kb;
   return stages < tile ? tile : stages;
 }
@@ -365,7 +391,8 @@ static bool wide_clusters(int ks, int num_sms) {
 // the two slots of an SM hold, while a part keeps 16 k-blocks.  Clusters of 3 to 8 find place for 264 CTAs (288: a second round, 48 tiles in 6 parts
 // 17.8 us, in 4 12.6), pairs for 2 x SMs.  16 tokens, us: 32 tiles, K 14336: 4 parts 24.1, 8 22.9; 86 tiles, K 4096: 1 part 23.3, 2 18.7, 3 18.4; 112
 // tiles 1 24.8, 2 22.1; 128 tokens: 32 x 14336 33.4 -> 29.6, 86 x 4096 31.0 -> 21.7, 112 x 4096 34.0 -> 25.3; shorter parts give nothing (32 tiles, K 4096, 4 parts
-// 10.6, 8 10.4; 128 tokens 15.5 and 15.7).
+// 10.6, 8 10.4; 128 tokens 15.5 and 15.7).  Pairs that fill both slots of nearly every SM have to have longer parts where the tokens are few (16 tokens, 148 tiles: K 2048
+// 1 part 15.2, 2 16.2, K 3072 22.1 and 22.2; 133 tiles, K 4096 27.8 and 25.1; 64 tokens, 148 tiles, K 2048 16.5 and 16.5).
 // Eight CTAs are what every GPU takes as a cluster.  More pay with a long K over few tiles (9 to 16 rows of 1024 x 14336: 8 parts 11.8 us, 16
 // parts 10.1; 1536 x 14336 12.8 and 12.0 in 12 parts); at K 8192 and below, and with less than half as many again, the wider meeting costs
 // what it gives or more (1024 x 4096 5.8 and 5.9 us, 64 rows 7.8 and 8.5; 2048 x 14336, 9 parts, 13.7 and 14.1).
@@ -382,7 +409,7 @@ static int swap_parts(int nb, int tiles, int num_kb, int num_sms) {
     if (ks > 8 && (ks < 12 || num_kb <= 128 || !wide_clusters<EPI, OUT_F32>(ks, num_sms))) ks = 8;
     int more = num_kb / 16 < 8 ? num_kb / 16 : 8;
     while (more > 2 && tiles * more > 2 * num_sms - 32) --more;
-    if (more == 2 && tiles > num_sms) more = 1;
+    if (more == 2 && (tiles > num_sms || (nb <= 32 && tiles > num_sms - 16 && num_kb < 48))) more = 1;
     if (more > ks) ks = more;
   }
   if (ks > num_kb / 4) ks = num_kb / 4;

@@ -121,10 +121,8 @@ __global__ void __launch_bounds__(LR_WARPS * 32) linear_rows_kernel(const T* __r
 // weights are known to be a parameter the first ones are requested BEFORE the wait for the kernels ahead.  Bound: the weights' way from
 // memory; a CTA per group spends itself on coming and going where K is short (one load round each).
 // One B200, us in a chain of cold weights, linear_rows_kernel -> this -> this with the early request (features x K): 1 token 2048 x 2048 3.9 -> 3.4 ->
-// 2.4, 8192 x 2048 9.1 -> 8.6 -> 7.6, 32000 x 2048 27.4 -> 26.1 -> 25.0, 2048 x 8192 8.7 -> 7.8 -> 6.9, 4096 x 14336 24.9 -> 22.1 -> 21.2 (5.5 TB/s); 2 tokens 2048 x 2048
-// 3.9 -> 4.0 -> 2.8, 8192 x 2048 9.8 -> 10.5 -> 9.2; 2 tokens with more k stay with linear_rows_kernel (4096 x 14336 21.4 against 25.5: more CTAs to hide a
-// round behind).  3 and 4 tokens: what linear_mma_rows_kernel leaves (4 tokens 2048 x 2048 5.8 -> 5.4 -> 4.2,
-// 2048 x 1024 4.6 -> 4.4 -> 3.6).
+// 2.4, 8192 x 2048 9.1 -> 8.6 -> 7.6, 32000 x 2048 27.4 -> 26.1 -> 25.0, 2048 x 8192 8.7 -> 7.8 -> 6.9, 4096 x 14336 24.9 -> 22.1 -> 21.2 (5.5 TB/s).
+// 3 and 4 tokens: what linear_mma_rows_kernel leaves (4 tokens 2048 x 2048 5.8 -> 5.4 -> 4.2, 2048 x 1024 4.6 -> 4.4 -> 3.6).  Where it is not taken: flow_takes.
 constexpr int fl_ctas(int m) { return m <= 2 ? 4 : 3; }          // per SM
 
 template <typename OutT, int M>
@@ -209,6 +207,21 @@ __global__ void __launch_bounds__(LR_WARPS * 32, fl_ctas(M)) linear_flow_kernel(
       for (int i = 0; i < NV; ++i) acc[i] = 0.0f;
     }
   }
+}
+
+// Where linear_flow_kernel is the faster of the two (the same bits).  What it gains it loses again where the last of its rounds is a short one, and with two tokens
+// more CTAs hide a round better than its few.  us, linear_rows_kernel | this | this with the early request (tokens: features x K):
+//   1: 3000 x 2048 4.3 | 4.6 | 3.4, 3000 x 4096 6.3 | 7.4 | 6.4, 3000 x 8192 10.4 | 12.9 | 11.8 (a quarter of the second round), 8192 x 3072 12.5 | 12.9 | 11.8;
+//   2: 2048 x 2048 3.7 | 3.9 | 2.7, 8192 x 2048 9.8 | 10.5 | 9.2, 16384 x 2048 17.4 | 17.0 | 15.8, 2048 x 4096 5.1 | 5.7 | 4.7, 8192 x 4096 15.1 | 17.2 | 16.1;
+//   4: 2048 x 4096 8.1 | 8.5 | 7.2, 2048 x 2048 5.6 | 5.3 | 4.1.
+static bool flow_takes(int M, int N, int K, bool early) {
+  const int groups = (N + LR_ROWS - 1) / LR_ROWS, most = 148 * fl_ctas(M);
+  if (M == 1) {
+    if (groups > most && 2 * groups <= 3 * most) return early && K <= 3072;
+    return early || groups <= 2 * most || K <= 2048;
+  }
+  if (M == 2) return early ? K <= 2048 || (groups <= most && K <= 4096) : groups >= 5 * most && K <= 2048;
+  return M <= 4 && K <= (M == 3 || early ? 4096 : 2048);
 }
 
 template <typename OutT>
@@ -321,13 +334,24 @@ __global__ void __launch_bounds__((KS > 4 ? KS : 4) * 32) linear_mma_rows_kernel
   }
 }
 
+static int lm_parts(long groups, int K) {
+  int ks = 1;
+  while (ks < 16 && (K > ks * LM_MAX_SEG || (groups * ks < 148 * 14 && K >= 2 * ks * (LM_BATCH / 2)))) ks *= 2;
+  return ks;
+}
+// Long K whose CTAs (8 parts: three to an SM) need a second round for a quarter of them or less: with 3 or 4 tokens linear_rows_kernel is the faster there
+// (3 tokens, 8192 x 8192 31.1 against 34.8 us; 4096 x 8192 18.9 against 13.8, 12288 x 8192 44.1 against 39.8).
+static bool lm_short_tail(int N, int K, int nbatch) {
+  const long groups = (long)((N + 15) / 16) * nbatch, slots = 148 * 3;
+  return K > 4096 && lm_parts(groups, K) == 8 && groups > slots && 4 * groups <= 5 * slots;
+}
+
 template <typename OutT>
 static void lm_launch(const __nv_bfloat16* x, int ldx, const __nv_bfloat16* w, OutT* out, int ldo, int M, int N, int K, int act, float p0,
                       float p1, cudaStream_t st, const LinearGroup& g, int nbatch) {
   // parts of K: some 14 warps on every SM (8 KB in flight each), each part at least half a batch long, at most LM_MAX_SEG
   const long groups = (long)((N + 15) / 16) * nbatch;
-  int ks = 1;
-  while (ks < 16 && (K > ks * LM_MAX_SEG || (groups * ks < 148 * 14 && K >= 2 * ks * (LM_BATCH / 2)))) ks *= 2;
+  const int ks = lm_parts(groups, K);
   const int per = (ks > 4 ? 1 : 4 / ks) * 16;
   const dim3 grid((N + per - 1) / per, nbatch), block((ks > 4 ? ks : 4) * 32);
 #define JL_LM(KS_) case KS_: JL_LAUNCH_PDL((linear_mma_rows_kernel<OutT, KS_>), grid, block, 0, st, x, ldx, w, out, ldo, M, N, K, act, p0, p1, g); break;
@@ -406,11 +430,12 @@ static int launch_linear(const void* x, int ldx, const void* w, void* out, int l
     const int vec_ok = (K % VN == 0) && (ldx % VN == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) &&
                        (g.x_bs % VN == 0) && (g.w_bs % VN == 0);
     if constexpr (sizeof(T) == 2) {
-      if (tensor_cores && vec_ok && M > 2 && K >= LM_MIN_K && K <= 16 * LM_MAX_SEG && (long)((N + 15) / 16) * nbatch >= (M > 4 ? 96 : 192)) {
+      if (tensor_cores && vec_ok && M > 2 && K >= LM_MIN_K && K <= 16 * LM_MAX_SEG && (long)((N + 15) / 16) * nbatch >= (M > 4 ? 96 : 192) &&
+          !(M <= 4 && lm_short_tail(N, K, nbatch))) {
         lm_launch<OutT>((const T*)x, ldx, (const T*)w, (OutT*)out, ldo, M, N, K, act, p0, p1, st, g, nbatch);
         return cudaGetLastError() == cudaSuccess ? JL_OK : JL_ERR_CUDA;
       }
-      if (vec_ok && (M == 1 || (M <= 4 && K <= 4096)) && nbatch == 1 && g.w_index == nullptr)
+      if (vec_ok && nbatch == 1 && g.w_index == nullptr && flow_takes(M, N, K, early))
         return flow_launch<OutT>((const T*)x, ldx, (const T*)w, (OutT*)out, ldo, M, N, K, act, p0, p1, early, st);
     }
     const dim3 blocks((N + LR_ROWS - 1) / LR_ROWS, nbatch);

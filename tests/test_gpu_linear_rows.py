@@ -170,13 +170,14 @@ def test_a_short_k_first_does_not_set_the_number_of_resident_pairs():
 
 @pytest.mark.parametrize("N,K", [(1536, 2048), (2048, 1536), (8192, 2048), (2048, 5464), (2048, 8192), (32000, 4096)])
 @pytest.mark.parametrize("draw", [torch.randn, torch.rand])
-def test_decode_rows_are_not_further_from_float64_than_the_exact_kernel(N, K, draw):
+@pytest.mark.parametrize("M", [8, 3, 4])
+def test_decode_rows_are_not_further_from_float64_than_the_exact_kernel(N, K, draw, M):
     """Operands of either sign and of one: what the tensor core cuts off when it adds must not add up.  Thousands of outputs each, so the
     2-norm errors are known to about half a percent; they lie two to twenty percent below those of the FMA kernel."""
     g = torch.Generator().manual_seed(N + K)
     fast = exact = 0.0
     for _ in range(3):
-        x, w = draw(8, K, generator=g).bfloat16().cuda(), draw(N, K, generator=g).bfloat16().cuda()
+        x, w = draw(M, K, generator=g).bfloat16().cuda(), draw(N, K, generator=g).bfloat16().cuda()
         ref = x.double() @ w.double().T
         fast += float((SK.linear(x, w).double() - ref).norm() / ref.norm()) ** 2
         exact += float((SK.linear(x, w, tensor_cores=False).double() - ref).norm() / ref.norm()) ** 2
@@ -184,7 +185,8 @@ def test_decode_rows_are_not_further_from_float64_than_the_exact_kernel(N, K, dr
 
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4])
-@pytest.mark.parametrize("N,K", [(1, 8), (3, 2048), (130, 2056), (2371, 1024), (2371, 4096), (9481, 264), (600, 1528)])
+@pytest.mark.parametrize("N,K", [(1, 8), (3, 2048), (130, 2056), (2371, 1024), (2371, 4096), (9481, 264), (600, 1528), (2368, 4096), (2372, 4096),
+                                 (3000, 1024), (12000, 1024), (7200, 8192)])
 def test_decode_rows_that_stay_give_the_same_bits(M, N, K, monkeypatch):
     """The kernel whose CTAs walk the features forms every sum in the order of the one with a CTA per four features (which batches take)."""
     g = torch.Generator().manual_seed(N + K + M)
@@ -216,3 +218,19 @@ def test_decode_rows_of_a_parameter_in_a_graph(M, K):
         assert torch.equal(out, SK.linear(y, w2))
         for t in (x, w1, w2):
             t.copy_(torch.randn(t.shape, generator=g).bfloat16())
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K", [(2368, 2048), (2372, 3072), (2372, 3080), (3000, 4096), (2372, 2056), (3000, 1024)])
+def test_early_and_late_decode_rows_have_the_same_bits(M, N, K):
+    """Sizes on either side of the lines between the two kernels of up to four tokens, whose place depends on the early request; one of them forms the sums."""
+    if K < 1536 or M < 3 or N < 3072:                       # (more features with 3 and 4 tokens: tensor cores)
+        g = torch.Generator().manual_seed(N + K + M)
+        x, w = torch.randn(M, K, generator=g).bfloat16().cuda(), torch.randn(N, K, generator=g).bfloat16().cuda()
+        late, out = SK.linear(x, w), torch.full((M, N), 7.0, device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            SK.linear(x, w, out=out, resident=True)
+        graph.replay()
+        assert torch.equal(out, late)
+        check(late, x, w)

@@ -372,7 +372,8 @@ __global__ void __launch_bounds__(THREADS) rownorm_gate_kernel(const float* __re
 // One warp per (token, head): out = o / sqrt(mean_v(o^2) + eps) * w[v] * act(gate)   (w == nullptr: no weight)
 // Heads of up to 128 * NV channels on the 16-byte path, NV at most HG_VEC: the instance decides how many rows an SM holds in flight (NV 1 in 32 registers, NV 4
 // in 56).  2048 tokens x 16 heads of 128 (42 MB: 6.4 us): 17.8 us without the wide accesses, 14.8 with NV 4 for all, 12.1 with NV 1, 11.3 with the four gates of
-// a lane side by side.
+// a lane side by side and the weights asked for with the row (in a chain 13.7 -> 10.3).  Wider heads load the weights behind the sum and go gate by gate: the other
+// way round their loads wait for one another (heads of 512 29.6 -> 40.6, of 256 15.4 -> 17.5).
 constexpr int HG_VEC = 4;
 
 template <typename T, int NV>
@@ -387,6 +388,7 @@ __global__ void __launch_bounds__(128) headnorm_gate_kernel(const float* __restr
   float ss = 0.0f;
   if (vec) {                                              // read-outs and gate in registers, 16 bytes per access
     const float* grow = gate + (size_t)m * ldg + (size_t)hh * V;
+    constexpr bool AHEAD = NV == 1;                       // weights with the row, the four gates of a lane side by side
     float ov[NV][4], gv[NV][4];
     Raw4<T> wr[NV];
 #pragma unroll
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(128) headnorm_gate_kernel(const float* __restr
       if (i < V) {
         load4(orow + i, ov[u]);
         load4(grow + i, gv[u]);
-        if (w) wr[u].load(w + i);
+        if constexpr (AHEAD) { if (w) wr[u].load(w + i); }
 #pragma unroll
         for (int e = 0; e < 4; ++e) ss += ov[u][e] * ov[u][e];
       }
@@ -406,10 +408,16 @@ __global__ void __launch_bounds__(128) headnorm_gate_kernel(const float* __restr
       const int i = 4 * lane + 128 * u;
       if (i < V) {
         float wv[4] = {1.0f, 1.0f, 1.0f, 1.0f};
-        if (w) wr[u].get(wv);
-        apply_act_n(gv[u], gate_act, 0.f, 0.f);
+        if constexpr (AHEAD) {
+          if (w) wr[u].get(wv);
+          apply_act_n(gv[u], gate_act, 0.f, 0.f);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) ov[u][e] = ov[u][e] * r * wv[e] * gv[u][e];
+          for (int e = 0; e < 4; ++e) ov[u][e] = ov[u][e] * r * wv[e] * gv[u][e];
+        } else {
+          if (w) load4(w + i, wv);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) ov[u][e] = ov[u][e] * r * wv[e] * apply_act(gv[u][e], gate_act, 0.f, 0.f);
+        }
         store4(out + ((size_t)m * H + hh) * V + i, ov[u]);
       }
     }

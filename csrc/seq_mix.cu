@@ -67,6 +67,8 @@ __global__ void __launch_bounds__(128) embed_pair_norm_kernel(const int* __restr
 
 constexpr int CC_MAX_TAPS = 32;      // instances of 4, 8 and 32: the history and the taps of a channel live in registers
 constexpr int CC_CHUNK = 64;       // tokens per CTA along time (or half of it)
+constexpr int CC_WALK = 4;         // tokens per row from which CC_AHEAD of them are worked on side by side (8 rows of 4096 channels: 1 token 2.3 us walked, 3.2 side by
+                                   // side; 3 tokens 2.7 and 3.1; 4 tokens 3.4 and 3.3)
 constexpr int CC_AHEAD = 8;        // inputs requested at once: a walk token by token paid a memory latency for each
 
 // grid (channel blocks, rows, time chunks); a thread owns one channel and walks its chunk with the last taps-1 inputs in
@@ -75,7 +77,7 @@ constexpr int CC_AHEAD = 8;        // inputs requested at once: a walk token by 
 // 2000 tokens x 4096 channels of 4 taps on one B200 (66 MB read and written: 10 us): 51 us token by token with the taps in local memory, 30 us with
 // eight inputs asked for at once, 28 with the next eight in flight meanwhile, 24 with the activations of eight tokens side by side.  Bound: instruction issue.
 // in_bias (fp32 per channel) belongs to the projection: it is part of every input, but not of the zeros before the start.
-template <typename T, int MT>
+template <typename T, int MT, int AHEAD>
 __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restrict__ y, int ldy, int col0, int C,
                                                           const float* __restrict__ in_bias,
                                                           const T* __restrict__ w, const T* __restrict__ bias,
@@ -119,21 +121,21 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restric
   }
   const float* yp = y + (size_t)(b * S + s0) * ldy + col0 + c;
   float* op = out + (size_t)(b * S + s0) * ldo + c;
-  float next[CC_AHEAD];
+  float next[AHEAD];
 #pragma unroll
-  for (int u = 0; u < CC_AHEAD; ++u) next[u] = s0 + u < s1 && s0 + u >= first ? yp[(size_t)u * ldy] + ib : 0.0f;
-  for (int t0 = s0; t0 < s1; t0 += CC_AHEAD) {
-    float xin[CC_AHEAD];
-    yp += (size_t)CC_AHEAD * ldy;
+  for (int u = 0; u < AHEAD; ++u) next[u] = s0 + u < s1 && s0 + u >= first ? yp[(size_t)u * ldy] + ib : 0.0f;
+  for (int t0 = s0; t0 < s1; t0 += AHEAD) {
+    float xin[AHEAD];
+    yp += (size_t)AHEAD * ldy;
 #pragma unroll
-    for (int u = 0; u < CC_AHEAD; ++u) {
+    for (int u = 0; u < AHEAD; ++u) {
       xin[u] = next[u];
-      const int s = t0 + CC_AHEAD + u;
+      const int s = t0 + AHEAD + u;
       next[u] = s < s1 && s >= first ? yp[(size_t)u * ldy] + ib : 0.0f;      // in flight while the eight before it are worked on
     }
-    float acc[CC_AHEAD];
+    float acc[AHEAD];
 #pragma unroll
-    for (int u = 0; u < CC_AHEAD; ++u) {
+    for (int u = 0; u < AHEAD; ++u) {
       acc[u] = fmaf(wv[0], xin[u], bv);
 #pragma unroll
       for (int j = 0; j < MT - 1; ++j) if (j < nh) acc[u] = fmaf(wv[j + 1], hist[j], acc[u]);
@@ -143,9 +145,9 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restric
     }
     apply_act_n(acc, act, 0.0f, 0.0f);
 #pragma unroll
-    for (int u = 0; u < CC_AHEAD; ++u)
+    for (int u = 0; u < AHEAD; ++u)
       if (t0 + u < s1) op[(size_t)u * ldo] = t0 + u >= first ? acc[u] : 0.0f;
-    op += (size_t)CC_AHEAD * ldo;
+    op += (size_t)AHEAD * ldo;
   }
 }
 
@@ -440,10 +442,12 @@ extern "C" JL_API int jl_causal_conv(const float* y, int ldy, int col0, int C, c
   // half the tokens per CTA where that many CTAs leave room (2048 tokens x 2048 channels 33 -> 22 us a cold launch; at least taps - 1 tokens: 31)
   const int chunk = (long)((C + 127) / 128) * B * ((S + CC_CHUNK - 1) / CC_CHUNK) < 148 * 6 ? CC_CHUNK / 2 : CC_CHUNK;
   dim3 grid((C + 127) / 128, B, (S + chunk - 1) / chunk);
-#define JL_CC(MT_)                                                                                                              \
-  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((causal_conv_kernel<T, MT_>), dim3(grid), dim3(128), 0, stream, y, ldy, col0, C, in_bias, \
+#define JL_CC(MT_, AHEAD_)                                                                                                      \
+  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((causal_conv_kernel<T, MT_, AHEAD_>), dim3(grid), dim3(128), 0, stream, y, ldy, col0, C, in_bias, \
                                          (const T*)w, (const T*)bias, state, out, ldo, cache_len, pad_left, S, taps, act, chunk))
-  if (taps <= 4) JL_CC(4); else if (taps <= 8) JL_CC(8); else JL_CC(CC_MAX_TAPS);
+#define JL_CCS(MT_) do { if (S < CC_WALK) JL_CC(MT_, 1); else JL_CC(MT_, CC_AHEAD); } while (0)
+  if (taps <= 4) JL_CCS(4); else if (taps <= 8) JL_CCS(8); else JL_CCS(CC_MAX_TAPS);
+#undef JL_CCS
 #undef JL_CC
   JL_CUDA(cudaGetLastError());
   return JL_OK;

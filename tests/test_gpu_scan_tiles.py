@@ -101,3 +101,27 @@ def test_decay_projections_in_whole_pieces_match_the_general_preparation(dtype, 
             res += [out, state]
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), R
         assert bool(torch.isfinite(got[0]).all())
+
+
+@pytest.mark.parametrize("S", [1, 2, 3, 4, 5, 8, 9])
+@pytest.mark.parametrize("taps", [2, 4, 8, 31])
+@pytest.mark.parametrize("pad", [0, 2])
+def test_convolution_of_few_tokens(S, taps, pad):
+    """Token counts on either side of the one from which several tokens are worked on side by side, against float64; the state afterwards, padding included."""
+    g = torch.Generator().manual_seed(S + 100 * taps)
+    B, C, off = 2, 130, 3
+    y, w, bias = torch.randn(B * S, C + 5, generator=g), torch.randn(C, taps, generator=g), torch.randn(C, generator=g)
+    state = torch.randn(B, taps - 1, C, generator=g)
+    pads = torch.tensor([0, pad], dtype=torch.int32)
+    x = y[:, off:off + C].reshape(B, S, C).double()
+    for b in range(B):
+        x[b, :int(pads[b])] = 0.0
+    full = torch.cat([state.double(), x], 1)                                   # [B, taps - 1 + S, C]
+    acc = bias.double() + sum(full[:, j:j + S] * w[:, j].double() for j in range(taps))
+    want = acc * torch.sigmoid(acc)
+    for b in range(B):
+        want[b, :int(pads[b])] = 0.0
+    kept = state.cuda()
+    got = SK.causal_conv(y.cuda(), off, w.cuda(), bias.cuda(), kept, torch.zeros(1, dtype=torch.int32, device="cuda"), pads.cuda(), B, S, act=SK.ACT_SILU)
+    assert float((got.view(B, S, C).double().cpu() - want).abs().max()) < 1e-5 * taps
+    assert torch.equal(kept.cpu().double(), full[:, S:].float().double())

@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) moe_route_kernel(RouteParams p)
 // One CTA orders the n = M * top pairs by expert.  counts / offsets live in shared memory (E + 1 ints each).
 constexpr int MS_KEEP = 16;
 
+template <int KEEP>
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ idx, int n, int top, int E, int tile, int cap,
                                                         int* __restrict__ pos, int* __restrict__ row_src,
                                                         int* __restrict__ tile_group, int* __restrict__ tiles_used) {
@@ -135,13 +136,14 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
   extern __shared__ int si[];
   int* count = si;                 // [E]
   int* start = si + E;             // [E + 1], in rows
-  // One CTA, so what counts is its chain of latencies: up to MS_KEEP pairs a thread stay in registers with their ranks (all their experts
-  // asked for at once), a warp adds up the counts.  2048 tokens x 4 of 32 experts: 11.4 -> 8.7 us.
-  const bool keep = n <= MS_KEEP * (int)blockDim.x;
-  int ex[MS_KEEP], rank[MS_KEEP];
+  // One CTA, so what counts is its chain of latencies: up to KEEP pairs a thread stay in registers with their ranks (all their experts
+  // asked for at once), a warp adds up the counts.  2048 tokens x 4 of 32 experts: 11.4 -> 8.7 us.  KEEP is the smallest of 1, 4 and MS_KEEP that holds the
+  // pairs: sixteen steps of which fifteen have nothing to do are a us (200 tokens x 2 of 8 experts: 2.8 us with pairs in memory, 3.8 with MS_KEEP, 2.6 with 1).
+  const bool keep = n <= KEEP * (int)blockDim.x;
+  int ex[KEEP], rank[KEEP];
   if (keep) {
 #pragma unroll
-    for (int u = 0; u < MS_KEEP; ++u) {
+    for (int u = 0; u < KEEP; ++u) {
       const int i = threadIdx.x + u * blockDim.x;
       ex[u] = i < n ? idx[i] : -1;
     }
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
   __syncthreads();
   if (keep) {                                                      // rank within its expert (expert < 0: a pair that runs no expert)
 #pragma unroll
-    for (int u = 0; u < MS_KEEP; ++u) rank[u] = ex[u] >= 0 ? atomicAdd(&count[ex[u]], 1) : -1;
+    for (int u = 0; u < KEEP; ++u) rank[u] = ex[u] >= 0 ? atomicAdd(&count[ex[u]], 1) : -1;
   } else {
     for (int i = threadIdx.x; i < n; i += blockDim.x) pos[i] = idx[i] >= 0 ? atomicAdd(&count[idx[i]], 1) : -1;
   }
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
     for (int t = start[e] / tile; t < start[e + 1] / tile; ++t) tile_group[t] = e;
   if (keep) {
 #pragma unroll
-    for (int u = 0; u < MS_KEEP; ++u) {
+    for (int u = 0; u < KEEP; ++u) {
       const int i = threadIdx.x + u * blockDim.x;
       if (i >= n) break;
       const int at = ex[u] >= 0 ? start[ex[u]] + rank[u] : -1;     // (-1: the combine pass skips the pair)
@@ -345,7 +347,9 @@ extern "C" JL_API int jl_moe_sort(const int* idx, int M, int top, int E, int til
   JL_CHECK_ARG(cap % tile == 0 && cap >= jl_moe_sorted_rows(M * top, E, tile), "jl_moe_sort: %d rows are too few", cap);
   const size_t smem = (size_t)(2 * E + 1) * sizeof(int);
   JL_CHECK_ARG(smem <= 48 * 1024, "jl_moe_sort: %d experts do not fit shared memory", E);
-  JL_LAUNCH_PDL(moe_sort_kernel, dim3(1), dim3(1024), smem, stream, idx, M * top, top, E, tile, cap, pos, row_src, tile_group, tiles_used);
+  const int n = M * top;
+  auto* kernel = n <= 1024 ? moe_sort_kernel<1> : n <= 4096 ? moe_sort_kernel<4> : moe_sort_kernel<MS_KEEP>;
+  JL_LAUNCH_PDL(kernel, dim3(1), dim3(1024), smem, stream, idx, n, top, E, tile, cap, pos, row_src, tile_group, tiles_used);
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }

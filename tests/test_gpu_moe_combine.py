@@ -66,10 +66,11 @@ def test_buffers_that_nobody_cleared_reach_no_result(M, experts, top, dtype, mon
     assert bool(torch.isfinite(want).all()) and torch.equal(got, want)
 
 
-@pytest.mark.parametrize("M,top,E,tile", [(1, 1, 1, 16), (9, 4, 31, 16), (33, 3, 33, 64), (2048, 4, 32, 128), (4096, 4, 300, 128), (4097, 4, 5, 128)])
+@pytest.mark.parametrize("M,top,E,tile", [(1, 1, 1, 16), (9, 4, 31, 16), (33, 3, 33, 64), (512, 2, 8, 16), (1025, 1, 8, 128), (1024, 4, 8, 128), (4097, 1, 6, 128),
+                                            (2048, 4, 32, 128), (4096, 4, 300, 128), (4097, 4, 5, 128)])
 @pytest.mark.parametrize("W", [8, 12, 2056])
 def test_sorted_pairs_and_their_rows(M, top, E, tile, W):
-    """Pairs a thread keeps in registers (up to 16384) and more, experts that do not divide among a warp's lanes, pairs without an expert; every
+    """Pairs a thread keeps in registers (one, four, sixteen) and more, rows on either side of the count up to which a CTA copies one, experts that do not divide among a warp's lanes, pairs without an expert; every
     pair's place lies in its expert's segment, the places are distinct, and the gathered rows are copies (zeros where no pair is)."""
     g = torch.Generator().manual_seed(M + E)
     idx = torch.randint(-1, E, (M, top), generator=g, dtype=torch.int32)

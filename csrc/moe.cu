@@ -260,33 +260,34 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
 
 // xs[p, :] = x[row_src[p], :] (row_src[p] < 0: zeros): the rows of a step in sorted order, for kernels that cannot gather.
 // A CTA takes GR_ROWS of them, a thread a 16-byte column of each: the rows' loads are in flight together (a CTA per row: 14.2 us for 12256 rows of 2048
-// bfloat16, 50 MB written; now 9.2).
+// bfloat16, 50 MB written; now 9.2).  Few rows that fill a CTA each go one to a CTA, which then are enough to fill the SMs (2176 rows of 2048: 2.9 us, four to a
+// CTA 3.7; 4992 rows: 5.9 and 4.7; 2176 rows of 512: 2.8 and 1.6).
 constexpr int GR_ROWS = 4;
 
-template <typename T>
+template <typename T, int ROWS>
 __global__ void __launch_bounds__(256) moe_gather_kernel(const T* __restrict__ x, int ldx, const int* __restrict__ row_src,
                                                          T* __restrict__ xs, int rows, int W) {
   pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
   pdl_launch_dependents();
-  const size_t p = (size_t)blockIdx.x * GR_ROWS;
-  int src[GR_ROWS];
+  const size_t p = (size_t)blockIdx.x * ROWS;
+  int src[ROWS];
 #pragma unroll
-  for (int r = 0; r < GR_ROWS; ++r) src[r] = p + r < (size_t)rows ? row_src[p + r] : -1;
+  for (int r = 0; r < ROWS; ++r) src[r] = p + r < (size_t)rows ? row_src[p + r] : -1;
   constexpr int VN = 16 / sizeof(T);
   if (W % VN == 0 && ldx % VN == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)xs & 15) == 0) {
     for (int i = threadIdx.x; i < W / VN; i += blockDim.x) {
-      uint4 v[GR_ROWS];
+      uint4 v[ROWS];
 #pragma unroll
-      for (int r = 0; r < GR_ROWS; ++r)
+      for (int r = 0; r < ROWS; ++r)
         v[r] = src[r] >= 0 ? reinterpret_cast<const uint4*>(x + (size_t)src[r] * ldx)[i] : make_uint4(0, 0, 0, 0);
 #pragma unroll
-      for (int r = 0; r < GR_ROWS; ++r)
+      for (int r = 0; r < ROWS; ++r)
         if (p + r < (size_t)rows) reinterpret_cast<uint4*>(xs + (p + r) * W)[i] = v[r];
     }
     return;
   }
 #pragma unroll
-  for (int r = 0; r < GR_ROWS; ++r) {
+  for (int r = 0; r < ROWS; ++r) {
     if (p + r >= (size_t)rows) break;
     for (int i = threadIdx.x; i < W; i += blockDim.x) xs[(p + r) * W + i] = src[r] >= 0 ? x[(size_t)src[r] * ldx + i] : from_f<T>(0.0f);
   }
@@ -380,8 +381,12 @@ extern "C" JL_API int jl_moe_combine_ex(const float* z, int ldz, const int* pos,
 
 extern "C" JL_API int jl_moe_gather(const void* x, int ldx, const int* row_src, void* xs, int rows, int W, int dtype, void* stream) {
   JL_CHECK_ARG(rows >= 1 && W >= 1 && ldx >= W, "jl_moe_gather: bad shape");
-  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(moe_gather_kernel<T>, dim3((rows + GR_ROWS - 1) / GR_ROWS), dim3(256), 0, stream, (const T*)x, ldx,
-                                         row_src, (T*)xs, rows, W));
+  const bool few = rows <= 3072 && (long)W * (dtype == DT_BF16 ? 2 : 4) >= 2048;
+  if (few)
+    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((moe_gather_kernel<T, 1>), dim3(rows), dim3(128), 0, stream, (const T*)x, ldx, row_src, (T*)xs, rows, W));
+  else
+    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((moe_gather_kernel<T, GR_ROWS>), dim3((rows + GR_ROWS - 1) / GR_ROWS), dim3(256), 0, stream, (const T*)x, ldx,
+                                           row_src, (T*)xs, rows, W));
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }

@@ -9,8 +9,9 @@
 //     persistent CTA per SM took 224 tiles in two rounds, the second half empty.  More tiles: the same CTAs walk the list;
 //   * few tiles: the CTAs of a cluster of `ksplit` share one and take a part of K each; the finished ring takes the fp32 partial, partials
 //     meet in distributed shared memory, each CTA sums its share of the tokens in rank order — deterministic, no scratch in global memory;
-//   * the weights do not depend on the previous kernel: the ring is filled before the wait for it.  (Not in the turned form, whose A operand is the
-//     tokens: the kernels ahead let this one start before they have written a row.)
+//   * up to 128 tokens W is a parameter, which no kernel ahead writes (jllama_b200.h): the ring is filled before the wait for them.  Not above, where W may be any
+//     kernel's result (a layer's four products of 129 to 256 tokens: 44.3 us with, 44.9 without at width 1024, 76.4 and 76.8 at 4096), and not in the turned form,
+//     whose A operand is the tokens: the kernels ahead let this one start before they have written a row.
 // Epilogues: plain bf16 / fp32, residual add, SwiGLU over interleaved (w1, w3) output features.
 // One B200, us in a chain of cold weights, one persistent CTA per SM -> this (tokens x features x K): 16 x 28672 x 4096 45.8 -> 38.3 (6.1 TB/s), 16 x
 // 24000 x 2048 25.0 -> 17.8, 16 x 11008 x 4096 22.5 -> 18.4, 100 x 28672 x 4096 55 -> 44.5, 100 x 4096 x 4096 17.0 -> 14.1, 100 x 4096 x 14336 34.4 -> 27.8, 128 x 14336 x
@@ -159,7 +160,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     // ===================================================== TMA producer
     if (lane == 0) {
       // weights stream from HBM while the previous kernel runs its tail; the tokens follow after the wait for it
-      int pre = p.turned ? 0 : kb1 - kb0 < stages ? kb1 - kb0 : stages;
+      int pre = p.turned || p.M > 128 ? 0 : kb1 - kb0 < stages ? kb1 - kb0 : stages;
       const uint64_t hint_a = p.turned ? tc::EVICT_NORMAL : tc::EVICT_FIRST;      // (tokens are read again by the kernels behind)
       for (int i = 0; i < pre; ++i) {
         tc::mbar_expect_tx(full_bar(i), stage_bytes);

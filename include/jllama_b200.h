@@ -58,7 +58,8 @@ int jl_gemv_tma(const void* x, const void* w, const void* norm_w, const void* re
 /* Same linear layers for any M on the tcgen05 tensor cores (TMA-fed, TMEM accumulators).  M > 128 runs
  * token-major tiles (prefill); M <= 128, and M <= 256 with few weight rows, runs swap-AB so the weight rows fill the
  * 128-wide MMA and the batch is the MMA N (decode, short prompts).  Modes / out_f32 as in jl_gemv.  N % 8 == 0, K % 8 == 0;
- * SwiGLU needs N % 16 == 0. */
+ * SwiGLU needs N % 16 == 0.  Up to 128 rows, and in jl_gemv and jl_gemv_tma, w is a parameter: it is read ahead of the kernels before
+ * the call, so the library's own kernels directly before it must not write it. */
 int jl_gemm(const void* x, const void* w, const void* residual, void* out, int M, int N, int K, int mode,
             int out_f32, int num_sms, void* stream);
 /* Allows split-K in jl_gemm on the CURRENT device (ws != NULL; NULL forbids it): launches of few tokens with fewer

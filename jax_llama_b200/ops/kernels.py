@@ -182,7 +182,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, norm_w: Optional[torch.Tensor] =
     """y = f(x) Wᵀ with W [N, K] for the per-op path (the whole-step decode kernel has its own GEMV).  Dispatch
     by token count: M ≤ 4 → register-streaming GEMV with RMSNorm fused (JLLAMA_SMALL_M=gemv_tma selects the
     TMA-ring GEMV, which falls back when the activations do not fit next to its ring), otherwise the tcgen05
-    GEMM (swap-AB up to M = 128).  `force` ∈ {"gemv_tma", "gemv", "gemm"} pins the kernel."""
+    GEMM (swap-AB up to M = 128, and to 256 with few features).  `force` ∈ {"gemv_tma", "gemv", "gemm"} pins the kernel.  Up to 128
+    rows w is a parameter: it is read ahead of this library's kernels directly before the call, which must not write it."""
     if not x.is_cuda:
         return _linear_ref(x, w, norm_w, eps, residual, mode, out_f32)
     _bf16c(x, "x"); _bf16c(w, "w")

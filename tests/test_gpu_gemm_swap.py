@@ -154,3 +154,32 @@ def test_few_features_wait_for_the_kernel_that_writes_the_tokens(M, N, Kd, betwe
 @pytest.mark.parametrize("M,N,Kd,between", [(100, 2048, 2048, False), (128, 512, 2048, True), (200, 2048, 2048, False), (256, 4096, 1024, True)])
 def test_few_tokens_wait_for_the_kernel_that_writes_them(M, N, Kd, between, captured):
     _behind_their_writer(M, N, Kd, between, captured, 100)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("M,N,Kd", [(129, 2048, 2048), (200, 512, 4096), (256, 4096, 1024)])
+def test_weights_of_more_than_128_tokens_may_be_a_kernels_result(M, N, Kd, captured):
+    """A cast writes the weights, which held NaN, directly ahead of the product."""
+    K.ensure_gemm_workspace(torch.device(DEV))
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    masters = torch.randn(4, N, Kd, generator=g, device=DEV) * Kd ** -0.5
+    x = torch.randn(M, Kd, generator=g, device=DEV).bfloat16()
+    w, master, out = torch.empty(N, Kd, dtype=torch.bfloat16, device=DEV), masters[0].clone(), torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    want = [K.linear(x, m.bfloat16()) for m in masters]
+
+    def chain(src):
+        w.fill_(float("nan"))
+        SK.act_cast(src, torch.bfloat16, out=w)
+        K.linear(x, w, out=out)
+
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            chain(master)
+    for r in range(100):
+        if captured:
+            master.copy_(masters[r % 4])
+            graph.replay()
+        else:
+            chain(masters[r % 4])
+        assert torch.equal(out, want[r % 4])

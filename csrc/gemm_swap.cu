@@ -369,7 +369,11 @@ static bool wide_clusters(int ks, int num_sms) {
   if (v == 0) {
     auto kern = gemm_swap_kernel<EPI, OUT_F32, true>;
     int n = 0;
-    const size_t smem = gs_smem(gs_stages(16, 1 << 20, true), 16, true);      // the largest of all token counts
+    size_t smem = 0;                                       // the largest of all token counts (48: 5 stages of 22 KB, 16: 6 of 18)
+    for (int nb = 16; nb <= 128; nb += 16) {
+      const size_t s = gs_smem(gs_stages(nb, 1 << 20, true), nb, true);
+      if (s > smem) smem = s;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_sms / ks * ks);
     cfg.blockDim = dim3(GS_THREADS);

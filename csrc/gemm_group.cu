@@ -33,6 +33,7 @@ struct GroupGemm {
   const int* a_blocks_used;          // optional device count of leading A tiles that hold rows
   int kind, act;
   float limit, alpha;
+  void* narrow;                      // result of fewer than 32 columns off the 16-byte boundary (GG_F32, GG_BF16): stored element by element; else nullptr
 };
 
 template <int ACT>
@@ -186,6 +187,20 @@ gemm_group_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             for (int j = 0; j < 8; ++j) w[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
           }
         }
+        if constexpr (EPI != GG_GLU) {
+          if (p.narrow != nullptr) {
+            constexpr int ES = EPI == GG_F32 ? 4 : 2;
+            const uint32_t* e = reinterpret_cast<const uint32_t*>(w);
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (col0 + c0 + j < p.N) {
+                uint8_t* o = reinterpret_cast<uint8_t*>(p.narrow) + ((size_t)(row0 + lane) * p.N + col0 + c0 + j) * ES;
+                if constexpr (EPI == GG_F32) *reinterpret_cast<uint32_t*>(o) = e[j];
+                else *reinterpret_cast<unsigned short*>(o) = (unsigned short)(e[j / 2] >> (16 * (j & 1)));
+              }
+            continue;
+          }
+        }
         // the store before must have finished reading the buffer
         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         __syncwarp();
@@ -230,8 +245,13 @@ static int group_launch(int epi, const void* x, const void* w, void* out, int M,
   int rc;
   if ((rc = make_tmap_2d_bf16(&ta, x, M, p.K, p.K, GG_BM))) return rc;
   if ((rc = make_tmap_2d_bf16(&tb, w, w_rows, p.K, p.K, GG_BN / 2))) return rc;
-  rc = epi == GG_F32 ? make_tmap_2d_f32(&to, out, M, p.N, p.N, 32) : make_tmap_2d_bf16(&to, out, M, p.N, p.N, 32);
-  if (rc) return rc;
+  if (epi != GG_GLU && p.N < 32 && ((uintptr_t)out & 15) != 0) {
+    JL_CHECK_ARG((uintptr_t)out % (epi == GG_F32 ? 4 : 2) == 0, "jl_gemm_grouped: result off its elements' boundary");
+    p.narrow = out;
+    to = tb;                                                 // (not used)
+  } else if ((rc = epi == GG_F32 ? make_tmap_2d_f32(&to, out, M, p.N, p.N, 32) : make_tmap_2d_bf16(&to, out, M, p.N, p.N, 32))) {
+    return rc;
+  }
   const int cols = epi == GG_GLU ? GG_BN / 2 : GG_BN;
   p.a_blocks = (M + GG_BM - 1) / GG_BM;
   p.b_blocks = (p.N + cols - 1) / cols;

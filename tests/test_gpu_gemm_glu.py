@@ -4,6 +4,7 @@ import torch
 
 from jax_llama_b200.config import DenseMlpSpec
 from jax_llama_b200.models.feedforward import DenseFeedForward, _takes_gated_product
+from jax_llama_b200.ops import _lib
 from jax_llama_b200.ops import seq_kernels as SK
 
 pytestmark = pytest.mark.gpu
@@ -76,3 +77,21 @@ def test_gated_layers_on_either_side_of_the_line(M, W, F, one):
     gate = h.double() @ d["gate"].T
     want = (gate * torch.sigmoid(gate) * (h.double() @ d["up"].T)) @ d["down"].T
     assert float((layer.run(h).double() - want).norm() / want.norm()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("N", [8, 24])
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("shift", [0, 1, 3])
+def test_sorted_rows_of_few_columns_at_any_element(N, f32, shift):
+    """The C entry's result may start at any element where it has fewer than 32 columns; nothing around it is written."""
+    Kd = 72
+    g = torch.Generator().manual_seed(N)
+    x, w = torch.randn(384, Kd, generator=g).bfloat16().cuda(), torch.randn(2, N, Kd, generator=g).bfloat16().cuda()
+    group = torch.tensor([1, 0, 1], dtype=torch.int32, device="cuda")
+    room = torch.full((384 * N + 16,), 7.0, dtype=torch.float32 if f32 else torch.bfloat16, device="cuda")
+    out = room[shift:shift + 384 * N].view(384, N)
+    _lib.check(_lib.lib().jl_gemm_grouped(x.data_ptr(), w.data_ptr(), out.data_ptr(), 384, N, Kd, 2, group.data_ptr(), 0, int(f32), 0,
+                                          torch.cuda.current_stream().cuda_stream), "jl_gemm_grouped")
+    want = torch.cat([x[t * 128:(t + 1) * 128].double() @ w[int(group[t])].double().T for t in range(3)])
+    assert bool(((out.double() - want).abs() <= (1e-4 if f32 else 2.0 ** -8 * want.abs() + 1e-4)).all())
+    assert bool((room[:shift] == 7.0).all()) and bool((room[shift + 384 * N:] == 7.0).all())

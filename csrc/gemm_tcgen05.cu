@@ -40,10 +40,6 @@ struct GemmParams {
   unsigned long long* trace;         // optional [grid][16] %globaltimer stamps (jl_gemm_set_trace), NULL = off
 };
 
-__host__ __device__ constexpr int tmem_cols_for(int bn) {
-  return 2 * bn <= 32 ? 32 : (2 * bn <= 64 ? 64 : (2 * bn <= 128 ? 128 : (2 * bn <= 256 ? 256 : 512)));
-}
-
 // one thread records when it reached a point of the kernel (scripts/gemm_trace.py prints the timeline)
 __device__ __forceinline__ void gemm_stamp(const GemmParams& p, int ev) {
   if (p.trace != nullptr) {
@@ -59,8 +55,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   extern __shared__ uint8_t smem_raw[];
   constexpr uint32_t A_BYTES = GEMM_BM * GEMM_BK * 2;
   constexpr uint32_t B_BYTES = BN * GEMM_BK * 2;
-  constexpr uint32_t STAGE_BYTES = A_BYTES + (B_BYTES < 1024 ? 1024 : B_BYTES);
-  constexpr uint32_t TMEM_COLS = tmem_cols_for(BN);
+  constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
+  constexpr uint32_t TMEM_COLS = 2 * BN;                    // 256 or 512, double-buffered
   constexpr uint32_t IDESC = tc::idesc_bf16_f32(GEMM_BM, BN);
 
   const uint32_t smem_base = (tc::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -156,81 +152,78 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       if (it == 0 && threadIdx.x == 128) gemm_stamp(p, 5);
       const int ra = a_blk * GEMM_BM + quarter * 32 + lane;  // A-side row of this thread
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + as * BN;
-      constexpr int CH = BN >= 32 ? 32 : 16;
+      constexpr int CH = 32;
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += CH) {
         uint32_t v[CH];
-        if constexpr (CH == 32) tc::tmem_ld32(t_row + c0, reinterpret_cast<uint32_t(&)[32]>(v));
-        else tc::tmem_ld16(t_row + c0, reinterpret_cast<uint32_t(&)[16]>(v));
+        tc::tmem_ld32(t_row + c0, v);
         tc::tmem_ld_wait();
         const int cb0 = b_blk * BN + c0;                    // first B-side row of this chunk
-        {
-          // thread owns one token row, CH consecutive output columns
-          if (ra < p.Ra) {
-            if constexpr (EPI == EPI_SWIGLU) {
-              __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)ra * p.ldo + cb0 / 2;
-              uint32_t w[CH / 4];
+        // thread owns one token row, CH consecutive output columns
+        if (ra < p.Ra) {
+          if constexpr (EPI == EPI_SWIGLU) {
+            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)ra * p.ldo + cb0 / 2;
+            uint32_t w[CH / 4];
 #pragma unroll
-              for (int j = 0; j < CH / 4; ++j) {
-                float g0 = __bfloat162float(__float2bfloat16(__uint_as_float(v[4 * j])));
-                float u0 = __bfloat162float(__float2bfloat16(__uint_as_float(v[4 * j + 1])));
-                float g1 = __bfloat162float(__float2bfloat16(__uint_as_float(v[4 * j + 2])));
-                float u1 = __bfloat162float(__float2bfloat16(__uint_as_float(v[4 * j + 3])));
-                w[j] = pack_bf16(silu(g0) * u0, silu(g1) * u1);
-              }
-              if (cb0 + CH <= p.Rb) {
+            for (int j = 0; j < CH / 4; ++j) {
+              float g0 = __bfloat162float(__float2bfloat16(__uint_as_float(v[4 * j])));
+              float u0 = __bfloat162float(__float2bfloat16(__uint_as_float(v[4 * j + 1])));
+              float g1 = __bfloat162float(__float2bfloat16(__uint_as_float(v[4 * j + 2])));
+              float u1 = __bfloat162float(__float2bfloat16(__uint_as_float(v[4 * j + 3])));
+              w[j] = pack_bf16(silu(g0) * u0, silu(g1) * u1);
+            }
+            if (cb0 + CH <= p.Rb) {
 #pragma unroll
-                for (int j = 0; j < CH / 16; ++j)
-                  reinterpret_cast<uint4*>(o)[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
-              } else {
-                for (int j = 0; j < CH / 2; ++j)
-                  if (cb0 + 2 * j + 1 < p.Rb)
-                    o[j] = reinterpret_cast<__nv_bfloat16*>(w)[j];
-              }
-            } else if constexpr (OUT_F32) {
-              float* o = reinterpret_cast<float*>(p.out) + (size_t)ra * p.ldo + cb0;
-              if (cb0 + CH <= p.Rb) {
-#pragma unroll
-                for (int j = 0; j < CH / 4; ++j)
-                  reinterpret_cast<uint4*>(o)[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-              } else {
-                for (int j = 0; j < CH; ++j) if (cb0 + j < p.Rb) o[j] = __uint_as_float(v[j]);
-              }
+              for (int j = 0; j < CH / 16; ++j)
+                reinterpret_cast<uint4*>(o)[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
             } else {
-              __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)ra * p.ldo + cb0;
-              const bool full = cb0 + CH <= p.Rb;
-              uint32_t w[CH / 2];
-              if constexpr (EPI == EPI_RESIDUAL) {
-                const __nv_bfloat16* r = p.residual + (size_t)ra * p.ldo + cb0;
-                if (full) {
+              for (int j = 0; j < CH / 2; ++j)
+                if (cb0 + 2 * j + 1 < p.Rb)
+                  o[j] = reinterpret_cast<__nv_bfloat16*>(w)[j];
+            }
+          } else if constexpr (OUT_F32) {
+            float* o = reinterpret_cast<float*>(p.out) + (size_t)ra * p.ldo + cb0;
+            if (cb0 + CH <= p.Rb) {
 #pragma unroll
-                  for (int j = 0; j < CH / 8; ++j) {
-                    const uint4 rr = reinterpret_cast<const uint4*>(r)[j];
-                    const uint32_t rw[4] = {rr.x, rr.y, rr.z, rr.w};
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                      const uint32_t acc = pack_bf16(__uint_as_float(v[8 * j + 2 * q]), __uint_as_float(v[8 * j + 2 * q + 1]));
-                      w[4 * j + q] = pack_bf16(bf16_lo(acc) + bf16_lo(rw[q]), bf16_hi(acc) + bf16_hi(rw[q]));
-                    }
-                  }
-                } else {
-                  for (int j = 0; j < CH; ++j)
-                    if (cb0 + j < p.Rb)
-                      o[j] = __float2bfloat16(__bfloat162float(__float2bfloat16(__uint_as_float(v[j]))) +
-                                              __bfloat162float(r[j]));
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < CH / 2; ++j) w[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-              }
+              for (int j = 0; j < CH / 4; ++j)
+                reinterpret_cast<uint4*>(o)[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            } else {
+              for (int j = 0; j < CH; ++j) if (cb0 + j < p.Rb) o[j] = __uint_as_float(v[j]);
+            }
+          } else {
+            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)ra * p.ldo + cb0;
+            const bool full = cb0 + CH <= p.Rb;
+            uint32_t w[CH / 2];
+            if constexpr (EPI == EPI_RESIDUAL) {
+              const __nv_bfloat16* r = p.residual + (size_t)ra * p.ldo + cb0;
               if (full) {
 #pragma unroll
-                for (int j = 0; j < CH / 8; ++j)
-                  reinterpret_cast<uint4*>(o)[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
-              } else if constexpr (EPI != EPI_RESIDUAL) {
+                for (int j = 0; j < CH / 8; ++j) {
+                  const uint4 rr = reinterpret_cast<const uint4*>(r)[j];
+                  const uint32_t rw[4] = {rr.x, rr.y, rr.z, rr.w};
+#pragma unroll
+                  for (int q = 0; q < 4; ++q) {
+                    const uint32_t acc = pack_bf16(__uint_as_float(v[8 * j + 2 * q]), __uint_as_float(v[8 * j + 2 * q + 1]));
+                    w[4 * j + q] = pack_bf16(bf16_lo(acc) + bf16_lo(rw[q]), bf16_hi(acc) + bf16_hi(rw[q]));
+                  }
+                }
+              } else {
                 for (int j = 0; j < CH; ++j)
-                  if (cb0 + j < p.Rb) o[j] = reinterpret_cast<__nv_bfloat16*>(w)[j];
+                  if (cb0 + j < p.Rb)
+                    o[j] = __float2bfloat16(__bfloat162float(__float2bfloat16(__uint_as_float(v[j]))) +
+                                            __bfloat162float(r[j]));
               }
+            } else {
+#pragma unroll
+              for (int j = 0; j < CH / 2; ++j) w[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+            }
+            if (full) {
+#pragma unroll
+              for (int j = 0; j < CH / 8; ++j)
+                reinterpret_cast<uint4*>(o)[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+            } else if constexpr (EPI != EPI_RESIDUAL) {
+              for (int j = 0; j < CH; ++j)
+                if (cb0 + j < p.Rb) o[j] = reinterpret_cast<__nv_bfloat16*>(w)[j];
             }
           }
         }
@@ -249,7 +242,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
 static unsigned long long* g_gemm_trace = nullptr;
 
-constexpr uint32_t gemm_stage_bytes(int bn) { return GEMM_BM * GEMM_BK * 2 + (bn * GEMM_BK * 2 < 1024 ? 1024 : bn * GEMM_BK * 2); }
+constexpr uint32_t gemm_stage_bytes(int bn) { return (GEMM_BM + bn) * GEMM_BK * 2; }
 constexpr size_t gemm_smem(int stages, int bn) { return (size_t)stages * gemm_stage_bytes(bn) + 8 * (2 * stages + 4) + 16 + 1024; }
 
 template <int BN, int EPI, bool OUT_F32>

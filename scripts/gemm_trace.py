@@ -1,6 +1,6 @@
-"""Timeline of the swap-AB (decode) GEMM: where the microseconds of a 20 us kernel go.
+"""Timeline of the few-token GEMM: where the microseconds of a 20 us kernel go.
 
-Every CTA stamps %globaltimer at ten points (csrc/gemm_tcgen05.cu `gemm_stamp`); this prints, per shape, the median /
+Every CTA stamps %globaltimer at ten points (csrc/gemm_swap.cu `swap_stamp`); this prints, per shape, the median /
 max over CTAs of each point relative to the first CTA's entry, once for an isolated launch and once for the second
 of two back-to-back launches (programmatic dependent launch: its set-up and weight prefetch overlap the first)."""
 import os, sys

@@ -533,19 +533,20 @@ extern "C" JL_API size_t jl_delta_head_scan_ws_floats(int B, int S, int H, int G
   return delta_head_ws(delta_head_plan(B, H, D, Dv), B, S, H, G, off);
 }
 
+// a few tokens per row: one launch
 template <typename T, int DP>
-static int delta_head_launch(DeltaHeadParams p, const DeltaHeadPlan& plan, const void* a_bias, const void* a_log, void* stream) {
-  const dim3 grid(plan.ns, p.H, p.B), block(plan.NT);
-  const int QK = 2 * p.P * (DP + 4), SF = QK + DH_PAIR + DH_GATE + p.cols;
-  if (p.S <= DS_FUSED_MAX_TOKENS) {
-    const size_t smem = (size_t)(QK + 8) * sizeof(float);
-    JL_LAUNCH_PDL((delta_head_scan_kernel<T, DP, true>), grid, block, smem, stream, p, p.S, (const T*)a_bias, (const T*)a_log);
-    JL_CUDA(cudaGetLastError());
-    return JL_OK;
-  }
-  if constexpr (DP < 32) {
-    return JL_ERR_UNSUPPORTED;                                  // (prompts of up to 128 channels go in chunks: delta_chunk.cu)
-  } else {
+static int delta_head_step(const DeltaHeadParams& p, const DeltaHeadPlan& plan, const void* a_bias, const void* a_log, void* stream) {
+  const size_t smem = (size_t)(2 * p.P * (DP + 4) + 8) * sizeof(float);
+  JL_LAUNCH_PDL((delta_head_scan_kernel<T, DP, true>), dim3(plan.ns, p.H, p.B), dim3(plan.NT), smem, stream, p, p.S, (const T*)a_bias, (const T*)a_log);
+  JL_CUDA(cudaGetLastError());
+  return JL_OK;
+}
+
+// prompts of keys above 128 channels (narrower ones: delta_chunk.cu)
+template <typename T>
+static int delta_head_prompt(const DeltaHeadParams& p, const DeltaHeadPlan& plan, const void* a_bias, const void* a_log, void* stream) {
+  constexpr int DP = 32;                                        // (delta_head_plan)
+  const int SF = 2 * p.P * (DP + 4) + DH_PAIR + DH_GATE + p.cols;
   JL_LAUNCH_PDL((delta_head_prep_kernel<T, DP>), dim3(p.B * p.S, p.G), dim3(32 * DH_NB), 0, stream, p, (const T*)a_bias, (const T*)a_log);
   JL_CUDA(cudaGetLastError());
   int tc = DS_TC;                                               // tokens per pipeline stage: two stages have to fit
@@ -554,10 +555,9 @@ static int delta_head_launch(DeltaHeadParams p, const DeltaHeadPlan& plan, const
   JL_CHECK_ARG(smem <= 200 * 1024, "jl_delta_head_scan: key size %d does not fit the pipeline stages", p.D);
   if (smem > 48 * 1024)
     JL_CUDA(cudaFuncSetAttribute(delta_head_scan_kernel<T, DP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  JL_LAUNCH_PDL((delta_head_scan_kernel<T, DP, false>), grid, block, smem, stream, p, tc, (const T*)a_bias, (const T*)a_log);
+  JL_LAUNCH_PDL((delta_head_scan_kernel<T, DP, false>), dim3(plan.ns, p.H, p.B), dim3(plan.NT), smem, stream, p, tc, (const T*)a_bias, (const T*)a_log);
   JL_CUDA(cudaGetLastError());
   return JL_OK;
-  }
 }
 
 // The delta rule with one decay per head: a_t = exp(-exp(a_log[h]) * softplus(y[m, a_off + h] + a_bias[h])); otherwise as jl_delta_scan.
@@ -571,13 +571,19 @@ extern "C" JL_API int jl_delta_head_scan(const float* u, int ldu, int q_off, int
   JL_CHECK_ARG(plan.P <= 32, "jl_delta_head_scan: key size %d above 1024", D);
   JL_CHECK_ARG(S <= DS_FUSED_MAX_TOKENS || ws != nullptr, "jl_delta_head_scan: %d tokens per row need the workspace", S);
   JL_CHECK_ARG((uintptr_t)ws % 16 == 0, "jl_delta_head_scan: workspace on a 16-byte boundary");
-  size_t off[4];
-  delta_head_ws(plan, B, S, H, G, off);
   DeltaHeadParams p{u, ldu, q_off, k_off, v_off, G, y, ldy, b_off, a_off, B, S, H, D, Dv, plan.P, plan.cols, cache_len, pad_left, state, o,
-                    ws ? ws + off[0] : nullptr, ws ? ws + off[1] : nullptr, ws ? ws + off[2] : nullptr, ws ? ws + off[3] : nullptr};
-  if (S > DS_FUSED_MAX_TOKENS && delta_chunk_takes(D)) return delta_chunk_launch(p, ws, a_bias, a_log, dtype, (cudaStream_t)stream);
-  if (plan.DP == 8) JL_DISPATCH_DTYPE(dtype, return (delta_head_launch<T, 8>(p, plan, a_bias, a_log, stream)));
-  if (plan.DP == 16) JL_DISPATCH_DTYPE(dtype, return (delta_head_launch<T, 16>(p, plan, a_bias, a_log, stream)));
-  JL_DISPATCH_DTYPE(dtype, return (delta_head_launch<T, 32>(p, plan, a_bias, a_log, stream)));
+                    nullptr, nullptr, nullptr, nullptr};
+  if (S <= DS_FUSED_MAX_TOKENS) {
+    if (plan.DP == 8) JL_DISPATCH_DTYPE(dtype, return (delta_head_step<T, 8>(p, plan, a_bias, a_log, stream)));
+    if (plan.DP == 16) JL_DISPATCH_DTYPE(dtype, return (delta_head_step<T, 16>(p, plan, a_bias, a_log, stream)));
+    JL_DISPATCH_DTYPE(dtype, return (delta_head_step<T, 32>(p, plan, a_bias, a_log, stream)));
+  } else if (delta_chunk_takes(D)) {
+    return delta_chunk_launch(p, ws, a_bias, a_log, dtype, (cudaStream_t)stream);
+  } else {
+    size_t off[4];
+    delta_head_ws(plan, B, S, H, G, off);
+    p.qk = ws + off[0]; p.pair = ws + off[1]; p.gate = ws + off[2]; p.val = ws + off[3];
+    JL_DISPATCH_DTYPE(dtype, return (delta_head_prompt<T>(p, plan, a_bias, a_log, stream)));
+  }
   return JL_OK;
 }

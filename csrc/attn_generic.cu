@@ -1148,7 +1148,7 @@ extern "C" JL_API int jl_latent_heads(void* q, int ldq, const void* kr, int ldkr
 extern "C" JL_API int jl_head_gate(void* out, const float* gate, int ldg, int M, int H, int Dv, int dtype, void* stream) {
   JL_CHECK_ARG(M >= 1 && H >= 1 && Dv >= 1, "jl_head_gate: bad shape");
   const size_t total = (size_t)M * H * Dv;
-  const int blocks = (int)((total + 255) / 256 < 148 * 8 ? (total + 255) / 256 : 148 * 8);
+  const int blocks = (int)((total + 255) / 256 < SMS * 8 ? (total + 255) / 256 : SMS * 8);
   JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(head_gate_kernel<T>, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, (T*)out, gate, ldg, M, H, Dv));
   JL_CUDA(cudaGetLastError());
   return JL_OK;

@@ -436,10 +436,10 @@ static DeltaHeadPlan delta_head_plan(int B, int H, int D, int Dv) {
   DeltaHeadPlan r;
   r.DP = D <= 64 ? 8 : (D <= 128 ? 16 : 32);
   auto lanes = [&] { int P = 1; while (P * r.DP < D) P *= 2; return P; };
-  while (r.DP < 32 && (long)B * H * Dv * lanes() / 32 >= 148 * 4) r.DP *= 2;
+  while (r.DP < 32 && (long)B * H * Dv * lanes() / 32 >= SMS * 4) r.DP *= 2;
   r.P = lanes();
   r.NT = DS_THREADS;
-  while (r.NT / 2 >= 32 && r.NT / 2 >= 4 * r.P && (long)((Dv + r.NT / r.P - 1) / (r.NT / r.P)) * H * B < 148) r.NT /= 2;
+  while (r.NT / 2 >= 32 && r.NT / 2 >= 4 * r.P && (long)((Dv + r.NT / r.P - 1) / (r.NT / r.P)) * H * B < SMS) r.NT /= 2;
   r.cols = r.NT / r.P;
   r.ns = (Dv + r.cols - 1) / r.cols;
   return r;
@@ -460,7 +460,7 @@ static int delta_channels(int B, int H, int D, int Dv) {
   if (D > 256) return 32;
   int P = 1;
   while (P * 8 < D) P *= 2;
-  return (long)B * H * Dv * P / 32 >= 148 * 8 ? 32 : 8;
+  return (long)B * H * Dv * P / 32 >= SMS * 8 ? 32 : 8;
 }
 static int delta_lanes(int D, int DP) {
   int P = 1;
@@ -481,7 +481,7 @@ static int delta_launch(DeltaParams p, const void* a2, const void* a_bias, const
   // Threads per CTA: while the grid is short of one CTA per SM the value columns are spread over more, smaller CTAs; the
   // value part of a stage needs at least four columns per CTA (16-byte copies).
   int NT = DS_THREADS;
-  while (NT / 2 >= 32 && NT / 2 >= 4 * P && (long)((p.Dv + NT / P - 1) / (NT / P)) * p.H * p.B < 148) NT /= 2;
+  while (NT / 2 >= 32 && NT / 2 >= 4 * P && (long)((p.Dv + NT / P - 1) / (NT / P)) * p.H * p.B < SMS) NT /= 2;
   const int cols = NT / P, SF = 3 * P * (DP + 4) + cols + 4;
   dim3 grid((p.Dv + cols - 1) / cols, p.H, p.B);
   if (S <= DS_FUSED_MAX_TOKENS) {

@@ -597,7 +597,7 @@ static int gla_chunks(int B, int S, int H, int D, int Dv) {
   static const int forced = [] { const char* e = getenv("JLLAMA_GLA_CHUNKS"); return e ? atoi(e) : 0; }();
   const int P = gla_lanes(D), threads = gla_threads(P, Dv), cols = threads / P * GT_C;
   const long warps = (long)B * H * ((Dv + cols - 1) / cols) * (threads / 32);
-  int nc = (int)(148L * 12 / (warps > 0 ? warps : 1));
+  int nc = (int)((long)SMS * 12 / (warps > 0 ? warps : 1));
   if (forced > 0) nc = forced;
   if (nc > S / 64) nc = S / 64;
   if (nc > 64) nc = 64;

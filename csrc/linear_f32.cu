@@ -304,7 +304,7 @@ cudaError_t linear_f32_launch(const float* x, int ldx, const float* w, float* ou
     if (g.tile_group && sh.bn > LT_BM) continue;
     for (int s = 1; s <= 8; s *= 2) {
       if (s > 1 && k_blocks / s < 2) break;
-      const double t = (double)((tiles * s + 147) / 148) * (4000.0 + sh.cycles * ((k_blocks + s - 1) / s) + (s == 1 ? 0.0 : s < 8 ? 5000.0 : 9000.0));
+      const double t = (double)((tiles * s + SMS - 1) / SMS) * (4000.0 + sh.cycles * ((k_blocks + s - 1) / s) + (s == 1 ? 0.0 : s < 8 ? 5000.0 : 9000.0));
       if (t < best) { best = t; bn = sh.bn; splits = s; }
     }
   }

@@ -306,7 +306,7 @@ static int combine_vec(const float* z, int ldz, int top, const float* shared, in
 // Threads of a row: 128 where the rows fill every SM four times over, because a thread's rows then wait behind one look at the indices (2048
 // tokens x 4 experts, 2048 columns: 256 threads 26 us, 128 21, 512 35; 600 x 2 x 4096: 20.5 and 16.4); with fewer rows the columns' parallelism
 // counts (200 x 4 x 2048: 256 threads 10.2, 128 11.2; 64 x 4 x 4096 10.2 and 14.3).
-static int combine_threads(int M, int vec) { return vec && M >= 4 * 148 ? 128 : 256; }
+static int combine_threads(int M, int vec) { return vec && M >= 4 * SMS ? 128 : 256; }
 
 static int moe_route_launch(const float* z, int ldz, int M, int E, int top, int groups, int keep, int group_top, int score,
                             int normalise, float scale, const float* bias, const float* choice_bias, int n_real, float* ident_w,

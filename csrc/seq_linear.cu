@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(LR_WARPS * 32, fl_ctas(M)) linear_flow_kernel(
 //   2: 2048 x 2048 3.7 | 3.9 | 2.7, 8192 x 2048 9.8 | 10.5 | 9.2, 16384 x 2048 17.4 | 17.0 | 15.8, 2048 x 4096 5.1 | 5.7 | 4.7, 8192 x 4096 15.1 | 17.2 | 16.1;
 //   4: 2048 x 4096 8.1 | 8.5 | 7.2, 2048 x 2048 5.6 | 5.3 | 4.1.
 static bool flow_takes(int M, int N, int K, bool early) {
-  const int groups = (N + LR_ROWS - 1) / LR_ROWS, most = 148 * fl_ctas(M);
+  const int groups = (N + LR_ROWS - 1) / LR_ROWS, most = SMS * fl_ctas(M);
   if (M == 1) {
     if (groups > most && 2 * groups <= 3 * most) return early && K <= 3072;
     return early || groups <= 2 * most || K <= 2048;
@@ -230,7 +230,7 @@ static int flow_launch(const __nv_bfloat16* x, int ldx, const __nv_bfloat16* w, 
   const int groups = (N + LR_ROWS - 1) / LR_ROWS;
 #define JL_FL(MM)                                                                                                        \
   case MM: {                                                                                                             \
-    const int most = 148 * fl_ctas(MM);                                                                          \
+    const int most = SMS * fl_ctas(MM);                                                                          \
     JL_LAUNCH_PDL((linear_flow_kernel<OutT, MM>), dim3(groups < most ? groups : most), dim3(LR_WARPS * 32), 0, st, x, ldx, w, out, ldo, N, K, act, \
                   p0, p1, early ? 1 : 0);                                                                                \
     break;                                                                                                               \
@@ -336,13 +336,13 @@ __global__ void __launch_bounds__((KS > 4 ? KS : 4) * 32) linear_mma_rows_kernel
 
 static int lm_parts(long groups, int K) {
   int ks = 1;
-  while (ks < 16 && (K > ks * LM_MAX_SEG || (groups * ks < 148 * 14 && K >= 2 * ks * (LM_BATCH / 2)))) ks *= 2;
+  while (ks < 16 && (K > ks * LM_MAX_SEG || (groups * ks < SMS * 14 && K >= 2 * ks * (LM_BATCH / 2)))) ks *= 2;
   return ks;
 }
 // Long K whose CTAs (8 parts: three to an SM) need a second round for a quarter of them or less: with 3 or 4 tokens linear_rows_kernel is the faster there
 // (3 tokens, 8192 x 8192 31.1 against 34.8 us; 4096 x 8192 18.9 against 13.8, 12288 x 8192 44.1 against 39.8).
 static bool lm_short_tail(int N, int K, int nbatch) {
-  const long groups = (long)((N + 15) / 16) * nbatch, slots = 148 * 3;
+  const long groups = (long)((N + 15) / 16) * nbatch, slots = SMS * 3;
   return K > 4096 && lm_parts(groups, K) == 8 && groups > slots && 4 * groups <= 5 * slots;
 }
 

@@ -440,7 +440,7 @@ extern "C" JL_API int jl_causal_conv(const float* y, int ldy, int col0, int C, c
   JL_CHECK_ARG(taps >= 1 && taps <= CC_MAX_TAPS, "jl_causal_conv: %d taps (1 .. %d)", taps, CC_MAX_TAPS);
   JL_CHECK_ARG(taps == 1 || state != nullptr, "jl_causal_conv: no state for %d taps", taps);
   // half the tokens per CTA where that many CTAs leave room (2048 tokens x 2048 channels 33 -> 22 us a cold launch; at least taps - 1 tokens: 31)
-  const int chunk = (long)((C + 127) / 128) * B * ((S + CC_CHUNK - 1) / CC_CHUNK) < 148 * 6 ? CC_CHUNK / 2 : CC_CHUNK;
+  const int chunk = (long)((C + 127) / 128) * B * ((S + CC_CHUNK - 1) / CC_CHUNK) < SMS * 6 ? CC_CHUNK / 2 : CC_CHUNK;
   dim3 grid((C + 127) / 128, B, (S + chunk - 1) / chunk);
 #define JL_CC(MT_, AHEAD_)                                                                                                      \
   JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((causal_conv_kernel<T, MT_, AHEAD_>), dim3(grid), dim3(128), 0, stream, y, ldy, col0, C, in_bias, \
@@ -483,7 +483,7 @@ extern "C" JL_API int jl_glu_act(const float* in, int ldi, int g_off, int u_off,
   JL_CHECK_ARG(M >= 1 && F >= 1 && (kind == 0 || kind == 1), "jl_glu_act: bad arguments");
   const int vec = F % 4 == 0 && ldi % 4 == 0 && ldo % 4 == 0 && g_off % 4 == 0 && u_off % 4 == 0 && ((uintptr_t)in | (uintptr_t)out) % 16 == 0;
   const size_t total = (size_t)M * F / (vec ? 4 : 1);
-  const int blocks = (int)((total + 255) / 256 < 148 * 8 ? (total + 255) / 256 : 148 * 8);
+  const int blocks = (int)((total + 255) / 256 < SMS * 8 ? (total + 255) / 256 : SMS * 8);
   JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(glu_act_kernel<T>, dim3(blocks), dim3(256), 0, stream, in, ldi, g_off, u_off, (T*)out, ldo,
                                          M, F, kind, act, limit, alpha, rows_used, rows_mult, vec));
   JL_CUDA(cudaGetLastError());

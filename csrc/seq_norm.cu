@@ -477,7 +477,7 @@ extern "C" JL_API int jl_act_inplace(void* data, int ld, int M, int N, int act, 
   const int vn = dtype == DT_BF16 ? 8 : 4;
   const int vec = N % vn == 0 && ld % vn == 0 && (uintptr_t)data % 16 == 0;
   const size_t work = (size_t)M * N / (vec ? vn : 1);
-  const int blocks = (int)((work + 255) / 256 < 148 * 8 ? (work + 255) / 256 : 148 * 8);
+  const int blocks = (int)((work + 255) / 256 < SMS * 8 ? (work + 255) / 256 : SMS * 8);
   JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(act_inplace_kernel<T>, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, (T*)data, ld, M, N, act, p0, p1, vec));
   JL_CUDA(cudaGetLastError());
   return JL_OK;
@@ -563,7 +563,7 @@ extern "C" JL_API int jl_weighted_sum2(const float* y1, int ld1, const void* bia
                                        float* out, int M, int W, int dtype, void* stream) {
   JL_CHECK_ARG(M >= 1 && W >= 1 && y1 != nullptr && ld1 >= W && (y2 == nullptr || ld2 >= W), "jl_weighted_sum2: bad shape M=%d W=%d", M, W);
   const size_t total = (size_t)M * W;
-  const int blocks = (int)((total + 255) / 256 < 148 * 8 ? (total + 255) / 256 : 148 * 8);
+  const int blocks = (int)((total + 255) / 256 < SMS * 8 ? (total + 255) / 256 : SMS * 8);
   JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(weighted_sum2_kernel<T>, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, y1, ld1, (const T*)bias, c1,
                                          y2, ld2, c2, out, M, W));
   JL_CUDA(cudaGetLastError());
@@ -599,7 +599,7 @@ extern "C" JL_API int jl_act_cast(const float* in, int ldi, void* out, int ldo, 
                                   int out_dtype, void* stream) {
   JL_CHECK_ARG(M >= 1 && N >= 1 && ldi >= N && ldo >= N, "jl_act_cast: bad shape M=%d N=%d ldi=%d ldo=%d", M, N, ldi, ldo);
   const size_t total = (size_t)M * N;
-  const int blocks = (int)((total + 255) / 256 < 148 * 8 ? (total + 255) / 256 : 148 * 8);
+  const int blocks = (int)((total + 255) / 256 < SMS * 8 ? (total + 255) / 256 : SMS * 8);
   JL_DISPATCH_DTYPE(out_dtype, JL_LAUNCH_PDL(act_cast_kernel<T>, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, in, ldi, (T*)out, ldo, M, N, act, p0, p1));
   JL_CUDA(cudaGetLastError());
   return JL_OK;

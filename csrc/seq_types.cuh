@@ -17,6 +17,7 @@ inline bool hybrid_tensor_cores() {
   return e == nullptr || strcmp(e, "0") != 0;
 }
 
+constexpr int SMS = 148;             // of a B200: what grids and rules of entry points without a num_sms are sized for
 enum { DT_BF16 = 0, DT_F32 = 1 };
 // epilogue / activation codes shared by the generic linears and jl_act_cast
 // ACT_XIELU: z > 0: p0 z^2 + z/2;  z <= 0: p1 (e^z - 1 - z) + z/2  (p0, p1 positive, formed by the caller from the layer's two numbers)

@@ -12,8 +12,8 @@
 // products along contiguous numbers: four rows x TC columns per thread, two FMAs an instruction (fma.rn.f32x2), the state in registers and, for the next
 // chunk's dot products, in shared memory by columns.
 // Bound: FMA issue of the few warps that the heads and columns give (64 x 128 keys x values, 32 tokens: 960 packed FMAs a thread, and three barriers).
-// Shared memory is what the walk asks most of (ncu: two thirds of its rate; a third of
-// the FMA pipe's).  One B200, 2 rows x 1000 tokens x 16 heads of 64 x 128, blocks of four tokens one after the other -> this: both launches 350 -> 101 us, the
+// Shared memory is what the walk asks most of (61 % of its wavefronts, 44 % of the FMA
+// pipe, 39 % of the issue slots).  One B200, 2 rows x 1000 tokens x 16 heads of 64 x 128, blocks of four tokens one after the other -> this: both launches 350 -> 101 us, the
 // layer 383 -> 217; 4 x 512 x 16 heads of 128 x 128 298 -> 188, 1 x 2048 x 4 heads of 128 x 128 481 -> 145, 1 x 24 x 4 heads of 32 x 64 12.4 -> 12.5, 8 x 2000 x 16 heads of
 // 64 x 128 1125 -> 695.  Error against float64 (2-norm of the read-outs, of the state): 2.0e-7, 2.0e-7 -> 1.9e-7, 1.9e-7; 128 channels 2.1e-7, 3.0e-7 -> 2.1e-7, 2.9e-7.
 #include "delta_chunk.cuh"

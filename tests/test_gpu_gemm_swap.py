@@ -183,3 +183,22 @@ def test_weights_of_more_than_128_tokens_may_be_a_kernels_result(M, N, Kd, captu
         else:
             chain(masters[r % 4])
         assert torch.equal(out, want[r % 4])
+
+
+def test_kernels_that_share_tensor_memory_take_turns():
+    """Products with little shared memory, so that the next one's CTAs come to the same SMs, before products that take all columns of tensor memory."""
+    K.ensure_gemm_workspace(torch.device(DEV))
+    g = torch.Generator(device=DEV).manual_seed(1)
+    few, many = torch.randn(16, 64, generator=g, device=DEV).bfloat16(), torch.randn(300, 64, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(20000, 64, generator=g, device=DEV) / 8).bfloat16()
+    want_few, want_many = (few.double() @ w.double().T), (many.double() @ w[:2048].double().T)
+    out_few, out_many = torch.empty(16, 20000, device=DEV), torch.empty(300, 2048, device=DEV)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(50):
+            K.linear(few, w, out=out_few, out_f32=True)
+            K.linear(many, w[:2048], out=out_many, out_f32=True)
+    for _ in range(10):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert float((out_few.double() - want_few).abs().max()) < 1e-4 and float((out_many.double() - want_many).abs().max()) < 1e-4

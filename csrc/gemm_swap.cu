@@ -478,8 +478,9 @@ static int launch_swap(const void* x, const void* w, const void* residual, void*
 // Up to 128 tokens always; up to 256 where K can be split over a cluster: the token-major kernel has (M / 128) x (N / 256) tiles there and no
 // split (200 tokens, us: 4096 x 4096 31.1 -> 14.5, 4096 x 14336 90.8 -> 30.6, 6144 x 4096 30.0 -> 18.7, 2048 x 2048 18.9 -> 9.8, 1024 x 1024 8.9 -> 7.7); with more
 // weights the two are equal (28672 x 4096: 62 us).  What a split costs more the tokens and the tile of few features have to earn: of 256 and more features it pays from K 512
-// (200 tokens, K 512: 6.6 and 6.7 us), above 200 tokens from 768 (256 tokens x 256, fp32: K 512 6.9 -> 7.8, 768 8.0 -> 8.1, 1024 9.1 -> 8.5), of fewer from 1024 (200 x 128: K 768
-// 6.2 -> 6.9, 1024 7.3 -> 7.2) or 1536 (256 x 128: K 1024 7.3 -> 8.1, 2048 11.6 -> 9.3).  A result or residual off the 16-byte boundary comes here at every size.
+// (200 tokens x 512, K 512: fp32 9.3 -> 7.6 us, bfloat16 6.7 -> 7.1), above 200 tokens from 768 (256 x 256, fp32: K 512 6.9 -> 7.8, 768 7.9 -> 8.3, 1024 9.1 -> 8.9;
+// bfloat16, K 768 9.5 -> 7.9), of fewer from 1024 (200 x 128, K 1024: fp32 8.5 -> 8.0, bfloat16 7.2 -> 7.6; K 768, bfloat16 6.2 -> 6.9) or 1536 (256 x 128, bfloat16: K 1024 7.3 -> 8.1,
+// 2048 11.6 -> 9.7).  A result or residual off the 16-byte boundary comes here at every size.
 bool gemm_swap_takes(int M, int N, int K, int num_sms, bool aligned) {
   if (M <= 128) return true;
   const int from = !aligned ? 8 * GS_BK : N >= 256 ? (M <= 200 ? 512 : 768) : (M <= 200 ? 1024 : 1536);

@@ -41,14 +41,14 @@ def _takes_gated_product(h: torch.Tensor, w: torch.Tensor, F: int) -> bool:
     10.4 | 16.6; 200 × 256 × 512 8.9 | 9.6, 200 × 4736 × 512 11.4 | 10.8, × 768 12.2 | 12.4; 256 × 1024 × 768 10.1 | 11.2; 256 × 2736 × 1024 13.5 | 13.5, × 2048 16.7 | 17.0;
     beyond the line 200 × 5464 × 2048 24.8 | 18.8, 300 × 256 × 2048 15.3 | 14.2)."""
     M, K = h.shape
-    tiles, sms = -(-w.shape[0] // 128), SK.num_sms(h.device)
-    if M <= 256 and 2 * tiles <= sms:
+    if M <= 128 or h.dtype != torch.bfloat16:
+        return False
+    if M <= 256:
+        tiles, sms = -(-w.shape[0] // 128), SK.num_sms(h.device)
         wide = 4 * tiles > sms
-        few = K >= ((2048 if wide else 768) if M > 200 else (768 if wide else 512))
-    else:
-        few = False
-    return (SK.tensor_cores_enabled() and h.dtype == torch.bfloat16 and M > 128 and not few and K % 8 == 0 and F % 8 == 0
-            and h.is_contiguous() and h.data_ptr() % 16 == 0)
+        if 2 * tiles <= sms and K >= ((2048 if wide else 768) if M > 200 else (768 if wide else 512)):
+            return False
+    return SK.tensor_cores_enabled() and K % 8 == 0 and F % 8 == 0 and h.is_contiguous() and h.data_ptr() % 16 == 0
 
 
 def _gated_layer(h: torch.Tensor, w: torch.Tensor, u_off: int, F: int, act: str, limit: float) -> torch.Tensor:

@@ -1,4 +1,5 @@
-// float32 linears of more than a few rows on tcgen05 tensor cores, with the accuracy of fp32 FMAs.
+// float32 linears of more than a few rows on tcgen05 tensor cores, with the accuracy of fp32 FMAs.  (Many rows over enough features: linear_f32_pair.cu; batches,
+// sorted rows and what is small run here.)
 //
 // A float32 number is the sum of three bfloat16 numbers, x = x1 + x2 + x3 exactly (Henry, Tang, Heinecke, "Leveraging the bfloat16 Artificial
 // Intelligence Datatype For Higher-Precision Computations", 2019): x1 is x rounded to nearest, x2 the rest rounded to nearest, |x2| <= 2^-8 |x|,
@@ -43,23 +44,6 @@ struct LinearF32 {
   float p0, p1;
   LinearGroup g;
 };
-
-// eight consecutive floats -> the 16 bytes of each part
-__device__ __forceinline__ void lf_split8(const float4& a, const float4& b, uint4 (&part)[3]) {
-  const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-  uint32_t h[3][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float r0 = v[2 * i], r1 = v[2 * i + 1];
-    h[0][i] = pack_bf16(r0, r1);
-    r0 -= bf16_lo(h[0][i]);
-    r1 -= bf16_hi(h[0][i]);
-    h[1][i] = pack_bf16(r0, r1);
-    h[2][i] = pack_bf16(r0 - bf16_lo(h[1][i]), r1 - bf16_hi(h[1][i]));            // at most 8 significant bits: exact
-  }
-#pragma unroll
-  for (int p = 0; p < 3; ++p) part[p] = make_uint4(h[p][0], h[p][1], h[p][2], h[p][3]);
-}
 
 template <int BN>
 __global__ void __launch_bounds__(LF_THREADS, 1) linear_f32_kernel(const LinearF32 p) {

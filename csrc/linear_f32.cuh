@@ -1,6 +1,8 @@
-// Host interface of the float32 linears on tensor cores (linear_f32.cu).
+// What the float32 linears on tensor cores share (linear_f32.cu, linear_f32_pair.cu), and the host interface of the first.
 #pragma once
 #include <cuda_runtime.h>
+
+#include "common.cuh"
 
 namespace jl {
 
@@ -19,6 +21,23 @@ struct LinearGroup {
 };
 
 constexpr int LT_BM = 64;           // rows of a sorted tile
+
+// eight consecutive floats -> the 16 bytes of each part
+__device__ __forceinline__ void lf_split8(const float4& a, const float4& b, uint4 (&part)[3]) {
+  const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  uint32_t h[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float r0 = v[2 * i], r1 = v[2 * i + 1];
+    h[0][i] = pack_bf16(r0, r1);
+    r0 -= bf16_lo(h[0][i]);
+    r1 -= bf16_hi(h[0][i]);
+    h[1][i] = pack_bf16(r0, r1);
+    h[2][i] = pack_bf16(r0 - bf16_lo(h[1][i]), r1 - bf16_hi(h[1][i]));            // at most 8 significant bits: exact
+  }
+#pragma unroll
+  for (int p = 0; p < 3; ++p) part[p] = make_uint4(h[p][0], h[p][1], h[p][2], h[p][3]);
+}
 
 // whether the tensor-core kernel takes these sizes, pitches and addresses
 bool linear_f32_takes(int M, int K, int ldx, const LinearGroup& g, const void* x, const void* w);

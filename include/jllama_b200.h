@@ -283,6 +283,10 @@ int jl_linear_any(const void* x, int ldx, const void* w, void* out, int ldo, int
  * kernels before it. */
 int jl_linear_resident(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1,
                        int dtype, int out_f32, void* stream);
+/* out = x W^T in float32 on CTA pairs (csrc/linear_f32_pair.cu).  jl_linear_f32_pair_ws: bytes of workspace (16-byte aligned, contents arbitrary)
+ * that a call with these operands needs, -1 where the other kernels are to be used (JL_ERR_UNSUPPORTED of the call itself). */
+long long jl_linear_f32_pair_ws(const void* x, int ldx, const void* w, int M, int N, int K, int num_sms);
+int jl_linear_f32_pair(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int num_sms, void* ws, void* stream);
 /* The same on the SIMT kernels whatever the sizes (fp32 FMAs in order of k within a thread): what JLLAMA_HYBRID_TC=0 gives every call. */
 int jl_linear_exact(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1,
                     int dtype, int out_f32, void* stream);

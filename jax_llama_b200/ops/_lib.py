@@ -64,6 +64,8 @@ _HYBRID = {
     "jl_linear_any": (i32, [vp, i32, vp, vp, i32, i32, i32, i32, i32, f32, f32, i32, i32, vp]),
     "jl_linear_resident": (i32, [vp, i32, vp, vp, i32, i32, i32, i32, i32, f32, f32, i32, i32, vp]),
     "jl_linear_exact": (i32, [vp, i32, vp, vp, i32, i32, i32, i32, i32, f32, f32, i32, i32, vp]),
+    "jl_linear_f32_pair_ws": (i64, [vp, i32, vp, i32, i32, i32, i32]),
+    "jl_linear_f32_pair": (i32, [vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, vp]),
     "jl_attn_prep": (i32, [fp, i32, i32, i32, i32, vp, vp, vp, fp, fp, i32, i32, i32, f32, ip, ip] + [i32] * 7 + [fp, i32, i32, i32, vp]),
     "jl_attn_generic": (i32, [vp, vp, vp, vp, fp, i32, ip, ip] + [i32] * 7 + [f32, fp, i32, i32, vp]),
     "jl_attn_generic_splits": (i32, [i32, i32, i32, i32]),

@@ -116,7 +116,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
     """act(x Wᵀ): x [M, K] and W [N, K] of one dtype (bf16 or fp32) → fp32 (or the operand dtype) [M, N].
 
     bfloat16 with more than 8 rows and 16-byte pitches runs the tcgen05 GEMM (fp32 accumulate; the activation is
-    then an in-place pass over the stored result), float32 with more than 8 rows the three-part tcgen05 kernel (csrc/linear_f32.cu),
+    then an in-place pass over the stored result), float32 with more than 8 rows the three-part tcgen05 kernels (csrc/linear_f32.cu,
+    from 65 rows on csrc/linear_f32_pair.cu, activations then in place as well),
     8 rows or fewer a weight-streaming kernel (bfloat16 from 3 rows on: mma.sync); everything else — and every size with
     `tensor_cores=False` or JLLAMA_HYBRID_TC=0 — the exact SIMT kernels.  `resident`: W is a parameter, written by no kernel of the
     graph a call is captured in; a decode step then reads it ahead of the kernels before."""
@@ -143,6 +144,16 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
             _lib.check(L.jl_act_inplace(out.data_ptr(), out.stride(0), M, N, act, float(p0), float(p1),
                                         dtype_code(out.dtype), _stream()), "jl_act_inplace")
         return out
+    if use_tc and x.dtype == torch.float32 and out.dtype == torch.float32 and M > 64:
+        need = L.jl_linear_f32_pair_ws(x.data_ptr(), x.stride(0), w.data_ptr(), M, N, K, num_sms(x.device))
+        if need >= 0:
+            ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
+            _lib.check(L.jl_linear_f32_pair(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), M, N, K, num_sms(x.device),
+                                            _p(ws), _stream()), "jl_linear_f32_pair")
+            if act != ACT_NONE:
+                _lib.check(L.jl_act_inplace(out.data_ptr(), out.stride(0), M, N, act, float(p0), float(p1), dtype_code(out.dtype), _stream()),
+                           "jl_act_inplace")
+            return out
     call = (L.jl_linear_resident if resident else L.jl_linear_any) if use_tc else L.jl_linear_exact
     _lib.check(call(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), M, N, K, act,
                     float(p0), float(p1), dtype_code(x.dtype), int(out.dtype == torch.float32), _stream()),

@@ -1,0 +1,90 @@
+"""float32 linears on CTA pairs (csrc/linear_f32_pair.cu) at the edges of their tiles, runs and sums, against float64.
+
+Bound of an output, with A = sum |x w|: what the six products leave out (2^-24 A), what the tensor core cuts off (at most 2^-24 of the running sum at each
+of the 24 steps of 64 k, so 24 · 2^-24 A; half of it is put back), and the rounded additions of K / 64 sums, of the folds and of the parts (2^-24 A each)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from jax_llama_b200.ops import _lib  # noqa: E402
+from jax_llama_b200.ops import seq_kernels as SK  # noqa: E402
+from jax_llama_b200.ops.kernels import num_sms  # noqa: E402
+
+
+def workspace(x, w):
+    return _lib.lib().jl_linear_f32_pair_ws(x.data_ptr(), x.stride(0), w.data_ptr(), x.shape[0], w.shape[0], x.shape[1], num_sms(x.device))
+
+
+def operands(M, N, K, seed=0, positive=False):
+    g = torch.Generator(device="cuda").manual_seed(seed + M + N + K)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    return (x.abs(), w.abs()) if positive else (x, w)
+
+
+def check(got, x, w):
+    K = x.shape[1]
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert bool(((got.double() - want).abs() <= 2.0 ** -24 * (24 + 8 + K / 64) * size).all())
+
+
+# rows at the edges of the tiles of 128, 192, 224 and 256; features and K off them; runs inside one tile, over several, whole tiles only; sums of more than 32 x 64
+@pytest.mark.parametrize("M,N,K", [(65, 2048, 1024), (128, 2050, 1028), (129, 1024, 1024), (192, 4097, 260), (193, 1031, 1100), (200, 5464, 2048), (224, 1025, 2052),
+                                   (225, 2048, 5464), (257, 256, 256), (300, 777, 256), (449, 512, 2116), (700, 257, 4228), (1025, 300, 300), (2000, 3001, 1024)])
+@pytest.mark.parametrize("positive", [False, True])
+def test_against_float64(M, N, K, positive):
+    x, w = operands(M, N, K, positive=positive)
+    assert workspace(x, w) >= 0                                # these sizes run the kernel under test
+    check(SK.linear(x, w), x, w)
+
+
+def test_same_bits_again_and_inside_a_wider_result():
+    x, w = operands(200, 1100, 2048)
+    first = SK.linear(x, w)
+    wide = torch.full((200, 1407), 7.0, device="cuda")
+    SK.linear(x, w, out=wide[:, 101:1201])                     # an odd pitch and start
+    assert torch.equal(wide[:, 101:1201], first)
+    assert bool((wide[:, :101] == 7).all()) and bool((wide[:, 1201:] == 7).all())
+    assert torch.equal(SK.linear(x, w), first)
+
+
+def test_rows_of_a_wider_input():
+    x, w = operands(150, 2048, 1024)
+    wide = torch.randn(150, 1032, device="cuda")
+    wide[:, 4:1028] = x
+    assert torch.equal(SK.linear(wide[:, 4:1028], w), SK.linear(x, w))
+
+
+@pytest.mark.parametrize("act,f", [(SK.ACT_RELU2, lambda z: torch.relu(z) ** 2), (SK.ACT_SILU, lambda z: z * torch.sigmoid(z))])
+def test_activation(act, f):
+    x, w = operands(140, 1100, 1024)
+    z = SK.linear(x, w)
+    got, want = SK.linear(x, w, act=act, out_f32=False).double(), f(z.double())
+    assert float((got - want).abs().max()) <= 2.0 ** -20 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 512, 512), (200, 1100, 2048)])      # whole tiles; parts that meet
+def test_not_finite_operands(M, N, K):
+    """What is infinite or not a number in one row or feature stays there, as FMAs give it; finite operands above bfloat16's range too."""
+    x, w = operands(M, N, K)
+    plain = SK.linear(x, w)
+    x[3, 5], x[17, K - 1], w[7, 9], w[30, 0], x[40, 70] = float("inf"), float("nan"), float("-inf"), float("nan"), 3.4e38
+    got, want = SK.linear(x, w), SK.linear(x, w, tensor_cores=False)
+    rows = torch.tensor([m for m in range(M) if m not in (3, 17, 40)], device="cuda")
+    cols = torch.tensor([n for n in range(N) if n not in (7, 30)], device="cuda")
+    assert torch.equal(got[rows][:, cols], plain[rows][:, cols])
+    for a, b in ((got[[3, 17, 40]], want[[3, 17, 40]]), (got[:, [7, 30]], want[:, [7, 30]])):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+        fin = b.isfinite()
+        assert bool(((a - b).abs()[fin] <= 1e-3 * b.abs()[fin].clamp(min=1.0)).all())
+
+
+def test_what_stays_with_the_other_kernels():
+    for M, N, K in [(64, 4096, 1024), (128, 1024, 1024), (200, 512, 1024), (300, 255, 512), (300, 512, 252), (300, 512, 510)]:
+        x, w = operands(M, N, K)
+        assert workspace(x, w) == -1
+        check(SK.linear(x, w), x, w)
+    room = torch.randn(300 * 512 + 1, device="cuda")
+    x, w = room[1:].view(300, 512), torch.randn(512, 512, device="cuda")     # rows off the 16-byte boundary
+    assert workspace(x, w) == -1
+    check(SK.linear(x, w), x, w)

@@ -1,4 +1,4 @@
-// Gated linear attention: the per-head matrix state S [D x Dv] with one decay per key channel,
+// Gated linear attention: the per-head matrix state S [D x Dv] with one decay per key channel (prompts of up to 128 key channels: gla_chunk.cu),
 //     S_t = diag(alpha_t) S_(t-1) + k_t v_t^T,     o_t = S_t^T q_t,
 // advanced token by token in fp32, for prompts (S tokens per row) and for decoding (S = 1) alike.
 //
@@ -13,6 +13,7 @@
 // the state of a left-padded row starts at its first real token.
 #include <stdlib.h>
 
+#include "gla_scan.cuh"
 #include "jllama_b200.h"
 #include "seq_types.cuh"
 #include "tcgen05.cuh"
@@ -23,86 +24,6 @@ constexpr int GS_DP = 32;        // state rows per thread
 constexpr int GS_TC = 8;         // tokens staged per chunk
 constexpr int GS_THREADS = 128;
 constexpr int GS_PITCH = GS_DP + 4;   // floats per 32 channels in shared memory: 16-byte aligned rows, distinct banks per lane group
-
-__device__ __forceinline__ float log_sigmoid(float z) {
-  return fminf(z, 0.0f) - log1pf(expf(-fabsf(z)));           // (no branch: lanes of either sign took both sides one after the other)
-}
-
-struct GlaParams {
-  const float* y; int ldy;
-  int q_off, k_off, v_off, a_off;      // columns of y: q [H*D], k [H*D], v [H*Dv], low-rank decay input [R]
-  int B, S, H, D, Dv, R, P;
-  float q_scale, inv_tau;
-  const int* cache_len; const int* pad_left;
-  float* state;                        // [B][H][D][Dv] fp32, read and written
-  float* o;                            // [B*S][H][Dv] fp32
-  // time chunks of the prompt scan (gla_stream_kernel): NC chunks of L tokens per row
-  int NC, L;
-  float* cstate;                       // [B][NC][H][D][Dv]: local end states (after mode 1), incoming states (after the combine)
-  float* cdecay;                       // [B][NC][H][D]: product of the chunk's decays per key channel
-  // retention (jl_retention_scan): one fixed decay per head instead of the projected one, rotary embedding of q and k at the
-  // token's position, k scaled after the rotation
-  const float* head_decay;             // [H] fp32, or nullptr: alpha from the low-rank projection
-  const float* cos_t; const float* sin_t; int rot, layout, max_pos;      // tables [max_pos][rot/2]; rot == 0: no rotation
-  float k_scale;
-  // state space scan (jl_ssd_scan): q / k are shared by the qk_div heads of a group; the decay of (token, head) is
-  // aux[m * ld_aux + h] and the value row is scaled by aux[m * ld_aux + H + h]
-  int qk_div;                          // heads per q / k head (1: every head has its own)
-  const float* aux; int ld_aux;
-  // linear attention over activated projections: q, k and v pass `act` (ACT_NONE: as they are)
-  int act;
-  // matrix memory (jl_mlstm_scan): the last `ones` (0 or 1) of the Dv columns are not in y but constantly one before the value
-  // scale, so the state's last column is the normaliser n and the last read-out column n . q
-  int ones;
-};
-
-__device__ __forceinline__ float scan_value(const GlaParams& p, size_t m, int h, int c) {
-  if (c >= p.Dv) return 0.0f;
-  const int dv = p.Dv - p.ones;
-  float v = c < dv ? p.y[m * p.ldy + p.v_off + h * dv + c] : 1.0f;
-  if (p.act != ACT_NONE) v = apply_act(v, p.act, 0.0f, 0.0f);
-  return p.aux ? v * p.aux[m * p.ld_aux + p.H + h] : v;
-}
-
-// q and k of channel d of head h for the token whose projection row is y[m] (position pos).
-__device__ __forceinline__ void scan_qk(const GlaParams& p, size_t m, int h, int d, int pos, float& qv, float& kv) {
-  const float* yr = p.y + m * p.ldy;
-  const int hq = p.qk_div > 1 ? h / p.qk_div : h;
-  const float* qh = yr + p.q_off + hq * p.D;
-  const float* kh = yr + p.k_off + hq * p.D;
-  if (p.rot > 0) {
-    const float* ct = p.cos_t + (size_t)pos * (p.rot / 2);
-    const float* st = p.sin_t + (size_t)pos * (p.rot / 2);
-    qv = rotary_channel(qh, d, p.rot, p.layout, ct, st) * p.q_scale;
-    kv = rotary_channel(kh, d, p.rot, p.layout, ct, st) * p.k_scale;
-  } else if (p.act != ACT_NONE) {
-    qv = apply_act(qh[d], p.act, 0.0f, 0.0f) * p.q_scale;
-    kv = apply_act(kh[d], p.act, 0.0f, 0.0f) * p.k_scale;
-  } else {
-    qv = qh[d] * p.q_scale;
-    kv = kh[d] * p.k_scale;
-  }
-}
-
-// q, k and alpha; zs: the token's low-rank decay input
-template <typename T>
-__device__ __forceinline__ void scan_channel(const GlaParams& p, size_t m, int h, int d, int pos,
-                                             const float* __restrict__ zs, const T* __restrict__ a2, const T* __restrict__ a2b,
-                                             float& qv, float& kv, float& av) {
-  scan_qk(p, m, h, d, pos, qv, kv);
-  if (p.aux) { av = p.aux[m * p.ld_aux + h]; return; }
-  if (p.head_decay) { av = p.head_decay[h]; return; }
-  const int n = h * p.D + d;
-  float z = to_f(a2b[n]);
-  for (int r = 0; r < p.R; ++r) z = fmaf(to_f(a2[(size_t)n * p.R + r]), zs[r], z);
-  av = expf(log_sigmoid(z) * p.inv_tau);
-}
-
-__device__ __forceinline__ int scan_position(const GlaParams& p, int b, int s) {
-  if (p.rot <= 0) return 0;
-  const int pos = (p.cache_len ? *p.cache_len : 0) + s - (p.pad_left ? p.pad_left[b] : 0);
-  return pos < 0 ? 0 : (pos >= p.max_pos ? p.max_pos - 1 : pos);
-}
 
 
 template <typename T>
@@ -198,6 +119,7 @@ __global__ void __launch_bounds__(GS_THREADS, 3) gla_scan_kernel(GlaParams p, co
 // 2048 tokens, 16 heads of 64 x 128, one row on one B200, both passes: 189 us with the 32 x 1 tile, 93 us with this one.
 constexpr int GS_TS = 16;        // tokens per pipeline stage
 constexpr int GT_DP = 16, GT_C = 4, GT_PITCH = GT_DP + 4;      // 16 channels in rows of 20 floats: the lanes of a group read different banks
+constexpr int GT_CUT_P = 16;     // lanes of a column group from which a prompt may be cut in time
 constexpr int GT_MAX_D = 256;    // wider keys: the fused kernel above
 
 __host__ __device__ inline int gla_lanes(int D) {
@@ -592,7 +514,7 @@ using namespace jl;
 // Time chunks of a prompt scan.  A token costs some 250 cycles of dependent latency however few warps run, so while the grid is short
 // of three CTAs per SM the prompt is cut into chunks that run side by side, in two passes (a local scan without read-outs, two thirds
 // of the work, then the read-out pass) with a small kernel between them.  16 heads of 64 x 128, 2048 tokens of one row, both passes: 170 us in 10
-// chunks, 143 in 20, 105 in 27 (one wave), 115 in 32.
+// chunks, 143 in 20, 105 in 27 (one wave), 115 in 32.  (Keys of up to 128 channels go to gla_chunk.cu from 48 to 80 tokens on and are never cut here.)
 static int gla_chunks(int B, int S, int H, int D, int Dv) {
   static const int forced = [] { const char* e = getenv("JLLAMA_GLA_CHUNKS"); return e ? atoi(e) : 0; }();
   const int P = gla_lanes(D), threads = gla_threads(P, Dv), cols = threads / P * GT_C;
@@ -601,10 +523,11 @@ static int gla_chunks(int B, int S, int H, int D, int Dv) {
   if (forced > 0) nc = forced;
   if (nc > S / 64) nc = S / 64;
   if (nc > 64) nc = 64;
-  return nc < 2 ? 1 : nc;
+  return nc < 2 || P < GT_CUT_P ? 1 : nc;
 }
 
 extern "C" JL_API size_t jl_gla_scan_ws_floats(int B, int S, int H, int D, int Dv) {
+  if (gla_chunk_takes(B, S, H, D, Dv)) return gla_chunk_ws_floats(B, S, H, D, Dv);
   const int nc = gla_chunks(B, S, H, D, Dv);
   size_t n = (size_t)B * S * H * gla_record_floats(gla_lanes(D), Dv);
   if (nc > 1) n += (size_t)B * nc * H * D * Dv + (size_t)B * nc * H * D;
@@ -622,23 +545,25 @@ static int launch_stream(GlaParams p, float* ws, cudaStream_t st) {
   p.cstate = ws + (size_t)B * S * H * gla_record_floats(P, Dv);
   p.cdecay = p.cstate + (size_t)B * nc * H * D * Dv;
   const dim3 grid((Dv + cols - 1) / cols, H, B * nc), block(threads);
-  if (smem > 48 * 1024) {
-    JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  }
+  if (smem > 48 * 1024) JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (nc == 1) {
     JL_LAUNCH_PDL((gla_stream_kernel<P, 0>), grid, block, smem, st, p, ws);
     JL_CUDA(cudaGetLastError());
     return JL_OK;
   }
-  const size_t total = (size_t)B * H * D * Dv;
-  JL_LAUNCH_PDL((gla_stream_kernel<P, 1>), grid, block, smem, st, p, ws);
-  JL_CUDA(cudaGetLastError());
-  JL_LAUNCH_PDL(gla_combine_kernel, dim3((unsigned)((total + 255) / 256 < 1184 ? (total + 255) / 256 : 1184)), dim3(256), 0, st, p);
-  JL_CUDA(cudaGetLastError());
-  JL_LAUNCH_PDL((gla_stream_kernel<P, 3>), grid, block, smem, st, p, ws);
-  JL_CUDA(cudaGetLastError());
+  if constexpr (P >= GT_CUT_P) {
+    if (smem > 48 * 1024) {
+      JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
+    const size_t total = (size_t)B * H * D * Dv;
+    JL_LAUNCH_PDL((gla_stream_kernel<P, 1>), grid, block, smem, st, p, ws);
+    JL_CUDA(cudaGetLastError());
+    JL_LAUNCH_PDL(gla_combine_kernel, dim3((unsigned)((total + 255) / 256 < 1184 ? (total + 255) / 256 : 1184)), dim3(256), 0, st, p);
+    JL_CUDA(cudaGetLastError());
+    JL_LAUNCH_PDL((gla_stream_kernel<P, 3>), grid, block, smem, st, p, ws);
+    JL_CUDA(cudaGetLastError());
+  }
   return JL_OK;
 }
 
@@ -655,6 +580,7 @@ static int launch_scan(GlaParams p, const void* a2, const void* a2_bias, float* 
   dim3 grid((Dv + cols - 1) / cols, H, B), block(GS_THREADS);
   if (ws != nullptr && D <= GT_MAX_D) {                      // prompts: token-parallel preparation, then the pipe
     cudaStream_t st = (cudaStream_t)stream;
+    if (gla_chunk_takes(B, S, H, D, Dv)) return gla_chunk_launch(p, a2, a2_bias, ws, dtype, st);
     p.P = gla_lanes(D);
     const int slots = H * (p.P * GT_DP + ((Dv + 3) & ~3));
     const dim3 pgrid((B * S + GP_TOK - 1) / GP_TOK, (slots + GP_THREADS - 1) / GP_THREADS);

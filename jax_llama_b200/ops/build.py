@@ -25,14 +25,14 @@ LIB_PATH = OUT_DIR / "libjllama_b200.so"
 STAMP = OUT_DIR / "build.stamp"
 
 # Sources whose arithmetic has to be exact float32 (true division, expf, tanhf, sqrtf): built without --use_fast_math.
-PRECISE_SOURCES = {"gemm_group.cu", "seq_norm.cu", "seq_linear.cu", "linear_f32.cu", "linear_f32_pair.cu", "attn_generic.cu", "flash_wide.cu", "gla_scan.cu", "moe.cu", "seq_mix.cu",
+PRECISE_SOURCES = {"gemm_group.cu", "seq_norm.cu", "seq_linear.cu", "linear_f32.cu", "linear_f32_pair.cu", "attn_generic.cu", "flash_wide.cu", "gla_scan.cu", "gla_chunk.cu", "moe.cu", "seq_mix.cu",
                    "delta_scan.cu", "delta_chunk.cu", "seq_token.cu"}
 
 # Named subsets of the library: a model family that needs only some kernels gets a small library of its own at the
 # first use in a fresh tree (seconds instead of the minutes of the whole-step decode kernels).  The full library
 # contains every subset; `ops/_lib.py` prefers it when it is already built.
 SUBSETS = {
-    "hybrid": ["error.cu", "seq_norm.cu", "seq_linear.cu", "linear_f32.cu", "linear_f32_pair.cu", "attn_generic.cu", "gla_scan.cu", "moe.cu", "seq_mix.cu", "delta_scan.cu", "delta_chunk.cu", "seq_token.cu", "sample_full.cu",
+    "hybrid": ["error.cu", "seq_norm.cu", "seq_linear.cu", "linear_f32.cu", "linear_f32_pair.cu", "attn_generic.cu", "gla_scan.cu", "gla_chunk.cu", "moe.cu", "seq_mix.cu", "delta_scan.cu", "delta_chunk.cu", "seq_token.cu", "sample_full.cu",
                "gemm_tcgen05.cu", "gemm_swap.cu", "gemm_group.cu", "gemm_2cta.cu", "tensormap.cu", "flash_prefill.cu", "flash_wide.cu", "prefill_attn_mma.cu", "decode_attn.cu"],
     # the members of the hybrid family whose only mixer is softmax attention: no recurrent scans, no one-token kernel of the
     # fixed head sizes
@@ -40,7 +40,7 @@ SUBSETS = {
                          "sample_full.cu", "gemm_tcgen05.cu", "gemm_swap.cu", "gemm_group.cu", "gemm_2cta.cu", "tensormap.cu", "flash_prefill.cu",
                          "flash_wide.cu", "prefill_attn_mma.cu"],
     # softmax attention (masked forms) and linear scans: no experts, no delta rule, no per-token inputs
-    "hybrid_scan": ["error.cu", "seq_norm.cu", "seq_linear.cu", "linear_f32.cu", "linear_f32_pair.cu", "attn_generic.cu", "gla_scan.cu", "seq_mix.cu", "sample_full.cu",
+    "hybrid_scan": ["error.cu", "seq_norm.cu", "seq_linear.cu", "linear_f32.cu", "linear_f32_pair.cu", "attn_generic.cu", "gla_scan.cu", "gla_chunk.cu", "seq_mix.cu", "sample_full.cu",
                     "gemm_tcgen05.cu", "gemm_swap.cu", "gemm_group.cu", "gemm_2cta.cu", "tensormap.cu", "flash_prefill.cu", "flash_wide.cu", "prefill_attn_mma.cu"],
     # softmax attention (masked forms, latents), the delta rule and experts: no other scans, no per-token inputs
     "hybrid_delta": ["error.cu", "seq_norm.cu", "seq_linear.cu", "linear_f32.cu", "linear_f32_pair.cu", "attn_generic.cu", "moe.cu", "seq_mix.cu", "delta_scan.cu", "delta_chunk.cu",

@@ -20,13 +20,46 @@ namespace jl {
 constexpr int DA_WARPS = 4;
 constexpr int DA_KPI = 4;   // keys per lane-group per iteration
 
-template <int G, int HD>
+// What the hybrid layers put around the attention of one new token (jl_attn_step): rotation and unit norm of the query heads and the key, the append, and
+// a gate per head, from the row of the fp32 projection.
+struct AttnStep {
+  const float* y; int ldy;
+  int q_off, k_off, v_off, g_off;      // columns of y; k_off < 0: another layer has appended this token's key and value; g_off < 0: no gate
+  const float* cos_t; const float* sin_t; int rot, max_pos;      // tables [max_pos][rot/2], pairs (2i, 2i+1); rot == 0: no rotation
+  int unit_norm; float eps;
+};
+
+// One head of a projection row -> bfloat16, by a warp: the rotation, then (unit) the norm over the head, in exact fp32 as attn_prep_kernel has it.
+template <int HD>
+__device__ __forceinline__ void step_head(const AttnStep& a, const float* src, int pos, bool turn, bool unit, __nv_bfloat16* dst) {
+  const int lane = threadIdx.x & 31;
+  float2 v[HD / 64];
+  float ss = 0.0f;
+#pragma unroll
+  for (int u = 0; u < HD / 64; ++u) {
+    const int i = lane + 32 * u;
+    v[u] = *reinterpret_cast<const float2*>(src + 2 * i);
+    if (turn && 2 * i + 1 < a.rot) {
+      const float c = a.cos_t[(size_t)pos * (a.rot / 2) + i], s = a.sin_t[(size_t)pos * (a.rot / 2) + i];
+      v[u] = make_float2(v[u].x * c - v[u].y * s, v[u].y * c + v[u].x * s);
+    }
+    ss += v[u].x * v[u].x + v[u].y * v[u].y;
+  }
+  const float r = unit ? __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(warp_sum(ss), (float)HD) + a.eps)) : 1.0f;
+#pragma unroll
+  for (int u = 0; u < HD / 64; ++u) *reinterpret_cast<uint32_t*>(dst + 2 * (lane + 32 * u)) = pack_bf16(v[u].x * r, v[u].y * r);
+}
+
+// STEP: the queries (and, unless another layer has them, the new key and value) come from the projection; every CTA of a key / value head prepares its
+// queries, the one whose keys include the new slot its key and value, which it also appends.  Such a step is latency: preparation, attention and gate in three
+// launches -> one, us in a graph: 2 rows x 16 heads over 4 of 128, 100 keys 8.5 -> 6.2, 8 rows 200 keys 10.8 -> 8.8, 2 x 32 heads over 8, 4000 keys (16 parts and a merge) 19.3 -> 14.5.
+template <int G, int HD, bool STEP = false>
 __global__ void __launch_bounds__(DA_WARPS * 32)
 decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc,
                    const __nv_bfloat16* __restrict__ vc, const int* __restrict__ cache_len_ptr,
                    const int* __restrict__ pad_left, float* __restrict__ o_part,
                    float* __restrict__ ml_part, __nv_bfloat16* __restrict__ out, int nkv, int T,
-                   int n_new, float scale_log2, int splits, int q_bstride) {
+                   int n_new, float scale_log2, int splits, int q_bstride, AttnStep step = AttnStep()) {
   constexpr int LPK = HD / 8;            // lanes per key row
   constexpr int GPW = 32 / LPK;          // lane-groups per warp
   constexpr int NG = DA_WARPS * GPW;     // lane-groups per CTA
@@ -54,11 +87,36 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   const int lo = first + split * chunk;
   const int hi = lo + chunk < len ? lo + chunk : len;
 
+  __shared__ __align__(16) __nv_bfloat16 s_new[STEP ? G + 2 : 1][HD];      // query heads | new key | new value
+  int slot = -1;                                                           // of the new token, where this CTA holds its key and value
+  if constexpr (STEP) {
+    const float* row = step.y + (size_t)b * step.ldy;
+    const int at = len - 1;                                                // (a full cache: the last slot, which nothing is written to)
+    const bool fits = (cache_len_ptr ? *cache_len_ptr : 0) + n_new <= T;
+    int pos = (cache_len_ptr ? *cache_len_ptr : 0) - first;
+    pos = pos < 0 ? 0 : (pos >= step.max_pos ? step.max_pos - 1 : pos);
+    const bool own = step.k_off >= 0 && fits && (valid > 0 ? at >= lo && at < hi : split == 0);
+    for (int i = warp; i < G + (own ? 2 : 0); i += DA_WARPS) {
+      if (i < G) step_head<HD>(step, row + step.q_off + (kvh * G + i) * HD, pos, true, step.unit_norm != 0, s_new[i]);
+      else if (i == G) step_head<HD>(step, row + step.k_off + kvh * HD, pos, true, step.unit_norm != 0, s_new[i]);
+      else step_head<HD>(step, row + step.v_off + kvh * HD, pos, false, false, s_new[i]);
+    }
+    __syncthreads();
+    if (own) {
+      slot = at;
+      const size_t to = (((size_t)b * nkv + kvh) * T + at) * HD + (threadIdx.x % LPK) * 8;
+      if (threadIdx.x < 2 * LPK)
+        *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(threadIdx.x < LPK ? kc : vc) + to) =
+            *reinterpret_cast<const uint4*>(&s_new[G + threadIdx.x / LPK][(threadIdx.x % LPK) * 8]);
+    }
+  }
+
   // q for the G heads of this KV group, pre-scaled by softmax_scale·log2(e)
   float qf[G][8];
 #pragma unroll
   for (int g = 0; g < G; ++g) {
-    const uint4 a = *reinterpret_cast<const uint4*>(q + (size_t)b * q_bstride + (size_t)(kvh * G + g) * HD + lig * 8);
+    const uint4 a = STEP ? *reinterpret_cast<const uint4*>(&s_new[g][lig * 8])
+                         : *reinterpret_cast<const uint4*>(q + (size_t)b * q_bstride + (size_t)(kvh * G + g) * HD + lig * 8);
     qf[g][0] = bf16_lo(a.x) * scale_log2; qf[g][1] = bf16_hi(a.x) * scale_log2;
     qf[g][2] = bf16_lo(a.y) * scale_log2; qf[g][3] = bf16_hi(a.y) * scale_log2;
     qf[g][4] = bf16_lo(a.z) * scale_log2; qf[g][5] = bf16_hi(a.z) * scale_log2;
@@ -83,9 +141,14 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     uint4 kr[DA_KPI], vr[DA_KPI];
 #pragma unroll
     for (int i = 0; i < DA_KPI; ++i) {
-      const bool ok = key0 + i < hi;
+      const bool ok = key0 + i < hi && (!STEP || key0 + i != slot);
       kr[i] = ok ? ldg_stream(kbase + (size_t)(key0 + i) * HD) : make_uint4(0, 0, 0, 0);
       vr[i] = ok ? ldg_stream(vbase + (size_t)(key0 + i) * HD) : make_uint4(0, 0, 0, 0);
+      if constexpr (STEP)
+        if (key0 + i == slot) {
+          kr[i] = *reinterpret_cast<const uint4*>(&s_new[G][lig * 8]);
+          vr[i] = *reinterpret_cast<const uint4*>(&s_new[G + 1][lig * 8]);
+        }
     }
     float part[G][DA_KPI];
 #pragma unroll
@@ -167,7 +230,10 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     }
     const int h = kvh * G + g;
     if (splits == 1) {
-      out[((size_t)b * nh + h) * HD + d] = __float2bfloat16(L > 0.f ? acc / L : 0.f);
+      float v = L > 0.f ? acc / L : 0.f;
+      if constexpr (STEP)
+        if (step.g_off >= 0) v = __fdiv_rn(v, 1.0f + expf(-step.y[(size_t)b * step.ldy + step.g_off + h]));
+      out[((size_t)b * nh + h) * HD + d] = __float2bfloat16(v);
     } else {
       const size_t pi = ((size_t)b * nh + h) * splits + split;
       o_part[pi * HD + d] = acc;
@@ -179,7 +245,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 template <int HD>
 __global__ void __launch_bounds__(HD)
 attn_combine_kernel(const float* __restrict__ o_part, const float* __restrict__ ml_part,
-                    __nv_bfloat16* __restrict__ out, int splits) {
+                    __nv_bfloat16* __restrict__ out, int splits, const float* __restrict__ gate, int ldg, int nh) {
   pdl_wait();
   pdl_launch_dependents();
   const size_t bh = blockIdx.x;
@@ -193,20 +259,23 @@ attn_combine_kernel(const float* __restrict__ o_part, const float* __restrict__ 
     acc += w * o_part[(bh * splits + s) * HD + d];
     L += w * ml_part[(bh * splits + s) * 2 + 1];
   }
-  out[bh * HD + d] = __float2bfloat16(L > 0.f ? acc / L : 0.f);
+  float v = L > 0.f ? acc / L : 0.f;
+  if (gate != nullptr) v = __fdiv_rn(v, 1.0f + expf(-gate[bh / nh * ldg + bh % nh]));
+  out[bh * HD + d] = __float2bfloat16(v);
 }
 
 template <int G, int HD>
 static cudaError_t launch_decode(const void* q, const void* kc, const void* vc, const int* cache_len_ptr,
                                  const int* pad_left, float* o_part, float* ml_part, void* out, int B,
-                                 int nkv, int T, int n_new, float scale, int splits, int q_bstride, cudaStream_t s) {
-  cudaError_t e = launch_pdl(decode_attn_kernel<G, HD>, dim3(splits, nkv, B), dim3(DA_WARPS * 32), 0, s,
+                                 int nkv, int T, int n_new, float scale, int splits, int q_bstride, cudaStream_t s, const AttnStep* step = nullptr) {
+  cudaError_t e = launch_pdl(step ? decode_attn_kernel<G, HD, true> : decode_attn_kernel<G, HD>, dim3(splits, nkv, B), dim3(DA_WARPS * 32), 0, s,
                              (const __nv_bfloat16*)q, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc,
                              cache_len_ptr, pad_left, o_part, ml_part, (__nv_bfloat16*)out, nkv, T, n_new,
-                             scale * 1.4426950408889634f, splits, q_bstride);
+                             scale * 1.4426950408889634f, splits, q_bstride, step ? *step : AttnStep());
   if (e != cudaSuccess || splits == 1) return e;
+  const float* gate = step && step->g_off >= 0 ? step->y + step->g_off : nullptr;
   return launch_pdl(attn_combine_kernel<HD>, dim3(B * nkv * G), dim3(HD), 0, s, (const float*)o_part,
-                    (const float*)ml_part, (__nv_bfloat16*)out, splits);
+                    (const float*)ml_part, (__nv_bfloat16*)out, splits, gate, gate ? step->ldy : 0, nkv * G);
 }
 
 }  // namespace jl
@@ -226,10 +295,9 @@ extern "C" JL_API int jl_decode_attn_splits(int B, int nkv, int max_len, int num
   return s < 1 ? 1 : (s > 64 ? 64 : s);
 }
 
-extern "C" JL_API int jl_decode_attn(const void* q, const void* k_cache, const void* v_cache,
-                              const int* cache_len_ptr, const int* pad_left, void* scratch, void* out,
-                              int B, int nh, int nkv, int hd, int T, int n_new, float scale, int splits,
-                              int q_bstride, void* stream) {
+static int decode_attn(const void* q, const void* k_cache, const void* v_cache, const int* cache_len_ptr, const int* pad_left, void* scratch,
+                       void* out, int B, int nh, int nkv, int hd, int T, int n_new, float scale, int splits, int q_bstride, void* stream,
+                       const AttnStep* step) {
   JL_CHECK_ARG(nkv > 0 && nh % nkv == 0, "jl_decode_attn: nh=%d not a multiple of nkv=%d", nh, nkv);
   JL_CHECK_ARG(splits >= 1 && splits <= 64, "jl_decode_attn: splits=%d outside 1..64", splits);
   JL_CHECK_ARG(splits == 1 || scratch != nullptr, "jl_decode_attn: scratch buffer required for splits > 1");
@@ -242,7 +310,7 @@ extern "C" JL_API int jl_decode_attn(const void* q, const void* k_cache, const v
 #define JL_DA(G_, HD_)                                                                              \
   if (G == G_ && hd == HD_)                                                                         \
     e = launch_decode<G_, HD_>(q, k_cache, v_cache, cache_len_ptr, pad_left, o_part, ml_part, out, B, \
-                               nkv, T, n_new, scale, splits, q_bstride > 0 ? q_bstride : nh * hd, s);
+                               nkv, T, n_new, scale, splits, q_bstride > 0 ? q_bstride : nh * hd, s, step);
   JL_DA(1, 128) else JL_DA(2, 128) else JL_DA(4, 128) else JL_DA(8, 128)
   else JL_DA(1, 64) else JL_DA(2, 64) else JL_DA(4, 64) else JL_DA(8, 64)
   else {
@@ -252,6 +320,26 @@ extern "C" JL_API int jl_decode_attn(const void* q, const void* k_cache, const v
 #undef JL_DA
   JL_CUDA(e);
   return JL_OK;
+}
+
+extern "C" JL_API int jl_decode_attn(const void* q, const void* k_cache, const void* v_cache,
+                              const int* cache_len_ptr, const int* pad_left, void* scratch, void* out,
+                              int B, int nh, int nkv, int hd, int T, int n_new, float scale, int splits,
+                              int q_bstride, void* stream) {
+  return decode_attn(q, k_cache, v_cache, cache_len_ptr, pad_left, scratch, out, B, nh, nkv, hd, T, n_new, scale, splits, q_bstride, stream, nullptr);
+}
+
+// One new token per row from the fp32 projection y: rotation and (unit_norm) scaling of its heads, append at slot *cache_len_ptr (k_off >= 0), attention and
+// (g_off >= 0) a sigmoid gate per head; splits and scratch as in jl_decode_attn.  Rows of y and the heads in them start on 8-byte boundaries.
+extern "C" JL_API int jl_attn_step(const float* y, int ldy, int q_off, int k_off, int v_off, int g_off, const float* cos_t, const float* sin_t,
+                                   int max_pos, int rot, int unit_norm, float eps, void* k_cache, void* v_cache, const int* cache_len_ptr,
+                                   const int* pad_left, void* scratch, void* out, int B, int nh, int nkv, int hd, int T, float scale, int splits,
+                                   void* stream) {
+  JL_CHECK_ARG(ldy % 2 == 0 && q_off % 2 == 0 && (k_off < 0 || (k_off % 2 == 0 && v_off % 2 == 0)) && ((uintptr_t)y & 7) == 0,
+               "jl_attn_step: heads of y off their 8-byte boundary (pitch %d, columns %d %d %d)", ldy, q_off, k_off, v_off);
+  JL_CHECK_ARG(rot >= 0 && rot <= hd && rot % 2 == 0 && max_pos >= 1, "jl_attn_step: rot=%d of head_dim=%d, %d positions", rot, hd, max_pos);
+  const AttnStep step{y, ldy, q_off, k_off, v_off, g_off, cos_t, sin_t, rot, max_pos, unit_norm, eps};
+  return decode_attn(nullptr, k_cache, v_cache, cache_len_ptr, pad_left, scratch, out, B, nh, nkv, hd, T, 1, scale, splits, 0, stream, &step);
 }
 
 // ------------------------------------------------------------------------------------ allocation-free variant

@@ -101,6 +101,84 @@ __global__ void __launch_bounds__(GS_THREADS, 3) gla_scan_kernel(GlaParams p, co
 }
 
 
+// One token per row, with the head norm and the gate behind it (jl_gla_step): a CTA has a whole head, a thread DP key channels of one value column, so
+// that the read-outs meet in shared memory and leave normed, gated and in the operand type.  What bounds such a step is latency: the state (asked for into
+// L2 while the projection before still runs), the projection's row, the decays and the two sums.  One launch for the scan's and the norm's, us in a graph: 16 heads of 64 x
+// 128, 1 and 2 rows 6.6 -> 4.2, 8 rows 7.4 -> 4.2, 64 rows 28.1 -> 16.8; 8 heads of 128 x 128, 2 rows 7.0 -> 6.1, 64 rows 31.3 -> 15.5.
+struct GlaStep {
+  GlaParams p;
+  int g_off;                           // gate columns of y
+  float eps;
+  int gate_act;
+};
+
+template <typename T, int DP>
+__global__ void __launch_bounds__(1024) gla_step_kernel(const GlaStep a, const T* __restrict__ a2, const T* __restrict__ a2b, const T* __restrict__ norm,
+                                                        T* __restrict__ out) {
+  const GlaParams& p = a.p;
+  extern __shared__ float4 smem4[];
+  __shared__ float red[33];
+  const int cols = (p.Dv + 31) & ~31, P = blockDim.x / cols, D4 = P * DP;      // value columns in whole warps; channels in whole parts
+  float* qs = reinterpret_cast<float*>(smem4);                 // q | k | alpha [D4], then the partial read-outs [P][cols]
+  float* ks = qs + D4;
+  float* as = ks + D4;
+  float* part_o = as + D4;
+  const int tid = threadIdx.x, part = tid / cols, col = tid % cols, h = blockIdx.x, b = blockIdx.y;
+  float* sbase = p.state + ((size_t)b * p.H + h) * p.D * p.Dv;
+  for (int i = tid * 32; i < p.D * p.Dv; i += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(sbase + i));
+  pdl_wait();                      // nothing is read before the predecessor is done (the prefetch above returns nothing)
+  pdl_launch_dependents();
+  const bool real = (p.pad_left ? p.pad_left[b] : 0) <= (p.cache_len ? *p.cache_len : 0);
+  const float* yr = p.y + (size_t)b * p.ldy;
+  const bool on = col < p.Dv;
+  const int cc = min(col, p.Dv - 1), d0 = part * DP;
+  float st[DP];
+#pragma unroll
+  for (int r = 0; r < DP; ++r) st[r] = d0 + r < p.D ? sbase[(size_t)(d0 + r) * p.Dv + cc] : 0.0f;
+  const float v = yr[p.v_off + h * p.Dv + cc], gate = yr[a.g_off + h * p.Dv + cc], w = norm ? to_f(norm[cc]) : 1.0f;
+  for (int d = tid; d < D4; d += blockDim.x) {
+    float qv = 0.0f, kv = 0.0f, av = 1.0f;
+    if (d < p.D) {
+      const int n = h * p.D + d;
+      qv = yr[p.q_off + n] * p.q_scale;
+      kv = yr[p.k_off + n] * p.k_scale;
+      float z = to_f(a2b[n]);
+      for (int r = 0; r < p.R; r += 8) {                       // (all loads of a round first, the sum in order of r)
+        float wv[8], zv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int rr = min(r + u, p.R - 1);
+          wv[u] = to_f(a2[(size_t)n * p.R + rr]);
+          zv[u] = yr[p.a_off + rr];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) if (r + u < p.R) z = fmaf(wv[u], zv[u], z);
+      }
+      av = expf(log_sigmoid(z) * p.inv_tau);
+    }
+    qs[d] = qv; ks[d] = kv; as[d] = av;
+  }
+  __syncthreads();
+  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int r = 0; r < DP; ++r) {
+    st[r] = fmaf(as[d0 + r], st[r], ks[d0 + r] * v);
+    acc[r & 3] = fmaf(qs[d0 + r], st[r], acc[r & 3]);
+  }
+  part_o[part * cols + col] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+  if (real && on) {
+#pragma unroll
+    for (int r = 0; r < DP; ++r)
+      if (d0 + r < p.D) sbase[(size_t)(d0 + r) * p.Dv + col] = st[r];
+  }
+  __syncthreads();
+  float o = 0.0f;
+  if (part == 0 && on && real)                                 // (a padding token: a zero row, the state as it was)
+    for (int q = 0; q < P; ++q) o += part_o[q * cols + col];
+  const float r = 1.0f / sqrtf(block_sum(o * o, red) / (float)p.Dv + a.eps);
+  if (part == 0 && on) out[((size_t)b * p.H + h) * p.Dv + col] = from_f<T>(o * r * w * apply_act(gate, a.gate_act, 0.0f, 0.0f));
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // Prompts: the same recurrence in two launches.  gla_prep_kernel is token-parallel: it forms alpha (low-rank product,
 // bias, log-sigmoid, exponential — fp32), scales q, and writes q | k | alpha | v of every (token, head) as one
@@ -665,4 +743,29 @@ extern "C" JL_API int jl_mlstm_scan(const float* y, int ldy, int q_off, int k_of
   GlaParams p{y, ldy, q_off, k_off, v_off, 0, B, S, H, D, Dv + 1, 0, 1, q_scale, 1.0f, cache_len, pad_left, state, o};
   p.k_scale = 1.0f; p.aux = aux; p.ld_aux = ld_aux; p.ones = 1;
   return launch_scan(p, nullptr, nullptr, ws, DT_F32, stream);
+}
+
+// One token per row of the scan with projected decays, then the norm of every head's read-out (weight norm [Dv] or nullptr) and the gate
+// act(y[:, g_off + ...]): out [B, H * Dv] of dtype.  JL_ERR_UNSUPPORTED: sizes whose heads do not fit a CTA (the two launches take them).
+extern "C" JL_API int jl_gla_step(const float* y, int ldy, int q_off, int k_off, int v_off, int a_off, int g_off, const void* a2, const void* a2_bias,
+                                  const void* norm, float* state, void* out, const int* cache_len, const int* pad_left, int B, int H, int D, int Dv,
+                                  int R, float q_scale, float tau, float eps, int gate_act, int dtype, void* stream) {
+  JL_CHECK_ARG(B >= 1 && H >= 1 && D >= 1 && Dv >= 1 && R >= 1, "jl_gla_step: bad shape");
+  JL_CHECK_ARG(tau > 0.0f, "jl_gla_step: tau=%f must be positive", tau);
+  JL_CHECK_ARG(gate_act >= 0 && gate_act <= ACT_LAST, "jl_gla_step: bad activation %d", gate_act);
+  const int cols = (Dv + 31) & ~31;
+  // 16 channels a thread where that is at most 512 threads (more loads in flight than 32; above, 32 keep the CTA small)
+  const int dp = cols * ((D + 15) / 16) <= 512 ? 16 : 32, threads = cols * ((D + dp - 1) / dp);
+  if (threads > 1024 || B > 65535) return JL_ERR_UNSUPPORTED;
+  GlaStep s{GlaParams{y, ldy, q_off, k_off, v_off, a_off, B, 1, H, D, Dv, R, 1, q_scale, 1.0f / tau, cache_len, pad_left, state, nullptr}, g_off, eps, gate_act};
+  s.p.k_scale = 1.0f;
+  const size_t smem = (size_t)(3 * threads / cols * dp + threads) * sizeof(float);
+  if (dp == 16)
+    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((gla_step_kernel<T, 16>), dim3(H, B), dim3(threads), smem, (cudaStream_t)stream, s, (const T*)a2,
+                                           (const T*)a2_bias, (const T*)norm, (T*)out));
+  else
+    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((gla_step_kernel<T, 32>), dim3(H, B), dim3(threads), smem, (cudaStream_t)stream, s, (const T*)a2,
+                                           (const T*)a2_bias, (const T*)norm, (T*)out));
+  JL_CUDA(cudaGetLastError());
+  return JL_OK;
 }

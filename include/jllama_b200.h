@@ -290,6 +290,12 @@ int jl_linear_f32_pair(const void* x, int ldx, const void* w, void* out, int ldo
 /* The same on the SIMT kernels whatever the sizes (fp32 FMAs in order of k within a thread): what JLLAMA_HYBRID_TC=0 gives every call. */
 int jl_linear_exact(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int act, float p0, float p1,
                     int dtype, int out_f32, void* stream);
+/* One new token per row from the fp32 projection y (columns q_off, k_off, v_off, gate per head at g_off; k_off < 0: another layer has appended it, g_off < 0: no
+ * gate): rotation of the first rot channels of a head in pairs (2i, 2i + 1), scaling of q and k to unit RMS, append, attention and gate in one launch (and the
+ * merge, with splits > 1).  bfloat16 caches and result; sizes, splits and scratch as jl_decode_attn. */
+int jl_attn_step(const float* y, int ldy, int q_off, int k_off, int v_off, int g_off, const float* cos_t, const float* sin_t, int max_pos, int rot,
+                 int unit_norm, float eps, void* k_cache, void* v_cache, const int* cache_len_ptr, const int* pad_left, void* scratch, void* out,
+                 int B, int nh, int nkv, int hd, int T, float scale, int splits, void* stream);
 /* Rotary embedding (first `rot` channels, interleaved pairs), optional unit-RMS per head, cache append.  y fp32 [B*S, ldy] holds
  * q at q_off ([H*D]), k at k_off ([G*D]; < 0: queries only), v at v_off ([G*Dv]); caches [B][G][T_cap][D|Dv] of dtype. */
 int jl_attn_prep(const float* y, int ldy, int q_off, int k_off, int v_off, void* q_out, void* k_cache, void* v_cache,
@@ -312,6 +318,11 @@ int jl_head_gate(void* out, const float* gate, int ldg, int M, int H, int Dv, in
  * ws == NULL: one fused launch (decoding).  ws = jl_gla_scan_ws_floats(...) floats: token-parallel preparation into ws, then
  * a scan that streams it through a two-stage cp.async pipeline (prompts). */
 size_t jl_gla_scan_ws_floats(int B, int S, int H, int D, int Dv);
+/* One token per row (S = 1) with the head norm (weight norm [Dv] or NULL) and the gate act(y[:, g_off ..]) behind it: out [B, H * Dv] of dtype.
+ * JL_ERR_UNSUPPORTED where a head does not fit a CTA: jl_gla_scan and jl_headnorm_gate. */
+int jl_gla_step(const float* y, int ldy, int q_off, int k_off, int v_off, int a_off, int g_off, const void* a2, const void* a2_bias, const void* norm,
+                float* state, void* out, const int* cache_len, const int* pad_left, int B, int H, int D, int Dv, int R, float q_scale, float tau,
+                float eps, int gate_act, int dtype, void* stream);
 int jl_gla_scan(const float* y, int ldy, int q_off, int k_off, int v_off, int a_off, const void* a2, const void* a2_bias,
                 float* state, float* o, const int* cache_len, const int* pad_left, int B, int S, int H, int D, int Dv, int R,
                 float q_scale, float tau, float* ws, int dtype, void* stream);

@@ -265,6 +265,13 @@ class AttentionMixer(Mixer):
             ) -> torch.Tensor:
         s = self.spec
         y = SK.linear(h, self.w_in, resident=True)                                   # fp32 [M, q | k | v | gate]
+        if S == 1 and self.plain and self._library_shape() and _lib.has("jl_attn_step"):
+            # one launch instead of three while its CTAs (a key / value head's part of a row) are at most two to an SM; beyond, the preparation in each of them costs
+            # more than the launches (µs, three | one: 2 rows × 4 heads of 128, 100 keys 8.5 | 6.2, 2 × 8 in 16 parts, 4000 keys 19.3 | 14.5; 32 × 8 in 2 parts 38.8 | 39.0, 64 × 8
+            # with one query head each, 500 keys 37.9 | 45.8)
+            splits, _ = self._decode_plan(B, (cache.ks[s.kv_from if self.shares_kv else layer]).shape[2], y.device)
+            if B * s.kv_heads * splits <= 2 * K.num_sms(y.device):
+                return self._step(y, B, cache, layer, rope)
         q = torch.empty((B * S, s.heads * s.dim), dtype=self.dtype, device=h.device)
         src = layer if not self.shares_kv else s.kv_from
         kc, vc = cache.ks[src], cache.vs[src]
@@ -311,6 +318,29 @@ class AttentionMixer(Mixer):
             return out
         return SK.attn_generic(q, kc, vc, gate, cache.len_dev, cache.pad_left, B, S, s.heads, s.scale)
 
+    def _decode_plan(self, B: int, T: int, device: torch.device) -> Tuple[int, Optional[torch.Tensor]]:
+        """(splits, scratch) of the one-token attention over a cache of T slots."""
+        key = (B, T)
+        if key not in self._decode_plans:
+            s = self.spec
+            self._decode_plans[key] = K.decode_attn_plan(B, s.heads, s.kv_heads, s.dim, T, device)
+        return self._decode_plans[key]
+
+    def _step(self, y: torch.Tensor, B: int, cache: "object", layer: int, rope: Tuple[torch.Tensor, torch.Tensor]) -> torch.Tensor:
+        """One new token per row, from the projection to the gated heads, in one launch (plus the merge of split keys)."""
+        s = self.spec
+        src = s.kv_from if self.shares_kv else layer
+        kc, vc = cache.ks[src], cache.vs[src]
+        T = kc.shape[2]
+        splits, scratch = self._decode_plan(B, T, y.device)
+        out = torch.empty((B, s.heads * s.vdim), dtype=self.dtype, device=y.device)
+        _lib.check(_lib.lib().jl_attn_step(
+            y.data_ptr(), y.stride(0), self.q_off, self.k_off, self.v_off, self.g_off, rope[0].data_ptr(), rope[1].data_ptr(), rope[0].shape[0],
+            s.rot.dims if s.rot is not None else 0, int(s.qk_unit_norm), float(self.eps), kc.data_ptr(), vc.data_ptr(), cache.len_dev.data_ptr(),
+            cache.pad_left.data_ptr(), K._p(scratch), out.data_ptr(), B, s.heads, s.kv_heads, s.dim, T, float(s.scale), splits, K._stream()),
+            "jl_attn_step")
+        return out
+
     MAX_VALUE_ROW = 512            # widest value row the attention kernels take in one call
 
     def _attend_mixed(self, q: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, cache: "object", B: int, S: int
@@ -354,10 +384,7 @@ class AttentionMixer(Mixer):
                                           cache.pad_left.data_ptr(), out.data_ptr(), B, S, s.heads, s.kv_heads, s.dim, T,
                                           int(cache.index), float(s.scale), K._stream()), "jl_flash_prefill")
             return out
-        key = (B, T)
-        if key not in self._decode_plans:
-            self._decode_plans[key] = K.decode_attn_plan(B, s.heads, s.kv_heads, s.dim, T, q.device)
-        splits, scratch = self._decode_plans[key]
+        splits, scratch = self._decode_plan(B, T, q.device)
         _lib.check(L.jl_decode_attn(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), cache.len_dev.data_ptr(),
                                     cache.pad_left.data_ptr(), K._p(scratch), out.data_ptr(), B, s.heads, s.kv_heads, s.dim,
                                     T, 1, float(s.scale), splits, 0, K._stream()), "jl_decode_attn")
@@ -395,6 +422,9 @@ class GlaMixer(Mixer):
             ) -> torch.Tensor:
         s = self.spec
         y = SK.linear(h, self.w_in, resident=True)                                   # fp32 [M, q | k | v | gate | low-rank decay input]
+        if S == 1 and SK.gla_step_takes(s.dim, s.vdim):
+            return SK.gla_step(y, self.q_off, self.k_off, self.v_off, self.a_off, self.g_off, self.a2, self.a2_bias, self.norm, cache.states[layer],
+                               cache.len_dev, cache.pad_left, B, s.heads, s.dim, s.vdim, s.dim ** -0.5, s.tau, self.eps, SK.ACT_SILU)
         o = SK.gla_scan(y, self.q_off, self.k_off, self.v_off, self.a_off, self.a2, self.a2_bias, cache.states[layer],
                         cache.len_dev, cache.pad_left, B, S, s.heads, s.dim, s.vdim, s.dim ** -0.5, s.tau)
         gate = y[:, self.g_off:self.g_off + s.heads * s.vdim]

@@ -66,11 +66,13 @@ _HYBRID = {
     "jl_linear_exact": (i32, [vp, i32, vp, vp, i32, i32, i32, i32, i32, f32, f32, i32, i32, vp]),
     "jl_linear_f32_pair_ws": (i64, [vp, i32, vp, i32, i32, i32, i32]),
     "jl_linear_f32_pair": (i32, [vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, vp]),
+    "jl_attn_step": (i32, [fp] + [i32] * 5 + [fp, fp, i32, i32, i32, f32, vp, vp, ip, ip, vp, vp] + [i32] * 5 + [f32, i32, vp]),
     "jl_attn_prep": (i32, [fp, i32, i32, i32, i32, vp, vp, vp, fp, fp, i32, i32, i32, f32, ip, ip] + [i32] * 7 + [fp, i32, i32, i32, vp]),
     "jl_attn_generic": (i32, [vp, vp, vp, vp, fp, i32, ip, ip] + [i32] * 7 + [f32, fp, i32, i32, vp]),
     "jl_attn_generic_splits": (i32, [i32, i32, i32, i32]),
     "jl_head_gate": (i32, [vp, fp, i32, i32, i32, i32, i32, vp]),
     "jl_gla_scan": (i32, [fp, i32, i32, i32, i32, i32, vp, vp, fp, fp, ip, ip] + [i32] * 6 + [f32, f32, fp, i32, vp]),
+    "jl_gla_step": (i32, [fp] + [i32] * 6 + [vp, vp, vp, fp, vp, ip, ip] + [i32] * 5 + [f32, f32, f32, i32, i32, vp]),
     "jl_gla_scan_ws_floats": (sz, [i32, i32, i32, i32, i32]),
     "jl_retention_scan": (i32, [fp, i32, i32, i32, i32, fp, fp, fp, i32, i32, i32, f32, f32, fp, fp, ip, ip] + [i32] * 5 + [fp, vp]),
     "jl_branch_add_norm": (i32, [fp, i32, fp, i32, f32, fp, vp, vp, vp, vp, i32, i32, f32, i32, vp]),

@@ -240,6 +240,26 @@ def gla_scan(y: torch.Tensor, q_off: int, k_off: int, v_off: int, a_off: int, a2
     return out
 
 
+def gla_step_takes(D: int, Dv: int) -> bool:
+    """Whether a head's step fits one CTA (csrc/gla_scan.cu jl_gla_step)."""
+    cols = (Dv + 31) // 32 * 32
+    return cols * ((D + 31) // 32) <= 1024
+
+
+def gla_step(y: torch.Tensor, q_off: int, k_off: int, v_off: int, a_off: int, g_off: int, a2: torch.Tensor, a2_bias: torch.Tensor,
+             norm: Optional[torch.Tensor], state: torch.Tensor, cache_len: Optional[torch.Tensor], pad_left: Optional[torch.Tensor], B: int,
+             H: int, D: int, Dv: int, q_scale: float, tau: float, eps: float, gate_act: int) -> torch.Tensor:
+    """One token per row: gla_scan, headnorm_gate of its read-outs with the gate columns of y, in one launch; [B, H·Dv] of a2's type."""
+    _need(y, torch.float32, "y")
+    _need(state, torch.float32, "state")
+    out = torch.empty((B, H * Dv), dtype=a2.dtype, device=y.device)
+    _lib.check(_lib.lib().jl_gla_step(
+        y.data_ptr(), y.stride(0), q_off, k_off, v_off, a_off, g_off, a2.data_ptr(), a2_bias.data_ptr(), _p(norm), state.data_ptr(),
+        out.data_ptr(), _p(cache_len), _p(pad_left), B, H, D, Dv, a2.shape[1], float(q_scale), float(tau), float(eps), gate_act,
+        dtype_code(a2.dtype), _stream()), "jl_gla_step")
+    return out
+
+
 # --------------------------------------------------------------------------- parallel blocks, latent attention, retention, experts
 ROT_INTERLEAVED, ROT_HALF = 0, 1        # channel 2i with 2i+1 / channel i with i + dims/2
 ROT_LAYOUTS = {"interleaved": ROT_INTERLEAVED, "half": ROT_HALF}

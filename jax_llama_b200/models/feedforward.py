@@ -102,10 +102,11 @@ class DenseFeedForward:
         return self.weights()
 
     def run(self, h: torch.Tensor) -> torch.Tensor:
-        if self.spec.gated:
-            t = _gated_layer(h, self.up, self.u_off, self.spec.ff, self.spec.act, 0.0)
-        else:
-            t = SK.linear(h, self.up, act=self.act, p0=self.p0, p1=self.p1, out_f32=False, resident=True)
+        with SK.Scratch():
+            if self.spec.gated:
+                t = _gated_layer(h, self.up, self.u_off, self.spec.ff, self.spec.act, 0.0)
+            else:
+                t = SK.linear(h, self.up, act=self.act, p0=self.p0, p1=self.p1, out_f32=False, resident=True)
         return SK.linear(t, self.down, resident=True)
 
 
@@ -178,10 +179,16 @@ class MoeFeedForward:
         return [self.up[:n], self.down[:n]] + [t for t in (self.w_route, self.shared_up, self.shared_down) if t is not None]
 
     def run(self, h: torch.Tensor) -> torch.Tensor:
+        with SK.Scratch():
+            parts = self._parts(h)
+        return SK.moe_combine(*parts[0], **parts[1])
+
+    def _parts(self, h: torch.Tensor) -> Tuple[tuple, dict]:
+        """Everything ahead of the weighted sum: its arguments."""
         s = self.spec
         M, W = h.shape
         z = SK.linear(h, self.w_route, resident=True)                                             # fp32 [M, router logits | gate logit]
-        ident_w = torch.empty(M, dtype=torch.float32, device=h.device) if s.identity else None
+        ident_w = SK.empty(M, dtype=torch.float32, device=h.device) if s.identity else None
         idx, wt = SK.moe_route(z, self.n_route, s.top, s.groups, s.keep, s.group_top, self.score, s.normalise, s.scale,
                                bias=self.router_bias, choice_bias=self.choice_bias, n_real=s.experts, ident_w=ident_w)
         n_up = self.up.shape[1]                                                    # ff, or gate | up rows of a gated expert
@@ -189,14 +196,14 @@ class MoeFeedForward:
             n = M * s.top
             flat = idx.view(-1)
             if s.gated:
-                gu = torch.empty((n, n_up), dtype=torch.float32, device=h.device)
+                gu = SK.empty((n, n_up), dtype=torch.float32, device=h.device)
                 SK.linear_batched(h, self.up, gu, nbatch=n, rows=1, x_bs=h.stride(0), o_bs=n_up, x_div=s.top, w_index=flat)
                 t = _gated_act(gu, self.u_off, s.ff, s.act, s.limit, h.dtype)
             else:
-                t = torch.empty((n, s.ff), dtype=h.dtype, device=h.device)
+                t = SK.empty((n, s.ff), dtype=h.dtype, device=h.device)
                 SK.linear_batched(h, self.up, t, nbatch=n, rows=1, x_bs=h.stride(0), o_bs=s.ff, x_div=s.top, w_index=flat,
                                   act=self.act)
-            y = torch.empty((n, W), dtype=torch.float32, device=h.device)
+            y = SK.empty((n, W), dtype=torch.float32, device=h.device)
             SK.linear_batched(t, self.down, y, nbatch=n, rows=1, x_bs=s.ff, o_bs=W, w_index=flat)
             pos = None
         elif SK.tensor_cores_enabled() and h.dtype == torch.bfloat16 and W % 8 == 0 and s.ff % 8 == 0 and h.is_contiguous():
@@ -212,13 +219,13 @@ class MoeFeedForward:
             pos, row_src, tile_group, _ = SK.moe_sort(idx, s.experts)
             rows = row_src.shape[0]
             if s.gated:
-                gu = torch.empty((rows, n_up), dtype=torch.float32, device=h.device)
+                gu = SK.empty((rows, n_up), dtype=torch.float32, device=h.device)
                 SK.linear_sorted(h, self.up, gu, tile_group, row_src)
                 t = _gated_act(gu, self.u_off, s.ff, s.act, s.limit, h.dtype)
             else:
-                t = torch.empty((rows, s.ff), dtype=h.dtype, device=h.device)
+                t = SK.empty((rows, s.ff), dtype=h.dtype, device=h.device)
                 SK.linear_sorted(h, self.up, t, tile_group, row_src, act=self.act)
-            y = torch.empty((rows, W), dtype=torch.float32, device=h.device)
+            y = SK.empty((rows, W), dtype=torch.float32, device=h.device)
             SK.linear_sorted(t, self.down, y, tile_group, None)
         shared: Optional[torch.Tensor] = None
         gate = None
@@ -231,8 +238,8 @@ class MoeFeedForward:
             if self.gate_off >= 0:
                 gate = z[:, self.gate_off:self.gate_off + 1]
         if s.identity:                                     # pairs that chose an identity expert ran nothing: weight · input instead
-            return SK.moe_combine(y, pos, wt, shared, gate, W, idx=idx, ident_w=ident_w, x=h)
-        return SK.moe_combine(y, pos, wt, shared, gate, W)
+            return (y, pos, wt, shared, gate, W), dict(idx=idx, ident_w=ident_w, x=h)
+        return (y, pos, wt, shared, gate, W), {}
 
 
 FEED_FORWARDS = {"dense": DenseFeedForward, "moe": MoeFeedForward}

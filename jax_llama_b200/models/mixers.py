@@ -94,7 +94,9 @@ class Mixer:
         return p.y1 if p.bias is None and p.y2 is None and p.c1 == 1.0 else SK.weighted_sum2(*p)
 
     def parts(self, h: torch.Tensor, B: int, S: int, cache: "object", layer: int, rope: Optional[Tuple] = None) -> MixerParts:
-        return MixerParts(SK.linear(self.run(h, B, S, cache, layer, rope), self.wo, resident=True), bias=self.out_bias)
+        with SK.Scratch():
+            y = self.run(h, B, S, cache, layer, rope)
+        return MixerParts(SK.linear(y, self.wo, resident=True), bias=self.out_bias)
 
     out_bias: Optional[torch.Tensor] = None        # bias of the output projection
 
@@ -272,7 +274,7 @@ class AttentionMixer(Mixer):
             splits, _ = self._decode_plan(B, (cache.ks[s.kv_from if self.shares_kv else layer]).shape[2], y.device)
             if B * s.kv_heads * splits <= 2 * K.num_sms(y.device):
                 return self._step(y, B, cache, layer, rope)
-        q = torch.empty((B * S, s.heads * s.dim), dtype=self.dtype, device=h.device)
+        q = SK.empty((B * S, s.heads * s.dim), dtype=self.dtype, device=h.device)
         src = layer if not self.shares_kv else s.kv_from
         kc, vc = cache.ks[src], cache.vs[src]
         rot = s.rot.dims if s.rot is not None else 0
@@ -294,7 +296,7 @@ class AttentionMixer(Mixer):
             if S > 1 and self._flash_masked_shape():
                 # prompts of 128-wide heads in bfloat16: the tcgen05 kernel with the block bound, the window, the cap, the sink, the
                 # gate and the turn back in its softmax and epilogue; 64-wide heads: the warp-level kernel
-                out = torch.empty((B * S, s.heads * s.vdim), dtype=self.dtype, device=q.device)
+                out = SK.empty((B * S, s.heads * s.vdim), dtype=self.dtype, device=q.device)
                 _lib.check(_lib.lib().jl_flash_prefill_masked(
                     q.data_ptr(), kc.data_ptr(), vc.data_ptr(), cache.pad_left.data_ptr(), out.data_ptr(), B, S, s.heads,
                     s.kv_heads, s.dim, kc.shape[2], int(cache.index), float(s.scale), int(s.chunk), int(s.sink),
@@ -333,7 +335,7 @@ class AttentionMixer(Mixer):
         kc, vc = cache.ks[src], cache.vs[src]
         T = kc.shape[2]
         splits, scratch = self._decode_plan(B, T, y.device)
-        out = torch.empty((B, s.heads * s.vdim), dtype=self.dtype, device=y.device)
+        out = SK.empty((B, s.heads * s.vdim), dtype=self.dtype, device=y.device)
         _lib.check(_lib.lib().jl_attn_step(
             y.data_ptr(), y.stride(0), self.q_off, self.k_off, self.v_off, self.g_off, rope[0].data_ptr(), rope[1].data_ptr(), rope[0].shape[0],
             s.rot.dims if s.rot is not None else 0, int(s.qk_unit_norm), float(self.eps), kc.data_ptr(), vc.data_ptr(), cache.len_dev.data_ptr(),
@@ -349,7 +351,7 @@ class AttentionMixer(Mixer):
         taken `MAX_VALUE_ROW // vdim` at a time."""
         s = self.spec
         M, H, G, T = B * S, s.heads, s.kv_heads, kc.shape[2]
-        out = torch.empty((M, H * s.vdim), dtype=self.dtype, device=q.device)
+        out = SK.empty((M, H * s.vdim), dtype=self.dtype, device=q.device)
         per = max(1, min(G, self.MAX_VALUE_ROW // s.vdim))
         row = G * s.vdim
         for c0 in range(0, G, per):
@@ -377,7 +379,7 @@ class AttentionMixer(Mixer):
                                ) -> torch.Tensor:
         s = self.spec
         L = _lib.lib()
-        out = torch.empty((B * S, s.heads * s.vdim), dtype=self.dtype, device=q.device)
+        out = SK.empty((B * S, s.heads * s.vdim), dtype=self.dtype, device=q.device)
         T = kc.shape[2]
         if S > 1:
             _lib.check(L.jl_flash_prefill(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), cache.len_dev.data_ptr(),
@@ -527,14 +529,14 @@ class LatentAttentionMixer(Mixer):
         q = SK.linear(cq, self.uq, out_f32=False, resident=True) if s.q_rank else cq          # [M, H·(rot_dim + dim)]
         if starts:
             return self._attend_projected(q, c_new, kr_new, cache, B, S, rot, layout, rope, gate)
-        qa = torch.empty((M, H * self.row), dtype=self.dtype, device=h.device)
+        qa = SK.empty((M, H * self.row), dtype=self.dtype, device=h.device)
         a = q[:, s.rot_dim:] if s.rot_dim else q                               # head h's unrotated part starts at h·qd
         SK.linear_batched(a, self.uk_t, qa, nbatch=H, rows=M, x_bs=qd, o_bs=self.row)      # U_hᵀ a_h
         if s.rot_dim:
             SK.rotary_slice(q, qd, 0, qa, self.row, s.kv_rank, H, s.rot_dim, rot, layout, rope[0], rope[1],
                             cache.len_dev, cache.pad_left, B, S)
         ctx = self._attend(qa, kc, kc, cache, B, S, H, 1, self.row, s.kv_rank, kc.shape[1], self.row, self.row, gate)     # [M, H·kv_rank]
-        out = torch.empty((M, H * s.vdim), dtype=self.dtype, device=h.device)
+        out = SK.empty((M, H * s.vdim), dtype=self.dtype, device=h.device)
         SK.linear_batched(ctx, self.uv, out, nbatch=H, rows=M, x_bs=s.kv_rank, o_bs=s.vdim)
         return out
 

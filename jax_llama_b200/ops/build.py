@@ -154,6 +154,42 @@ def build_library(force: bool = False, verbose: bool = False, subset: Optional[s
     return lib
 
 
+def binding_path() -> Path:
+    """Where the built-in Python form of the hot entry points lies (csrc/binding.cc)."""
+    import sysconfig
+    return OUT_DIR / f"_jl_binding{sysconfig.get_config_var('EXT_SUFFIX') or '.so'}"
+
+
+def build_binding(force: bool = False) -> Optional[Path]:
+    """Compile csrc/binding.cc for this interpreter; None where its headers or a C++ compiler are missing (the entry points are then called
+    through ctypes, with the same results)."""
+    import sysconfig
+    out, src = binding_path(), CSRC / "binding.cc"
+    include = Path(sysconfig.get_paths()["include"])
+    h = hashlib.sha256()
+    for f in (src, INCLUDE / "jllama_b200.h"):
+        h.update(f.read_bytes())
+    h.update(sys.version.encode())
+    stamp = out.with_suffix(".stamp")
+    if not force and out.exists() and stamp.exists() and stamp.read_text().strip() == h.hexdigest():
+        return out
+    if not (include / "Python.h").exists():
+        return None
+    OUT_DIR.mkdir(parents=True, exist_ok=True)
+    tmp = out.with_suffix(f".tmp{os.getpid()}.so")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-I{include}", f"-I{INCLUDE}", str(src), "-o", str(tmp)]
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+    except OSError as e:
+        logger.warning("no C++ compiler for %s: %s", src.name, e)
+        return None
+    if r.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed for {src.name}:\n{r.stderr}")
+    os.replace(tmp, out)
+    stamp.write_text(h.hexdigest() + "\n")
+    return out
+
+
 if __name__ == "__main__":
     logging.basicConfig(level=logging.INFO)
     names = [a.split("=", 1)[1] for a in sys.argv[1:] if a.startswith("--subset=")]

@@ -15,6 +15,7 @@ import torch
 
 from . import _lib
 from .kernels import _p, _stream, ensure_gemm_workspace, num_sms
+from .scratch import Scratch, empty  # noqa: F401  (Scratch: for the layers)
 
 ACT_NONE, ACT_RELU2, ACT_GELU_TANH, ACT_SILU, ACT_SCALE_SOFTCAP, ACT_SIGMOID, ACT_XIELU, ACT_RELU = 0, 1, 2, 3, 4, 5, 6, 7
 DELTA_FUSED_MAX_TOKENS = 8    # the same for the delta-rule scan (csrc/delta_scan.cu DS_FUSED_MAX_TOKENS)
@@ -49,7 +50,7 @@ def embed_f32(ids: torch.Tensor, table: torch.Tensor, out: Optional[torch.Tensor
     ids32 = ids.to(torch.int32).contiguous().view(-1)
     V, W = table.shape
     if out is None:
-        out = torch.empty((ids32.numel(), W), dtype=torch.float32, device=table.device)
+        out = empty((ids32.numel(), W), dtype=torch.float32, device=table.device)
     _lib.check(_lib.lib().jl_embed_f32(ids32.data_ptr(), table.data_ptr(), out.data_ptr(), ids32.numel(), W, V, float(scale),
                                        dtype_code(table.dtype), _stream()), "jl_embed_f32")
     return out
@@ -61,7 +62,7 @@ def norm_f32(x: torch.Tensor, w: torch.Tensor, eps: float, offset: float, out: O
     _need(x, torch.float32, "x")
     M, W = x.shape
     if out is None:
-        out = torch.empty((M, W), dtype=w.dtype, device=x.device)
+        out = empty((M, W), dtype=w.dtype, device=x.device)
     _lib.check(_lib.lib().jl_norm_f32(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, W, float(eps), float(offset),
                                       dtype_code(w.dtype), _stream()), "jl_norm_f32")
     return out
@@ -74,7 +75,7 @@ def postnorm_add(y: torch.Tensor, w_post: torch.Tensor, x: torch.Tensor, eps: fl
     _need(x, torch.float32, "x")
     M, W = x.shape
     if w_next is not None and h_out is None:
-        h_out = torch.empty((M, W), dtype=w_next.dtype, device=x.device)
+        h_out = empty((M, W), dtype=w_next.dtype, device=x.device)
     _lib.check(_lib.lib().jl_postnorm_add(y.data_ptr(), y.stride(0), w_post.data_ptr(), x.data_ptr(), _p(w_next),
                                           _p(h_out) if w_next is not None else 0, M, W, float(eps), float(offset),
                                           dtype_code(w_post.dtype), _stream()), "jl_postnorm_add")
@@ -91,7 +92,7 @@ def headnorm_gate(o: torch.Tensor, w: Optional[torch.Tensor], gate: torch.Tensor
     M = o.shape[0]
     odt = w.dtype if w is not None else dtype
     if out is None:
-        out = torch.empty((M, H * V), dtype=odt, device=o.device)
+        out = empty((M, H * V), dtype=odt, device=o.device)
     _lib.check(_lib.lib().jl_headnorm_gate(o.data_ptr(), _p(w), gate.data_ptr(), gate.stride(0), out.data_ptr(),
                                            M, H, V, float(eps), gate_act, dtype_code(odt), _stream()),
                "jl_headnorm_gate")
@@ -104,7 +105,7 @@ def act_cast(y: torch.Tensor, out_dtype: torch.dtype, act: int = ACT_NONE, p0: f
     _need(y, torch.float32, "y")
     M, N = y.shape
     if out is None:
-        out = torch.empty((M, N), dtype=out_dtype, device=y.device)
+        out = empty((M, N), dtype=out_dtype, device=y.device)
     _lib.check(_lib.lib().jl_act_cast(y.data_ptr(), y.stride(0), out.data_ptr(), out.stride(0), M, N, act, float(p0),
                                       float(p1), dtype_code(out_dtype), _stream()), "jl_act_cast")
     return out
@@ -126,10 +127,11 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
     _need(w, x.dtype, "w")
     N, K = w.shape
     M = x.numel() // K
-    x = x.view(M, K) if x.is_contiguous() else x
+    if (x.dim() != 2 or x.shape[1] != K) and x.is_contiguous():
+        x = x.view(M, K)
     odt = torch.float32 if out_f32 else x.dtype
     if out is None:
-        out = x.new_empty((M, N), dtype=odt)
+        out = empty((M, N), dtype=odt, device=x.device)
     L = _lib.lib()
     use_tc = tensor_cores_enabled() if tensor_cores is None else tensor_cores
     if (use_tc and x.dtype == torch.bfloat16 and M > 8 and K % 8 == 0 and N % 8 == 0 and x.is_contiguous()
@@ -147,7 +149,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
     if use_tc and x.dtype == torch.float32 and out.dtype == torch.float32 and M > 64:
         need = L.jl_linear_f32_pair_ws(x.data_ptr(), x.stride(0), w.data_ptr(), M, N, K, num_sms(x.device))
         if need >= 0:
-            ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
+            ws = empty(need, dtype=torch.uint8, device=x.device) if need else None
             _lib.check(L.jl_linear_f32_pair(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), M, N, K, num_sms(x.device),
                                             _p(ws), _stream()), "jl_linear_f32_pair")
             if act != ACT_NONE:
@@ -199,13 +201,13 @@ def attn_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     G, T_cap, D = k_cache.shape[1], k_cache.shape[2], k_cache.shape[3]
     Dv = v_cache.shape[3]
     if out is None:
-        out = torch.empty((B * S, H * Dv), dtype=q.dtype, device=q.device)
+        out = empty((B * S, H * Dv), dtype=q.dtype, device=q.device)
     L = _lib.lib()
     splits, scratch = 0, None
     if S == 1:                     # one new token: keys split over CTAs, partial results meet in scratch
         splits = int(L.jl_attn_generic_splits(B, H, G, T_cap))
         if splits:
-            scratch = torch.empty(B * H * splits * (Dv + 2), dtype=torch.float32, device=q.device)
+            scratch = empty(B * H * splits * (Dv + 2), dtype=torch.float32, device=q.device)
     _lib.check(L.jl_attn_generic(
         q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), _p(gate),
         gate.stride(0) if gate is not None else 0, _p(cache_len), _p(pad_left), B, S, H, G, D, Dv, T_cap, float(scale),
@@ -228,11 +230,11 @@ def gla_scan(y: torch.Tensor, q_off: int, k_off: int, v_off: int, a_off: int, a2
     _need(state, torch.float32, "state")
     R = a2.shape[1]
     if out is None:
-        out = torch.empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
+        out = empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
     L = _lib.lib()
     ws = None
     if S > GLA_FUSED_MAX_TOKENS:          # prompts: token-parallel preparation + pipelined scan (two launches)
-        ws = torch.empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
+        ws = empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
     _lib.check(L.jl_gla_scan(
         y.data_ptr(), y.stride(0), q_off, k_off, v_off, a_off, a2.data_ptr(), a2_bias.data_ptr(), state.data_ptr(),
         out.data_ptr(), _p(cache_len), _p(pad_left), B, S, H, D, Dv, R, float(q_scale), float(tau), _p(ws),
@@ -252,7 +254,7 @@ def gla_step(y: torch.Tensor, q_off: int, k_off: int, v_off: int, a_off: int, g_
     """One token per row: gla_scan, headnorm_gate of its read-outs with the gate columns of y, in one launch; [B, H·Dv] of a2's type."""
     _need(y, torch.float32, "y")
     _need(state, torch.float32, "state")
-    out = torch.empty((B, H * Dv), dtype=a2.dtype, device=y.device)
+    out = empty((B, H * Dv), dtype=a2.dtype, device=y.device)
     _lib.check(_lib.lib().jl_gla_step(
         y.data_ptr(), y.stride(0), q_off, k_off, v_off, a_off, g_off, a2.data_ptr(), a2_bias.data_ptr(), _p(norm), state.data_ptr(),
         out.data_ptr(), _p(cache_len), _p(pad_left), B, H, D, Dv, a2.shape[1], float(q_scale), float(tau), float(eps), gate_act,
@@ -278,8 +280,8 @@ def branch_add_norm(x: torch.Tensor, y1: Optional[torch.Tensor], y2: Optional[to
     for y in (y1, y2):
         if y is not None:
             _need(y, torch.float32, "y")
-    h1 = torch.empty((M, W), dtype=w1.dtype, device=x.device) if w1 is not None else None
-    h2 = torch.empty((M, W), dtype=w2.dtype, device=x.device) if w2 is not None else None
+    h1 = empty((M, W), dtype=w1.dtype, device=x.device) if w1 is not None else None
+    h2 = empty((M, W), dtype=w2.dtype, device=x.device) if w2 is not None else None
     if y1 is None and y2 is None and w1 is None and w2 is None:
         return None, None
     dt = w1.dtype if w1 is not None else (w2.dtype if w2 is not None else torch.float32)
@@ -325,9 +327,9 @@ def latent_prep(y: torch.Tensor, q_off: int, q_rank: int, kv_off: int, kv_rank: 
     not a latent but the queries themselves, brought into the operand type as they are."""
     _need(y, torch.float32, "y")
     M = B * S
-    cq = torch.empty((M, q_rank), dtype=cache.dtype, device=y.device) if q_rank else None
-    c_out = torch.empty((M, kv_rank), dtype=cache.dtype, device=y.device) if token_major else None
-    kr_out = torch.empty((M, max(rot_dim, 1)), dtype=cache.dtype, device=y.device) if token_major else None
+    cq = empty((M, q_rank), dtype=cache.dtype, device=y.device) if q_rank else None
+    c_out = empty((M, kv_rank), dtype=cache.dtype, device=y.device) if token_major else None
+    kr_out = empty((M, max(rot_dim, 1)), dtype=cache.dtype, device=y.device) if token_major else None
     _lib.check(_lib.lib().jl_latent_prep(
         y.data_ptr(), y.stride(0), q_off, q_rank, kv_off, kv_rank, rot_dim, rot, layout, _p(wq_norm), wkv_norm.data_ptr(),
         _p(cq), cache.data_ptr(), cos.data_ptr(), sin.data_ptr(), cos.shape[0], float(eps), _p(cache_len), _p(pad_left), B, S,
@@ -352,7 +354,7 @@ def latent_heads(q: torch.Tensor, kr: torch.Tensor, kv: torch.Tensor, H: int, ro
     same layout: per head [kr [B·S, rot_dim], shared by the heads | its `dim` columns of kv [B·S, ≥ H·dim]]."""
     _need(kr, q.dtype, "kr")
     _need(kv, q.dtype, "kv")
-    kf = torch.empty((B * S, H * (rot_dim + dim)), dtype=q.dtype, device=q.device)
+    kf = empty((B * S, H * (rot_dim + dim)), dtype=q.dtype, device=q.device)
     _lib.check(_lib.lib().jl_latent_heads(
         q.data_ptr(), q.stride(0), kr.data_ptr(), kr.stride(0), kv.data_ptr(), kv.stride(0), kf.data_ptr(), kf.stride(0), H, rot_dim, dim, rot,
         layout, cos.data_ptr(), sin.data_ptr(), cos.shape[0], _p(cache_len), _p(pad_left), B, S, dtype_code(q.dtype), _stream()),
@@ -371,14 +373,14 @@ def attn_windowed(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
     token-major projections [B·T, G, d] have (T·G·d, d) and a row pitch of G·d.  sink: one more term exp(0) in the softmax
     denominator (a key with score 0 and no value); out_f32: the result in fp32 whatever the operand type."""
     if out is None:
-        out = torch.empty((B * S, H * Dv), dtype=torch.float32 if out_f32 else q.dtype, device=q.device)
+        out = empty((B * S, H * Dv), dtype=torch.float32 if out_f32 else q.dtype, device=q.device)
     f32_out = out.dtype == torch.float32 and q.dtype != torch.float32
     L = _lib.lib()
     splits, scratch = 0, None
     if S == 1:
         splits = int(L.jl_attn_generic_splits(B, H, G, min(T_cap, window) if window > 0 else T_cap))
         if splits:
-            scratch = torch.empty(B * H * splits * (Dv + 2), dtype=torch.float32, device=q.device)
+            scratch = empty(B * H * splits * (Dv + 2), dtype=torch.float32, device=q.device)
     _lib.check(L.jl_attn_windowed(
         q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), 0 if f32_out else out.data_ptr(), _p(cache_len), _p(pad_left),
         B, S, H, G, D, Dv, T_cap, ldk, ldv, *(int(v) for v in strides), int(window), float(scale), _p(scratch), splits,
@@ -402,7 +404,7 @@ def attn_masked(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, c
     if gate_cols and gate.shape[1] != H * Dv:
         raise ValueError(f"gate of {gate.shape[1]} columns for {H} heads of {Dv}")
     if out is None:
-        out = torch.empty((B * S, H * Dv), dtype=q.dtype, device=q.device)
+        out = empty((B * S, H * Dv), dtype=q.dtype, device=q.device)
     if sink_logit is not None:
         _need(sink_logit, torch.float32, "sink_logit")
     L = _lib.lib()
@@ -411,7 +413,7 @@ def attn_masked(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, c
         reach = min([T_cap] + [int(v) for v in (window, chunk) if v > 0])
         splits = int(L.jl_attn_generic_splits(B, H, G, reach))
         if splits:
-            scratch = torch.empty(B * H * splits * (Dv + 2), dtype=torch.float32, device=q.device)
+            scratch = empty(B * H * splits * (Dv + 2), dtype=torch.float32, device=q.device)
     _lib.check(L.jl_attn_masked(
         q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), _p(gate), gate.stride(0) if gate is not None else 0,
         int(gate_cols), _p(cache_len), _p(pad_left), B, S, H, G, D, Dv, T_cap, ldk, ldv, *(int(v) for v in strides), int(window), int(chunk), float(scale), float(softcap), _p(scratch),
@@ -430,11 +432,11 @@ def retention_scan(y: torch.Tensor, q_off: int, k_off: int, v_off: int, head_dec
     _need(state, torch.float32, "state")
     _need(head_decay, torch.float32, "head_decay")
     if out is None:
-        out = torch.empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
+        out = empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
     L = _lib.lib()
     ws = None
     if S > GLA_FUSED_MAX_TOKENS:
-        ws = torch.empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
+        ws = empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
     _lib.check(L.jl_retention_scan(
         y.data_ptr(), y.stride(0), q_off, k_off, v_off, head_decay.data_ptr(), cos.data_ptr(), sin.data_ptr(), cos.shape[0],
         rot, layout, 1.0, float(k_scale), state.data_ptr(), out.data_ptr(), _p(cache_len), _p(pad_left), B, S, H, D, Dv,
@@ -450,8 +452,8 @@ def moe_route(z: torch.Tensor, E: int, top: int, groups: int, keep: int, group_t
     n_real on are identity experts; a chosen one is reported as expert -1 and its weight is added to ident_w fp32 [M]."""
     _need(z, torch.float32, "z")
     M = z.shape[0]
-    idx = torch.empty((M, top), dtype=torch.int32, device=z.device)
-    wt = torch.empty((M, top), dtype=torch.float32, device=z.device)
+    idx = empty((M, top), dtype=torch.int32, device=z.device)
+    wt = empty((M, top), dtype=torch.float32, device=z.device)
     if choice_bias is not None or (n_real is not None and n_real != E):
         _lib.check(_lib.lib().jl_moe_route_ex(z.data_ptr(), z.stride(0), M, E, top, groups, keep, group_top, score, int(normalise),
                                               float(scale), _p(bias), _p(choice_bias), E if n_real is None else int(n_real),
@@ -471,10 +473,10 @@ def moe_sort(idx: torch.Tensor, E: int, tile: Optional[int] = None
     M, top = idx.shape
     tile = int(L.jl_linear_tile_rows()) if tile is None else int(tile)
     cap = int(L.jl_moe_sorted_rows(M * top, E, tile))
-    pos = torch.empty(M * top, dtype=torch.int32, device=idx.device)
-    row_src = torch.empty(cap, dtype=torch.int32, device=idx.device)
-    tile_group = torch.empty(cap // tile, dtype=torch.int32, device=idx.device)
-    used = torch.empty(1, dtype=torch.int32, device=idx.device)
+    pos = empty(M * top, dtype=torch.int32, device=idx.device)
+    row_src = empty(cap, dtype=torch.int32, device=idx.device)
+    tile_group = empty(cap // tile, dtype=torch.int32, device=idx.device)
+    used = empty(1, dtype=torch.int32, device=idx.device)
     _lib.check(L.jl_moe_sort(idx.data_ptr(), M, top, E, tile, cap, pos.data_ptr(), row_src.data_ptr(), tile_group.data_ptr(),
                              used.data_ptr(), _stream()), "jl_moe_sort")
     return pos, row_src, tile_group, used
@@ -486,7 +488,7 @@ GEMM_TILE_ROWS = 128                    # row tile of the tcgen05 GEMM: the segm
 def moe_gather(x: torch.Tensor, row_src: torch.Tensor) -> torch.Tensor:
     """xs[p] = x[row_src[p]] (zeros where row_src[p] < 0)."""
     W = x.shape[1]
-    xs = torch.empty((row_src.shape[0], W), dtype=x.dtype, device=x.device)
+    xs = empty((row_src.shape[0], W), dtype=x.dtype, device=x.device)
     _lib.check(_lib.lib().jl_moe_gather(x.data_ptr(), x.stride(0), row_src.data_ptr(), xs.data_ptr(), row_src.shape[0], W,
                                         dtype_code(x.dtype), _stream()), "jl_moe_gather")
     return xs
@@ -502,7 +504,7 @@ def gemm_grouped(x: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, *, 
     _need(w, torch.bfloat16, "w")
     n, N, K = w.shape
     rows = x.shape[0]
-    out = torch.empty((rows, N), dtype=torch.float32 if out_f32 else torch.bfloat16, device=x.device)
+    out = empty((rows, N), dtype=torch.float32 if out_f32 else torch.bfloat16, device=x.device)
     L = _lib.lib()
     if act != ACT_NONE and not out_f32:
         _lib.check(L.jl_gemm_grouped_act(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, N, K, n, tile_group.data_ptr(), _p(tiles_used),
@@ -526,7 +528,7 @@ def gemm_glu(x: torch.Tensor, w: torch.Tensor, u_off: int, F: int, *, kind: int 
         raise ValueError("gemm_glu: contiguous operands")
     n, N, K = w.shape if w.dim() == 3 else (1, *w.shape)
     rows = x.shape[0]
-    out = x.new_empty((rows, F))
+    out = empty((rows, F), dtype=x.dtype, device=x.device)
     _lib.check(_lib.lib().jl_gemm_glu(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, F, K, N, 0, int(u_off), n, _p(tile_group), _p(tiles_used), kind,
                                       act, float(limit), float(alpha), num_sms(x.device), _stream()), "jl_gemm_glu")
     return out
@@ -538,7 +540,7 @@ def moe_combine(z: torch.Tensor, pos: Optional[torch.Tensor], wt: torch.Tensor, 
     """Σ_k wt[m, k] · z[pos[m, k]] (+ sigmoid(gate[m]) · shared[m]) → fp32 [M, W]; gate: fp32 view [M, 1] (any pitch).
     With `idx` the pairs whose expert is < 0 are skipped, and ident_w[m] · x[m] (identity experts) is added."""
     M, top = wt.shape
-    out = torch.empty((M, W), dtype=torch.float32, device=z.device)
+    out = empty((M, W), dtype=torch.float32, device=z.device)
     if idx is not None:
         _lib.check(_lib.lib().jl_moe_combine_ex(z.data_ptr(), z.stride(0), _p(pos), wt.data_ptr(), top, _p(shared),
                                                 shared.stride(0) if shared is not None else 0, _p(gate),
@@ -562,7 +564,7 @@ def embed_pair_norm(ids: torch.Tensor, table: torch.Tensor, pair: torch.Tensor, 
     ids32 = ids.to(torch.int32).contiguous().view(-1)
     V, W = table.shape
     if out is None:
-        out = torch.empty((B * S, W), dtype=torch.float32, device=table.device)
+        out = empty((B * S, W), dtype=torch.float32, device=table.device)
     _lib.check(_lib.lib().jl_embed_pair_norm(ids32.data_ptr(), table.data_ptr(), pair.data_ptr(), _p(norm_w), out.data_ptr(),
                                              prev_tok.data_ptr(), _p(cache_len), _p(pad_left), B, S, W, V, int(buckets),
                                              int(mul_prev), int(mul_cur), float(eps), dtype_code(table.dtype), _stream()),
@@ -581,7 +583,7 @@ def causal_conv(y: torch.Tensor, col0: int, w: torch.Tensor, bias: Optional[torc
         _need(in_bias, torch.float32, "in_bias")
     C, taps = w.shape
     if out is None:
-        out = torch.empty((B * S, C), dtype=torch.float32, device=y.device)
+        out = empty((B * S, C), dtype=torch.float32, device=y.device)
     _lib.check(_lib.lib().jl_causal_conv(y.data_ptr(), y.stride(0), int(col0), C, _p(in_bias), w.data_ptr(), _p(bias), _p(state),
                                          out.data_ptr(), out.stride(0), _p(cache_len), _p(pad_left), B, S, taps, act, dtype_code(w.dtype), _stream()),
                "jl_causal_conv")
@@ -593,7 +595,7 @@ def norm_mean2(a: torch.Tensor, wa: torch.Tensor, b: Optional[torch.Tensor], wb:
     """c · (norm(a) · wa + norm(b) · wb), fp32 [M, W]."""
     _need(a, torch.float32, "a")
     M, W = a.shape
-    out = torch.empty((M, W), dtype=torch.float32, device=a.device)
+    out = empty((M, W), dtype=torch.float32, device=a.device)
     _lib.check(_lib.lib().jl_norm_mean2(a.data_ptr(), a.stride(0), wa.data_ptr(), _p(b), b.stride(0) if b is not None else 0,
                                         _p(wb), float(c), out.data_ptr(), M, W, float(eps), dtype_code(wa.dtype), _stream()),
                "jl_norm_mean2")
@@ -605,7 +607,7 @@ def gated_groupnorm(o: torch.Tensor, x: Optional[torch.Tensor], skip: Optional[t
     """((o + skip[head] · x) · act(z)) normed over each of `groups` equal parts of a row, times w; o fp32 [M, N]; x, z fp32 views."""
     _need(o, torch.float32, "o")
     M, N = o.shape
-    out = torch.empty((M, N), dtype=w.dtype, device=o.device)
+    out = empty((M, N), dtype=w.dtype, device=o.device)
     _lib.check(_lib.lib().jl_gated_groupnorm(o.data_ptr(), _p(x), x.stride(0) if x is not None else 0, _p(skip), int(P),
                                              z.data_ptr(), z.stride(0), w.data_ptr(), out.data_ptr(), M, N, int(groups),
                                              float(eps), gate_act, dtype_code(w.dtype), _stream()), "jl_gated_groupnorm")
@@ -619,7 +621,7 @@ def glu_act(y: torch.Tensor, g_off: int, u_off: int, F: int, out_dtype: torch.dt
     rows_used · rows_mult rows are computed (`zero`: the rest reads as zero)."""
     _need(y, torch.float32, "y")
     M = y.shape[0]
-    out = (torch.zeros if zero else torch.empty)((M, F), dtype=out_dtype, device=y.device)
+    out = torch.zeros((M, F), dtype=out_dtype, device=y.device) if zero else empty((M, F), dtype=out_dtype, device=y.device)
     _lib.check(_lib.lib().jl_glu_act(y.data_ptr(), y.stride(0), int(g_off), int(u_off), out.data_ptr(), out.stride(0), M, F, kind,
                                      act, float(limit), float(alpha), _p(rows_used), int(rows_mult), dtype_code(out_dtype), _stream()),
                "jl_glu_act")
@@ -644,13 +646,13 @@ def ssd_scan(y: torch.Tensor, dt_off: int, dt_bias: torch.Tensor, a_log: torch.T
     _need(state, torch.float32, "state")
     M = B * S
     L = _lib.lib()
-    aux = torch.empty((M, 2 * H), dtype=torch.float32, device=y.device)
+    aux = empty((M, 2 * H), dtype=torch.float32, device=y.device)
     _lib.check(L.jl_ssd_gates(y.data_ptr(), y.stride(0), int(dt_off), dt_bias.data_ptr(), a_log.data_ptr(), aux.data_ptr(), M, H,
                               dtype_code(a_log.dtype), _stream()), "jl_ssd_gates")
-    out = torch.empty((M, H * Dv), dtype=torch.float32, device=y.device)
+    out = empty((M, H * Dv), dtype=torch.float32, device=y.device)
     ws = None
     if S > GLA_FUSED_MAX_TOKENS:
-        ws = torch.empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
+        ws = empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
     _lib.check(L.jl_ssd_scan(u.data_ptr(), u.stride(0), q_off, k_off, v_off, G, aux.data_ptr(), state.data_ptr(), out.data_ptr(),
                              _p(cache_len), _p(pad_left), B, S, H, D, Dv, _p(ws), _stream()), "jl_ssd_scan")
     return out
@@ -666,10 +668,10 @@ def delta_scan(u: torch.Tensor, q_off: int, k_off: int, v_off: int, G: int, y: t
     _need(state, torch.float32, "state")
     L = _lib.lib()
     R = a2.shape[1]
-    out = torch.empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
+    out = empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
     ws = None
     if S > DELTA_FUSED_MAX_TOKENS:        # prompts: token-parallel records + pipelined scan; fewer tokens: one fused launch
-        ws = torch.empty(int(L.jl_delta_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
+        ws = empty(int(L.jl_delta_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
     _lib.check(L.jl_delta_scan(u.data_ptr(), u.stride(0), q_off, k_off, v_off, G, y.data_ptr(), y.stride(0), b_off, a_off,
                                a2.data_ptr(), a_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), out.data_ptr(),
                                _p(cache_len), _p(pad_left), B, S, H, D, Dv, R, _p(ws), dtype_code(a2.dtype), _stream()),
@@ -686,10 +688,10 @@ def delta_head_scan(u: torch.Tensor, q_off: int, k_off: int, v_off: int, G: int,
     _need(y, torch.float32, "y")
     _need(state, torch.float32, "state")
     L = _lib.lib()
-    out = torch.empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
+    out = empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
     ws = None
     if S > DELTA_FUSED_MAX_TOKENS:
-        ws = torch.empty(int(L.jl_delta_head_scan_ws_floats(B, S, H, G, D, Dv)), dtype=torch.float32, device=y.device)
+        ws = empty(int(L.jl_delta_head_scan_ws_floats(B, S, H, G, D, Dv)), dtype=torch.float32, device=y.device)
     _lib.check(L.jl_delta_head_scan(u.data_ptr(), u.stride(0), q_off, k_off, v_off, G, y.data_ptr(), y.stride(0), b_off, a_off,
                                     a_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), out.data_ptr(), _p(cache_len), _p(pad_left),
                                     B, S, H, D, Dv, _p(ws), dtype_code(a_log.dtype), _stream()), "jl_delta_head_scan")
@@ -703,7 +705,7 @@ def embed_pos(ids: torch.Tensor, table: torch.Tensor, pos_table: torch.Tensor, c
     ids32 = ids if ids.dtype == torch.int32 and ids.is_contiguous() else ids.to(torch.int32).contiguous()
     V, W = table.shape
     if out is None:
-        out = torch.empty((B * S, W), dtype=torch.float32, device=table.device)
+        out = empty((B * S, W), dtype=torch.float32, device=table.device)
     _lib.check(_lib.lib().jl_embed_pos(ids32.data_ptr(), table.data_ptr(), pos_table.data_ptr(), out.data_ptr(), _p(cache_len),
                                        _p(pad_left), B, S, W, V, pos_table.shape[0], dtype_code(table.dtype), _stream()),
                "jl_embed_pos")
@@ -715,7 +717,7 @@ def side_gate(t: torch.Tensor, ids: torch.Tensor, side: torch.Tensor, col0: int,
     _need(t, torch.float32, "t")
     _need(ids, torch.int32, "ids")
     M = t.shape[0]
-    out = torch.empty((M, n), dtype=out_dtype, device=t.device)
+    out = empty((M, n), dtype=out_dtype, device=t.device)
     _lib.check(_lib.lib().jl_side_gate(t.data_ptr(), t.stride(0), ids.data_ptr(), side.data_ptr(), side.stride(0), int(col0),
                                        out.data_ptr(), out.stride(0), M, int(n), side.shape[0], dtype_code(out_dtype), _stream()),
                "jl_side_gate")
@@ -729,7 +731,7 @@ def side_gate_rows(x: torch.Tensor, ids: torch.Tensor, side: torch.Tensor, col0:
     _need(ids, torch.int32, "ids")
     M, W = x.shape
     n = w_gate.shape[0]
-    out = torch.empty((M, n), dtype=w_gate.dtype, device=x.device)
+    out = empty((M, n), dtype=w_gate.dtype, device=x.device)
     _lib.check(_lib.lib().jl_side_gate_rows(x.data_ptr(), x.stride(0), ids.data_ptr(), side.data_ptr(), side.stride(0), int(col0),
                                             w_gate.data_ptr(), out.data_ptr(), out.stride(0), M, W, n, side.shape[0],
                                             dtype_code(w_gate.dtype), _stream()), "jl_side_gate_rows")
@@ -741,7 +743,7 @@ def branch_add_cast(x: torch.Tensor, y1: Optional[torch.Tensor], y2: Optional[to
     """x += mult · (y1 + y2) in place (fp32; either branch may be None); returns the updated rows in `dtype`."""
     _need(x, torch.float32, "x")
     M, W = x.shape
-    xc = torch.empty((M, W), dtype=dtype, device=x.device)
+    xc = empty((M, W), dtype=dtype, device=x.device)
     _lib.check(_lib.lib().jl_branch_add_cast(_p(y1), y1.stride(0) if y1 is not None else 0, _p(y2),
                                              y2.stride(0) if y2 is not None else 0, float(mult), x.data_ptr(), xc.data_ptr(), M, W,
                                              dtype_code(dtype), _stream()), "jl_branch_add_cast")
@@ -757,7 +759,7 @@ def postnorm_cast(y1: torch.Tensor, w: torch.Tensor, x: torch.Tensor, eps: float
     if y2 is not None:
         _need(y2, torch.float32, "y2")
     M, W = x.shape
-    h = torch.empty((M, W), dtype=w.dtype, device=x.device) if w.dtype != torch.float32 else None
+    h = empty((M, W), dtype=w.dtype, device=x.device) if w.dtype != torch.float32 else None
     _lib.check(_lib.lib().jl_postnorm_cast(y1.data_ptr(), y1.stride(0), _p(bias), float(c1), _p(y2), y2.stride(0) if y2 is not None else 0,
                                            float(c2), w.data_ptr(), x.data_ptr(), _p(h), M, W, float(eps), dtype_code(w.dtype),
                                            _stream()), "jl_postnorm_cast")
@@ -768,7 +770,7 @@ def weighted_sum2(y1: torch.Tensor, bias: Optional[torch.Tensor], c1: float, y2:
     """c1 · (y1 + bias) + c2 · y2, fp32 [M, W]."""
     _need(y1, torch.float32, "y1")
     M, W = y1.shape
-    out = torch.empty((M, W), dtype=torch.float32, device=y1.device)
+    out = empty((M, W), dtype=torch.float32, device=y1.device)
     _lib.check(_lib.lib().jl_weighted_sum2(y1.data_ptr(), y1.stride(0), _p(bias), float(c1), _p(y2), y2.stride(0) if y2 is not None else 0,
                                            float(c2), out.data_ptr(), M, W, dtype_code(bias.dtype) if bias is not None else 1,
                                            _stream()), "jl_weighted_sum2")
@@ -780,7 +782,7 @@ def rownorm_gate(o: torch.Tensor, w: torch.Tensor, gate: torch.Tensor, eps: floa
     _need(o, torch.float32, "o")
     _need(gate, torch.float32, "gate")
     M, N = o.shape
-    out = torch.empty((M, N), dtype=w.dtype, device=o.device)
+    out = empty((M, N), dtype=w.dtype, device=o.device)
     _lib.check(_lib.lib().jl_rownorm_gate(o.data_ptr(), w.data_ptr(), gate.data_ptr(), gate.stride(0), out.data_ptr(), M, N, float(eps),
                                           gate_act, dtype_code(w.dtype), _stream()), "jl_rownorm_gate")
     return out
@@ -815,10 +817,10 @@ def activated_scan(y: torch.Tensor, q_off: int, k_off: int, v_off: int, head_dec
     _need(state, torch.float32, "state")
     _need(head_decay, torch.float32, "head_decay")
     L = _lib.lib()
-    out = torch.empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
+    out = empty((B * S, H * Dv), dtype=torch.float32, device=y.device)
     ws = None
     if S > GLA_FUSED_MAX_TOKENS:
-        ws = torch.empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
+        ws = empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
     _lib.check(L.jl_activated_scan(y.data_ptr(), y.stride(0), q_off, k_off, v_off, head_decay.data_ptr(), act, state.data_ptr(),
                                    out.data_ptr(), _p(cache_len), _p(pad_left), B, S, H, D, Dv, _p(ws), _stream()), "jl_activated_scan")
     return out
@@ -835,14 +837,14 @@ def mlstm_scan(y: torch.Tensor, q_off: int, k_off: int, v_off: int, i_off: int, 
     _need(m_state, torch.float32, "m_state")
     L = _lib.lib()
     M = B * S
-    aux = torch.empty((M, 3 * H), dtype=torch.float32, device=y.device)
+    aux = empty((M, 3 * H), dtype=torch.float32, device=y.device)
     _lib.check(L.jl_mlstm_gates(y.data_ptr(), y.stride(0), int(i_off), int(f_off), i_bias.data_ptr(), f_bias.data_ptr(), float(cap),
                                 m_state.data_ptr(), aux.data_ptr(), _p(cache_len), _p(pad_left), B, S, H, dtype_code(i_bias.dtype),
                                 _stream()), "jl_mlstm_gates")
-    out = torch.empty((M, H * (Dv + 1)), dtype=torch.float32, device=y.device)
+    out = empty((M, H * (Dv + 1)), dtype=torch.float32, device=y.device)
     ws = None
     if S > GLA_FUSED_MAX_TOKENS:
-        ws = torch.empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv + 1)), dtype=torch.float32, device=y.device)
+        ws = empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv + 1)), dtype=torch.float32, device=y.device)
     _lib.check(L.jl_mlstm_scan(y.data_ptr(), y.stride(0), q_off, k_off, v_off, aux.data_ptr(), 3 * H, float(q_scale), state.data_ptr(),
                                out.data_ptr(), _p(cache_len), _p(pad_left), B, S, H, D, Dv, _p(ws), _stream()), "jl_mlstm_scan")
     return out, aux
@@ -854,7 +856,7 @@ def mlstm_finish(o: torch.Tensor, aux: torch.Tensor, w: torch.Tensor, gate: torc
     _need(o, torch.float32, "o")
     _need(gate, torch.float32, "gate")
     M = o.shape[0]
-    out = torch.empty((M, H * Dv), dtype=w.dtype, device=o.device)
+    out = empty((M, H * Dv), dtype=w.dtype, device=o.device)
     _lib.check(_lib.lib().jl_mlstm_finish(o.data_ptr(), aux.data_ptr(), w.data_ptr(), gate.data_ptr(), gate.stride(0), out.data_ptr(), M, H,
                                           Dv, float(eps), gate_act, dtype_code(w.dtype), _stream()), "jl_mlstm_finish")
     return out

@@ -1,0 +1,104 @@
+"""The host side of a kernel call: the built-in form of the entry points (csrc/binding.cc) beside ctypes', and the room of a layer's intermediates (ops/scratch.py).
+What is called here computes on the host; nothing needs a GPU."""
+import ctypes as C
+import threading
+
+import pytest
+import torch
+
+from jax_llama_b200.ops import _lib, build
+from jax_llama_b200.ops.scratch import ALIGN, CHUNK, LARGEST, Array, Scratch, empty
+
+
+@pytest.fixture(scope="module")
+def pair():
+    """(the library with built-in entry points, the same library through ctypes alone)"""
+    fast = _lib.lib()
+    if build.build_binding() is None:
+        pytest.skip("no interpreter headers: ctypes is what runs")
+    slow = C.CDLL(fast._name)
+    for name, (res, args) in {**_lib._SIGNATURES, **_lib._HYBRID}.items():
+        getattr(slow, name).restype, getattr(slow, name).argtypes = res, args
+    return fast, slow
+
+
+def test_the_hot_entry_points_are_built_in(pair):
+    fast, _ = pair
+    for name in ("jl_gemm", "jl_linear_resident", "jl_gla_scan", "jl_attn_step", "jl_moe_combine", "jl_delta_head_scan", "jl_sample_full", "jl_decode_attn_fused"):
+        assert type(getattr(fast, name)).__name__ == "builtin_function_or_method"
+
+
+@pytest.mark.parametrize("name,args", [("jl_attn_generic_splits", (1, 16, 4, 4096)), ("jl_gla_scan_ws_floats", (3, 700, 16, 64, 128)),
+                                       ("jl_gla_scan_ws_floats", (1, 2048, 4, 200, 64)), ("jl_delta_head_scan_ws_floats", (2, 1000, 16, 16, 64, 128)),
+                                       ("jl_linear_f32_pair_ws", (4096, 2048, 8192, 200, 5464, 2048, 148)), ("jl_linear_f32_pair_ws", (4100, 2048, 8192, 200, 5464, 2048, 148)),
+                                       ("jl_linear_f32_pair_ws", (None, 2048, 8192, 64, 64, 64, 148)), ("jl_attn_generic_splits", (True, 2, 1, 2 ** 31 - 1))])
+def test_same_answers(pair, name, args):
+    fast, slow = pair
+    assert getattr(fast, name)(*args) == getattr(slow, name)(*args)
+
+
+def test_refusals_and_messages_are_the_same(pair):
+    fast, slow = pair
+    bad = (16, 16, 16, 16, 0, 8, 8, 0, 0, 148, 0)               # M = 0: refused before anything is launched
+    assert fast.jl_gemm(*bad) == slow.jl_gemm(*bad) == 1
+    assert b"M=0" in fast.jl_last_error()
+    for call in ((), (1, 2), ("1", 2, 3, 4), (1.5, 2, 3, 4)):
+        with pytest.raises((TypeError, C.ArgumentError)) as a:
+            slow.jl_attn_generic_splits(*call)
+        with pytest.raises(type(a.value)):
+            fast.jl_attn_generic_splits(*call)
+    assert fast.jl_attn_generic_splits(2 ** 32 + 1, 2, 1, 64) == slow.jl_attn_generic_splits(2 ** 32 + 1, 2, 1, 64)      # ctypes takes the low bits
+
+
+def test_numbers_arrive_as_declared(pair):
+    """Whole numbers for a float, None and 0 for an address: through the checks of a call that refuses its shape last."""
+    fast, slow = pair
+    args = lambda eps: (0, None, 0, 0, None, 0, 5, eps, 0)       # noqa: E731  jl_rmsnorm with M = 0 rows
+    for eps in (1, 1e-5, True):
+        assert fast.jl_rmsnorm(*args(eps)) == slow.jl_rmsnorm(*args(eps))
+
+
+CPU = torch.device("cpu")
+
+
+def test_outside_a_block_arrays_are_tensors():
+    t = empty((3, 5), dtype=torch.float32, device=CPU)
+    assert isinstance(t, torch.Tensor) and t.shape == (3, 5)
+
+
+def test_arrays_of_a_block():
+    with Scratch() as s:
+        a, b, c = empty((3, 5), dtype=torch.float32, device=CPU), empty(7, dtype=torch.int32, device=CPU), empty((4, 6), dtype=torch.bfloat16, device=CPU)
+        room = s.room
+        assert all(isinstance(x, Array) for x in (a, b, c))
+        assert a.data_ptr() == room.data_ptr() and b.data_ptr() - a.data_ptr() == ALIGN and c.data_ptr() - b.data_ptr() == ALIGN
+        big = empty((LARGEST // 4 + 1, 1), dtype=torch.float32, device=CPU)
+        none = empty((0, 4), dtype=torch.float32, device=CPU)
+        assert isinstance(big, torch.Tensor) and isinstance(none, torch.Tensor)
+        with Scratch() as inner:
+            d = empty(3, dtype=torch.uint8, device=CPU)
+            assert d.room is inner.room and d.room is not room
+        assert empty(1, dtype=torch.uint8, device=CPU).room is room
+        other = []
+        th = threading.Thread(target=lambda: other.append(empty((2, 2), dtype=torch.float32, device=CPU)))
+        th.start()
+        th.join()
+        assert isinstance(other[0], torch.Tensor)               # the block is its thread's
+        first = s.room
+        for _ in range(CHUNK // LARGEST + 1):                   # a full room: another one, the arrays keep theirs
+            e = empty(LARGEST, dtype=torch.uint8, device=CPU)
+        assert s.room is not first and e.room is s.room and a.room is first
+    assert isinstance(empty(2, dtype=torch.uint8, device=CPU), torch.Tensor)
+
+
+def test_an_array_answers_as_the_tensor_it_stands_for():
+    t = torch.empty((6, 10), dtype=torch.bfloat16)
+    a = Array(t.data_ptr(), (6, 10), 10, t.dtype, CPU, t)
+    pairs = [(a, t), (a[:, 2:7], t[:, 2:7]), (a[:, :4], t[:, :4]), (a[:, 3:], t[:, 3:]), (a[:, 3:][:, 1:2], t[:, 3:][:, 1:2]), (a.view(60), t.view(60)),
+             (a.view(4, 15), t.view(4, 15)), (a.view(-1), t.view(-1)), (a.view(-1, 5), t.view(-1, 5)), (a[:, :-4], t[:, :-4])]
+    for x, y in pairs:
+        assert x.data_ptr() == y.data_ptr() and tuple(x.shape) == tuple(y.shape) and x.numel() == y.numel() and x.dim() == y.dim()
+        assert x.is_contiguous() == y.is_contiguous() and x.stride(0) == y.stride(0) and x.dtype == y.dtype and x.device == y.device
+    for wrong in (lambda: a.view(7, 9), lambda: a[:, 1:3].view(-1), lambda: a[1:, :], lambda: a[:, ::2]):
+        with pytest.raises((ValueError, IndexError)):
+            wrong()

@@ -3,7 +3,7 @@
 //  * embed_pair_norm_kernel — token embedding plus one row of a hashed pair table chosen by (previous token, token), then
 //    the model norm; the previous token of every row of the batch is state that the kernel reads and replaces.
 //  * causal_conv_kernel     — short causal convolution over time per channel with an activation; the last taps-1 inputs
-//    of every row are state.
+//    of every row are state; causal_conv_vec_kernel: prompts of up to four taps.
 //  * norm_mean2_kernel      — c * (norm(a) * wa + norm(b) * wb): two mixers that run side by side on the same input.
 //  * gated_groupnorm_kernel — (o + skip * x) * act(z), then an RMS norm over equal parts of the row, times a weight.
 //  * glu_act_kernel         — gated activations of a fused gate | up product (act(g) * u; the clamped sigmoid form).
@@ -148,6 +148,74 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restric
     for (int u = 0; u < AHEAD; ++u)
       if (t0 + u < s1) op[(size_t)u * ldo] = t0 + u >= first ? acc[u] : 0.0f;
     op += (size_t)AHEAD * ldo;
+  }
+}
+
+// Prompts of few taps: a thread has four channels of TOK tokens (at least CV_TAPS - 1) and asks for all it needs at once, 16 bytes each; the tokens before them
+// come a second time, from L1 or L2.  Every sum and state is formed as above, bit for bit.
+// Bound: bytes where they do not fit the L2 (8 rows x 2000 tokens x 4096 channels: 4.2 TB/s), a memory latency and the activations' issue below.  One B200, in a chain of
+// itself, us, walking a chunk of tokens (above) -> 4 tokens a thread | 8 (five CTAs per SM; one to four 21.7, six 19.5, eight 21.2; 12 tokens 18.9, 16 21.7): 2 rows x 1000 x 4096
+// 23.6 -> 21.9 | 17.6, 1 x 2048 x 2048 12.6 -> 12.6 | 11.0, 8 x 2000 x 4096 146 -> 169 | 124, 1 x 1000 x 2048 7.9 -> 7.5 | 7.4, 1 x 1000 x 1536 7.3 -> 6.8 | 7.1, 2 x 500 x 1024 6.8 -> 4.7 |
+// 5.7, 1 x 100 x 256 6.5 -> 3.2 | 4.7, 1 x 12 x 512 4.1 -> 3.2 | 4.9: eight tokens from CV_LARGE values on.  Up to 8 tokens the walk is one round too: 16 x 8 x 512 3.3 -> 3.4 | 4.7
+// (a delta-rule layer of 2 x 1000 tokens 205.3 -> 202.7).
+constexpr int CV_TAPS = 4, CV_MIN = 9;
+constexpr long CV_LARGE = 2000000;
+template <typename T, int ACT, int TOK>
+__global__ void __launch_bounds__(128, TOK > 4 ? 5 : 1) causal_conv_vec_kernel(const float* __restrict__ y, int ldy, int col0, int C, const float* __restrict__ in_bias,
+                                                              const T* __restrict__ w, const T* __restrict__ bias, float* __restrict__ state,
+                                                              float* __restrict__ out, int ldo, const int* __restrict__ cache_len,
+                                                              const int* __restrict__ pad_left, int S, int taps, int threads) {
+  pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
+  pdl_launch_dependents();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y, quads = C / 4;
+  if (i >= threads) return;
+  const int c = i % quads * 4, s0 = i / quads * TOK, nh = taps - 1;
+  const int first = (pad_left ? pad_left[b] : 0) - (cache_len ? *cache_len : 0);      // tokens before it are padding
+  const float* yp = y + (size_t)b * S * ldy + col0 + c;
+  float x[TOK + CV_TAPS - 1][4];                         // token s0 - (CV_TAPS - 1) and on
+#pragma unroll
+  for (int r = 0; r < TOK + CV_TAPS - 1; ++r) load4(yp + (size_t)min(max(s0 + r - (CV_TAPS - 1), 0), S - 1) * ldy, x[r]);
+  float wv[CV_TAPS][4], bv[4] = {}, ib[4] = {};
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int j = 0; j < CV_TAPS; ++j) wv[j][e] = j < taps ? to_f(w[(size_t)(c + e) * taps + taps - 1 - j]) : 0.0f;
+  if (bias) load4(bias + c, bv);
+  if (in_bias) load4(in_bias + c, ib);
+#pragma unroll
+  for (int r = 0; r < TOK + CV_TAPS - 1; ++r) {
+    const bool in = s0 + r - (CV_TAPS - 1) >= max(first, 0);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x[r][e] = in ? x[r][e] + ib[e] : 0.0f;
+  }
+  if (s0 == 0) {                                               // this thread alone reads and replaces the state of its channels (S >= TOK: all new)
+    float* st = state + (size_t)b * nh * C + c;
+#pragma unroll
+    for (int r = 0; r < CV_TAPS - 1; ++r)
+      if (r >= CV_TAPS - 1 - nh) load4(st + (size_t)(r - (CV_TAPS - 1 - nh)) * C, x[r]);
+    for (int t = 0; t < nh; ++t) {
+      const int s = S - nh + t;
+      float v[4];
+      load4(yp + (size_t)s * ldy, v);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = s >= first ? v[e] + ib[e] : 0.0f;
+      store4(st + (size_t)t * C, v);
+    }
+  }
+  float* op = out + ((size_t)b * S + s0) * ldo + c;
+#pragma unroll
+  for (int u = 0; u < TOK; ++u) {
+    float acc[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      acc[e] = fmaf(wv[0][e], x[u + CV_TAPS - 1][e], bv[e]);
+#pragma unroll
+      for (int j = 0; j < CV_TAPS - 1; ++j) if (j < nh) acc[e] = fmaf(wv[j + 1][e], x[u + CV_TAPS - 2 - j][e], acc[e]);
+    }
+    apply_act_n(acc, ACT, 0.0f, 0.0f);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] = s0 + u >= first ? acc[e] : 0.0f;
+    if (s0 + u < S) store4(op + (size_t)u * ldo, acc);
   }
 }
 
@@ -439,6 +507,20 @@ extern "C" JL_API int jl_causal_conv(const float* y, int ldy, int col0, int C, c
   JL_CHECK_ARG(B >= 1 && S >= 1 && C >= 1 && ldo >= C, "jl_causal_conv: bad shape");
   JL_CHECK_ARG(taps >= 1 && taps <= CC_MAX_TAPS, "jl_causal_conv: %d taps (1 .. %d)", taps, CC_MAX_TAPS);
   JL_CHECK_ARG(taps == 1 || state != nullptr, "jl_causal_conv: no state for %d taps", taps);
+  const bool vec = C % 4 == 0 && ldy % 4 == 0 && col0 % 4 == 0 && ldo % 4 == 0 &&
+                   ((uintptr_t)y | (uintptr_t)out | (uintptr_t)state | (uintptr_t)bias | (uintptr_t)in_bias) % 16 == 0;
+  if (vec && taps <= CV_TAPS && (act == ACT_SILU || act == ACT_NONE) && S >= CV_MIN && (long)C * S < (1L << 31)) {
+    const int tok = (long)B * S * C >= CV_LARGE ? 8 : 4, threads = C / 4 * ((S + tok - 1) / tok);
+#define JL_CV(ACT_, TOK_)                                                                                                                          \
+  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((causal_conv_vec_kernel<T, ACT_, TOK_>), dim3((threads + 127) / 128, B), dim3(128), 0, stream, y, ldy, col0, C, \
+                                         in_bias, (const T*)w, (const T*)bias, state, out, ldo, cache_len, pad_left, S, taps, threads))
+    if (act == ACT_SILU) { if (tok == 8) JL_CV(ACT_SILU, 8); else JL_CV(ACT_SILU, 4); }
+    else if (tok == 8) JL_CV(ACT_NONE, 8);
+    else JL_CV(ACT_NONE, 4);
+#undef JL_CV
+    JL_CUDA(cudaGetLastError());
+    return JL_OK;
+  }
   // half the tokens per CTA where that many CTAs leave room (2048 tokens x 2048 channels 33 -> 22 us a cold launch; at least taps - 1 tokens: 31)
   const int chunk = (long)((C + 127) / 128) * B * ((S + CC_CHUNK - 1) / CC_CHUNK) < SMS * 6 ? CC_CHUNK / 2 : CC_CHUNK;
   dim3 grid((C + 127) / 128, B, (S + chunk - 1) / chunk);

@@ -8,15 +8,17 @@
 //     LEADER's (cluster rank 0) mbarrier; the leader's single MMA thread issues the pair-wide MMAs, and
 //     `tcgen05.commit ... .multicast::cluster` releases the stage / publishes the accumulator in BOTH CTAs at once;
 //   * each CTA holds the fp32 accumulator rows of its own 128 tokens in its own TMEM (double buffered: 2 x 256
-//     columns = all 512), drained by its four epilogue warps while the next tile's MMAs run;
+//     columns = all 512), drained by its epilogue warps while the next tile's MMAs run;
 //   * the epilogue goes through shared memory and leaves the SM as TMA tensor stores (`cp.async.bulk.tensor` shared →
-//     global, 32 x 64 element boxes): full 128-byte rows on the wire instead of one 64-byte row write per thread, and
-//     rows beyond M are clipped by the tensor map.
+//     global) of 32 rows of 128 bytes, swizzled so that a warp's rows lie on all banks; rows beyond M and columns beyond N are
+//     clipped by the tensor map.  bf16 results: eight warps, a buffer each; fp32 results: four warps, two buffers each.
 // All TMA loads here read this GPU's own memory through tensor maps over local buffers.
 //
-// fp32 results (the projections of the hybrid family) leave the same way in 32 x 32 boxes of 128-byte rows, swizzled, through two
-// staging buffers per warp.  2048 tokens on one B200, single-CTA kernel -> this one: 10928 x 2048 91 -> 73 us, 6160 x 2048
-// 57 -> 46, 2048 x 5464 60 -> 43.
+// Bound: the operands' way from L2 into the SMs (10.5 TB/s over the chip: 450 ns per 64 k of a tile against 277 of products); up to some 100 tiles also the last
+// epilogue, which nothing overlaps.  One B200, us: single-CTA kernel -> this one, 2048 tokens x 10928 x 2048 91 -> 73, 6160 x 2048 57 -> 46, 2048 x 5464 60 -> 43.  In a
+// chain of itself, bf16 results through rows on the same banks by four warps -> this: 2048 x 2048 x 2048 17.7 -> 15.4, 2048 x 4096 x 512 14.3 -> 10.6, 2048 x 3072 x
+// 768 16.0 -> 12.4, 512 x 2048 x 2048 15.9 -> 13.7, 256 x 256 x 256 7.5 -> 5.0, 2048 x 6160 x 2048 37.6 -> 35.8, 4096 x 4096 x 4096 92.5 -> 92.6.  fp32 results with eight warps were
+// slower, with one buffer (2048 x 2048 x 2048 16.3 -> 16.7) or two and a shorter ring (2048 x 6160 x 2048 39.6 -> 41.4).
 //
 // Used for token-major GEMMs with M >= 256 and N and K multiples of 256 and 64 (every prefill GEMM of the LLaMA shapes); plain bf16 and
 // fp32 results with any N and K that are multiples of 8 (the tensor maps read zeros and clip beyond the matrix).  Other shapes take the
@@ -34,16 +36,18 @@ namespace jl {
 constexpr int G2_BM = 128;            // token rows per CTA (256 per pair)
 constexpr int G2_BN = 256;            // weight rows per pair tile (128 staged per CTA)
 constexpr int G2_BK = 64;
-constexpr int G2_THREADS = 256;       // warp0 TMA, warp1 MMA (leader), warp2 TMEM alloc, warp3 idle, warps 4-7 epilogue
 constexpr uint32_t G2_A_BYTES = G2_BM * G2_BK * 2;                 // 16 KB
 constexpr uint32_t G2_B_BYTES = (G2_BN / 2) * G2_BK * 2;           // 16 KB
 constexpr uint32_t G2_STAGE_BYTES = G2_A_BYTES + G2_B_BYTES;
-constexpr uint32_t G2_EPI_BYTES = 4 * 32 * 64 * 2;                 // per CTA: 4 warps x [32 rows][64 cols] bf16 (fp32: [32][32], twice)
+constexpr uint32_t G2_EPI_BUF = 32 * 128;                          // 32 rows of 128 bytes
 constexpr int G2_MAX_STAGES = 6;
 constexpr uint32_t G2_PEER_MASK = 0xFEFFFFFFu;                     // shared::cluster address of the same offset in CTA 0
 
 enum { G2_PLAIN = 0, G2_RESIDUAL = 1, G2_SWIGLU = 2, G2_F32 = 3 };
-__host__ __device__ constexpr uint32_t g2_epi_bytes(int epi) { return epi == G2_F32 ? 2 * G2_EPI_BYTES : G2_EPI_BYTES; }
+__host__ __device__ constexpr uint32_t g2_epi_bufs(int epi) { return epi == G2_F32 ? 2 : 1; }          // of a warp
+__host__ __device__ constexpr int g2_epi_warps(int epi) { return epi == G2_F32 ? 4 : 8; }
+__host__ __device__ constexpr uint32_t g2_epi_bytes(int epi) { return g2_epi_warps(epi) * g2_epi_bufs(epi) * G2_EPI_BUF; }
+__host__ __device__ constexpr int g2_threads(int epi) { return 128 + 32 * g2_epi_warps(epi); }      // warp 0 TMA, 1 MMA (leader), 2 TMEM, 3 idle, 4 .. epilogue
 
 struct Gemm2Params {
   const __nv_bfloat16* residual;
@@ -102,7 +106,7 @@ __device__ __forceinline__ void g2_commit_both(uint32_t bar) {
 }
 
 template <int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2_threads(EPI), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
              const __grid_constant__ CUtensorMap tmap_out, const Gemm2Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -137,7 +141,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     }
     for (int s = 0; s < 2; ++s) {
       tc::mbar_init(tfull_bar(s), 1);                       // one multicast commit per tile
-      tc::mbar_init(tempty_bar(s), 8);                      // leader's: 4 epilogue warps of each CTA
+      tc::mbar_init(tempty_bar(s), 2 * g2_epi_warps(EPI));  // leader's: the epilogue warps of both CTAs
     }
     tc::fence_barrier_init();
   }
@@ -195,10 +199,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       }
     }
   } else if (warp >= 4) {
-    // ===================================================== epilogue: TMEM → registers → shared → TMA store
-    const int quarter = warp & 3;                           // TMEM lanes [32·quarter, 32·quarter+32)
-    const uint32_t my_smem = epi_smem + quarter * (g2_epi_bytes(EPI) / 4);
-    uint8_t* my_ptr = epi_ptr + quarter * (g2_epi_bytes(EPI) / 4);
+    // ===================================================== epilogue: TMEM → registers → shared → TMA store; every four warps have their share of the columns
+    const int quarter = warp & 3, part = (warp >> 2) - 1;   // TMEM lanes [32·quarter, 32·quarter+32)
+    constexpr uint32_t BUFS = g2_epi_bufs(EPI);
+    constexpr int PART = G2_BN / (g2_epi_warps(EPI) / 4);
+    const uint32_t my_smem = epi_smem + (warp - 4) * BUFS * G2_EPI_BUF;
+    uint8_t* my_row = epi_ptr + (warp - 4) * BUFS * G2_EPI_BUF + lane * 128;
     const uint32_t tempty_leader = g2_mapa(tempty_bar(0), 0);
     int it = 0;
     for (int t = pair; t < num_tiles; t += n_pairs, ++it) {
@@ -207,41 +213,20 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       tc::mbar_wait(tfull_bar(as), aphase);
       tc::fence_after_sync();
       const int row0 = a_blk * 2 * G2_BM + (int)rank * G2_BM + quarter * 32;      // first token row of this warp
-      const int ra = row0 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + as * G2_BN;
-      if constexpr (EPI == G2_F32) {
+      constexpr int STEP = EPI == G2_F32 ? 32 : EPI == G2_SWIGLU ? 128 : 64;      // accumulator columns of a 128-byte row of the result
 #pragma unroll 1
-        for (int c0 = 0; c0 < G2_BN; c0 += 32) {
-          uint32_t v[32];
-          tc::tmem_ld32(t_row + c0, v);
-          tc::tmem_ld_wait();
-          const uint32_t buf = (uint32_t)(c0 >> 5 & 1) * 4096u;
-          // the store before the previous one, from this buffer, must have finished reading it
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          __syncwarp();
-          uint8_t* row = my_ptr + buf + lane * 128;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)                                     // 16-byte chunks, swizzled as the tensor map expects
-            *reinterpret_cast<uint4*>(row + ((j ^ (lane & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) {
-            // rows >= M and columns >= N are clipped; a box that lies beyond the last column is not sent at all
-            if (b_blk * G2_BN + c0 < p.N) g2_tma_store_2d(&tmap_out, my_smem + buf, b_blk * G2_BN + c0, row0);
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          }
-        }
-      } else {
-#pragma unroll 1
-      for (int c0 = 0; c0 < G2_BN; c0 += 64) {
-        // 64 accumulator columns of this thread's row → up to 64 bf16 (32 for SwiGLU) in shared memory
+      for (int c0 = part * PART; c0 < (part + 1) * PART; c0 += STEP) {
         uint32_t w[32];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < STEP / 32; ++h) {
           uint32_t v[32];
           tc::tmem_ld32(t_row + c0 + h * 32, v);
           tc::tmem_ld_wait();
-          if constexpr (EPI == G2_SWIGLU) {
+          if constexpr (EPI == G2_F32) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) w[j] = v[j];
+          } else if constexpr (EPI == G2_SWIGLU) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const float g0 = __bfloat162float(__float2bfloat16(__uint_as_float(v[4 * j])));
@@ -251,7 +236,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
               w[h * 8 + j] = pack_bf16(silu(g0) * u0, silu(g1) * u1);
             }
           } else if constexpr (EPI == G2_RESIDUAL) {
-            const int col = b_blk * G2_BN + c0 + h * 32;
+            const int ra = row0 + lane, col = b_blk * G2_BN + c0 + h * 32;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               uint4 rr = make_uint4(0, 0, 0, 0);
@@ -268,22 +253,21 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             for (int j = 0; j < 16; ++j) w[h * 16 + j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
           }
         }
-        // the previous TMA store of this warp must have finished READING the staging buffer
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        // the TMA store of this warp before (two buffers: the one before that) must have finished READING the staging buffer
+        const uint32_t buf = BUFS > 1 ? (uint32_t)(c0 / STEP & 1) * G2_EPI_BUF : 0u;
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(BUFS - 1) : "memory");
         __syncwarp();
-        constexpr int OUT_COLS = EPI == G2_SWIGLU ? 32 : 64;              // bf16 columns this chunk produces
-        // staging layout [32 rows][OUT_COLS] bf16, row-major: what a plain (unswizzled) tensor-map box expects
-        uint4* dst = reinterpret_cast<uint4*>(my_ptr + lane * (OUT_COLS * 2));
 #pragma unroll
-        for (int j = 0; j < OUT_COLS / 8; ++j) dst[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+        for (int j = 0; j < 8; ++j)                                         // 16-byte chunks, swizzled as the tensor map expects
+          *reinterpret_cast<uint4*>(my_row + buf + ((j ^ (lane & 7)) << 4)) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy writes → async-proxy (TMA) reads
         __syncwarp();
         if (lane == 0) {
-          const int out_col = EPI == G2_SWIGLU ? (b_blk * G2_BN + c0) / 2 : b_blk * G2_BN + c0;
-          if (b_blk * G2_BN + c0 < p.N) g2_tma_store_2d(&tmap_out, my_smem, out_col, row0);     // rows >= M are clipped by the tensor map
+          // rows >= M and columns >= N are clipped; a box that lies beyond the last column is not sent at all
+          const int col = b_blk * G2_BN + c0;
+          if (col < p.N) g2_tma_store_2d(&tmap_out, my_smem + buf, EPI == G2_SWIGLU ? col / 2 : col, row0);
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
-      }
       }
       tc::fence_before_sync();
       __syncwarp();
@@ -296,9 +280,6 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   g2_cluster_sync();                                        // neither CTA frees TMEM / exits while the pair still uses it
   if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
 }
-
-int make_tmap_2d_bf16_plain(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
-                            uint32_t box_cols, uint32_t box_rows);
 
 }  // namespace jl
 
@@ -338,7 +319,7 @@ static int g2_resident_pairs(Gemm2Kernel kern, int mode, int stages, size_t smem
   if (cached) n = known[dev][mode][stages].load(std::memory_order_relaxed);
   if (n == 0) {
     cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(G2_THREADS);
+    cfg.blockDim = dim3(g2_threads(mode));
     cfg.dynamicSmemBytes = smem;
     cfg.gridDim = dim3((num_sms / 2) * 2);
     cudaLaunchAttribute attr[1];
@@ -383,11 +364,11 @@ static int gemm_2cta(const void* x, const void* w, const void* residual, void* o
   int rc;
   if ((rc = make_tmap_2d_bf16(&ta, x, M, K, K, G2_BM))) return rc;
   if ((rc = make_tmap_2d_bf16(&tb, w, N, K, K, G2_BN / 2))) return rc;
-  rc = mode == G2_F32 ? make_tmap_2d_f32(&to, out, M, odim, odim, 32) : make_tmap_2d_bf16_plain(&to, out, M, odim, odim, mode == G2_SWIGLU ? 32 : 64, 32);
+  rc = mode == G2_F32 ? make_tmap_2d_f32(&to, out, M, odim, odim, 32) : make_tmap_2d_bf16(&to, out, M, odim, odim, 32);
   if (rc) return rc;
   p.stages = stages;
   cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(G2_THREADS);
+  cfg.blockDim = dim3(g2_threads(mode));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = (cudaStream_t)stream;
   int grid = p.a_blocks * p.b_blocks * 2;

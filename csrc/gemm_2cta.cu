@@ -14,8 +14,8 @@
 //     clipped by the tensor map.  bf16 results: eight warps, a buffer each; fp32 results: four warps, two buffers each.
 // All TMA loads here read this GPU's own memory through tensor maps over local buffers.
 //
-// Bound: the operands' way from L2 into the SMs (10.5 TB/s over the chip: 450 ns per 64 k of a tile against 277 of products); up to some 100 tiles also the last
-// epilogue, which nothing overlaps.  One B200, us: single-CTA kernel -> this one, 2048 tokens x 10928 x 2048 91 -> 73, 6160 x 2048 57 -> 46, 2048 x 5464 60 -> 43.  In a
+// Bound: the products, 376 ns per 64 k of a tile with 64 pairs at work (2048 x 2048 x 8192, launch and epilogue included; without loads 343, loads alone 258, a ring of three
+// stages 465), and the rounds of tiles; short K and few tiles also the start and the last epilogue, which nothing overlaps, some 4 us.  One B200, us: single-CTA kernel -> this one, 2048 tokens x 10928 x 2048 91 -> 73, 6160 x 2048 57 -> 46, 2048 x 5464 60 -> 43.  In a
 // chain of itself, bf16 results through rows on the same banks by four warps -> this: 2048 x 2048 x 2048 17.7 -> 15.4, 2048 x 4096 x 512 14.3 -> 10.6, 2048 x 3072 x
 // 768 16.0 -> 12.4, 512 x 2048 x 2048 15.9 -> 13.7, 256 x 256 x 256 7.5 -> 5.0, 2048 x 6160 x 2048 37.6 -> 35.8, 4096 x 4096 x 4096 92.5 -> 92.6.  fp32 results with eight warps were
 // slower, with one buffer (2048 x 2048 x 2048 16.3 -> 16.7) or two and a shorter ring (2048 x 6160 x 2048 39.6 -> 41.4).

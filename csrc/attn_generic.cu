@@ -212,6 +212,96 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(LatentPrepParams p, co
   }
 }
 
+// The same where sizes and addresses allow 16-byte reads and a row fits the CTA's registers (queries of up to 512 QV columns with a norm, latents of up to 512
+// KV): everything is asked for at once and read once, both sums of squares meet in one exchange.
+// Bound: latencies (launch, one round of loads, one exchange), and bytes for thousands of tokens.  One B200, in a chain of itself, us, element by element and every row read twice
+// (above) -> this: 2048 tokens with 768 + 512 + 64 columns 9.0 -> 4.9, 1536 + 512 + 64 12.4 -> 5.8, 4000 with 2048 + 1024 + 64 32.2 -> 11.3, 2048 with 3072 columns without a norm 7.8
+// -> 6.7, 60 tokens 5.9 -> 2.2, one token 5.6 -> 2.1.
+constexpr int LP_THREADS = 128;
+template <typename T, int QV, int KV>
+__global__ void __launch_bounds__(LP_THREADS) latent_prep_vec_kernel(LatentPrepParams p, const T* __restrict__ wq, const T* __restrict__ wkv,
+                                                                     T* __restrict__ cq, T* __restrict__ cache) {
+  pdl_wait();                      // programmatic dependent launch: nothing is read before the predecessor is done
+  pdl_launch_dependents();
+  __shared__ float2 red[LP_THREADS / 32];
+  const int m = blockIdx.x, b = m / p.S, s = m % p.S, tid = threadIdx.x;
+  const float* yr = p.y + (size_t)m * p.ldy;
+  float qv[QV][4], kv[KV][4], wqv[QV][4], wkvv[KV][4];
+#pragma unroll
+  for (int u = 0; u < KV; ++u) {
+    const int i = min(4 * (tid + LP_THREADS * u), p.kv_rank - 4);
+    load4(yr + p.kv_off + i, kv[u]);
+    load4(wkv + i, wkvv[u]);
+  }
+  if (wq != nullptr) {
+#pragma unroll
+    for (int u = 0; u < QV; ++u) {
+      const int i = min(4 * (tid + LP_THREADS * u), p.q_rank - 4);
+      load4(yr + p.q_off + i, qv[u]);
+      load4(wq + i, wqv[u]);
+    }
+  }
+  const int slot = (p.cache_len ? *p.cache_len : 0) + s;
+  int pos = slot - (p.pad_left ? p.pad_left[b] : 0);
+  pos = pos < 0 ? 0 : (pos >= p.max_pos ? p.max_pos - 1 : pos);
+  T* row = cache + ((size_t)b * p.T + slot) * (p.kv_rank + p.rot_dim);
+  T* kr_out = p.kr_out ? (T*)p.kr_out + (size_t)m * p.rot_dim : nullptr;
+  for (int d = tid; d < p.rot_dim; d += LP_THREADS) {
+    const T v = from_f<T>(rotary_channel(yr + p.kv_off + p.kv_rank, d, p.rot, p.layout, p.cos_t + (size_t)pos * (p.rot / 2), p.sin_t + (size_t)pos * (p.rot / 2)));
+    row[p.kv_rank + d] = v;
+    if (kr_out) kr_out[d] = v;
+  }
+  if (wq == nullptr && p.q_rank > 0)
+    for (int i = 4 * tid; i < p.q_rank; i += 4 * LP_THREADS) {
+      float v[4];
+      load4(yr + p.q_off + i, v);
+      store4(cq + (size_t)m * p.q_rank + i, v);
+    }
+  float qs = 0.0f, ks = 0.0f;
+#pragma unroll
+  for (int u = 0; u < KV; ++u)
+    if (4 * (tid + LP_THREADS * u) < p.kv_rank)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ks += kv[u][e] * kv[u][e];
+  if (wq != nullptr)
+#pragma unroll
+    for (int u = 0; u < QV; ++u)
+      if (4 * (tid + LP_THREADS * u) < p.q_rank)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) qs += qv[u][e] * qv[u][e];
+  qs = warp_sum(qs);
+  ks = warp_sum(ks);
+  if ((tid & 31) == 0) red[tid >> 5] = make_float2(qs, ks);
+  __syncthreads();
+  qs = ks = 0.0f;
+#pragma unroll
+  for (int w = 0; w < LP_THREADS / 32; ++w) { qs += red[w].x; ks += red[w].y; }
+  const float rk = 1.0f / sqrtf(ks / (float)p.kv_rank + p.eps);
+  T* c_out = p.c_out ? (T*)p.c_out + (size_t)m * p.kv_rank : nullptr;
+#pragma unroll
+  for (int u = 0; u < KV; ++u) {
+    const int i = 4 * (tid + LP_THREADS * u);
+    if (i < p.kv_rank) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) kv[u][e] = kv[u][e] * rk * wkvv[u][e];
+      store4(row + i, kv[u]);
+      if (c_out) store4(c_out + i, kv[u]);
+    }
+  }
+  if (wq != nullptr) {
+    const float rq = 1.0f / sqrtf(qs / (float)p.q_rank + p.eps);
+#pragma unroll
+    for (int u = 0; u < QV; ++u) {
+      const int i = 4 * (tid + LP_THREADS * u);
+      if (i < p.q_rank) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) qv[u][e] = qv[u][e] * rq * wqv[u][e];
+        store4(cq + (size_t)m * p.q_rank + i, qv[u]);
+      }
+    }
+  }
+}
+
 // out[m, h, out_off + d] = rotary(in[m, h, in_off + d]), d < n: a slice of every head rotated at the token's position and
 // copied into another head layout (in / out head pitches in_hs / out_hs, row pitches ldi / ldo).
 template <typename T>
@@ -1112,8 +1202,20 @@ extern "C" JL_API int jl_latent_prep(const float* y, int ldy, int q_off, int q_r
   LatentPrepParams p{y, ldy, q_off, q_rank, kv_off, kv_rank, rot_dim, rot, layout, cos_t, sin_t, max_pos, eps, B, S, T_cap,
                      cache_len, pad_left, c_out, kr_out,
                      q_rank % 4 == 0 && ldy % 4 == 0 && q_off % 4 == 0 && (((uintptr_t)y | (uintptr_t)cq) % 16) == 0};
-  JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(latent_prep_kernel<T>, dim3(B * S), dim3(128), 0, (cudaStream_t)stream, p, (const T*)wq_norm,
-                                         (const T*)wkv_norm, (T*)cq, (T*)cache));
+  const int q_normed = wq_norm != nullptr ? q_rank : 0;
+  const bool vec = kv_rank % 4 == 0 && q_rank % 4 == 0 && rot_dim % 4 == 0 && ldy % 4 == 0 && (q_rank == 0 || q_off % 4 == 0) && kv_off % 4 == 0 &&
+                   (((uintptr_t)y | (uintptr_t)cq | (uintptr_t)cache | (uintptr_t)wq_norm | (uintptr_t)wkv_norm | (uintptr_t)c_out) & 15) == 0 &&
+                   (q_rank > 0 || wq_norm == nullptr);
+  const bool one = vec && q_normed <= 1024 && kv_rank <= 512, two = vec && q_normed <= 2048 && kv_rank <= 1024;
+  if (one)
+    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((latent_prep_vec_kernel<T, 2, 1>), dim3(B * S), dim3(LP_THREADS), 0, (cudaStream_t)stream, p, (const T*)wq_norm,
+                                           (const T*)wkv_norm, (T*)cq, (T*)cache));
+  else if (two)
+    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((latent_prep_vec_kernel<T, 4, 2>), dim3(B * S), dim3(LP_THREADS), 0, (cudaStream_t)stream, p, (const T*)wq_norm,
+                                           (const T*)wkv_norm, (T*)cq, (T*)cache));
+  else
+    JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL(latent_prep_kernel<T>, dim3(B * S), dim3(128), 0, (cudaStream_t)stream, p, (const T*)wq_norm,
+                                           (const T*)wkv_norm, (T*)cq, (T*)cache));
   JL_CUDA(cudaGetLastError());
   return JL_OK;
 }

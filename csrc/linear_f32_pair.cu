@@ -15,8 +15,9 @@
 // there is no second kernel.  A sum of more than LP_FOLD units is folded through the workspace on its way, because a long chain of additions costs precision.
 // Bound: 24 MMAs of 12 BN cycles together per unit, with the loads (64 KB per CTA and unit at BN 256) right behind.  One B200, single CTAs -> this, us (rows x features x
 // K): 200 x 10928 x 2048 153 -> 52 (1.0 PFLOP/s of bfloat16 products), 200 x 2048 x 5464 54 -> 33, 128 x 10928 x 2048 78 -> 38, 1000 x 1024 x 1024 31.5 -> 20.8, 2048 x 6176 x 1024
-// 263 -> 121, 2048 x 10928 x 2048 759 -> 395.  Error against float64 (2-norm), normal operands; one sign: 200 x 10928 x 2048 1.04e-7 -> 1.11e-7; 8.8e-8 -> 5.4e-8, 200 x
-// 2048 x 5464 1.25e-7 -> 1.15e-7; 9.9e-8 -> 5.8e-8, 2048 x 6176 x 1024 1.09e-7 -> 1.06e-7, 2048 x 10928 x 2048 1.31e-7 -> 1.28e-7, 400 x 512 x 512 9.2e-8 -> 9.0e-8; 8.8e-8 -> 4.1e-8.
+// 263 -> 121, 2048 x 10928 x 2048 759 -> 395.  Error against float64 (2-norm), normal operands; one sign: 200 x 10928 x 2048 1.04e-7 -> 1.13e-7; 9.6e-8 -> 1.02e-7, 200 x
+// 2048 x 5464 1.25e-7 -> 1.16e-7; 9.6e-8 -> 9.8e-8, 2048 x 6176 x 1024 1.09e-7 -> 1.07e-7; 1.07e-7 -> 1.04e-7, 2048 x 10928 x 2048 1.31e-7 -> 1.29e-7; 1.23e-7 -> 1.20e-7, 400 x 512 x 512
+// 9.2e-8 -> 9.2e-8; 9.5e-8 -> 9.5e-8.  (Sums are added as they come: a factor on them against the mean of what the tensor core cuts off would change those that are exact.)
 #include "jllama_b200.h"
 #include "linear_f32.cuh"
 #include "seq_types.cuh"
@@ -27,9 +28,6 @@ namespace jl {
 constexpr int LP_BM = 128, LP_BK = 64, LP_PROD = 8, LP_EPI = 8, LP_THREADS = (LP_PROD + LP_EPI) * 32;
 constexpr uint32_t LP_A_BYTES = LP_BM * LP_BK * 2;                   // one part of a CTA's weights
 constexpr int LP_STAGES = 2, LP_FOLD = 32;
-// The tensor core cuts off: a sum of 64 products is short by 2^-24 of itself in the mean.  Every second one is multiplied by 1 + 2^-23 where it is added (one FMA,
-// one rounding): mean error -6.1e-8 -> 0.
-constexpr float LP_UP = 1.00000011920928955f;
 constexpr uint32_t lp_stage_bytes(int bn) { return 3 * (LP_A_BYTES + bn / 2 * LP_BK * 2); }
 constexpr size_t lp_smem(int bn) { return LP_STAGES * lp_stage_bytes(bn) + 1024; }
 constexpr int LP_PROD_REGS = 104, LP_EPI_REGS = 152;                 // 256 threads each: together the 128 x 512 of the launch
@@ -208,7 +206,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LP_THREADS, 1) linea
     int tile = tile0, kb = kb0;
 #pragma unroll 1
     for (int u = 0; u < n; ++tile, kb = 0) {                         // the tiles of this run
-      const int kstart = kb, units = min(p.blocks - kb, n - u), odd = kb - u;
+      const int kstart = kb, units = min(p.blocks - kb, n - u);
       float* const fold = p.ws + ((size_t)pair * LP_SLOTS + 2) * lp_part(BN) + (size_t)half * HALF * (2 * LP_BM) + rank * LP_BM + feature;
       float acc[HALF];
 #pragma unroll 1
@@ -218,7 +216,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LP_THREADS, 1) linea
 #pragma unroll 1
         for (const int end = u + min(LP_FOLD, units - done); u < end; ++u) {
           const int buf = u & 1;
-          const float up = (odd + u) & 1 ? LP_UP : 1.0f;
           if (issuer && u + 1 < n) issue(u + 1);
           tc::mbar_wait(tfull(buf), (u >> 1) & 1);
           tc::fence_after_sync();
@@ -228,7 +225,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LP_THREADS, 1) linea
             tc::tmem_ld16(row + buf * 256 + c0, v);
             tc::tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) acc[c0 + j] = fmaf(__uint_as_float(v[j]), up, acc[c0 + j]);
+            for (int j = 0; j < 16; ++j) acc[c0 + j] += __uint_as_float(v[j]);
           }
           tc::fence_before_sync();
           __syncwarp();

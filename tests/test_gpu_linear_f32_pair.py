@@ -1,7 +1,7 @@
 """float32 linears on CTA pairs (csrc/linear_f32_pair.cu) at the edges of their tiles, runs and sums, against float64.
 
 Bound of an output, with A = sum |x w|: what the six products leave out (2^-24 A), what the tensor core cuts off (at most 2^-24 of the running sum at each
-of the 24 steps of 64 k, so 24 · 2^-24 A; half of it is put back), and the rounded additions of K / 64 sums, of the folds and of the parts (2^-24 A each)."""
+of the 24 steps of 64 k, so 24 · 2^-24 A), and the rounded additions of K / 64 sums, of the folds and of the parts (2^-24 A each)."""
 import pytest
 import torch
 
@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 from jax_llama_b200.ops import _lib  # noqa: E402
 from jax_llama_b200.ops import seq_kernels as SK  # noqa: E402
-from jax_llama_b200.ops.kernels import num_sms  # noqa: E402
+from jax_llama_b200.ops.kernels import _stream, num_sms  # noqa: E402
 
 
 def workspace(x, w):
@@ -36,6 +36,34 @@ def test_against_float64(M, N, K, positive):
     x, w = operands(M, N, K, positive=positive)
     assert workspace(x, w) >= 0                                # these sizes run the kernel under test
     check(SK.linear(x, w), x, w)
+
+
+# whole tiles; parts that meet in one or several tiles; sums of more than 32 x 64
+@pytest.mark.parametrize("M,N,K", [(300, 256, 256), (300, 512, 512), (200, 1100, 2048), (700, 257, 4228)])
+def test_sums_that_need_no_rounding_are_exact(M, N, K):
+    """One-hot rows and features (the one lies in every position of a block of 64 k, in even and odd blocks) give numbers back bit for bit; whole numbers whose
+    sums stay below 2^24 add up exactly, with partial sums that cancel."""
+    x, w = operands(M, N, K)
+    hot = torch.zeros(M, K, device="cuda")
+    at = torch.arange(M, device="cuda") * 61 % K
+    hot[torch.arange(M, device="cuda"), at] = 1.0
+    assert workspace(hot, w) >= 0
+    assert torch.equal(SK.linear(hot, w), w[:, at].T)
+    hot = torch.zeros(N, K, device="cuda")
+    at = torch.arange(N, device="cuda") * 67 % K
+    hot[torch.arange(N, device="cuda"), at] = 1.0
+    assert torch.equal(SK.linear(x, hot), x[:, at])
+    xi, wi = (x * 4).round(), (w * 4).round()
+    assert torch.equal(SK.linear(xi, wi).double(), xi.double() @ wi.double().T)
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 256, 256), (300, 256, 256)])
+def test_a_sum_that_one_pair_walks_alone_has_the_bits_of_the_single_ctas(M, N, K):
+    x, w = operands(M, N, K)
+    assert workspace(x, w) == 0                                # no runs that end inside a tile, no sums to fold
+    single, L = torch.empty(M, N, device="cuda"), _lib.lib()
+    _lib.check(L.jl_linear_any(x.data_ptr(), K, w.data_ptr(), single.data_ptr(), N, M, N, K, 0, 0.0, 0.0, 1, 1, _stream()), "jl_linear_any")
+    assert torch.equal(SK.linear(x, w), single)
 
 
 def test_same_bits_again_and_inside_a_wider_result():

@@ -275,23 +275,35 @@ bool linear_f32_takes(int M, int K, int ldx, const LinearGroup& g, const void* x
   return M > 8 && K >= 256 && K % 4 == 0 && ldx % 4 == 0 && g.x_bs % 4 == 0 && g.w_bs % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
 }
 
-cudaError_t linear_f32_launch(const float* x, int ldx, const float* w, float* out, int ldo, int M, int N, int K, int act, float p0, float p1,
-                              cudaStream_t st, const LinearGroup& g, int nbatch) {
-  // Rows per tile and parts of K: the least time of the busiest SM in cycles, from what a CTA takes per 64 k, to begin and end, and to
-  // meet its cluster (fitted to the times above and their neighbours; clusters of eight wait for a place).
+// Rows per tile and parts of K: the least time of the busiest SM in cycles, from what a CTA takes per 64 k, to begin and end, and to
+// meet its cluster (fitted to the times above and their neighbours; clusters of eight wait for a place).
+static void lf_plan(int M, int N, int K, int nbatch, bool sorted, int& bn, int& splits) {
   static const struct { int bn; double cycles; } shapes[] = {{32, 2000.0}, {64, 2300.0}, {128, 3400.0}};
   const int k_blocks = (K + LF_BK - 1) / LF_BK;
   double best = 1e300;
-  int bn = 64, splits = 1;
+  bn = 64;
+  splits = 1;
   for (const auto& sh : shapes) {
-    const long tiles = (long)((M + sh.bn - 1) / sh.bn) * ((N + LF_BM - 1) / LF_BM) * (g.tile_group ? 1 : nbatch);
-    if (g.tile_group && sh.bn > LT_BM) continue;
+    const long tiles = (long)((M + sh.bn - 1) / sh.bn) * ((N + LF_BM - 1) / LF_BM) * nbatch;
+    if (sorted && sh.bn > LT_BM) continue;
     for (int s = 1; s <= 8; s *= 2) {
       if (s > 1 && k_blocks / s < 2) break;
       const double t = (double)((tiles * s + SMS - 1) / SMS) * (4000.0 + sh.cycles * ((k_blocks + s - 1) / s) + (s == 1 ? 0.0 : s < 8 ? 5000.0 : 9000.0));
       if (t < best) { best = t; bn = sh.bn; splits = s; }
     }
   }
+}
+
+int linear_f32_chain(int M, int N, int K) {
+  int bn, splits;
+  lf_plan(M, N, K, 1, false, bn, splits);
+  return ((K + LF_BK - 1) / LF_BK + splits - 1) / splits;
+}
+
+cudaError_t linear_f32_launch(const float* x, int ldx, const float* w, float* out, int ldo, int M, int N, int K, int act, float p0, float p1,
+                              cudaStream_t st, const LinearGroup& g, int nbatch) {
+  int bn, splits;
+  lf_plan(M, N, K, g.tile_group ? 1 : nbatch, g.tile_group != nullptr, bn, splits);
   const LinearF32 p{x, w, out, ldx, ldo, M, N, K, act, splits, p0, p1, g};
   if (bn == 32) return lf_launch<32>(p, nbatch, st);
   if (bn == 64) return lf_launch<64>(p, nbatch, st);

@@ -12,12 +12,13 @@
 //   * 8 epilogue warps per CTA add the finished sum (two in TMEM, alternating) to their registers: a thread owns one feature of BN / 2 rows.
 // The (tile, 64 k) units of the whole product are dealt to the pairs in even runs, so that no round of tiles is incomplete: a run that ends
 // inside a tile leaves a partial tile in the workspace, and a second kernel adds a tile's parts in order of k.  Where whole tiles are as fast
-// there is no second kernel.  A sum of more than LP_FOLD units is folded through the workspace on its way, because a long chain of additions costs precision.
+// there is no second kernel.  A long chain of additions costs precision: what is more than LP_FOLD units, or than a CTA of linear_f32.cu adds in a row for the same product, is
+// folded through the workspace on its way.
 // Bound: 24 MMAs of 12 BN cycles together per unit, with the loads (64 KB per CTA and unit at BN 256) right behind.  One B200, single CTAs -> this, us (rows x features x
-// K): 200 x 10928 x 2048 153 -> 52 (1.0 PFLOP/s of bfloat16 products), 200 x 2048 x 5464 54 -> 33, 128 x 10928 x 2048 78 -> 38, 1000 x 1024 x 1024 31.5 -> 20.8, 2048 x 6176 x 1024
-// 263 -> 121, 2048 x 10928 x 2048 759 -> 395.  Error against float64 (2-norm), normal operands; one sign: 200 x 10928 x 2048 1.04e-7 -> 1.13e-7; 9.6e-8 -> 1.02e-7, 200 x
-// 2048 x 5464 1.25e-7 -> 1.16e-7; 9.6e-8 -> 9.8e-8, 2048 x 6176 x 1024 1.09e-7 -> 1.07e-7; 1.07e-7 -> 1.04e-7, 2048 x 10928 x 2048 1.31e-7 -> 1.29e-7; 1.23e-7 -> 1.20e-7, 400 x 512 x 512
-// 9.2e-8 -> 9.2e-8; 9.5e-8 -> 9.5e-8.  (Sums are added as they come: a factor on them against the mean of what the tensor core cuts off would change those that are exact.)
+// K): 200 x 10928 x 2048 153 -> 58 (52 with sums of 32 units), 200 x 2048 x 5464 54 -> 35, 128 x 10928 x 2048 78 -> 43, 1000 x 1024 x 1024 31.5 -> 22, 2048 x 6176 x 1024
+// 263 -> 128, 2048 x 10928 x 2048 759 -> 400.  Error against float64 (2-norm), normal operands; one sign: 200 x 10928 x 2048 1.04e-7 -> 1.05e-7 (1.13e-7 with sums of 32); 9.6e-8 -> 9.7e-8,
+// 200 x 2048 x 5464 1.25e-7 -> 1.16e-7; 9.6e-8 -> 9.8e-8, 2048 x 6176 x 1024 1.09e-7 -> 1.07e-7; 1.07e-7 -> 1.04e-7, 2048 x 10928 x 2048 1.31e-7 -> 1.29e-7; 1.23e-7 -> 1.20e-7,
+// 400 x 512 x 512 9.2e-8 -> 9.1e-8; 9.5e-8 -> 9.4e-8.  (Sums are added as they come: a factor on them against the mean of what the tensor core cuts off would change those that are exact.)
 #include "jllama_b200.h"
 #include "linear_f32.cuh"
 #include "seq_types.cuh"
@@ -36,6 +37,7 @@ struct LinearPair {
   const float* x; const float* w; float* out; float* ws;
   int ldx, ldo, M, N, K;
   int m_tiles, tiles, blocks, pairs, split;                          // blocks: of 64 k per tile; split: runs may end inside a tile
+  int fold;                                                          // most units that are added in a row
 };
 
 // first unit of a pair's run
@@ -207,14 +209,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LP_THREADS, 1) linea
 #pragma unroll 1
     for (int u = 0; u < n; ++tile, kb = 0) {                         // the tiles of this run
       const int kstart = kb, units = min(p.blocks - kb, n - u);
-      float* const fold = p.ws + ((size_t)pair * LP_SLOTS + 2) * lp_part(BN) + (size_t)half * HALF * (2 * LP_BM) + rank * LP_BM + feature;
+      float* const sofar = p.ws + ((size_t)pair * LP_SLOTS + 2) * lp_part(BN) + (size_t)half * HALF * (2 * LP_BM) + rank * LP_BM + feature;
       float acc[HALF];
 #pragma unroll 1
-      for (int done = 0; done < units; done += LP_FOLD) {            // sums of LP_FOLD units, which then meet
+      for (int done = 0; done < units; done += p.fold) {             // sums of `fold` units, which then meet
 #pragma unroll
         for (int j = 0; j < HALF; ++j) acc[j] = 0.0f;
 #pragma unroll 1
-        for (const int end = u + min(LP_FOLD, units - done); u < end; ++u) {
+        for (const int end = u + min(p.fold, units - done); u < end; ++u) {
           const int buf = u & 1;
           if (issuer && u + 1 < n) issue(u + 1);
           tc::mbar_wait(tfull(buf), (u >> 1) & 1);
@@ -233,11 +235,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LP_THREADS, 1) linea
         }
         if (done > 0) {
 #pragma unroll
-          for (int j = 0; j < HALF; ++j) acc[j] += fold[(size_t)j * (2 * LP_BM)];
+          for (int j = 0; j < HALF; ++j) acc[j] += sofar[(size_t)j * (2 * LP_BM)];
         }
-        if (done + LP_FOLD < units) {
+        if (done + p.fold < units) {
 #pragma unroll
-          for (int j = 0; j < HALF; ++j) fold[(size_t)j * (2 * LP_BM)] = acc[j];
+          for (int j = 0; j < HALF; ++j) sofar[(size_t)j * (2 * LP_BM)] = acc[j];
         }
       }
       if (units < p.blocks) {                                        // a part of the tile
@@ -315,6 +317,7 @@ __global__ void __launch_bounds__(LPS_THREADS) linear_f32_pair_sum_kernel(const 
 static double lp_plan(int M, int N, int K, int num_sms, LinearPair& p, int& bn) {
   static const int sizes[] = {128, 192, 224, 256};
   double best = 1e300;
+  p.fold = linear_f32_chain(M, N, K) < LP_FOLD ? linear_f32_chain(M, N, K) : LP_FOLD;
   for (int b : sizes) {
     const int mt = (M + b - 1) / b, tiles = mt * ((N + 2 * LP_BM - 1) / (2 * LP_BM)), blocks = (K + LP_BK - 1) / LP_BK;
     const double unit = b * 12.0 > 13.0 * (LP_BM + b / 2) ? b * 12.0 + 100 : 13.0 * (LP_BM + b / 2) + 100;
@@ -358,7 +361,7 @@ extern "C" JL_API long long jl_linear_f32_pair_ws(const void* x, int ldx, const 
   LinearPair p{};
   int bn = 0;
   lp_plan(M, N, K, num_sms, p, bn);
-  return p.split || p.blocks > LP_FOLD ? (long long)(p.pairs * LP_SLOTS * lp_part(bn) * sizeof(float)) : 0;
+  return p.split || p.blocks > p.fold ? (long long)(p.pairs * LP_SLOTS * lp_part(bn) * sizeof(float)) : 0;
 }
 
 extern "C" JL_API int jl_linear_f32_pair(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int num_sms, void* ws,
@@ -368,7 +371,7 @@ extern "C" JL_API int jl_linear_f32_pair(const void* x, int ldx, const void* w, 
   LinearPair p{};
   int bn = 0;
   lp_plan(M, N, K, num_sms, p, bn);
-  JL_CHECK_ARG((!p.split && p.blocks <= LP_FOLD) || (ws != nullptr && ((uintptr_t)ws & 15) == 0), "jl_linear_f32_pair: a workspace of 16-byte alignment is needed");
+  JL_CHECK_ARG((!p.split && p.blocks <= p.fold) || (ws != nullptr && ((uintptr_t)ws & 15) == 0), "jl_linear_f32_pair: a workspace of 16-byte alignment is needed");
   p.x = (const float*)x; p.w = (const float*)w; p.out = (float*)out; p.ws = (float*)ws;
   p.ldx = ldx; p.ldo = ldo; p.M = M; p.N = N; p.K = K;
   cudaStream_t st = (cudaStream_t)stream;

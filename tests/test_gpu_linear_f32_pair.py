@@ -66,6 +66,28 @@ def test_a_sum_that_one_pair_walks_alone_has_the_bits_of_the_single_ctas(M, N, K
     assert torch.equal(SK.linear(x, w), single)
 
 
+@pytest.mark.parametrize("M,N,K", [(300, 256, 256), (400, 512, 512), (65, 2048, 1024), (200, 10928, 2048), (200, 2048, 5464), (1000, 1024, 1024), (200, 2048, 11000)])
+@pytest.mark.parametrize("positive", [False, True])
+def test_error_in_the_mean(M, N, K, positive):
+    """2-norm of the error: 2^-23 of the result for what the six products leave out and the tensor core cuts off a block of 64 k (twice the 2^-24 that the latter
+    measures), and sqrt(K / 64) / 4 · 2^-24 for the rounded additions.  Without the smallest of the six products normal operands give 2^-19."""
+    x, w = operands(M, N, K, positive=positive)
+    assert workspace(x, w) >= 0
+    want = x.double() @ w.double().T
+    assert float((SK.linear(x, w).double() - want).norm() / want.norm()) <= 2.0 ** -24 * (2.0 + (K / 64) ** 0.5 / 4)
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 10928, 2048), (200, 10928, 2048), (200, 10928, 4228), (200, 2048, 5464), (200, 2048, 11000), (400, 512, 512), (2048, 6176, 1024)])
+@pytest.mark.parametrize("positive", [False, True])
+def test_error_is_not_above_the_single_ctas(M, N, K, positive):
+    """Sums of as many blocks in a row at most: the same mean error, but for the sums that meet elsewhere (3 %)."""
+    x, w = operands(M, N, K, positive=positive)
+    assert workspace(x, w) >= 0
+    single, L, want = torch.empty(M, N, device="cuda"), _lib.lib(), x.double() @ w.double().T
+    _lib.check(L.jl_linear_any(x.data_ptr(), K, w.data_ptr(), single.data_ptr(), N, M, N, K, 0, 0.0, 0.0, 1, 1, _stream()), "jl_linear_any")
+    assert float((SK.linear(x, w).double() - want).norm()) <= 1.03 * float((single.double() - want).norm())
+
+
 def test_same_bits_again_and_inside_a_wider_result():
     x, w = operands(200, 1100, 2048)
     first = SK.linear(x, w)

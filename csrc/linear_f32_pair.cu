@@ -272,17 +272,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LP_THREADS, 1) linea
   if (warp == LP_PROD) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
-// The tiles that several pairs took parts of: their sums, in order of k.  grid (BN / 16 groups of rows, tiles), a thread takes four features of four rows.
+// The tiles that several pairs took parts of: their sums, in order of k.  grid (tiles, BN / 16 groups of rows), a thread takes four features of four rows.
 constexpr int LPS_ROWS = 16, LPS_THREADS = 256;
 
 __global__ void __launch_bounds__(LPS_THREADS) linear_f32_pair_sum_kernel(const LinearPair p, int bn) {
   pdl_wait();
   pdl_launch_dependents();
-  const int tile = blockIdx.y;
+  const int tile = blockIdx.x;
   const long long total = (long long)p.tiles * p.blocks, u0 = (long long)tile * p.blocks, u1 = u0 + p.blocks - 1;
   const int p0 = (int)(((u0 + 1) * p.pairs - 1) / total), p1 = (int)(((u1 + 1) * p.pairs - 1) / total);      // owners of its first and last unit
   if (p0 == p1) return;                                              // written by one pair
-  const int c = (threadIdx.x & 63) * 4, r0 = blockIdx.x * LPS_ROWS + (threadIdx.x >> 6);
+  const int c = (threadIdx.x & 63) * 4, r0 = blockIdx.y * LPS_ROWS + (threadIdx.x >> 6);
   const int nf = tile / p.m_tiles * (2 * LP_BM) + c, m0 = tile % p.m_tiles * bn;
   const size_t part = lp_part(bn);
   const float* src = p.ws + (size_t)r0 * (2 * LP_BM) + c;
@@ -376,6 +376,6 @@ extern "C" JL_API int jl_linear_f32_pair(const void* x, int ldx, const void* w, 
   p.ldx = ldx; p.ldo = ldo; p.M = M; p.N = N; p.K = K;
   cudaStream_t st = (cudaStream_t)stream;
   JL_CUDA(bn == 128 ? lp_launch<128>(p, st) : bn == 192 ? lp_launch<192>(p, st) : bn == 224 ? lp_launch<224>(p, st) : lp_launch<256>(p, st));
-  if (p.split) JL_CUDA(launch_pdl(linear_f32_pair_sum_kernel, dim3(bn / LPS_ROWS, p.tiles), dim3(LPS_THREADS), 0, st, p, bn));
+  if (p.split) JL_CUDA(launch_pdl(linear_f32_pair_sum_kernel, dim3(p.tiles, bn / LPS_ROWS), dim3(LPS_THREADS), 0, st, p, bn));
   return JL_OK;
 }

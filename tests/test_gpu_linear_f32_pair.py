@@ -88,6 +88,16 @@ def test_error_is_not_above_the_single_ctas(M, N, K, positive):
     assert float((SK.linear(x, w).double() - want).norm()) <= 1.03 * float((single.double() - want).norm())
 
 
+def test_more_tiles_than_one_dimension_of_a_grid_takes():
+    M, N, K = 524368, 8192, 256                                # 65568 tiles of 256 x 256 in runs that end inside tiles: 17 GB of results
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    assert workspace(x, w) > 0
+    got = SK.linear(x, w)
+    for rows in (slice(0, 300), slice(260000, 260300), slice(M - 300, M)):
+        check(got[rows], x[rows], w)
+
+
 def test_same_bits_again_and_inside_a_wider_result():
     x, w = operands(200, 1100, 2048)
     first = SK.linear(x, w)

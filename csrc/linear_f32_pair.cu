@@ -38,14 +38,15 @@ struct LinearPair {
   int ldx, ldo, M, N, K;
   int m_tiles, tiles, blocks, pairs, split;                          // blocks: of 64 k per tile; split: runs may end inside a tile
   int fold;                                                          // most units that are added in a row
+  int slots;                                                         // partial tiles that a pair keeps in the workspace
 };
 
 // first unit of a pair's run
 __host__ __device__ __forceinline__ long long lp_begin(const LinearPair& p, int pair) {
   return p.split ? (long long)p.tiles * p.blocks * pair / p.pairs : (long long)p.blocks * ((long long)p.tiles * pair / p.pairs);
 }
-// floats of a partial tile; a pair leaves at most two (slot 0 continues a tile, slot 1 begins one) and keeps the sum so far of a long run in slot 2
-constexpr int LP_SLOTS = 3;
+// Floats of a partial tile.  Where runs end inside tiles a pair leaves at most two (slot 0 continues a tile, slot 1 begins one); where a run has more units of a tile than are
+// added in a row, the sum so far lies in its last slot.
 __host__ __device__ __forceinline__ size_t lp_part(int bn) { return (size_t)2 * LP_BM * bn; }
 
 __device__ __forceinline__ void lp_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
@@ -209,7 +210,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LP_THREADS, 1) linea
 #pragma unroll 1
     for (int u = 0; u < n; ++tile, kb = 0) {                         // the tiles of this run
       const int kstart = kb, units = min(p.blocks - kb, n - u);
-      float* const sofar = p.ws + ((size_t)pair * LP_SLOTS + 2) * lp_part(BN) + (size_t)half * HALF * (2 * LP_BM) + rank * LP_BM + feature;
+      float* const sofar = p.ws + ((size_t)(pair + 1) * p.slots - 1) * lp_part(BN) + (size_t)half * HALF * (2 * LP_BM) + rank * LP_BM + feature;
       float acc[HALF];
 #pragma unroll 1
       for (int done = 0; done < units; done += p.fold) {             // sums of `fold` units, which then meet
@@ -243,7 +244,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LP_THREADS, 1) linea
         }
       }
       if (units < p.blocks) {                                        // a part of the tile
-        float* o = p.ws + ((size_t)pair * LP_SLOTS + (kstart == 0)) * lp_part(BN) + (size_t)half * HALF * (2 * LP_BM) + rank * LP_BM + feature;
+        float* o = p.ws + ((size_t)pair * p.slots + (kstart == 0)) * lp_part(BN) + (size_t)half * HALF * (2 * LP_BM) + rank * LP_BM + feature;
 #pragma unroll
         for (int j = 0; j < HALF; ++j) o[(size_t)j * (2 * LP_BM)] = acc[j];
       } else {
@@ -288,11 +289,11 @@ __global__ void __launch_bounds__(LPS_THREADS) linear_f32_pair_sum_kernel(const 
   const float* src = p.ws + (size_t)r0 * (2 * LP_BM) + c;
   float4 s[LPS_ROWS / 4];
 #pragma unroll
-  for (int i = 0; i < LPS_ROWS / 4; ++i) s[i] = *reinterpret_cast<const float4*>(src + ((size_t)p0 * LP_SLOTS + 1) * part + (size_t)i * 4 * (2 * LP_BM));
+  for (int i = 0; i < LPS_ROWS / 4; ++i) s[i] = *reinterpret_cast<const float4*>(src + ((size_t)p0 * p.slots + 1) * part + (size_t)i * 4 * (2 * LP_BM));
   for (int q = p0 + 1; q <= p1; ++q) {
     float4 v[LPS_ROWS / 4];
 #pragma unroll
-    for (int i = 0; i < LPS_ROWS / 4; ++i) v[i] = *reinterpret_cast<const float4*>(src + (size_t)q * LP_SLOTS * part + (size_t)i * 4 * (2 * LP_BM));
+    for (int i = 0; i < LPS_ROWS / 4; ++i) v[i] = *reinterpret_cast<const float4*>(src + (size_t)q * p.slots * part + (size_t)i * 4 * (2 * LP_BM));
 #pragma unroll
     for (int i = 0; i < LPS_ROWS / 4; ++i) { s[i].x += v[i].x; s[i].y += v[i].y; s[i].z += v[i].z; s[i].w += v[i].w; }
   }
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(LPS_THREADS) linear_f32_pair_sum_kernel(const 
 
 // Rows per tile, and whether runs end inside tiles: the least time of the busiest pair.  A unit costs the longer of its MMAs and its loads (cycles); parts
 // are written, read and added in some 10000 cycles.
-static double lp_plan(int M, int N, int K, int num_sms, LinearPair& p, int& bn) {
+static void lp_plan(int M, int N, int K, int num_sms, LinearPair& p, int& bn) {
   static const int sizes[] = {128, 192, 224, 256};
   double best = 1e300;
   p.fold = linear_f32_chain(M, N, K) < LP_FOLD ? linear_f32_chain(M, N, K) : LP_FOLD;
@@ -334,7 +335,8 @@ static double lp_plan(int M, int N, int K, int num_sms, LinearPair& p, int& bn) 
       }
     }
   }
-  return best;
+  const long long run = p.split ? ((long long)p.tiles * p.blocks + p.pairs - 1) / p.pairs : p.blocks;      // most units of a tile in a run
+  p.slots = (p.split ? 2 : 0) + ((run < p.blocks ? run : p.blocks) > p.fold);
 }
 
 template <int BN>
@@ -361,7 +363,7 @@ extern "C" JL_API long long jl_linear_f32_pair_ws(const void* x, int ldx, const 
   LinearPair p{};
   int bn = 0;
   lp_plan(M, N, K, num_sms, p, bn);
-  return p.split || p.blocks > p.fold ? (long long)(p.pairs * LP_SLOTS * lp_part(bn) * sizeof(float)) : 0;
+  return (long long)((size_t)p.pairs * p.slots * lp_part(bn) * sizeof(float));
 }
 
 extern "C" JL_API int jl_linear_f32_pair(const void* x, int ldx, const void* w, void* out, int ldo, int M, int N, int K, int num_sms, void* ws,
@@ -371,7 +373,7 @@ extern "C" JL_API int jl_linear_f32_pair(const void* x, int ldx, const void* w, 
   LinearPair p{};
   int bn = 0;
   lp_plan(M, N, K, num_sms, p, bn);
-  JL_CHECK_ARG((!p.split && p.blocks <= p.fold) || (ws != nullptr && ((uintptr_t)ws & 15) == 0), "jl_linear_f32_pair: a workspace of 16-byte alignment is needed");
+  JL_CHECK_ARG(p.slots == 0 || (ws != nullptr && ((uintptr_t)ws & 15) == 0), "jl_linear_f32_pair: a workspace of 16-byte alignment is needed");
   p.x = (const float*)x; p.w = (const float*)w; p.out = (float*)out; p.ws = (float*)ws;
   p.ldx = ldx; p.ldo = ldo; p.M = M; p.N = N; p.K = K;
   cudaStream_t st = (cudaStream_t)stream;

@@ -28,9 +28,10 @@ def check(got, x, w):
     assert bool(((got.double() - want).abs() <= 2.0 ** -24 * (24 + 8 + K / 64) * size).all())
 
 
-# rows at the edges of the tiles of 128, 192, 224 and 256; features and K off them; runs inside one tile, over several, whole tiles only; sums of more than 32 x 64
+# rows at the edges of the tiles of 128, 192, 224 and 256; features and K off them; runs inside one tile, over several, whole tiles only; sums of more than 32 x 64 (the last: of
+# whole tiles)
 @pytest.mark.parametrize("M,N,K", [(65, 2048, 1024), (128, 2050, 1028), (129, 1024, 1024), (192, 4097, 260), (193, 1031, 1100), (200, 5464, 2048), (224, 1025, 2052),
-                                   (225, 2048, 5464), (257, 256, 256), (300, 777, 256), (449, 512, 2116), (700, 257, 4228), (1025, 300, 300), (2000, 3001, 1024)])
+                                   (225, 2048, 5464), (257, 256, 256), (300, 777, 256), (449, 512, 2116), (700, 257, 4228), (1025, 300, 300), (2000, 3001, 1024), (18944, 256, 4096)])
 @pytest.mark.parametrize("positive", [False, True])
 def test_against_float64(M, N, K, positive):
     x, w = operands(M, N, K, positive=positive)

@@ -6,11 +6,13 @@ never a silent fall back to PyTorch ops.
 from __future__ import annotations
 
 import ctypes as C
+import logging
 import os
 from typing import Optional
 
 from .build import LIB_PATH, build_library
 
+logger = logging.getLogger(__name__)
 _lib: Optional[C.CDLL] = None
 
 vp, ip, fp = C.c_void_p, C.c_void_p, C.c_void_p   # all pointers travel as integers from tensor.data_ptr()
@@ -196,7 +198,11 @@ def _bind(handle: C.CDLL) -> None:
     import importlib.machinery
     import importlib.util
     spec = importlib.util.spec_from_loader("_jl_binding", importlib.machinery.ExtensionFileLoader("_jl_binding", str(path)))
-    module = importlib.util.module_from_spec(spec)
+    try:
+        module = importlib.util.module_from_spec(spec)
+    except ImportError as e:
+        logger.warning("no built-in entry points, ctypes is used instead: %s", e)
+        return
     known = {name: getattr(handle, name) for name in {**_SIGNATURES, **_HYBRID, **_OPTIONAL} if hasattr(handle, name)}
     for name, fn in module.bind(handle._handle, known).items():
         setattr(handle, name, fn)

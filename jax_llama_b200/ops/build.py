@@ -6,6 +6,7 @@ package directory so that it travels with the source tree to the GPU box.
 """
 from __future__ import annotations
 
+import contextlib
 import hashlib
 import logging
 import os
@@ -161,33 +162,40 @@ def binding_path() -> Path:
 
 
 def build_binding(force: bool = False) -> Optional[Path]:
-    """Compile csrc/binding.cc for this interpreter; None where its headers or a C++ compiler are missing (the entry points are then called
-    through ctypes, with the same results)."""
+    """Compile csrc/binding.cc for this interpreter.  None where that is not possible or not wanted (no interpreter headers, no compiler or one that refuses, a folder
+    that cannot be written, JLLAMA_NO_AUTOBUILD): the entry points are then called through ctypes, with the same results.  An installed package
+    without the sources takes the binding that came with its library."""
     import sysconfig
     out, src = binding_path(), CSRC / "binding.cc"
     include = Path(sysconfig.get_paths()["include"])
-    h = hashlib.sha256()
-    for f in (src, INCLUDE / "jllama_b200.h"):
-        h.update(f.read_bytes())
-    h.update(sys.version.encode())
     stamp = out.with_suffix(".stamp")
-    if not force and out.exists() and stamp.exists() and stamp.read_text().strip() == h.hexdigest():
-        return out
-    if not (include / "Python.h").exists():
-        return None
-    OUT_DIR.mkdir(parents=True, exist_ok=True)
     tmp = out.with_suffix(f".tmp{os.getpid()}.so")
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-I{include}", f"-I{INCLUDE}", str(src), "-o", str(tmp)]
     try:
+        if not src.exists():
+            return out if out.exists() else None
+        h = hashlib.sha256()
+        for f in (src, INCLUDE / "jllama_b200.h"):
+            h.update(f.read_bytes())
+        h.update(sys.version.encode())
+        if not force and out.exists() and stamp.exists() and stamp.read_text().strip() == h.hexdigest():
+            return out
+        if os.environ.get("JLLAMA_NO_AUTOBUILD") or not (include / "Python.h").exists():
+            return None
+        OUT_DIR.mkdir(parents=True, exist_ok=True)
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-I{include}", f"-I{INCLUDE}", str(src), "-o", str(tmp)]
         r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            logger.warning("%s failed for %s, ctypes is used instead:\n%s", cmd[0], src.name, r.stderr)
+            return None
+        os.replace(tmp, out)
+        stamp.write_text(h.hexdigest() + "\n")
+        return out
     except OSError as e:
-        logger.warning("no C++ compiler for %s: %s", src.name, e)
+        logger.warning("no built-in entry points, ctypes is used instead: %s", e)
         return None
-    if r.returncode != 0:
-        raise RuntimeError(f"{cmd[0]} failed for {src.name}:\n{r.stderr}")
-    os.replace(tmp, out)
-    stamp.write_text(h.hexdigest() + "\n")
-    return out
+    finally:
+        with contextlib.suppress(OSError):
+            tmp.unlink(missing_ok=True)
 
 
 if __name__ == "__main__":

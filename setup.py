@@ -15,8 +15,9 @@ class build_cuda(Command):
         pass
 
     def run(self):
-        from jax_llama_b200.ops.build import build_library
+        from jax_llama_b200.ops.build import build_binding, build_library
         build_library(force=bool(self.force), verbose=True)
+        build_binding(force=bool(self.force))
 
 
 class build_py_with_cuda(build_py):

@@ -1,6 +1,10 @@
 """The host side of a kernel call: the built-in form of the entry points (csrc/binding.cc) beside ctypes', and the room of a layer's intermediates (ops/scratch.py).
 What is called here computes on the host; nothing needs a GPU."""
 import ctypes as C
+import os
+import shutil
+import subprocess
+import sys
 import threading
 
 import pytest
@@ -63,6 +67,56 @@ def test_numbers_arrive_as_declared(pair):
     args = lambda eps: (0, None, 0, 0, None, 0, 5, eps, 0)       # noqa: E731  jl_rmsnorm with M = 0 rows
     for eps in (1, 1e-5, True):
         assert fast.jl_rmsnorm(*args(eps)) == slow.jl_rmsnorm(*args(eps))
+
+
+def _loaded(folder, **env):
+    """What a new process that finds the package in `folder` says of an entry point's form."""
+    code = "from jax_llama_b200.ops import _lib; f = _lib.lib(); print(type(f.jl_gemm).__name__, f.jl_attn_generic_splits(1, 16, 4, 4096))"
+    kept = {k: v for k, v in os.environ.items() if not k.startswith("JLLAMA_")}
+    r = subprocess.run([sys.executable, "-c", code], cwd=folder, env={**kept, "PYTHONPATH": str(folder), **env}, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return r.stdout.split()
+
+
+@pytest.fixture
+def installed(tmp_path, pair):
+    """The package as an installation has it: its folder with the libraries (no stamps), neither csrc nor include."""
+    shutil.copytree(build.ROOT / "jax_llama_b200", tmp_path / "jax_llama_b200", ignore=shutil.ignore_patterns("_C", "__pycache__"))
+    libs = tmp_path / "jax_llama_b200" / "ops" / "_C"
+    libs.mkdir()
+    for so in (build.LIB_PATH, build.binding_path()):
+        (libs / so.name).symlink_to(so)
+    return tmp_path
+
+
+def test_an_installed_package_without_sources_loads(installed, pair):
+    splits = str(pair[1].jl_attn_generic_splits(1, 16, 4, 4096))
+    assert _loaded(installed, JLLAMA_NO_AUTOBUILD="1") == ["builtin_function_or_method", splits]      # the binding that came with the library
+    lib = installed / "jax_llama_b200" / "ops" / "_C" / build.LIB_PATH.name
+    (installed / "another.so").symlink_to(build.LIB_PATH)
+    assert _loaded(installed, JLLAMA_LIB=str(installed / "another.so")) == ["builtin_function_or_method", splits]
+    (lib.parent / build.binding_path().name).unlink()
+    assert _loaded(installed, JLLAMA_NO_AUTOBUILD="1") == ["_FuncPtr", splits]
+    (lib.parent / build.binding_path().name).write_bytes(b"not a library")
+    assert _loaded(installed, JLLAMA_NO_AUTOBUILD="1") == ["_FuncPtr", splits]
+
+
+def test_a_binding_that_cannot_be_built_is_not_an_error(tmp_path, monkeypatch, caplog):
+    ran = tmp_path / "ran"
+    compiler = tmp_path / "cxx"
+    compiler.write_text(f"#!/bin/sh\ntouch {ran}\nexit 1\n")
+    compiler.chmod(0o755)
+    monkeypatch.setenv("CXX", str(compiler))
+    monkeypatch.setattr(build, "OUT_DIR", tmp_path / "out")
+    monkeypatch.setenv("JLLAMA_NO_AUTOBUILD", "1")
+    assert build.build_binding() is None and not ran.exists()                 # nothing is compiled where that is switched off
+    monkeypatch.delenv("JLLAMA_NO_AUTOBUILD")
+    assert build.build_binding() is None and ran.exists() and "ctypes" in caplog.text
+    monkeypatch.setenv("CXX", str(tmp_path / "none"))
+    assert build.build_binding() is None                                      # no compiler
+    (tmp_path / "file").write_text("")
+    monkeypatch.setattr(build, "OUT_DIR", tmp_path / "file" / "out")
+    assert build.build_binding() is None                                      # no folder to write to
 
 
 CPU = torch.device("cpu")

@@ -127,7 +127,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, act: int = ACT_NONE, p0: float =
     _need(w, x.dtype, "w")
     N, K = w.shape
     M = x.numel() // K
-    if (x.dim() != 2 or x.shape[1] != K) and x.is_contiguous():
+    if (x.dim() != 2 or x.shape[1] != K or x.stride(0) != K) and x.is_contiguous():      # (a single row has any pitch)
         x = x.view(M, K)
     odt = torch.float32 if out_f32 else x.dtype
     if out is None:

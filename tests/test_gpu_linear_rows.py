@@ -234,3 +234,15 @@ def test_early_and_late_decode_rows_have_the_same_bits(M, N, K):
         graph.replay()
         assert torch.equal(out, late)
         check(late, x, w)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("K", [64, 77, 1024])
+def test_a_single_row_of_any_pitch(dtype, K):
+    """A column read as a row, a row repeated with pitch 0, the first row of a wide matrix: contiguous for torch, whatever the pitch of their one row says."""
+    x, w = torch.randn(K, 1, device="cuda").to(dtype), torch.randn(96, K, device="cuda").to(dtype)
+    want = SK.linear(x.view(1, K).clone(), w)
+    wide = torch.randn(3, K + 5, device="cuda").to(dtype)
+    wide[:1, :K] = x.t()
+    for row in (x.t(), x.view(K).as_strided((1, K), (0, 1)), wide[:1, :K]):
+        assert row.is_contiguous() and row.stride(0) != K and torch.equal(SK.linear(row, w), want)

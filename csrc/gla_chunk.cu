@@ -1,4 +1,4 @@
-// Prompts of the linear recurrences S_t = diag(alpha_t) S_(t-1) + k_t v_tᵀ, o_t = S_tᵀ q_t, 64 tokens at a time on the tensor cores, with fp32 accuracy.
+// Prompts of gated linear attention S_t = diag(alpha_t) S_(t-1) + k_t v_tᵀ, o_t = S_tᵀ q_t with projected decays, 64 tokens at a time on the tensor cores, with fp32 accuracy.
 //
 // Within a chunk that starts from the state S, with A_i = alpha_1 ... alpha_i per key channel,
 //     o_i = (A_i q_i)·S + sum_{j<=i} P_ij v_j,     P_ij = sum_d q_i[d] k_j[d] alpha_(j+1)[d] ... alpha_i[d],
@@ -17,8 +17,6 @@
 // (gla_scan.cu) -> this, all launches of the scan: 2048 tokens x 16 heads of 64 x 128 124 -> 72 (a layer of width 2048 199 -> 149), 2 rows x 1000 120 -> 69, 500 99 -> 31, 4 rows x
 // 512 x 8 heads of 32 x 64 65 -> 34, 4 rows x 128 x 16 heads of 128 x 128 100 -> 55.  Error against float64 (2-norm of the read-outs; of the state), the decays' own included: 65 tokens
 // 3.1e-7; 4.0e-7 -> 2.4e-7; 3.5e-7, 500 1.9e-6; 2.9e-6 -> 1.8e-6; 2.8e-6, 2048 7.0e-6; 1.05e-5 -> 6.7e-6; 1.01e-5.
-#include <type_traits>
-
 #include "gla_scan.cuh"
 #include "jllama_b200.h"
 #include "linear_f32.cuh"
@@ -37,40 +35,16 @@ __host__ __device__ constexpr int gc_b(int q) { return 0x001102 >> (4 * q) & 15;
 
 struct GlaChunk {
   GlaParams p;
-  float* alpha;                        // [B*S][H][D], where the decays are projected
+  float* alpha;                        // [B*S][H][D]
 };
 
 __device__ __forceinline__ int gc_first(const GlaParams& p, int b) { return max(0, (p.pad_left ? p.pad_left[b] : 0) - (p.cache_len ? *p.cache_len : 0)); }
 
-// the decay of a token and channel, once alpha is there
-__device__ __forceinline__ float gc_alpha(const GlaChunk& c, size_t m, int h, int d) {
-  const GlaParams& p = c.p;
-  return p.aux ? p.aux[m * p.ld_aux + h] : p.head_decay ? p.head_decay[h] : c.alpha[(m * p.H + h) * p.D + d];
-}
-// Rotated or activated q, k and v: called, not inlined, and every loop around them short (these kernels run through their code once or a few times per
-// SM; the first version's 130 KB of unrolled code took 10 us a kernel to arrive)
-static __device__ __noinline__ float2 gc_qk_any(const GlaParams* p, size_t m, int h, int d, int pos) {
-  float2 r;
-  scan_qk(*p, m, h, d, pos, r.x, r.y);
-  return r;
-}
-static __device__ __noinline__ float gc_value_any(const GlaParams* p, size_t m, int h, int c) { return scan_value(*p, m, h, c); }
-
-// PLAIN: q, k and v neither rotated nor activated
-template <bool PLAIN>
-__device__ __forceinline__ float2 gc_qk(const GlaParams& p, size_t m, int b, int t, int h, int d) {
-  if constexpr (!PLAIN) return gc_qk_any(&p, m, h, d, scan_position(p, b, t));
-  const float* row = p.y + m * p.ldy + (p.qk_div > 1 ? h / p.qk_div : h) * p.D + d;
+__device__ __forceinline__ float2 gc_qk(const GlaParams& p, size_t m, int h, int d) {
+  const float* row = p.y + m * p.ldy + h * p.D + d;
   return make_float2(row[p.q_off] * p.q_scale, row[p.k_off] * p.k_scale);
 }
-template <bool PLAIN>
-__device__ __forceinline__ float gc_value(const GlaParams& p, size_t m, int h, int c) {
-  if constexpr (!PLAIN) return gc_value_any(&p, m, h, c);
-  if (c >= p.Dv) return 0.0f;
-  const int dv = p.Dv - p.ones;
-  const float v = c < dv ? p.y[m * p.ldy + p.v_off + h * dv + c] : 1.0f;
-  return p.aux ? v * p.aux[m * p.ld_aux + p.H + h] : v;
-}
+__device__ __forceinline__ float gc_value(const GlaParams& p, size_t m, int h, int c) { return c < p.Dv ? p.y[m * p.ldy + p.v_off + h * p.Dv + c] : 0.0f; }
 
 __device__ __forceinline__ void gc_store16(uint32_t at, const uint4& v) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
@@ -121,7 +95,7 @@ struct GcTile {
   }
 };
 
-template <typename T, int DB, bool PLAIN>
+template <typename T, int DB>
 __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_kernel(const __grid_constant__ GlaChunk g, const T* __restrict__ a2,
                                                                         const T* __restrict__ a2b, int wide) {
   const GlaParams& p = g.p;
@@ -144,7 +118,6 @@ __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_k
   const int rows = min(GC_T, p.S - t0);                                     // tokens of the chunk that exist
   const int lo = max(0, first - t0), hi = rows;                             // ... that are real
   const size_t m0 = (size_t)b * p.S + t0;
-  const bool projected = p.aux == nullptr && p.head_decay == nullptr;
   GcTile values;
   values.load(wide != 0, p.y + m0 * p.ldy + p.v_off + h * p.Dv + c0, p.ldy, rows, p.Dv - c0);
   const int quarter = tid >> 6, dl = tid & 63;                              // a thread has one channel of 16 tokens
@@ -167,14 +140,14 @@ __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_k
         wr[i] = r < p.R ? to_f(a2[(size_t)(h * p.D + min(db * 64 + t, p.D - 1)) * p.R + r]) : 0.0f;
       }
     };
-    if (projected) ask(0);
+    ask(0);
     float v[16];
 #pragma unroll
     for (int t = 0; t < 16; ++t) {
       const int s = min(quarter * 16 + t, rows - 1);
-      v[t] = gc_qk<PLAIN>(p, m0 + s, b, t0 + s, h, dc).y;
+      v[t] = gc_qk(p, m0 + s, h, dc).y;
     }
-    if (projected) {
+    {
       float a[16];
       const float bias = to_f(a2b[h * p.D + dc]);
 #pragma unroll
@@ -198,16 +171,11 @@ __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_k
       }
 #pragma unroll
       for (int t = 0; t < 16; ++t) at[t * 64] = a[t];
-    } else {
-      const float* decay = p.aux ? p.aux + m0 * p.ld_aux + h : p.head_decay + h;
-      const int step = p.aux ? p.ld_aux : 0;
-#pragma unroll
-      for (int t = 0; t < 16; ++t) at[t * 64] = decay[(size_t)min(quarter * 16 + t, rows - 1) * step];
     }
 #pragma unroll
     for (int t = 0; t < 16; ++t) kt[t * 64] = v[t];
     if (db == 0) {
-      values.put(sv, wide != 0, p.Dv - c0, lo, hi, [&](int row, int c) { return gc_value<PLAIN>(p, m0 + row, h, c0 + c); });
+      values.put(sv, wide != 0, p.Dv - c0, lo, hi, [&](int row, int c) { return gc_value(p, m0 + row, h, c0 + c); });
       __syncthreads();
       pdl_launch_dependents();                                              // (this CTA has its tensor memory)
     }
@@ -217,11 +185,8 @@ __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_k
     for (int t = 15; t >= 0; --t) {
       const int s = quarter * 16 + t;
       const bool in = s >= lo && s < hi && d < p.D;
-      float a = at[t * 64];
-      if (projected) {
-        a = expf(log_sigmoid(a) * p.inv_tau);
-        if (in && c0 == 0) g.alpha[((m0 + s) * p.H + h) * p.D + d] = a;
-      }
+      const float a = expf(log_sigmoid(at[t * 64]) * p.inv_tau);
+      if (in && c0 == 0) g.alpha[((m0 + s) * p.H + h) * p.D + d] = a;
       kt[t * 64] = in ? kt[t * 64] * all : 0.0f;
       if (in) all *= a;
     }
@@ -294,15 +259,15 @@ __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_k
 #pragma unroll 1
           for (int t = lo; t < hi; ++t) {
             float a;
-            if (projected && c0 > 0) {                          // (the first slice's CTAs may not have stored them yet)
+            if (c0 > 0) {                                       // (the first slice's CTAs may not have stored them yet)
               const int n = h * p.D + d;
               a = to_f(a2b[n]);
               for (int r = 0; r < p.R; ++r) a = fmaf(to_f(a2[(size_t)n * p.R + r]), p.y[(m0 + t) * p.ldy + p.a_off + r], a);
               a = expf(log_sigmoid(a) * p.inv_tau);
             } else {
-              a = gc_alpha(g, m0 + t, h, d);
+              a = g.alpha[((m0 + t) * p.H + h) * p.D + d];
             }
-            s = fmaf(a, s, gc_qk<PLAIN>(p, m0 + t, b, t0 + t, h, d).y * gc_value<PLAIN>(p, m0 + t, h, c));
+            s = fmaf(a, s, gc_qk(p, m0 + t, h, d).y * gc_value(p, m0 + t, h, c));
           }
           out[(size_t)d * p.Dv] = s;
         }
@@ -336,7 +301,6 @@ struct GcOut {
   static_assert(6 * LEVEL >= GC_V_BYTES, "state and values in the factors' place");
 };
 
-template <bool PLAIN>
 __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_out_kernel(const __grid_constant__ GlaChunk g, int wide) {
   const GlaParams& p = g.p;
   using L = GcOut;
@@ -394,16 +358,14 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_out_kernel(const __gr
 #pragma unroll 1
   for (int db = 0; db < blocks; ++db) {
     const int d = db * 64 + dl, dc = min(d, p.D - 1);
-    // the decay of (token, channel) as one strided load, wherever it lies
-    const float* decay = p.aux ? p.aux + m0 * p.ld_aux + h : p.head_decay ? p.head_decay + h : g.alpha + (m0 * p.H + h) * p.D + dc;
-    const int decay_step = p.aux ? p.ld_aux : p.head_decay ? 0 : p.H * p.D;
+    const float* decay = g.alpha + (m0 * p.H + h) * p.D + dc;
     float q[16], k[16], a[16];
 #pragma unroll
     for (int t = 0; t < 16; ++t) {
       const int s = min(quarter * 16 + t, rows - 1);
-      const float2 v = gc_qk<PLAIN>(p, m0 + s, b, t0 + s, h, dc);
+      const float2 v = gc_qk(p, m0 + s, h, dc);
       q[t] = v.x; k[t] = v.y;
-      a[t] = decay[(size_t)s * decay_step];
+      a[t] = decay[(size_t)s * p.H * p.D];
     }
     float p0 = 1.0f, p1 = 1.0f;                                             // decays of the first and the last eight tokens
 #pragma unroll
@@ -552,7 +514,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_out_kernel(const __gr
   }
   tile.load(wide != 0, p.y + m0 * p.ldy + p.v_off + h * p.Dv + c0, p.ldy, rows, p.Dv - c0);      // the values
   finished();                                                               // (and every thread has seen this phase of the barrier before the next can end)
-  tile.put(base + L::W, wide != 0, p.Dv - c0, lo, hi, [&](int row, int c) { return gc_value<PLAIN>(p, m0 + row, h, c0 + c); });
+  tile.put(base + L::W, wide != 0, p.Dv - c0, lo, hi, [&](int row, int c) { return gc_value(p, m0 + row, h, c0 + c); });
 #pragma unroll
   for (int i = 0; i < 2; ++i) {                                             // P [64][64] -> three K-major tiles
     const int row = tid / 8 + 32 * i, c = tid % 8;
@@ -596,12 +558,12 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_out_kernel(const __gr
       for (int d = 0; d < p.D; ++d) st[d] = s_in[(size_t)d * p.Dv + c];
 #pragma unroll 1
       for (int t = lo; t < min(s0 + 32, hi); ++t) {
-        const float v = gc_value<PLAIN>(p, m0 + t, h, c);
+        const float v = gc_value(p, m0 + t, h, c);
         float acc = 0.0f;
 #pragma unroll 1
         for (int d = 0; d < p.D; ++d) {
-          const float2 qk = gc_qk<PLAIN>(p, m0 + t, b, t0 + t, h, d);
-          st[d] = fmaf(gc_alpha(g, m0 + t, h, d), st[d], qk.y * v);
+          const float2 qk = gc_qk(p, m0 + t, h, d);
+          st[d] = fmaf(g.alpha[((m0 + t) * p.H + h) * p.D + d], st[d], qk.y * v);
           acc = fmaf(qk.x, st[d], acc);
         }
         if (t >= s0 && !(fabsf(out[t * step]) < INFINITY)) out[t * step] = acc;
@@ -617,8 +579,10 @@ static int gc_chunks(int S) { return (S + GC_T - 1) / GC_T; }
 
 // Up to 128 key channels, from the tokens on where three launches of parallel chunks beat the walk of gla_scan.cu.  us, walk -> this: D 64 x Dv 128, projected decays: 1
 // row x 16 heads 40 tokens 21.8 -> 23.3, 48 24.2 -> 23.6, 64 30.0 -> 23.5, 2 rows 40 31.1 -> 24.4, 64 60.9 -> 24.6; 4 rows x 16 heads of 32 x 64, 48 tokens 26.8 -> 23.2;
-// 128 x 128: 1 row x 4 heads 64 tokens 35.5 -> 39.2, 200 61.7 -> 40.1, 4 rows x 8 heads 40 39.9 -> 41.6, 48 52.7 -> 41.8.  One fixed decay per head: 1 x 16 heads of 64 x 128,
-// 48 tokens 26.3 -> 20.3.
+// 128 x 128: 1 row x 4 heads 64 tokens 35.5 -> 39.2, 200 61.7 -> 40.1, 4 rows x 8 heads 40 39.9 -> 41.6, 48 52.7 -> 41.8.  Decays that are given (one per head or per token and head)
+// always walk: nothing of their own covers what the tensor core cuts off and the roundings of products of 64 decays.  Error against float64 (2-norm of the read-outs), walk -> this:
+// one fixed decay of 0.9, operands of one sign, 500 tokens x 16 heads of 64 x 128 4.1e-8 -> 9.4e-8, decay 1 4.7e-8 -> 1.4e-7; a float32 retention layer of 3 x 608 tokens, its
+// state 1.18e-6 -> 1.49e-6.
 bool gla_chunk_takes(int B, int S, int H, int D, int Dv) {
   return D <= 128 && S >= (D <= 64 || B * H >= 32 ? 48 : 80) && (long)H * ((Dv + GC_DV - 1) / GC_DV) <= 65535 && B <= 65535;
 }
@@ -628,25 +592,17 @@ size_t gla_chunk_ws_floats(int B, int S, int H, int D, int Dv) {
   return states * Dv + (states + 3) / 4 * 4 + (size_t)B * S * H * D;
 }
 
-template <int DB, bool PLAIN>
+template <int DB>
 static int gc_launch(const GlaChunk& g, const void* a2, const void* a2_bias, int dtype, int wide, cudaStream_t st) {
   const GlaParams& p = g.p;
   const dim3 grid(p.NC, p.H * ((p.Dv + GC_DV - 1) / GC_DV), p.B);
   const size_t smem = GC_V_BYTES + DB * GC_K_BYTES + 2 * GC_T * 64 * 4 + 1024;
-  auto state = [&](auto* w, auto* bias) {
-    using T = std::remove_const_t<std::remove_pointer_t<decltype(w)>>;
-    JL_CUDA(cudaFuncSetAttribute((gla_chunk_state_kernel<T, DB, PLAIN>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    JL_CUDA(launch_pdl((gla_chunk_state_kernel<T, DB, PLAIN>), grid, dim3(GC_THREADS), smem, st, g, w, bias, wide));
-    return JL_OK;
-  };
-  int rc = JL_OK;
-  if constexpr (PLAIN) JL_DISPATCH_DTYPE(dtype, rc = state((const T*)a2, (const T*)a2_bias));
-  else rc = state((const float*)nullptr, (const float*)nullptr);             // (rotated or activated: fixed decays)
-  if (rc) return rc;
-  JL_CUDA(cudaFuncSetAttribute(gla_chunk_out_kernel<PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GcOut::BYTES));
+  JL_DISPATCH_DTYPE(dtype, JL_CUDA(cudaFuncSetAttribute((gla_chunk_state_kernel<T, DB>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                    JL_CUDA(launch_pdl((gla_chunk_state_kernel<T, DB>), grid, dim3(GC_THREADS), smem, st, g, (const T*)a2, (const T*)a2_bias, wide)));
+  JL_CUDA(cudaFuncSetAttribute(gla_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GcOut::BYTES));
   const size_t total = (size_t)p.B * p.H * p.D * p.Dv;
   JL_CUDA(launch_pdl(gla_combine_kernel, dim3((unsigned)((total + 255) / 256 < 1184 ? (total + 255) / 256 : 1184)), dim3(256), 0, st, p));
-  JL_CUDA(launch_pdl(gla_chunk_out_kernel<PLAIN>, grid, dim3(GC_THREADS), GcOut::BYTES, st, g, wide));
+  JL_CUDA(launch_pdl(gla_chunk_out_kernel, grid, dim3(GC_THREADS), GcOut::BYTES, st, g, wide));
   return JL_OK;
 }
 
@@ -657,10 +613,8 @@ int gla_chunk_launch(GlaParams p, const void* a2, const void* a2_bias, float* ws
   p.cstate = ws;
   p.cdecay = ws + states * p.Dv;
   const GlaChunk g{p, p.cdecay + (states + 3) / 4 * 4};
-  const int wide = p.aux == nullptr && p.act == ACT_NONE && p.ones == 0 && p.Dv % 8 == 0 && p.ldy % 4 == 0 && p.v_off % 4 == 0 && ((uintptr_t)p.y & 15) == 0;
-  const bool plain = p.rot == 0 && p.act == ACT_NONE;
-  if (p.D <= 64) return plain ? gc_launch<1, true>(g, a2, a2_bias, dtype, wide, st) : gc_launch<1, false>(g, a2, a2_bias, dtype, wide, st);
-  return plain ? gc_launch<2, true>(g, a2, a2_bias, dtype, wide, st) : gc_launch<2, false>(g, a2, a2_bias, dtype, wide, st);
+  const int wide = p.Dv % 8 == 0 && p.ldy % 4 == 0 && p.v_off % 4 == 0 && ((uintptr_t)p.y & 15) == 0;
+  return p.D <= 64 ? gc_launch<1>(g, a2, a2_bias, dtype, wide, st) : gc_launch<2>(g, a2, a2_bias, dtype, wide, st);
 }
 
 }  // namespace jl

@@ -1,4 +1,4 @@
-// Gated linear attention: the per-head matrix state S [D x Dv] with one decay per key channel (prompts of up to 128 key channels: gla_chunk.cu),
+// Gated linear attention: the per-head matrix state S [D x Dv] with one decay per key channel (prompts with projected decays and up to 128 key channels: gla_chunk.cu),
 //     S_t = diag(alpha_t) S_(t-1) + k_t v_t^T,     o_t = S_t^T q_t,
 // advanced token by token in fp32, for prompts (S tokens per row) and for decoding (S = 1) alike.
 //
@@ -197,7 +197,6 @@ __global__ void __launch_bounds__(1024) gla_step_kernel(const GlaStep a, const T
 // 2048 tokens, 16 heads of 64 x 128, one row on one B200, both passes: 189 us with the 32 x 1 tile, 93 us with this one.
 constexpr int GS_TS = 16;        // tokens per pipeline stage
 constexpr int GT_DP = 16, GT_C = 4, GT_PITCH = GT_DP + 4;      // 16 channels in rows of 20 floats: the lanes of a group read different banks
-constexpr int GT_CUT_P = 16;     // lanes of a column group from which a prompt may be cut in time
 constexpr int GT_MAX_D = 256;    // wider keys: the fused kernel above
 
 __host__ __device__ inline int gla_lanes(int D) {
@@ -592,7 +591,7 @@ using namespace jl;
 // Time chunks of a prompt scan.  A token costs some 250 cycles of dependent latency however few warps run, so while the grid is short
 // of three CTAs per SM the prompt is cut into chunks that run side by side, in two passes (a local scan without read-outs, two thirds
 // of the work, then the read-out pass) with a small kernel between them.  16 heads of 64 x 128, 2048 tokens of one row, both passes: 170 us in 10
-// chunks, 143 in 20, 105 in 27 (one wave), 115 in 32.  (Keys of up to 128 channels go to gla_chunk.cu from 48 to 80 tokens on and are never cut here.)
+// chunks, 143 in 20, 105 in 27 (one wave), 115 in 32.  (Projected decays and keys of up to 128 channels: gla_chunk.cu from 48 to 80 tokens on.)
 static int gla_chunks(int B, int S, int H, int D, int Dv) {
   static const int forced = [] { const char* e = getenv("JLLAMA_GLA_CHUNKS"); return e ? atoi(e) : 0; }();
   const int P = gla_lanes(D), threads = gla_threads(P, Dv), cols = threads / P * GT_C;
@@ -601,14 +600,17 @@ static int gla_chunks(int B, int S, int H, int D, int Dv) {
   if (forced > 0) nc = forced;
   if (nc > S / 64) nc = S / 64;
   if (nc > 64) nc = 64;
-  return nc < 2 || P < GT_CUT_P ? 1 : nc;
+  return nc < 2 ? 1 : nc;
 }
 
 extern "C" JL_API size_t jl_gla_scan_ws_floats(int B, int S, int H, int D, int Dv) {
-  if (gla_chunk_takes(B, S, H, D, Dv)) return gla_chunk_ws_floats(B, S, H, D, Dv);
   const int nc = gla_chunks(B, S, H, D, Dv);
   size_t n = (size_t)B * S * H * gla_record_floats(gla_lanes(D), Dv);
   if (nc > 1) n += (size_t)B * nc * H * D * Dv + (size_t)B * nc * H * D;
+  if (gla_chunk_takes(B, S, H, D, Dv)) {                    // (one size for the calls that go to gla_chunk.cu and those that walk)
+    const size_t chunked = gla_chunk_ws_floats(B, S, H, D, Dv);
+    n = n > chunked ? n : chunked;
+  }
   return n;
 }
 
@@ -623,25 +625,23 @@ static int launch_stream(GlaParams p, float* ws, cudaStream_t st) {
   p.cstate = ws + (size_t)B * S * H * gla_record_floats(P, Dv);
   p.cdecay = p.cstate + (size_t)B * nc * H * D * Dv;
   const dim3 grid((Dv + cols - 1) / cols, H, B * nc), block(threads);
-  if (smem > 48 * 1024) JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) {
+    JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  }
   if (nc == 1) {
     JL_LAUNCH_PDL((gla_stream_kernel<P, 0>), grid, block, smem, st, p, ws);
     JL_CUDA(cudaGetLastError());
     return JL_OK;
   }
-  if constexpr (P >= GT_CUT_P) {
-    if (smem > 48 * 1024) {
-      JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      JL_CUDA(cudaFuncSetAttribute(gla_stream_kernel<P, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
-    const size_t total = (size_t)B * H * D * Dv;
-    JL_LAUNCH_PDL((gla_stream_kernel<P, 1>), grid, block, smem, st, p, ws);
-    JL_CUDA(cudaGetLastError());
-    JL_LAUNCH_PDL(gla_combine_kernel, dim3((unsigned)((total + 255) / 256 < 1184 ? (total + 255) / 256 : 1184)), dim3(256), 0, st, p);
-    JL_CUDA(cudaGetLastError());
-    JL_LAUNCH_PDL((gla_stream_kernel<P, 3>), grid, block, smem, st, p, ws);
-    JL_CUDA(cudaGetLastError());
-  }
+  const size_t total = (size_t)B * H * D * Dv;
+  JL_LAUNCH_PDL((gla_stream_kernel<P, 1>), grid, block, smem, st, p, ws);
+  JL_CUDA(cudaGetLastError());
+  JL_LAUNCH_PDL(gla_combine_kernel, dim3((unsigned)((total + 255) / 256 < 1184 ? (total + 255) / 256 : 1184)), dim3(256), 0, st, p);
+  JL_CUDA(cudaGetLastError());
+  JL_LAUNCH_PDL((gla_stream_kernel<P, 3>), grid, block, smem, st, p, ws);
+  JL_CUDA(cudaGetLastError());
   return JL_OK;
 }
 
@@ -658,7 +658,7 @@ static int launch_scan(GlaParams p, const void* a2, const void* a2_bias, float* 
   dim3 grid((Dv + cols - 1) / cols, H, B), block(GS_THREADS);
   if (ws != nullptr && D <= GT_MAX_D) {                      // prompts: token-parallel preparation, then the pipe
     cudaStream_t st = (cudaStream_t)stream;
-    if (gla_chunk_takes(B, S, H, D, Dv)) return gla_chunk_launch(p, a2, a2_bias, ws, dtype, st);
+    if (p.aux == nullptr && p.head_decay == nullptr && gla_chunk_takes(B, S, H, D, Dv)) return gla_chunk_launch(p, a2, a2_bias, ws, dtype, st);
     p.P = gla_lanes(D);
     const int slots = H * (p.P * GT_DP + ((Dv + 3) & ~3));
     const dim3 pgrid((B * S + GP_TOK - 1) / GP_TOK, (slots + GP_THREADS - 1) / GP_THREADS);

@@ -84,8 +84,8 @@ struct Entry<R (*)(A...)> {
   X(jl_prefill_attn_mma) X(jl_sample_full) X(jl_swiglu) X(jl_argmax)                                                                     \
   X(jl_embed_f32) X(jl_norm_f32) X(jl_postnorm_add) X(jl_headnorm_gate) X(jl_act_cast) X(jl_act_inplace) X(jl_linear_any)                \
   X(jl_linear_resident) X(jl_linear_exact) X(jl_linear_f32_pair_ws) X(jl_linear_f32_pair) X(jl_attn_prep) X(jl_attn_prep_ex)             \
-  X(jl_attn_step) X(jl_attn_generic) X(jl_attn_generic_splits) X(jl_head_gate) X(jl_gla_scan) X(jl_gla_step) X(jl_gla_scan_ws_floats)    \
-  X(jl_retention_scan) X(jl_branch_add_norm) X(jl_moe_route) X(jl_moe_route_ex) X(jl_moe_sort)                      \
+  X(jl_attn_step) X(jl_attn_generic) X(jl_attn_generic_splits) X(jl_head_gate) X(jl_gla_scan) X(jl_gla_scan_exact) X(jl_gla_step)           \
+  X(jl_gla_scan_ws_floats) X(jl_retention_scan) X(jl_branch_add_norm) X(jl_moe_route) X(jl_moe_route_ex) X(jl_moe_sort)                      \
   X(jl_moe_sorted_rows) X(jl_moe_gather) X(jl_moe_combine) X(jl_moe_combine_ex) X(jl_gemm_grouped) X(jl_gemm_grouped_act) X(jl_gemm_glu) \
   X(jl_glu_act) X(jl_linear_grouped) X(jl_latent_prep) X(jl_latent_heads) X(jl_rotary_slice) X(jl_attn_masked) X(jl_attn_windowed)       \
   X(jl_flash_prefill_masked) X(jl_causal_conv) X(jl_ssd_gates) X(jl_ssd_scan) X(jl_gated_groupnorm) X(jl_delta_scan)                     \

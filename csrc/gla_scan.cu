@@ -592,8 +592,12 @@ using namespace jl;
 // of three CTAs per SM the prompt is cut into chunks that run side by side, in two passes (a local scan without read-outs, two thirds
 // of the work, then the read-out pass) with a small kernel between them.  16 heads of 64 x 128, 2048 tokens of one row, both passes: 170 us in 10
 // chunks, 143 in 20, 105 in 27 (one wave), 115 in 32.  (Projected decays and keys of up to 128 channels: gla_chunk.cu from 48 to 80 tokens on.)
-static int gla_chunks(int B, int S, int H, int D, int Dv) {
+static int gla_forced_chunks() {       // JLLAMA_GLA_CHUNKS: walks every prompt, in that many chunks where it has the tokens
   static const int forced = [] { const char* e = getenv("JLLAMA_GLA_CHUNKS"); return e ? atoi(e) : 0; }();
+  return forced;
+}
+static int gla_chunks(int B, int S, int H, int D, int Dv) {
+  const int forced = gla_forced_chunks();
   const int P = gla_lanes(D), threads = gla_threads(P, Dv), cols = threads / P * GT_C;
   const long warps = (long)B * H * ((Dv + cols - 1) / cols) * (threads / 32);
   int nc = (int)((long)SMS * 12 / (warps > 0 ? warps : 1));
@@ -645,8 +649,8 @@ static int launch_stream(GlaParams p, float* ws, cudaStream_t st) {
   return JL_OK;
 }
 
-// Both scans (projected decays; fixed decays with rotary q / k) share the kernels: what differs is in p.
-static int launch_scan(GlaParams p, const void* a2, const void* a2_bias, float* ws, int dtype, void* stream) {
+// Both scans (projected decays; fixed decays with rotary q / k) share the kernels: what differs is in p.  walk: in fp32 FMAs token by token, whatever the sizes.
+static int launch_scan(GlaParams p, const void* a2, const void* a2_bias, float* ws, int dtype, void* stream, bool walk = true) {
   const int B = p.B, S = p.S, H = p.H, D = p.D, Dv = p.Dv, R = p.R;
   int P = 1;
   while (P * GS_DP < D) P *= 2;
@@ -658,7 +662,7 @@ static int launch_scan(GlaParams p, const void* a2, const void* a2_bias, float* 
   dim3 grid((Dv + cols - 1) / cols, H, B), block(GS_THREADS);
   if (ws != nullptr && D <= GT_MAX_D) {                      // prompts: token-parallel preparation, then the pipe
     cudaStream_t st = (cudaStream_t)stream;
-    if (p.aux == nullptr && p.head_decay == nullptr && gla_chunk_takes(B, S, H, D, Dv)) return gla_chunk_launch(p, a2, a2_bias, ws, dtype, st);
+    if (!walk && gla_forced_chunks() <= 0 && gla_chunk_takes(B, S, H, D, Dv)) return gla_chunk_launch(p, a2, a2_bias, ws, dtype, st);
     p.P = gla_lanes(D);
     const int slots = H * (p.P * GT_DP + ((Dv + 3) & ~3));
     const dim3 pgrid((B * S + GP_TOK - 1) / GP_TOK, (slots + GP_THREADS - 1) / GP_THREADS);
@@ -687,15 +691,28 @@ static int launch_scan(GlaParams p, const void* a2, const void* a2_bias, float* 
   return JL_OK;
 }
 
-extern "C" JL_API int jl_gla_scan(const float* y, int ldy, int q_off, int k_off, int v_off, int a_off, const void* a2,
-                                  const void* a2_bias, float* state, float* o, const int* cache_len, const int* pad_left, int B,
-                                  int S, int H, int D, int Dv, int R, float q_scale, float tau, float* ws, int dtype,
-                                  void* stream) {
+static int gla_scan(const float* y, int ldy, int q_off, int k_off, int v_off, int a_off, const void* a2, const void* a2_bias, float* state, float* o,
+                    const int* cache_len, const int* pad_left, int B, int S, int H, int D, int Dv, int R, float q_scale, float tau, float* ws, int dtype,
+                    void* stream, bool walk) {
   JL_CHECK_ARG(B >= 1 && S >= 1 && H >= 1 && D >= 1 && Dv >= 1 && R >= 1, "jl_gla_scan: bad shape");
   JL_CHECK_ARG(tau > 0.0f, "jl_gla_scan: tau=%f must be positive", tau);
   GlaParams p{y, ldy, q_off, k_off, v_off, a_off, B, S, H, D, Dv, R, 1, q_scale, 1.0f / tau, cache_len, pad_left, state, o};
   p.k_scale = 1.0f;
-  return launch_scan(p, a2, a2_bias, ws, dtype, stream);
+  return launch_scan(p, a2, a2_bias, ws, dtype, stream, walk);
+}
+
+extern "C" JL_API int jl_gla_scan(const float* y, int ldy, int q_off, int k_off, int v_off, int a_off, const void* a2,
+                                  const void* a2_bias, float* state, float* o, const int* cache_len, const int* pad_left, int B,
+                                  int S, int H, int D, int Dv, int R, float q_scale, float tau, float* ws, int dtype,
+                                  void* stream) {
+  return gla_scan(y, ldy, q_off, k_off, v_off, a_off, a2, a2_bias, state, o, cache_len, pad_left, B, S, H, D, Dv, R, q_scale, tau, ws, dtype, stream, false);
+}
+
+extern "C" JL_API int jl_gla_scan_exact(const float* y, int ldy, int q_off, int k_off, int v_off, int a_off, const void* a2,
+                                        const void* a2_bias, float* state, float* o, const int* cache_len, const int* pad_left, int B,
+                                        int S, int H, int D, int Dv, int R, float q_scale, float tau, float* ws, int dtype,
+                                        void* stream) {
+  return gla_scan(y, ldy, q_off, k_off, v_off, a_off, a2, a2_bias, state, o, cache_len, pad_left, B, S, H, D, Dv, R, q_scale, tau, ws, dtype, stream, true);
 }
 
 extern "C" JL_API int jl_retention_scan(const float* y, int ldy, int q_off, int k_off, int v_off, const float* head_decay,

@@ -327,6 +327,11 @@ int jl_gla_scan(const float* y, int ldy, int q_off, int k_off, int v_off, int a_
                 float* state, float* o, const int* cache_len, const int* pad_left, int B, int S, int H, int D, int Dv, int R,
                 float q_scale, float tau, float* ws, int dtype, void* stream);
 
+/* The same in fp32 FMAs token by token whatever the sizes (jl_gla_scan takes prompts of up to 128 key channels in chunks on the tensor cores): what
+ * JLLAMA_HYBRID_TC=0 gives every call.  The same workspace. */
+int jl_gla_scan_exact(const float* y, int ldy, int q_off, int k_off, int v_off, int a_off, const void* a2, const void* a2_bias,
+                      float* state, float* o, const int* cache_len, const int* pad_left, int B, int S, int H, int D, int Dv, int R,
+                      float q_scale, float tau, float* ws, int dtype, void* stream);
 /* Retention scan: the scan above with one fixed decay per head (head_decay fp32 [H]) instead of the projected one, the rotary
  * embedding of q and k at the token's position on the first `rot` channels of a head (layout 0: channel 2i with 2i+1; 1: channel
  * i with i + rot/2; tables fp32 [max_pos][rot/2], any factor on cos / sin already in them) and k scaled by k_scale after it. */

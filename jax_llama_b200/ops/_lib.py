@@ -74,6 +74,7 @@ _HYBRID = {
     "jl_attn_generic_splits": (i32, [i32, i32, i32, i32]),
     "jl_head_gate": (i32, [vp, fp, i32, i32, i32, i32, i32, vp]),
     "jl_gla_scan": (i32, [fp, i32, i32, i32, i32, i32, vp, vp, fp, fp, ip, ip] + [i32] * 6 + [f32, f32, fp, i32, vp]),
+    "jl_gla_scan_exact": (i32, [fp, i32, i32, i32, i32, i32, vp, vp, fp, fp, ip, ip] + [i32] * 6 + [f32, f32, fp, i32, vp]),
     "jl_gla_step": (i32, [fp] + [i32] * 6 + [vp, vp, vp, fp, vp, ip, ip] + [i32] * 5 + [f32, f32, f32, i32, i32, vp]),
     "jl_gla_scan_ws_floats": (sz, [i32, i32, i32, i32, i32]),
     "jl_retention_scan": (i32, [fp, i32, i32, i32, i32, fp, fp, fp, i32, i32, i32, f32, f32, fp, fp, ip, ip] + [i32] * 5 + [fp, vp]),

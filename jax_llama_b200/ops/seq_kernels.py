@@ -41,7 +41,7 @@ def _need(t: torch.Tensor, dtype: torch.dtype, name: str) -> None:
 
 
 def tensor_cores_enabled() -> bool:
-    """JLLAMA_HYBRID_TC=0 keeps every linear layer on the exact SIMT kernels (A/B and debugging)."""
+    """JLLAMA_HYBRID_TC=0 keeps every linear layer and every scan on the exact SIMT kernels (A/B and debugging)."""
     return os.environ.get("JLLAMA_HYBRID_TC", "1") != "0"
 
 
@@ -235,7 +235,7 @@ def gla_scan(y: torch.Tensor, q_off: int, k_off: int, v_off: int, a_off: int, a2
     ws = None
     if S > GLA_FUSED_MAX_TOKENS:          # prompts: token-parallel preparation + pipelined scan (two launches)
         ws = empty(int(L.jl_gla_scan_ws_floats(B, S, H, D, Dv)), dtype=torch.float32, device=y.device)
-    _lib.check(L.jl_gla_scan(
+    _lib.check((L.jl_gla_scan if tensor_cores_enabled() else L.jl_gla_scan_exact)(
         y.data_ptr(), y.stride(0), q_off, k_off, v_off, a_off, a2.data_ptr(), a2_bias.data_ptr(), state.data_ptr(),
         out.data_ptr(), _p(cache_len), _p(pad_left), B, S, H, D, Dv, R, float(q_scale), float(tau), _p(ws),
         dtype_code(a2.dtype), _stream()), "jl_gla_scan")

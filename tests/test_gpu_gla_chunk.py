@@ -154,6 +154,23 @@ def test_fixed_decays_with_rotation(layout, rot):
     close(end, st, S, D)
 
 
+def test_the_exact_form_is_the_walk(monkeypatch):
+    """JLLAMA_HYBRID_TC=0: fp32 FMAs token by token, shown by the state that pieces of 8 tokens leave (another kernel, the same roundings); the chunks on the tensor cores
+    differ in the last bits."""
+    S = 100                                                    # (too few tokens for chunks in time)
+    c = Gla(2, S, 2, 64, 128)
+    states = [c.state.clone() for _ in range(3)]
+    a = c.scan(c.y, states[0], [0, 70])
+    monkeypatch.setenv("JLLAMA_HYBRID_TC", "0")
+    b = c.scan(c.y, states[1], [0, 70])
+    for s in range(0, S, 5):
+        c.scan(c.y.view(2, S, -1)[:, s:s + 5].reshape(10, -1).contiguous(), states[2], [0, 70], filled=s, S=5)
+    assert torch.equal(states[1], states[2]) and not torch.equal(states[0], states[1]) and not torch.equal(a, b)
+    want, _ = c.exact([0, 70])
+    close(a, want, S, 64)
+    close(b, want, S, 64)
+
+
 # What follows walks token by token (csrc/gla_scan.cu), in time chunks of its own: decays that are given need no fewer bits than fp32 additions have.
 
 @pytest.mark.parametrize("B,S,H,D,Dv", [(1, 65, 4, 64, 128), (1, 500, 16, 64, 128), (1, 2048, 16, 64, 128), (4, 128, 16, 128, 128)])

@@ -9,7 +9,8 @@
 //   gla_chunk_state_kernel  (chunk, head, row): decays (kept for the second kernel), sum_j (..k_j) v_jᵀ and A_64;
 //   gla_combine_kernel      walks the chunks: the state every chunk starts from;
 //   gla_chunk_out_kernel    (chunk, head, row): P, then the two products of o.
-// The products of 64 k are tcgen05 MMAs of bfloat16 parts, three per fp32 number and six products (linear_f32.cuh), value columns as the MMA's 128 rows
+// The products of 64 k are tcgen05 MMAs of bfloat16 parts, three per fp32 number and six products (linear_f32.cuh; a chunk's state sum in four sums of 16 tokens, as it is
+// what the following chunks inherit and the tensor core cuts off where it adds), value columns as the MMA's 128 rows
 // (tokens or key channels lie along K as they come: MN-major operands); P's cross terms are the same on mma.sync.  What comes out infinite or NaN is
 // formed again token by token, so that nothing of a token that is not finite reaches an earlier one.
 // Bound: the chain of phases of a CTA (loads 3, pairs and factors 3, cross terms 2.5, two rounds of tensor core with their operands 5, stores 2.5 thousand cycles of
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_k
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nv = (p.Dv + GC_DV - 1) / GC_DV, h = blockIdx.y / nv, c0 = blockIdx.y % nv * GC_DV, b = blockIdx.z, chunk = blockIdx.x;
   if (warp == 0) {
-    tc::tmem_alloc(tc::smem_u32(&tmem_slot), 64 * DB);
+    tc::tmem_alloc(tc::smem_u32(&tmem_slot), 256 * DB);
     if (lane == 0) { tc::mbar_init(bar, 1); tc::fence_barrier_init(); }
   }
   pdl_wait();
@@ -224,11 +225,11 @@ __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_k
 #pragma unroll
       for (int db = 0; db < DB; ++db)
 #pragma unroll
-        for (int q = 0; q < 6; ++q)
+        for (int k = 0; k < 4; ++k)
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            tc::mma_ss(tmem + db * 64, dv + ((gc_a(q) * 2 * GC_TILE + k * 2048) >> 4), dk + ((db * GC_K_BYTES + gc_b(q) * GC_TILE + k * 2048) >> 4), IDESC,
-                       q != 0 || k != 0);
+          for (int q = 0; q < 6; ++q)
+            tc::mma_ss(tmem + (k * DB + db) * 64, dv + ((gc_a(q) * 2 * GC_TILE + k * 2048) >> 4), dk + ((db * GC_K_BYTES + gc_b(q) * GC_TILE + k * 2048) >> 4), IDESC,
+                       q != 0);
       tc::mma_commit(bar);
     }
     __syncwarp();
@@ -240,16 +241,24 @@ __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_k
   float* out = p.cstate + (((size_t)b * p.NC + chunk) * p.H + h) * p.D * p.Dv + c;
 #pragma unroll 1
   for (int e0 = (warp >> 2) * 32 * DB; e0 < ((warp >> 2) + 1) * 32 * DB; e0 += 32) {
-    uint32_t v[32];
-    tc::tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + e0, v);
-    tc::tmem_ld_wait();
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; i += 16) {
+      uint32_t u[4][16];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) tc::tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + k * 64 * DB + e0 + i, u[k]);
+      tc::tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        v[i + j] = (__uint_as_float(u[0][j]) + __uint_as_float(u[1][j])) + (__uint_as_float(u[2][j]) + __uint_as_float(u[3][j]));
+    }
     if (c < p.Dv) {
       bool bad = false;
 #pragma unroll
       for (int e = 0; e < 32; ++e)
         if (e0 + e < p.D) {
-          out[(size_t)(e0 + e) * p.Dv] = __uint_as_float(v[e]);
-          bad |= !(fabsf(__uint_as_float(v[e])) < INFINITY);
+          out[(size_t)(e0 + e) * p.Dv] = v[e];
+          bad |= !(fabsf(v[e]) < INFINITY);
         }
       if (bad)
 #pragma unroll 1
@@ -276,7 +285,7 @@ __global__ void __launch_bounds__(GC_THREADS, DB == 1 ? 2 : 1) gla_chunk_state_k
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem, 64 * DB);
+  if (warp == 0) tc::tmem_dealloc(tmem, 256 * DB);
 }
 
 __device__ __forceinline__ void gc_mma16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {

@@ -50,6 +50,10 @@ __device__ __forceinline__ void step_head(const AttnStep& a, const float* src, i
   for (int u = 0; u < HD / 64; ++u) *reinterpret_cast<uint32_t*>(dst + 2 * (lane + 32 * u)) = pack_bf16(v[u].x * r, v[u].y * r);
 }
 
+// A gate's sigmoid.  This file is compiled with the approximated float functions, whose exponential is 2^-19 off at -50; in double it is exact to float, and formed
+// by lanes that have no head to prepare (2 rows x 16 heads over 4, 100 keys, us in a graph 6.04 with the division at the end -> 5.86).
+__device__ __forceinline__ float gate_sigmoid(float g) { return (float)(1.0 / (1.0 + exp(-(double)g))); }
+
 // STEP: the queries (and, unless another layer has them, the new key and value) come from the projection; every CTA of a key / value head prepares its
 // queries, the one whose keys include the new slot its key and value, which it also appends.  Such a step is latency: preparation, attention and gate in three
 // launches -> one, us in a graph: 2 rows x 16 heads over 4 of 128, 100 keys 8.5 -> 6.2, 8 rows 200 keys 10.8 -> 8.8, 2 x 32 heads over 8, 4000 keys (16 parts and a merge) 19.3 -> 14.5.
@@ -88,6 +92,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   const int hi = lo + chunk < len ? lo + chunk : len;
 
   __shared__ __align__(16) __nv_bfloat16 s_new[STEP ? G + 2 : 1][HD];      // query heads | new key | new value
+  __shared__ float s_gate[STEP ? G : 1];
   int slot = -1;                                                           // of the new token, where this CTA holds its key and value
   if constexpr (STEP) {
     const float* row = step.y + (size_t)b * step.ldy;
@@ -100,6 +105,10 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
       if (i < G) step_head<HD>(step, row + step.q_off + (kvh * G + i) * HD, pos, true, step.unit_norm != 0, s_new[i]);
       else if (i == G) step_head<HD>(step, row + step.k_off + kvh * HD, pos, true, step.unit_norm != 0, s_new[i]);
       else step_head<HD>(step, row + step.v_off + kvh * HD, pos, false, false, s_new[i]);
+    }
+    if (step.g_off >= 0 && splits == 1 && threadIdx.x >= DA_WARPS * 32 - G) {      // (read behind the barrier at the end)
+      const int g = threadIdx.x - (DA_WARPS * 32 - G);
+      s_gate[g] = gate_sigmoid(row[step.g_off + kvh * G + g]);
     }
     __syncthreads();
     if (own) {
@@ -232,7 +241,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     if (splits == 1) {
       float v = L > 0.f ? acc / L : 0.f;
       if constexpr (STEP)
-        if (step.g_off >= 0) v = __fdiv_rn(v, 1.0f + expf(-step.y[(size_t)b * step.ldy + step.g_off + h]));
+        if (step.g_off >= 0) v *= s_gate[g];
       out[((size_t)b * nh + h) * HD + d] = __float2bfloat16(v);
     } else {
       const size_t pi = ((size_t)b * nh + h) * splits + split;
@@ -260,7 +269,7 @@ attn_combine_kernel(const float* __restrict__ o_part, const float* __restrict__ 
     L += w * ml_part[(bh * splits + s) * 2 + 1];
   }
   float v = L > 0.f ? acc / L : 0.f;
-  if (gate != nullptr) v = __fdiv_rn(v, 1.0f + expf(-gate[bh / nh * ldg + bh % nh]));
+  if (gate != nullptr) v *= gate_sigmoid(gate[bh / nh * ldg + bh % nh]);
   out[bh * HD + d] = __float2bfloat16(v);
 }
 

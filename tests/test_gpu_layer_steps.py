@@ -87,6 +87,26 @@ def test_attn_step(B, G, nkv, hd, T, filled, pads, rot, unit, gate, own):
     assert float((got.double() - want.double()).abs().max()) <= 2.0 ** -7 * max(scale, 1e-6)
 
 
+@pytest.mark.parametrize("splits", [1, 3])
+def test_the_gates_exponential_is_not_approximated(splits):
+    """One key whose values are ones: the result is the gate's sigmoid, rounded to bfloat16.  Computed to 2^-22 it can differ from the rounded exact one only where that lies
+    within 2^-22 of the middle between two bfloat16 numbers; an exponential of the special-function unit is 2^-19 off at gates of -50: some of 65536 fall on the other side."""
+    B, G, nkv, hd, T = 1024, 8, 8, 64, 8
+    nh = G * nkv
+    y = torch.ones(B, (nh + 2 * nkv) * hd + nh, device="cuda")
+    y[:, -nh:] = torch.linspace(-80.0, 15.0, B * nh, device="cuda").view(B, nh)
+    kc, vc = (torch.zeros(B, nkv, T, hd, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    table, got = torch.zeros(1, 1, device="cuda"), torch.empty(B, nh * hd, dtype=torch.bfloat16, device="cuda")
+    scratch = torch.empty(B * nh * splits * (hd + 2), device="cuda")
+    L = _lib.lib()
+    _lib.check(L.jl_attn_step(y.data_ptr(), y.stride(0), 0, nh * hd, (nh + nkv) * hd, (nh + 2 * nkv) * hd, table.data_ptr(), table.data_ptr(), 1, 0, 0, 1e-5, kc.data_ptr(),
+                              vc.data_ptr(), i32(0).data_ptr(), i32(*[0] * B).data_ptr(), scratch.data_ptr(), got.data_ptr(), B, nh, nkv, hd, T, 1.0, splits,
+                              K._stream()), "jl_attn_step")
+    exact = torch.sigmoid(y[:, -nh:].double())[..., None].expand(B, nh, hd).reshape(B, -1)
+    lo, hi = ((exact * (1 + e)).float().bfloat16() for e in (-2.0 ** -22, 2.0 ** -22))
+    assert bool(((got >= lo) & (got <= hi)).all()), int(((got < lo) | (got > hi)).sum()) // hd
+
+
 def test_attn_step_refuses_rows_off_their_boundary():
     y = torch.randn(1, 999, device="cuda")
     L, p = _lib.lib(), y.data_ptr()

@@ -102,7 +102,7 @@ class DenseFeedForward:
         return self.weights()
 
     def run(self, h: torch.Tensor) -> torch.Tensor:
-        with SK.Scratch():
+        with SK.room_of(self):
             if self.spec.gated:
                 t = _gated_layer(h, self.up, self.u_off, self.spec.ff, self.spec.act, 0.0)
             else:
@@ -179,7 +179,7 @@ class MoeFeedForward:
         return [self.up[:n], self.down[:n]] + [t for t in (self.w_route, self.shared_up, self.shared_down) if t is not None]
 
     def run(self, h: torch.Tensor) -> torch.Tensor:
-        with SK.Scratch():
+        with SK.room_of(self):
             parts = self._parts(h)
         return SK.moe_combine(*parts[0], **parts[1])
 

@@ -84,7 +84,8 @@ class MixerParts(NamedTuple):
 
 class Mixer:
     """What the layer stack asks of a mixer.  `run` gives the input of the output projection `wo`; `parts` the terms of the mixer's
-    contribution, `forward` their fp32 sum [M, width] (a mixer made of several overrides them).  `shapes(spec, W, rank_of)` lists the checkpoint
+    contribution, `forward` their fp32 sum [M, width] (a mixer made of several overrides them).  A mixer derived outside this package has torch tensors between its
+    kernels, the package's own have arrays of a room (ops/scratch.py).  `shapes(spec, W, rank_of)` lists the checkpoint
     tensors under the mixer's prefix; `rank_of(name, default)` is the first dimension the checkpoint gives a tensor whose
     inner size no configuration key fixes."""
 
@@ -94,7 +95,7 @@ class Mixer:
         return p.y1 if p.bias is None and p.y2 is None and p.c1 == 1.0 else SK.weighted_sum2(*p)
 
     def parts(self, h: torch.Tensor, B: int, S: int, cache: "object", layer: int, rope: Optional[Tuple] = None) -> MixerParts:
-        with SK.Scratch():
+        with SK.room_of(self):
             y = self.run(h, B, S, cache, layer, rope)
         return MixerParts(SK.linear(y, self.wo, resident=True), bias=self.out_bias)
 

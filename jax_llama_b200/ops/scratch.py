@@ -4,11 +4,15 @@ The layers allocate their results between two kernels with `empty`.  Outside a `
 single allocation instead: a torch tensor costs the host 2.3 to 2.7 µs, a layer over few tokens has up to ten of them, and they are only ever handed to the next
 kernel as an address, a shape and a pitch.  The room belongs to the call: it is an ordinary allocation on the current stream and lives as long as an array in
 it does.  What a layer returns is allocated outside the block and is a torch tensor.
+
+Only the classes that come with this package compute in such a block (`room_of`): a mixer or feed-forward derived elsewhere may do with its intermediates what a torch tensor
+allows, and gets torch tensors.
 """
 from __future__ import annotations
 
+import contextlib
 import threading
-from typing import Any, Optional, Tuple, Union
+from typing import Any, ContextManager, Optional, Tuple, Union
 
 import torch
 
@@ -28,6 +32,10 @@ class Array:
 
     def __init__(self, ptr: int, shape: Tuple[int, ...], pitch: int, dtype: torch.dtype, device: torch.device, room: torch.Tensor):
         self.ptr, self.shape, self.pitch, self.dtype, self.device, self.room = ptr, shape, pitch, dtype, device, room
+
+    def __getattr__(self, name: str) -> Any:
+        raise AttributeError(f"{name!r}: an intermediate inside a layer of this package is an address with a shape (ops/scratch.py), not a torch tensor; a class derived "
+                             "from the layer's outside the package gets tensors")
 
     def data_ptr(self) -> int:
         return self.ptr
@@ -92,6 +100,14 @@ class Scratch:
         at = self.base + self.used
         self.used += (nbytes + ALIGN - 1) // ALIGN * ALIGN
         return Array(at, shape, pitch, dtype, device, self.room)
+
+
+_PACKAGE = __name__.partition(".")[0] + "."
+
+
+def room_of(layer: object) -> ContextManager:
+    """A Scratch block for what `layer` computes, if its class is one of this package's; else a block in which `empty` is torch.empty as outside."""
+    return Scratch() if type(layer).__module__.startswith(_PACKAGE) else contextlib.nullcontext()
 
 
 def empty(shape: Union[int, Tuple[int, ...]], *, dtype: torch.dtype, device: torch.device) -> Union[Array, torch.Tensor]:

@@ -2,6 +2,8 @@
 gla_scan.cu): fp32 residual stream, operands in bfloat16 or true float32, softmax attention with arbitrary head sizes
 and linear-recurrence mixers.
 
+Inside a layer of this package the results are arrays of its room (ops/scratch.py) where they are small; anywhere else they are torch tensors.
+
 CUDA tensors only: these ops are the product path and have no PyTorch stand-in (the numerical oracles live with the
 tests).  Every call runs on the current stream and is legal under CUDA-graph capture when the caller passes `out`
 buffers (otherwise outputs come from the caching allocator, which a torch graph capture also handles).
@@ -15,7 +17,7 @@ import torch
 
 from . import _lib
 from .kernels import _p, _stream, ensure_gemm_workspace, num_sms
-from .scratch import Scratch, empty  # noqa: F401  (Scratch: for the layers)
+from .scratch import empty, room_of  # noqa: F401  (room_of: for the layers)
 
 ACT_NONE, ACT_RELU2, ACT_GELU_TANH, ACT_SILU, ACT_SCALE_SOFTCAP, ACT_SIGMOID, ACT_XIELU, ACT_RELU = 0, 1, 2, 3, 4, 5, 6, 7
 DELTA_FUSED_MAX_TOKENS = 8    # the same for the delta-rule scan (csrc/delta_scan.cu DS_FUSED_MAX_TOKENS)

@@ -7,6 +7,10 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+from jax_llama_b200.config import GlaMixerSpec, MoeMlpSpec  # noqa: E402
+from jax_llama_b200.models.feedforward import MoeFeedForward  # noqa: E402
+from jax_llama_b200.models.hybrid_engine import HybridCache  # noqa: E402
+from jax_llama_b200.models.mixers import GlaMixer  # noqa: E402
 from jax_llama_b200.ops import _lib  # noqa: E402
 from jax_llama_b200.ops import kernels as K  # noqa: E402
 from jax_llama_b200.ops import seq_kernels as SK  # noqa: E402
@@ -112,3 +116,37 @@ def test_attn_step_refuses_rows_off_their_boundary():
     L, p = _lib.lib(), y.data_ptr()
     assert L.jl_attn_step(p, 999, 0, 128, 256, -1, p, p, 4, 0, 0, 1e-5, p, p, 0, 0, 0, p, 1, 1, 1, 128, 4, 1.0, 1, K._stream()) != 0
     assert L.jl_attn_step(p, 998, 1, 128, 256, -1, p, p, 4, 0, 0, 1e-5, p, p, 0, 0, 0, p, 1, 1, 1, 128, 4, 1.0, 1, K._stream()) != 0
+
+
+@pytest.mark.parametrize("M", [3, 20000])                      # intermediates that fit a room, and larger ones
+def test_layers_derived_elsewhere_compute_with_tensors(M):
+    """What a derived layer does with its base's intermediates is torch's to answer, whatever their size."""
+    class Twice(GlaMixer):
+        def run(self, h, B, S, cache, layer, rope=None):
+            y = super().run(h, B, S, cache, layer, rope)
+            return torch.cat([y[:, :7].float() * 2, 2 * y[:, 7:].float()], 1).to(y.dtype)
+
+    class Shifted(MoeFeedForward):
+        def _parts(self, h):
+            args, more = super()._parts(h)
+            return (args[0] + 1.0, *args[1:]), more
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    mat = lambda n, k: (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).bfloat16()        # noqa: E731
+    W, H, D, Dv = 64, 2, 16, 32
+    w = {"q": mat(H * D, W), "k": mat(H * D, W), "v": mat(H * Dv, W), "g": mat(H * Dv, W), "a1": mat(16, W), "a2": mat(H * D, 16), "a2.b": mat(1, H * D)[0], "norm": mat(1, Dv)[0],
+         "o": mat(W, H * Dv)}
+    h = mat(M, W)
+    results = []
+    for cls in (GlaMixer, Twice):
+        m = cls(GlaMixerSpec(heads=H, dim=D, vdim=Dv, tau=16.0), w, 1e-5)
+        cache = HybridCache(k=torch.zeros(1, device="cuda"), v=torch.zeros(1, device="cuda"), index=0, pad_left=i32(0), len_dev=i32(0), ks=[None], vs=[None],
+                            states=[m.new_state(1, h.device)], length=M)
+        results.append(m.forward(h, 1, M, cache, 0))
+    assert torch.equal(results[1], 2 * results[0])             # a factor of two is exact
+    ew = {"router": mat(4, W)}
+    for e in range(4):
+        ew[f"e{e}.gate"], ew[f"e{e}.up"], ew[f"e{e}.down"] = mat(24, W), mat(24, W), mat(W, 24)
+    spec = MoeMlpSpec(experts=4, top=2, ff=24, act="silu", score="softmax", gated=True, shared_ff=0, shared_gate=False)
+    plain, moved = MoeFeedForward(spec, ew).run(h), Shifted(spec, ew).run(h)
+    assert float((moved - plain - 1.0).abs().max()) <= 2.0 ** -20 * float(plain.abs().max() + 1.0) * 4      # the weights of a token add up to one

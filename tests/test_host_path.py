@@ -11,7 +11,9 @@ import pytest
 import torch
 
 from jax_llama_b200.ops import _lib, build
-from jax_llama_b200.ops.scratch import ALIGN, CHUNK, LARGEST, Array, Scratch, empty
+from jax_llama_b200.models.feedforward import DenseFeedForward, MoeFeedForward
+from jax_llama_b200.models.mixers import GlaMixer, LatentAttentionMixer
+from jax_llama_b200.ops.scratch import ALIGN, CHUNK, LARGEST, Array, Scratch, empty, room_of
 
 
 @pytest.fixture(scope="module")
@@ -163,3 +165,19 @@ def test_an_array_answers_as_the_tensor_it_stands_for():
     for wrong in (lambda: a.view(7, 9), lambda: a[:, 1:3].view(-1), lambda: a[1:, :], lambda: a[:, ::2]):
         with pytest.raises((ValueError, IndexError)):
             wrong()
+
+
+def test_an_array_says_what_it_is_not():
+    t = torch.empty(4, 4)
+    with pytest.raises(AttributeError, match="not a torch tensor"):
+        Array(t.data_ptr(), (4, 4), 4, t.dtype, CPU, t).float()
+
+
+@pytest.mark.parametrize("base", [GlaMixer, LatentAttentionMixer, DenseFeedForward, MoeFeedForward])
+def test_a_layer_derived_elsewhere_has_tensors(base):
+    class Own(base):
+        pass
+
+    for cls, kind in ((base, Array), (Own, torch.Tensor)):
+        with room_of(object.__new__(cls)):
+            assert type(empty((2, 2), dtype=torch.float32, device=CPU)) is kind

@@ -50,9 +50,25 @@ __device__ __forceinline__ void step_head(const AttnStep& a, const float* src, i
   for (int u = 0; u < HD / 64; ++u) *reinterpret_cast<uint32_t*>(dst + 2 * (lane + 32 * u)) = pack_bf16(v[u].x * r, v[u].y * r);
 }
 
-// A gate's sigmoid.  This file is compiled with the approximated float functions, whose exponential is 2^-19 off at -50; in double it is exact to float, and formed
-// by lanes that have no head to prepare (2 rows x 16 heads over 4, 100 keys, us in a graph 6.04 with the division at the end -> 5.86).
-__device__ __forceinline__ float gate_sigmoid(float g) { return (float)(1.0 / (1.0 + exp(-(double)g))); }
+// A gate's sigmoid to the last bits of fp32.  This file is compiled with the approximated float functions, whose exponential is 2^-19 off at -50.  e^-g = 2^n e^r: reduction
+// by n ln 2 in two parts (Cody and Waite, Software Manual for the Elementary Functions, 1980), then the Taylor series to r^7 (|r| <= ln 2 / 2: the rest is below 2^-26).
+__device__ __forceinline__ float gate_sigmoid(float g) {
+  float x = -g;                                                            // (comparisons, not fminf: a gate that is not a number gives none)
+  x = x > 88.0f ? 88.0f : x;
+  x = x < -87.0f ? -87.0f : x;
+  const float n = rintf(x * 1.44269504f);
+  float r = fmaf(n, -0.693147182f, x);                                     // ln 2 = 0.693147182464599609 - 1.904654323e-9
+  r = fmaf(n, 1.904654323e-9f, r);
+  float e = 1.0f / 5040.0f;
+  e = fmaf(e, r, 1.0f / 720.0f);
+  e = fmaf(e, r, 1.0f / 120.0f);
+  e = fmaf(e, r, 1.0f / 24.0f);
+  e = fmaf(e, r, 1.0f / 6.0f);
+  e = fmaf(e, r, 0.5f);
+  e = fmaf(e, r, 1.0f);
+  e = fmaf(e, r, 1.0f);
+  return __fdiv_rn(1.0f, fmaf(e, __int_as_float(((int)n + 127) << 23), 1.0f));
+}
 
 // STEP: the queries (and, unless another layer has them, the new key and value) come from the projection; every CTA of a key / value head prepares its
 // queries, the one whose keys include the new slot its key and value, which it also appends.  Such a step is latency: preparation, attention and gate in three
@@ -101,15 +117,15 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     int pos = (cache_len_ptr ? *cache_len_ptr : 0) - first;
     pos = pos < 0 ? 0 : (pos >= step.max_pos ? step.max_pos - 1 : pos);
     const bool own = step.k_off >= 0 && fits && (valid > 0 ? at >= lo && at < hi : split == 0);
+    const int g = threadIdx.x - (DA_WARPS * 32 - G);                       // (the last warp has the fewest heads)
+    const bool gates = step.g_off >= 0 && splits == 1 && g >= 0;
+    const float gate = gates ? row[step.g_off + kvh * G + g] : 0.0f;
     for (int i = warp; i < G + (own ? 2 : 0); i += DA_WARPS) {
       if (i < G) step_head<HD>(step, row + step.q_off + (kvh * G + i) * HD, pos, true, step.unit_norm != 0, s_new[i]);
       else if (i == G) step_head<HD>(step, row + step.k_off + kvh * HD, pos, true, step.unit_norm != 0, s_new[i]);
       else step_head<HD>(step, row + step.v_off + kvh * HD, pos, false, false, s_new[i]);
     }
-    if (step.g_off >= 0 && splits == 1 && threadIdx.x >= DA_WARPS * 32 - G) {      // (read behind the barrier at the end)
-      const int g = threadIdx.x - (DA_WARPS * 32 - G);
-      s_gate[g] = gate_sigmoid(row[step.g_off + kvh * G + g]);
-    }
+    if (gates) s_gate[g] = gate_sigmoid(gate);                             // (read behind the barrier at the end)
     __syncthreads();
     if (own) {
       slot = at;

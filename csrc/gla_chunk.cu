@@ -13,11 +13,14 @@
 // what the following chunks inherit and the tensor core cuts off where it adds), value columns as the MMA's 128 rows
 // (tokens or key channels lie along K as they come: MN-major operands); P's cross terms are the same on mma.sync.  What comes out infinite or NaN is
 // formed again token by token, so that nothing of a token that is not finite reaches an earlier one.
-// Bound: the chain of phases of a CTA (loads 3, pairs and factors 3, cross terms 2.5, two rounds of tensor core with their operands 5, stores 2.5 thousand cycles of
-// the second kernel's 20; decays 4-5, loads 5 of the first's 16) with two CTAs per SM; the operands' way from L2 is 60 MB.  One B200, us, walking twice over chunks of tokens
-// (gla_scan.cu) -> this, all launches of the scan: 2048 tokens x 16 heads of 64 x 128 124 -> 72 (a layer of width 2048 199 -> 149), 2 rows x 1000 120 -> 69, 500 99 -> 31, 4 rows x
-// 512 x 8 heads of 32 x 64 65 -> 34, 4 rows x 128 x 16 heads of 128 x 128 100 -> 55.  Error against float64 (2-norm of the read-outs; of the state), the decays' own included: 65 tokens
-// 3.1e-7; 4.0e-7 -> 2.4e-7; 3.5e-7, 500 1.9e-6; 2.9e-6 -> 1.8e-6; 2.8e-6, 2048 7.0e-6; 1.05e-5 -> 6.7e-6; 1.01e-5.
+// Bound: latencies of a CTA's chain of phases (loads, decays, pairs and factors, cross terms, two rounds of tensor core, stores) with two CTAs per SM: 21 % of the warps are active, half
+// of the issue slots, 5 and 13 % of the tensor pipe are used, 105 and 130 MB pass the L2 (2048 tokens x 16 heads of 64 x 128).  One B200, us, walking twice over chunks of tokens
+// (gla_scan.cu) -> this, all launches of the scan: 2048 tokens x 16 heads of 64 x 128 123 -> 77 (a layer of width 2048 199 -> 149), 2 rows x 1000 120 -> 73, 500 89 -> 30, 4 rows x
+// 512 x 8 heads of 32 x 64 68 -> 34, 4 rows x 128 x 16 heads of 128 x 128 101 -> 53.
+// Error against float64 (2-norm of the read-outs; of the state), the decays' own included, walk -> this: decays of 0.99 in the mean, 65 tokens 2.2e-7; 2.7e-7 -> 1.9e-7; 2.6e-7, 500
+// 1.01e-6; 1.53e-6 -> 9.5e-7; 1.49e-6, 2048 2.30e-6; 3.14e-6 -> 2.25e-6; 3.17e-6; operands of one sign, 65 8.8e-8; 2.4e-7 -> 5.7e-8; 2.2e-7, 500 6.5e-7; 1.82e-6 -> 5.4e-7; 1.78e-6, 2048
+// 1.70e-6; 5.93e-6 -> 1.59e-6; 5.99e-6.  Decays of 0.72, where few tokens are summed and the cut-off shows: 500 1.04e-7; 8.3e-8 -> 1.07e-7; 8.9e-8, of one sign 5.4e-8; 9.0e-8 ->
+// 5.9e-8; 8.7e-8.
 #include "gla_scan.cuh"
 #include "jllama_b200.h"
 #include "linear_f32.cuh"
@@ -586,12 +589,12 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_out_kernel(const __gr
 
 static int gc_chunks(int S) { return (S + GC_T - 1) / GC_T; }
 
-// Up to 128 key channels, from the tokens on where three launches of parallel chunks beat the walk of gla_scan.cu.  us, walk -> this: D 64 x Dv 128, projected decays: 1
-// row x 16 heads 40 tokens 21.8 -> 23.3, 48 24.2 -> 23.6, 64 30.0 -> 23.5, 2 rows 40 31.1 -> 24.4, 64 60.9 -> 24.6; 4 rows x 16 heads of 32 x 64, 48 tokens 26.8 -> 23.2;
-// 128 x 128: 1 row x 4 heads 64 tokens 35.5 -> 39.2, 200 61.7 -> 40.1, 4 rows x 8 heads 40 39.9 -> 41.6, 48 52.7 -> 41.8.  Decays that are given (one per head or per token and head)
-// always walk: nothing of their own covers what the tensor core cuts off and the roundings of products of 64 decays.  Error against float64 (2-norm of the read-outs), walk -> this:
-// one fixed decay of 0.9, operands of one sign, 500 tokens x 16 heads of 64 x 128 4.1e-8 -> 9.4e-8, decay 1 4.7e-8 -> 1.4e-7; a float32 retention layer of 3 x 608 tokens, its
-// state 1.18e-6 -> 1.49e-6.
+// Up to 128 key channels, from the tokens on where three launches of parallel chunks beat the walk of gla_scan.cu.  us, walk -> this: D 64 x Dv 128: 1 row x 16 heads 40 tokens 21.8 -> 23.3,
+// 48 24.1 -> 21.9, 64 29.9 -> 21.9, 2 rows 48 27.9 -> 23.3, 64 33.7 -> 23.4; 4 rows x 16 heads of 32 x 64, 48 tokens 25.3 -> 21.6; 128 x 128: 1 row x 4 heads 64 tokens 35.4 -> 39.2, 80
+// 42.2 -> 34.1, 200 61.3 -> 34.9, 4 rows x 8 heads 40 39.9 -> 41.6, 48 41.3 -> 37.6.
+// Decays that are given (one per head, or per token and head) always walk: nothing of their own covers what the tensor core cuts off and the roundings of products of 64 decays.  Error
+// against float64 (2-norm of the read-outs), walk -> this: one fixed decay of 0.9, operands of one sign, 500 tokens x 16 heads of 64 x 128 4.1e-8 -> 9.4e-8, decay 1 4.7e-8 ->
+// 1.4e-7; a float32 retention layer of 3 x 608 tokens, its state 1.18e-6 -> 1.49e-6.
 bool gla_chunk_takes(int B, int S, int H, int D, int Dv) {
   return D <= 128 && S >= (D <= 64 || B * H >= 32 ? 48 : 80) && (long)H * ((Dv + GC_DV - 1) / GC_DV) <= 65535 && B <= 65535;
 }

@@ -14,8 +14,8 @@
 // inside a tile leaves a partial tile in the workspace, and a second kernel adds a tile's parts in order of k.  Where whole tiles are as fast
 // there is no second kernel.  A long chain of additions costs precision: what is more than LP_FOLD units, or than a CTA of linear_f32.cu adds in a row for the same product, is
 // folded through the workspace on its way.
-// Bound: 24 MMAs of 12 BN cycles together per unit, with the loads (64 KB per CTA and unit at BN 256) right behind.  One B200, single CTAs -> this, us (rows x features x
-// K): 200 x 10928 x 2048 153 -> 58 (52 with sums of 32 units), 200 x 2048 x 5464 54 -> 35, 128 x 10928 x 2048 78 -> 43, 1000 x 1024 x 1024 31.5 -> 22, 2048 x 6176 x 1024
+// Bound: 24 MMAs of 12 BN cycles together per unit, with the loads (64 KB per CTA and unit at BN 256) and the folds right behind: tensor pipe 59 % active, load and store pipe 53 %
+// (200 x 10928 x 2048).  One B200, single CTAs -> this, us (rows x features x K): 200 x 10928 x 2048 153 -> 58 (52 with sums of 32 units), 200 x 2048 x 5464 54 -> 35, 128 x 10928 x 2048 78 -> 43, 1000 x 1024 x 1024 31.5 -> 22, 2048 x 6176 x 1024
 // 263 -> 128, 2048 x 10928 x 2048 759 -> 400.  Error against float64 (2-norm), normal operands; one sign: 200 x 10928 x 2048 1.04e-7 -> 1.05e-7 (1.13e-7 with sums of 32); 9.6e-8 -> 9.7e-8,
 // 200 x 2048 x 5464 1.25e-7 -> 1.16e-7; 9.6e-8 -> 9.8e-8, 2048 x 6176 x 1024 1.09e-7 -> 1.07e-7; 1.07e-7 -> 1.04e-7, 2048 x 10928 x 2048 1.31e-7 -> 1.29e-7; 1.23e-7 -> 1.20e-7,
 // 400 x 512 x 512 9.2e-8 -> 9.1e-8; 9.5e-8 -> 9.4e-8.  (Sums are added as they come: a factor on them against the mean of what the tensor core cuts off would change those that are exact.)

@@ -156,8 +156,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(const float* __restric
 // Bound: bytes where they do not fit the L2 (8 rows x 2000 tokens x 4096 channels: 4.2 TB/s), a memory latency and the activations' issue below.  One B200, in a chain of
 // itself, us, walking a chunk of tokens (above) -> 4 tokens a thread | 8 (five CTAs per SM; one to four 21.7, six 19.5, eight 21.2; 12 tokens 18.9, 16 21.7): 2 rows x 1000 x 4096
 // 23.6 -> 21.9 | 17.6, 1 x 2048 x 2048 12.6 -> 12.6 | 11.0, 8 x 2000 x 4096 146 -> 169 | 124, 1 x 1000 x 2048 7.9 -> 7.5 | 7.4, 1 x 1000 x 1536 7.3 -> 6.8 | 7.1, 2 x 500 x 1024 6.8 -> 4.7 |
-// 5.7, 1 x 100 x 256 6.5 -> 3.2 | 4.7, 1 x 12 x 512 4.1 -> 3.2 | 4.9: eight tokens from CV_LARGE values on.  Up to 8 tokens the walk is one round too: 16 x 8 x 512 3.3 -> 3.4 | 4.7
-// (a delta-rule layer of 2 x 1000 tokens 205.3 -> 202.7).
+// 5.7, 1 x 100 x 256 6.5 -> 3.2 | 4.7, 1 x 12 x 512 4.1 -> 3.2 | 4.9: eight tokens from CV_LARGE values on.  Up to 8 tokens the walk is one round too: 16 x 8 x 512 3.3 -> 3.4 | 4.7.
 constexpr int CV_TAPS = 4, CV_MIN = 9;
 constexpr long CV_LARGE = 2000000;
 template <typename T, int ACT, int TOK>

@@ -277,36 +277,31 @@ bool linear_f32_takes(int M, int K, int ldx, const LinearGroup& g, const void* x
 
 // Rows per tile and parts of K: the least time of the busiest SM in cycles, from what a CTA takes per 64 k, to begin and end, and to
 // meet its cluster (fitted to the times above and their neighbours; clusters of eight wait for a place).
-static void lf_plan(int M, int N, int K, int nbatch, bool sorted, int& bn, int& splits) {
+static LinearF32Plan lf_plan(int M, int N, int K, int nbatch, bool sorted) {
   static const struct { int bn; double cycles; } shapes[] = {{32, 2000.0}, {64, 2300.0}, {128, 3400.0}};
   const int k_blocks = (K + LF_BK - 1) / LF_BK;
   double best = 1e300;
-  bn = 64;
-  splits = 1;
+  LinearF32Plan p{64, 1, 0, 0};
   for (const auto& sh : shapes) {
     const long tiles = (long)((M + sh.bn - 1) / sh.bn) * ((N + LF_BM - 1) / LF_BM) * nbatch;
     if (sorted && sh.bn > LT_BM) continue;
     for (int s = 1; s <= 8; s *= 2) {
       if (s > 1 && k_blocks / s < 2) break;
       const double t = (double)((tiles * s + SMS - 1) / SMS) * (4000.0 + sh.cycles * ((k_blocks + s - 1) / s) + (s == 1 ? 0.0 : s < 8 ? 5000.0 : 9000.0));
-      if (t < best) { best = t; bn = sh.bn; splits = s; }
+      if (t < best) { best = t; p = {sh.bn, s, (k_blocks + s - 1) / s, tiles}; }
     }
   }
+  return p;
 }
 
-int linear_f32_chain(int M, int N, int K) {
-  int bn, splits;
-  lf_plan(M, N, K, 1, false, bn, splits);
-  return ((K + LF_BK - 1) / LF_BK + splits - 1) / splits;
-}
+LinearF32Plan linear_f32_plan(int M, int N, int K) { return lf_plan(M, N, K, 1, false); }
 
 cudaError_t linear_f32_launch(const float* x, int ldx, const float* w, float* out, int ldo, int M, int N, int K, int act, float p0, float p1,
                               cudaStream_t st, const LinearGroup& g, int nbatch) {
-  int bn, splits;
-  lf_plan(M, N, K, g.tile_group ? 1 : nbatch, g.tile_group != nullptr, bn, splits);
-  const LinearF32 p{x, w, out, ldx, ldo, M, N, K, act, splits, p0, p1, g};
-  if (bn == 32) return lf_launch<32>(p, nbatch, st);
-  if (bn == 64) return lf_launch<64>(p, nbatch, st);
+  const LinearF32Plan plan = lf_plan(M, N, K, g.tile_group ? 1 : nbatch, g.tile_group != nullptr);
+  const LinearF32 p{x, w, out, ldx, ldo, M, N, K, act, plan.splits, p0, p1, g};
+  if (plan.bn == 32) return lf_launch<32>(p, nbatch, st);
+  if (plan.bn == 64) return lf_launch<64>(p, nbatch, st);
   return lf_launch<128>(p, nbatch, st);
 }
 

@@ -41,8 +41,9 @@ __device__ __forceinline__ void lf_split8(const float4& a, const float4& b, uint
 
 // whether the tensor-core kernel takes these sizes, pitches and addresses
 bool linear_f32_takes(int M, int K, int ldx, const LinearGroup& g, const void* x, const void* w);
-// sums of 64 k that one of its accumulators adds in a row for a plain product of these sizes
-int linear_f32_chain(int M, int N, int K);
+// how it takes a plain product of these sizes: rows per tile, CTAs that share one, sums of 64 k that each of them adds in a row, tiles
+struct LinearF32Plan { int bn, splits, chain; long tiles; };
+LinearF32Plan linear_f32_plan(int M, int N, int K);
 cudaError_t linear_f32_launch(const float* x, int ldx, const float* w, float* out, int ldo, int M, int N, int K, int act, float p0, float p1,
                               cudaStream_t st, const LinearGroup& g, int nbatch);
 

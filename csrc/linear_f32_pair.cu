@@ -4,7 +4,7 @@
 // long before the tensor core does.  Here the two CTAs of a pair each read and cut 128 features and HALF of the BN rows, and
 // `tcgen05.mma.cta_group::2` multiplies all 256 features with all BN rows: twice the products for the same loads, cuts and shared
 // memory.  The products of 64 k, their order and the rounded fp32 additions of their sums are those of the single CTA, so a sum over K that
-// one pair walks alone has the same bits.
+// neither of them parts has the same bits.
 //
 //   * 8 producer warps per CTA read float32 rows, cut them into three bfloat16 parts each and write 2 x 3 swizzled tiles; both CTAs'
 //     warps arrive on the leader's barrier;
@@ -313,30 +313,39 @@ __global__ void __launch_bounds__(LPS_THREADS) linear_f32_pair_sum_kernel(const 
   }
 }
 
-// Rows per tile, and whether runs end inside tiles: the least time of the busiest pair.  A unit costs the longer of its MMAs and its loads (cycles); parts
-// are written, read and added in some 10000 cycles.
-static void lp_plan(int M, int N, int K, int num_sms, LinearPair& p, int& bn) {
-  static const int sizes[] = {128, 192, 224, 256};
+// Rows per tile, and whether runs end inside tiles: the least time in us, from what the busiest pair takes to begin, per unit, tile and fold, and what partial tiles
+// cost (fitted to 130 sizes with every choice of the two and weights out of memory: 6 % off in the mean, its picks 0.3 % above the best).  False: the single CTAs are faster.
+static bool lp_plan(int M, int N, int K, int num_sms, LinearPair& p, int& bn) {
+  static const struct { int bn; double unit; } shapes[] = {{256, 2.47}, {224, 2.11}, {192, 1.77}, {128, 1.28}};
+  const LinearF32Plan single = linear_f32_plan(M, N, K);
   double best = 1e300;
-  p.fold = linear_f32_chain(M, N, K) < LP_FOLD ? linear_f32_chain(M, N, K) : LP_FOLD;
-  for (int b : sizes) {
-    const int mt = (M + b - 1) / b, tiles = mt * ((N + 2 * LP_BM - 1) / (2 * LP_BM)), blocks = (K + LP_BK - 1) / LP_BK;
-    const double unit = b * 12.0 > 13.0 * (LP_BM + b / 2) ? b * 12.0 + 100 : 13.0 * (LP_BM + b / 2) + 100;
+  p.fold = single.chain < LP_FOLD ? single.chain : LP_FOLD;
+  for (const auto& sh : shapes) {
+    const int mt = (M + sh.bn - 1) / sh.bn, tiles = mt * ((N + 2 * LP_BM - 1) / (2 * LP_BM)), blocks = (K + LP_BK - 1) / LP_BK;
     for (int split = 0; split < 2; ++split) {
       int pairs = num_sms / 2;
       if (!split && pairs > tiles) pairs = tiles;
       if (split && (long long)pairs * 4 > (long long)tiles * blocks) pairs = tiles * blocks / 4;
       if (pairs < 1) continue;
-      const double units = split ? (double)(((long long)tiles * blocks + pairs - 1) / pairs) : (double)((tiles + pairs - 1) / pairs) * blocks;
-      const double t = 5000.0 + units * unit + (split ? 10000.0 : 0.0);
-      if (t < best) {
-        best = t; bn = b;
+      const long long units = split ? ((long long)tiles * blocks + pairs - 1) / pairs : (long long)((tiles + pairs - 1) / pairs) * blocks;
+      const int run = units < blocks ? (int)units : blocks;                 // most units of a tile
+      const double of_run = (double)units / run;
+      const double t = 3.9 + sh.unit * units + of_run * (1.6 + 2.4 * ((run - 1) / p.fold) * sh.bn / 256) +
+                       (split ? 0.4 + (double)blocks / run * (0.26 + 0.48e-3 * (tiles < pairs ? tiles : pairs) * sh.bn) : 0.0);
+      if (t < (sh.bn == bn ? best : 0.97 * best)) {                         // (fewer rows a tile: more ways of the weights through the L2)
+        best = t; bn = sh.bn;
         p.m_tiles = mt; p.tiles = tiles; p.blocks = blocks; p.pairs = pairs; p.split = split;
+        p.slots = (split ? 2 : 0) + (run > p.fold);
       }
     }
   }
-  const long long run = p.split ? ((long long)p.tiles * p.blocks + p.pairs - 1) / p.pairs : p.blocks;      // most units of a tile in a run
-  p.slots = (p.split ? 2 : 0) + ((run < p.blocks ? run : p.blocks) > p.fold);
+  // What the single CTAs take, likewise, with as many clusters of 2, 4 and 8 at once as find a place.  Of 1806 sizes (65 to 2500 rows, 256 to 12000 features, K 256 to 8200, weights out
+  // of memory) six that go to the pairs are slower there by more than 2 % (at most 11 %), 64 that stay would be faster by more than 3 % (at most 18 %).  Near the line, us, single CTAs |
+  // pairs: 300 x 300 x 512 8.1 | 12.8, 512 x 256 x 1024 10.2 | 12.0, 128 x 2048 x 1024 13.1 | 13.7, 160 x 512 x 2048 13.8 | 16.2, 288 x 908 x 356 10.5 | 14.0; 257 x 256 x 256 9.7 | 9.0,
+  // 540 x 674 x 884 18.8 | 15.9, 257 x 256 x 4096 26.9 | 16.1.
+  const int at_once = single.splits == 8 ? 15 : single.splits == 4 ? 33 : num_sms / single.splits;
+  const double more = single.splits == 8 ? -1.9 : single.splits == 4 ? -0.8 : single.splits == 2 ? 1.9 : 0.0, block = single.bn == 32 ? 0.80 : single.bn == 64 ? 1.36 : 2.43;
+  return best < 1.1 + (double)((single.tiles + at_once - 1) / at_once) * (7.0 + more + block * single.chain);
 }
 
 template <int BN>
@@ -351,8 +360,8 @@ static cudaError_t lp_launch(const LinearPair& p, cudaStream_t st) {
 
 using namespace jl;
 
-// From the sizes on where it beats the single CTAs (us, single CTAs | this: 128 x 1024 x 1024 10.4 | 11.9, 128 x 2048 x 1024 13.0 | 12.4; 256 x 512 x 1024 10.4 | 12.2, 256 x 1024 x
-// 512 10.2 | 11.3, 129 x 1024 x 1024 12.6 | 12.4; 300 x 512 x 1024 12.8 | 12.2, 400 x 256 x 256 9.9 | 9.3); 16-byte loads along K.
+// Where it may beat the single CTAs (lp_plan compares; us, single CTAs | this: 128 x 1024 x 1024 10.4 | 11.9, 256 x 512 x 1024 10.4 | 12.2, 256 x 1024 x 512 10.2 | 11.3); 16-byte
+// loads along K.
 static bool lp_takes(int M, int N, int K, int ldx, const void* x, const void* w) {
   return M > 64 && N >= 256 && (M > 256 || (long long)N * K >= (M > 128 ? 1 << 20 : 1 << 21)) && K >= 256 && K % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 && (long long)N * K < (1ll << 31) &&
          (long long)M * ldx < (1ll << 31);
@@ -362,7 +371,7 @@ extern "C" JL_API long long jl_linear_f32_pair_ws(const void* x, int ldx, const 
   if (!lp_takes(M, N, K, ldx, x, w)) return -1;
   LinearPair p{};
   int bn = 0;
-  lp_plan(M, N, K, num_sms, p, bn);
+  if (!lp_plan(M, N, K, num_sms, p, bn)) return -1;
   return (long long)((size_t)p.pairs * p.slots * lp_part(bn) * sizeof(float));
 }
 
@@ -372,7 +381,7 @@ extern "C" JL_API int jl_linear_f32_pair(const void* x, int ldx, const void* w, 
   JL_CHECK_ARG(ldx >= K && ldo >= N, "jl_linear_f32_pair: bad pitch ldx=%d ldo=%d (N=%d K=%d)", ldx, ldo, N, K);
   LinearPair p{};
   int bn = 0;
-  lp_plan(M, N, K, num_sms, p, bn);
+  if (!lp_plan(M, N, K, num_sms, p, bn)) return JL_ERR_UNSUPPORTED;
   JL_CHECK_ARG(p.slots == 0 || (ws != nullptr && ((uintptr_t)ws & 15) == 0), "jl_linear_f32_pair: a workspace of 16-byte alignment is needed");
   p.x = (const float*)x; p.w = (const float*)w; p.out = (float*)out; p.ws = (float*)ws;
   p.ldx = ldx; p.ldo = ldo; p.M = M; p.N = N; p.K = K;

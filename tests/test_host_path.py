@@ -43,8 +43,8 @@ def test_same_answers(pair, name, args):
     assert getattr(fast, name)(*args) == getattr(slow, name)(*args)
 
 
-@pytest.mark.parametrize("M,N,K,pairs,slots,rows", [(300, 256, 256, 0, 0, 0), (65, 2048, 1024, 32, 2, 128), (2048, 6176, 1024, 74, 2, 256), (200, 10928, 2048, 74, 3, 224),
-                                                    (2000, 256, 4096, 74, 2, 256), (18944, 256, 4096, 74, 1, 256)])
+@pytest.mark.parametrize("M,N,K,pairs,slots,rows", [(300, 256, 256, 0, 0, 0), (65, 3000, 1024, 48, 2, 128), (2048, 6176, 1024, 74, 2, 256), (200, 10928, 2048, 74, 3, 224),
+                                                    (2000, 256, 4096, 74, 2, 128), (18944, 256, 4096, 74, 1, 256)])
 def test_workspace_of_the_float32_pairs(pair, M, N, K, pairs, slots, rows):
     """Two partial tiles a pair where runs end inside tiles, a further one only where a pair adds more blocks than it may in a row (148 SMs)."""
     assert pair[0].jl_linear_f32_pair_ws(4096, K, 8192, M, N, K, 148) == pairs * slots * rows * 256 * 4

@@ -14,6 +14,7 @@
 
 #include "common.cuh"
 #include "jllama_b200.h"
+#include "seq_types.cuh"
 
 namespace jl {
 
@@ -83,8 +84,8 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   constexpr int LPK = HD / 8;            // lanes per key row
   constexpr int GPW = 32 / LPK;          // lane-groups per warp
   constexpr int NG = DA_WARPS * GPW;     // lane-groups per CTA
-  __shared__ float s_o[NG][G][HD];
-  __shared__ float s_ml[NG][G][2];
+  __shared__ float s_o[NG + STEP][G][HD];      // STEP: the new key is a group of its own
+  __shared__ float s_ml[NG + STEP][G][2];
 
   pdl_wait();
   pdl_launch_dependents();
@@ -105,11 +106,11 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   int chunk = (valid + splits - 1) / splits;
   chunk = ((chunk + KEYS_PER_ITER - 1) / KEYS_PER_ITER) * KEYS_PER_ITER;
   const int lo = first + split * chunk;
-  const int hi = lo + chunk < len ? lo + chunk : len;
+  int hi = lo + chunk < len ? lo + chunk : len;
 
   __shared__ __align__(16) __nv_bfloat16 s_new[STEP ? G + 2 : 1][HD];      // query heads | new key | new value
   __shared__ float s_gate[STEP ? G : 1];
-  int slot = -1;                                                           // of the new token, where this CTA holds its key and value
+  bool fresh = false;                                                      // the new token's key is one of this CTA's: the last, and only in shared memory
   if constexpr (STEP) {
     const float* row = step.y + (size_t)b * step.ldy;
     const int at = len - 1;                                                // (a full cache: the last slot, which nothing is written to)
@@ -128,11 +129,28 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     if (gates) s_gate[g] = gate_sigmoid(gate);                             // (read behind the barrier at the end)
     __syncthreads();
     if (own) {
-      slot = at;
       const size_t to = (((size_t)b * nkv + kvh) * T + at) * HD + (threadIdx.x % LPK) * 8;
       if (threadIdx.x < 2 * LPK)
         *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(threadIdx.x < LPK ? kc : vc) + to) =
             *reinterpret_cast<const uint4*>(&s_new[G + threadIdx.x / LPK][(threadIdx.x % LPK) * 8]);
+    }
+    fresh = own && valid > 0;
+    if (fresh) {
+      hi = at;
+      for (int i = warp; i < G; i += DA_WARPS) {
+        float s = 0.0f;
+#pragma unroll
+        for (int u = 0; u < HD / 64; ++u) {
+          const int c = 2 * (lane + 32 * u);
+          const uint32_t qv = *reinterpret_cast<const uint32_t*>(&s_new[i][c]), kv = *reinterpret_cast<const uint32_t*>(&s_new[G][c]),
+                         vv = *reinterpret_cast<const uint32_t*>(&s_new[G + 1][c]);
+          s = fmaf(bf16_lo(qv) * scale_log2, bf16_lo(kv), s);
+          s = fmaf(bf16_hi(qv) * scale_log2, bf16_hi(kv), s);
+          *reinterpret_cast<float2*>(&s_o[NG][i][c]) = make_float2(bf16_lo(vv), bf16_hi(vv));
+        }
+        s = warp_sum(s);
+        if (lane == 0) { s_ml[NG][i][0] = s; s_ml[NG][i][1] = 1.0f; }
+      }
     }
   }
 
@@ -166,14 +184,9 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     uint4 kr[DA_KPI], vr[DA_KPI];
 #pragma unroll
     for (int i = 0; i < DA_KPI; ++i) {
-      const bool ok = key0 + i < hi && (!STEP || key0 + i != slot);
+      const bool ok = key0 + i < hi;
       kr[i] = ok ? ldg_stream(kbase + (size_t)(key0 + i) * HD) : make_uint4(0, 0, 0, 0);
       vr[i] = ok ? ldg_stream(vbase + (size_t)(key0 + i) * HD) : make_uint4(0, 0, 0, 0);
-      if constexpr (STEP)
-        if (key0 + i == slot) {
-          kr[i] = *reinterpret_cast<const uint4*>(&s_new[G][lig * 8]);
-          vr[i] = *reinterpret_cast<const uint4*>(&s_new[G + 1][lig * 8]);
-        }
     }
     float part[G][DA_KPI];
 #pragma unroll
@@ -245,6 +258,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     float M = -INFINITY;
 #pragma unroll
     for (int j = 0; j < NG; ++j) M = fmaxf(M, s_ml[j][g][0]);
+    if (fresh) M = fmaxf(M, s_ml[NG][g][0]);
     const float Ms = M == -INFINITY ? 0.f : M;
     float acc = 0.f, L = 0.f;
 #pragma unroll
@@ -252,6 +266,11 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
       const float w = exp2f(s_ml[j][g][0] - Ms);
       acc += w * s_o[j][g][d];
       L += w * s_ml[j][g][1];
+    }
+    if (fresh) {
+      const float w = exp2f(s_ml[NG][g][0] - Ms);
+      acc += w * s_o[NG][g][d];
+      L += w * s_ml[NG][g][1];
     }
     const int h = kvh * G + g;
     if (splits == 1) {
@@ -293,7 +312,17 @@ template <int G, int HD>
 static cudaError_t launch_decode(const void* q, const void* kc, const void* vc, const int* cache_len_ptr,
                                  const int* pad_left, float* o_part, float* ml_part, void* out, int B,
                                  int nkv, int T, int n_new, float scale, int splits, int q_bstride, cudaStream_t s, const AttnStep* step = nullptr) {
-  cudaError_t e = launch_pdl(step ? decode_attn_kernel<G, HD, true> : decode_attn_kernel<G, HD>, dim3(splits, nkv, B), dim3(DA_WARPS * 32), 0, s,
+  // A step's CTAs are placed while the projection before them still fills most SMs, and came to lie many to an SM.  Shared memory that only one or two of them find on an SM spreads
+  // them (us in a graph, the layer without | with: 2 rows x 4 heads of 128, 1000 keys 16.4 | 11.5, 4 x 8 heads over 2, 2000 keys 20.8 | 16.2; in three launches 13.5, 16.9).
+  constexpr size_t FIXED = ((DA_WARPS * 256 / HD + 1) * G * (HD + 2) + G) * sizeof(float) + (G + 2) * HD * 2;
+  size_t smem = 0;
+  if (step) {
+    const long ctas = (long)splits * nkv * B;
+    if (ctas <= 2 * SMS) smem = (ctas <= SMS ? 116 : 80) * 1024 - FIXED;
+    const cudaError_t ae = cudaFuncSetAttribute(decode_attn_kernel<G, HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024 - (int)FIXED);
+    if (ae != cudaSuccess) return ae;
+  }
+  cudaError_t e = launch_pdl(step ? decode_attn_kernel<G, HD, true> : decode_attn_kernel<G, HD>, dim3(splits, nkv, B), dim3(DA_WARPS * 32), smem, s,
                              (const __nv_bfloat16*)q, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc,
                              cache_len_ptr, pad_left, o_part, ml_part, (__nv_bfloat16*)out, nkv, T, n_new,
                              scale * 1.4426950408889634f, splits, q_bstride, step ? *step : AttnStep());

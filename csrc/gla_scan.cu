@@ -776,7 +776,14 @@ extern "C" JL_API int jl_gla_step(const float* y, int ldy, int q_off, int k_off,
   if (threads > 1024 || B > 65535) return JL_ERR_UNSUPPORTED;
   GlaStep s{GlaParams{y, ldy, q_off, k_off, v_off, a_off, B, 1, H, D, Dv, R, 1, q_scale, 1.0f / tau, cache_len, pad_left, state, nullptr}, g_off, eps, gate_act};
   s.p.k_scale = 1.0f;
-  const size_t smem = (size_t)(3 * threads / cols * dp + threads) * sizeof(float);
+  size_t smem = (size_t)(3 * threads / cols * dp + threads) * sizeof(float);             // (16 KB at most)
+  if ((long)H * B <= SMS) {
+    // placed while the projection before fills most SMs, the CTAs came to lie many to an SM: with this much each has its own (us in a graph, a layer of 3 rows x 16 heads of 16 x 64
+    // 12.0 -> 11.1, 7 x 8 heads of 100 x 128 18.6 -> 17.3; in two launches 11.3 and 19.7)
+    smem = 116 * 1024;
+    if (dp == 16) JL_DISPATCH_DTYPE(dtype, JL_CUDA(cudaFuncSetAttribute((gla_step_kernel<T, 16>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
+    else JL_DISPATCH_DTYPE(dtype, JL_CUDA(cudaFuncSetAttribute((gla_step_kernel<T, 32>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
+  }
   if (dp == 16)
     JL_DISPATCH_DTYPE(dtype, JL_LAUNCH_PDL((gla_step_kernel<T, 16>), dim3(H, B), dim3(threads), smem, (cudaStream_t)stream, s, (const T*)a2,
                                            (const T*)a2_bias, (const T*)norm, (T*)out));

@@ -594,7 +594,8 @@ static int gc_chunks(int S) { return (S + GC_T - 1) / GC_T; }
 // 42.2 -> 34.1, 200 61.3 -> 34.9, 4 rows x 8 heads 40 39.9 -> 41.6, 48 41.3 -> 37.6.
 // Decays that are given (one per head, or per token and head) always walk: nothing of their own covers what the tensor core cuts off and the roundings of products of 64 decays.  Error
 // against float64 (2-norm of the read-outs), walk -> this: one fixed decay of 0.9, operands of one sign, 500 tokens x 16 heads of 64 x 128 4.1e-8 -> 9.4e-8, decay 1 4.7e-8 ->
-// 1.4e-7; a float32 retention layer of 3 x 608 tokens, its state 1.18e-6 -> 1.49e-6.
+// 1.4e-7; a float32 retention layer of 3 x 608 tokens, its state 1.18e-6 -> 1.49e-6; 40 drawn float32 state space layers, their states 9 % further
+// off in the mean and 19 % at most (what is cut off has the sign of what the projections before lose), outputs 0 and 4 %.
 // Narrow heads, which are padded to 64 (128) channels and 128 columns here and not there: keys of 16 channels from 64 tokens on (4 rows x 4 heads of 16 x 64, 48 tokens 18.1 -> 21.0, 64 22.2 -> 21.0); once the
 // chunks fill the SMs several times the walk has them (4 rows x 16 heads, 1000 tokens of 16 x 64 91 -> 100, of 32 x 16 94 -> 98, 400 tokens of 100 x 32 97 -> 112, of 128 x 16 76 -> 111; of
 // 128 x 64 and 64 x 64 this).

@@ -143,7 +143,7 @@ def test_not_finite_operands(M, N, K):
 
 def test_what_stays_with_the_other_kernels():
     for M, N, K in [(64, 4096, 1024), (128, 1024, 1024), (200, 512, 1024), (300, 255, 512), (300, 512, 252), (300, 512, 510), (300, 300, 512), (512, 256, 1024), (160, 512, 2048),
-                    (65, 2048, 1024)]:
+                    (65, 2048, 1024), (129, 1024, 1024), (140, 1100, 1024)]:
         x, w = operands(M, N, K)
         assert workspace(x, w) == -1
         check(SK.linear(x, w), x, w)
